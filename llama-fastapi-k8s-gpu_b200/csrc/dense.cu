@@ -1,12 +1,14 @@
 // Dense products for the layer-list models: Y[T][N] = epi(X[T][K] . W[N][K]^T + bias), weights bf16 or f32 as stored
-// in the file, activations f32 in memory. Three kernels:
+// in the file, activations f32 in memory. Four kernels:
 //   dense_rows_kernel   T <= 8 (decode steps): one warp per weight row, the row is streamed once for all tokens
-//   dense_mma_kernel    T > 8, bf16 weights: tensor cores (mma.sync m16n8k16 bf16, f32 accumulate), X rounded to bf16
+//   dense_tc_kernel     T > 8, bf16 weights: tensor cores (dense_tc.cu), X rounded to bf16
+//   dense_mma_kernel    the same for rows that tensor copies cannot take (K % 8 != 0): mma.sync m16n8k16 bf16, f32 accumulate
 //   dense_fma_kernel    T > 8, exact mode (or f32 weights): 32-bit multiply-adds, nothing rounded
-// Every output element is one sum over k in a fixed order that depends only on (K, kernel), never on T or on the
+// Every output element is one sum over k in a fixed order that depends only on the matrix and the kernel, never on the
 // other rows, so a token's result is the same whatever else shares the step. Arbitrary T, N, K (edges are guarded).
 // The llama graph's counterpart (quantised blocks, tcgen05) is gemm.cu / matvec.cu.
 #include "kernels.h"
+#include "dense_dev.cuh"
 #include "layered.h"
 #include "ptx.cuh"
 #include "quant_blocks.cuh"
@@ -18,99 +20,6 @@ namespace b2 {
 
 __device__ __forceinline__ float ld_w(const __nv_bfloat16* w, size_t i) { return __bfloat162float(w[i]); }
 __device__ __forceinline__ float ld_w(const float* w, size_t i) { return w[i]; }
-
-// what a kernel needs beyond its operands: epilogue, batch strides, grouping (DenseArgs, by value)
-struct DenseDev {
-    const float* x; int ldx;
-    const void* w;
-    const float* bias;
-    float* y; int ldy;
-    int T, N, K, epi;
-    int n_act, n_act_end;          // EPI_BIAS_PART_RELU2
-    __nv_bfloat16* yb;             // large-tile kernel: rounded output instead of y, or null
-    float scale, p0, p1;
-    const float* aux; int ldaux, aux_ns;      // aux column of output column n: n * aux_ns
-    long x_bs, w_bs, y_bs, aux_bs;
-    int grouped;                   // 0 plain, 1 one pair per blockIdx.y, 2 tiles
-    DenseGroups g;
-};
-
-// The rows [t0, t1) this CTA computes and the operands they use. false: nothing to do.
-template <typename TW>
-__device__ __forceinline__ bool dense_tile(const DenseDev& a, int rows_per_cta, const float*& x, const TW*& w, float*& y, const float*& aux,
-                                           int& t0, int& t1, unsigned by, unsigned bz) {
-    x = a.x; w = reinterpret_cast<const TW*>(a.w); y = a.y; aux = a.aux;
-    if (a.grouped == 0) {
-        const long b = bz;
-        x += b * a.x_bs; w += b * a.w_bs; y += b * a.y_bs;
-        if (aux) aux += b * a.aux_bs;
-        t0 = by * rows_per_cta; t1 = a.T;
-        return t0 < t1;
-    }
-    if (a.grouped == 1) {
-        const int p = by, g = a.g.group[p];
-        if (g < 0 || g >= a.g.n_groups) return false;
-        w += (long)g * a.g.w_stride;
-        t0 = p; t1 = p + 1;
-        return true;
-    }
-    const int tile = by;
-    if (tile >= *a.g.n_tiles) return false;
-    w += (long)a.g.tile_group[tile] * a.g.w_stride;
-    t0 = a.g.tile_row0[tile]; t1 = t0 + a.g.tile_rows[tile];
-    return true;
-}
-__device__ __forceinline__ int x_row(const DenseDev& a, int t) { return (a.grouped && a.g.x_rows) ? a.g.x_rows[t] : t; }
-
-__device__ __forceinline__ float silu_act(float z) { return z / (1.f + expf(-z)); }
-__device__ __forceinline__ float gelu_tanh_act(float z) { return 0.5f * z * (1.f + tanhf(0.7978845608028654f * fmaf(0.044715f * z * z, z, z))); }
-// The epilogue kind is a.epi, or EPI when that is >= 0 (compiled in: the large-tile kernel, where products over a short K are
-// bound by their epilogue).
-template <int EPI>
-__device__ __forceinline__ float epi_value(const DenseDev& a, const float* aux, int t, int n, float v) {
-    const int epi = EPI >= 0 ? EPI : a.epi;
-    if (epi == EPI_BIAS || epi == EPI_BIAS_RELU2 || epi == EPI_BIAS_PART_RELU2) { if (a.bias) v += a.bias[n]; }
-    if (epi == EPI_BIAS_RELU2 || (epi == EPI_BIAS_PART_RELU2 && n >= a.n_act && n < a.n_act_end)) { v = fmaxf(v, 0.f); v = v * v; }
-    if (epi == EPI_MUL_SIGMOID) v *= 1.f / (1.f + expf(-aux[(size_t)t * a.ldaux + n * a.aux_ns]));
-    if (epi == EPI_PIECEWISE) v = v > 0.f ? fmaf(a.p0 * v, v, 0.5f * v) : fmaf(a.p1, expm1f(v) - v, 0.5f * v);
-    return v * a.scale;
-}
-// one output column
-__device__ __forceinline__ void epi_store(const DenseDev& a, float* y, const float* aux, int t, int n, float v) {
-    y[(size_t)t * a.ldy + n] = epi_value<-1>(a, aux, t, n, v);
-}
-// two neighbouring columns n (even) and n + 1; rs: scales of the product rows (GLU epilogues) or null; vec2: pairs of y are
-// 8-byte aligned
-template <int EPI = -1, bool ROUNDED = false>
-__device__ __forceinline__ void epi_store2(const DenseDev& a, float* y, const float* aux, const float* rs, int t, int n, float v0, float v1,
-                                           bool vec2 = false) {
-    const int epi = EPI >= 0 ? EPI : a.epi;
-    if (epi == EPI_GLU_SILU || epi == EPI_GLU_GELU || epi == EPI_GLU_CLAMP) {
-        if (n + 1 >= a.N) return;
-        if (rs) { v0 *= rs[t]; v1 *= rs[t]; }
-        float v;
-        if (epi == EPI_GLU_CLAMP) {
-            const float g = fminf(v0, a.p0), u = fminf(fmaxf(v1, -a.p0), a.p0);
-            v = g / (1.f + expf(-a.p1 * g)) * (u + 1.f);
-        } else v = (epi == EPI_GLU_SILU ? silu_act(v0) : gelu_tanh_act(v0)) * v1;
-        if constexpr (ROUNDED) a.yb[(size_t)t * a.ldy + (n >> 1)] = __float2bfloat16(v * a.scale);
-        else y[(size_t)t * a.ldy + (n >> 1)] = v * a.scale;
-        return;
-    }
-    if constexpr (ROUNDED) {
-        __nv_bfloat16* out = a.yb + (size_t)t * a.ldy + n;
-        if (n < a.N) out[0] = __float2bfloat16(epi_value<EPI>(a, aux, t, n, v0));
-        if (n + 1 < a.N) out[1] = __float2bfloat16(epi_value<EPI>(a, aux, t, n + 1, v1));
-        return;
-    }
-    float* dst = y + (size_t)t * a.ldy + n;
-    if (vec2 && n + 1 < a.N) {
-        *reinterpret_cast<float2*>(dst) = make_float2(epi_value<EPI>(a, aux, t, n, v0), epi_value<EPI>(a, aux, t, n + 1, v1));
-        return;
-    }
-    if (n < a.N) dst[0] = epi_value<EPI>(a, aux, t, n, v0);
-    if (n + 1 < a.N) dst[1] = epi_value<EPI>(a, aux, t, n + 1, v1);
-}
 
 // ---------------------------------------------------------------- few tokens: a warp per R weight rows
 // TT = compiled token count (1, 2, 4 or 8 >= T), R = rows per warp (the activations a lane loads serve R rows: with several
@@ -370,117 +279,14 @@ __global__ void __launch_bounds__(128) dense_mma_kernel(DenseDev a) {
             }
 }
 
-// ---------------------------------------------------------------- tensor cores, large steps: 128 x 128 x 64 tiles, 8 warps of
-// 64 x 32, three stages of 16-byte asynchronous copies, ldmatrix fragments. X is rounded to bf16 ONCE per product by
-// rows_to_bf16_kernel (the 64 x 64 kernel above converts every tile it loads, N / 64 times per element). Needs K % 8 == 0.
-__global__ void rows_to_bf16_kernel(const float* __restrict__ x, int ldx, int T, int K, __nv_bfloat16* __restrict__ y) {
-    griddep_launch();
-    griddep_wait();
-    const long n = (long)T * (K / 2);
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        const long t = i / (K / 2);
-        const int k = (int)(i % (K / 2)) * 2;
-        const float* p = x + t * ldx + k;
-        *reinterpret_cast<__nv_bfloat162*>(y + t * K + k) = __floats2bfloat162_rn(p[0], p[1]);
-    }
-}
-
-__device__ __forceinline__ void cp_async_16(void* smem_dst, const void* gsrc, int src_bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(smem_dst)), "l"(gsrc), "r"(src_bytes) : "memory");
-}
-__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const void* smem_src) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(smem_src)));
-}
-
-constexpr int BIG_BM = 128, BIG_BN = 128, BIG_BK = 64, BIG_LD = BIG_BK + 8, BIG_STAGES = 3;
-constexpr int BIG_SMEM = BIG_STAGES * (BIG_BM + BIG_BN) * BIG_LD * 2;
-template <int EPI, bool ROUNDED = false>
-__global__ void __launch_bounds__(256, 2) dense_mma_big_kernel(const __nv_bfloat16* __restrict__ xb, int ldxb, DenseDev a) {
-    griddep_launch();
-    griddep_wait();
-    extern __shared__ __align__(16) unsigned char big_smem[];
-    __nv_bfloat16* As = reinterpret_cast<__nv_bfloat16*>(big_smem);                       // [stage][BM][LD]
-    __nv_bfloat16* Bs = As + BIG_STAGES * BIG_BM * BIG_LD;                                  // [stage][BN][LD]
-    const float* x; const __nv_bfloat16* w; float* y; const float* aux; int t0, T;
-    if (!dense_tile<__nv_bfloat16>(a, BIG_BM, x, w, y, aux, t0, T, blockIdx.y, blockIdx.z)) return;
-    const int N = a.N, K = a.K;
-    const int n0 = blockIdx.x * BIG_BN;
-    // the rounded copy holds the input rows as [row][ldxb] (grouped: gathered here; batched: batch b starts at column b * x_bs)
-    if (!a.grouped) xb += (long)blockIdx.z * a.x_bs;
-    int my_rows[BIG_BK / 16];
-#pragma unroll
-    for (int it = 0; it < BIG_BK / 16; it++) {
-        const int row = (threadIdx.x + it * 256) / (BIG_BK / 8);
-        my_rows[it] = x_row(a, min(t0 + row, T - 1));
-    }
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int wm = (warp >> 2) * 64, wn = (warp & 3) * 32;
-    const int KT = (K + BIG_BK - 1) / BIG_BK;
-    auto load_stage = [&](int stage, int kt) {
-        const int k0 = kt * BIG_BK;
-#pragma unroll
-        for (int it = 0; it < BIG_BK / 16; it++) {
-            const int c = threadIdx.x + it * 256;          // 128 rows x BK / 8 chunks of 16 bytes per operand tile
-            const int row = c / (BIG_BK / 8), kk = (c % (BIG_BK / 8)) * 8;
-            const int k = k0 + kk;
-            const int t = t0 + row, n = n0 + row;
-            const bool ka = k < K;
-            cp_async_16(As + ((size_t)stage * BIG_BM + row) * BIG_LD + kk, xb + (size_t)my_rows[it] * ldxb + (ka ? k : 0), (ka && t < T) ? 16 : 0);
-            cp_async_16(Bs + ((size_t)stage * BIG_BN + row) * BIG_LD + kk, w + (size_t)min(n, N - 1) * K + (ka ? k : 0), (ka && n < N) ? 16 : 0);
-        }
-    };
-    float acc[4][4][4] = {};
-    for (int s = 0; s < BIG_STAGES - 1; s++) {
-        if (s < KT) load_stage(s, s);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-    for (int kt = 0; kt < KT; kt++) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(BIG_STAGES - 2) : "memory");
-        __syncthreads();
-        const int nxt = kt + BIG_STAGES - 1;
-        if (nxt < KT) load_stage(nxt % BIG_STAGES, nxt);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        const __nv_bfloat16* A = As + (size_t)(kt % BIG_STAGES) * BIG_BM * BIG_LD;
-        const __nv_bfloat16* B = Bs + (size_t)(kt % BIG_STAGES) * BIG_BN * BIG_LD;
-#pragma unroll
-        for (int ks = 0; ks < BIG_BK; ks += 16) {
-            uint32_t af[4][4], bf[2][4];
-#pragma unroll
-            for (int mi = 0; mi < 4; mi++) ldmatrix_x4(af[mi], A + (size_t)(wm + mi * 16 + (lane & 15)) * BIG_LD + ks + (lane >> 4) * 8);
-#pragma unroll
-            for (int nj = 0; nj < 2; nj++)
-                ldmatrix_x4(bf[nj], B + (size_t)(wn + nj * 16 + (lane & 7) + ((lane >> 4) << 3)) * BIG_LD + ks + ((lane >> 3) & 1) * 8);
-#pragma unroll
-            for (int mi = 0; mi < 4; mi++)
-#pragma unroll
-                for (int ni = 0; ni < 4; ni++) {
-                    const uint32_t b2[2] = {bf[ni >> 1][(ni & 1) * 2], bf[ni >> 1][(ni & 1) * 2 + 1]};
-                    mma_bf16_16816(acc[mi][ni], af[mi], b2);
-                }
-        }
-    }
-    const int g = lane >> 2, tq = lane & 3;
-    const bool vec2 = a.ldy % 2 == 0 && (reinterpret_cast<uintptr_t>(y) & 7) == 0;
-#pragma unroll
-    for (int mi = 0; mi < 4; mi++)
-#pragma unroll
-        for (int ni = 0; ni < 4; ni++)
-#pragma unroll
-            for (int e = 0; e < 4; e += 2) {
-                const int t = t0 + wm + mi * 16 + g + (e >> 1) * 8;
-                if (t < T) epi_store2<EPI, ROUNDED>(a, y, aux, a.g.row_scale, t, n0 + wn + ni * 8 + 2 * tq, acc[mi][ni][e], acc[mi][ni][e + 1], vec2);
-            }
-}
-
-// The large-tile kernel reads a rounded copy of the input: [T][K]; batched: [T][x_span] with batch b at column b * x_bs; grouped
-// (128-row tiles): [x_total_rows][K], gathered by the kernel.
+// The tcgen05 kernel reads a rounded copy of the input: [T][K]; batched: [T][x_span] with batch b at column b * x_bs; grouped: the rows of
+// the sorted pairs. Its operands are tensor maps: rows of whole 16-byte pieces on 16-byte boundaries.
 bool dense_takes_rounded(const DenseArgs& a) {
     const int span = a.batch > 1 ? a.x_span : a.K;
     const bool tiled = a.groups && a.groups->tile_group;
     const bool ok = a.w_type == T_BF16 && !a.exact && a.xb && a.K % 8 == 0 && (reinterpret_cast<uintptr_t>(a.w) & 15) == 0 && span % 8 == 0 &&
                     (a.batch == 1 || (a.x_span > 0 && a.x_bs % 8 == 0 && a.w_bs % 8 == 0));
-    return ok && (a.groups ? tiled && a.groups->tile_max == BIG_BM : a.T >= 64);
+    return ok && (a.groups ? tiled : a.T > ROWS_MAX_T);
 }
 
 static DenseDev dense_dev(const DenseArgs& a) {
@@ -533,43 +339,8 @@ cudaError_t dense_launch(const DenseArgs& a, cudaStream_t s) {
         return wb ? launch_rows<__nv_bfloat16>(c, 1, s) : launch_rows<float>(c, 1, s);
     }
     const unsigned gz = d.grouped ? 1 : a.batch;
-    const int x_rows_total = d.grouped ? a.groups->x_total_rows : a.T;
-    const int span = a.batch > 1 ? a.x_span : a.K;
-    const bool big = dense_takes_rounded(a);
-    if ((d.grouped == 2 && a.groups->tile_max == BIG_BM && !big) || (!big && (a.x_rounded || a.y_rounded))) return cudaErrorInvalidValue;
-    if (big) {
-        static const auto kernels = [] {
-            std::array<void (*)(const __nv_bfloat16*, int, DenseDev), 9> k = {
-                dense_mma_big_kernel<EPI_NONE>, dense_mma_big_kernel<EPI_BIAS>, dense_mma_big_kernel<EPI_BIAS_RELU2>, dense_mma_big_kernel<EPI_GLU_SILU>,
-                dense_mma_big_kernel<EPI_MUL_SIGMOID>, dense_mma_big_kernel<EPI_GLU_CLAMP>, dense_mma_big_kernel<EPI_PIECEWISE>, dense_mma_big_kernel<EPI_GLU_GELU>,
-                dense_mma_big_kernel<EPI_BIAS_PART_RELU2>};
-            for (auto f : k) cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, BIG_SMEM);
-            return k;
-        }();
-        if (a.epi < 0 || a.epi >= (int)kernels.size()) return cudaErrorInvalidValue;
-        const __nv_bfloat16* xb = a.x_rounded;
-        if (!xb) {
-            const long pairs = (long)x_rows_total * (span / 2);
-            const cudaError_t ce = launch_chain(rows_to_bf16_kernel, dim3((unsigned)std::min<long>((pairs + 255) / 256, 148 * 8)), dim3(256), 0, s,
-                                                a.x, a.ldx, x_rows_total, span, a.xb);
-            if (ce != cudaSuccess) return ce;
-            xb = a.xb;
-        }
-        const unsigned gy = d.grouped ? (unsigned)a.groups->max_tiles : (unsigned)((a.T + BIG_BM - 1) / BIG_BM);
-        auto kernel = kernels[a.epi];
-        if (a.y_rounded) {             // outputs that only feed the next product: the activations of experts
-            static const auto rounded = [] {
-                std::array<void (*)(const __nv_bfloat16*, int, DenseDev), 3> k = {
-                    dense_mma_big_kernel<EPI_BIAS_RELU2, true>, dense_mma_big_kernel<EPI_GLU_SILU, true>, dense_mma_big_kernel<EPI_GLU_CLAMP, true>};
-                for (auto f : k) cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, BIG_SMEM);
-                return k;
-            }();
-            const int which = a.epi == EPI_BIAS_RELU2 ? 0 : a.epi == EPI_GLU_SILU ? 1 : a.epi == EPI_GLU_CLAMP ? 2 : -1;
-            if (which < 0) return cudaErrorInvalidValue;
-            kernel = rounded[which];
-        }
-        return launch_chain(kernel, dim3((a.N + BIG_BN - 1) / BIG_BN, gy, gz), dim3(256), (size_t)BIG_SMEM, s, xb, span, d);
-    }
+    if (dense_takes_rounded(a)) return dense_tc_launch(a, d, s);
+    if (a.x_rounded || a.y_rounded || (d.grouped == 2 && a.groups->tile_max != 64)) return cudaErrorInvalidValue;
     dim3 grid((a.N + 63) / 64, d.grouped ? (unsigned)a.groups->max_tiles : (unsigned)((a.T + 63) / 64), gz);
     if (wb && !a.exact) return launch_chain(dense_mma_kernel, grid, dim3(128), 0, s, d);
     if (wb) return launch_chain(dense_fma_kernel<__nv_bfloat16>, grid, dim3(256), 0, s, d);

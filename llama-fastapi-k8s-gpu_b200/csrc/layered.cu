@@ -341,7 +341,7 @@ int layered_finalize(b2_engine* e) {
     if (c.block_style == B2_BLOCK_PRENORM_RMS && (rc = vec_f32(e, m, "embed.norm", W, 1, &m->embed_norm))) return rc;
     const size_t cache_esz = m->exact ? 4 : 2;
     size_t max_proj = 1, max_buf = 1, max_ff = 1, max_attn = 0, max_attn_d = 0, max_glu = 0;
-    size_t moe_pairs = 0, moe_slots = 0, moe_ff = 0, moe_experts = 0, moe_xb = 0;     // moe_xb: expert activations per step token
+    size_t moe_pairs = 0, moe_slots = 0, moe_ff = 0, moe_experts = 0, moe_xb = 0;     // moe_xb: entries of the gathered inputs of the experts per step token
     const bool hyper = c.block_style == B2_BLOCK_HYPER_RMS;
     const int n_streams = std::max(1, c.n_streams);
     size_t max_mix = 0;                                    // mixer output row, with what rides along
@@ -651,7 +651,7 @@ int layered_finalize(b2_engine* e) {
             moe_pairs = std::max<size_t>(moe_pairs, (size_t)Tm * d.moe_top);
             if (!table) moe_slots = std::max<size_t>(moe_slots, slots);
             moe_ff = std::max<size_t>(moe_ff, d.n_ff);
-            moe_xb = std::max<size_t>(moe_xb, (size_t)d.moe_top * d.n_ff);
+            moe_xb = std::max<size_t>(moe_xb, (size_t)d.moe_top * std::max(d.n_ff, W));
             moe_experts = std::max<size_t>(moe_experts, d.moe_experts);
         } else if (d.n_ff > 0 && d.ff_kind == B2_FF_PIECEWISE) {
             float* act = nullptr;
@@ -996,6 +996,11 @@ static bool takes_rounded(const LayeredModel* m, const DenseW& w, int T) {
     return dense_takes_rounded(a);
 }
 
+// the grouped products of a mixture (more than MOE_FEW_TOKENS tokens) take rounded inputs
+static bool moe_takes_rounded(const LayeredModel* m, const LyLayer& L) {
+    return !m->exact && m->xb && L.gate_up.type == T_BF16 && m->c.n_embd % 8 == 0 && L.d.n_ff % 8 == 0;
+}
+
 // ---- token mixers: each reads the sublayer input `in` [T][W] and leaves its output in m->oL (the two-branch mixer also m->oR)
 static int mix_window_scan(b2_engine* e, LayeredModel* m, LyLayer& L, const RaggedDev& r, const float* in) {
     const b2_layered_config& c = m->c;
@@ -1338,8 +1343,8 @@ static int moe_prepare(b2_engine* e, LayeredModel* m, LyLayer& L, const RaggedDe
     DenseGroups& g = j.g;
     g.n_groups = d.moe_experts;
     const bool tiled = T > MOE_FEW_TOKENS, table = d.moe_route == B2_ROUTE_TABLE;
-    // long prompts in the serving mode: 128-row tiles through the large tensor-core kernel
-    const bool big = tiled && !m->exact && L.gate_up.type == T_BF16 && pairs >= MOE_BIG_PAIRS && W % 8 == 0 && ff % 8 == 0 && m->xb;
+    // the serving mode rounds what its products read; long prompts take 128-row tiles
+    const bool rounded = tiled && moe_takes_rounded(m, L), big = rounded && pairs >= MOE_BIG_PAIRS;
     g.tile_max = big ? 128 : 64;
     const int *sel = m->moe_sel, *tok = m->moe_tok, *pos = m->moe_pos, *x_rows = m->moe_rows, *tiles = m->moe_tiles;
     int max_tiles = m->moe_max_tiles;
@@ -1379,7 +1384,7 @@ static int moe_prepare(b2_engine* e, LayeredModel* m, LyLayer& L, const RaggedDe
     DenseArgs up = {};
     up.groups = &j.g;
     up.p0 = (float)d.moe_limit; up.p1 = (float)d.moe_alpha;
-    if (big) {                                     // the activations only feed the down maps: left rounded
+    if (rounded) {                                 // the activations only feed the down maps: left rounded
         if (in == m->hn) up.x_rounded = m->hn_rounded;
         up.y_rounded = m->moe_hb;
     }
@@ -1389,7 +1394,7 @@ static int moe_prepare(b2_engine* e, LayeredModel* m, LyLayer& L, const RaggedDe
     j.g2.x_rows = nullptr; j.g2.row_scale = nullptr; j.g2.w_stride = (long)W * ff; j.g2.x_total_rows = pairs;
     DenseArgs dn = {};
     dn.groups = &j.g2;
-    if (big) dn.x_rounded = m->moe_hb;
+    if (rounded) dn.x_rounded = m->moe_hb;
     if (table) dn.scale = 1.f / (float)d.moe_top;
     j.down = dense_args(m, L.e_down, m->moe_h, ff, m->moe_y, W, pairs, nullptr, EPI_NONE, &dn);
     j.join.sel = sel; j.join.weight = out_weight; j.join.pos = tiled ? pos : nullptr; j.join.rows = m->moe_y; j.join.h = in;
@@ -1539,8 +1544,7 @@ static int run_layers(b2_engine* e, LayeredModel* m, const RaggedDev& r) {
             if (one_norm && m->hn_b && N.d.mixer == B2_MIX_SINK_ATTN && takes_rounded(m, N.sk_proj, T)) {
                 m->hn_rounded = p.y1_bf16 = m->hn_b;
                 const bool moe = N.d.n_ff > 0 && N.d.ff_kind == B2_FF_MOE;
-                const bool big = moe && T * N.d.moe_top >= MOE_BIG_PAIRS && N.gate_up.type == T_BF16 && W % 8 == 0 && N.d.n_ff % 8 == 0;
-                if (N.d.n_ff == 0 || (big && N.d.moe_route == B2_ROUTE_TABLE)) p.y1 = nullptr;
+                if (N.d.n_ff == 0 || (moe && moe_takes_rounded(m, N) && N.d.moe_route == B2_ROUTE_TABLE)) p.y1 = nullptr;
             }
         };
         ParallelJoinArgs pj = {};

@@ -53,8 +53,8 @@ struct DenseGroups {
     int n_groups = 0;
     long w_stride = 0;                 // elements between the matrices of two groups
     int max_tiles = 0;                 // grid size of a tiled launch
-    int tile_max = 64;                 // most rows of a tile: 64, or 128 (large tensor-core tiles; bf16 serving mode only)
-    int x_total_rows = 0;              // rows of the input matrix (128-row tiles: it is rounded to bf16 as a whole first)
+    int tile_max = 64;                 // most rows of a tile: 64, or 128 (tcgen05 kernel only)
+    int x_total_rows = 0;              // rows of the input matrix
 };
 struct DenseArgs {
     const float* x; int ldx;
@@ -64,14 +64,14 @@ struct DenseArgs {
     int T, N, K;
     int epi;
     bool exact;                     // true: 32-bit multiply-adds (no tensor cores, inputs not rounded)
-    __nv_bfloat16* xb;              // scratch [T][K] for X rounded to bf16 (large tensor-core steps); null: not available
+    __nv_bfloat16* xb;              // scratch for X rounded to bf16, [T][K] ([T][x_span] batched; pair rows when gathered); null: not available
     float scale = 1.f;              // the product (after the epilogue) times this
     int n_act = 0, n_act_end = 0;   // EPI_BIAS_PART_RELU2
     float p0 = 0.f, p1 = 0.f;       // constants of EPI_GLU_CLAMP / EPI_PIECEWISE
     const float* aux = nullptr; int ldaux = 0; bool aux_one = false;      // EPI_MUL_SIGMOID
     // batch > 1: `batch` independent products, operand b at x + b * x_bs, w + b * w_bs (elements), y + b * y_bs, aux + b * aux_bs
     int batch = 1; long x_bs = 0, w_bs = 0, y_bs = 0, aux_bs = 0;
-    // products of the large tensor-core kernel (dense_takes_rounded): the input rounded to bf16 [rows][K] if the producer has left it, and
+    // products of the tcgen05 kernel (dense_takes_rounded): the input rounded to bf16 [rows][K] if the producer has left it, and
     // the output rounded to bf16 [rows][ldy] instead of f32 for the next one
     const __nv_bfloat16* x_rounded = nullptr;
     __nv_bfloat16* y_rounded = nullptr;
