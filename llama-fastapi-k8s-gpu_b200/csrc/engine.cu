@@ -798,7 +798,7 @@ __global__ void set_ints_kernel(int* ints, int tok, int pos) { if (tok >= 0) int
 
 // enqueue: sample from the slot's logit buffer (the token at position n_past - 1 was the last one evaluated); the token
 // lands in e->pinned[pinned_index] once the stream has been synchronised
-int b2_sample_enqueue(b2_engine* e, Slot& s, int pinned_index) {
+static int sample_enqueue(b2_engine* e, Slot& s, int pinned_index) {
     // sampler bumps pos: make it point at the last evaluated token first
     set_ints_kernel<<<1, 1, 0, e->stream>>>(s.ints, -1, s.n_past - 1);
     CK(sample_launch(s.logits, e->cfg.n_vocab, s.sp, s.sst, s.uniforms, s.ints + 3, s.ints + 2, s.ints + 0,
@@ -814,7 +814,7 @@ extern "C" int b2_sample(b2_engine* e, int slot, int32_t* out) {
     std::lock_guard<std::mutex> lk(e->mu);
     Slot& s = e->slots[slot];
     CK(cudaSetDevice(e->cfg.device));
-    if ((rc = b2_sample_enqueue(e, s, 0))) return rc;
+    if ((rc = sample_enqueue(e, s, 0))) return rc;
     CK(cudaStreamSynchronize(e->stream));
     if (out) *out = e->pinned[0];
     return B2_OK;

@@ -249,5 +249,10 @@ cudaError_t sample_launch(float* logits, int n_vocab, const SampleParams* params
 // logits row z (row_stride floats apart) belongs to slot b.slot[z]; also writes the token to out_tokens[z]
 cudaError_t sample_batch_launch(float* logits, long row_stride, int n_vocab, const SlotDev* tab, const BatchIdx& b,
                                 int ring_len, int* out_tokens, cudaStream_t s);
+// ragged steps: which rows of the step's logits belong to which entries (by value)
+struct SampleRows { int n; int entry[BATCH_MAX]; int row[BATCH_MAX]; };
+// rows [n_vocab] of `logits` are copied to slot_logits[slot] and sampled there; the token of entry e goes to out_tokens[e]
+cudaError_t sample_rows_launch(const float* logits, int n_vocab, const SlotDev* tab, float* const* slot_logits, const SampleRows& rows, const int* seg_slot,
+                               const int* seg_pos0, const int* seg_len, int ring_len, int* out_tokens, cudaStream_t s);
 
 }  // namespace b2

@@ -97,6 +97,9 @@ struct LayeredModel {
     float *final_norm = nullptr, *final_norm_b = nullptr, *embed_norm = nullptr;
     bool exact = false;                // B2_FLAG_F32
     int** block_tables = nullptr;      // device [max_seqs] -> page table
+    SlotDev* slot_tab = nullptr;       // device [max_seqs]: what the sampler needs of a slot
+    float** slot_logits = nullptr;     // device [max_seqs] -> the slot's logit buffer
+    int* sampled = nullptr;            // device [B2_STEP_MAX_ENTRIES]: tokens sampled in a step, by entry
     // step workspace (max_step_tokens rows)
     float *xs = nullptr, *hc = nullptr, *cross = nullptr;     // copies of the stream [S][max_step_tokens][W]; convolved sublayer input; per-(query head, value head) attention sums
     float *x = nullptr, *proj = nullptr, *buf[4] = {}, *oL = nullptr, *oR = nullptr, *hn = nullptr, *hn2 = nullptr, *ff = nullptr, *rows = nullptr, *logits = nullptr;
@@ -738,6 +741,17 @@ int layered_finalize(b2_engine* e) {
         for (int i = 0; i < S; i++) tabs[i] = e->slots[i].block_table;
         if ((rc = dev_alloc(m, (void**)&m->block_tables, sizeof(int*) * S))) return rc;
         CK(cudaMemcpy(m->block_tables, tabs.data(), sizeof(int*) * S, cudaMemcpyHostToDevice));
+        std::vector<SlotDev> dev(S);
+        std::vector<float*> lg(S);
+        for (int i = 0; i < S; i++) {
+            const Slot& sl = e->slots[i];
+            dev[i] = SlotDev{sl.ints, sl.block_table, sl.ring, sl.sst, sl.sp, sl.uniforms};
+            lg[i] = sl.logits;
+        }
+        if ((rc = dev_alloc(m, (void**)&m->slot_tab, sizeof(SlotDev) * S)) || (rc = dev_alloc(m, (void**)&m->slot_logits, sizeof(float*) * S)) ||
+            (rc = dev_alloc(m, (void**)&m->sampled, sizeof(int) * B2_STEP_MAX_ENTRIES))) return rc;
+        CK(cudaMemcpy(m->slot_tab, dev.data(), sizeof(SlotDev) * S, cudaMemcpyHostToDevice));
+        CK(cudaMemcpy(m->slot_logits, lg.data(), sizeof(float*) * S, cudaMemcpyHostToDevice));
     }
     CK(cudaStreamSynchronize(e->stream));
     e->finalized = true;
@@ -1666,8 +1680,6 @@ struct StepChainPdl {
     ~StepChainPdl() { g_chain_pdl = prev; }
 };
 
-int b2_sample_enqueue(b2_engine* e, Slot& s, int pinned_index);
-
 extern "C" int b2_step(b2_engine* e, int n_entries, const int32_t* slots, const int32_t* n_tokens, const int32_t* tokens,
                        const int32_t* want_rows, int n_want, float* host_logits, const int32_t* sample, int32_t* host_sampled) {
     if (!e || !e->layered) return b2_fail(B2_ERR_UNSUPPORTED, "b2_step needs an engine made by b2_engine_create_layered");
@@ -1727,7 +1739,7 @@ extern "C" int b2_step(b2_engine* e, int n_entries, const int32_t* slots, const 
     }
     const int W = c.n_embd, V = c.n_vocab;
     int rc;
-    // logits of rows [r0, r0 + nr): final norm, head, wanted rows to the pinned buffer, sampled rows to their slots
+    // logits of rows [r0, r0 + nr): final norm, head, wanted rows to the pinned buffer, sampled rows to their slots and sampled there
     auto head_chunk = [&](int r0, int nr) -> int {
         {
             StepProfiler sp(m, st, 5);
@@ -1744,9 +1756,14 @@ extern "C" int b2_step(b2_engine* e, int n_entries, const int32_t* slots, const 
         if (rc2) return rc2;
         const int n_w = std::max(0, std::min(n_want - r0, nr));
         if (n_w > 0) CK(cudaMemcpyAsync(m->logits_host, m->logits, (size_t)n_w * V * 4, cudaMemcpyDeviceToHost, st));
+        SampleRows sr = {};
         for (int i = 0; i < n; i++)
-            if (samp_row[i] >= r0 && samp_row[i] < r0 + nr)
-                CK(cudaMemcpyAsync(e->slots[slots[i]].logits, m->logits + (size_t)(samp_row[i] - r0) * V, (size_t)V * 4, cudaMemcpyDeviceToDevice, st));
+            if (samp_row[i] >= r0 && samp_row[i] < r0 + nr) { sr.entry[sr.n] = i; sr.row[sr.n++] = samp_row[i] - r0; }
+        if (sr.n > 0) {
+            CK(sample_rows_launch(m->logits, V, m->slot_tab, m->slot_logits, sr, r.seg_slot, r.seg_pos0, r.seg_len, c.n_ctx + 1, m->sampled, st));
+            CK(cudaMemcpyAsync(e->pinned, m->sampled, sizeof(int) * n, cudaMemcpyDeviceToHost, st));
+            e->launches++;
+        }
         return B2_OK;
     };
     // everything the step enqueues up to the logits, for steps whose rows fit one head chunk
@@ -1824,13 +1841,12 @@ extern "C" int b2_step(b2_engine* e, int n_entries, const int32_t* slots, const 
         e->slots[slots[i]].n_past += n_tokens[i];
         e->slots[slots[i]].last_token = h_id[h_start[i] + h_len[i] - 1];
     }
-    for (int i = 0; i < n; i++) {
-        if (host_sampled) host_sampled[i] = -1;
-        if (samp_row[i] >= 0) { if ((rc = b2_sample_enqueue(e, e->slots[slots[i]], i))) return rc; }
-    }
     CK(cudaStreamSynchronize(st));
     if ((rc = b2_check_kernel_error())) return rc;
-    if (host_sampled) for (int i = 0; i < n; i++) if (samp_row[i] >= 0) host_sampled[i] = e->pinned[i];
+    for (int i = 0; i < n; i++) {
+        if (host_sampled) host_sampled[i] = samp_row[i] >= 0 ? e->pinned[i] : -1;
+        if (samp_row[i] >= 0) e->slots[slots[i]].n_sampled += 1;
+    }
     if (m->profile) {
         for (int k = 0; k < 8; k++) { m->prof_ms[k] = 0.f; m->prof_n[k] = 0; }
         for (auto& pe : m->prof_ev) {

@@ -246,6 +246,36 @@ __global__ void __launch_bounds__(SM_THREADS) sample_batch_kernel(float* logits,
                 sd.ints + 1, sd.ring, ring_len, out_tokens + z);
 }
 
+// Ragged steps: entry e's logits (row e.row of the step's output) move into its slot's own buffer and are sampled there. One launch
+// for all sequences of a step; it stands in for a copy, a position update, a sampler launch and a read-back per sequence (32
+// sequences: 370 us of a 1.1 ms step).
+__global__ void __launch_bounds__(SM_THREADS) sample_rows_kernel(const float* __restrict__ logits, int V, const SlotDev* tab, float* const* slot_logits,
+                                                                 const SampleRows rows, const int* seg_slot, const int* seg_pos0, const int* seg_len,
+                                                                 int n_uniform, int ring_len, int* out_tokens) {
+    griddep_launch();
+    griddep_wait();
+    const int entry = rows.entry[blockIdx.x], slot = seg_slot[entry];
+    const SlotDev sd = tab[slot];
+    const float* src = logits + (size_t)rows.row[blockIdx.x] * V;
+    float* dst = slot_logits[slot];
+    if (V % 4 == 0) {
+#pragma unroll 4
+        for (int i = threadIdx.x; i < V / 4; i += SM_THREADS) reinterpret_cast<float4*>(dst)[i] = reinterpret_cast<const float4*>(src)[i];
+    } else {
+#pragma unroll 4
+        for (int i = threadIdx.x; i < V; i += SM_THREADS) dst[i] = src[i];
+    }
+    if (threadIdx.x == 0) sd.ints[1] = seg_pos0[entry] + seg_len[entry] - 1;      // the token that was evaluated last
+    __syncthreads();
+    sample_body(dst, V, sd.sp, sd.sst, sd.uniforms, n_uniform, sd.ints + 3, sd.ints + 2, sd.ints + 0, sd.ints + 1, sd.ring, ring_len, out_tokens + entry);
+}
+
+cudaError_t sample_rows_launch(const float* logits, int n_vocab, const SlotDev* tab, float* const* slot_logits, const SampleRows& rows, const int* seg_slot,
+                               const int* seg_pos0, const int* seg_len, int ring_len, int* out_tokens, cudaStream_t s) {
+    return launch_chain(sample_rows_kernel, dim3(rows.n), dim3(SM_THREADS), 0, s, logits, n_vocab, tab, slot_logits, rows, seg_slot, seg_pos0, seg_len, 8192,
+                        ring_len, out_tokens);
+}
+
 cudaError_t sample_batch_launch(float* logits, long row_stride, int n_vocab, const SlotDev* tab, const BatchIdx& b,
                                 int ring_len, int* out_tokens, cudaStream_t s) {
     return launch_chain(sample_batch_kernel, dim3(b.n), dim3(SM_THREADS), 0, s, logits, row_stride, n_vocab, tab, b, 8192, ring_len, out_tokens);
