@@ -147,48 +147,103 @@ static cudaError_t launch_rows(const DenseDev& d, int batch, cudaStream_t s) {
     return launch_chain(dense_rows_kernel<TW, 8, 4>, dim3((N + 31) / 32, gy, gz), block, 0, s, d);
 }
 
-// ---------------------------------------------------------------- exact: 64 x 64 tile, 16-deep, 4 x 4 per thread
+// ---------------------------------------------------------------- exact: 64 x 64 tile, 32-deep, 4 x 4 per thread
+// Bound by the multiply-adds once the loads are out of the way: the next slice of both operands is in registers while the current one
+// is used (16-byte loads along K where rows allow), both live in shared memory as rows padded by 16 bytes, and four K steps cost
+// eight 16-byte shared loads for 64 multiply-adds. A thread's rows and columns are 16 apart: neighbouring lanes read neighbouring
+// rows, on different banks. The order of every sum is that of k.
 template <typename TW>
 __global__ void __launch_bounds__(256) dense_fma_kernel(DenseDev a) {
     griddep_launch();
     griddep_wait();
-    constexpr int BM = 64, BN = 64, BK = 16;
-    __shared__ float xs[BK][BM + 4];
-    __shared__ float ws[BK][BN + 4];
+    constexpr int BM = 64, BN = 64, BK = 32, LD = BK + 4;
+    __shared__ __align__(16) float xs[2][BM][LD];
+    __shared__ __align__(16) float ws[2][BN][LD];
     const float* x; const TW* w; float* y; const float* aux; int t0, T;
     if (!dense_tile<TW>(a, BM, x, w, y, aux, t0, T, blockIdx.y, blockIdx.z)) return;
     const int N = a.N, K = a.K, ldx = a.ldx;
     const int n0 = blockIdx.x * BN;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;      // thread tile: rows ty*4.., cols tx*4..
-    const float* rs = a.g.row_scale;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += BK) {
-        for (int i = threadIdx.x; i < BM * BK; i += 256) {
-            const int r = i / BK, kk = i % BK;
-            const int t = t0 + r, k = k0 + kk;
-            xs[kk][r] = (t < T && k < K) ? x[(size_t)x_row(a, t) * ldx + k] : 0.f;
-            const int n = n0 + r;
-            ws[kk][r] = (n < N && k < K) ? ld_w(w, (size_t)n * K + k) : 0.f;
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;      // rows ty + 16 i, columns tx + 16 j
+    // a thread fetches 8 consecutive K entries of one row of each operand
+    const int fr = threadIdx.x >> 2, fk = (threadIdx.x & 3) * 8;
+    const int xt = t0 + fr, wn = n0 + fr;
+    const bool x_in = xt < T, w_in = wn < N;
+    const float* xr = x + (size_t)(x_in ? x_row(a, xt) : 0) * ldx;
+    const TW* wr = w + (size_t)(w_in ? wn : 0) * K;
+    const bool vec = K % 8 == 0 && ldx % 4 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
+    float xv[8], wv[8];
+    auto fetch = [&](int k0) {
+        const int k = k0 + fk;
+        if (vec) {
+            const bool in = k < K;
+            float4 p = make_float4(0.f, 0.f, 0.f, 0.f), q = p;
+            if (x_in && in) { p = *reinterpret_cast<const float4*>(xr + k); q = *reinterpret_cast<const float4*>(xr + k + 4); }
+            xv[0] = p.x; xv[1] = p.y; xv[2] = p.z; xv[3] = p.w; xv[4] = q.x; xv[5] = q.y; xv[6] = q.z; xv[7] = q.w;
+            if constexpr (sizeof(TW) == 2) {
+                uint4 u = make_uint4(0u, 0u, 0u, 0u);
+                if (w_in && in) u = *reinterpret_cast<const uint4*>(wr + k);
+                const uint32_t h[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+                for (int i = 0; i < 4; i++) { wv[2 * i] = __uint_as_float(h[i] << 16); wv[2 * i + 1] = __uint_as_float(h[i] & 0xffff0000u); }
+            } else {
+                p = make_float4(0.f, 0.f, 0.f, 0.f); q = p;
+                if (w_in && in) { p = *reinterpret_cast<const float4*>(wr + k); q = *reinterpret_cast<const float4*>(wr + k + 4); }
+                wv[0] = p.x; wv[1] = p.y; wv[2] = p.z; wv[3] = p.w; wv[4] = q.x; wv[5] = q.y; wv[6] = q.z; wv[7] = q.w;
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                xv[i] = x_in && k + i < K ? xr[k + i] : 0.f;
+                wv[i] = w_in && k + i < K ? ld_w(wr, k + i) : 0.f;
+            }
         }
-        __syncthreads();
+    };
+    auto put = [&](int buf) {
+        *reinterpret_cast<float4*>(&xs[buf][fr][fk]) = make_float4(xv[0], xv[1], xv[2], xv[3]);
+        *reinterpret_cast<float4*>(&xs[buf][fr][fk + 4]) = make_float4(xv[4], xv[5], xv[6], xv[7]);
+        *reinterpret_cast<float4*>(&ws[buf][fr][fk]) = make_float4(wv[0], wv[1], wv[2], wv[3]);
+        *reinterpret_cast<float4*>(&ws[buf][fr][fk + 4]) = make_float4(wv[4], wv[5], wv[6], wv[7]);
+    };
+    float acc[4][4] = {};
+    fetch(0);
+    put(0);
+    __syncthreads();
+    int buf = 0;
+    for (int k0 = 0; k0 < K; k0 += BK, buf ^= 1) {
+        const bool more = k0 + BK < K;
+        if (more) fetch(k0 + BK);
 #pragma unroll
-        for (int kk = 0; kk < BK; kk++) {
-            float a[4], b[4];
+        for (int kk = 0; kk < BK; kk += 4) {
+            float4 p[4], q[4];
 #pragma unroll
-            for (int i = 0; i < 4; i++) { a[i] = xs[kk][ty * 4 + i]; b[i] = ws[kk][tx * 4 + i]; }
+            for (int i = 0; i < 4; i++) { p[i] = *reinterpret_cast<const float4*>(&xs[buf][ty + 16 * i][kk]); q[i] = *reinterpret_cast<const float4*>(&ws[buf][tx + 16 * i][kk]); }
 #pragma unroll
             for (int i = 0; i < 4; i++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                for (int j = 0; j < 4; j++) {
+                    acc[i][j] = fmaf(p[i].x, q[j].x, acc[i][j]);
+                    acc[i][j] = fmaf(p[i].y, q[j].y, acc[i][j]);
+                    acc[i][j] = fmaf(p[i].z, q[j].z, acc[i][j]);
+                    acc[i][j] = fmaf(p[i].w, q[j].w, acc[i][j]);
+                }
         }
+        if (more) put(buf ^ 1);
         __syncthreads();
     }
+    const float* rs = a.g.row_scale;
+    const bool glu = a.epi == EPI_GLU_SILU || a.epi == EPI_GLU_GELU || a.epi == EPI_GLU_CLAMP;
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        const int t = t0 + ty * 4 + i;
-        if (t >= T) continue;
+        const int t = t0 + ty + 16 * i;
 #pragma unroll
-        for (int j = 0; j < 4; j += 2) epi_store2(a, y, aux, rs, t, n0 + tx * 4 + j, acc[i][j], acc[i][j + 1]);
+        for (int j = 0; j < 4; j++) {
+            const int n = n0 + tx + 16 * j;
+            const float other = __shfl_xor_sync(0xffffffffu, acc[i][j], 1);      // the neighbouring column
+            if (t < T) {
+                if (!glu) { if (n < N) epi_store(a, y, aux, t, n, acc[i][j]); }
+                else if (!(tx & 1)) epi_store2(a, y, aux, rs, t, n, acc[i][j], other);
+            }
+        }
     }
 }
 
