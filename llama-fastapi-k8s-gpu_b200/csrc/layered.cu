@@ -1053,7 +1053,7 @@ static int mix_window_scan(b2_engine* e, LayeredModel* m, LyLayer& L, const Ragg
     {
         StepProfiler sp(m, st, 3);
         CK(scan_recurrence_launch(s, r, st));
-        e->launches += d.d_state <= 32 ? 2 : 1;      // states up to a warp wide: a preparation pass goes first
+        e->launches++;
     }
     return dense(e, m, L.scan_o, m->buf[1], d.d_inner, m->oR, W, T);
 }

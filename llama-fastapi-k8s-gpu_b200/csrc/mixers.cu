@@ -789,95 +789,119 @@ __global__ void __launch_bounds__(SCAN_CH) scan_recurrence_chan_kernel(ScanArgs 
     }
 }
 
-// States up to a warp wide (N <= LPC <= 32): LPC lanes per channel, one state each, so a step keeps 16-32 times more warps in
-// flight than a thread per channel; the read-out is a shuffle reduction over the LPC lanes. Step sizes and output gates are
-// made beforehand, in place, by scan_prepare_kernel (softplus(dt + bias) over dt_raw, silu over the z columns); inputs are
-// fetched four tokens ahead.
-__global__ void scan_prepare_kernel(ScanArgs a, int T) {
+// States up to a warp wide (N <= 32): four lanes per channel, N / 4 states each (lane q: states q, q + 4, ...), so that what a token
+// costs beside its states -- inputs, loop, read-out -- is paid once per four lanes, not once per state. A CTA owns SC_CH channels;
+// blocks of SC_TB tokens (step size, convolved input and gate of its channels, the B and C rows, ordered so that a lane's states are
+// one 16-byte read) arrive in shared memory as asynchronous copies two blocks ahead, where softplus(dt + bias) and silu(z) are
+// applied once per entry. Every global access is a run of SC_CH channels. The sums over the states keep the order of a butterfly over N
+// lanes, whatever the number of states a lane has.
+constexpr int SC_CH = 64, SC_TB = 16;
+template <int SPL>
+__global__ void __launch_bounds__(SC_CH * 4) scan_recurrence_lanes_kernel(ScanArgs a, RaggedDev r) {
     griddep_launch();
     griddep_wait();
-    const long n = (long)T * a.inner;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        const long t = i / a.inner;
-        const int c = (int)(i % a.inner);
-        float* dtp = const_cast<float*>(a.dt_raw) + i;
-        *dtp = softplus_f(*dtp + a.dt_bias[c]);
-        float* zp = const_cast<float*>(a.proj) + t * a.ldp + a.z_off + c;
-        *zp = silu_f(*zp);
-    }
-}
-
-template <int LPC>
-__global__ void __launch_bounds__(256) scan_recurrence_lanes_kernel(ScanArgs a, RaggedDev r) {
-    griddep_launch();
-    griddep_wait();
-    constexpr int CPB = 256 / LPC, AHEAD = 4;
-    const int seg = blockIdx.x, n = threadIdx.x % LPC, c = blockIdx.y * CPB + threadIdx.x / LPC;
+    constexpr int NP = 4 * SPL, STEP = SC_CH * 4;
+    __shared__ __align__(16) float in[3][3][SC_TB][SC_CH];          // [buffer][dt, x, gate][token][channel]
+    __shared__ __align__(16) float bc[3][2][SC_TB][NP];             // [buffer][B, C][token][lane][state of the lane]
+    const int seg = blockIdx.x, q = threadIdx.x & 3, lc = threadIdx.x >> 2, c0 = blockIdx.y * SC_CH, c = c0 + lc;
     const int N = a.N;
-    const bool c_ok = c < a.inner, ok = c_ok && n < N;
-    const int cc = c_ok ? c : a.inner - 1, nn = n < N ? n : 0;
+    const bool c_ok = c < a.inner;
+    const int cc = c_ok ? c : a.inner - 1;
     const int slot = r.seg_slot[seg], start = r.seg_start[seg], len = r.seg_len[seg];
     const int hist = a.taps - 1;
-    if (c_ok && n == 0) {
+    if (c_ok && q == 0) {
         float* st = a.conv_state + ((size_t)slot * a.inner + c) * hist;
         for (int k = 0; k < hist; k++) {
             const int srci = len + k - hist;
             st[k] = srci >= 0 ? a.proj[(size_t)(start + srci) * a.ldp + a.x_off + c] : st[k + len];
         }
     }
-    float* sst = a.ssm_state + ((size_t)slot * a.inner + cc) * N + nn;
-    const float A = -expf(a.A_log[(size_t)cc * N + nn]);
-    float S = ok ? *sst : 0.f;
+    float* sst = a.ssm_state + ((size_t)slot * a.inner + cc) * N;
+    float A[SPL], S[SPL];
+#pragma unroll
+    for (int j = 0; j < SPL; j++) {
+        const int n = q + 4 * j;
+        A[j] = n < N ? -expf(a.A_log[(size_t)cc * N + n]) : 0.f;
+        S[j] = n < N && c_ok ? sst[n] : 0.f;
+    }
     const float Dc = a.D[cc];
-    struct In { float dt, x, B, C, gate; };
-    auto fetch = [&](int i) {
-        In v;
-        const int t = start + min(i, len - 1);
-        v.dt = a.dt_raw[(size_t)t * a.inner + cc];
-        v.x = a.xc[(size_t)t * a.inner + cc];
-        v.B = ok ? a.xproj[(size_t)t * a.ldx + a.R + nn] : 0.f;
-        v.C = ok ? a.xproj[(size_t)t * a.ldx + a.R + N + nn] : 0.f;
-        v.gate = a.proj[(size_t)t * a.ldp + a.z_off + cc];
-        return v;
-    };
-    In cur[AHEAD], nxt[AHEAD];
-#pragma unroll
-    for (int u = 0; u < AHEAD; u++) cur[u] = fetch(u);
-    for (int i0 = 0; i0 < len; i0 += AHEAD) {
-        if (i0 + AHEAD < len) {
-#pragma unroll
-            for (int u = 0; u < AHEAD; u++) nxt[u] = fetch(i0 + AHEAD + u);
+    const int fch = threadIdx.x % SC_CH, fcc = min(c0 + fch, a.inner - 1);      // the channel this thread fetches for
+    const float dtb = a.dt_bias[fcc];
+    for (int j = threadIdx.x; j < 3 * 2 * SC_TB * NP; j += STEP) (&bc[0][0][0][0])[j] = 0.f;      // states past N stay zero
+    __syncthreads();
+    auto stage = [&](int i0, int buf) {
+        const int nb = min(SC_TB, len - i0);
+        for (int u = threadIdx.x / SC_CH; u < nb; u += STEP / SC_CH) {
+            const size_t t = start + i0 + u;
+            cp_async_4(&in[buf][0][u][fch], a.dt_raw + t * a.inner + fcc);
+            cp_async_4(&in[buf][1][u][fch], a.xc + t * a.inner + fcc);
+            cp_async_4(&in[buf][2][u][fch], a.proj + t * a.ldp + a.z_off + fcc);
         }
+        for (int j = threadIdx.x; j < nb * 2 * N; j += STEP) {
+            const int u = j / (2 * N), e = j % (2 * N), n = e < N ? e : e - N;
+            cp_async_4(&bc[buf][e < N ? 0 : 1][u][(n & 3) * SPL + (n >> 2)], a.xproj + (size_t)(start + i0 + u) * a.ldx + a.R + e);
+        }
+    };
+    stage(0, 0);
+    cp_async_commit();
+    if (SC_TB < len) stage(SC_TB, 1);
+    cp_async_commit();
+    int buf = 0;
+    for (int i0 = 0; i0 < len; i0 += SC_TB) {
+        const int nb = min(SC_TB, len - i0);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        // what this thread fetched of the block, made ready in place; then everybody's is visible
+        for (int u = threadIdx.x / SC_CH; u < nb; u += STEP / SC_CH) {
+            in[buf][0][u][fch] = softplus_f(in[buf][0][u][fch] + dtb);
+            in[buf][2][u][fch] = silu_f(in[buf][2][u][fch]);
+        }
+        __syncthreads();
+        const int nxt = buf == 0 ? 2 : buf - 1;
+        if (i0 + 2 * SC_TB < len) stage(i0 + 2 * SC_TB, nxt);        // everybody has left that buffer
+        cp_async_commit();
+        float keep = 0.f;
+#pragma unroll 4
+        for (int u = 0; u < nb; u++) {
+            const float dt = in[buf][0][u][lc], xv = in[buf][1][u][lc], gate = in[buf][2][u][lc];
+            const float* Bp = &bc[buf][0][u][q * SPL];
+            const float* Cp = &bc[buf][1][u][q * SPL];
+            float p[SPL];
 #pragma unroll
-        for (int u = 0; u < AHEAD; u++) {
-            if (i0 + u < len) {
-                const In v = cur[u];
-                S = expf(v.dt * A) * S + v.dt * v.x * v.B;
-                float part = S * v.C;
+            for (int j = 0; j < SPL; j++) {
+                S[j] = expf(dt * A[j]) * S[j] + dt * xv * Bp[j];
+                p[j] = __fmul_rn(S[j], Cp[j]);
+            }
 #pragma unroll
-                for (int o = LPC / 2; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-                if (n == 0 && c_ok) a.y[(size_t)(start + i0 + u) * a.inner + c] = (part + Dc * v.x) * v.gate;
+            for (int w = SPL / 2; w > 0; w >>= 1)
+#pragma unroll
+                for (int j = 0; j < w; j++) p[j] += p[j + w];
+            float sum = p[0];
+            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+            const float yv = (sum + Dc * xv) * gate;
+            if ((u & 3) == q) keep = yv;                             // lane q stores every fourth token
+            if ((u & 3) == 3 || u == nb - 1) {
+                const int mine = (u & ~3) + q;
+                if (c_ok && mine < nb) a.y[(size_t)(start + i0 + mine) * a.inner + c] = keep;
             }
         }
-#pragma unroll
-        for (int u = 0; u < AHEAD; u++) cur[u] = nxt[u];
+        buf = buf == 2 ? 0 : buf + 1;
     }
-    if (ok) *sst = S;
+    if (c_ok) {
+#pragma unroll
+        for (int j = 0; j < SPL; j++) { const int n = q + 4 * j; if (n < N) sst[n] = S[j]; }
+    }
 }
 
 cudaError_t scan_recurrence_launch(const ScanArgs& a, const RaggedDev& r, cudaStream_t s) {
     if (a.N > SCAN_MAXS * 32) return cudaErrorInvalidValue;
     PlainLaunch pl;        // latency-bound over the prompt: CTAs spread over all SMs (see kernels.h)
     if (a.N <= 32) {
-        const long n = (long)r.T * a.inner;
-        cudaError_t ce = launch_chain(scan_prepare_kernel, dim3((unsigned)std::min<long>((n + 255) / 256, 148 * 8)), dim3(256), 0, s, a, r.T);
-        if (ce != cudaSuccess) return ce;
-        const int lpc = a.N <= 4 ? 4 : a.N <= 8 ? 8 : a.N <= 16 ? 16 : 32;
-        const dim3 grid(r.n_seg, (a.inner + 256 / lpc - 1) / (256 / lpc));
-        if (lpc == 4) return launch_chain(scan_recurrence_lanes_kernel<4>, grid, dim3(256), 0, s, a, r);
-        if (lpc == 8) return launch_chain(scan_recurrence_lanes_kernel<8>, grid, dim3(256), 0, s, a, r);
-        if (lpc == 16) return launch_chain(scan_recurrence_lanes_kernel<16>, grid, dim3(256), 0, s, a, r);
-        return launch_chain(scan_recurrence_lanes_kernel<32>, grid, dim3(256), 0, s, a, r);
+        const dim3 grid(r.n_seg, (a.inner + SC_CH - 1) / SC_CH), block(SC_CH * 4);
+        if (a.N <= 4) return launch_chain(scan_recurrence_lanes_kernel<1>, grid, block, 0, s, a, r);
+        if (a.N <= 8) return launch_chain(scan_recurrence_lanes_kernel<2>, grid, block, 0, s, a, r);
+        if (a.N <= 16) return launch_chain(scan_recurrence_lanes_kernel<4>, grid, block, 0, s, a, r);
+        return launch_chain(scan_recurrence_lanes_kernel<8>, grid, block, 0, s, a, r);
     }
     if (a.N <= 64) {
         const dim3 grid(r.n_seg, (a.inner + SCAN_CH - 1) / SCAN_CH), block(SCAN_CH);
