@@ -625,7 +625,7 @@ int layered_finalize(b2_engine* e) {
             if ((rc = dev_alloc(m, (void**)&L.nvec, (size_t)S * d.mm_heads * d.mm_dim * 4, true))) return rc;
             if ((rc = dev_alloc(m, (void**)&L.mmax, (size_t)S * d.mm_heads * 4, true))) return rc;
             max_proj = std::max<size_t>(max_proj, L.mm_proj.N);
-            max_buf = std::max<size_t>(max_buf, (size_t)vd);
+            max_buf = std::max<size_t>({max_buf, (size_t)vd, (size_t)2 * d.mm_heads});
         }
         if (d.n_ff > 0 && d.ff_kind == B2_FF_MOE) {
             const int slots = d.moe_experts + d.moe_identity;
@@ -1069,6 +1069,7 @@ static int mix_matrix_memory(b2_engine* e, LayeredModel* m, LyLayer& L, const Ra
     a.proj = m->proj; a.ldp = Np; a.q_off = L.mq; a.k_off = L.mk; a.v_off = L.mv; a.g_off = L.mg; a.i_off = L.mi; a.f_off = L.mf;
     a.i_bias = L.i_b; a.f_bias = L.f_b; a.norm_w = L.mm_norm; a.H = d.mm_heads; a.d = d.mm_dim; a.dv = d.mm_vdim;
     a.cap = (float)d.gate_cap; a.eps = c.norm_eps; a.S = L.S; a.n = L.nvec; a.m = L.mmax; a.o_raw = m->buf[0]; a.out = m->buf[1];
+    a.nq = m->buf[2]; a.m_scale = m->buf[2] + (size_t)T * d.mm_heads;
     {
         StepProfiler sp(m, e->stream, 4);
         CK(matrix_mem_launch(a, r, e->stream));

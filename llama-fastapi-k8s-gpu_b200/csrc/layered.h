@@ -160,7 +160,8 @@ struct MatrixMemArgs {         // mLSTM
     int H, d, dv;
     float cap, eps;
     float* S; float* n; float* m;      // per slot: [H][d][dv], [H][d], [H]
-    float* o_raw;              // [T][H*dv] scratch: memory read-out before the head norm
+    float* o_raw;              // [T][H*dv] scratch: memory read-out before the normaliser and the head norm
+    float *nq, *m_scale;       // [T][H] scratch: n . q and exp(-m) of every token
     float* out;                // [T][H*dv]
 };
 cudaError_t matrix_mem_launch(const MatrixMemArgs& a, const RaggedDev& r, cudaStream_t s);

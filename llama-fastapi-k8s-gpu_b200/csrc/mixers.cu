@@ -914,26 +914,55 @@ cudaError_t scan_recurrence_launch(const ScanArgs& a, const RaggedDev& r, cudaSt
 }
 
 // ---------------------------------------------------------------- matrix memory (mLSTM)
-// Gate activations for every (token, head), in place over the projection's i and f columns: i <- cap tanh((i + b_i) / cap),
-// f <- logsigmoid(cap tanh((f + b_f) / cap)). Parallel over the step, so the recurrence below only carries the maximum.
-__global__ void matrix_mem_gates_kernel(MatrixMemArgs a, int T) {
+// Everything of the recurrence that the memory itself does not enter, ahead of it: per (sequence, head) the log gates
+// i = cap tanh((i + b_i) / cap) and f = logsigmoid(cap tanh((f + b_f) / cap)), the running maximum m_t = max(f + m_(t-1), i) and the two
+// factors exp(f + m_(t-1) - m_t) and exp(i - m_t) that a token's update takes. The maximum is one thread's serial chain over a block
+// of tokens in shared memory (two dependent operations a token); the rest is one token per thread. Left in place: decay over the
+// projection's f column, write weight over its i column; exp(-m_t) in m_scale [T][H].
+constexpr int MG_TB = 256;
+__global__ void __launch_bounds__(MG_TB) matrix_mem_gates_kernel(MatrixMemArgs a, RaggedDev r) {
     griddep_launch();
     griddep_wait();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= T * a.H) return;
-    const int t = i / a.H, h = i % a.H;
-    float* p = const_cast<float*>(a.proj) + (size_t)t * a.ldp;
-    p[a.i_off + h] = a.cap * tanhf((p[a.i_off + h] + a.i_bias[h]) / a.cap);
-    p[a.f_off + h] = log_sigmoid_f(a.cap * tanhf((p[a.f_off + h] + a.f_bias[h]) / a.cap));
+    __shared__ float ig[MG_TB], fg[MG_TB], ms[MG_TB + 1];
+    const int seg = blockIdx.x, h = blockIdx.y;
+    const int slot = r.seg_slot[seg], start = r.seg_start[seg], len = r.seg_len[seg];
+    const float ib = a.i_bias[h], fb = a.f_bias[h];
+    if (threadIdx.x == 0) ms[0] = a.m[(size_t)slot * a.H + h];
+    for (int i0 = 0; i0 < len; i0 += MG_TB) {
+        const int nb = min(MG_TB, len - i0), u = threadIdx.x;
+        float* p = const_cast<float*>(a.proj) + (size_t)(start + i0 + min(u, nb - 1)) * a.ldp;
+        if (u < nb) {
+            ig[u] = a.cap * tanhf((p[a.i_off + h] + ib) / a.cap);
+            fg[u] = log_sigmoid_f(a.cap * tanhf((p[a.f_off + h] + fb) / a.cap));
+        }
+        __syncthreads();
+        if (u == 0) {
+            float m = ms[0];
+#pragma unroll 8
+            for (int k = 0; k < nb; k++) { m = fmaxf(fg[k] + m, ig[k]); ms[k + 1] = m; }
+        }
+        __syncthreads();
+        if (u < nb) {
+            const float m_new = ms[u + 1];
+            p[a.f_off + h] = expf(fg[u] + ms[u] - m_new);
+            p[a.i_off + h] = expf(ig[u] - m_new);
+            a.m_scale[(size_t)(start + i0 + u) * a.H + h] = expf(-m_new);
+        }
+        const float last = ms[nb];
+        __syncthreads();
+        if (u == 0) ms[0] = last;
+    }
+    if (threadIdx.x == 0) a.m[(size_t)slot * a.H + h] = ms[0];
 }
 
-// grid (n_seg, H, ceil(dv / 32)): a CTA owns 32 columns of one head's d x dv memory. Thread (col, grp) keeps rows grp * MM_ROWS ..
-// of its column in registers; a warp is one row group, and its lanes each carry one row of the normaliser n. Tokens go in blocks of MM_TB: a thread's state update for token t + 1 needs
-// only its own registers after token t, so the block barrier is paid once per block -- for the inputs (q, k, v and the two gate
-// values of the next block arrive in shared memory as asynchronous copies while this block is computed) and for the partial
-// read-outs per row group, which all threads then sum in a fixed order, one (token, column) each. The normaliser n and the
-// running maximum m are carried by every CTA of the head (same arithmetic, same values); the first one writes them back.
-constexpr int MM_ROWS = 16, MM_COLS = 32, MM_TB = 8;      // key size <= 16 * 16 = 256 (512 threads)
+// grid (n_seg, H, ceil(dv / 32) + 1): a CTA owns 32 columns of one head's d x dv memory. Thread (col, grp) keeps rows grp * MM_ROWS ..
+// of its column in registers. Tokens go in blocks of MM_TB: a thread's state update for token t + 1 needs only its own registers
+// after token t, so the block barrier is paid once per block -- for the inputs (q, k, v and the two factors of the next block arrive
+// in shared memory as asynchronous copies while this block is computed) and for the partial read-outs per row group, which all
+// threads then sum in a fixed order, one (token, column) each. The CTA past the last columns carries the normaliser n (a lane per
+// row) and leaves n . q; the division by it waits for matrix_mem_out_kernel.
+// Bound by issue slots: 48 operations on the memory and 8 shared loads per token and warp.
+constexpr int MM_ROWS = 16, MM_COLS = 32, MM_TB = 16;      // key size <= 16 * 16 = 256 (512 threads)
 __global__ void __launch_bounds__(512) matrix_mem_kernel(MatrixMemArgs a, RaggedDev r, int RG) {
     griddep_launch();
     griddep_wait();
@@ -942,27 +971,27 @@ __global__ void __launch_bounds__(512) matrix_mem_kernel(MatrixMemArgs a, Ragged
     float* qs = sm;                                // [2][MM_TB][d]
     float* ks = qs + 2 * MM_TB * d;                // [2][MM_TB][d]
     float* vs = ks + 2 * MM_TB * d;                // [2][MM_TB][MM_COLS]
-    float* gs = vs + 2 * MM_TB * MM_COLS;          // [2][MM_TB][2]: log input gate, log forget gate
-    float* ms = gs + 2 * MM_TB * 2;                // [2][MM_TB]: running maximum after each token
-    float* red = ms + 2 * MM_TB;                   // [2][MM_TB][RG][MM_COLS + 1]: partial read-outs, last column = partial n.q
-    const int red_tok = RG * (MM_COLS + 1);
-    const int seg = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * MM_COLS;
+    float* gs = vs + 2 * MM_TB * MM_COLS;          // [2][MM_TB][2]: write weight, decay
+    float* red = gs + 2 * MM_TB * 2;               // [2][MM_TB][RG][MM_COLS]: partial read-outs
+    const int red_tok = RG * MM_COLS;
+    const bool norm_cta = blockIdx.z == gridDim.z - 1;
+    const int seg = blockIdx.x, h = blockIdx.y, c0 = norm_cta ? 0 : blockIdx.z * MM_COLS, n_cols = norm_cta ? 0 : min(MM_COLS, dv - c0);
     const int slot = r.seg_slot[seg], start = r.seg_start[seg], len = r.seg_len[seg];
-    const int lc = threadIdx.x % MM_COLS, grp = threadIdx.x / MM_COLS, col = c0 + lc;
-    const bool col_ok = col < dv, act = grp < RG;       // threads past the last row group only help with copies and sums
-    float* Sg = a.S + (((size_t)slot * a.H + h) * d) * dv;
+    const int lc = threadIdx.x % MM_COLS, grp = threadIdx.x / MM_COLS;
+    const bool act = grp < RG;                     // threads past the last row group only help with copies and sums
+    const bool mem = act && lc < n_cols;
+    float* Sg = a.S + (((size_t)slot * a.H + h) * d) * dv + c0 + lc;
     float* ng = a.n + ((size_t)slot * a.H + h) * d;
     float S[MM_ROWS];
 #pragma unroll
     for (int i = 0; i < MM_ROWS; i++) {
         const int row = grp * MM_ROWS + i;
-        S[i] = (act && col_ok && row < d) ? Sg[(size_t)row * dv + col] : 0.f;
+        S[i] = (mem && row < d) ? Sg[(size_t)row * dv] : 0.f;
     }
     const int nrow = grp * MM_ROWS + lc;                      // lanes 0 .. MM_ROWS-1 of a warp: one row of n each
-    const bool n_ok = act && lc < MM_ROWS && nrow < d;
+    const bool n_ok = norm_cta && act && lc < MM_ROWS && nrow < d;
     float nr = n_ok ? ng[nrow] : 0.f;
     const bool vec4 = (d % 4) == 0;
-    float m = a.m[(size_t)slot * a.H + h];
     const float qscale = 1.f / sqrtf((float)d);
     auto stage = [&](int i0, int buf) {                  // tokens i0 .. of the segment into buffer `buf`
         const int nb = min(MM_TB, len - i0);
@@ -975,20 +1004,20 @@ __global__ void __launch_bounds__(512) matrix_mem_kernel(MatrixMemArgs a, Ragged
         for (int j = threadIdx.x; j < nb * MM_COLS; j += blockDim.x) {
             const int u = j / MM_COLS, e = j % MM_COLS;
             const float* p = a.proj + (size_t)(start + i0 + u) * a.ldp;
-            if (c0 + e < dv) cp_async_4(&vs[(buf * MM_TB + u) * MM_COLS + e], p + a.v_off + h * dv + c0 + e);
+            if (e < n_cols) cp_async_4(&vs[(buf * MM_TB + u) * MM_COLS + e], p + a.v_off + h * dv + c0 + e);
             if (e < 2) cp_async_4(&gs[(buf * MM_TB + u) * 2 + e], p + (e == 0 ? a.i_off : a.f_off) + h);
         }
     };
-    auto finish = [&](int i0, int buf) {                 // sum of the row groups in a fixed order, then the read-out
-        const int nb = min(MM_TB, len - i0);
-        for (int j = threadIdx.x; j < nb * MM_COLS; j += blockDim.x) {
-            const int u = j / MM_COLS, e = j % MM_COLS;
-            if (c0 + e >= dv) continue;
+    auto finish = [&](int i0, int buf) {                 // sum of the row groups in a fixed order
+        const int nb = min(MM_TB, len - i0), cols = norm_cta ? 1 : MM_COLS;
+        for (int j = threadIdx.x; j < nb * cols; j += blockDim.x) {
+            const int u = j / cols, e = j % cols;
+            if (!norm_cta && e >= n_cols) continue;
             const float* rd = red + (size_t)(buf * MM_TB + u) * red_tok;
-            float num = 0.f, nq = 0.f;
-            for (int g2 = 0; g2 < RG; g2++) { num += rd[g2 * (MM_COLS + 1) + e]; nq += rd[g2 * (MM_COLS + 1) + MM_COLS]; }
-            const float den = fmaxf(fabsf(nq), expf(-ms[buf * MM_TB + u])) + 1e-6f;
-            a.o_raw[(size_t)(start + i0 + u) * a.H * dv + (size_t)h * dv + c0 + e] = num / den;
+            float sum = 0.f;
+            for (int g2 = 0; g2 < RG; g2++) sum += rd[g2 * MM_COLS + e];
+            if (norm_cta) a.nq[(size_t)(start + i0 + u) * a.H + h] = sum;
+            else a.o_raw[(size_t)(start + i0 + u) * a.H * dv + (size_t)h * dv + c0 + e] = sum;
         }
     };
     for (int j = threadIdx.x; j < 2 * MM_TB * MM_COLS; j += blockDim.x) vs[j] = 0.f;
@@ -1002,19 +1031,27 @@ __global__ void __launch_bounds__(512) matrix_mem_kernel(MatrixMemArgs a, Ragged
         if (i0 + MM_TB < len) stage(i0 + MM_TB, buf ^ 1);
         cp_async_commit();
         if (i0 > 0) finish(i0 - MM_TB, buf ^ 1);
-        for (int u = 0; u < nb; u++) {
-            const int bu = buf * MM_TB + u;
-            const float ig = gs[bu * 2], fg = gs[bu * 2 + 1];
-            const float m_new = fmaxf(fg + m, ig);
-            const float da = expf(fg + m - m_new), ib = expf(ig - m_new);
-            m = m_new;
-            if (threadIdx.x == 0) ms[bu] = m;
-            const float vb = ib * vs[bu * MM_COLS + lc];
-            float part = 0.f;
-            if (act) {
+        if (norm_cta) {
+            for (int u = 0; u < nb; u++) {
+                const int bu = buf * MM_TB + u;
+                const float ib = gs[bu * 2], da = gs[bu * 2 + 1];
+                float npart = 0.f;
+                if (n_ok) { nr = fmaf(da, nr, ib * ks[bu * d + nrow]); npart = nr * qs[bu * d + nrow]; }
+#pragma unroll
+                for (int o = MM_ROWS / 2; o > 0; o >>= 1) npart += __shfl_xor_sync(0xffffffffu, npart, o);
+                if (act && lc == 0) red[(size_t)bu * red_tok + grp * MM_COLS] = npart * qscale;
+            }
+        } else if (act) {
+            const bool full = vec4 && grp * MM_ROWS + MM_ROWS <= d;
+#pragma unroll 2
+            for (int u = 0; u < nb; u++) {
+                const int bu = buf * MM_TB + u;
+                const float2 g2 = *reinterpret_cast<const float2*>(gs + bu * 2);
+                const float da = g2.y, vb = g2.x * vs[bu * MM_COLS + lc];
+                float part = 0.f;
                 const float* kr = ks + bu * d + grp * MM_ROWS;
                 const float* qr = qs + bu * d + grp * MM_ROWS;
-                if (vec4 && grp * MM_ROWS + MM_ROWS <= d) {
+                if (full) {
 #pragma unroll
                     for (int k4 = 0; k4 < MM_ROWS; k4 += 4) {
                         const float4 k4v = *reinterpret_cast<const float4*>(kr + k4), q4v = *reinterpret_cast<const float4*>(qr + k4);
@@ -1028,18 +1065,7 @@ __global__ void __launch_bounds__(512) matrix_mem_kernel(MatrixMemArgs a, Ragged
                     for (int k = 0; k < MM_ROWS; k++)
                         if (grp * MM_ROWS + k < d) { S[k] = fmaf(da, S[k], kr[k] * vb); part = fmaf(S[k], qr[k], part); }
                 }
-            }
-            part *= qscale;
-            // normaliser: lane l of the warp has row l of this group; n . q summed over the group's lanes
-            float npart = 0.f;
-            if (n_ok) { nr = fmaf(da, nr, ib * ks[bu * d + nrow]); npart = nr * qs[bu * d + nrow]; }
-#pragma unroll
-            for (int o = MM_ROWS / 2; o > 0; o >>= 1) npart += __shfl_xor_sync(0xffffffffu, npart, o);
-            npart *= qscale;
-            if (act) {
-                float* rd = red + (size_t)bu * red_tok;
-                rd[grp * (MM_COLS + 1) + lc] = part;
-                if (lc == 0) rd[grp * (MM_COLS + 1) + MM_COLS] = npart;
+                red[(size_t)bu * red_tok + grp * MM_COLS + lc] = part * qscale;
             }
         }
     }
@@ -1048,39 +1074,39 @@ __global__ void __launch_bounds__(512) matrix_mem_kernel(MatrixMemArgs a, Ragged
 #pragma unroll
     for (int i = 0; i < MM_ROWS; i++) {
         const int row = grp * MM_ROWS + i;
-        if (act && col_ok && row < d) Sg[(size_t)row * dv + col] = S[i];
+        if (mem && row < d) Sg[(size_t)row * dv] = S[i];
     }
-    if (n_ok && blockIdx.z == 0) ng[nrow] = nr;
-    if (threadIdx.x == 0 && blockIdx.z == 0) a.m[(size_t)slot * a.H + h] = m;
+    if (n_ok) ng[nrow] = nr;
 }
 
-// per (token, head): out = o / rms(o) * norm_w * sigmoid(gate)
+// per (token, head): o = read-out / normaliser; out = o / rms(o) * norm_w * sigmoid(gate)
 __global__ void __launch_bounds__(128) matrix_mem_out_kernel(MatrixMemArgs a) {
     griddep_launch();
     griddep_wait();
     __shared__ float red[33];
     const int t = blockIdx.x, h = blockIdx.y;
     const size_t base = (size_t)t * a.H * a.dv + (size_t)h * a.dv;
+    const float den = fmaxf(fabsf(a.nq[(size_t)t * a.H + h]), a.m_scale[(size_t)t * a.H + h]) + 1e-6f;
     float ss = 0.f;
-    for (int i = threadIdx.x; i < a.dv; i += blockDim.x) { const float v = a.o_raw[base + i]; ss += v * v; }
+    for (int i = threadIdx.x; i < a.dv; i += blockDim.x) { const float v = a.o_raw[base + i] / den; ss += v * v; }
     const float rinv = 1.f / sqrtf(block_sum(ss, red) / (float)a.dv + a.eps);
     for (int i = threadIdx.x; i < a.dv; i += blockDim.x) {
         const float gate = sigmoid_f(a.proj[(size_t)t * a.ldp + a.g_off + h * a.dv + i]);
-        a.out[base + i] = a.o_raw[base + i] * rinv * a.norm_w[h * a.dv + i] * gate;
+        a.out[base + i] = a.o_raw[base + i] / den * rinv * a.norm_w[h * a.dv + i] * gate;
     }
 }
 
 cudaError_t matrix_mem_launch(const MatrixMemArgs& a, const RaggedDev& r, cudaStream_t s) {
     if (a.dv <= 0 || a.d <= 0 || a.d > MM_ROWS * 16) return cudaErrorInvalidValue;
     const int RG = (a.d + MM_ROWS - 1) / MM_ROWS;
-    const size_t smem = (size_t)(2 * MM_TB * (2 * a.d + MM_COLS + 2 + 1 + RG * (MM_COLS + 1))) * 4;
+    const size_t smem = (size_t)(2 * MM_TB * (2 * a.d + MM_COLS + 2 + RG * MM_COLS)) * 4;
     static bool attr_done = false;
-    if (!attr_done) { cudaFuncSetAttribute(matrix_mem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024); attr_done = true; }
-    cudaError_t ce = launch_chain(matrix_mem_gates_kernel, dim3((r.T * a.H + 127) / 128), dim3(128), 0, s, a, r.T);
+    if (!attr_done) { cudaFuncSetAttribute(matrix_mem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 140 * 1024); attr_done = true; }
+    cudaError_t ce = launch_chain(matrix_mem_gates_kernel, dim3(r.n_seg, a.H), dim3(MG_TB), 0, s, a, r);
     if (ce != cudaSuccess) return ce;
     {
         PlainLaunch pl;    // latency-bound over the prompt: CTAs spread over all SMs (see kernels.h)
-        ce = launch_chain(matrix_mem_kernel, dim3(r.n_seg, a.H, (a.dv + MM_COLS - 1) / MM_COLS), dim3(std::max(RG * MM_COLS, 64)), smem, s, a, r, RG);
+        ce = launch_chain(matrix_mem_kernel, dim3(r.n_seg, a.H, (a.dv + MM_COLS - 1) / MM_COLS + 1), dim3(std::max(RG * MM_COLS, 64)), smem, s, a, r, RG);
     }
     if (ce != cudaSuccess) return ce;
     return launch_chain(matrix_mem_out_kernel, dim3(r.T, a.H), dim3(128), 0, s, a);
