@@ -17,8 +17,8 @@
 #include "dense_dev.cuh"
 #include "ptx.cuh"
 #include "quant_blocks.cuh"
-
-#include <cuda.h>
+#include "tc05.cuh"
+#include "tensor_map.h"
 
 #include <algorithm>
 
@@ -56,28 +56,6 @@ __device__ __forceinline__ bool tc_tile(const TcParams& p, int i, int n_tiles, T
     w.t0 = t * p.NT;
     w.t1 = p.a.T;
     return true;
-}
-
-__device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                 ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void tc_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-// K-major operand in 128-byte-swizzled rows: 8-row groups 1024 bytes apart; a 16-entry K step is 32 bytes further on
-__device__ __forceinline__ uint64_t tc_desc(uint32_t addr) {
-    return (uint64_t)((addr >> 4) & 0x3FFF) | (uint64_t)1 << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)2 << 61;
-}
-__device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
-    uint32_t r[16];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr) : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
 
 // long steps: 16 (or fewer, `count`) token columns t.. of weight row n; lanes of a warp hold neighbouring rows
@@ -203,12 +181,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) dense_tc_kernel(const __grid_co
             fence_mbar_init();
         }
         __syncwarp();
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_at)), "r"(tmem_cols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        tc_alloc(&tmem_at, tmem_cols);
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    tc_before_sync();
     __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    tc_after_sync();
     griddep_launch();
     const uint32_t tmem = tmem_at;
     const int nk = (a.K + TC_K - 1) / TC_K, first = blockIdx.x, step = gridDim.x;
@@ -248,7 +225,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) dense_tc_kernel(const __grid_co
         // ================= matrix instructions
         griddep_wait();
         const int n_tiles = a.grouped ? *a.g.n_tiles : 0;
-        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)((SHORT ? p.NW : p.NT) >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);
+        const uint32_t idesc = tc_idesc_bf16(TC_M, SHORT ? p.NW : p.NT);
         int s = 0, tile = 0;
         uint32_t use = 0;
         for (int i = first; i < p.n_work; i += step) {
@@ -256,10 +233,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) dense_tc_kernel(const __grid_co
             if (!tc_tile(p, i, n_tiles, w)) continue;
             const int b = tile & 1;
             if (tile >= 2) mbar_wait(&acc_empty[b], ((tile >> 1) - 1) & 1, p.err, 0x50002u, (unsigned)tile);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            tc_after_sync();
             for (int k = 0; k < nk; k++) {
                 mbar_wait(&full[s], use & 1, p.err, 0x50003u, (unsigned)k);
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                tc_after_sync();
                 const uint32_t at = smem_u32(ring + (size_t)s * stage_bytes);
                 const uint64_t dw = tc_desc(at), dx = tc_desc(at + w_bytes);
 #pragma unroll
@@ -281,11 +258,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) dense_tc_kernel(const __grid_co
             if (!tc_tile(p, i, n_tiles, w)) continue;
             const int b = tile & 1;
             mbar_wait(&acc_full[b], (tile >> 1) & 1, p.err, 0x50004u, (unsigned)tile);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            tc_after_sync();
             const uint32_t acc = tmem + b * p.cols + ((uint32_t)(warp * 32) << 16);
             float* y = a.y;
             const float* aux = a.aux;
-            if (!a.grouped) { y += w.z * a.y_bs; if (aux) aux += w.z * a.aux_bs; }
+            __nv_bfloat16* yb = a.yb;
+            if (!a.grouped) { y += w.z * a.y_bs; yb += w.z * a.y_bs; if (aux) aux += w.z * a.aux_bs; }
             if constexpr (SHORT) {
                 const int t = w.t0 + threadIdx.x, n_end = min(w.n0 + p.NW, a.N);
                 if (w.t0 + warp * 32 < w.t1) {
@@ -293,7 +271,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) dense_tc_kernel(const __grid_co
                         float v[16];
                         __syncwarp();
                         tc_ld16(acc + c, v);
-                        if (w.n0 + c < n_end) tc_store_rows<EPI, ROUNDED>(a, y, a.yb, aux, (int)threadIdx.x < p.NT && t < w.t1, w.n0 + c, n_end, t, v);
+                        if (w.n0 + c < n_end) tc_store_rows<EPI, ROUNDED>(a, y, yb, aux, (int)threadIdx.x < p.NT && t < w.t1, w.n0 + c, n_end, t, v);
                     }
                 }
             } else {
@@ -303,17 +281,17 @@ __global__ void __launch_bounds__(TC_THREADS, 1) dense_tc_kernel(const __grid_co
                     float v[16];
                     __syncwarp();
                     tc_ld16(acc + c, v);
-                    tc_store<EPI, ROUNDED>(a, y, a.yb, aux, bias, n, w.t0 + c, min(16, left - c), v);
+                    tc_store<EPI, ROUNDED>(a, y, yb, aux, bias, n, w.t0 + c, min(16, left - c), v);
                 }
             }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            tc_before_sync();
             mbar_arrive(&acc_empty[b]);
             tile++;
         }
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    tc_before_sync();
     __syncthreads();
-    if (warp == 5) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols) : "memory");
+    if (warp == 5) tc_dealloc(tmem, tmem_cols);
 }
 
 // ---------------------------------------------------------------- rounded inputs
@@ -356,8 +334,7 @@ __global__ void rows_to_bf16_kernel(const TX* __restrict__ x, int ldx, const int
 typedef CUresult (*TcEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-// [nb][rows][K] bf16, rows `ld` and batch entries `bs` entries apart; boxes of 64 x box_rows
-static bool tc_map(CUtensorMap* m, const void* base, int K, long rows, long ld, long nb, long bs, int box_rows) {
+static bool encode_map(CUtensorMap* m, const void* base, const cuuint64_t (&dims)[3], const cuuint64_t (&strides)[2], const cuuint32_t (&box)[3]) {
     static const TcEncodeFn encode = [] {
         void* fn = nullptr;
         cudaDriverEntryPointQueryResult q;
@@ -365,12 +342,21 @@ static bool tc_map(CUtensorMap* m, const void* base, int K, long rows, long ld, 
         cudaGetLastError();
         return (TcEncodeFn)fn;
     }();
-    if (!encode) return false;
-    const cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)rows, (cuuint64_t)nb};
+    const cuuint32_t es[3] = {1, 1, 1};
+    return encode && encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+bool bf16_rows_map(CUtensorMap* m, const void* base, long cols, long rows, long ld, long nb, long bs, int box_rows) {
+    const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)nb};
     const cuuint64_t strides[2] = {(cuuint64_t)ld * 2, (cuuint64_t)(nb > 1 ? bs * 2 : ld * 2)};
-    const cuuint32_t box[3] = {TC_K, (cuuint32_t)box_rows, 1}, es[3] = {1, 1, 1};
-    return encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    const cuuint32_t box[3] = {TC_K, (cuuint32_t)box_rows, 1};
+    return encode_map(m, base, dims, strides, box);
+}
+bool bf16_heads_map(CUtensorMap* m, const void* base, long cols, long heads, long rows, int box_rows) {
+    const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)heads, (cuuint64_t)rows};
+    const cuuint64_t strides[2] = {(cuuint64_t)cols * 2, (cuuint64_t)(cols * heads) * 2};
+    const cuuint32_t box[3] = {TC_K, 1, (cuuint32_t)box_rows};
+    return encode_map(m, base, dims, strides, box);
 }
 
 typedef void (*TcKernel)(const CUtensorMap, const CUtensorMap, const TcParams);
@@ -385,7 +371,11 @@ static TcKernel tc_kernel_of(bool short_step) {
 static TcKernel tc_kernel(int epi, bool rounded, bool short_step) {
     if (rounded) {
         switch (epi) {
+            case EPI_NONE: return tc_kernel_of<EPI_NONE, true>(short_step);
+            case EPI_MUL_SIGMOID: return tc_kernel_of<EPI_MUL_SIGMOID, true>(short_step);
             case EPI_BIAS_RELU2: return tc_kernel_of<EPI_BIAS_RELU2, true>(short_step);
+            case EPI_GLU_GELU: return tc_kernel_of<EPI_GLU_GELU, true>(short_step);
+            case EPI_PIECEWISE: return tc_kernel_of<EPI_PIECEWISE, true>(short_step);
             case EPI_GLU_SILU: return tc_kernel_of<EPI_GLU_SILU, true>(short_step);
             case EPI_GLU_CLAMP: return tc_kernel_of<EPI_GLU_CLAMP, true>(short_step);
             default: return nullptr;
@@ -461,8 +451,8 @@ cudaError_t dense_tc_launch(const DenseArgs& a, const DenseDev& d, cudaStream_t 
     if (!kernel) return cudaErrorInvalidValue;
     CUtensorMap mw, mx;
     const long w_entries = grouped ? a.groups->n_groups : a.batch, w_bs = grouped ? a.groups->w_stride : a.w_bs;
-    if (!tc_map(&mw, a.w, a.K, a.N, a.K, w_entries, w_bs, p.NW)) return cudaErrorInvalidValue;
-    if (!tc_map(&mx, xb, a.K, rows, span, grouped ? 1 : a.batch, a.x_bs, p.NT)) return cudaErrorInvalidValue;
+    if (!bf16_rows_map(&mw, a.w, a.K, a.N, a.K, w_entries, w_bs, p.NW)) return cudaErrorInvalidValue;
+    if (!bf16_rows_map(&mx, xb, a.K, rows, span, grouped ? 1 : a.batch, a.x_bs, p.NT)) return cudaErrorInvalidValue;
     return launch_chain(kernel, dim3(std::min(p.n_work, SMS)), dim3(TC_THREADS), (size_t)p.stages * stage_bytes + TC_M * TC_K * 2 + 1024, s, mw, mx, p);
 }
 

@@ -1,0 +1,260 @@
+// Latent attention of long steps on the 5th-generation tensor cores (bf16 pages). Same arithmetic as latent_attn_mma_kernel
+// (latent_attn.cu): queries scaled, then rounded to bf16; cached rows as they are; probabilities rounded to bf16 for the weighted
+// sum, 32-bit everywhere else.
+//
+// A CTA takes 128 consecutive queries of one head and up to 256 latent columns of the output (tensor memory holds 128 lanes x 512
+// columns: 256 for the output, two score tiles of 64, two probability tiles of 32, so a 512-wide latent is two CTAs that both
+// compute the scores). The queries stay in shared memory; blocks of 64 cached rows come by tensor copies as parts of 64 columns and
+// serve both products: as rows of K for the scores, and, read across (N contiguous), as the values. Probabilities go to tensor
+// memory and are the second product's A operand.
+// Warps 0-3: softmax, one query a thread; 4: copies; 5: matrix instructions. The parts that are not values of this CTA are reloaded
+// while the softmax runs, and their share of the next block's scores is computed under it. The output is rescaled only when a
+// row's maximum has grown by more than 2^8 since the last time.
+#include "kernels.h"
+#include "layered.h"
+#include "ptx.cuh"
+#include "tc05.cuh"
+#include "tensor_map.h"
+
+#include <algorithm>
+
+namespace b2 {
+
+constexpr int LC_Q = 128, LC_K = 64, LC_PART = 64;          // queries, cached rows of a block, columns of a part
+constexpr int LC_QPART = LC_Q * LC_PART * 2, LC_KPART = LC_K * LC_PART * 2;
+constexpr int LC_V = 256;                                   // latent columns of the output per CTA
+
+namespace {
+__device__ __forceinline__ uint32_t lc_pack(float lo, float hi) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+// entry i of the rotated part of a head's query (see latent_attn.cu)
+__device__ __forceinline__ float lc_rotated(const LatentAttnArgs& a, int t, int h, int i, int pos) {
+    if (!a.q_raw) return a.qv[((size_t)t * a.H + h) * (a.rank + a.dr) + a.rank + i];
+    const float* v = a.q_raw + ((size_t)t * a.H + h) * (a.d + a.dr) + a.d;
+    const int half = a.rot.rot_dims / 2;
+    if (i >= a.rot.rot_dims) return v[i];
+    if (a.rot.pairs) {
+        const float cs = a.rot.cos[(size_t)pos * half + i / 2], sn = a.rot.sin[(size_t)pos * half + i / 2];
+        return i & 1 ? v[i] * cs + v[i - 1] * sn : v[i] * cs - v[i + 1] * sn;
+    }
+    const int p = i < half ? i : i - half;
+    const float cs = a.rot.cos[(size_t)pos * half + p], sn = a.rot.sin[(size_t)pos * half + p];
+    return i < half ? v[i] * cs - v[i + half] * sn : v[i] * cs + v[i - half] * sn;
+}
+}  // namespace
+
+// grid (heads x column chunks, 64-query tiles of the step, latest first; odd tiles of a sequence belong to the CTA before them)
+__global__ void __launch_bounds__(192, 1) latent_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_q,
+                                                                const LatentAttnArgs a, const RaggedDev r, int n_chunks, __nv_bfloat16* out, unsigned int* err) {
+    griddep_launch();
+    griddep_wait();
+    extern __shared__ uint8_t lc_smem[];
+    __shared__ uint64_t rest_full, val_full, rest_empty, val_empty, q_full, s_full[2], p_full[2], pv_done;
+    __shared__ uint32_t tmem_at;
+    const int tile = r.n_tiles - 1 - (int)blockIdx.y, h = blockIdx.x / n_chunks, chunk = blockIdx.x % n_chunks;
+    const int seg = r.tile_seg[tile], row0 = r.tile_row0[tile];
+    if (((row0 - r.seg_start[seg]) / 64) & 1) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nq = min(LC_Q, r.seg_start[seg] + r.seg_len[seg] - row0);
+    const int p0 = r.seg_pos0[seg] + row0 - r.seg_start[seg], p_last = p0 + nq - 1;
+    const int* table = a.block_tables[r.seg_slot[seg]];
+    const int n_parts = (a.rank + a.dr + LC_PART - 1) / LC_PART, v0 = chunk * (LC_V / LC_PART), n_val = min(LC_V, a.rank - chunk * LC_V) / LC_PART;
+    uint8_t* qs = reinterpret_cast<uint8_t*>(((uintptr_t)lc_smem + 1023) & ~(uintptr_t)1023);
+    uint8_t* ks = qs + (size_t)n_parts * LC_QPART;
+    const int b0 = max(0, p0 - a.window + 1) / LC_K, n_blocks = p_last / LC_K + 1 - b0;
+    if (warp == 5) {
+        if (lane == 0) {
+            mbar_init(&rest_full, 1); mbar_init(&val_full, 1); mbar_init(&rest_empty, 1); mbar_init(&val_empty, 1); mbar_init(&q_full, 1 + 128);
+            for (int i = 0; i < 2; i++) { mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 128); }
+            mbar_init(&pv_done, 1);
+            fence_mbar_init();
+        }
+        __syncwarp();
+        tc_alloc(&tmem_at, 512);
+    }
+    tc_before_sync();
+    __syncthreads();
+    tc_after_sync();
+    const uint32_t tmem = tmem_at, o_at = tmem, s_at = tmem + LC_V, p_at = tmem + LC_V + 2 * LC_K;
+
+    if (warp == 4 && lane == 0) {
+        // ================= copies: the latent parts of the queries, then blocks of cached rows
+        const int q_parts = a.rank / LC_PART, n_rest = n_parts - n_val;
+        mbar_arrive_expect_tx(&q_full, (uint32_t)(q_parts * LC_QPART));
+        for (int c = 0; c < q_parts; c++) tma_load_3d(qs + (size_t)c * LC_QPART, &map_q, c * LC_PART, h, row0, &q_full);
+        for (int i = 0; i < n_blocks; i++) {
+            const int j0 = (b0 + i) * LC_K, row = table[j0 / a.block_tokens] * a.block_tokens + j0 % a.block_tokens;
+            for (int half = 0; half < 2; half++) {
+                uint64_t *full = half ? &val_full : &rest_full, *empty = half ? &val_empty : &rest_empty;
+                if (half == 0 && n_rest == 0) continue;
+                if (i > 0) mbar_wait(empty, (i - 1) & 1, err, 0x60001u, (unsigned)i);
+                mbar_arrive_expect_tx(full, (uint32_t)((half ? n_val : n_rest) * LC_KPART));
+                for (int c = 0; c < n_parts; c++)
+                    if ((c >= v0 && c < v0 + n_val) == (half == 1)) tma_load_3d(ks + (size_t)c * LC_KPART, &map_k, c * LC_PART, row, 0, full);
+            }
+        }
+    } else if (warp == 5 && lane == 0) {
+        // ================= matrix instructions
+        const uint32_t id_s = tc_idesc_bf16(LC_Q, LC_K), id_o = tc_idesc_bf16(LC_Q, n_val * LC_PART, true);
+        const uint32_t qa = smem_u32(qs), ka = smem_u32(ks);
+        bool first = true;
+        auto scores = [&](int i, bool values) {              // one group of parts of block i's scores
+            for (int c = 0; c < n_parts; c++) {
+                if ((c >= v0 && c < v0 + n_val) != values) continue;
+                const uint64_t dq = tc_desc(qa + c * LC_QPART), dk = tc_desc(ka + c * LC_KPART);
+#pragma unroll
+                for (int k = 0; k < LC_PART / 16; k++) { tc_mma(s_at + (i & 1) * LC_K, dq + 2 * k, dk + 2 * k, id_s, first ? 0u : 1u); first = false; }
+            }
+        };
+        const bool any_rest = n_parts > n_val;
+        mbar_wait(&q_full, 0, err, 0x60002u);
+        tc_after_sync();
+        if (any_rest) { mbar_wait(&rest_full, 0, err, 0x60003u); tc_after_sync(); scores(0, false); tc_commit(&rest_empty); }
+        mbar_wait(&val_full, 0, err, 0x60004u);
+        tc_after_sync();
+        scores(0, true);
+        tc_commit(&s_full[0]);
+        for (int i = 0; i < n_blocks; i++) {
+            const bool more = i + 1 < n_blocks;
+            first = true;
+            if (more && any_rest) { mbar_wait(&rest_full, (i + 1) & 1, err, 0x60005u, (unsigned)i); tc_after_sync(); scores(i + 1, false); tc_commit(&rest_empty); }
+            mbar_wait(&p_full[i & 1], (i >> 1) & 1, err, 0x60006u, (unsigned)i);
+            tc_after_sync();
+#pragma unroll
+            for (int k = 0; k < LC_K / 16; k++)
+                tc_mma_ts(o_at, p_at + (i & 1) * (LC_K / 2) + k * 8, tc_desc(ka + v0 * LC_KPART + k * 2048, LC_KPART), id_o, (i | k) ? 1u : 0u);
+            tc_commit(&pv_done);
+            tc_commit(&val_empty);
+            if (more) {
+                mbar_wait(&val_full, (i + 1) & 1, err, 0x60007u, (unsigned)i);
+                tc_after_sync();
+                scores(i + 1, true);
+                tc_commit(&s_full[(i + 1) & 1]);
+            }
+        }
+    } else if (warp < 4) {
+        // ================= softmax: thread = query row
+        const int row = threadIdx.x, pos = p0 + row;
+        const uint32_t lanes = (uint32_t)(warp * 32) << 16;
+        // the rotated part of the queries (and zeros up to the part's 64 columns), rows past the tile as zeros
+        for (int c = a.rank; c < n_parts * LC_PART; c += 8) {
+            float v[8];
+#pragma unroll
+            for (int e = 0; e < 8; e++) v[e] = row < nq && c + e < a.rank + a.dr ? lc_rotated(a, row0 + row, h, c + e - a.rank, pos) * a.scale : 0.f;
+            uint8_t* dst = qs + (size_t)(c / LC_PART) * LC_QPART + row * 128 + ((((c % LC_PART) / 8) ^ (row & 7)) << 4);
+            *reinterpret_cast<uint4*>(dst) = make_uint4(lc_pack(v[0], v[1]), lc_pack(v[2], v[3]), lc_pack(v[4], v[5]), lc_pack(v[6], v[7]));
+        }
+        fence_proxy_async();
+        mbar_arrive(&q_full);
+        constexpr float LOG2E = 1.4426950408889634f;
+        float m_ref = a.sink ? a.sink[h] * LOG2E : -INFINITY, l = a.sink ? 1.f : 0.f;           // log2 domain: weights are 2^(score - m_ref)
+        for (int i = 0; i < n_blocks; i++) {
+            const int j0 = (b0 + i) * LC_K;
+            mbar_wait(&s_full[i & 1], (i >> 1) & 1, err, 0x60008u, (unsigned)i);
+            tc_after_sync();
+            uint32_t raw[2][32];
+            __syncwarp();
+            tc_ld32(s_at + (i & 1) * LC_K + lanes, raw[0]);
+            tc_ld32(s_at + (i & 1) * LC_K + 32 + lanes, raw[1]);
+            tc_wait_ld();
+            float s[LC_K];
+#pragma unroll
+            for (int j = 0; j < LC_K; j++) s[j] = __uint_as_float(raw[j >> 5][j & 31]) * LOG2E;
+            if (j0 + LC_K - 1 > p0 || p_last - j0 >= a.window) {
+                const int lo = pos - a.window + 1 - j0, hi = pos - j0;          // visible columns of this row
+#pragma unroll
+                for (int j = 0; j < LC_K; j++) if (j < lo || j > hi) s[j] = -INFINITY;
+            }
+            float mx = -INFINITY;
+#pragma unroll
+            for (int j = 0; j < LC_K; j++) mx = fmaxf(mx, s[j]);
+            const bool grow = mx > m_ref + 8.f || (m_ref == -INFINITY && mx > -INFINITY);
+            // the previous block's sum must be in before the output is rescaled, and before the older probability tile is rewritten
+            if (i > 0) { mbar_wait(&pv_done, (i - 1) & 1, err, 0x60009u, (unsigned)i); tc_after_sync(); }
+            if (__any_sync(0xffffffffu, grow)) {
+                const float m_new = grow ? mx : m_ref, f = grow ? exp2f(m_ref - m_new) : 1.f;
+                m_ref = m_new;
+                l *= f;
+                if (i > 0) {
+                    for (int c = 0; c < n_val * LC_PART; c += 32) {
+                        uint32_t o[32];
+                        tc_ld32(o_at + c + lanes, o);
+                        tc_wait_ld();
+#pragma unroll
+                        for (int e = 0; e < 32; e++) o[e] = __float_as_uint(__uint_as_float(o[e]) * f);
+                        tc_st32(o_at + c + lanes, o);
+                    }
+                }
+            }
+            const float ref = m_ref > -INFINITY ? m_ref : 0.f;                  // a row that has seen no key yet: all weights are 0
+            uint32_t p[32];
+#pragma unroll
+            for (int j = 0; j < LC_K; j += 2) {
+                const float e0 = exp2f(s[j] - ref), e1 = exp2f(s[j + 1] - ref);
+                l += e0 + e1;
+                p[j >> 1] = lc_pack(e0, e1);
+            }
+            __syncwarp();
+            tc_st32(p_at + (i & 1) * (LC_K / 2) + lanes, p);
+            tc_wait_st();
+            if (i == n_blocks - 1 && p_last - j0 + 1 < LC_K) {
+                // rows of the last block past the sequence: whatever the page holds must not meet the zero weights as values
+                const int r0 = p_last - j0 + 1, n_bad = LC_K - r0;
+                for (int e = threadIdx.x; e < n_val * n_bad * 8; e += 128) {
+                    const int c = e / (n_bad * 8), rr = r0 + e / 8 % n_bad;
+                    *reinterpret_cast<uint4*>(ks + (size_t)(v0 + c) * LC_KPART + rr * 128 + (e & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
+                }
+                fence_proxy_async();
+            }
+            tc_before_sync();
+            mbar_arrive(&p_full[i & 1]);
+        }
+        mbar_wait(&pv_done, (n_blocks - 1) & 1, err, 0x6000au);
+        tc_after_sync();
+        const float inv = 1.f / l;
+        __nv_bfloat16* dst = out + ((size_t)(row0 + row) * a.H + h) * a.rank + chunk * LC_V;
+        for (int c = 0; c < n_val * LC_PART; c += 32) {
+            uint32_t o[32];
+            __syncwarp();
+            tc_ld32(o_at + c + lanes, o);
+            tc_wait_ld();
+            if (row < nq) {
+#pragma unroll
+                for (int e = 0; e < 32; e += 8) {
+                    uint32_t u[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) u[q] = lc_pack(__uint_as_float(o[e + 2 * q]) * inv, __uint_as_float(o[e + 2 * q + 1]) * inv);
+                    *reinterpret_cast<uint4*>(dst + c + e) = make_uint4(u[0], u[1], u[2], u[3]);
+                }
+            }
+        }
+        tc_before_sync();
+    }
+    __syncthreads();
+    if (warp == 5) tc_dealloc(tmem, 512);
+}
+
+// ---------------------------------------------------------------- host side
+// Rows of 64-column parts that fit shared memory beside the queries (9 of them), whole chunks of output columns, pages of whole blocks.
+bool latent_attn_takes_tc(const LatentAttnArgs& a, int T) {
+    const int parts = (a.rank + a.dr + LC_PART - 1) / LC_PART;
+    return !a.cache_f32 && T >= LATENT_TC_MIN && a.rank % LC_PART == 0 && (a.rank <= LC_V || a.rank % LC_V == 0) && parts <= 9 && a.ld_row % 8 == 0 &&
+           a.block_tokens % LC_K == 0;
+}
+
+cudaError_t latent_attn_tc_launch(const LatentAttnArgs& a, const RaggedDev& r, const __nv_bfloat16* q, long pool_rows, __nv_bfloat16* out, cudaStream_t s) {
+    static const bool ready = cudaFuncSetAttribute(latent_attn_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 9 * (LC_QPART + LC_KPART) + 1024) == cudaSuccess;
+    if (!ready || !latent_attn_takes_tc(a, r.T)) return cudaErrorInvalidValue;
+    const int parts = (a.rank + a.dr + LC_PART - 1) / LC_PART, chunks = (a.rank + LC_V - 1) / LC_V;
+    CUtensorMap mk, mq;
+    // rows of the pages [pages * block_tokens][ld_row]; columns past rank + dr arrive as zeros
+    if (!bf16_rows_map(&mk, a.pool, a.rank + a.dr, pool_rows, a.ld_row, 1, 0, LC_K)) return cudaErrorInvalidValue;
+    // queries [T][H][rank]: 128 tokens of one head
+    if (!bf16_heads_map(&mq, q, a.rank, a.H, r.T, LC_Q)) return cudaErrorInvalidValue;
+    return launch_chain(latent_attn_tc_kernel, dim3(a.H * chunks, r.n_tiles), dim3(192), (size_t)parts * (LC_QPART + LC_KPART) + 1024, s, mk, mq, a, r, chunks,
+                        out, kernel_error_word());
+}
+
+}  // namespace b2

@@ -1108,19 +1108,34 @@ static int mix_latent_attn(b2_engine* e, LayeredModel* m, LyLayer& L, const Ragg
     // every head's unrotated query through its transposed key map: the head's query in the latent's coordinates
     DenseArgs b = {};
     b.batch = H; b.x_bs = dq; b.w_bs = (long)d.la_rank * d.head_dim; b.y_bs = Dk; b.x_span = H * dq;
-    if ((rc = dense(e, m, L.uk_t, q, ldq, m->buf[0], H * Dk, T, nullptr, EPI_NONE, 1, &b))) return rc;
-    {
-        StepProfiler sp(m, st, 2);
-        CK(latent_attn_launch(a, r, st));
-        e->launches += 2;
-    }
     // values of the weighted latent sums, head by head, times the sigmoid output gate (one number per entry or per head)
     const bool gate = !(d.attn_flags & B2_ATTN_NO_GATE), head_gate = (d.attn_flags & B2_ATTN_HEAD_GATE) != 0;
     DenseArgs v = {};
     v.batch = H; v.x_bs = d.la_rank; v.w_bs = (long)d.la_vdim * d.la_rank; v.y_bs = d.la_vdim; v.x_span = H * d.la_rank;
     if (gate) { v.aux = m->proj + L.g_off; v.ldaux = Np; v.aux_bs = head_gate ? 1 : d.la_vdim; v.aux_one = head_gate; }
-    if ((rc = dense(e, m, L.uv, m->buf[1], H * d.la_rank, m->buf[2], H * d.la_vdim, T, nullptr, gate ? EPI_MUL_SIGMOID : EPI_NONE, 1, &v))) return rc;
-    return dense(e, m, L.attn_o, m->buf[2], H * d.la_vdim, m->oL, W, T);
+    const int v_epi = gate ? EPI_MUL_SIGMOID : EPI_NONE;
+    DenseArgs op = {};
+    if (latent_attn_takes_tc(a, T) && dense_takes_rounded(dense_args(m, L.uk_t, q, ldq, m->buf[0], H * Dk, T, nullptr, EPI_NONE, &b)) &&
+        dense_takes_rounded(dense_args(m, L.uv, m->buf[1], H * d.la_rank, m->buf[2], H * d.la_vdim, T, nullptr, v_epi, &v)) && takes_rounded(m, L.attn_o, T)) {
+        // long steps: what these products and the attention hand on is left rounded
+        __nv_bfloat16* qb = reinterpret_cast<__nv_bfloat16*>(m->buf[1]);
+        b.scale = a.scale; b.y_bs = d.la_rank; b.y_rounded = qb;
+        if ((rc = dense(e, m, L.uk_t, q, ldq, nullptr, H * d.la_rank, T, nullptr, EPI_NONE, 1, &b))) return rc;
+        {
+            StepProfiler sp(m, st, 2);
+            CK(latent_attn_tc_launch(a, r, qb, (long)c.kv_num_blocks * c.kv_block_tokens, m->xb, st));
+            e->launches++;
+        }
+        v.x_rounded = m->xb; v.y_rounded = qb;
+        op.x_rounded = qb;
+    } else {
+        if ((rc = dense(e, m, L.uk_t, q, ldq, m->buf[0], H * Dk, T, nullptr, EPI_NONE, 1, &b))) return rc;
+        StepProfiler sp(m, st, 2);
+        CK(latent_attn_launch(a, r, st));
+        e->launches += 2;
+    }
+    if ((rc = dense(e, m, L.uv, m->buf[1], H * d.la_rank, m->buf[2], H * d.la_vdim, T, nullptr, v_epi, 1, &v))) return rc;
+    return dense(e, m, L.attn_o, m->buf[2], H * d.la_vdim, m->oL, W, T, nullptr, EPI_NONE, 1, &op);
 }
 
 static int mix_delta_rule(b2_engine* e, LayeredModel* m, LyLayer& L, const RaggedDev& r, const float* in) {
@@ -1323,15 +1338,19 @@ static int ff_piecewise(b2_engine* e, LayeredModel* m, LyLayer& L, const RaggedD
     DenseArgs up = {};
     up.p0 = L.act_p0; up.p1 = L.act_p1;
     int rc;
+    DenseArgs down = {};
+    if (takes_rounded(m, L.up, T) && takes_rounded(m, L.down, T)) down.x_rounded = up.y_rounded = reinterpret_cast<__nv_bfloat16*>(m->ff);
     if ((rc = dense(e, m, L.up, in, W, m->ff, L.d.n_ff, T, nullptr, EPI_PIECEWISE, 1, &up))) return rc;
-    return dense(e, m, L.down, m->ff, L.d.n_ff, out, W, T);
+    return dense(e, m, L.down, m->ff, L.d.n_ff, out, W, T, nullptr, EPI_NONE, 1, &down);
 }
 
 static int ff_relu2(b2_engine* e, LayeredModel* m, LyLayer& L, const RaggedDev& r, const float* in, float* out) {
     const int T = r.T, W = m->c.n_embd;
     int rc;
-    if ((rc = dense(e, m, L.up, in, W, m->ff, L.d.n_ff, T, L.up_b, EPI_BIAS_RELU2))) return rc;
-    return dense(e, m, L.down, m->ff, L.d.n_ff, out, W, T, L.down_b, EPI_BIAS);
+    DenseArgs up = {}, down = {};
+    if (takes_rounded(m, L.up, T) && takes_rounded(m, L.down, T)) down.x_rounded = up.y_rounded = reinterpret_cast<__nv_bfloat16*>(m->ff);
+    if ((rc = dense(e, m, L.up, in, W, m->ff, L.d.n_ff, T, L.up_b, EPI_BIAS_RELU2, 1, &up))) return rc;
+    return dense(e, m, L.down, m->ff, L.d.n_ff, out, W, T, L.down_b, EPI_BIAS, 1, &down);
 }
 
 static int ff_glu(b2_engine* e, LayeredModel* m, LyLayer& L, const RaggedDev& r, const float* in, float* out) {
@@ -1339,8 +1358,10 @@ static int ff_glu(b2_engine* e, LayeredModel* m, LyLayer& L, const RaggedDev& r,
     int rc;
     // ff_act belongs to the dense block; a mixture's shared expert is a SiLU unit
     const int epi = L.d.ff_kind == B2_FF_GLU && L.d.ff_act == B2_ACT_GELU_TANH ? EPI_GLU_GELU : EPI_GLU_SILU;
-    if ((rc = dense(e, m, L.glu_gate_up, in, W, m->ff, ff, T, nullptr, epi))) return rc;
-    return dense(e, m, L.glu_down, m->ff, ff, out, W, T);
+    DenseArgs up = {}, down = {};
+    if (takes_rounded(m, L.glu_gate_up, T) && takes_rounded(m, L.glu_down, T)) down.x_rounded = up.y_rounded = reinterpret_cast<__nv_bfloat16*>(m->ff);
+    if ((rc = dense(e, m, L.glu_gate_up, in, W, m->ff, ff, T, nullptr, epi, 1, &up))) return rc;
+    return dense(e, m, L.glu_down, m->ff, ff, out, W, T, nullptr, EPI_NONE, 1, &down);
 }
 
 // The two grouped products of a mixture, ready to launch, and what the residual kernel needs to add up their output.

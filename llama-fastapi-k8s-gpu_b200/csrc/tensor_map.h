@@ -1,0 +1,12 @@
+// Tensor maps over bf16 matrices for copies into 128-byte-swizzled shared memory (boxes 64 entries wide); made in dense_tc.cu.
+#pragma once
+#include <cuda.h>
+
+namespace b2 {
+
+// [nb][rows][cols], rows `ld` and batch entries `bs` entries apart; boxes of 64 x box_rows. Entries past the end are read as zeros.
+bool bf16_rows_map(CUtensorMap* m, const void* base, long cols, long rows, long ld, long nb, long bs, int box_rows);
+// [rows][heads][cols]: boxes of 64 columns of one head, box_rows rows; coordinates (column, head, row)
+bool bf16_heads_map(CUtensorMap* m, const void* base, long cols, long heads, long rows, int box_rows);
+
+}  // namespace b2
