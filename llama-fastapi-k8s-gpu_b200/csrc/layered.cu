@@ -1028,7 +1028,8 @@ static int mix_window_scan(b2_engine* e, LayeredModel* m, LyLayer& L, const Ragg
     a.proj = m->proj; a.ldp = Np; a.q_off = L.q_off; a.k_off = L.k_off; a.q_norm_w = L.q_norm; a.k_norm_w = L.k_norm;
     a.rot.cos = L.rot_cos; a.rot.sin = L.rot_sin; a.rot.rot_dims = d.rot_dims;
     a.k_pool = L.k_pool; a.v_pool = L.v_pool; a.cache_f32 = m->exact ? 1 : 0; a.block_tables = m->block_tables;
-    a.block_tokens = c.kv_block_tokens; a.H = d.n_head; a.G = d.n_head_kv; a.d = d.head_dim; a.window = d.window;
+    a.block_tokens = c.kv_block_tokens; a.pool_rows = (long)c.kv_num_blocks * d.n_head_kv * c.kv_block_tokens;
+    a.H = d.n_head; a.G = d.n_head_kv; a.d = d.head_dim; a.window = d.window;
     a.keep_first = d.keep_first; a.scale = (float)d.attn_scale; a.eps = c.norm_eps; a.q_rot = m->buf[0]; a.out = m->buf[1];
     a.split_scratch = m->attn_split; a.split_capacity = m->attn_split_floats;
     {
@@ -1275,6 +1276,7 @@ static int mix_sink(b2_engine* e, LayeredModel* m, LyLayer& L, const RaggedDev& 
     a.proj = m->proj; a.ldp = Np; a.q_off = L.q_off; a.k_off = L.k_off; a.v_off = L.v_off;
     a.rot.cos = L.rot_cos; a.rot.sin = L.rot_sin; a.rot.rot_dims = d.rot_dims; a.unit_qk = (d.attn_flags & B2_ATTN_UNIT_QK) ? 1 : 0;
     a.k_pool = L.k_pool; a.v_pool = L.v_pool; a.cache_f32 = m->exact ? 1 : 0; a.block_tables = m->block_tables; a.block_tokens = c.kv_block_tokens;
+    a.pool_rows = (long)c.kv_num_blocks * d.n_head_kv * c.kv_block_tokens;
     a.H = H; a.G = d.n_head_kv; a.d = d.head_dim; a.dv = d.attn_vdim; a.window = d.window; a.scale = (float)d.attn_scale; a.eps = c.norm_eps;
     a.sink = L.sink; a.talk = L.talk; a.gate = L.gl_off >= 0 ? m->proj + L.gl_off : nullptr; a.ld_gate = Np; a.gate_per_head = (d.attn_flags & B2_ATTN_HEAD_GATE) ? 1 : 0;
     a.q_rot = m->buf[0]; a.cross = m->cross; a.out = m->buf[1]; a.ld_out = Ko;

@@ -126,6 +126,7 @@ struct WindowAttnArgs {
     void* k_pool; void* v_pool; int cache_f32;        // pages [page][G][block_tokens][d]; bf16 or f32
     int* const* block_tables;                         // [slot] -> page table
     int block_tokens;
+    long pool_rows;                                   // rows of a pool: pages * G * block_tokens
     int H, G, d;
     int window, keep_first;
     float scale, eps;
@@ -372,6 +373,7 @@ struct SinkAttnArgs {
     int side_off, side_gate, side_n, side_col;                 // side_n == 0: none
     void* k_pool; void* v_pool; int cache_f32;                 // pages [page][G][block_tokens][d] and [page][G][block_tokens][dv]
     int* const* block_tables; int block_tokens;
+    long pool_rows;                                            // rows of a pool: pages * G * block_tokens
     int H, G, d, dv, window;
     float scale, eps;
     const float* sink;                                         // [H] or null

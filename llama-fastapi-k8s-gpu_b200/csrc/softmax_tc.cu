@@ -1,0 +1,301 @@
+// Softmax attention of long steps on the 5th-generation tensor cores, for the layer-list models (bf16 pages, key and value sizes up to
+// 128). Same precision as the mma.sync kernels that shorter steps take: queries and probabilities enter the products as TWO bf16 each
+// (leading part + remainder), so the only 16-bit rounding is that of the cached keys and values; everything else is 32-bit.
+//
+// A CTA takes 128 consecutive queries of one head; blocks of 128 keys and values come by tensor copies (two pages rows of 64 each, parts
+// of 64 columns in 128-byte-swizzled rows, two stages). Tensor memory holds the output (128 columns), two score tiles (2 x 128) and the two
+// halves of the probabilities (64 + 64), which are the A operand of the second product. The next block's scores are computed while
+// this one's softmax runs. Eight softmax warps, two threads a query row with 64 key columns each (capped scores take three special-function
+// operations a score, which is what bounds the kernel); they exchange their maxima through shared memory. The output is rescaled only
+// when a row's maximum has grown by more than 2^8.
+#include "kernels.h"
+#include "layered.h"
+#include "ptx.cuh"
+#include "softmax_tc.h"
+#include "tc05.cuh"
+#include "tensor_map.h"
+
+#include <algorithm>
+
+namespace b2 {
+
+constexpr int SX_Q = 128, SX_K = 128, SX_PART = SX_Q * 128;       // queries, keys of a block; bytes of a part (128 rows x 64 columns)
+constexpr int SX_THREADS = 320;                                   // warps 0-7 softmax, 8 copies, 9 matrix instructions
+
+namespace {
+__device__ __forceinline__ float sx_exp2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+__device__ __forceinline__ float sx_rcp(float x) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+__device__ __forceinline__ void sx_split(float a, float b, uint32_t& hi, uint32_t& lo) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    const __nv_bfloat162 l = __floats2bfloat162_rn(a - __low2float(h), b - __high2float(h));
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+}  // namespace
+
+// grid (heads, 64-query tiles of the step, latest first; odd tiles of a sequence belong to the CTA before them)
+template <bool CAP>
+__global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
+                                                                   const SoftmaxTcArgs a, const RaggedDev r, unsigned int* err) {
+    griddep_launch();
+    griddep_wait();
+    extern __shared__ uint8_t sx_smem[];
+    __shared__ uint64_t k_full[2], k_empty[2], v_full[2], v_empty[2], q_full, s_full[2], p_full, pv_done;
+    __shared__ uint32_t tmem_at;
+    __shared__ float row_max[2][2][SX_Q], row_sum[2][SX_Q];
+    const int tile = r.n_tiles - 1 - (int)blockIdx.y, h = blockIdx.x;
+    const int seg = r.tile_seg[tile], row0 = r.tile_row0[tile];
+    if (((row0 - r.seg_start[seg]) / 64) & 1) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nq = min(SX_Q, r.seg_start[seg] + r.seg_len[seg] - row0);
+    const int p0 = r.seg_pos0[seg] + row0 - r.seg_start[seg], p_last = p0 + nq - 1;
+    const int* table = a.block_tables[r.seg_slot[seg]];
+    const int g = h / (a.H / a.G), bt = a.block_tokens;
+    const int k_parts = (a.d + 63) / 64, v_parts = (a.dv + 63) / 64;
+    uint8_t* qs = reinterpret_cast<uint8_t*>(((uintptr_t)sx_smem + 1023) & ~(uintptr_t)1023);      // [leading, remainder][part]
+    uint8_t* ks = qs + 2 * k_parts * SX_PART;                                                      // [stage][part]
+    uint8_t* vs = ks + 2 * k_parts * SX_PART;
+    // key blocks: those of the kept prefix, then those of the window
+    const int lo_first = a.window > 0 ? max(0, p0 - a.window + 1) : 0;
+    const int n_kept = lo_first > 0 ? (min(a.keep_first, lo_first) + SX_K - 1) / SX_K : 0;
+    const int w0 = max(lo_first / SX_K, n_kept), n_blocks = n_kept + p_last / SX_K + 1 - w0;
+    auto block_at = [&](int i) { return (i < n_kept ? i : w0 + i - n_kept) * SX_K; };
+    if (warp == 9) {
+        if (lane == 0) {
+            for (int i = 0; i < 2; i++) {
+                mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); mbar_init(&s_full[i], 1);
+            }
+            mbar_init(&q_full, 256); mbar_init(&p_full, 256); mbar_init(&pv_done, 1);
+            fence_mbar_init();
+        }
+        __syncwarp();
+        tc_alloc(&tmem_at, 512);
+    }
+    tc_before_sync();
+    __syncthreads();
+    tc_after_sync();
+    const uint32_t o_at = tmem_at, s_at = tmem_at + 128, p_at = tmem_at + 384;       // probabilities: 64 columns leading, 64 remainder
+
+    if (warp == 8 && lane == 0) {
+        // ================= copies
+        for (int i = 0; i < n_blocks; i++) {
+            const int st = i & 1, j0 = block_at(i), halves = j0 + 64 <= p_last ? 2 : 1;
+            for (int kv = 0; kv < 2; kv++) {
+                uint64_t *full = kv ? &v_full[st] : &k_full[st], *empty = kv ? &v_empty[st] : &k_empty[st];
+                const int parts = kv ? v_parts : k_parts;
+                uint8_t* dst = (kv ? vs : ks) + (size_t)st * parts * SX_PART;
+                if (i >= 2) mbar_wait(empty, ((i >> 1) - 1) & 1, err, 0x70001u, (unsigned)i);
+                mbar_arrive_expect_tx(full, (uint32_t)(halves * parts * (SX_PART / 2)));
+                for (int hf = 0; hf < halves; hf++) {
+                    const int j = j0 + 64 * hf, row = (table[j / bt] * a.G + g) * bt + j % bt;
+                    for (int c = 0; c < parts; c++) tma_load_3d(dst + (size_t)c * SX_PART + hf * (SX_PART / 2), kv ? &map_v : &map_k, c * 64, row, 0, full);
+                }
+            }
+        }
+    } else if (warp == 9 && lane == 0) {
+        // ================= matrix instructions
+        const uint32_t id_s = tc_idesc_bf16(SX_Q, SX_K), id_o = tc_idesc_bf16(SX_Q, a.dv, true);
+        const uint32_t qa = smem_u32(qs), ka = smem_u32(ks), va = smem_u32(vs);
+        auto scores = [&](int i) {
+            mbar_wait(&k_full[i & 1], (i >> 1) & 1, err, 0x70002u, (unsigned)i);
+            tc_after_sync();
+            for (int part = 0; part < 2 * k_parts; part++) {             // remainders first
+                const int c = part % k_parts, lead = part / k_parts;
+                const uint64_t dq = tc_desc(qa + ((lead ? 0 : k_parts) + c) * SX_PART), dk = tc_desc(ka + ((i & 1) * k_parts + c) * SX_PART);
+#pragma unroll
+                for (int k = 0; k < 4; k++) tc_mma(s_at + (i & 1) * SX_K, dq + 2 * k, dk + 2 * k, id_s, (part | k) ? 1u : 0u);
+            }
+            tc_commit(&s_full[i & 1]);
+            tc_commit(&k_empty[i & 1]);
+        };
+        mbar_wait(&q_full, 0, err, 0x70003u);
+        tc_after_sync();
+        scores(0);
+        for (int i = 0; i < n_blocks; i++) {
+            if (i + 1 < n_blocks) scores(i + 1);
+            mbar_wait(&v_full[i & 1], (i >> 1) & 1, err, 0x70004u, (unsigned)i);
+            mbar_wait(&p_full, i & 1, err, 0x70005u, (unsigned)i);
+            tc_after_sync();
+            const uint32_t v_at = va + (i & 1) * v_parts * SX_PART;
+#pragma unroll
+            for (int half = 0; half < 2; half++)                         // remainders first
+#pragma unroll
+                for (int k = 0; k < SX_K / 16; k++)
+                    tc_mma_ts(o_at, p_at + (half ? 0 : 64) + k * 8, tc_desc(v_at + k * 2048, SX_PART), id_o, (i | half | k) ? 1u : 0u);
+            tc_commit(&pv_done);
+            tc_commit(&v_empty[i & 1]);
+        }
+    } else if (warp < 8) {
+        // ================= softmax: threads t and t + 128 share query row t, key columns 0-63 and 64-127 of a block
+        const int row = threadIdx.x & 127, side = threadIdx.x >> 7, pos = p0 + row;
+        const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
+        constexpr float LOG2E = 1.4426950408889634f;
+        // scores live in the log2 domain. Capped: cap tanh(s / cap) = cap - 2 cap / (exp(2 s / cap) + 1), the exponential's factor folded
+        // into the query as well
+        const float q_mul = CAP ? a.scale * (2.f * LOG2E) / a.softcap : a.scale * LOG2E;
+        [[maybe_unused]] const float cap2 = CAP ? a.softcap * LOG2E : 0.f;
+        {   // queries, 8 columns at a time: neighbouring threads take neighbouring pieces of a row
+            const int per = k_parts * 8, d8 = a.d / 8;
+            for (int e = threadIdx.x; e < SX_Q * per; e += 256) {
+                const int rr = e / per, c8 = e % per;
+                float v[8] = {};
+                if (rr < nq && c8 < d8) {
+                    const float4* src = reinterpret_cast<const float4*>(a.q + ((size_t)(row0 + rr) * a.H + h) * a.d + c8 * 8);
+                    const float4 x = src[0], y = src[1];
+                    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
+                }
+                uint32_t hi[4], lo[4];
+#pragma unroll
+                for (int k = 0; k < 4; k++) sx_split(v[2 * k] * q_mul, v[2 * k + 1] * q_mul, hi[k], lo[k]);
+                uint8_t* dst = qs + (size_t)(c8 >> 3) * SX_PART + rr * 128 + (((c8 & 7) ^ (rr & 7)) << 4);
+                *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                *reinterpret_cast<uint4*>(dst + (size_t)k_parts * SX_PART) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            }
+            fence_proxy_async();
+            mbar_arrive(&q_full);
+        }
+        const float sink = a.sink ? a.sink[h] * LOG2E : -INFINITY;
+        float m_ref = sink, l = 0.f;                              // weights are 2^(score - m_ref); the sink's term joins at the end
+        const int lo_key = a.window > 0 ? max(0, pos - a.window + 1) : 0;
+        for (int i = 0; i < n_blocks; i++) {
+            const int j0 = block_at(i), c0 = j0 + side * 64;      // this thread's first key
+            mbar_wait(&s_full[i & 1], (i >> 1) & 1, err, 0x70006u, (unsigned)i);
+            tc_after_sync();
+            float s[64];
+            {
+                uint32_t raw[2][32];
+                __syncwarp();
+                tc_ld32(s_at + (i & 1) * SX_K + side * 64 + lanes, raw[0]);
+                tc_ld32(s_at + (i & 1) * SX_K + side * 64 + 32 + lanes, raw[1]);
+                tc_wait_ld();
+#pragma unroll
+                for (int j = 0; j < 64; j++) s[j] = __uint_as_float(raw[j >> 5][j & 31]);
+            }
+            if constexpr (CAP)
+#pragma unroll
+                for (int j = 0; j < 64; j++) s[j] = fmaf(-2.f * cap2, sx_rcp(sx_exp2(s[j]) + 1.f), cap2);
+            if (j0 + SX_K - 1 > p0 || (a.window > 0 && p_last - j0 >= a.window)) {
+#pragma unroll
+                for (int j = 0; j < 64; j++) if (c0 + j > pos || (c0 + j < lo_key && c0 + j >= a.keep_first)) s[j] = -INFINITY;
+            }
+            float mx = -INFINITY;
+#pragma unroll
+            for (int j = 0; j < 64; j++) mx = fmaxf(mx, s[j]);
+            row_max[i & 1][side][row] = mx;
+            named_bar_sync(1, 256);
+            mx = fmaxf(mx, row_max[i & 1][side ^ 1][row]);
+            const bool grow = mx > m_ref + 8.f || (m_ref == -INFINITY && mx > -INFINITY);
+            // the previous block's products must be in before the output is rescaled and the probabilities are rewritten
+            if (i > 0) { mbar_wait(&pv_done, (i - 1) & 1, err, 0x70007u, (unsigned)i); tc_after_sync(); }
+            if (__any_sync(0xffffffffu, grow)) {
+                const float m_new = grow ? mx : m_ref, f = grow ? sx_exp2(m_ref - m_new) : 1.f;
+                m_ref = m_new;
+                l *= f;
+                if (i > 0) {                                      // this side's 64 columns of the output
+                    for (int c = side * 64; c < min(side * 64 + 64, v_parts * 64); c += 32) {
+                        uint32_t o[32];
+                        tc_ld32(o_at + c + lanes, o);
+                        tc_wait_ld();
+#pragma unroll
+                        for (int e = 0; e < 32; e++) o[e] = __float_as_uint(__uint_as_float(o[e]) * f);
+                        tc_st32(o_at + c + lanes, o);
+                    }
+                }
+            }
+            const float ref = m_ref > -INFINITY ? m_ref : 0.f;    // nothing visible yet and no sink: every weight is 0
+            uint32_t hi[32], lo[32];
+#pragma unroll
+            for (int j = 0; j < 64; j += 2) {
+                const float e0 = sx_exp2(s[j] - ref), e1 = sx_exp2(s[j + 1] - ref);
+                l += e0 + e1;
+                sx_split(e0, e1, hi[j >> 1], lo[j >> 1]);
+            }
+            __syncwarp();
+            tc_st32(p_at + side * 32 + lanes, hi);
+            tc_st32(p_at + 64 + side * 32 + lanes, lo);
+            tc_wait_st();
+            if (i == n_blocks - 1 && p_last - j0 + 1 < SX_K) {
+                // rows past the sequence: whatever shared memory or the page holds must not meet the zero weights as values
+                mbar_wait(&v_full[i & 1], (i >> 1) & 1, err, 0x70008u, (unsigned)i);
+                const int r0 = p_last - j0 + 1, n_bad = SX_K - r0;
+                for (int e = threadIdx.x; e < v_parts * n_bad * 8; e += 256) {
+                    const int c = e / (n_bad * 8), rr = r0 + e / 8 % n_bad;
+                    *reinterpret_cast<uint4*>(vs + (size_t)((i & 1) * v_parts + c) * SX_PART + rr * 128 + (e & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
+                }
+                fence_proxy_async();
+            }
+            tc_before_sync();
+            mbar_arrive(&p_full);
+        }
+        row_sum[side][row] = l;
+        named_bar_sync(1, 256);
+        l += row_sum[side ^ 1][row];
+        if (a.sink) l += sx_exp2(sink - m_ref);
+        const float inv = l > 0.f ? 1.f / l : 0.f;
+        mbar_wait(&pv_done, (n_blocks - 1) & 1, err, 0x70009u);
+        tc_after_sync();
+        const int t = row0 + row, dv = a.dv;
+        const size_t at = (size_t)t * a.ld_out + (size_t)h * dv;
+        const float* gate = a.gate && row < nq ? a.gate + (size_t)t * a.ld_gate + (a.gate_per_head ? h : h * dv) : nullptr;
+        const float head_gate = gate && a.gate_per_head ? 1.f / (1.f + expf(-gate[0])) : 1.f;
+        for (int c = side * 64; c < min(side * 64 + 64, dv); c += 32) {
+            uint32_t o[32];
+            __syncwarp();
+            tc_ld32(o_at + c + lanes, o);
+            tc_wait_ld();
+            if (row >= nq) continue;
+#pragma unroll
+            for (int e = 0; e < 32; e += 8) {                     // dv is a multiple of 16
+                if (c + e >= dv) break;
+                float v[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++) {
+                    v[k] = __uint_as_float(o[e + k]) * inv;
+                    if (gate && !a.gate_per_head) v[k] *= 1.f / (1.f + expf(-gate[c + e + k]));
+                    else v[k] *= head_gate;
+                }
+                if (a.out_bf16) {
+                    uint32_t u[4];
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const __nv_bfloat162 b = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
+                        u[k] = *reinterpret_cast<const uint32_t*>(&b);
+                    }
+                    *reinterpret_cast<uint4*>(a.out_bf16 + at + c + e) = make_uint4(u[0], u[1], u[2], u[3]);
+                } else {
+                    *reinterpret_cast<float4*>(a.out + at + c + e) = make_float4(v[0], v[1], v[2], v[3]);
+                    *reinterpret_cast<float4*>(a.out + at + c + e + 4) = make_float4(v[4], v[5], v[6], v[7]);
+                }
+            }
+        }
+        tc_before_sync();
+    }
+    __syncthreads();
+    if (warp == 9) tc_dealloc(tmem_at, 512);
+}
+
+// ---------------------------------------------------------------- host side
+// Steps whose sequences bring whole tiles: below about 48 rows a tile the 64-row kernels waste less. Sizes that the tiles and 16-byte
+// stores take, pages of whole 64-key halves.
+bool softmax_takes_tc(const SoftmaxTcArgs& a, int T, int n_tiles) {
+    return T >= 128 && T >= 48 * n_tiles && a.d % 16 == 0 && a.dv % 16 == 0 && a.d <= 128 && a.dv <= 128 && a.block_tokens % 64 == 0 && a.ld_out % 8 == 0 &&
+           ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.out) | reinterpret_cast<uintptr_t>(a.out_bf16)) & 15) == 0;
+}
+
+cudaError_t softmax_tc_launch(const SoftmaxTcArgs& a, const RaggedDev& r, cudaStream_t s) {
+    const int k_parts = (a.d + 63) / 64, v_parts = (a.dv + 63) / 64;
+    static const bool ready = [] {
+        const int most = 12 * SX_PART + 1024;
+        return cudaFuncSetAttribute(softmax_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess &&
+               cudaFuncSetAttribute(softmax_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess;
+    }();
+    if (!ready || !softmax_takes_tc(a, r.T, r.n_tiles)) return cudaErrorInvalidValue;
+    CUtensorMap mk, mv;
+    if (!bf16_rows_map(&mk, a.k_pool, a.d, a.pool_rows, a.d, 1, 0, 64) || !bf16_rows_map(&mv, a.v_pool, a.dv, a.pool_rows, a.dv, 1, 0, 64)) return cudaErrorInvalidValue;
+    const size_t smem = (size_t)(4 * k_parts + 2 * v_parts) * SX_PART + 1024;
+    const dim3 grid(a.H, r.n_tiles), block(SX_THREADS);
+    return a.softcap > 0.f ? launch_chain(softmax_tc_kernel<true>, grid, block, smem, s, mk, mv, a, r, kernel_error_word())
+                           : launch_chain(softmax_tc_kernel<false>, grid, block, smem, s, mk, mv, a, r, kernel_error_word());
+}
+
+}  // namespace b2
