@@ -651,7 +651,10 @@ __device__ __forceinline__ void sk_split_bf16(float a, float b, uint32_t& hi, ui
 }
 }  // namespace
 
-template <int DMAX, int DVMAX, bool CAP>
+// PACK: every sequence of the step brings one token. The rows of a CTA's tile are then the query heads of one key/value head (a row's
+// arithmetic is the same), so a step of 32 sequences with 16 heads over 4 runs 128 CTAs with one busy warp each instead of 512 that
+// multiply 63 rows of nothing beside theirs.
+template <int DMAX, int DVMAX, bool CAP, bool PACK>
 __global__ void __launch_bounds__(128) sink_attn_mma_kernel(SinkAttnArgs a, RaggedDev r) {
     griddep_launch();
     griddep_wait();
@@ -663,13 +666,16 @@ __global__ void __launch_bounds__(128) sink_attn_mma_kernel(SinkAttnArgs a, Ragg
     __nv_bfloat16* Vs = Ks + SKM_K * LD;                                // [64][LDV]
     const int Gv = a.talk ? a.G : 1;
     // late tiles of a segment have the most key blocks: they start first
-    const int tile = gridDim.x - 1 - blockIdx.x, h = blockIdx.y / Gv, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int HG = a.H / a.G;
+    const int tile = gridDim.x - 1 - blockIdx.x, h = PACK ? (int)blockIdx.y * HG : (int)blockIdx.y / Gv, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int seg = r.tile_seg[tile], row0 = r.tile_row0[tile];
     const int nq = min(SKM_Q, r.seg_start[seg] + r.seg_len[seg] - row0);
     const int p0 = r.tok_pos[row0], p_last = p0 + nq - 1;
     const int* table = a.block_tables[r.seg_slot[seg]];
-    const int g = h / (a.H / a.G);
-    const int vg = a.talk ? (int)(blockIdx.y % Gv) : g;
+    const int g = h / HG;
+    const int rows = PACK ? HG : nq;               // rows of the tile: (PACK ? head h + row, the one token : head h, token row)
+    const bool busy = !PACK || warp * 16 < rows;
+    const int vg = !PACK && a.talk ? (int)(blockIdx.y % Gv) : g;
     const __nv_bfloat16* kp = reinterpret_cast<const __nv_bfloat16*>(a.k_pool);
     const __nv_bfloat16* vp = reinterpret_cast<const __nv_bfloat16*>(a.v_pool);
     // scores live in the log2 domain (exp2 below). Capped: cap tanh(s / cap) = cap - 2 cap / (exp(2 s / cap) + 1), the exponential's
@@ -680,7 +686,7 @@ __global__ void __launch_bounds__(128) sink_attn_mma_kernel(SinkAttnArgs a, Ragg
     for (int i = threadIdx.x; i < SKM_Q * (d / 2); i += blockDim.x) {
         const int rr = i / (d / 2), c = (i % (d / 2)) * 2;
         float2 v = make_float2(0.f, 0.f);
-        if (rr < nq) v = *reinterpret_cast<const float2*>(a.q_rot + ((size_t)(row0 + rr) * a.H + h) * d + c);
+        if (rr < rows) v = *reinterpret_cast<const float2*>(a.q_rot + (PACK ? (size_t)row0 * a.H + h + rr : (size_t)(row0 + rr) * a.H + h) * d + c);
         v.x *= q_mul; v.y *= q_mul;
         const __nv_bfloat162 hi = __floats2bfloat162_rn(v.x, v.y);
         *reinterpret_cast<__nv_bfloat162*>(Qs + rr * LD + c) = hi;
@@ -695,12 +701,13 @@ __global__ void __launch_bounds__(128) sink_attn_mma_kernel(SinkAttnArgs a, Ragg
     const int qrow[2] = {warp * 16 + gq, warp * 16 + gq + 8};
     int qlo[2];                                    // oldest visible key of the lane's two query rows
     float m_run[2], l_run[2];
-    const float sink = a.sink ? a.sink[h] * LOG2E : -INFINITY;
+    float sink[2];
 #pragma unroll
     for (int q2 = 0; q2 < 2; q2++) {
-        const int i = p0 + qrow[q2];
+        const int i = PACK ? p0 : p0 + qrow[q2];
+        sink[q2] = a.sink ? a.sink[PACK ? min(h + qrow[q2], a.H - 1) : h] * LOG2E : -INFINITY;
         qlo[q2] = a.window > 0 ? max(0, i - a.window + 1) : 0;
-        m_run[q2] = sink; l_run[q2] = 0.f;         // the running maximum starts at the sink; its term joins the sum at the end
+        m_run[q2] = sink[q2]; l_run[q2] = 0.f;         // the running maximum starts at the sink; its term joins the sum at the end
     }
     // the next block's keys arrive while this block's weights meet the values, its values while the next scores are formed
     // (the thread's chunks of 16 bytes advance through the block without divisions; pages that hold whole blocks are looked up once)
@@ -731,7 +738,7 @@ __global__ void __launch_bounds__(128) sink_attn_mma_kernel(SinkAttnArgs a, Ragg
         for (int ni = 0; ni < SKM_K / 8; ni++) sacc[ni][0] = sacc[ni][1] = sacc[ni][2] = sacc[ni][3] = 0.f;
 #pragma unroll
         for (int ks = 0; ks < DMAX; ks += 16) {
-            if (ks < d) {
+            if (ks < d && busy) {
                 uint32_t af[4], al[4];
                 sk_ldsm_x4(af, Qs + (warp * 16 + (lane & 15)) * LD + ks + (lane >> 4) * 8);
                 sk_ldsm_x4(al, Ql + (warp * 16 + (lane & 15)) * LD + ks + (lane >> 4) * 8);
@@ -757,15 +764,15 @@ __global__ void __launch_bounds__(128) sink_attn_mma_kernel(SinkAttnArgs a, Ragg
 #pragma unroll
                 for (int e = 0; e < 4; e++) sacc[ni][e] = fmaf(-2.f * cap2, sk_rcp(sk_exp2(sacc[ni][e]) + 1.f), cap2);
         // the warp's rows all see the whole block: from its last key on, and not beyond the oldest key of its last row
-        const int w_first = p0 + warp * 16, w_last = w_first + 15;
-        const bool all = warp * 16 + 15 < nq && j0 + SKM_K - 1 <= w_first && (a.window <= 0 || j0 > w_last - a.window);
+        const int w_first = PACK ? p0 : p0 + warp * 16, w_last = PACK ? p0 : w_first + 15;
+        const bool all = warp * 16 + 15 < rows && j0 + SKM_K - 1 <= w_first && (a.window <= 0 || j0 > w_last - a.window);
         if (!all)
 #pragma unroll
             for (int ni = 0; ni < SKM_K / 8; ni++)
 #pragma unroll
                 for (int e = 0; e < 4; e++) {
-                    const int rr = qrow[e >> 1], i = p0 + rr, j = j0 + ni * 8 + 2 * tq + (e & 1);
-                    const bool vis = rr < nq && j <= i && j >= qlo[e >> 1];
+                    const int rr = qrow[e >> 1], i = PACK ? p0 : p0 + rr, j = j0 + ni * 8 + 2 * tq + (e & 1);
+                    const bool vis = rr < rows && j <= i && j >= qlo[e >> 1];
                     sacc[ni][e] = vis ? sacc[ni][e] : -INFINITY;
                 }
 #pragma unroll
@@ -808,7 +815,7 @@ __global__ void __launch_bounds__(128) sink_attn_mma_kernel(SinkAttnArgs a, Ragg
             sk_split_bf16(sacc[2 * kc + 1][2], sacc[2 * kc + 1][3], pf[3], pl[3]);
 #pragma unroll
             for (int nd = 0; nd < DVMAX / 16; nd++) {
-                if (nd * 16 < dv) {
+                if (nd * 16 < dv && busy) {
                     uint32_t vf[4];
                     sk_ldsm_x4_t(vf, Vs + (kc * 16 + (lane & 15)) * LDV + nd * 16 + (lane >> 4) * 8);
                     sk_mma_16816(o[2 * nd], pl, vf[0], vf[1]);
@@ -824,7 +831,7 @@ __global__ void __launch_bounds__(128) sink_attn_mma_kernel(SinkAttnArgs a, Ragg
     float inv[2];
 #pragma unroll
     for (int q2 = 0; q2 < 2; q2++) {
-        const float l = l_run[q2] + (a.sink ? sk_exp2(sink - m_run[q2]) : 0.f);
+        const float l = l_run[q2] + (a.sink ? sk_exp2(sink[q2] - m_run[q2]) : 0.f);
         inv[q2] = l > 0.f ? 1.f / l : 0.f;
     }
 #pragma unroll
@@ -832,18 +839,18 @@ __global__ void __launch_bounds__(128) sink_attn_mma_kernel(SinkAttnArgs a, Ragg
 #pragma unroll
         for (int e = 0; e < 4; e++) {
             const int rr = qrow[e >> 1], c = i * 8 + 2 * tq + (e & 1);
-            if (rr >= nq || c >= dv) continue;
+            if (rr >= rows || c >= dv) continue;
             const float v = o[i][e] * inv[e >> 1];
-            const int t = row0 + rr;
+            const int t = PACK ? row0 : row0 + rr, ho = PACK ? h + rr : h;
             if (a.out_bf16) {                  // two neighbouring columns of a row (dv is even)
                 if (e & 1) continue;
                 const float v2 = o[i][e + 1] * inv[e >> 1];
-                *reinterpret_cast<__nv_bfloat162*>(a.out_bf16 + (size_t)t * a.ld_out + (size_t)h * dv + c) =
-                    __floats2bfloat162_rn(v * sk_gate(a, t, h, c), v2 * sk_gate(a, t, h, c + 1));
+                *reinterpret_cast<__nv_bfloat162*>(a.out_bf16 + (size_t)t * a.ld_out + (size_t)ho * dv + c) =
+                    __floats2bfloat162_rn(v * sk_gate(a, t, ho, c), v2 * sk_gate(a, t, ho, c + 1));
                 continue;
             }
-            if (a.talk) a.cross[(((size_t)t * a.H + h) * a.G + vg) * dv + c] = v;
-            else a.out[(size_t)t * a.ld_out + (size_t)h * dv + c] = v * sk_gate(a, t, h, c);
+            if (!PACK && a.talk) a.cross[(((size_t)t * a.H + h) * a.G + vg) * dv + c] = v;
+            else a.out[(size_t)t * a.ld_out + (size_t)ho * dv + c] = v * sk_gate(a, t, ho, c);
         }
 }
 
@@ -1127,10 +1134,13 @@ static cudaError_t sink_attn_mma_pick(const SinkAttnArgs& a, const RaggedDev& r,
     const size_t smem = (size_t)(3 * 64 * (a.d + 8) + 64 * (a.dv + 8)) * 2;
     static bool attr_done = false;
     if (!attr_done) {
-        cudaFuncSetAttribute(sink_attn_mma_kernel<DMAX, DVMAX, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (3 * 64 * (DMAX + 8) + 64 * (DVMAX + 8)) * 2);
+        const int most = (3 * 64 * (DMAX + 8) + 64 * (DVMAX + 8)) * 2;
+        cudaFuncSetAttribute(sink_attn_mma_kernel<DMAX, DVMAX, CAP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        cudaFuncSetAttribute(sink_attn_mma_kernel<DMAX, DVMAX, CAP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
         attr_done = true;
     }
-    return launch_chain(sink_attn_mma_kernel<DMAX, DVMAX, CAP>, dim3(r.n_tiles, a.H * (a.talk ? a.G : 1)), dim3(128), smem, s, a, r);
+    if (!a.talk && r.T == r.n_seg && a.H / a.G <= SKM_Q) return launch_chain(sink_attn_mma_kernel<DMAX, DVMAX, CAP, true>, dim3(r.n_tiles, a.G), dim3(128), smem, s, a, r);
+    return launch_chain(sink_attn_mma_kernel<DMAX, DVMAX, CAP, false>, dim3(r.n_tiles, a.H * (a.talk ? a.G : 1)), dim3(128), smem, s, a, r);
 }
 
 template <bool CAP>
