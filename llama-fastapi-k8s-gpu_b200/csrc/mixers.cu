@@ -864,9 +864,38 @@ __global__ void __launch_bounds__(SC_CH * 4) scan_recurrence_lanes_kernel(ScanAr
         const int nxt = buf == 0 ? 2 : buf - 1;
         if (i0 + 2 * SC_TB < len) stage(i0 + 2 * SC_TB, nxt);        // everybody has left that buffer
         cp_async_commit();
-        float keep = 0.f;
-#pragma unroll 4
-        for (int u = 0; u < nb; u++) {
+        // four tokens at a time: their exponentials do not wait for one another, and the sums over the lanes cost three shuffles for the
+        // four, each lane ending up with the token it stores
+        int u = 0;
+        for (; u + 4 <= nb; u += 4) {
+            float part[4], xu[4];
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                const float dt = in[buf][0][u + t][lc], xv = in[buf][1][u + t][lc];
+                xu[t] = xv;
+                const float* Bp = &bc[buf][0][u + t][q * SPL];
+                const float* Cp = &bc[buf][1][u + t][q * SPL];
+                float p[SPL];
+#pragma unroll
+                for (int j = 0; j < SPL; j++) {
+                    S[j] = expf(dt * A[j]) * S[j] + dt * xv * Bp[j];
+                    p[j] = __fmul_rn(S[j], Cp[j]);
+                }
+#pragma unroll
+                for (int w = SPL / 2; w > 0; w >>= 1)
+#pragma unroll
+                    for (int j = 0; j < w; j++) p[j] += p[j + w];
+                part[t] = p[0];
+            }
+            // lane q keeps token q: first halves two lanes apart (lanes 0, 1 keep tokens 0, 1), then neighbours
+            const bool up = q & 2, odd = q & 1;
+            const float s0 = (up ? part[2] : part[0]) + __shfl_xor_sync(0xffffffffu, up ? part[0] : part[2], 2);
+            const float s1 = (up ? part[3] : part[1]) + __shfl_xor_sync(0xffffffffu, up ? part[1] : part[3], 2);
+            const float sum = (odd ? s1 : s0) + __shfl_xor_sync(0xffffffffu, odd ? s0 : s1, 1);
+            const float xq = up ? (odd ? xu[3] : xu[2]) : (odd ? xu[1] : xu[0]);
+            if (c_ok) a.y[(size_t)(start + i0 + u + q) * a.inner + c] = (sum + Dc * xq) * in[buf][2][u + q][lc];
+        }
+        for (; u < nb; u++) {
             const float dt = in[buf][0][u][lc], xv = in[buf][1][u][lc], gate = in[buf][2][u][lc];
             const float* Bp = &bc[buf][0][u][q * SPL];
             const float* Cp = &bc[buf][1][u][q * SPL];
@@ -883,12 +912,7 @@ __global__ void __launch_bounds__(SC_CH * 4) scan_recurrence_lanes_kernel(ScanAr
             float sum = p[0];
             sum += __shfl_xor_sync(0xffffffffu, sum, 2);
             sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-            const float yv = (sum + Dc * xv) * gate;
-            if ((u & 3) == q) keep = yv;                             // lane q stores every fourth token
-            if ((u & 3) == 3 || u == nb - 1) {
-                const int mine = (u & ~3) + q;
-                if (c_ok && mine < nb) a.y[(size_t)(start + i0 + mine) * a.inner + c] = keep;
-            }
+            if (q == 0 && c_ok) a.y[(size_t)(start + i0 + u) * a.inner + c] = (sum + Dc * xv) * gate;
         }
         buf = buf == 2 ? 0 : buf + 1;
     }
@@ -960,15 +984,16 @@ __global__ void __launch_bounds__(MG_TB) matrix_mem_gates_kernel(MatrixMemArgs a
     if (threadIdx.x == 0) a.m[(size_t)slot * a.H + h] = ms[0];
 }
 
-// grid (n_seg, H, ceil(dv / 32) + 1): a CTA owns 32 columns of one head's d x dv memory. Thread (col, grp) keeps rows grp * MM_ROWS ..
-// of its column in registers. Tokens go in blocks of MM_TB: a thread's state update for token t + 1 needs only its own registers
+// grid (n_seg, H, ceil(dv / 32) + 1): a CTA owns 32 columns of one head's d x dv memory. Thread (pair, grp) keeps rows grp * MM_ROWS ..
+// of two neighbouring columns in registers: a 16-byte read of k or q out of shared memory occupies its pipe for four cycles even when all
+// lanes want the same bytes, so with one column a thread the reads (8 a token and warp, 8 warps) bounded the kernel. Tokens go in blocks of MM_TB: a thread's state update for token t + 1 needs only its own registers
 // after token t, so the block barrier is paid once per block -- for the inputs (q, k, v and the two factors of the next block arrive
 // in shared memory as asynchronous copies while this block is computed) and for the partial read-outs per row group, which all
 // threads then sum in a fixed order, one (token, column) each. The CTA past the last columns carries the normaliser n (a lane per
 // row) and leaves n . q; the division by it waits for matrix_mem_out_kernel.
-// Bound by issue slots: 48 operations on the memory and 8 shared loads per token and warp.
-constexpr int MM_ROWS = 16, MM_COLS = 32, MM_TB = 16;      // key size <= 16 * 16 = 256 (512 threads)
-__global__ void __launch_bounds__(512) matrix_mem_kernel(MatrixMemArgs a, RaggedDev r, int RG) {
+// Bound by issue slots: 96 operations on the memory and 8 shared loads per token and warp.
+constexpr int MM_ROWS = 16, MM_COLS = 32, MM_TB = 16;      // key size <= 16 * 16 = 256 (256 threads)
+__global__ void __launch_bounds__(256) matrix_mem_kernel(MatrixMemArgs a, RaggedDev r, int RG) {
     griddep_launch();
     griddep_wait();
     extern __shared__ float sm[];
@@ -982,30 +1007,38 @@ __global__ void __launch_bounds__(512) matrix_mem_kernel(MatrixMemArgs a, Ragged
     const bool norm_cta = blockIdx.z == gridDim.z - 1;
     const int seg = blockIdx.x, h = blockIdx.y, c0 = norm_cta ? 0 : blockIdx.z * MM_COLS, n_cols = norm_cta ? 0 : min(MM_COLS, dv - c0);
     const int slot = r.seg_slot[seg], start = r.seg_start[seg], len = r.seg_len[seg];
-    const int lc = threadIdx.x % MM_COLS, grp = threadIdx.x / MM_COLS;
+    const int lp = threadIdx.x % 16, grp = threadIdx.x / 16;      // column pair, row group
     const bool act = grp < RG;                     // threads past the last row group only help with copies and sums
-    const bool mem = act && lc < n_cols;
-    float* Sg = a.S + (((size_t)slot * a.H + h) * d) * dv + c0 + lc;
+    const bool mem0 = act && 2 * lp < n_cols, mem1 = act && 2 * lp + 1 < n_cols;
+    float* Sg = a.S + (((size_t)slot * a.H + h) * d) * dv + c0 + 2 * lp;
     float* ng = a.n + ((size_t)slot * a.H + h) * d;
-    float S[MM_ROWS];
+    float S0[MM_ROWS], S1[MM_ROWS];
 #pragma unroll
     for (int i = 0; i < MM_ROWS; i++) {
         const int row = grp * MM_ROWS + i;
-        S[i] = (mem && row < d) ? Sg[(size_t)row * dv] : 0.f;
+        S0[i] = (mem0 && row < d) ? Sg[(size_t)row * dv] : 0.f;
+        S1[i] = (mem1 && row < d) ? Sg[(size_t)row * dv + 1] : 0.f;
     }
-    const int nrow = grp * MM_ROWS + lc;                      // lanes 0 .. MM_ROWS-1 of a warp: one row of n each
-    const bool n_ok = norm_cta && act && lc < MM_ROWS && nrow < d;
+    const int nrow = grp * MM_ROWS + lp;                      // a lane per row of n
+    const bool n_ok = norm_cta && act && nrow < d;
     float nr = n_ok ? ng[nrow] : 0.f;
     const bool vec4 = (d % 4) == 0;
     const float qscale = 1.f / sqrtf((float)d);
+    // q and k rows as 16-byte copies where they start on 16 bytes
+    const bool wide = d % 4 == 0 && a.ldp % 4 == 0 && a.q_off % 4 == 0 && a.k_off % 4 == 0 && (reinterpret_cast<uintptr_t>(a.proj) & 15) == 0;
+    const int per = wide ? d / 4 : d, piece = wide ? 4 : 1;
+    const int f_e = (threadIdx.x % per) * piece, f_u = threadIdx.x / per, f_du = blockDim.x / per;      // (only when per divides the CTA)
+    const bool even = blockDim.x % per == 0;
     auto stage = [&](int i0, int buf) {                  // tokens i0 .. of the segment into buffer `buf`
         const int nb = min(MM_TB, len - i0);
-        for (int j = threadIdx.x; j < nb * d; j += blockDim.x) {
-            const int u = j / d, e = j % d;
-            const float* p = a.proj + (size_t)(start + i0 + u) * a.ldp;
-            cp_async_4(&qs[(buf * MM_TB + u) * d + e], p + a.q_off + h * d + e);
-            cp_async_4(&ks[(buf * MM_TB + u) * d + e], p + a.k_off + h * d + e);
-        }
+        auto copy = [&](int u, int e) {
+            const float* p = a.proj + (size_t)(start + i0 + u) * a.ldp + h * d + e;
+            float *qd = &qs[(buf * MM_TB + u) * d + e], *kd = &ks[(buf * MM_TB + u) * d + e];
+            if (wide) { cp_async_16z(qd, p + a.q_off, 16); cp_async_16z(kd, p + a.k_off, 16); }
+            else { cp_async_4(qd, p + a.q_off); cp_async_4(kd, p + a.k_off); }
+        };
+        if (even) for (int u = f_u; u < nb; u += f_du) copy(u, f_e);
+        else for (int j = threadIdx.x; j < nb * per; j += blockDim.x) copy(j / per, (j % per) * piece);
         for (int j = threadIdx.x; j < nb * MM_COLS; j += blockDim.x) {
             const int u = j / MM_COLS, e = j % MM_COLS;
             const float* p = a.proj + (size_t)(start + i0 + u) * a.ldp;
@@ -1016,7 +1049,7 @@ __global__ void __launch_bounds__(512) matrix_mem_kernel(MatrixMemArgs a, Ragged
     auto finish = [&](int i0, int buf) {                 // sum of the row groups in a fixed order
         const int nb = min(MM_TB, len - i0), cols = norm_cta ? 1 : MM_COLS;
         for (int j = threadIdx.x; j < nb * cols; j += blockDim.x) {
-            const int u = j / cols, e = j % cols;
+            const int u = norm_cta ? j : j / MM_COLS, e = norm_cta ? 0 : j % MM_COLS;
             if (!norm_cta && e >= n_cols) continue;
             const float* rd = red + (size_t)(buf * MM_TB + u) * red_tok;
             float sum = 0.f;
@@ -1037,6 +1070,7 @@ __global__ void __launch_bounds__(512) matrix_mem_kernel(MatrixMemArgs a, Ragged
         cp_async_commit();
         if (i0 > 0) finish(i0 - MM_TB, buf ^ 1);
         if (norm_cta) {
+#pragma unroll 4
             for (int u = 0; u < nb; u++) {
                 const int bu = buf * MM_TB + u;
                 const float ib = gs[bu * 2], da = gs[bu * 2 + 1];
@@ -1044,33 +1078,38 @@ __global__ void __launch_bounds__(512) matrix_mem_kernel(MatrixMemArgs a, Ragged
                 if (n_ok) { nr = fmaf(da, nr, ib * ks[bu * d + nrow]); npart = nr * qs[bu * d + nrow]; }
 #pragma unroll
                 for (int o = MM_ROWS / 2; o > 0; o >>= 1) npart += __shfl_xor_sync(0xffffffffu, npart, o);
-                if (act && lc == 0) red[(size_t)bu * red_tok + grp * MM_COLS] = npart * qscale;
+                if (act && lp == 0) red[(size_t)bu * red_tok + grp * MM_COLS] = npart * qscale;
             }
         } else if (act) {
             const bool full = vec4 && grp * MM_ROWS + MM_ROWS <= d;
 #pragma unroll 2
             for (int u = 0; u < nb; u++) {
                 const int bu = buf * MM_TB + u;
-                const float2 g2 = *reinterpret_cast<const float2*>(gs + bu * 2);
-                const float da = g2.y, vb = g2.x * vs[bu * MM_COLS + lc];
-                float part = 0.f;
+                const float2 g2 = *reinterpret_cast<const float2*>(gs + bu * 2), v2 = *reinterpret_cast<const float2*>(vs + bu * MM_COLS + 2 * lp);
+                const float da = g2.y, v0 = g2.x * v2.x, v1 = g2.x * v2.y;
+                float p0 = 0.f, p1 = 0.f;
                 const float* kr = ks + bu * d + grp * MM_ROWS;
                 const float* qr = qs + bu * d + grp * MM_ROWS;
                 if (full) {
 #pragma unroll
                     for (int k4 = 0; k4 < MM_ROWS; k4 += 4) {
-                        const float4 k4v = *reinterpret_cast<const float4*>(kr + k4), q4v = *reinterpret_cast<const float4*>(qr + k4);
-                        S[k4 + 0] = fmaf(da, S[k4 + 0], k4v.x * vb); part = fmaf(S[k4 + 0], q4v.x, part);
-                        S[k4 + 1] = fmaf(da, S[k4 + 1], k4v.y * vb); part = fmaf(S[k4 + 1], q4v.y, part);
-                        S[k4 + 2] = fmaf(da, S[k4 + 2], k4v.z * vb); part = fmaf(S[k4 + 2], q4v.z, part);
-                        S[k4 + 3] = fmaf(da, S[k4 + 3], k4v.w * vb); part = fmaf(S[k4 + 3], q4v.w, part);
+                        const float4 kv = *reinterpret_cast<const float4*>(kr + k4), qv = *reinterpret_cast<const float4*>(qr + k4);
+                        const float kk[4] = {kv.x, kv.y, kv.z, kv.w}, qq[4] = {qv.x, qv.y, qv.z, qv.w};
+#pragma unroll
+                        for (int i = 0; i < 4; i++) {
+                            S0[k4 + i] = fmaf(da, S0[k4 + i], kk[i] * v0); p0 = fmaf(S0[k4 + i], qq[i], p0);
+                            S1[k4 + i] = fmaf(da, S1[k4 + i], kk[i] * v1); p1 = fmaf(S1[k4 + i], qq[i], p1);
+                        }
                     }
                 } else {
 #pragma unroll
                     for (int k = 0; k < MM_ROWS; k++)
-                        if (grp * MM_ROWS + k < d) { S[k] = fmaf(da, S[k], kr[k] * vb); part = fmaf(S[k], qr[k], part); }
+                        if (grp * MM_ROWS + k < d) {
+                            S0[k] = fmaf(da, S0[k], kr[k] * v0); p0 = fmaf(S0[k], qr[k], p0);
+                            S1[k] = fmaf(da, S1[k], kr[k] * v1); p1 = fmaf(S1[k], qr[k], p1);
+                        }
                 }
-                red[(size_t)bu * red_tok + grp * MM_COLS + lc] = part * qscale;
+                *reinterpret_cast<float2*>(red + (size_t)bu * red_tok + grp * MM_COLS + 2 * lp) = make_float2(p0 * qscale, p1 * qscale);
             }
         }
     }
@@ -1079,7 +1118,8 @@ __global__ void __launch_bounds__(512) matrix_mem_kernel(MatrixMemArgs a, Ragged
 #pragma unroll
     for (int i = 0; i < MM_ROWS; i++) {
         const int row = grp * MM_ROWS + i;
-        if (mem && row < d) Sg[(size_t)row * dv] = S[i];
+        if (mem0 && row < d) Sg[(size_t)row * dv] = S0[i];
+        if (mem1 && row < d) Sg[(size_t)row * dv + 1] = S1[i];
     }
     if (n_ok) ng[nrow] = nr;
 }
@@ -1111,7 +1151,7 @@ cudaError_t matrix_mem_launch(const MatrixMemArgs& a, const RaggedDev& r, cudaSt
     if (ce != cudaSuccess) return ce;
     {
         PlainLaunch pl;    // latency-bound over the prompt: CTAs spread over all SMs (see kernels.h)
-        ce = launch_chain(matrix_mem_kernel, dim3(r.n_seg, a.H, (a.dv + MM_COLS - 1) / MM_COLS + 1), dim3(std::max(RG * MM_COLS, 64)), smem, s, a, r, RG);
+        ce = launch_chain(matrix_mem_kernel, dim3(r.n_seg, a.H, (a.dv + MM_COLS - 1) / MM_COLS + 1), dim3(std::max((RG * 16 + 31) / 32 * 32, 64)), smem, s, a, r, RG);
     }
     if (ce != cudaSuccess) return ce;
     return launch_chain(matrix_mem_out_kernel, dim3(r.T, a.H), dim3(128), 0, s, a);
