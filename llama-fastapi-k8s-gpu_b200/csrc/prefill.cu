@@ -31,7 +31,7 @@ __global__ void embed_rows_kernel(int type, const uint8_t* table, int K, const i
         x[(size_t)t * K + i] = dequant_elem(type, row + (size_t)(i / be) * bb, i % be);
 }
 cudaError_t embed_rows_launch(int type, const uint8_t* table, int K, const int* tokens, int T, float* x, cudaStream_t s) {
-    return launch_chain(embed_rows_kernel, dim3(T), dim3(256), 0, s, type, table, K, tokens, x);
+    return launch_chain(embed_rows_kernel, dim3(T), dim3(T > 148 ? 256 : 1024), 0, s, type, table, K, tokens, x);
 }
 
 __device__ __forceinline__ size_t op_index(int t, int k, int T_pad) { return ((size_t)(k >> 3) * T_pad + t) * 8 + (k & 7); }
@@ -180,7 +180,7 @@ __global__ void embed_batch_kernel(int type, const uint8_t* table, int K, const 
         x[(size_t)t * K + i] = dequant_elem(type, row + (size_t)(i / be) * bb, i % be);
 }
 cudaError_t embed_batch_launch(int type, const uint8_t* table, int K, const SlotDev* tab, const BatchIdx& b, float* x, cudaStream_t s) {
-    return launch_chain(embed_batch_kernel, dim3(b.n), dim3(256), 0, s, type, table, K, tab, b, x);
+    return launch_chain(embed_batch_kernel, dim3(b.n), dim3(1024), 0, s, type, table, K, tab, b, x);
 }
 
 // like rope_store, but row t belongs to slot b.slot[t] at that slot's own position; q stays float32 for flash-decode
@@ -230,14 +230,18 @@ cudaError_t rope_store_batch_launch(const float* parts, int n_parts, long part_s
 __global__ void prefill_finish_kernel(const int* prompt, int n, int pos_last, int* ints, SamplerState* st) {
     griddep_launch();
     griddep_wait();
-    int nh = st->n_hist;
-    for (int i = 0; i < n; i++) { st->history[nh & (HISTORY_LEN - 1)] = prompt[i]; nh++; }
-    st->n_hist = nh;
-    ints[0] = prompt[n - 1];
-    ints[1] = pos_last;
+    // only the last HISTORY_LEN tokens stay in the ring: one thread each (one thread walking 512 tokens took 27 us)
+    const int nh = st->n_hist, i = n - HISTORY_LEN + (int)threadIdx.x;
+    if (i >= 0) st->history[(nh + i) & (HISTORY_LEN - 1)] = prompt[i];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        st->n_hist = nh + n;
+        ints[0] = prompt[n - 1];
+        ints[1] = pos_last;
+    }
 }
 cudaError_t prefill_finish_launch(const int* prompt, int n, int pos_last, int* ints, SamplerState* st, cudaStream_t s) {
-    return launch_chain(prefill_finish_kernel, dim3(1), dim3(1), 0, s, prompt, n, pos_last, ints, st);
+    return launch_chain(prefill_finish_kernel, dim3(1), dim3(HISTORY_LEN), 0, s, prompt, n, pos_last, ints, st);
 }
 
 // ---------------------------------------------------------------- causal attention for T queries
