@@ -26,8 +26,6 @@ __device__ __forceinline__ float ld_w(const float* w, size_t i) { return w[i]; }
 // tokens the activation loads, not the weights, fill the load pipe). Fast path (K % 8 == 0, 16-byte aligned rows): a lane takes
 // 8 consecutive weights per load and keeps R x U = 4 loads in flight, 2 KB per warp on the wire. Each output is still one sum
 // over k in an order that depends on K alone.
-// A step of few tokens is a chain of small products, each a few microseconds of weights: a plain product requests its first PRE chunks of
-// weights before it waits for the previous kernel (they do not depend on it), so the stream does not stop between two links.
 constexpr int ROWS_MAX_T = 8;
 template <typename TW, int TT, int R>
 __device__ __forceinline__ void dense_rows_cta(const DenseDev& a, unsigned bx, unsigned by, unsigned bz) {
@@ -37,7 +35,6 @@ __device__ __forceinline__ void dense_rows_cta(const DenseDev& a, unsigned bx, u
     const int n0 = (bx * 8 + warp) * R;
     if (n0 >= N) return;
     const float* x; const TW* w; float* y; const float* aux; int t0, t1;
-    if (a.grouped) griddep_wait();                // which matrix a row takes comes from an earlier kernel
     if (!dense_tile<TW>(a, ROWS_MAX_T, x, w, y, aux, t0, t1, by, bz)) return;
     const int T = a.grouped ? 1 : a.T;
     const float* rs = a.g.row_scale;
@@ -51,39 +48,18 @@ __device__ __forceinline__ void dense_rows_cta(const DenseDev& a, unsigned bx, u
 #pragma unroll
         for (int r = 0; r < R; r++) acc[t][r] = 0.f;
     const bool vec = (K % 8 == 0) && (ldx % 4 == 0) && ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(x)) & 15) == 0;
-    constexpr int PRE = (sizeof(TW) == 2 ? 8 : 4) / R > 0 ? (sizeof(TW) == 2 ? 8 : 4) / R : 1;
-    struct Raw { uint4 v[sizeof(TW) / 2]; };      // 8 weights
-    auto fetch8 = [&](const TW* row, int k) {     // streamed once: do not keep in L1
-        Raw raw;
-#pragma unroll
-        for (int i = 0; i < (int)(sizeof(TW) / 2); i++) raw.v[i] = __ldcs(reinterpret_cast<const uint4*>(row + k) + i);
-        return raw;
-    };
-    Raw pre[PRE][R];
-    if (!a.grouped) {
-        if (vec) {
-#pragma unroll
-            for (int u = 0; u < PRE; u++)
-#pragma unroll
-                for (int r = 0; r < R; r++) if (lane * 8 + u * 256 < K) pre[u][r] = fetch8(rows[r], lane * 8 + u * 256);
-        }
-        griddep_wait();
-    }
     if (vec) {
-        auto widen8 = [&](const Raw& raw, float (&wv)[8]) {
+        auto load8 = [&](const TW* row, int k, float (&wv)[8]) {
             if constexpr (sizeof(TW) == 2) {
-                const uint32_t u[4] = {raw.v[0].x, raw.v[0].y, raw.v[0].z, raw.v[0].w};
+                const uint4 raw = __ldcs(reinterpret_cast<const uint4*>(row + k));       // streamed once: do not keep in L1
+                const uint32_t u[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
                 for (int i = 0; i < 4; i++) { wv[2 * i] = __uint_as_float(u[i] << 16); wv[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u); }
             } else {
-#pragma unroll
-                for (int i = 0; i < 2; i++) {
-                    wv[4 * i] = __uint_as_float(raw.v[i].x); wv[4 * i + 1] = __uint_as_float(raw.v[i].y);
-                    wv[4 * i + 2] = __uint_as_float(raw.v[i].z); wv[4 * i + 3] = __uint_as_float(raw.v[i].w);
-                }
+                const float4 a = __ldcs(reinterpret_cast<const float4*>(row + k)), b = __ldcs(reinterpret_cast<const float4*>(row + k + 4));
+                wv[0] = a.x; wv[1] = a.y; wv[2] = a.z; wv[3] = a.w; wv[4] = b.x; wv[5] = b.y; wv[6] = b.z; wv[7] = b.w;
             }
         };
-        auto load8 = [&](const TW* row, int k, float (&wv)[8]) { widen8(fetch8(row, k), wv); };
         auto fma8 = [&](const float (&wv)[R][8], int k) {
 #pragma unroll
             for (int t = 0; t < TT; t++)
@@ -100,17 +76,6 @@ __device__ __forceinline__ void dense_rows_cta(const DenseDev& a, unsigned bx, u
                 }
         };
         int k = lane * 8;
-        if (!a.grouped) {
-#pragma unroll
-            for (int u = 0; u < PRE; u++)
-                if (k + u * 256 < K) {
-                    float wv[R][8];
-#pragma unroll
-                    for (int r = 0; r < R; r++) widen8(pre[u][r], wv[r]);
-                    fma8(wv, k + u * 256);
-                }
-            k += PRE * 256;
-        }
         for (; k + (U - 1) * 256 < K; k += U * 256) {
             float wv[U][R][8];
 #pragma unroll
@@ -156,12 +121,14 @@ __device__ __forceinline__ void dense_rows_cta(const DenseDev& a, unsigned bx, u
 template <typename TW, int TT, int R>
 __global__ void __launch_bounds__(256) dense_rows_kernel(DenseDev a) {
     griddep_launch();
+    griddep_wait();
     dense_rows_cta<TW, TT, R>(a, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 // two independent products in one launch: the CTAs of a, then those of b (grouped pairs, `nb` CTAs each)
 template <typename TW, int TT, int R>
 __global__ void __launch_bounds__(256) dense_rows_pair_kernel(DenseDev a, DenseDev b, unsigned na, unsigned nb) {
     griddep_launch();
+    griddep_wait();
     if (blockIdx.x < na) dense_rows_cta<TW, TT, R>(a, blockIdx.x, 0, 0);
     else dense_rows_cta<TW, 1, 1>(b, (blockIdx.x - na) % nb, (blockIdx.x - na) / nb, 0);
 }
