@@ -186,13 +186,9 @@ cudaError_t resid_norm_half_launch(float* x, const float* parts, int n_parts, lo
 cudaError_t rope_store_launch(const float* parts, int n_parts, long part_stride, int T, int pos0, int n_head, int n_kv, int hd,
                               int bt, const int* block_table, const float* rope_freq, __half* qh, __half* k_cache,
                               __half* v_cache, cudaStream_t s);
-// causal attention of T queries at pos0.. over the paged cache (pool_rows = pages * n_kv * bt rows); out in operand order (T_pad)
-cudaError_t attn_prefill_launch(const __half* qh, const __half* k_cache, const __half* v_cache, long pool_rows, const int* block_table,
+// causal attention of T queries at pos0.. over the paged cache; out in operand order (T_pad)
+cudaError_t attn_prefill_launch(const __half* qh, const __half* k_cache, const __half* v_cache, const int* block_table,
                                 int T, int T_pad, int pos0, int n_head, int n_kv, int hd, int bt, __half* out, cudaStream_t s);
-// the same for prompts of whole tiles (prompt_attn_tc.cu)
-bool prompt_attn_takes_tc(int T, int hd, int bt);
-cudaError_t prompt_attn_tc_launch(const __half* qh, const __half* k_cache, const __half* v_cache, long pool_rows, const int* block_table, int T, int T_pad, int pos0,
-                                  int n_head, int n_kv, int hd, int bt, __half* out, cudaStream_t s);
 // gate|up parts [T][2F] -> h = f16(silu(gate) * up) in operand order
 cudaError_t silu_mul_half_launch(const float* parts, int n_parts, long part_stride, int F, int T, int T_pad, __half* h, cudaStream_t s);
 // batched decode step (one token per slot of b)

@@ -385,12 +385,11 @@ __global__ void __launch_bounds__(256) attn_prefill_kernel(const __half* qh, con
     }
 }
 
-cudaError_t attn_prefill_launch(const __half* qh, const __half* k_cache, const __half* v_cache, long pool_rows, const int* block_table,
+cudaError_t attn_prefill_launch(const __half* qh, const __half* k_cache, const __half* v_cache, const int* block_table,
                                 int T, int T_pad, int pos0, int n_head, int n_kv, int hd, int bt, __half* out, cudaStream_t s) {
     if (n_kv <= 0 || n_head % n_kv) return cudaErrorInvalidValue;
     const int G = n_head / n_kv;
     if (G > 8) return cudaErrorInvalidValue;
-    if (prompt_attn_takes_tc(T, hd, bt)) return prompt_attn_tc_launch(qh, k_cache, v_cache, pool_rows, block_table, T, T_pad, pos0, n_head, n_kv, hd, bt, out, s);
     const int QW = G >= 4 ? 1 : 4 / G;
     const int q_tile = 16 * QW;
     dim3 grid((T + q_tile - 1) / q_tile, n_kv), block(32 * G * QW);
