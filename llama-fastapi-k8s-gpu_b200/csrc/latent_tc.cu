@@ -238,15 +238,15 @@ __global__ void __launch_bounds__(192, 1) latent_attn_tc_kernel(const __grid_con
 
 // ---------------------------------------------------------------- host side
 // Rows of 64-column parts that fit shared memory beside the queries (9 of them), whole chunks of output columns, pages of whole blocks.
-bool latent_attn_takes_tc(const LatentAttnArgs& a, int T) {
+bool latent_attn_takes_tc(const LatentAttnArgs& a, int T, int n_seg) {
     const int parts = (a.rank + a.dr + LC_PART - 1) / LC_PART;
-    return !a.cache_f32 && T >= LATENT_TC_MIN && a.rank % LC_PART == 0 && (a.rank <= LC_V || a.rank % LC_V == 0) && parts <= 9 && a.ld_row % 8 == 0 &&
+    return !a.cache_f32 && T >= LATENT_TC_MIN * n_seg && a.rank % LC_PART == 0 && (a.rank <= LC_V || a.rank % LC_V == 0) && parts <= 9 && a.ld_row % 8 == 0 &&
            a.block_tokens % LC_K == 0;
 }
 
 cudaError_t latent_attn_tc_launch(const LatentAttnArgs& a, const RaggedDev& r, const __nv_bfloat16* q, long pool_rows, __nv_bfloat16* out, cudaStream_t s) {
     static const bool ready = cudaFuncSetAttribute(latent_attn_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 9 * (LC_QPART + LC_KPART) + 1024) == cudaSuccess;
-    if (!ready || !latent_attn_takes_tc(a, r.T)) return cudaErrorInvalidValue;
+    if (!ready || !latent_attn_takes_tc(a, r.T, r.n_seg)) return cudaErrorInvalidValue;
     const int parts = (a.rank + a.dr + LC_PART - 1) / LC_PART, chunks = (a.rank + LC_V - 1) / LC_V;
     CUtensorMap mk, mq;
     // rows of the pages [pages * block_tokens][ld_row]; columns past rank + dr arrive as zeros

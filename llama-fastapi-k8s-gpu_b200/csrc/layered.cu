@@ -1116,7 +1116,7 @@ static int mix_latent_attn(b2_engine* e, LayeredModel* m, LyLayer& L, const Ragg
     if (gate) { v.aux = m->proj + L.g_off; v.ldaux = Np; v.aux_bs = head_gate ? 1 : d.la_vdim; v.aux_one = head_gate; }
     const int v_epi = gate ? EPI_MUL_SIGMOID : EPI_NONE;
     DenseArgs op = {};
-    if (latent_attn_takes_tc(a, T) && dense_takes_rounded(dense_args(m, L.uk_t, q, ldq, m->buf[0], H * Dk, T, nullptr, EPI_NONE, &b)) &&
+    if (latent_attn_takes_tc(a, T, r.n_seg) && dense_takes_rounded(dense_args(m, L.uk_t, q, ldq, m->buf[0], H * Dk, T, nullptr, EPI_NONE, &b)) &&
         dense_takes_rounded(dense_args(m, L.uv, m->buf[1], H * d.la_rank, m->buf[2], H * d.la_vdim, T, nullptr, v_epi, &v)) && takes_rounded(m, L.attn_o, T)) {
         // long steps: what these products and the attention hand on is left rounded
         __nv_bfloat16* qb = reinterpret_cast<__nv_bfloat16*>(m->buf[1]);

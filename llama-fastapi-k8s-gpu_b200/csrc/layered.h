@@ -259,8 +259,8 @@ cudaError_t latent_attn_launch(const LatentAttnArgs& a, const RaggedDev& r, cuda
 
 // Long steps over bf16 pages (latent_tc.cu): queries q [T][H][rank] are the folded ones, scaled and rounded (their rotated parts come
 // from a.q_raw or a.qv); the weighted latents go to `out` [T][H][rank], rounded. pool_rows: rows of the pages in all.
-constexpr int LATENT_TC_MIN = 128;
-bool latent_attn_takes_tc(const LatentAttnArgs& a, int T);
+constexpr int LATENT_TC_MIN = 256;             // tokens per sequence of the step, on average: two tiles of 128 queries
+bool latent_attn_takes_tc(const LatentAttnArgs& a, int T, int n_seg);
 cudaError_t latent_attn_tc_launch(const LatentAttnArgs& a, const RaggedDev& r, const __nv_bfloat16* q, long pool_rows, __nv_bfloat16* out, cudaStream_t s);
 
 // ---------------------------------------------------------------- mixture of experts (moe.cu)

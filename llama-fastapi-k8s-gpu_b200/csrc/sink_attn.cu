@@ -1168,7 +1168,7 @@ cudaError_t sink_attn_launch(const SinkAttnArgs& a, const RaggedDev& r, cudaStre
         x.q = a.q_rot; x.k_pool = a.k_pool; x.v_pool = a.v_pool; x.pool_rows = a.pool_rows; x.block_tables = a.block_tables; x.block_tokens = a.block_tokens;
         x.H = a.H; x.G = a.G; x.d = a.d; x.dv = a.dv; x.window = a.window; x.scale = a.scale; x.softcap = a.softcap; x.sink = a.sink;
         x.gate = a.gate; x.ld_gate = a.ld_gate; x.gate_per_head = a.gate_per_head; x.out = a.out; x.out_bf16 = a.out_bf16; x.ld_out = a.ld_out;
-        if (!a.talk && softmax_takes_tc(x, r.T, r.n_tiles)) return softmax_tc_launch(x, r, s);
+        if (!a.talk && softmax_takes_tc(x, r.T, r.n_seg)) return softmax_tc_launch(x, r, s);
         e = a.softcap > 0.f ? sink_attn_mma_sizes<true>(a, r, s) : sink_attn_mma_sizes<false>(a, r, s);
     } else if (!a.talk && a.d % 8 == 0 && a.dv % 8 == 0) {
         return a.cache_f32 ? sink_attn_vec_launch<true>(a, r, s) : sink_attn_vec_launch<false>(a, r, s);

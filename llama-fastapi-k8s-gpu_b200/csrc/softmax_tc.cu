@@ -275,10 +275,10 @@ __global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_
 }
 
 // ---------------------------------------------------------------- host side
-// Steps whose sequences bring whole tiles: below about 48 rows a tile the 64-row kernels waste less. Sizes that the tiles and 16-byte
-// stores take, pages of whole 64-key halves.
-bool softmax_takes_tc(const SoftmaxTcArgs& a, int T, int n_tiles) {
-    return T >= 128 && T >= 48 * n_tiles && a.d % 16 == 0 && a.dv % 16 == 0 && a.d <= 128 && a.dv <= 128 && a.block_tokens % 64 == 0 && a.ld_out % 8 == 0 &&
+// Steps whose sequences bring at least 256 tokens each on average: two tiles of 128 rows, enough CTAs and key blocks for the copies and
+// the next block's scores to hide under the softmax. Sizes that the tiles and 16-byte stores take, pages of whole 64-key halves.
+bool softmax_takes_tc(const SoftmaxTcArgs& a, int T, int n_seg) {
+    return T >= 256 * n_seg && a.d % 16 == 0 && a.dv % 16 == 0 && a.d <= 128 && a.dv <= 128 && a.block_tokens % 64 == 0 && a.ld_out % 8 == 0 &&
            ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.out) | reinterpret_cast<uintptr_t>(a.out_bf16)) & 15) == 0;
 }
 
@@ -289,7 +289,7 @@ cudaError_t softmax_tc_launch(const SoftmaxTcArgs& a, const RaggedDev& r, cudaSt
         return cudaFuncSetAttribute(softmax_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess &&
                cudaFuncSetAttribute(softmax_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess;
     }();
-    if (!ready || !softmax_takes_tc(a, r.T, r.n_tiles)) return cudaErrorInvalidValue;
+    if (!ready || !softmax_takes_tc(a, r.T, r.n_seg)) return cudaErrorInvalidValue;
     CUtensorMap mk, mv;
     if (!bf16_rows_map(&mk, a.k_pool, a.d, a.pool_rows, a.d, 1, 0, 64) || !bf16_rows_map(&mv, a.v_pool, a.dv, a.pool_rows, a.dv, 1, 0, 64)) return cudaErrorInvalidValue;
     const size_t smem = (size_t)(4 * k_parts + 2 * v_parts) * SX_PART + 1024;

@@ -16,7 +16,7 @@ struct SoftmaxTcArgs {
     const float* gate; int ld_gate; int gate_per_head; // sigmoid output gate or null (as in SinkAttnArgs)
     float* out; __nv_bfloat16* out_bf16; int ld_out;   // out[t][h * dv + i], or rounded
 };
-bool softmax_takes_tc(const SoftmaxTcArgs& a, int T, int n_tiles);
+bool softmax_takes_tc(const SoftmaxTcArgs& a, int T, int n_seg);
 cudaError_t softmax_tc_launch(const SoftmaxTcArgs& a, const RaggedDev& r, cudaStream_t s);
 
 }  // namespace b2
