@@ -36,6 +36,7 @@ struct TcParams {
     int nN, nT;              // weight-row tiles; token tiles (grouped: tiles of the sorted pairs)
     int n_work;              // tiles in all
     int stages, cols;        // ring stages; tensor-memory columns of one accumulator
+    int ks;                  // 64-wide K slices of a stage (1; short steps also 2 and 4)
     unsigned int* err;
 };
 
@@ -171,7 +172,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) dense_tc_kernel(const __grid_co
     uint8_t* ring = reinterpret_cast<uint8_t*>(((uintptr_t)tc_smem + 1023) & ~(uintptr_t)1023);
     const int S = p.stages;
     // a stage: weights, then tokens (short steps: the MMA reads 128 token rows whatever NT is; what it finds there is dropped)
-    const uint32_t w_bytes = (uint32_t)p.NW * TC_K * 2, stage_bytes = w_bytes + (uint32_t)p.NT * TC_K * 2;
+    const int ks = SHORT ? p.ks : 1;
+    const uint32_t w_slice = (uint32_t)p.NW * TC_K * 2, x_slice = (uint32_t)p.NT * TC_K * 2, w_bytes = ks * w_slice, stage_bytes = w_bytes + ks * x_slice;
     uint32_t tmem_cols = 32;
     while ((int)tmem_cols < 2 * p.cols) tmem_cols <<= 1;
     if (warp == 5) {
@@ -188,7 +190,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) dense_tc_kernel(const __grid_co
     tc_after_sync();
     griddep_launch();
     const uint32_t tmem = tmem_at;
-    const int nk = (a.K + TC_K - 1) / TC_K, first = blockIdx.x, step = gridDim.x;
+    const int slices = (a.K + TC_K - 1) / TC_K, nk = (slices + ks - 1) / ks, first = blockIdx.x, step = gridDim.x;
+    auto load_w = [&](uint8_t* st, int k, const TcTile& w, uint64_t* bar) {
+        if (SHORT && ks > 1) tma_load_4d(st, &map_w, 0, w.n0, k * ks, w.z, bar);
+        else tma_load_3d(st, &map_w, k * TC_K, w.n0, w.z, bar);
+    };
 
     if (warp == 4 && lane == 0) {
         // ================= copies
@@ -200,7 +206,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) dense_tc_kernel(const __grid_co
             tc_tile(p, first, 0, w);
             for (; ahead < S && ahead < nk; ahead++) {
                 mbar_arrive_expect_tx(&full[ahead], stage_bytes);
-                tma_load_3d(ring + (size_t)ahead * stage_bytes, &map_w, ahead * TC_K, w.n0, w.z, &full[ahead]);
+                load_w(ring + (size_t)ahead * stage_bytes, ahead, w, &full[ahead]);
             }
         }
         griddep_wait();
@@ -214,9 +220,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) dense_tc_kernel(const __grid_co
                 } else {
                     if (use > 0) mbar_wait(&empty[s], (use - 1) & 1, p.err, 0x50001u, (unsigned)k);
                     mbar_arrive_expect_tx(&full[s], stage_bytes);
-                    tma_load_3d(st, &map_w, k * TC_K, w.n0, w.z, &full[s]);
+                    load_w(st, k, w, &full[s]);
                 }
-                tma_load_3d(st + w_bytes, &map_x, k * TC_K, w.t0, a.grouped ? 0 : w.z, &full[s]);
+                if (SHORT && ks > 1) tma_load_4d(st + w_bytes, &map_x, 0, w.t0, k * ks, a.grouped ? 0 : w.z, &full[s]);
+                else tma_load_3d(st + w_bytes, &map_x, k * TC_K, w.t0, a.grouped ? 0 : w.z, &full[s]);
                 if (++s == S) { s = 0; use++; }
             }
             waited = true;
@@ -238,10 +245,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) dense_tc_kernel(const __grid_co
                 mbar_wait(&full[s], use & 1, p.err, 0x50003u, (unsigned)k);
                 tc_after_sync();
                 const uint32_t at = smem_u32(ring + (size_t)s * stage_bytes);
-                const uint64_t dw = tc_desc(at), dx = tc_desc(at + w_bytes);
+                const int n_slices = min(ks, slices - k * ks);
+                for (int q = 0; q < n_slices; q++) {
+                    const uint64_t dw = tc_desc(at + q * w_slice), dx = tc_desc(at + w_bytes + q * x_slice);
 #pragma unroll
-                for (int kk = 0; kk < TC_K / 16; kk++)
-                    tc_mma(tmem + b * p.cols, (SHORT ? dx : dw) + 2 * kk, (SHORT ? dw : dx) + 2 * kk, idesc, (k | kk) ? 1u : 0u);
+                    for (int kk = 0; kk < TC_K / 16; kk++)
+                        tc_mma(tmem + b * p.cols, (SHORT ? dx : dw) + 2 * kk, (SHORT ? dw : dx) + 2 * kk, idesc, (k | q | kk) ? 1u : 0u);
+                }
                 tc_commit(&empty[s]);
                 if (++s == S) { s = 0; use++; }
             }
@@ -334,7 +344,8 @@ __global__ void rows_to_bf16_kernel(const TX* __restrict__ x, int ldx, const int
 typedef CUresult (*TcEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-static bool encode_map(CUtensorMap* m, const void* base, const cuuint64_t (&dims)[3], const cuuint64_t (&strides)[2], const cuuint32_t (&box)[3]) {
+template <int N>
+static bool encode_map(CUtensorMap* m, const void* base, const cuuint64_t (&dims)[N], const cuuint64_t (&strides)[N - 1], const cuuint32_t (&box)[N]) {
     static const TcEncodeFn encode = [] {
         void* fn = nullptr;
         cudaDriverEntryPointQueryResult q;
@@ -342,8 +353,8 @@ static bool encode_map(CUtensorMap* m, const void* base, const cuuint64_t (&dims
         cudaGetLastError();
         return (TcEncodeFn)fn;
     }();
-    const cuuint32_t es[3] = {1, 1, 1};
-    return encode && encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    const cuuint32_t es[4] = {1, 1, 1, 1};
+    return encode && encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, N, const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 bool bf16_rows_map(CUtensorMap* m, const void* base, long cols, long rows, long ld, long nb, long bs, int box_rows) {
@@ -351,6 +362,12 @@ bool bf16_rows_map(CUtensorMap* m, const void* base, long cols, long rows, long 
     const cuuint64_t strides[2] = {(cuuint64_t)ld * 2, (cuuint64_t)(nb > 1 ? bs * 2 : ld * 2)};
     const cuuint32_t box[3] = {TC_K, (cuuint32_t)box_rows, 1};
     return encode_map(m, base, dims, strides, box);
+}
+bool bf16_slices_map(CUtensorMap* m, const void* base, long cols, long rows, long ld, long nb, long bs, int box_rows, int slices) {
+    const cuuint64_t dims[4] = {TC_K, (cuuint64_t)rows, (cuuint64_t)(cols / TC_K), (cuuint64_t)nb};
+    const cuuint64_t strides[3] = {(cuuint64_t)ld * 2, TC_K * 2, (cuuint64_t)(nb > 1 ? bs * 2 : ld * 2)};
+    const cuuint32_t box[4] = {TC_K, (cuuint32_t)box_rows, (cuuint32_t)slices, 1};
+    return cols % TC_K == 0 && encode_map(m, base, dims, strides, box);
 }
 bool bf16_heads_map(CUtensorMap* m, const void* base, long cols, long heads, long rows, int box_rows) {
     const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)heads, (cuuint64_t)rows};
@@ -445,14 +462,19 @@ cudaError_t dense_tc_launch(const DenseArgs& a, const DenseDev& d, cudaStream_t 
     p.nN = (a.N + p.NW - 1) / p.NW;
     p.n_work = p.nN * p.nT * (grouped ? 1 : a.batch);
     p.cols = ((short_step ? p.NW : p.NT) + 31) / 32 * 32;
-    const int stage_bytes = (p.NW + p.NT) * TC_K * 2;
+    // short steps: several K slices per copy and barrier while a stage stays within 32 KB (with one, a 16-row tile moved 2 KB per copy and the
+    // copying thread set the pace)
+    p.ks = 1;
+    if (short_step && a.K % TC_K == 0) while (p.ks < 4 && (p.NW + p.NT) * TC_K * 2 * p.ks * 2 <= 32 * 1024 && a.K / TC_K >= 4 * p.ks) p.ks *= 2;
+    const int stage_bytes = (p.NW + p.NT) * TC_K * 2 * p.ks;
     p.stages = std::min(TC_MAX_STAGES, TC_RING / stage_bytes);
     TcKernel kernel = tc_kernel(a.epi, a.y_rounded != nullptr, short_step);
     if (!kernel) return cudaErrorInvalidValue;
     CUtensorMap mw, mx;
     const long w_entries = grouped ? a.groups->n_groups : a.batch, w_bs = grouped ? a.groups->w_stride : a.w_bs;
-    if (!bf16_rows_map(&mw, a.w, a.K, a.N, a.K, w_entries, w_bs, p.NW)) return cudaErrorInvalidValue;
-    if (!bf16_rows_map(&mx, xb, a.K, rows, span, grouped ? 1 : a.batch, a.x_bs, p.NT)) return cudaErrorInvalidValue;
+    const long x_entries = grouped ? 1 : a.batch;
+    if (p.ks > 1 ? !bf16_slices_map(&mw, a.w, a.K, a.N, a.K, w_entries, w_bs, p.NW, p.ks) : !bf16_rows_map(&mw, a.w, a.K, a.N, a.K, w_entries, w_bs, p.NW)) return cudaErrorInvalidValue;
+    if (p.ks > 1 ? !bf16_slices_map(&mx, xb, a.K, rows, span, x_entries, a.x_bs, p.NT, p.ks) : !bf16_rows_map(&mx, xb, a.K, rows, span, x_entries, a.x_bs, p.NT)) return cudaErrorInvalidValue;
     return launch_chain(kernel, dim3(std::min(p.n_work, SMS)), dim3(TC_THREADS), (size_t)p.stages * stage_bytes + TC_M * TC_K * 2 + 1024, s, mw, mx, p);
 }
 
