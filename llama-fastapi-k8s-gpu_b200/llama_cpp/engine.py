@@ -329,6 +329,21 @@ class LayeredEngine(EngineBase):
         n_want = sum(len(w) for w in want)
         logits = np.empty((n_want, self.dims.n_vocab), dtype=np.float32)
         sampled = [None] * n
+        lens = [len(toks) for _, toks in entries]
+        if (0 < n <= _cabi.B2_STEP_MAX_ENTRIES and n == len(want) == len(sample) and min(lens) > 0 and sum(lens) <= self.max_step_tokens and
+                all(0 <= wi < k for w, k in zip(want, lens) for wi in w)):
+            # the usual case: one native step, whose wanted rows are the result
+            flat, rows, at = [], [], 0
+            for (_, toks), w, k in zip(entries, want, lens):
+                flat.extend(toks)
+                rows.extend([at + wi for wi in w])
+                at += k
+            ints = ctypes.c_int32
+            out_tok = (ints * n)()
+            check(self.lib.b2_step(self._h, n, (ints * n)(*[slot for slot, _ in entries]), (ints * n)(*lens), (ints * at)(*flat),
+                                   (ints * n_want)(*rows) if n_want else None, n_want,
+                                   logits.ctypes.data_as(ctypes.c_void_p) if n_want else None, (ints * n)(*[1 if f else 0 for f in sample]), out_tok), "b2_step")
+            return logits, [t if f else None for t, f in zip(out_tok, sample)]
         base, acc = [], 0
         for w in want:
             base.append(acc)
