@@ -991,9 +991,11 @@ __global__ void __launch_bounds__(MG_TB) matrix_mem_gates_kernel(MatrixMemArgs a
 // in shared memory as asynchronous copies while this block is computed) and for the partial read-outs per row group, which all
 // threads then sum in a fixed order, one (token, column) each. The CTA past the last columns carries the normaliser n (a lane per
 // row) and leaves n . q; the division by it waits for matrix_mem_out_kernel.
-// Bound by issue slots: 96 operations on the memory and 8 shared loads per token and warp.
+// Bound by the latency of the updates and read-outs, one or two warps a scheduler: 64 multiply-adds, 32 products and 8 shared loads per
+// token and warp. A 2048-token prompt of 8 heads of 128 x 128 (B200): 966 us with one column a thread, 580 with two, 428 with the next
+// token's operands fetched ahead and the read-outs apart from the updates.
 constexpr int MM_ROWS = 16, MM_COLS = 32, MM_TB = 16;      // key size <= 16 * 16 = 256 (256 threads)
-__global__ void __launch_bounds__(256) matrix_mem_kernel(MatrixMemArgs a, RaggedDev r, int RG) {
+__global__ void __launch_bounds__(256, 1) matrix_mem_kernel(MatrixMemArgs a, RaggedDev r, int RG) {
     griddep_launch();
     griddep_wait();
     extern __shared__ float sm[];
@@ -1082,7 +1084,35 @@ __global__ void __launch_bounds__(256) matrix_mem_kernel(MatrixMemArgs a, Ragged
             }
         } else if (act) {
             const bool full = vec4 && grp * MM_ROWS + MM_ROWS <= d;
+            if (full) {
+                // the next token's row pieces and factors are read while this one is computed, the updates of all rows stand apart from the
+                // two read-out chains: a scheduler has one warp of this kernel, so latency hides only behind the warp's own work
+                float4 kn[4], qn[4];
+                float2 gn, vn;
+                auto fetch = [&](int u) {
+                    const int bu = buf * MM_TB + u;
+                    const float *kr = ks + bu * d + grp * MM_ROWS, *qr = qs + bu * d + grp * MM_ROWS;
+#pragma unroll
+                    for (int i = 0; i < 4; i++) { kn[i] = *reinterpret_cast<const float4*>(kr + 4 * i); qn[i] = *reinterpret_cast<const float4*>(qr + 4 * i); }
+                    gn = *reinterpret_cast<const float2*>(gs + bu * 2); vn = *reinterpret_cast<const float2*>(vs + bu * MM_COLS + 2 * lp);
+                };
+                fetch(0);
 #pragma unroll 2
+                for (int u = 0; u < nb; u++) {
+                    const float kk[16] = {kn[0].x, kn[0].y, kn[0].z, kn[0].w, kn[1].x, kn[1].y, kn[1].z, kn[1].w,
+                                          kn[2].x, kn[2].y, kn[2].z, kn[2].w, kn[3].x, kn[3].y, kn[3].z, kn[3].w};
+                    const float qq[16] = {qn[0].x, qn[0].y, qn[0].z, qn[0].w, qn[1].x, qn[1].y, qn[1].z, qn[1].w,
+                                          qn[2].x, qn[2].y, qn[2].z, qn[2].w, qn[3].x, qn[3].y, qn[3].z, qn[3].w};
+                    const float da = gn.y, v0 = gn.x * vn.x, v1 = gn.x * vn.y;
+                    fetch(min(u + 1, nb - 1));
+                    float p0 = 0.f, p1 = 0.f;
+#pragma unroll
+                    for (int i = 0; i < 16; i++) { S0[i] = fmaf(da, S0[i], kk[i] * v0); S1[i] = fmaf(da, S1[i], kk[i] * v1); }
+#pragma unroll
+                    for (int i = 0; i < 16; i++) { p0 = fmaf(S0[i], qq[i], p0); p1 = fmaf(S1[i], qq[i], p1); }
+                    *reinterpret_cast<float2*>(red + (size_t)(buf * MM_TB + u) * red_tok + grp * MM_COLS + 2 * lp) = make_float2(p0 * qscale, p1 * qscale);
+                }
+            } else
             for (int u = 0; u < nb; u++) {
                 const int bu = buf * MM_TB + u;
                 const float2 g2 = *reinterpret_cast<const float2*>(gs + bu * 2), v2 = *reinterpret_cast<const float2*>(vs + bu * MM_COLS + 2 * lp);
@@ -1090,25 +1120,12 @@ __global__ void __launch_bounds__(256) matrix_mem_kernel(MatrixMemArgs a, Ragged
                 float p0 = 0.f, p1 = 0.f;
                 const float* kr = ks + bu * d + grp * MM_ROWS;
                 const float* qr = qs + bu * d + grp * MM_ROWS;
-                if (full) {
-#pragma unroll
-                    for (int k4 = 0; k4 < MM_ROWS; k4 += 4) {
-                        const float4 kv = *reinterpret_cast<const float4*>(kr + k4), qv = *reinterpret_cast<const float4*>(qr + k4);
-                        const float kk[4] = {kv.x, kv.y, kv.z, kv.w}, qq[4] = {qv.x, qv.y, qv.z, qv.w};
-#pragma unroll
-                        for (int i = 0; i < 4; i++) {
-                            S0[k4 + i] = fmaf(da, S0[k4 + i], kk[i] * v0); p0 = fmaf(S0[k4 + i], qq[i], p0);
-                            S1[k4 + i] = fmaf(da, S1[k4 + i], kk[i] * v1); p1 = fmaf(S1[k4 + i], qq[i], p1);
-                        }
-                    }
-                } else {
 #pragma unroll
                     for (int k = 0; k < MM_ROWS; k++)
                         if (grp * MM_ROWS + k < d) {
                             S0[k] = fmaf(da, S0[k], kr[k] * v0); p0 = fmaf(S0[k], qr[k], p0);
                             S1[k] = fmaf(da, S1[k], kr[k] * v1); p1 = fmaf(S1[k], qr[k], p1);
                         }
-                }
                 *reinterpret_cast<float2*>(red + (size_t)bu * red_tok + grp * MM_COLS + 2 * lp) = make_float2(p0 * qscale, p1 * qscale);
             }
         }
