@@ -651,10 +651,7 @@ __device__ __forceinline__ void sk_split_bf16(float a, float b, uint32_t& hi, ui
 }
 }  // namespace
 
-// PACK: every sequence of the step brings one token. The rows of a CTA's tile are then the query heads of one key/value head (a row's
-// arithmetic is the same), so a step of 32 sequences with 16 heads over 4 runs 128 CTAs with one busy warp each instead of 512 that
-// multiply 63 rows of nothing beside theirs.
-template <int DMAX, int DVMAX, bool CAP, bool PACK>
+template <int DMAX, int DVMAX, bool CAP>
 __global__ void __launch_bounds__(128) sink_attn_mma_kernel(SinkAttnArgs a, RaggedDev r) {
     griddep_launch();
     griddep_wait();
@@ -666,16 +663,13 @@ __global__ void __launch_bounds__(128) sink_attn_mma_kernel(SinkAttnArgs a, Ragg
     __nv_bfloat16* Vs = Ks + SKM_K * LD;                                // [64][LDV]
     const int Gv = a.talk ? a.G : 1;
     // late tiles of a segment have the most key blocks: they start first
-    const int HG = a.H / a.G;
-    const int tile = gridDim.x - 1 - blockIdx.x, h = PACK ? (int)blockIdx.y * HG : (int)blockIdx.y / Gv, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tile = gridDim.x - 1 - blockIdx.x, h = blockIdx.y / Gv, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int seg = r.tile_seg[tile], row0 = r.tile_row0[tile];
     const int nq = min(SKM_Q, r.seg_start[seg] + r.seg_len[seg] - row0);
     const int p0 = r.tok_pos[row0], p_last = p0 + nq - 1;
     const int* table = a.block_tables[r.seg_slot[seg]];
-    const int g = h / HG;
-    const int rows = PACK ? HG : nq;               // rows of the tile: (PACK ? head h + row, the one token : head h, token row)
-    const bool busy = !PACK || warp * 16 < rows;
-    const int vg = !PACK && a.talk ? (int)(blockIdx.y % Gv) : g;
+    const int g = h / (a.H / a.G);
+    const int vg = a.talk ? (int)(blockIdx.y % Gv) : g;
     const __nv_bfloat16* kp = reinterpret_cast<const __nv_bfloat16*>(a.k_pool);
     const __nv_bfloat16* vp = reinterpret_cast<const __nv_bfloat16*>(a.v_pool);
     // scores live in the log2 domain (exp2 below). Capped: cap tanh(s / cap) = cap - 2 cap / (exp(2 s / cap) + 1), the exponential's
@@ -686,7 +680,7 @@ __global__ void __launch_bounds__(128) sink_attn_mma_kernel(SinkAttnArgs a, Ragg
     for (int i = threadIdx.x; i < SKM_Q * (d / 2); i += blockDim.x) {
         const int rr = i / (d / 2), c = (i % (d / 2)) * 2;
         float2 v = make_float2(0.f, 0.f);
-        if (rr < rows) v = *reinterpret_cast<const float2*>(a.q_rot + (PACK ? (size_t)row0 * a.H + h + rr : (size_t)(row0 + rr) * a.H + h) * d + c);
+        if (rr < nq) v = *reinterpret_cast<const float2*>(a.q_rot + ((size_t)(row0 + rr) * a.H + h) * d + c);
         v.x *= q_mul; v.y *= q_mul;
         const __nv_bfloat162 hi = __floats2bfloat162_rn(v.x, v.y);
         *reinterpret_cast<__nv_bfloat162*>(Qs + rr * LD + c) = hi;
@@ -701,13 +695,12 @@ __global__ void __launch_bounds__(128) sink_attn_mma_kernel(SinkAttnArgs a, Ragg
     const int qrow[2] = {warp * 16 + gq, warp * 16 + gq + 8};
     int qlo[2];                                    // oldest visible key of the lane's two query rows
     float m_run[2], l_run[2];
-    float sink[2];
+    const float sink = a.sink ? a.sink[h] * LOG2E : -INFINITY;
 #pragma unroll
     for (int q2 = 0; q2 < 2; q2++) {
-        const int i = PACK ? p0 : p0 + qrow[q2];
-        sink[q2] = a.sink ? a.sink[PACK ? min(h + qrow[q2], a.H - 1) : h] * LOG2E : -INFINITY;
+        const int i = p0 + qrow[q2];
         qlo[q2] = a.window > 0 ? max(0, i - a.window + 1) : 0;
-        m_run[q2] = sink[q2]; l_run[q2] = 0.f;         // the running maximum starts at the sink; its term joins the sum at the end
+        m_run[q2] = sink; l_run[q2] = 0.f;         // the running maximum starts at the sink; its term joins the sum at the end
     }
     // the next block's keys arrive while this block's weights meet the values, its values while the next scores are formed
     // (the thread's chunks of 16 bytes advance through the block without divisions; pages that hold whole blocks are looked up once)
@@ -738,7 +731,7 @@ __global__ void __launch_bounds__(128) sink_attn_mma_kernel(SinkAttnArgs a, Ragg
         for (int ni = 0; ni < SKM_K / 8; ni++) sacc[ni][0] = sacc[ni][1] = sacc[ni][2] = sacc[ni][3] = 0.f;
 #pragma unroll
         for (int ks = 0; ks < DMAX; ks += 16) {
-            if (ks < d && busy) {
+            if (ks < d) {
                 uint32_t af[4], al[4];
                 sk_ldsm_x4(af, Qs + (warp * 16 + (lane & 15)) * LD + ks + (lane >> 4) * 8);
                 sk_ldsm_x4(al, Ql + (warp * 16 + (lane & 15)) * LD + ks + (lane >> 4) * 8);
@@ -764,15 +757,15 @@ __global__ void __launch_bounds__(128) sink_attn_mma_kernel(SinkAttnArgs a, Ragg
 #pragma unroll
                 for (int e = 0; e < 4; e++) sacc[ni][e] = fmaf(-2.f * cap2, sk_rcp(sk_exp2(sacc[ni][e]) + 1.f), cap2);
         // the warp's rows all see the whole block: from its last key on, and not beyond the oldest key of its last row
-        const int w_first = PACK ? p0 : p0 + warp * 16, w_last = PACK ? p0 : w_first + 15;
-        const bool all = warp * 16 + 15 < rows && j0 + SKM_K - 1 <= w_first && (a.window <= 0 || j0 > w_last - a.window);
+        const int w_first = p0 + warp * 16, w_last = w_first + 15;
+        const bool all = warp * 16 + 15 < nq && j0 + SKM_K - 1 <= w_first && (a.window <= 0 || j0 > w_last - a.window);
         if (!all)
 #pragma unroll
             for (int ni = 0; ni < SKM_K / 8; ni++)
 #pragma unroll
                 for (int e = 0; e < 4; e++) {
-                    const int rr = qrow[e >> 1], i = PACK ? p0 : p0 + rr, j = j0 + ni * 8 + 2 * tq + (e & 1);
-                    const bool vis = rr < rows && j <= i && j >= qlo[e >> 1];
+                    const int rr = qrow[e >> 1], i = p0 + rr, j = j0 + ni * 8 + 2 * tq + (e & 1);
+                    const bool vis = rr < nq && j <= i && j >= qlo[e >> 1];
                     sacc[ni][e] = vis ? sacc[ni][e] : -INFINITY;
                 }
 #pragma unroll
@@ -815,7 +808,7 @@ __global__ void __launch_bounds__(128) sink_attn_mma_kernel(SinkAttnArgs a, Ragg
             sk_split_bf16(sacc[2 * kc + 1][2], sacc[2 * kc + 1][3], pf[3], pl[3]);
 #pragma unroll
             for (int nd = 0; nd < DVMAX / 16; nd++) {
-                if (nd * 16 < dv && busy) {
+                if (nd * 16 < dv) {
                     uint32_t vf[4];
                     sk_ldsm_x4_t(vf, Vs + (kc * 16 + (lane & 15)) * LDV + nd * 16 + (lane >> 4) * 8);
                     sk_mma_16816(o[2 * nd], pl, vf[0], vf[1]);
@@ -831,7 +824,7 @@ __global__ void __launch_bounds__(128) sink_attn_mma_kernel(SinkAttnArgs a, Ragg
     float inv[2];
 #pragma unroll
     for (int q2 = 0; q2 < 2; q2++) {
-        const float l = l_run[q2] + (a.sink ? sk_exp2(sink[q2] - m_run[q2]) : 0.f);
+        const float l = l_run[q2] + (a.sink ? sk_exp2(sink - m_run[q2]) : 0.f);
         inv[q2] = l > 0.f ? 1.f / l : 0.f;
     }
 #pragma unroll
@@ -839,19 +832,200 @@ __global__ void __launch_bounds__(128) sink_attn_mma_kernel(SinkAttnArgs a, Ragg
 #pragma unroll
         for (int e = 0; e < 4; e++) {
             const int rr = qrow[e >> 1], c = i * 8 + 2 * tq + (e & 1);
-            if (rr >= rows || c >= dv) continue;
+            if (rr >= nq || c >= dv) continue;
             const float v = o[i][e] * inv[e >> 1];
-            const int t = PACK ? row0 : row0 + rr, ho = PACK ? h + rr : h;
+            const int t = row0 + rr;
             if (a.out_bf16) {                  // two neighbouring columns of a row (dv is even)
                 if (e & 1) continue;
                 const float v2 = o[i][e + 1] * inv[e >> 1];
-                *reinterpret_cast<__nv_bfloat162*>(a.out_bf16 + (size_t)t * a.ld_out + (size_t)ho * dv + c) =
-                    __floats2bfloat162_rn(v * sk_gate(a, t, ho, c), v2 * sk_gate(a, t, ho, c + 1));
+                *reinterpret_cast<__nv_bfloat162*>(a.out_bf16 + (size_t)t * a.ld_out + (size_t)h * dv + c) =
+                    __floats2bfloat162_rn(v * sk_gate(a, t, h, c), v2 * sk_gate(a, t, h, c + 1));
                 continue;
             }
-            if (!PACK && a.talk) a.cross[(((size_t)t * a.H + h) * a.G + vg) * dv + c] = v;
-            else a.out[(size_t)t * a.ld_out + (size_t)ho * dv + c] = v * sk_gate(a, t, ho, c);
+            if (a.talk) a.cross[(((size_t)t * a.H + h) * a.G + vg) * dv + c] = v;
+            else a.out[(size_t)t * a.ld_out + (size_t)h * dv + c] = v * sk_gate(a, t, h, c);
         }
+}
+
+// Steps in which every sequence brings one token: a CTA takes one sequence and one key/value head, its 16 rows are the query heads that
+// share it. The arithmetic of a row is that of the prompt kernel, operation for operation (the same 64-key blocks, accumulation and sums),
+// spread over the warps by columns: a warp forms the scores of its 16 keys, all exchange them, each repeats the softmax of the rows and
+// adds up a quarter of the output columns. (32 sequences of 60 keys, 16 heads over 4: a 64-row tile per query head took 61 us a launch, one
+// warp per key/value head 33, most of it instruction fetch, the four warps of this form 17.)
+template <int DMAX, int DVMAX, bool CAP>
+__global__ void __launch_bounds__(128) sink_attn_pack_kernel(SinkAttnArgs a, RaggedDev r) {
+    griddep_launch();
+    griddep_wait();
+    extern __shared__ __align__(16) unsigned char sk_smem[];
+    const int d = a.d, dv = a.dv, LD = d + 8, LDV = dv + 8, HG = a.H / a.G;
+    constexpr int LDS = SKM_K + 8;
+    __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(sk_smem);     // [16][LD] leading bf16 of the queries
+    __nv_bfloat16* Ql = Qs + 16 * LD;                                   // [16][LD] what the first bf16 leaves over
+    __nv_bfloat16* Ks = Ql + 16 * LD;                                   // [64][LD]
+    __nv_bfloat16* Vs = Ks + SKM_K * LD;                                // [64][LDV]
+    float* Ss = reinterpret_cast<float*>(Vs + SKM_K * LDV);             // [16][LDS] scores of a block
+    const int seg = blockIdx.x, g = blockIdx.y, h0 = g * HG, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int t = r.seg_start[seg], pos = r.tok_pos[t];
+    const int* table = a.block_tables[r.seg_slot[seg]];
+    const __nv_bfloat16* kp = reinterpret_cast<const __nv_bfloat16*>(a.k_pool);
+    const __nv_bfloat16* vp = reinterpret_cast<const __nv_bfloat16*>(a.v_pool);
+    constexpr float LOG2E = 1.4426950408889634f;
+    const float q_mul = CAP ? a.scale * (2.f * LOG2E) / a.softcap : a.scale * LOG2E;
+    [[maybe_unused]] const float cap2 = CAP ? a.softcap * LOG2E : 0.f;
+    const int b0 = (a.window > 0 ? max(0, pos - a.window + 1) : 0) / SKM_K, b1 = pos / SKM_K;
+    const bool whole = a.block_tokens % SKM_K == 0;
+    auto load_rows = [&](const __nv_bfloat16* pool, int n, int ld, __nv_bfloat16* dst, int kb) {
+        const int per = n / 8, j0 = kb * SKM_K, last = pos - j0;        // rows past `last` are zero
+        int rr = threadIdx.x / per, c = threadIdx.x - rr * per;
+        const int drr = 128 / per, dc = 128 - drr * per;
+        const __nv_bfloat16* block = whole ? pool + (((size_t)table[j0 / a.block_tokens] * a.G + g) * a.block_tokens + j0 % a.block_tokens) * n : nullptr;
+        while (rr < SKM_K) {
+            const int row = min(rr, last);
+            const __nv_bfloat16* src = whole ? block + row * n
+                                             : pool + (((size_t)table[(j0 + row) / a.block_tokens] * a.G + g) * a.block_tokens + (j0 + row) % a.block_tokens) * n;
+            sk_cp_async_16z(dst + rr * ld + c * 8, src + c * 8, rr <= last ? 16 : 0);
+            rr += drr; c += dc;
+            if (c >= per) { c -= per; rr++; }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    load_rows(kp, d, LD, Ks, b0);
+    load_rows(vp, dv, LDV, Vs, b0);
+    for (int i = threadIdx.x; i < 16 * (d / 2); i += blockDim.x) {
+        const int rr = i / (d / 2), c = (i % (d / 2)) * 2;
+        float2 v = make_float2(0.f, 0.f);
+        if (rr < HG) v = *reinterpret_cast<const float2*>(a.q_rot + ((size_t)t * a.H + h0 + rr) * d + c);
+        v.x *= q_mul; v.y *= q_mul;
+        const __nv_bfloat162 hi = __floats2bfloat162_rn(v.x, v.y);
+        *reinterpret_cast<__nv_bfloat162*>(Qs + rr * LD + c) = hi;
+        *reinterpret_cast<__nv_bfloat162*>(Ql + rr * LD + c) = __floats2bfloat162_rn(v.x - __low2float(hi), v.y - __high2float(hi));
+    }
+    constexpr int ND = (DVMAX / 16 + 3) / 4;                            // 16-column pieces of the output per warp: warp, warp + 4
+    float o[2 * ND][4];
+#pragma unroll
+    for (int i = 0; i < 2 * ND; i++) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+    const int gq = lane >> 2, tq = lane & 3;
+    const int qlo = a.window > 0 ? max(0, pos - a.window + 1) : 0;
+    float m_run[2], l_run[2] = {0.f, 0.f}, sink[2];
+#pragma unroll
+    for (int q2 = 0; q2 < 2; q2++) m_run[q2] = sink[q2] = a.sink ? a.sink[min(h0 + gq + 8 * q2, a.H - 1)] * LOG2E : -INFINITY;
+    for (int kb = b0; kb <= b1; kb++) {
+        const int j0 = kb * SKM_K;
+        asm volatile("cp.async.wait_group 1;" ::: "memory");            // this block's keys
+        __syncthreads();
+        {   // scores of keys 16 warp .. + 15
+            float part[2][4] = {};
+#pragma unroll 2
+            for (int ks = 0; ks < d; ks += 16) {
+                uint32_t af[4], al[4], bf[4];
+                sk_ldsm_x4(af, Qs + (lane & 15) * LD + ks + (lane >> 4) * 8);
+                sk_ldsm_x4(al, Ql + (lane & 15) * LD + ks + (lane >> 4) * 8);
+                sk_ldsm_x4(bf, Ks + (warp * 16 + (lane & 7) + ((lane >> 4) << 3)) * LD + ks + ((lane >> 3) & 1) * 8);
+                sk_mma_16816(part[0], al, bf[0], bf[1]);
+                sk_mma_16816(part[1], al, bf[2], bf[3]);
+                sk_mma_16816(part[0], af, bf[0], bf[1]);
+                sk_mma_16816(part[1], af, bf[2], bf[3]);
+            }
+            if constexpr (CAP)
+#pragma unroll
+                for (int ni = 0; ni < 2; ni++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) part[ni][e] = fmaf(-2.f * cap2, sk_rcp(sk_exp2(part[ni][e]) + 1.f), cap2);
+#pragma unroll
+            for (int ni = 0; ni < 2; ni++)
+#pragma unroll
+                for (int q2 = 0; q2 < 2; q2++)
+                    *reinterpret_cast<float2*>(Ss + (gq + 8 * q2) * LDS + warp * 16 + ni * 8 + 2 * tq) = make_float2(part[ni][2 * q2], part[ni][2 * q2 + 1]);
+        }
+        __syncthreads();                                                // everybody's scores are there, and the keys are done with
+        if (kb < b1) load_rows(kp, d, LD, Ks, kb + 1);
+        else asm volatile("cp.async.commit_group;" ::: "memory");      // keep the count of groups
+        float sacc[SKM_K / 8][4];
+#pragma unroll
+        for (int ni = 0; ni < SKM_K / 8; ni++)
+#pragma unroll
+            for (int q2 = 0; q2 < 2; q2++) {
+                const float2 v = *reinterpret_cast<const float2*>(Ss + (gq + 8 * q2) * LDS + ni * 8 + 2 * tq);
+                sacc[ni][2 * q2] = v.x; sacc[ni][2 * q2 + 1] = v.y;
+            }
+        float mx[2] = {m_run[0], m_run[1]};
+        if (j0 + SKM_K - 1 > pos || j0 < qlo)
+#pragma unroll
+            for (int ni = 0; ni < SKM_K / 8; ni++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int j = j0 + ni * 8 + 2 * tq + (e & 1);
+                    sacc[ni][e] = j <= pos && j >= qlo ? sacc[ni][e] : -INFINITY;
+                }
+#pragma unroll
+        for (int ni = 0; ni < SKM_K / 8; ni++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) mx[e >> 1] = fmaxf(mx[e >> 1], sacc[ni][e]);
+        float corr[2], msafe[2], rs[2] = {0.f, 0.f};
+#pragma unroll
+        for (int q2 = 0; q2 < 2; q2++) {
+            mx[q2] = fmaxf(mx[q2], __shfl_xor_sync(0xffffffffu, mx[q2], 1));
+            mx[q2] = fmaxf(mx[q2], __shfl_xor_sync(0xffffffffu, mx[q2], 2));
+            msafe[q2] = mx[q2] > -INFINITY ? mx[q2] : 0.f;
+            corr[q2] = sk_exp2(m_run[q2] - msafe[q2]);
+            m_run[q2] = mx[q2];
+        }
+#pragma unroll
+        for (int ni = 0; ni < SKM_K / 8; ni++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const float p = sk_exp2(sacc[ni][e] - msafe[e >> 1]);
+                sacc[ni][e] = p;
+                rs[e >> 1] += p;
+            }
+#pragma unroll
+        for (int q2 = 0; q2 < 2; q2++) {
+            rs[q2] += __shfl_xor_sync(0xffffffffu, rs[q2], 1);
+            rs[q2] += __shfl_xor_sync(0xffffffffu, rs[q2], 2);
+            l_run[q2] = fmaf(l_run[q2], corr[q2], rs[q2]);
+        }
+#pragma unroll
+        for (int i = 0; i < 2 * ND; i++) { o[i][0] *= corr[0]; o[i][1] *= corr[0]; o[i][2] *= corr[1]; o[i][3] *= corr[1]; }
+        asm volatile("cp.async.wait_group 1;" ::: "memory");            // this block's values
+        __syncthreads();
+#pragma unroll
+        for (int kc = 0; kc < SKM_K / 16; kc++) {
+            uint32_t pf[4], pl[4];
+            sk_split_bf16(sacc[2 * kc][0], sacc[2 * kc][1], pf[0], pl[0]);
+            sk_split_bf16(sacc[2 * kc][2], sacc[2 * kc][3], pf[1], pl[1]);
+            sk_split_bf16(sacc[2 * kc + 1][0], sacc[2 * kc + 1][1], pf[2], pl[2]);
+            sk_split_bf16(sacc[2 * kc + 1][2], sacc[2 * kc + 1][3], pf[3], pl[3]);
+#pragma unroll
+            for (int i = 0; i < ND; i++) {
+                const int c = (warp + 4 * i) * 16;
+                if (c < dv) {
+                    uint32_t vf[4];
+                    sk_ldsm_x4_t(vf, Vs + (kc * 16 + (lane & 15)) * LDV + c + (lane >> 4) * 8);
+                    sk_mma_16816(o[2 * i], pl, vf[0], vf[1]);
+                    sk_mma_16816(o[2 * i + 1], pl, vf[2], vf[3]);
+                    sk_mma_16816(o[2 * i], pf, vf[0], vf[1]);
+                    sk_mma_16816(o[2 * i + 1], pf, vf[2], vf[3]);
+                }
+            }
+        }
+        __syncthreads();                                                // everybody is done with the values and the scores
+        if (kb < b1) load_rows(vp, dv, LDV, Vs, kb + 1);
+    }
+#pragma unroll
+    for (int q2 = 0; q2 < 2; q2++) {
+        const int rr = gq + 8 * q2, h = h0 + rr;
+        if (rr >= HG) continue;
+        const float l = l_run[q2] + (a.sink ? sk_exp2(sink[q2] - m_run[q2]) : 0.f), inv = l > 0.f ? 1.f / l : 0.f;
+#pragma unroll
+        for (int i = 0; i < 2 * ND; i++) {
+            const int c = (warp + 4 * (i >> 1)) * 16 + (i & 1) * 8 + 2 * tq;
+            if (c >= dv) continue;
+            const float v0 = o[i][2 * q2] * inv * sk_gate(a, t, h, c), v1 = o[i][2 * q2 + 1] * inv * sk_gate(a, t, h, c + 1);
+            const size_t at = (size_t)t * a.ld_out + (size_t)h * dv + c;
+            if (a.out_bf16) *reinterpret_cast<__nv_bfloat162*>(a.out_bf16 + at) = __floats2bfloat162_rn(v0, v1);
+            else { a.out[at] = v0; a.out[at + 1] = v1; }
+        }
+    }
 }
 
 // ---- prompts with mixed heads (bf16 pages): the weights are mixed BEFORE they meet the values, in three passes over a group of
@@ -1135,12 +1309,15 @@ static cudaError_t sink_attn_mma_pick(const SinkAttnArgs& a, const RaggedDev& r,
     static bool attr_done = false;
     if (!attr_done) {
         const int most = (3 * 64 * (DMAX + 8) + 64 * (DVMAX + 8)) * 2;
-        cudaFuncSetAttribute(sink_attn_mma_kernel<DMAX, DVMAX, CAP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-        cudaFuncSetAttribute(sink_attn_mma_kernel<DMAX, DVMAX, CAP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        cudaFuncSetAttribute(sink_attn_mma_kernel<DMAX, DVMAX, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        cudaFuncSetAttribute(sink_attn_pack_kernel<DMAX, DVMAX, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
         attr_done = true;
     }
-    if (!a.talk && r.T == r.n_seg && a.H / a.G <= SKM_Q) return launch_chain(sink_attn_mma_kernel<DMAX, DVMAX, CAP, true>, dim3(r.n_tiles, a.G), dim3(128), smem, s, a, r);
-    return launch_chain(sink_attn_mma_kernel<DMAX, DVMAX, CAP, false>, dim3(r.n_tiles, a.H * (a.talk ? a.G : 1)), dim3(128), smem, s, a, r);
+    if (!a.talk && r.T == r.n_seg && a.H / a.G <= 16) {
+        const size_t pack = (size_t)((32 + SKM_K) * (a.d + 8) + SKM_K * (a.dv + 8)) * 2 + 16 * (SKM_K + 8) * 4;
+        return launch_chain(sink_attn_pack_kernel<DMAX, DVMAX, CAP>, dim3(r.n_seg, a.G), dim3(128), pack, s, a, r);
+    }
+    return launch_chain(sink_attn_mma_kernel<DMAX, DVMAX, CAP>, dim3(r.n_tiles, a.H * (a.talk ? a.G : 1)), dim3(128), smem, s, a, r);
 }
 
 template <bool CAP>
