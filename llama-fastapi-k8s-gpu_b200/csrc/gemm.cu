@@ -418,6 +418,9 @@ __device__ __noinline__ void deq_loop(const DeqCtx cx) {
 
 // ROWS weight rows per CTA, ROWS / 32 dequantising warps + 3 service warps.
 // SWAP = false (T > 128): weights are the MMA's A operand (M = 128 rows = TMEM lanes), tokens its N (TMEM columns).
+//   ROWS = 256 (T > 256): two M halves over the same tokens, half of the step's tokens a CTA. With 128 rows and all 512 tokens a block of
+//   64 K entries brought 64 KB of activations for 1024 cycles of products, and the 148 CTAs together asked more of L2 than it gives;
+//   now a CTA brings 32 KB for the same products (and expands twice the weights, which the idle issue slots have room for).
 // SWAP = true  (T <= 128): tokens are the A operand (M = 128, rows past T are don't-care), 256 weight rows are the N:
 //   with few tokens an instruction costs ~130 cycles whatever N is (measured), so each MMA should cover as many
 //   weight rows as an instruction can: 256.
@@ -427,16 +430,19 @@ __global__ void __launch_bounds__((ROWS / 32 + 3) * 32) gemm_q_kernel(const __gr
     extern __shared__ __align__(128) uint8_t smem_raw[];
     GemmBars& sh = *reinterpret_cast<GemmBars*>(smem_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int T = p.T_pad, S = p.n_stages, SB = p.n_bstages;
+    constexpr bool WIDE = !SWAP && ROWS == 256;
+    const int S = p.n_stages, SB = p.n_bstages;
+    const int n_tt = WIDE ? p.n_tt : 1, tt = WIDE ? blockIdx.x / p.n_splits % n_tt : 0;
+    const int t_base = tt * p.t_tile, T = min(p.t_tile, p.T_pad - t_base);      // this CTA's tokens
     const uint32_t a_bytes = ROWS * GM_BK * 2, b_bytes = (uint32_t)T * GM_BK * 2;
     uint8_t* stage0 = smem_raw + GM_HDR;                               // A tiles: S x 16 KB
     uint8_t* bst0 = stage0 + (size_t)S * a_bytes;                      // activation tiles: SB x T*128 B
     uint8_t* raw0 = bst0 + (size_t)SB * b_bytes;                       // raw weight spans: n_raw x [128][box]
     uint32_t ncols = 32;
-    while ((int)ncols < (SWAP ? ROWS : T)) ncols <<= 1;
+    while ((int)ncols < (SWAP ? ROWS : WIDE ? 2 * T : T)) ncols <<= 1;
 
     // ---- which tile / K range (in 256-weight spans = 4 blocks)
-    const int split = blockIdx.x % p.n_splits, tile_g = blockIdx.x / p.n_splits;
+    const int split = blockIdx.x % p.n_splits, tile_g = blockIdx.x / p.n_splits / n_tt;
     int seg = 0;
     while (seg + 1 < p.nseg && tile_g >= p.seg[seg + 1].tile0) seg++;
     const GemmSeg& sg = p.seg[seg];
@@ -491,15 +497,15 @@ __global__ void __launch_bounds__((ROWS / 32 + 3) * 32) gemm_q_kernel(const __gr
         griddep_wait();
         if (!SWAP) {                               // TMEM lane = weight row, columns = tokens
             const int row = m0 + tid;
-            const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
-            float* ybase = p.y + (size_t)split * p.split_stride + sg.out_off + row;
+            const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(warp >> 2) * (ncols / 2);
+            float* ybase = p.y + (size_t)split * p.split_stride + (size_t)t_base * p.ldy + sg.out_off + row;
             for (int c0 = 0; c0 < T; c0 += 16) {
                 float v[16];
                 tmem_ld16(lane_addr + c0, v);
                 if (row < sg.n_rows) {
 #pragma unroll
                     for (int j = 0; j < 16; j++)
-                        if (c0 + j < p.T) ybase[(size_t)(c0 + j) * p.ldy] = v[j];
+                        if (t_base + c0 + j < p.T) ybase[(size_t)(c0 + j) * p.ldy] = v[j];
                 }
             }
         } else if (warp < 4 && warp * 32 < p.T) {  // TMEM lane = token (warps 0-3 own the 128 lanes), columns = weight rows
@@ -522,8 +528,8 @@ __global__ void __launch_bounds__((ROWS / 32 + 3) * 32) gemm_q_kernel(const __gr
         }
     } else if (warp == DW && lane == 0) {
         // ================= MMA thread
-        const uint32_t idesc_lo = SWAP ? instr_desc(128, ROWS) : instr_desc(ROWS, T > 256 ? 256 : T);
-        const uint32_t idesc_hi = (!SWAP && T > 256) ? instr_desc(ROWS, T - 256) : 0u;
+        const uint32_t idesc_lo = SWAP ? instr_desc(128, ROWS) : instr_desc(GM_BM, T > 256 ? 256 : T);
+        const uint32_t idesc_hi = (!SWAP && T > 256) ? instr_desc(GM_BM, T - 256) : 0u;
         int s = 0, sb = 0;
         uint32_t use = 0, useb = 0;
         const uint32_t a_lo0 = (smem_u32(stage0) >> 4) | ((lbo_a >> 4) << 16), b_lo0 = (smem_u32(bst0) >> 4) | ((lbo_b >> 4) << 16);
@@ -545,7 +551,8 @@ __global__ void __launch_bounds__((ROWS / 32 + 3) * 32) gemm_q_kernel(const __gr
                     umma_f16(tmem, db, da, idesc_lo, acc);          // A = tokens (rows past T read whatever follows: dropped), B = weights
                 } else {
                     umma_f16(tmem, da, db, idesc_lo, acc);
-                    if (T > 256) umma_f16(tmem + 256, da, desc_join(b_lo + ks * (2 * lbo_b >> 4) + 256, desc_hi), idesc_hi, acc);
+                    if (WIDE) umma_f16(tmem + ncols / 2, desc_join(a_lo + ks * (2 * lbo_a >> 4) + GM_BM, desc_hi), db, idesc_lo, acc);      // rows 128 ..
+                    else if (T > 256) umma_f16(tmem + 256, da, desc_join(b_lo + ks * (2 * lbo_b >> 4) + 256, desc_hi), idesc_hi, acc);
                 }
             }
             umma_commit(&sh.empty[s]);      // both arrive when the MMAs above have finished reading their tiles
@@ -563,7 +570,12 @@ __global__ void __launch_bounds__((ROWS / 32 + 3) * 32) gemm_q_kernel(const __gr
         for (int i = 0; i < n; i++) {
             if (useb > 0) mbar_wait(&sh.b_empty[sb], (useb - 1) & 1, p.err, 0x40005u, (unsigned)i);
             mbar_arrive_expect_tx(&sh.b_full[sb], b_bytes);
-            tma_load_1d(bst0 + (size_t)sb * b_bytes, xb + (size_t)(kb0 + i) * b_bytes, b_bytes, &sh.b_full[sb]);
+            if (WIDE) {                 // part of the tokens: one run per chunk of 8 K entries
+                for (int c = 0; c < GM_BK / 8; c++)
+                    tma_load_1d(bst0 + (size_t)sb * b_bytes + (size_t)c * lbo_b, xb + ((size_t)((kb0 + i) * (GM_BK / 8) + c) * p.T_pad + t_base) * 16, lbo_b, &sh.b_full[sb]);
+            } else {
+                tma_load_1d(bst0 + (size_t)sb * b_bytes, xb + (size_t)(kb0 + i) * b_bytes, b_bytes, &sh.b_full[sb]);
+            }
             if (++sb == SB) { sb = 0; useb++; }
         }
     } else if (warp == DW + 1 && lane == 0 && sg.use_tma) {
@@ -583,7 +595,7 @@ __global__ void __launch_bounds__((ROWS / 32 + 3) * 32) gemm_q_kernel(const __gr
 }
 
 // ---------------------------------------------------------------- host side
-static int gemm_rows(const GemmParams& p) { return p.swap ? 256 : GM_BM; }
+static int gemm_rows(const GemmParams& p) { return p.swap || p.n_tt > 1 ? 256 : GM_BM; }
 static size_t gemm_raw_bytes(const GemmParams& p) {
     size_t m = 0;
     for (int s = 0; s < p.nseg; s++) if (p.seg[s].use_tma) m = std::max(m, (size_t)p.n_raw * gemm_rows(p) * p.seg[s].box_bytes);
@@ -591,7 +603,7 @@ static size_t gemm_raw_bytes(const GemmParams& p) {
 }
 size_t gemm_smem_bytes(const GemmParams& p) {
     // swap: the MMA reads 128 token rows per K chunk whatever T is; the rows past the tile must still be shared memory
-    return GM_HDR + (size_t)p.n_stages * gemm_rows(p) * GM_BK * 2 + (size_t)p.n_bstages * p.T_pad * GM_BK * 2 + gemm_raw_bytes(p) +
+    return GM_HDR + (size_t)p.n_stages * gemm_rows(p) * GM_BK * 2 + (size_t)p.n_bstages * p.t_tile * GM_BK * 2 + gemm_raw_bytes(p) +
            (p.swap ? 4096 : 0);
 }
 
@@ -611,6 +623,8 @@ cudaError_t gemm_init() {
     }
     cudaError_t e = cudaFuncSetAttribute(gemm_q_kernel<GM_BM, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(gemm_q_kernel<256, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(gemm_q_kernel<256, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
 }
 
@@ -622,6 +636,8 @@ int gemm_plan(GemmParams& p, int n_sms, int max_splits) {
     if (p.T < 1 || p.T > 512) return -2;
     p.T_pad = (p.T + 15) / 16 * 16;
     p.swap = (p.T_pad <= 128 && !getenv("B2_GEMM_NOSWAP")) ? 1 : 0;
+    p.n_tt = p.T_pad > 256 ? 2 : 1;
+    p.t_tile = p.n_tt == 1 ? p.T_pad : (p.T_pad / 2 + 15) / 16 * 16;
     const int ROWS = gemm_rows(p);
     int tiles = 0;
     const bool no_tma = getenv("B2_GEMM_NO_TMA") != nullptr;
@@ -652,11 +668,11 @@ int gemm_plan(GemmParams& p, int n_sms, int max_splits) {
         }
     }
     p.n_tiles = tiles;
-    const size_t a_st = (size_t)ROWS * GM_BK * 2, b_st = (size_t)p.T_pad * GM_BK * 2;
+    const size_t a_st = (size_t)ROWS * GM_BK * 2, b_st = (size_t)p.t_tile * GM_BK * 2;
     const size_t cap = 227 * 1024 - 1024;
     // activation ring: deep when the tiles are small (their TMA latency must not gate the MMAs)
-    int SB = p.T_pad <= 32 ? 8 : p.T_pad <= 64 ? 6 : p.T_pad <= 128 ? 4 : p.T_pad <= 256 ? 3 : 2;
-    int S = p.swap ? 3 : (p.T_pad <= 64 ? 2 : 3);
+    int SB = p.T_pad <= 32 ? 8 : p.T_pad <= 64 ? 6 : p.T_pad <= 128 ? 4 : 3;
+    int S = p.swap ? 3 : (p.T_pad <= 64 || p.n_tt > 1 ? 2 : 3);
     int per_sm = (!p.swap && p.T_pad <= 64) ? 2 : 1;   // 128-row variant at small T: two CTAs per SM
     if (const char* v = getenv("B2_GEMM_PER_SM")) if (atoi(v) > 0) per_sm = atoi(v);
     if (const char* v = getenv("B2_GEMM_STAGES")) if (atoi(v) > 1) S = atoi(v);
@@ -681,7 +697,7 @@ int gemm_plan(GemmParams& p, int n_sms, int max_splits) {
     long best_cost = -1;
     int best = 1;
     for (int s = 1; s <= max_splits && s <= 16 && s <= n_sp; s++) {
-        const long waves = ((long)tiles * s + slots - 1) / slots;
+        const long waves = ((long)tiles * p.n_tt * s + slots - 1) / slots;
         const long cost = waves * (4 * ((n_sp + s - 1) / s) + fixed);
         if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = s; }
     }
@@ -694,6 +710,7 @@ cudaError_t gemm_launch(const GemmParams& p, cudaStream_t stream) {
         p.n_tiles < 1) return cudaErrorInvalidValue;
     if (p.T_pad < 16 || p.T_pad > 512 || p.T_pad % 16 || p.T > p.T_pad || p.n_splits > p.K / 256) return cudaErrorInvalidValue;
     if (p.swap) return launch_chain(gemm_q_kernel<256, true>, dim3(p.n_tiles * p.n_splits), dim3((256 / 32 + 3) * 32), gemm_smem_bytes(p), stream, p);
+    if (p.n_tt > 1) return launch_chain(gemm_q_kernel<256, false>, dim3(p.n_tiles * p.n_tt * p.n_splits), dim3((256 / 32 + 3) * 32), gemm_smem_bytes(p), stream, p);
     return launch_chain(gemm_q_kernel<GM_BM, false>, dim3(p.n_tiles * p.n_splits), dim3((GM_BM / 32 + 3) * 32), gemm_smem_bytes(p), stream, p);
 }
 
