@@ -5,25 +5,31 @@
 // (/root/reference/api.py:55-63), and its batched mul_mat_q path for several sequences per step. No f16 copy
 // of W ever exists in HBM: quant blocks go from HBM to registers to the shared-memory operand tile of the MMA.
 //
-// Work decomposition. A CTA owns one tile of 128 weight rows (MMA "M" = TMEM lanes) of one of up to three
-// matrices that share the input (q|k|v, gate|up), ALL T <= 512 tokens (MMA "N" = TMEM columns) and one of
-// n_splits contiguous K ranges; split s writes its partial sums to y + s * split_stride and the consumer
-// kernel (RoPE/KV store, residual+RMSNorm, SiLU*mul: prefill.cu) adds the splits in a fixed order, so results
-// are deterministic. Splitting K is what fills 148 SMs when N is only 1024-4096 rows.
+// Work decomposition. A CTA owns 256 weight rows (two halves of 128, the MMA's M and the lanes of tensor memory) of one of up to three
+// matrices that share the input (q|k|v, gate|up), one of up to two token tiles (the MMA's N) and one of n_splits
+// contiguous K ranges; split s writes its partial sums to y + s * split_stride and the consumer kernel (RoPE/KV store,
+// residual+RMSNorm, SiLU*mul: prefill.cu) adds the splits in a fixed order, so results are deterministic. Splitting K is what fills
+// 148 SMs when N is only 1024-4096 rows.
 //
-// Pipeline per CTA, S stages of 64 K-elements (A tile 16 KB + B tile T*128 B):
-//   warps 0-3 (thread r <-> weight row r): raw quant bytes of the NEXT block are already in registers
-//       (software prefetch) while the current block is expanded to f16 with byte-permute + half2 arithmetic
-//       (exact small integers 1024+q via byte-permute; scales applied without losing bits: ~2-2.5 instr/weight)
-//       and stored as 8 core-matrix rows of the A tile; fence.proxy.async; arrive on a_full[stage].
-//   warp 4, one thread: the B tile of a block is ONE 1-D TMA bulk copy (cp.async.bulk + mbarrier complete_tx):
-//       activations live in HBM in the MMA's own K-major core-matrix order [K/8][T][8] (the producing kernels
-//       write that layout), so the tile is contiguous. Waits a_full/b_full, issues 4 (x2 when T > 256)
-//       tcgen05.mma kind::f16 M=128 N=T K=16 accumulating in TMEM; tcgen05.commit arrives on empty[stage].
-//   epilogue: warps 0-3 read their 32 TMEM lanes (tcgen05.ld 32x32b.x16) and store float32, token-major.
-// Shared-memory operand layout: K-major, no swizzle: 8x8 f16 core matrices (8 rows x 16 B), LBO = byte stride
-// between core matrices along K, SBO = stride between 8-row groups (128 B).
-// Roofline: tensor pipe for large T; for T <= ~64 HBM (weights read once per call) and the dequantisation.
+// Pipeline per CTA, in blocks of 64 K-elements:
+//   weight producer (one thread): TMA boxes of 256 rows x one 256-weight span, raw block bytes -> shared memory.
+//   16 dequantising warps, two threads a row, each two of every four blocks: raw bytes -> f16 with byte-permute + half2 arithmetic (exact small
+//       integers 1024+q; scales applied without losing bits: ~2-2.5 instr/weight) -> tensor memory (tcgen05.st), as the MMA's A operand;
+//       one arrival per warp on a_full[stage].
+//   activation producer (one thread): activations live in HBM in the MMA's own K-major core-matrix order [K/8][T][8] (the producing
+//       kernels write that layout), so a tile is one 1-D TMA bulk copy (or one per 8 K entries for part of the tokens).
+//   MMA thread: waits a_full/b_full, issues 4 x 2 tcgen05.mma kind::f16 M=128 N=T K=16, A and sums in tensor memory; tcgen05.commit
+//       arrives on empty[stage].
+//   epilogue: the 16 warps read their TMEM lanes (tcgen05.ld 32x32b.x16) and store float32, token-major.
+// Shared-memory operand layout (activations): K-major, no swizzle: 8x8 f16 core matrices (8 rows x 16 B), LBO = byte stride between core
+// matrices along K, SBO = stride between 8-row groups (128 B).
+// Why the weights go to tensor memory: with both operands in shared memory a block of 256 rows costs that memory 32 KB of stores and 48 KB
+// of operand reads for 32 tokens (tokens as the 128-row operand), 96 KB of reads for 256 tokens: 800 and 1400 cycles of its 128 bytes a
+// cycle, against 512 and 1024 of products. The expansion itself needs about 500 with 16 warps (950 with 8, two a scheduler).
+// 32 sequences, 4 layers of 4096 (Q4_K/Q6_K), mean product: 23.1 us with both operands in shared memory and 8 warps; 25.7 with 16; 27 with the
+// weights in tensor memory (the MMA thread, one lane of a busy scheduler, took 1200 cycles a block); 17.5 with that loop run by the whole
+// warp and one lane issuing. A 37-token prompt: 9.7 -> 7 us a product.
+// Roofline: tensor pipe for large T; for T <= ~64 the dequantisation, then HBM (weights read once per call).
 #include "kernels.h"
 #include "ptx.cuh"
 #include "quant_blocks.cuh"
@@ -34,10 +40,14 @@
 
 namespace b2 {
 
-constexpr int GM_BM = 128;          // weight rows per CTA
+constexpr int GM_ROWS = 256;        // weight rows per CTA
 constexpr int GM_BK = 64;           // K per stage
+constexpr int GM_BM = 128;          // of one MMA: lanes of tensor memory
+constexpr int GM_ABYTES = GM_ROWS * GM_BK * 2;      // SS: bytes of a weight block
+constexpr int GM_DW = 16;           // dequantising warps: two threads a row
+constexpr int GM_THREADS = (GM_DW + 3) * 32;
 constexpr int GM_HDR = 512;         // barriers at the start of dynamic shared memory
-constexpr int GM_MAX_STAGES = 6;     // A-tile ring
+constexpr int GM_MAX_STAGES = 6;     // weight blocks in tensor memory
 constexpr int GM_MAX_BSTAGES = 8;    // activation-tile ring
 constexpr int GM_RAW_STAGES = 2;    // raw weight spans in flight (TMA), at most
 constexpr int GM_SPAN_WORDS = 68;   // largest 256-weight span: Q8_0, 272 bytes
@@ -51,12 +61,30 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+// D (+)= A . B, A [128 lanes][16 f16 in 8 columns] from tensor memory
+__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
+// the same with A from shared memory
+__device__ __forceinline__ void umma_f16_ss(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+                 "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+                   "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
+                   "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
+                   "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]) : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -189,9 +217,9 @@ __device__ __forceinline__ void split_f16(float v, __half2& hi, __half2& lo) {
 }
 __device__ __forceinline__ __half2 h2_from_bits16(uint32_t b) { return __half2half2(__ushort_as_half((unsigned short)b)); }
 
-// dst: this thread's 16-byte slot in chunk 0 of the A tile; chunk ch is at dst + ch * lbo
-__device__ __forceinline__ void dequant_store(int type, const RawKB& r, int k0, uint8_t* dst, uint32_t lbo) {
-    auto put = [&](int ch, const uint4& v) { *reinterpret_cast<uint4*>(dst + ch * lbo) = v; };
+// the 64 weights of the block -> f16 in order of k
+__device__ __forceinline__ void dequant_block(int type, const RawKB& r, int k0, uint32_t (&out)[32]) {
+    auto put = [&](int ch, const uint4& v) { out[4 * ch] = v.x; out[4 * ch + 1] = v.y; out[4 * ch + 2] = v.z; out[4 * ch + 3] = v.w; };
     if (type == T_Q4_K || type == T_Q5_K) {
         const int c = (k0 & 255) >> 6;                                 // 64-chunk: sub-blocks 2c (low nibbles), 2c+1 (high)
         const uint32_t sh = (c & 1) * 16, w0 = r.w[1] >> sh, w1 = r.w[2] >> sh, w2 = r.w[3] >> sh;
@@ -268,20 +296,13 @@ __device__ __forceinline__ void dequant_store(int type, const RawKB& r, int k0, 
 // 64 weights of a K block straight from global memory, one f16 rounding per weight like the fast paths. Slow per weight
 // (byte loads), but it keeps prompts and batched steps of such models on the tensor cores instead of token by token.
 constexpr int T_GENERIC = -1;
-__device__ __forceinline__ void dequant_store_generic(int type, const uint8_t* row, int k0, uint8_t* dst, uint32_t lbo) {
+__device__ __forceinline__ void dequant_block_generic(int type, const uint8_t* row, int k0, uint32_t (&out)[32]) {
     const int be = block_elems(type), bb = block_bytes(type);
-#pragma unroll 1
-    for (int ch = 0; ch < 8; ch++) {
-        uint32_t h[4];
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int e0 = k0 + 8 * ch + 2 * j, e1 = e0 + 1;
-            const float a = dequant_elem(type, row + (size_t)(e0 / be) * bb, e0 % be);
-            const float b = dequant_elem(type, row + (size_t)(e1 / be) * bb, e1 % be);
-            const __half2 v = __floats2half2_rn(a, b);
-            h[j] = *reinterpret_cast<const uint32_t*>(&v);
-        }
-        *reinterpret_cast<uint4*>(dst + ch * lbo) = make_uint4(h[0], h[1], h[2], h[3]);
+    for (int ch = 0; ch < 32; ch++) {
+        const int e0 = k0 + 2 * ch, e1 = e0 + 1;
+        const __half2 v = __floats2half2_rn(dequant_elem(type, row + (size_t)(e0 / be) * bb, e0 % be), dequant_elem(type, row + (size_t)(e1 / be) * bb, e1 % be));
+        out[ch] = *reinterpret_cast<const uint32_t*>(&v);
     }
 }
 
@@ -289,6 +310,7 @@ struct GemmBars {
     uint64_t a_full[GM_MAX_STAGES], empty[GM_MAX_STAGES];
     uint64_t b_full[GM_MAX_BSTAGES], b_empty[GM_MAX_BSTAGES];
     uint64_t raw_full[GM_RAW_STAGES], raw_empty[GM_RAW_STAGES];
+    uint64_t done;                      // all products
     uint32_t tmem_base;
 };
 static_assert(sizeof(GemmBars) <= GM_HDR, "barrier header");
@@ -327,35 +349,60 @@ __device__ __forceinline__ void span_block(int type, const uint32_t (&W)[GM_SPAN
 
 struct DeqCtx {
     GemmBars* sh;
-    uint8_t* stage0;
     const uint8_t* raw0;
     const uint8_t* wrow;
-    int S, NR, tid, n, n_sp, sp0, kb0, use_tma, span_bytes, type;
-    uint32_t raw_stage_bytes, box, a_bytes, lbo_a;      // weight tile: rows * 128 B per stage, rows * 16 B between K chunks
+    int S, NR, row, n, n_sp, sp0, kb0, use_tma, span_bytes, type;
+    uint8_t* stage0;                                    // SS: this thread's 16 bytes of the first chunk of stage 0
+    uint32_t raw_stage_bytes, box, tmem_a;              // tmem_a: this thread's lane, first column of its rows in stage 0
     unsigned int* err;
     long long* dbg;
 };
 
-template <int TYPE>
+// blocks 2 GRP and 2 GRP + 1 of every four
+template <bool SS, int TYPE, int GRP>
 __device__ __noinline__ void deq_loop(const DeqCtx cx) {
     GemmBars& sh = *cx.sh;
-    const uint32_t a_bytes = cx.a_bytes, lbo_a = cx.lbo_a;
+    const int lane = threadIdx.x & 31;
     int st = 0;                 // A stage of the next block and how often the ring has wrapped
     uint32_t wraps = 0;
-    auto emit = [&](const RawKB& r, int i) {               // block i of this CTA's range -> A tile of its stage
+    // past the other group's two blocks. With four stages each group has two of its own; with another number it meets a stage whose barrier
+    // has moved on two phases, which a parity does not tell from none, so the phase between is waited for as well.
+    auto skip = [&]() {
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            if (cx.S % 4 && wraps > 0) mbar_wait(&sh.empty[st], (wraps - 1) & 1, cx.err, 0x40008u, (unsigned)st);
+            if (++st == cx.S) { st = 0; wraps++; }
+        }
+    };
+    if (GRP) skip();
+    auto emit = [&](const RawKB& r, int i) {               // block i of this CTA's range -> its stage in tensor memory
+        uint32_t out[32];
+        if (TYPE == T_GENERIC) dequant_block_generic(cx.type, cx.wrow, (cx.kb0 + i) * GM_BK, out);
+        else dequant_block(TYPE, r, (i & 3) * GM_BK, out);
         if (cx.dbg && i < 64) cx.dbg[i * 8 + 0] = clock64();
         if (wraps > 0) mbar_wait(&sh.empty[st], (wraps - 1) & 1, cx.err, 0x40001u, (unsigned)i);   // MMAs that read the stage are done
         if (cx.dbg && i < 64) cx.dbg[i * 8 + 1] = clock64();
-        if (TYPE == T_GENERIC) dequant_store_generic(cx.type, cx.wrow, (cx.kb0 + i) * GM_BK, cx.stage0 + (size_t)st * a_bytes + cx.tid * 16, lbo_a);
-        else dequant_store(TYPE, r, (i & 3) * GM_BK, cx.stage0 + (size_t)st * a_bytes + cx.tid * 16, lbo_a);
-        fence_proxy_async();            // generic-proxy writes -> visible to the tensor core (async proxy)
-        mbar_arrive(&sh.a_full[st]);
+        if constexpr (SS) {
+            uint8_t* dst = cx.stage0 + (size_t)st * GM_ABYTES;
+#pragma unroll
+            for (int ch = 0; ch < 8; ch++)
+                *reinterpret_cast<uint4*>(dst + ch * GM_ROWS * 16) = make_uint4(out[4 * ch], out[4 * ch + 1], out[4 * ch + 2], out[4 * ch + 3]);
+            fence_proxy_async();        // generic-proxy writes -> visible to the tensor core (async proxy)
+        } else {
+            __syncwarp();
+            tc_fence_after();
+            tmem_st32(cx.tmem_a + st * GM_BK, out);      // (a stage: GM_BK / 2 columns for each half of the rows)
+            tc_fence_before();
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh.a_full[st]);      // once per warp: the arrivals of 32 lanes go one after the other
         if (cx.dbg && i < 64) cx.dbg[i * 8 + 2] = clock64();
         if (++st == cx.S) { st = 0; wraps++; }
+        if (i & 1) skip();
     };
     if (TYPE == T_GENERIC) {
         RawKB none;
-        for (int i = 0; i < cx.n; i++) emit(none, i);
+        for (int i = 2 * GRP; i < cx.n; i += 4) { emit(none, i); emit(none, i + 1); }
     } else if (cx.use_tma) {
         // raw spans arrive in shared memory by TMA; this thread's row is one box row. The box starts at the 16-byte
         // boundary below the span (TMA needs it); only Q6_K spans (210 B) can be off it.
@@ -367,7 +414,7 @@ __device__ __noinline__ void deq_loop(const DeqCtx cx) {
             if (cx.dbg && sp < 16) cx.dbg[sp * 4 * 8 + 6] = clock64();
             mbar_wait(&sh.raw_full[rs], rwraps & 1, cx.err, 0x40006u, (unsigned)sp);
             if (cx.dbg && sp < 16) cx.dbg[sp * 4 * 8 + 7] = clock64();
-            const uint8_t* slot = cx.raw0 + (size_t)rs * cx.raw_stage_bytes + (size_t)cx.tid * cx.box;
+            const uint8_t* slot = cx.raw0 + (size_t)rs * cx.raw_stage_bytes + (size_t)cx.row * cx.box;
             uint32_t W[GM_SPAN_WORDS];
 #pragma unroll
             for (int j = 0; j < n16; j++) {
@@ -375,7 +422,8 @@ __device__ __noinline__ void deq_loop(const DeqCtx cx) {
                 W[4 * j] = v.x; W[4 * j + 1] = v.y; W[4 * j + 2] = v.z; W[4 * j + 3] = v.w;
             }
             fence_proxy_async();                           // these generic-proxy reads before the TMA (async proxy) rewrite
-            mbar_arrive(&sh.raw_empty[rs]);                // the span is in registers: the stage can be refilled
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh.raw_empty[rs]); // the span is in registers: the stage can be refilled
             if (++rs == cx.NR) { rs = 0; rwraps++; }
             if (TYPE == T_Q6_K) {                          // shift the 53 words of the span down by its misalignment (0,2,..14 bytes)
                 const uint32_t mis = ((uint32_t)(cx.sp0 + sp) * 210u) & 15u, sh16 = (mis & 2u) * 8u;
@@ -399,50 +447,43 @@ __device__ __noinline__ void deq_loop(const DeqCtx cx) {
                 }
             }
             RawKB r;
-            span_block<0>(TYPE, W, r); emit(r, sp * 4 + 0);
-            span_block<1>(TYPE, W, r); emit(r, sp * 4 + 1);
-            span_block<2>(TYPE, W, r); emit(r, sp * 4 + 2);
-            span_block<3>(TYPE, W, r); emit(r, sp * 4 + 3);
+            span_block<2 * GRP>(TYPE, W, r); emit(r, sp * 4 + 2 * GRP);
+            span_block<2 * GRP + 1>(TYPE, W, r); emit(r, sp * 4 + 2 * GRP + 1);
         }
     } else {
         // rows that are not 16-byte multiples (Q6_K with K % 2048 != 0): direct loads, next block prefetched in registers
         RawKB cur, nxt;
-        load_raw(TYPE, cx.wrow, cx.kb0 * GM_BK, cur);
-        for (int i = 0; i < cx.n; i++) {
-            if (i + 1 < cx.n) load_raw(TYPE, cx.wrow, (cx.kb0 + i + 1) * GM_BK, nxt);
+        load_raw(TYPE, cx.wrow, (cx.kb0 + 2 * GRP) * GM_BK, cur);
+        for (int i = 2 * GRP; i < cx.n;) {
+            const int next = i + (i & 1 ? 3 : 1);
+            if (next < cx.n) load_raw(TYPE, cx.wrow, (cx.kb0 + next) * GM_BK, nxt);
             emit(cur, i);
             cur = nxt;
+            i = next;
         }
     }
 }
 
-// ROWS weight rows per CTA, ROWS / 32 dequantising warps + 3 service warps.
-// SWAP = false (T > 128): weights are the MMA's A operand (M = 128 rows = TMEM lanes), tokens its N (TMEM columns).
-//   ROWS = 256 (T > 256): two M halves over the same tokens, half of the step's tokens a CTA. With 128 rows and all 512 tokens a block of
-//   64 K entries brought 64 KB of activations for 1024 cycles of products, and the 148 CTAs together asked more of L2 than it gives;
-//   now a CTA brings 32 KB for the same products (and expands twice the weights, which the idle issue slots have room for).
-// SWAP = true  (T <= 128): tokens are the A operand (M = 128, rows past T are don't-care), 256 weight rows are the N:
-//   with few tokens an instruction costs ~130 cycles whatever N is (measured), so each MMA should cover as many
-//   weight rows as an instruction can: 256.
-template <int ROWS, bool SWAP>
-__global__ void __launch_bounds__((ROWS / 32 + 3) * 32) gemm_q_kernel(const __grid_constant__ GemmParams p) {
-    constexpr int DW = ROWS / 32;          // dequantising warps; then: MMA warp, weight producer, activation producer
+// SS: expanded weights in shared memory (K-major core matrices like the activations), T up to 256. Above 256 tokens tensor memory cannot hold
+// two halves of 256 sums and weights as well, and three narrower token tiles lose more than they save: 112 row tiles x 3 are 2.3 waves
+// (512 tokens, the four products of a layer of 4096: 304 us, this form 251; 128 rows and all tokens a CTA before: 290).
+template <bool SS>
+__global__ void __launch_bounds__(GM_THREADS) gemm_q_kernel(const __grid_constant__ GemmParams p) {
+    constexpr int DW = GM_DW, ROWS = GM_ROWS;      // dequantising warps; then: MMA warp, weight producer, activation producer
     extern __shared__ __align__(128) uint8_t smem_raw[];
     GemmBars& sh = *reinterpret_cast<GemmBars*>(smem_raw);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    constexpr bool WIDE = !SWAP && ROWS == 256;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;      // (warp: known to be uniform)
     const int S = p.n_stages, SB = p.n_bstages;
-    const int n_tt = WIDE ? p.n_tt : 1, tt = WIDE ? blockIdx.x / p.n_splits % n_tt : 0;
-    const int t_base = tt * p.t_tile, T = min(p.t_tile, p.T_pad - t_base);      // this CTA's tokens
-    const uint32_t a_bytes = ROWS * GM_BK * 2, b_bytes = (uint32_t)T * GM_BK * 2;
-    uint8_t* stage0 = smem_raw + GM_HDR;                               // A tiles: S x 16 KB
-    uint8_t* bst0 = stage0 + (size_t)S * a_bytes;                      // activation tiles: SB x T*128 B
-    uint8_t* raw0 = bst0 + (size_t)SB * b_bytes;                       // raw weight spans: n_raw x [128][box]
-    uint32_t ncols = 32;
-    while ((int)ncols < (SWAP ? ROWS : WIDE ? 2 * T : T)) ncols <<= 1;
+    const int tt = blockIdx.x / p.n_splits % p.n_tt, t_base = tt * p.t_tile, T = min(p.t_tile, p.T_pad - t_base);      // this CTA's tokens
+    const uint32_t b_bytes = (uint32_t)T * GM_BK * 2;
+    uint8_t* stage0 = smem_raw + GM_HDR;                               // SS: expanded weight blocks, S x 32 KB
+    uint8_t* bst0 = stage0 + (SS ? S * GM_ABYTES : 0);                 // activation tiles: SB x T*128 B
+    uint8_t* raw0 = bst0 + (size_t)SB * b_bytes;                       // raw weight spans: n_raw x [256][box]
+    uint32_t ncols = 32;                                               // two halves of T sums, S stages of 2 x GM_BK / 2 columns
+    while ((int)ncols < 2 * T + (SS ? 0 : S * GM_BK)) ncols <<= 1;
 
     // ---- which tile / K range (in 256-weight spans = 4 blocks)
-    const int split = blockIdx.x % p.n_splits, tile_g = blockIdx.x / p.n_splits / n_tt;
+    const int split = blockIdx.x % p.n_splits, tile_g = blockIdx.x / p.n_splits / p.n_tt;
     int seg = 0;
     while (seg + 1 < p.nseg && tile_g >= p.seg[seg + 1].tile0) seg++;
     const GemmSeg& sg = p.seg[seg];
@@ -454,9 +495,10 @@ __global__ void __launch_bounds__((ROWS / 32 + 3) * 32) gemm_q_kernel(const __gr
 
     if (warp == DW) {
         if (lane == 0) {
-            for (int i = 0; i < S; i++) { mbar_init(&sh.a_full[i], ROWS); mbar_init(&sh.empty[i], 1); }
+            for (int i = 0; i < S; i++) { mbar_init(&sh.a_full[i], DW / 2); mbar_init(&sh.empty[i], 1); }
             for (int i = 0; i < SB; i++) { mbar_init(&sh.b_full[i], 1); mbar_init(&sh.b_empty[i], 1); }
-            for (int i = 0; i < GM_RAW_STAGES; i++) { mbar_init(&sh.raw_full[i], 1); mbar_init(&sh.raw_empty[i], ROWS); }
+            for (int i = 0; i < GM_RAW_STAGES; i++) { mbar_init(&sh.raw_full[i], 1); mbar_init(&sh.raw_empty[i], DW); }
+            mbar_init(&sh.done, 1);
             fence_mbar_init();
         }
         __syncwarp();
@@ -471,97 +513,94 @@ __global__ void __launch_bounds__((ROWS / 32 + 3) * 32) gemm_q_kernel(const __gr
     griddep_launch();
     const uint32_t tmem = sh.tmem_base;
     // K-major, no swizzle: element (r, k) of a tile with R rows sits at (k/8) * (R*16) + r*16 + (k%8)*2
-    const uint32_t lbo_a = ROWS * 16, lbo_b = (uint32_t)T * 16, sbo = 128;
+    const uint32_t lbo_b = (uint32_t)T * 16, sbo = 128, tmem_a0 = tmem + 2 * T;
 
     if (warp < DW) {
-        // ================= dequantising threads: thread <-> weight row. One instantiation per quant type keeps the
+        // ================= dequantising threads: two per weight row. One instantiation per quant type keeps the
         // loop a CTA actually runs small enough for the instruction cache (all five inlined make a very large loop body).
         DeqCtx cx;
-        cx.sh = &sh; cx.stage0 = stage0; cx.raw0 = raw0; cx.S = S; cx.NR = NR; cx.raw_stage_bytes = raw_stage_bytes; cx.box = box;
-        cx.tid = tid; cx.n = n; cx.n_sp = n_sp; cx.sp0 = sp0; cx.kb0 = kb0; cx.err = p.err; cx.a_bytes = a_bytes; cx.lbo_a = lbo_a;
+        cx.sh = &sh; cx.raw0 = raw0; cx.S = S; cx.NR = NR; cx.raw_stage_bytes = raw_stage_bytes; cx.box = box;
+        const int row_in = tid % ROWS;
+        cx.tmem_a = tmem_a0 + ((uint32_t)((warp & 3) * 32) << 16) + (row_in / GM_BM) * (GM_BK / 2);
+        cx.stage0 = stage0 + row_in * 16;
+        cx.row = row_in; cx.n = n; cx.n_sp = n_sp; cx.sp0 = sp0; cx.kb0 = kb0; cx.err = p.err;
         cx.dbg = (p.dbg && blockIdx.x == 0 && tid == 0) ? p.dbg : nullptr;
         cx.use_tma = sg.use_tma; cx.span_bytes = sg.span_bytes; cx.type = sg.type;
-        cx.wrow = sg.w + (size_t)min(m0 + tid, sg.n_rows - 1) * sg.row_bytes;      // rows past N are computed and dropped
-        switch (sg.type) {
-            case T_Q4_K: deq_loop<T_Q4_K>(cx); break;
-            case T_Q5_K: deq_loop<T_Q5_K>(cx); break;
-            case T_Q6_K: deq_loop<T_Q6_K>(cx); break;
-            case T_Q8_0: deq_loop<T_Q8_0>(cx); break;
-            case T_Q4_0: deq_loop<T_Q4_0>(cx); break;
-            default: deq_loop<T_GENERIC>(cx); break;
+        cx.wrow = sg.w + (size_t)min(m0 + row_in, sg.n_rows - 1) * sg.row_bytes;      // rows past N are computed and dropped
+        if (tid < ROWS) switch (sg.type) {
+            case T_Q4_K: deq_loop<SS, T_Q4_K, 0>(cx); break;
+            case T_Q5_K: deq_loop<SS, T_Q5_K, 0>(cx); break;
+            case T_Q6_K: deq_loop<SS, T_Q6_K, 0>(cx); break;
+            case T_Q8_0: deq_loop<SS, T_Q8_0, 0>(cx); break;
+            case T_Q4_0: deq_loop<SS, T_Q4_0, 0>(cx); break;
+            default: deq_loop<SS, T_GENERIC, 0>(cx); break;
+        } else switch (sg.type) {
+            case T_Q4_K: deq_loop<SS, T_Q4_K, 1>(cx); break;
+            case T_Q5_K: deq_loop<SS, T_Q5_K, 1>(cx); break;
+            case T_Q6_K: deq_loop<SS, T_Q6_K, 1>(cx); break;
+            case T_Q8_0: deq_loop<SS, T_Q8_0, 1>(cx); break;
+            case T_Q4_0: deq_loop<SS, T_Q4_0, 1>(cx); break;
+            default: deq_loop<SS, T_GENERIC, 1>(cx); break;
         }
         // ================= epilogue
-        const int last = n - 1;
-        mbar_wait(&sh.empty[last % S], (last / S) & 1, p.err, 0x40002u, (unsigned)last);
+        mbar_wait(&sh.done, 0, p.err, 0x40002u, (unsigned)n);
+        __syncwarp();
         tc_fence_after();
         griddep_wait();
-        if (!SWAP) {                               // TMEM lane = weight row, columns = tokens
-            const int row = m0 + tid;
-            const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(warp >> 2) * (ncols / 2);
-            float* ybase = p.y + (size_t)split * p.split_stride + (size_t)t_base * p.ldy + sg.out_off + row;
-            for (int c0 = 0; c0 < T; c0 += 16) {
-                float v[16];
-                tmem_ld16(lane_addr + c0, v);
-                if (row < sg.n_rows) {
+        const int row = m0 + row_in;                // TMEM lane = weight row, columns = tokens; the two threads of a row take every other 16
+        const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(row_in / GM_BM) * T;
+        float* ybase = p.y + (size_t)split * p.split_stride + (size_t)t_base * p.ldy + sg.out_off + row;
+        for (int c0 = 16 * (tid / ROWS); c0 < T; c0 += 32) {
+            float v[16];
+            tmem_ld16(lane_addr + c0, v);
+            if (row < sg.n_rows) {
 #pragma unroll
-                    for (int j = 0; j < 16; j++)
-                        if (t_base + c0 + j < p.T) ybase[(size_t)(c0 + j) * p.ldy] = v[j];
-                }
-            }
-        } else if (warp < 4 && warp * 32 < p.T) {  // TMEM lane = token (warps 0-3 own the 128 lanes), columns = weight rows
-            const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
-            float* yrow = p.y + (size_t)split * p.split_stride + (size_t)tid * p.ldy + sg.out_off + m0;
-            const int n_valid = min(ROWS, sg.n_rows - m0);
-            for (int c0 = 0; c0 < ROWS; c0 += 16) {
-                float v[16];
-                tmem_ld16(lane_addr + c0, v);      // warp-wide: every lane takes part, only tokens < T store
-                if (tid < p.T) {
-                    if (c0 + 16 <= n_valid) {
-#pragma unroll
-                        for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4*>(yrow + c0 + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 16; j++) if (c0 + j < n_valid) yrow[c0 + j] = v[j];
-                    }
-                }
+                for (int j = 0; j < 16; j++)
+                    if (t_base + c0 + j < p.T) ybase[(size_t)(c0 + j) * p.ldy] = v[j];
             }
         }
-    } else if (warp == DW && lane == 0) {
-        // ================= MMA thread
-        const uint32_t idesc_lo = SWAP ? instr_desc(128, ROWS) : instr_desc(GM_BM, T > 256 ? 256 : T);
-        const uint32_t idesc_hi = (!SWAP && T > 256) ? instr_desc(GM_BM, T - 256) : 0u;
+    } else if (warp == DW) {
+        // ================= MMA warp. All lanes run the loop, one issues: descriptors and counters then live in uniform registers, where
+        // the instructions take them from (with a loop of one lane each product was preceded by moves there)
+        const uint32_t idesc = instr_desc(GM_BM, T);
         int s = 0, sb = 0;
         uint32_t use = 0, useb = 0;
-        const uint32_t a_lo0 = (smem_u32(stage0) >> 4) | ((lbo_a >> 4) << 16), b_lo0 = (smem_u32(bst0) >> 4) | ((lbo_b >> 4) << 16);
+        const uint32_t b_lo0 = (smem_u32(bst0) >> 4) | ((lbo_b >> 4) << 16), a_lo0 = (smem_u32(stage0) >> 4) | (uint32_t)GM_ROWS << 16;
         const uint32_t desc_hi = (sbo >> 4) | (1u << 14);          // SBO, descriptor version 1, no swizzle
+        const bool dbg = p.dbg && blockIdx.x == 0 && lane == 0;
         for (int i = 0; i < n; i++) {
             mbar_wait(&sh.b_full[sb], useb & 1, p.err, 0x40003u, (unsigned)i);
-            if (p.dbg && blockIdx.x == 0 && i < 64) p.dbg[i * 8 + 3] = clock64();
+            if (dbg && i < 64) p.dbg[i * 8 + 3] = clock64();
             mbar_wait(&sh.a_full[s], use & 1, p.err, 0x40004u, (unsigned)i);
-            if (p.dbg && blockIdx.x == 0 && i < 64) p.dbg[i * 8 + 4] = clock64();
+            if (dbg && i < 64) p.dbg[i * 8 + 4] = clock64();
+            __syncwarp();
             tc_fence_after();
             // descriptors differ only in the 14-bit start-address field (units of 16 B): add, do not rebuild
-            const uint32_t a_lo = a_lo0 + (uint32_t)s * (a_bytes >> 4), b_lo = b_lo0 + (uint32_t)sb * (b_bytes >> 4);
+            const uint32_t a_at = tmem_a0 + (uint32_t)s * GM_BK, b_lo = b_lo0 + (uint32_t)sb * (b_bytes >> 4);
+            if (elect_one()) {
 #pragma unroll
-            for (int ks = 0; ks < GM_BK / 16; ks++) {
-                const uint64_t da = desc_join(a_lo + ks * (2 * lbo_a >> 4), desc_hi);
-                const uint64_t db = desc_join(b_lo + ks * (2 * lbo_b >> 4), desc_hi);
-                const uint32_t acc = (i > 0 || ks > 0) ? 1u : 0u;
-                if (SWAP) {
-                    umma_f16(tmem, db, da, idesc_lo, acc);          // A = tokens (rows past T read whatever follows: dropped), B = weights
-                } else {
-                    umma_f16(tmem, da, db, idesc_lo, acc);
-                    if (WIDE) umma_f16(tmem + ncols / 2, desc_join(a_lo + ks * (2 * lbo_a >> 4) + GM_BM, desc_hi), db, idesc_lo, acc);      // rows 128 ..
-                    else if (T > 256) umma_f16(tmem + 256, da, desc_join(b_lo + ks * (2 * lbo_b >> 4) + 256, desc_hi), idesc_hi, acc);
+                for (int ks = 0; ks < GM_BK / 16; ks++) {
+                    const uint64_t db = desc_join(b_lo + ks * (2 * lbo_b >> 4), desc_hi);
+                    const uint32_t acc = (i > 0 || ks > 0) ? 1u : 0u;
+                    if constexpr (SS) {
+                        const uint32_t at = a_lo0 + (uint32_t)s * (GM_ABYTES >> 4) + ks * (2 * GM_ROWS);
+                        umma_f16_ss(tmem, desc_join(at, desc_hi), db, idesc, acc);
+                        umma_f16_ss(tmem + T, desc_join(at + GM_BM, desc_hi), db, idesc, acc);      // rows 128 ..
+                    } else {
+                        umma_f16(tmem, a_at + ks * 8, db, idesc, acc);
+                        umma_f16(tmem + T, a_at + GM_BK / 2 + ks * 8, db, idesc, acc);
+                    }
                 }
+                umma_commit(&sh.empty[s]);      // both arrive when the MMAs above have finished reading their tiles
+                umma_commit(&sh.b_empty[sb]);
+                if (i + 1 == n) umma_commit(&sh.done);
             }
-            umma_commit(&sh.empty[s]);      // both arrive when the MMAs above have finished reading their tiles
-            umma_commit(&sh.b_empty[sb]);
-            if (p.dbg && blockIdx.x == 0 && i < 64) p.dbg[i * 8 + 5] = clock64();
+            __syncwarp();
+            if (dbg && i < 64) p.dbg[i * 8 + 5] = clock64();
             if (++s == S) { s = 0; use++; }
             if (++sb == SB) { sb = 0; useb++; }
         }
-    } else if (warp == DW + 2 && lane == 0) {
+    } else if (warp == DW + 2) {
         // ================= activation producer: the tile of a block is one contiguous 1-D bulk copy (operand order in HBM)
         const uint8_t* xb = reinterpret_cast<const uint8_t*>(p.x);
         int sb = 0;
@@ -569,24 +608,34 @@ __global__ void __launch_bounds__((ROWS / 32 + 3) * 32) gemm_q_kernel(const __gr
         griddep_wait();                 // the activations come from the previous kernel
         for (int i = 0; i < n; i++) {
             if (useb > 0) mbar_wait(&sh.b_empty[sb], (useb - 1) & 1, p.err, 0x40005u, (unsigned)i);
-            mbar_arrive_expect_tx(&sh.b_full[sb], b_bytes);
-            if (WIDE) {                 // part of the tokens: one run per chunk of 8 K entries
-                for (int c = 0; c < GM_BK / 8; c++)
-                    tma_load_1d(bst0 + (size_t)sb * b_bytes + (size_t)c * lbo_b, xb + ((size_t)((kb0 + i) * (GM_BK / 8) + c) * p.T_pad + t_base) * 16, lbo_b, &sh.b_full[sb]);
-            } else {
-                tma_load_1d(bst0 + (size_t)sb * b_bytes, xb + (size_t)(kb0 + i) * b_bytes, b_bytes, &sh.b_full[sb]);
+            __syncwarp();
+            uint8_t* dst = bst0 + (size_t)sb * b_bytes;
+            if (elect_one()) {
+                mbar_arrive_expect_tx(&sh.b_full[sb], b_bytes);
+                if (p.n_tt > 1) {       // part of the tokens: one run per chunk of 8 K entries
+#pragma unroll
+                    for (int c = 0; c < GM_BK / 8; c++)
+                        tma_load_1d(dst + (size_t)c * lbo_b, xb + ((size_t)((kb0 + i) * (GM_BK / 8) + c) * p.T_pad + t_base) * 16, lbo_b, &sh.b_full[sb]);
+                } else {
+                    tma_load_1d(dst, xb + (size_t)(kb0 + i) * b_bytes, b_bytes, &sh.b_full[sb]);
+                }
             }
+            __syncwarp();
             if (++sb == SB) { sb = 0; useb++; }
         }
-    } else if (warp == DW + 1 && lane == 0 && sg.use_tma) {
-        // ================= weight producer: one 2-D TMA box (128 rows x one 256-weight span) per stage
+    } else if (warp == DW + 1 && sg.use_tma) {
+        // ================= weight producer: one 2-D TMA box (256 rows x one 256-weight span) per stage
         const void* tmap = &sg.tmap;
         int rs = 0;
         uint32_t ruse = 0;
         for (int sp = 0; sp < n_sp; sp++, rs = (rs + 1 == NR ? 0 : rs + 1), ruse += (rs == 0)) {
             if (ruse > 0) mbar_wait(&sh.raw_empty[rs], (ruse - 1) & 1, p.err, 0x40007u, (unsigned)sp);
-            mbar_arrive_expect_tx(&sh.raw_full[rs], raw_stage_bytes);
-            tma_load_2d(raw0 + (size_t)rs * raw_stage_bytes, tmap, (int)((((size_t)(sp0 + sp) * sg.span_bytes) & ~(size_t)15) >> 1), m0, &sh.raw_full[rs]);
+            __syncwarp();
+            if (elect_one()) {
+                mbar_arrive_expect_tx(&sh.raw_full[rs], raw_stage_bytes);
+                tma_load_2d(raw0 + (size_t)rs * raw_stage_bytes, tmap, (int)((((size_t)(sp0 + sp) * sg.span_bytes) & ~(size_t)15) >> 1), m0, &sh.raw_full[rs]);
+            }
+            __syncwarp();
         }
     }
     tc_fence_before();
@@ -595,16 +644,13 @@ __global__ void __launch_bounds__((ROWS / 32 + 3) * 32) gemm_q_kernel(const __gr
 }
 
 // ---------------------------------------------------------------- host side
-static int gemm_rows(const GemmParams& p) { return p.swap || p.n_tt > 1 ? 256 : GM_BM; }
 static size_t gemm_raw_bytes(const GemmParams& p) {
     size_t m = 0;
-    for (int s = 0; s < p.nseg; s++) if (p.seg[s].use_tma) m = std::max(m, (size_t)p.n_raw * gemm_rows(p) * p.seg[s].box_bytes);
+    for (int s = 0; s < p.nseg; s++) if (p.seg[s].use_tma) m = std::max(m, (size_t)p.n_raw * GM_ROWS * p.seg[s].box_bytes);
     return m;
 }
 size_t gemm_smem_bytes(const GemmParams& p) {
-    // swap: the MMA reads 128 token rows per K chunk whatever T is; the rows past the tile must still be shared memory
-    return GM_HDR + (size_t)p.n_stages * gemm_rows(p) * GM_BK * 2 + (size_t)p.n_bstages * p.t_tile * GM_BK * 2 + gemm_raw_bytes(p) +
-           (p.swap ? 4096 : 0);
+    return GM_HDR + (size_t)(p.ss ? p.n_stages * GM_ABYTES : 0) + (size_t)p.n_bstages * p.t_tile * GM_BK * 2 + gemm_raw_bytes(p);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -621,11 +667,9 @@ cudaError_t gemm_init() {
         if (qres != cudaDriverEntryPointSuccess || !fn) return cudaErrorNotSupported;
         g_encode = (EncodeTiledFn)fn;
     }
-    cudaError_t e = cudaFuncSetAttribute(gemm_q_kernel<GM_BM, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaError_t e = cudaFuncSetAttribute(gemm_q_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(gemm_q_kernel<256, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(gemm_q_kernel<256, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    return cudaFuncSetAttribute(gemm_q_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
 }
 
 // Fill tile ranges, tensor maps, the stage count and the K split. n_sms: SMs to fill; max_splits: what the partial
@@ -635,10 +679,10 @@ int gemm_plan(GemmParams& p, int n_sms, int max_splits) {
     if (p.nseg < 1 || p.nseg > 3 || p.K <= 0 || p.K % 256) return -1;
     if (p.T < 1 || p.T > 512) return -2;
     p.T_pad = (p.T + 15) / 16 * 16;
-    p.swap = (p.T_pad <= 128 && !getenv("B2_GEMM_NOSWAP")) ? 1 : 0;
-    p.n_tt = p.T_pad > 256 ? 2 : 1;
-    p.t_tile = p.n_tt == 1 ? p.T_pad : (p.T_pad / 2 + 15) / 16 * 16;
-    const int ROWS = gemm_rows(p);
+    p.ss = p.T_pad > 256 ? 1 : 0;
+    p.n_tt = p.T_pad <= 128 ? 1 : 2;
+    p.t_tile = ((p.T_pad + p.n_tt - 1) / p.n_tt + 15) / 16 * 16;
+    const int ROWS = GM_ROWS;
     int tiles = 0;
     const bool no_tma = getenv("B2_GEMM_NO_TMA") != nullptr;
     for (int s = 0; s < p.nseg; s++) {
@@ -668,36 +712,33 @@ int gemm_plan(GemmParams& p, int n_sms, int max_splits) {
         }
     }
     p.n_tiles = tiles;
-    const size_t a_st = (size_t)ROWS * GM_BK * 2, b_st = (size_t)p.t_tile * GM_BK * 2;
-    const size_t cap = 227 * 1024 - 1024;
+    const size_t b_st = (size_t)p.t_tile * GM_BK * 2, cap = 227 * 1024 - 1024;
     // activation ring: deep when the tiles are small (their TMA latency must not gate the MMAs)
-    int SB = p.T_pad <= 32 ? 8 : p.T_pad <= 64 ? 6 : p.T_pad <= 128 ? 4 : 3;
-    int S = p.swap ? 3 : (p.T_pad <= 64 || p.n_tt > 1 ? 2 : 3);
-    int per_sm = (!p.swap && p.T_pad <= 64) ? 2 : 1;   // 128-row variant at small T: two CTAs per SM
-    if (const char* v = getenv("B2_GEMM_PER_SM")) if (atoi(v) > 0) per_sm = atoi(v);
-    if (const char* v = getenv("B2_GEMM_STAGES")) if (atoi(v) > 1) S = atoi(v);
-    if (const char* v = getenv("B2_GEMM_BSTAGES")) if (atoi(v) > 1) SB = atoi(v);
-    if (S > GM_MAX_STAGES) S = GM_MAX_STAGES;
-    if (SB > GM_MAX_BSTAGES) SB = GM_MAX_BSTAGES;
+    int SB = p.t_tile <= 64 ? 8 : p.ss ? 3 : 6, S = p.ss ? 2 : 4;
+    if (const char* v = getenv("B2_GEMM_STAGES")) if (atoi(v) > 1) S = std::min(atoi(v), p.ss ? 3 : 4);
+    if (const char* v = getenv("B2_GEMM_BSTAGES")) if (atoi(v) > 1) SB = std::min(atoi(v), GM_MAX_BSTAGES);
     p.n_raw = GM_RAW_STAGES;
     if (const char* v = getenv("B2_GEMM_RAW")) if (atoi(v) == 1) p.n_raw = 1;
-    const size_t budget = per_sm > 1 ? (228 * 1024) / per_sm - 1024 : cap;
-    auto total = [&]() { return GM_HDR + S * a_st + SB * b_st + gemm_raw_bytes(p) + (p.swap ? 4096 : 0); };
-    if (total() > budget && p.n_raw > 1) p.n_raw = 1;
-    while (total() > budget && SB > 2) SB--;
-    while (total() > budget && S > 2) S--;
-    if (total() > budget && per_sm > 1) per_sm = 1;
+    auto total = [&]() { return GM_HDR + (p.ss ? (size_t)S * GM_ABYTES : 0) + SB * b_st + gemm_raw_bytes(p); };
+    while (total() > cap && SB > 3) SB--;
+    if (total() > cap) p.n_raw = 1;
+    while (total() > cap && SB > 2) SB--;
+    while (total() > cap && S > 2) S--;
     if (total() > cap) { for (int s = 0; s < p.nseg; s++) p.seg[s].use_tma = 0; }
     if (total() > cap) return -4;
     p.n_stages = S; p.n_bstages = SB;
-    const int slots = n_sms * per_sm;
+    // The K split depends on the matrices and T alone, in units of the tiles that the sums were first split for (256 rows up to 128 tokens, 128
+    // above): the order of every sum is part of the results.
+    int split_tiles = 0;
+    for (int s = 0; s < p.nseg; s++) split_tiles += (p.seg[s].n_rows + (p.T_pad <= 128 ? 256 : 128) - 1) / (p.T_pad <= 128 ? 256 : 128);
+    const int slots = n_sms;
     const int n_sp = p.K / 256;
     // choose the K split that minimises (waves) x (blocks per CTA + fixed cost), fixed cost ~ epilogue + ramp
     const int fixed = 6 + p.T_pad / 32;
     long best_cost = -1;
     int best = 1;
     for (int s = 1; s <= max_splits && s <= 16 && s <= n_sp; s++) {
-        const long waves = ((long)tiles * p.n_tt * s + slots - 1) / slots;
+        const long waves = ((long)split_tiles * s + slots - 1) / slots;
         const long cost = waves * (4 * ((n_sp + s - 1) / s) + fixed);
         if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = s; }
     }
@@ -709,9 +750,7 @@ cudaError_t gemm_launch(const GemmParams& p, cudaStream_t stream) {
     if (p.n_stages < 2 || p.n_stages > GM_MAX_STAGES || p.n_bstages < 2 || p.n_bstages > GM_MAX_BSTAGES || p.n_splits < 1 ||
         p.n_tiles < 1) return cudaErrorInvalidValue;
     if (p.T_pad < 16 || p.T_pad > 512 || p.T_pad % 16 || p.T > p.T_pad || p.n_splits > p.K / 256) return cudaErrorInvalidValue;
-    if (p.swap) return launch_chain(gemm_q_kernel<256, true>, dim3(p.n_tiles * p.n_splits), dim3((256 / 32 + 3) * 32), gemm_smem_bytes(p), stream, p);
-    if (p.n_tt > 1) return launch_chain(gemm_q_kernel<256, false>, dim3(p.n_tiles * p.n_tt * p.n_splits), dim3((256 / 32 + 3) * 32), gemm_smem_bytes(p), stream, p);
-    return launch_chain(gemm_q_kernel<GM_BM, false>, dim3(p.n_tiles * p.n_splits), dim3((GM_BM / 32 + 3) * 32), gemm_smem_bytes(p), stream, p);
+    return launch_chain(p.ss ? gemm_q_kernel<true> : gemm_q_kernel<false>, dim3(p.n_tiles * p.n_tt * p.n_splits), dim3(GM_THREADS), gemm_smem_bytes(p), stream, p);
 }
 
 // x [T][K] float32 -> f16 in the MMA operand order [K/8][T_pad][8] (rows >= T zero)

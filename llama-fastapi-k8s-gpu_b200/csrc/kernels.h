@@ -165,8 +165,8 @@ struct GemmParams {
     long split_stride;
     unsigned int* err;
     long long* dbg;         // optional: CTA 0 records clock64() per K block (8 slots each), scripts/gemm_micro.py
-    int n_tiles, n_splits, n_stages, n_bstages, n_raw, swap;   // filled by gemm_plan (swap: 256-row variant, tokens as the MMA's M)
-    int n_tt, t_tile;       // token tiles of a step (2: 256 weight rows and half of the tokens a CTA) and the tokens of one
+    int n_tiles, n_splits, n_stages, n_bstages, n_raw;   // filled by gemm_plan
+    int n_tt, t_tile, ss;   // token tiles of a step and the tokens of one (a multiple of 16); expanded weights in shared memory
 };
 cudaError_t gemm_init();
 int gemm_plan(GemmParams& p, int n_sms, int max_splits);
