@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) dense_tc_kernel(const __grid_co
     __shared__ uint64_t full[TC_MAX_STAGES], empty[TC_MAX_STAGES], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_at;
     const DenseDev& a = p.a;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (warp: known to be uniform)
     uint8_t* ring = reinterpret_cast<uint8_t*>(((uintptr_t)tc_smem + 1023) & ~(uintptr_t)1023);
     const int S = p.stages;
     // a stage: weights, then tokens (short steps: the MMA reads 128 token rows whatever NT is; what it finds there is dropped)
@@ -196,18 +196,22 @@ __global__ void __launch_bounds__(TC_THREADS, 1) dense_tc_kernel(const __grid_co
         else tma_load_3d(st, &map_w, k * TC_K, w.n0, w.z, bar);
     };
 
-    if (warp == 4 && lane == 0) {
+    // The loops of the two issuing warps are run by all lanes, one of which issues: what the instructions take from uniform registers is
+    // computed there (as loops of one lane, each instruction was preceded by moves).
+    if (warp == 4) {
         // ================= copies
+        const bool one = elect_one();
         int s = 0, ahead = 0;
         uint32_t use = 0;
         bool waited = false;
         if (!a.grouped && first < p.n_work) {                      // weights of the first stages: no need to wait for the previous kernel
             TcTile w;
             tc_tile(p, first, 0, w);
-            for (; ahead < S && ahead < nk; ahead++) {
-                mbar_arrive_expect_tx(&full[ahead], stage_bytes);
-                load_w(ring + (size_t)ahead * stage_bytes, ahead, w, &full[ahead]);
-            }
+            for (; ahead < S && ahead < nk; ahead++)
+                if (one) {
+                    mbar_arrive_expect_tx(&full[ahead], stage_bytes);
+                    load_w(ring + (size_t)ahead * stage_bytes, ahead, w, &full[ahead]);
+                }
         }
         griddep_wait();
         const int n_tiles = a.grouped ? *a.g.n_tiles : 0;
@@ -216,20 +220,22 @@ __global__ void __launch_bounds__(TC_THREADS, 1) dense_tc_kernel(const __grid_co
             if (!tc_tile(p, i, n_tiles, w)) continue;
             for (int k = 0; k < nk; k++) {
                 uint8_t* st = ring + (size_t)s * stage_bytes;
-                if (!waited && k < ahead) {                        // the weights are on their way
-                } else {
-                    if (use > 0) mbar_wait(&empty[s], (use - 1) & 1, p.err, 0x50001u, (unsigned)k);
+                const bool weights = waited || k >= ahead;         // else they are on their way
+                if (weights && use > 0) mbar_wait(&empty[s], (use - 1) & 1, p.err, 0x50001u, (unsigned)k);
+                if (one && weights) {
                     mbar_arrive_expect_tx(&full[s], stage_bytes);
                     load_w(st, k, w, &full[s]);
                 }
-                if (SHORT && ks > 1) tma_load_4d(st + w_bytes, &map_x, 0, w.t0, k * ks, a.grouped ? 0 : w.z, &full[s]);
+                if (!one) {
+                } else if (SHORT && ks > 1) tma_load_4d(st + w_bytes, &map_x, 0, w.t0, k * ks, a.grouped ? 0 : w.z, &full[s]);
                 else tma_load_3d(st + w_bytes, &map_x, k * TC_K, w.t0, a.grouped ? 0 : w.z, &full[s]);
                 if (++s == S) { s = 0; use++; }
             }
             waited = true;
         }
-    } else if (warp == 5 && lane == 0) {
+    } else if (warp == 5) {
         // ================= matrix instructions
+        const bool one = elect_one();
         griddep_wait();
         const int n_tiles = a.grouped ? *a.g.n_tiles : 0;
         const uint32_t idesc = tc_idesc_bf16(TC_M, SHORT ? p.NW : p.NT);
@@ -246,16 +252,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1) dense_tc_kernel(const __grid_co
                 tc_after_sync();
                 const uint32_t at = smem_u32(ring + (size_t)s * stage_bytes);
                 const int n_slices = min(ks, slices - k * ks);
-                for (int q = 0; q < n_slices; q++) {
+                if (one) for (int q = 0; q < n_slices; q++) {
                     const uint64_t dw = tc_desc(at + q * w_slice), dx = tc_desc(at + w_bytes + q * x_slice);
 #pragma unroll
                     for (int kk = 0; kk < TC_K / 16; kk++)
                         tc_mma(tmem + b * p.cols, (SHORT ? dx : dw) + 2 * kk, (SHORT ? dw : dx) + 2 * kk, idesc, (k | q | kk) ? 1u : 0u);
                 }
-                tc_commit(&empty[s]);
+                if (one) tc_commit(&empty[s]);
                 if (++s == S) { s = 0; use++; }
             }
-            tc_commit(&acc_full[b]);
+            if (one) tc_commit(&acc_full[b]);
             tile++;
         }
     } else if (warp < 4) {

@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(192, 1) latent_attn_tc_kernel(const __grid_con
     const int tile = r.n_tiles - 1 - (int)blockIdx.y, h = blockIdx.x / n_chunks, chunk = blockIdx.x % n_chunks;
     const int seg = r.tile_seg[tile], row0 = r.tile_row0[tile];
     if (((row0 - r.seg_start[seg]) / 64) & 1) return;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (warp: known to be uniform)
     const int nq = min(LC_Q, r.seg_start[seg] + r.seg_len[seg] - row0);
     const int p0 = r.seg_pos0[seg] + row0 - r.seg_start[seg], p_last = p0 + nq - 1;
     const int* table = a.block_tables[r.seg_slot[seg]];
@@ -79,23 +79,26 @@ __global__ void __launch_bounds__(192, 1) latent_attn_tc_kernel(const __grid_con
     tc_after_sync();
     const uint32_t tmem = tmem_at, o_at = tmem, s_at = tmem + LC_V, p_at = tmem + LC_V + 2 * LC_K;
 
-    if (warp == 4 && lane == 0) {
-        // ================= copies: the latent parts of the queries, then blocks of cached rows
+    if (warp == 4) {
+        // ================= copies: the latent parts of the queries, then blocks of cached rows (all lanes run the loop, one issues: see dense_tc.cu)
+        const bool one = elect_one();
         const int q_parts = a.rank / LC_PART, n_rest = n_parts - n_val;
-        mbar_arrive_expect_tx(&q_full, (uint32_t)(q_parts * LC_QPART));
-        for (int c = 0; c < q_parts; c++) tma_load_3d(qs + (size_t)c * LC_QPART, &map_q, c * LC_PART, h, row0, &q_full);
+        if (one) mbar_arrive_expect_tx(&q_full, (uint32_t)(q_parts * LC_QPART));
+        if (one) for (int c = 0; c < q_parts; c++) tma_load_3d(qs + (size_t)c * LC_QPART, &map_q, c * LC_PART, h, row0, &q_full);
         for (int i = 0; i < n_blocks; i++) {
             const int j0 = (b0 + i) * LC_K, row = table[j0 / a.block_tokens] * a.block_tokens + j0 % a.block_tokens;
             for (int half = 0; half < 2; half++) {
                 uint64_t *full = half ? &val_full : &rest_full, *empty = half ? &val_empty : &rest_empty;
                 if (half == 0 && n_rest == 0) continue;
                 if (i > 0) mbar_wait(empty, (i - 1) & 1, err, 0x60001u, (unsigned)i);
+                if (!one) continue;
                 mbar_arrive_expect_tx(full, (uint32_t)((half ? n_val : n_rest) * LC_KPART));
                 for (int c = 0; c < n_parts; c++)
                     if ((c >= v0 && c < v0 + n_val) == (half == 1)) tma_load_3d(ks + (size_t)c * LC_KPART, &map_k, c * LC_PART, row, 0, full);
             }
         }
-    } else if (warp == 5 && lane == 0) {
+    } else if (warp == 5) {
+        const bool one = elect_one();
         // ================= matrix instructions
         const uint32_t id_s = tc_idesc_bf16(LC_Q, LC_K), id_o = tc_idesc_bf16(LC_Q, n_val * LC_PART, true);
         const uint32_t qa = smem_u32(qs), ka = smem_u32(ks);
@@ -104,34 +107,38 @@ __global__ void __launch_bounds__(192, 1) latent_attn_tc_kernel(const __grid_con
             for (int c = 0; c < n_parts; c++) {
                 if ((c >= v0 && c < v0 + n_val) != values) continue;
                 const uint64_t dq = tc_desc(qa + c * LC_QPART), dk = tc_desc(ka + c * LC_KPART);
+                if (one)
 #pragma unroll
-                for (int k = 0; k < LC_PART / 16; k++) { tc_mma(s_at + (i & 1) * LC_K, dq + 2 * k, dk + 2 * k, id_s, first ? 0u : 1u); first = false; }
+                    for (int k = 0; k < LC_PART / 16; k++) tc_mma(s_at + (i & 1) * LC_K, dq + 2 * k, dk + 2 * k, id_s, first && k == 0 ? 0u : 1u);
+                first = false;
             }
         };
         const bool any_rest = n_parts > n_val;
         mbar_wait(&q_full, 0, err, 0x60002u);
         tc_after_sync();
-        if (any_rest) { mbar_wait(&rest_full, 0, err, 0x60003u); tc_after_sync(); scores(0, false); tc_commit(&rest_empty); }
+        if (any_rest) { mbar_wait(&rest_full, 0, err, 0x60003u); tc_after_sync(); scores(0, false); if (one) tc_commit(&rest_empty); }
         mbar_wait(&val_full, 0, err, 0x60004u);
         tc_after_sync();
         scores(0, true);
-        tc_commit(&s_full[0]);
+        if (one) tc_commit(&s_full[0]);
         for (int i = 0; i < n_blocks; i++) {
             const bool more = i + 1 < n_blocks;
             first = true;
-            if (more && any_rest) { mbar_wait(&rest_full, (i + 1) & 1, err, 0x60005u, (unsigned)i); tc_after_sync(); scores(i + 1, false); tc_commit(&rest_empty); }
+            if (more && any_rest) { mbar_wait(&rest_full, (i + 1) & 1, err, 0x60005u, (unsigned)i); tc_after_sync(); scores(i + 1, false); if (one) tc_commit(&rest_empty); }
             mbar_wait(&p_full[i & 1], (i >> 1) & 1, err, 0x60006u, (unsigned)i);
             tc_after_sync();
+            if (one) {
 #pragma unroll
-            for (int k = 0; k < LC_K / 16; k++)
-                tc_mma_ts(o_at, p_at + (i & 1) * (LC_K / 2) + k * 8, tc_desc(ka + v0 * LC_KPART + k * 2048, LC_KPART), id_o, (i | k) ? 1u : 0u);
-            tc_commit(&pv_done);
-            tc_commit(&val_empty);
+                for (int k = 0; k < LC_K / 16; k++)
+                    tc_mma_ts(o_at, p_at + (i & 1) * (LC_K / 2) + k * 8, tc_desc(ka + v0 * LC_KPART + k * 2048, LC_KPART), id_o, (i | k) ? 1u : 0u);
+                tc_commit(&pv_done);
+                tc_commit(&val_empty);
+            }
             if (more) {
                 mbar_wait(&val_full, (i + 1) & 1, err, 0x60007u, (unsigned)i);
                 tc_after_sync();
                 scores(i + 1, true);
-                tc_commit(&s_full[(i + 1) & 1]);
+                if (one) tc_commit(&s_full[(i + 1) & 1]);
             }
         }
     } else if (warp < 4) {

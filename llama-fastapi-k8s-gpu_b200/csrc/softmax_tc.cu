@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_
     const int tile = r.n_tiles - 1 - (int)blockIdx.y, h = blockIdx.x;
     const int seg = r.tile_seg[tile], row0 = r.tile_row0[tile];
     if (((row0 - r.seg_start[seg]) / 64) & 1) return;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (warp: known to be uniform)
     const int nq = min(SX_Q, r.seg_start[seg] + r.seg_len[seg] - row0);
     const int p0 = r.seg_pos0[seg] + row0 - r.seg_start[seg], p_last = p0 + nq - 1;
     const int* table = a.block_tables[r.seg_slot[seg]];
@@ -76,8 +76,9 @@ __global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_
     tc_after_sync();
     const uint32_t o_at = tmem_at, s_at = tmem_at + 128, p_at = tmem_at + 384;       // probabilities: 64 columns leading, 64 remainder
 
-    if (warp == 8 && lane == 0) {
-        // ================= copies
+    if (warp == 8) {
+        // ================= copies (all lanes run the loop, one issues: see dense_tc.cu)
+        const bool one = elect_one();
         for (int i = 0; i < n_blocks; i++) {
             const int st = i & 1, j0 = block_at(i), halves = j0 + 64 <= p_last ? 2 : 1;
             for (int kv = 0; kv < 2; kv++) {
@@ -85,6 +86,7 @@ __global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_
                 const int parts = kv ? v_parts : k_parts;
                 uint8_t* dst = (kv ? vs : ks) + (size_t)st * parts * SX_PART;
                 if (i >= 2) mbar_wait(empty, ((i >> 1) - 1) & 1, err, 0x70001u, (unsigned)i);
+                if (!one) continue;
                 mbar_arrive_expect_tx(full, (uint32_t)(halves * parts * (SX_PART / 2)));
                 for (int hf = 0; hf < halves; hf++) {
                     const int j = j0 + 64 * hf, row = (table[j / bt] * a.G + g) * bt + j % bt;
@@ -92,21 +94,21 @@ __global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_
                 }
             }
         }
-    } else if (warp == 9 && lane == 0) {
+    } else if (warp == 9) {
+        const bool one = elect_one();
         // ================= matrix instructions
         const uint32_t id_s = tc_idesc_bf16(SX_Q, SX_K), id_o = tc_idesc_bf16(SX_Q, a.dv, true);
         const uint32_t qa = smem_u32(qs), ka = smem_u32(ks), va = smem_u32(vs);
         auto scores = [&](int i) {
             mbar_wait(&k_full[i & 1], (i >> 1) & 1, err, 0x70002u, (unsigned)i);
             tc_after_sync();
-            for (int part = 0; part < 2 * k_parts; part++) {             // remainders first
+            if (one) for (int part = 0; part < 2 * k_parts; part++) {    // remainders first
                 const int c = part % k_parts, lead = part / k_parts;
                 const uint64_t dq = tc_desc(qa + ((lead ? 0 : k_parts) + c) * SX_PART), dk = tc_desc(ka + ((i & 1) * k_parts + c) * SX_PART);
 #pragma unroll
                 for (int k = 0; k < 4; k++) tc_mma(s_at + (i & 1) * SX_K, dq + 2 * k, dk + 2 * k, id_s, (part | k) ? 1u : 0u);
             }
-            tc_commit(&s_full[i & 1]);
-            tc_commit(&k_empty[i & 1]);
+            if (one) { tc_commit(&s_full[i & 1]); tc_commit(&k_empty[i & 1]); }
         };
         mbar_wait(&q_full, 0, err, 0x70003u);
         tc_after_sync();
@@ -117,6 +119,7 @@ __global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_
             mbar_wait(&p_full, i & 1, err, 0x70005u, (unsigned)i);
             tc_after_sync();
             const uint32_t v_at = va + (i & 1) * v_parts * SX_PART;
+            if (!one) continue;
 #pragma unroll
             for (int half = 0; half < 2; half++)                         // remainders first
 #pragma unroll
