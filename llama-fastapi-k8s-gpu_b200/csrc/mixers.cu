@@ -174,7 +174,10 @@ cudaError_t layer_norm_launch(const float* x, const float* w, const float* b, fl
 }
 
 // parallel blocks: both sublayers' outputs (a mixture's expert rows are summed here) join the 32-bit stream, and both norms of
-// the next layer are made from one mean and one variance; the row lives in shared memory between the passes
+// the next layer are made from one mean and one variance; the row lives in shared memory between the passes. Bound by latency: the
+// entries of a thread are read JOIN_U at a time (the stores between them would otherwise keep every read behind the last one), with an
+// expert row's number looked up once per batch. 32 rows of 2048 with 4 experts each: 12.1 -> 7.0 us.
+constexpr int JOIN_U = 4;
 struct ParallelJoinDev { ParallelJoinArgs a; MoeJoinArgs j; int moe; };
 template <int NT>
 __global__ void __launch_bounds__(NT) parallel_join_kernel(ParallelJoinDev p, int W) {
@@ -188,36 +191,69 @@ __global__ void __launch_bounds__(NT) parallel_join_kernel(ParallelJoinDev p, in
     const size_t base = (size_t)t * W;
     const bool adds = a.a || a.b || p.moe;
     float sum = 0.f;
-    for (int i = threadIdx.x; i < W; i += NT) {
-        float v = a.x[base + i], y = a.a ? a.a[base + i] : 0.f;
-        if (a.b) y += a.b[base + i];
+    for (int i0 = threadIdx.x; i0 < W; i0 += NT * JOIN_U) {
+        float v[JOIN_U], y[JOIN_U], z[JOIN_U];
+#pragma unroll
+        for (int u = 0; u < JOIN_U; u++) {
+            const int i = i0 + u * NT;
+            const bool in = i < W;
+            v[u] = in ? a.x[base + i] : 0.f;
+            y[u] = in && a.a ? a.a[base + i] : 0.f;
+            z[u] = in && a.b ? a.b[base + i] : 0.f;
+        }
+        if (a.b)
+#pragma unroll
+            for (int u = 0; u < JOIN_U; u++) y[u] += z[u];
         if (p.moe) {
-            float acc = 0.f;
+            float acc[JOIN_U] = {};
             for (int c = 0; c < j.top; c++) {
                 const int q = t * j.top + c;
-                const float u = j.sel[q] < j.n_experts ? j.rows[(size_t)(j.pos ? j.pos[q] : q) * W + i] : j.h[base + i];
-                acc = fmaf(j.weight ? j.weight[q] : 1.f, u, acc);
+                const float wt = j.weight ? j.weight[q] : 1.f;
+                const float* from = j.sel[q] < j.n_experts ? j.rows + (size_t)(j.pos ? j.pos[q] : q) * W : j.h + base;
+#pragma unroll
+                for (int u = 0; u < JOIN_U; u++) z[u] = i0 + u * NT < W ? from[i0 + u * NT] : 0.f;
+#pragma unroll
+                for (int u = 0; u < JOIN_U; u++) acc[u] = fmaf(wt, z[u], acc[u]);
             }
-            y += acc;
+#pragma unroll
+            for (int u = 0; u < JOIN_U; u++) y[u] += acc[u];
         }
-        if (adds) { v += y; a.x[base + i] = v; }
-        if (a.x_copy) a.x_copy[(size_t)t * a.ld_copy + i] = v;
-        row[i] = v;
-        sum += v;
+#pragma unroll
+        for (int u = 0; u < JOIN_U; u++) {
+            const int i = i0 + u * NT;
+            if (i >= W) continue;
+            if (adds) { v[u] += y[u]; a.x[base + i] = v[u]; }
+            if (a.x_copy) a.x_copy[(size_t)t * a.ld_copy + i] = v[u];
+            row[i] = v[u];
+            sum += v[u];
+        }
     }
     if (!a.w1 && !a.w2) return;
     const float mean = block_sum(sum, red) / (float)W;
     float sq = 0.f;
     for (int i = threadIdx.x; i < W; i += NT) { const float dlt = row[i] - mean; sq = fmaf(dlt, dlt, sq); }
     const float rstd = 1.f / sqrtf(block_sum(sq, red) / (float)W + a.eps);
-    for (int i = threadIdx.x; i < W; i += NT) {
-        const float u = (row[i] - mean) * rstd;
-        if (a.w1) {
-            const float v = fmaf(u, a.w1[i], a.b1 ? a.b1[i] : 0.f);
-            if (a.y1) a.y1[base + i] = v;
-            if (a.y1_bf16) a.y1_bf16[base + i] = __float2bfloat16(v);
+    for (int i0 = threadIdx.x; i0 < W; i0 += NT * JOIN_U) {
+        float w1[JOIN_U], b1[JOIN_U], w2[JOIN_U], b2[JOIN_U];
+#pragma unroll
+        for (int u = 0; u < JOIN_U; u++) {
+            const int i = i0 + u * NT;
+            const bool in = i < W;
+            w1[u] = in && a.w1 ? a.w1[i] : 0.f; b1[u] = in && a.w1 && a.b1 ? a.b1[i] : 0.f;
+            w2[u] = in && a.y2 ? a.w2[i] : 0.f; b2[u] = in && a.y2 && a.b2 ? a.b2[i] : 0.f;
         }
-        if (a.y2) a.y2[base + i] = fmaf(u, a.w2[i], a.b2 ? a.b2[i] : 0.f);
+#pragma unroll
+        for (int k = 0; k < JOIN_U; k++) {
+            const int i = i0 + k * NT;
+            if (i >= W) continue;
+            const float u = (row[i] - mean) * rstd;
+            if (a.w1) {
+                const float v = fmaf(u, w1[k], b1[k]);
+                if (a.y1) a.y1[base + i] = v;
+                if (a.y1_bf16) a.y1_bf16[base + i] = __float2bfloat16(v);
+            }
+            if (a.y2) a.y2[base + i] = fmaf(u, w2[k], b2[k]);
+        }
     }
 }
 cudaError_t parallel_join_launch(const ParallelJoinArgs& a, int W, int T, cudaStream_t s) {
