@@ -1767,12 +1767,13 @@ extern "C" int b2_step(b2_engine* e, int n_entries, const int32_t* slots, const 
     auto head_chunk = [&](int r0, int nr) -> int {
         {
             StepProfiler sp(m, st, 5);
-            CK(gather_rows_launch(m->x, W, d_rows + r0, nr, m->rows, st));
+            const bool rms = c.block_style == B2_BLOCK_OUTNORM_RMS || c.block_style == B2_BLOCK_PRENORM_RMS || c.block_style == B2_BLOCK_HYPER_RMS;
+            if (rms) CK(gather_rows_launch(m->x, W, d_rows + r0, nr, m->rows, st));
             if (c.block_style == B2_BLOCK_OUTNORM_RMS) CK(outnorm_join_launch(nullptr, m->rows, nullptr, m->final_norm, std::max(1, c.norm_groups), c.norm_eps, W, nr, m->rows, st));
             else if (c.block_style == B2_BLOCK_PRENORM_RMS) CK(resid_rms_norm_launch(m->rows, nullptr, 0.f, m->final_norm, 1.f, 1.f, c.norm_eps, W, nr, m->rows, st));
             else if (c.block_style == B2_BLOCK_HYPER_RMS) CK(resid_rms_norm_launch(m->rows, nullptr, 0.f, m->final_norm, 0.f, 1.f, c.norm_eps, W, nr, m->rows, st));
-            else CK(layer_norm_launch(m->rows, m->final_norm, m->final_norm_b, c.norm_eps, W, nr, m->rows, st));
-            e->launches += 2;
+            else CK(layer_norm_rows_launch(m->x, d_rows + r0, m->final_norm, m->final_norm_b, c.norm_eps, W, nr, m->rows, st));
+            e->launches += rms ? 2 : 1;
         }
         DenseArgs hs = {};
         hs.scale = c.logit_scale != 0.f ? c.logit_scale : 1.f;

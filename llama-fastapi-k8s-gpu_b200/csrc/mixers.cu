@@ -155,22 +155,43 @@ cudaError_t resid_rms_norm_launch(float* x, const float* add, float mult, const 
     return launch_chain(resid_rms_norm_kernel, dim3(T), dim3(256), (size_t)W * 4, s, x, add, mult, w, w_offset, out_scale, eps, W, y);
 }
 
-__global__ void __launch_bounds__(256) layer_norm_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b,
-                                                         float eps, int W, float* __restrict__ y) {
+// Norm of rows rows[0], rows[1], .. of x. A thread keeps its entries of rows up to 256 LN_U in registers, read at once; longer rows are
+// read again for each pass.
+constexpr int LN_U = 16;
+__global__ void __launch_bounds__(256) layer_norm_kernel(const float* __restrict__ x, const int* __restrict__ rows, const float* __restrict__ w,
+                                                         const float* __restrict__ b, float eps, int W, float* __restrict__ y) {
     griddep_launch();
     griddep_wait();
     __shared__ float red[33];
-    const size_t base = (size_t)blockIdx.x * W;
-    float sum = 0.f;
-    for (int i = threadIdx.x; i < W; i += blockDim.x) sum += x[base + i];
+    const float* from = x + (size_t)rows[blockIdx.x] * W;
+    float* to = y + (size_t)blockIdx.x * W;
+    float sum = 0.f, sq = 0.f;
+    if (W <= 256 * LN_U) {
+        float v[LN_U], wv[LN_U], bv[LN_U];
+#pragma unroll
+        for (int u = 0; u < LN_U; u++) {
+            const int i = threadIdx.x + 256 * u;
+            const bool in = i < W;
+            v[u] = in ? from[i] : 0.f; wv[u] = in ? w[i] : 0.f; bv[u] = in && b ? b[i] : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < LN_U; u++) if (threadIdx.x + 256 * u < W) sum += v[u];
+        const float mean = block_sum(sum, red) / (float)W;
+#pragma unroll
+        for (int u = 0; u < LN_U; u++) if (threadIdx.x + 256 * u < W) { const float dlt = v[u] - mean; sq += dlt * dlt; }
+        const float rstd = 1.f / sqrtf(block_sum(sq, red) / (float)W + eps);
+#pragma unroll
+        for (int u = 0; u < LN_U; u++) if (threadIdx.x + 256 * u < W) to[threadIdx.x + 256 * u] = fmaf((v[u] - mean) * rstd, wv[u], bv[u]);
+        return;
+    }
+    for (int i = threadIdx.x; i < W; i += blockDim.x) sum += from[i];
     const float mean = block_sum(sum, red) / (float)W;
-    float sq = 0.f;
-    for (int i = threadIdx.x; i < W; i += blockDim.x) { const float dlt = x[base + i] - mean; sq += dlt * dlt; }
+    for (int i = threadIdx.x; i < W; i += blockDim.x) { const float dlt = from[i] - mean; sq += dlt * dlt; }
     const float rstd = 1.f / sqrtf(block_sum(sq, red) / (float)W + eps);
-    for (int i = threadIdx.x; i < W; i += blockDim.x) y[base + i] = fmaf((x[base + i] - mean) * rstd, w[i], b ? b[i] : 0.f);
+    for (int i = threadIdx.x; i < W; i += blockDim.x) to[i] = fmaf((from[i] - mean) * rstd, w[i], b ? b[i] : 0.f);
 }
-cudaError_t layer_norm_launch(const float* x, const float* w, const float* b, float eps, int W, int T, float* y, cudaStream_t s) {
-    return launch_chain(layer_norm_kernel, dim3(T), dim3(256), 0, s, x, w, b, eps, W, y);
+cudaError_t layer_norm_rows_launch(const float* x, const int* rows, const float* w, const float* b, float eps, int W, int n, float* y, cudaStream_t s) {
+    return launch_chain(layer_norm_kernel, dim3(n), dim3(256), 0, s, x, rows, w, b, eps, W, y);
 }
 
 // parallel blocks: both sublayers' outputs (a mixture's expert rows are summed here) join the 32-bit stream, and both norms of
