@@ -3,7 +3,7 @@
 // Replaces ggml-cuda's "dequantise the whole matrix to an f16 scratch copy, then cublasGemmEx" prompt
 // path (convert.cu + cuBLAS) that llama-cpp-python runs under create_chat_completion
 // (/root/reference/api.py:55-63), and its batched mul_mat_q path for several sequences per step. No f16 copy
-// of W ever exists in HBM: quant blocks go from HBM to registers to the shared-memory operand tile of the MMA.
+// of W ever exists in HBM: quant blocks go from HBM over shared memory and registers to the operand of the MMA.
 //
 // Work decomposition. A CTA owns 256 weight rows (two halves of 128, the MMA's M and the lanes of tensor memory) of one of up to three
 // matrices that share the input (q|k|v, gate|up), one of up to two token tiles (the MMA's N) and one of n_splits
@@ -26,7 +26,7 @@
 // Why the weights go to tensor memory: with both operands in shared memory a block of 256 rows costs that memory 32 KB of stores and 48 KB
 // of operand reads for 32 tokens (tokens as the 128-row operand), 96 KB of reads for 256 tokens: 800 and 1400 cycles of its 128 bytes a
 // cycle, against 512 and 1024 of products. The expansion itself needs about 500 with 16 warps (950 with 8, two a scheduler).
-// 32 sequences, 4 layers of 4096 (Q4_K/Q6_K), mean product: 23.1 us with both operands in shared memory and 8 warps; 25.7 with 16; 27 with the
+// 32 sequences, 4 layers of 4096 (Q8_0), mean product: 23.1 us with both operands in shared memory and 8 warps; 25.7 with 16; 27 with the
 // weights in tensor memory (the MMA thread, one lane of a busy scheduler, took 1200 cycles a block); 17.5 with that loop run by the whole
 // warp and one lane issuing. A 37-token prompt: 9.7 -> 7 us a product.
 // Roofline: tensor pipe for large T; for T <= ~64 the dequantisation, then HBM (weights read once per call).

@@ -8,6 +8,7 @@
 // this one's softmax runs. Eight softmax warps, two threads a query row with 64 key columns each (capped scores take three special-function
 // operations a score, which is what bounds the kernel); they exchange their maxima through shared memory. The output is rescaled only
 // when a row's maximum has grown by more than 2^8.
+// 2048 tokens (B200): 16 capped heads of 128, 300 us a layer with mma.sync, 67 here; 32 heads of 128 over a window of 1024 keys, 326 and 99.
 #include "kernels.h"
 #include "layered.h"
 #include "ptx.cuh"
