@@ -259,7 +259,10 @@ cudaError_t latent_attn_launch(const LatentAttnArgs& a, const RaggedDev& r, cuda
 
 // Long steps over bf16 pages (latent_tc.cu): queries q [T][H][rank] are the folded ones, scaled and rounded (their rotated parts come
 // from a.q_raw or a.qv); the weighted latents go to `out` [T][H][rank], rounded. pool_rows: rows of the pages in all.
-constexpr int LATENT_TC_MIN = 256;             // tokens per sequence of the step, on average: two tiles of 128 queries
+// Tokens per sequence of the step, on average. 16 heads, rows of 512 (us a launch, mma.sync / tcgen05): 128 tokens 74 / 17, 256 90 / 19, 384
+// 169 / 22. The times cross lower; the line is here because the kernels round probabilities against different running maxima, and
+// answers to short prompts stay what they were.
+constexpr int LATENT_TC_MIN = 256;
 bool latent_attn_takes_tc(const LatentAttnArgs& a, int T, int n_seg);
 cudaError_t latent_attn_tc_launch(const LatentAttnArgs& a, const RaggedDev& r, const __nv_bfloat16* q, long pool_rows, __nv_bfloat16* out, cudaStream_t s);
 

@@ -279,8 +279,9 @@ __global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_
 }
 
 // ---------------------------------------------------------------- host side
-// Steps whose sequences bring at least 256 tokens each on average: two tiles of 128 rows, enough CTAs and key blocks for the copies and
-// the next block's scores to hide under the softmax. Sizes that the tiles and 16-byte stores take, pages of whole 64-key halves.
+// Steps whose sequences bring at least 256 tokens each on average. 16 heads of 128 (us a launch, mma.sync / here): 128 tokens 54 / 18, 256 61 /
+// 17, 384 63 / 22; over a window 28 / 23, 39 / 18, 49 / 20. The line is not where the times cross, which is lower: the two kernels round
+// differently (where a probability is split depends on the running maximum), and answers to short prompts stay what they were. Sizes that the tiles and 16-byte stores take, pages of whole 64-key halves.
 bool softmax_takes_tc(const SoftmaxTcArgs& a, int T, int n_seg) {
     return T >= 256 * n_seg && a.d % 16 == 0 && a.dv % 16 == 0 && a.d <= 128 && a.dv <= 128 && a.block_tokens % 64 == 0 && a.ld_out % 8 == 0 &&
            ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.out) | reinterpret_cast<uintptr_t>(a.out_bf16)) & 15) == 0;
