@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) dense_tc_kernel(const __grid_co
             for (int k = 0; k < nk; k++) {
                 uint8_t* st = ring + (size_t)s * stage_bytes;
                 const bool weights = waited || k >= ahead;         // else they are on their way
-                if (weights && use > 0) mbar_wait(&empty[s], (use - 1) & 1, p.err, 0x50001u, (unsigned)k);
+                if (weights && use > 0) mbar_wait_warp(&empty[s], (use - 1) & 1, p.err, 0x50001u, (unsigned)k);
                 if (one && weights) {
                     mbar_arrive_expect_tx(&full[s], stage_bytes);
                     load_w(st, k, w, &full[s]);
@@ -246,10 +246,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) dense_tc_kernel(const __grid_co
             TcTile w;
             if (!tc_tile(p, i, n_tiles, w)) continue;
             const int b = tile & 1;
-            if (tile >= 2) mbar_wait(&acc_empty[b], ((tile >> 1) - 1) & 1, p.err, 0x50002u, (unsigned)tile);
+            if (tile >= 2) mbar_wait_warp(&acc_empty[b], ((tile >> 1) - 1) & 1, p.err, 0x50002u, (unsigned)tile);
             tc_after_sync();
             for (int k = 0; k < nk; k++) {
-                mbar_wait(&full[s], use & 1, p.err, 0x50003u, (unsigned)k);
+                mbar_wait_warp(&full[s], use & 1, p.err, 0x50003u, (unsigned)k);
                 tc_after_sync();
                 const uint32_t at = smem_u32(ring + (size_t)s * stage_bytes);
                 const int n_slices = min(ks, slices - k * ks);

@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(192, 1) latent_attn_tc_kernel(const __grid_con
             for (int half = 0; half < 2; half++) {
                 uint64_t *full = half ? &val_full : &rest_full, *empty = half ? &val_empty : &rest_empty;
                 if (half == 0 && n_rest == 0) continue;
-                if (i > 0) mbar_wait(empty, (i - 1) & 1, err, 0x60001u, (unsigned)i);
+                if (i > 0) mbar_wait_warp(empty, (i - 1) & 1, err, 0x60001u, (unsigned)i);
                 if (!one) continue;
                 mbar_arrive_expect_tx(full, (uint32_t)((half ? n_val : n_rest) * LC_KPART));
                 for (int c = 0; c < n_parts; c++)
@@ -116,18 +116,18 @@ __global__ void __launch_bounds__(192, 1) latent_attn_tc_kernel(const __grid_con
             }
         };
         const bool any_rest = n_parts > n_val;
-        mbar_wait(&q_full, 0, err, 0x60002u);
+        mbar_wait_warp(&q_full, 0, err, 0x60002u);
         tc_after_sync();
-        if (any_rest) { mbar_wait(&rest_full, 0, err, 0x60003u); tc_after_sync(); scores(0, false); if (one) tc_commit(&rest_empty); }
-        mbar_wait(&val_full, 0, err, 0x60004u);
+        if (any_rest) { mbar_wait_warp(&rest_full, 0, err, 0x60003u); tc_after_sync(); scores(0, false); if (one) tc_commit(&rest_empty); }
+        mbar_wait_warp(&val_full, 0, err, 0x60004u);
         tc_after_sync();
         scores(0, true);
         if (one) tc_commit(&s_full[0]);
         for (int i = 0; i < n_blocks; i++) {
             const bool more = i + 1 < n_blocks;
             first = true;
-            if (more && any_rest) { mbar_wait(&rest_full, (i + 1) & 1, err, 0x60005u, (unsigned)i); tc_after_sync(); scores(i + 1, false); if (one) tc_commit(&rest_empty); }
-            mbar_wait(&p_full[i & 1], (i >> 1) & 1, err, 0x60006u, (unsigned)i);
+            if (more && any_rest) { mbar_wait_warp(&rest_full, (i + 1) & 1, err, 0x60005u, (unsigned)i); tc_after_sync(); scores(i + 1, false); if (one) tc_commit(&rest_empty); }
+            mbar_wait_warp(&p_full[i & 1], (i >> 1) & 1, err, 0x60006u, (unsigned)i);
             tc_after_sync();
             if (one) {
 #pragma unroll
@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(192, 1) latent_attn_tc_kernel(const __grid_con
                 tc_commit(&val_empty);
             }
             if (more) {
-                mbar_wait(&val_full, (i + 1) & 1, err, 0x60007u, (unsigned)i);
+                mbar_wait_warp(&val_full, (i + 1) & 1, err, 0x60007u, (unsigned)i);
                 tc_after_sync();
                 scores(i + 1, true);
                 if (one) tc_commit(&s_full[(i + 1) & 1]);

@@ -52,6 +52,12 @@ __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, unsign
         }
     }
 }
+// The wait of a loop that a whole warp runs while one lane issues copies or products. The lanes leave it together: what is issued next
+// lets the barrier move on, and a lane still waiting when it has moved two phases on would read the parity of the phase before its own.
+__device__ __forceinline__ void mbar_wait_warp(uint64_t* bar, uint32_t parity, unsigned int* err, unsigned int code, unsigned int info = 0) {
+    mbar_wait(bar, parity, err, code, info);
+    __syncwarp();
+}
 // 1-D bulk async copy global -> shared, completion signalled on an mbarrier (complete_tx).
 // dst and src 16-byte aligned, bytes a multiple of 16.
 __device__ __forceinline__ void tma_load_1d(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {

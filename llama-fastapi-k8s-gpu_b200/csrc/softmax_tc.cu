@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_
                 uint64_t *full = kv ? &v_full[st] : &k_full[st], *empty = kv ? &v_empty[st] : &k_empty[st];
                 const int parts = kv ? v_parts : k_parts;
                 uint8_t* dst = (kv ? vs : ks) + (size_t)st * parts * SX_PART;
-                if (i >= 2) mbar_wait(empty, ((i >> 1) - 1) & 1, err, 0x70001u, (unsigned)i);
+                if (i >= 2) mbar_wait_warp(empty, ((i >> 1) - 1) & 1, err, 0x70001u, (unsigned)i);
                 if (!one) continue;
                 mbar_arrive_expect_tx(full, (uint32_t)(halves * parts * (SX_PART / 2)));
                 for (int hf = 0; hf < halves; hf++) {
@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_
         const uint32_t id_s = tc_idesc_bf16(SX_Q, SX_K), id_o = tc_idesc_bf16(SX_Q, a.dv, true);
         const uint32_t qa = smem_u32(qs), ka = smem_u32(ks), va = smem_u32(vs);
         auto scores = [&](int i) {
-            mbar_wait(&k_full[i & 1], (i >> 1) & 1, err, 0x70002u, (unsigned)i);
+            mbar_wait_warp(&k_full[i & 1], (i >> 1) & 1, err, 0x70002u, (unsigned)i);
             tc_after_sync();
             if (one) for (int part = 0; part < 2 * k_parts; part++) {    // remainders first
                 const int c = part % k_parts, lead = part / k_parts;
@@ -111,13 +111,13 @@ __global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_
             }
             if (one) { tc_commit(&s_full[i & 1]); tc_commit(&k_empty[i & 1]); }
         };
-        mbar_wait(&q_full, 0, err, 0x70003u);
+        mbar_wait_warp(&q_full, 0, err, 0x70003u);
         tc_after_sync();
         scores(0);
         for (int i = 0; i < n_blocks; i++) {
             if (i + 1 < n_blocks) scores(i + 1);
-            mbar_wait(&v_full[i & 1], (i >> 1) & 1, err, 0x70004u, (unsigned)i);
-            mbar_wait(&p_full, i & 1, err, 0x70005u, (unsigned)i);
+            mbar_wait_warp(&v_full[i & 1], (i >> 1) & 1, err, 0x70004u, (unsigned)i);
+            mbar_wait_warp(&p_full, i & 1, err, 0x70005u, (unsigned)i);
             tc_after_sync();
             const uint32_t v_at = va + (i & 1) * v_parts * SX_PART;
             if (!one) continue;
