@@ -13,7 +13,7 @@
 //
 // Pipeline per CTA, in blocks of 64 K-elements:
 //   weight producer (one thread): TMA boxes of 256 rows x one 256-weight span, raw block bytes -> shared memory.
-//   16 dequantising warps, two threads a row, each two of every four blocks: raw bytes -> f16 with byte-permute + half2 arithmetic (exact small
+//   16 dequantising warps, two threads a row, each every other block: raw bytes -> f16 with byte-permute + half2 arithmetic (exact small
 //       integers 1024+q; scales applied without losing bits: ~2-2.5 instr/weight) -> tensor memory (tcgen05.st), as the MMA's A operand;
 //       one arrival per warp on a_full[stage].
 //   activation producer (one thread): activations live in HBM in the MMA's own K-major core-matrix order [K/8][T][8] (the producing
@@ -30,6 +30,7 @@
 // weights in tensor memory (the MMA thread, one lane of a busy scheduler, took 1200 cycles a block); 17.5 with that loop run by the whole
 // warp and one lane issuing. A 37-token prompt: 9.7 -> 7 us a product.
 // Roofline: tensor pipe for large T; for T <= ~64 the dequantisation, then HBM (weights read once per call).
+#include "gemm_ring.h"
 #include "kernels.h"
 #include "ptx.cuh"
 #include "quant_blocks.cuh"
@@ -47,7 +48,7 @@ constexpr int GM_ABYTES = GM_ROWS * GM_BK * 2;      // SS: bytes of a weight blo
 constexpr int GM_DW = 16;           // dequantising warps: two threads a row
 constexpr int GM_THREADS = (GM_DW + 3) * 32;
 constexpr int GM_HDR = 512;         // barriers at the start of dynamic shared memory
-constexpr int GM_MAX_STAGES = 6;     // weight blocks in tensor memory
+constexpr int GM_MAX_STAGES = gm_stages(false, 0);     // expanded weight blocks
 constexpr int GM_MAX_BSTAGES = 8;    // activation-tile ring
 constexpr int GM_RAW_STAGES = 2;    // raw weight spans in flight (TMA), at most
 constexpr int GM_SPAN_WORDS = 68;   // largest 256-weight span: Q8_0, 272 bytes
@@ -358,23 +359,13 @@ struct DeqCtx {
     long long* dbg;
 };
 
-// blocks 2 GRP and 2 GRP + 1 of every four
+// blocks GRP, GRP + 2, .. of this CTA's range, into stages that no other group writes
 template <bool SS, int TYPE, int GRP>
 __device__ __noinline__ void deq_loop(const DeqCtx cx) {
     GemmBars& sh = *cx.sh;
     const int lane = threadIdx.x & 31;
-    int st = 0;                 // A stage of the next block and how often the ring has wrapped
+    int st = GRP;               // stage of the next block and how often the ring has wrapped
     uint32_t wraps = 0;
-    // past the other group's two blocks. With four stages each group has two of its own; with another number it meets a stage whose barrier
-    // has moved on two phases, which a parity does not tell from none, so the phase between is waited for as well.
-    auto skip = [&]() {
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-            if (cx.S % 4 && wraps > 0) mbar_wait(&sh.empty[st], (wraps - 1) & 1, cx.err, 0x40008u, (unsigned)st);
-            if (++st == cx.S) { st = 0; wraps++; }
-        }
-    };
-    if (GRP) skip();
     auto emit = [&](const RawKB& r, int i) {               // block i of this CTA's range -> its stage in tensor memory
         uint32_t out[32];
         if (TYPE == T_GENERIC) dequant_block_generic(cx.type, cx.wrow, (cx.kb0 + i) * GM_BK, out);
@@ -397,12 +388,11 @@ __device__ __noinline__ void deq_loop(const DeqCtx cx) {
         __syncwarp();
         if (lane == 0) mbar_arrive(&sh.a_full[st]);      // once per warp: the arrivals of 32 lanes go one after the other
         if (cx.dbg && i < 64) cx.dbg[i * 8 + 2] = clock64();
-        if (++st == cx.S) { st = 0; wraps++; }
-        if (i & 1) skip();
+        if ((st += GM_GROUPS) >= cx.S) { st -= cx.S; wraps++; }
     };
     if (TYPE == T_GENERIC) {
         RawKB none;
-        for (int i = 2 * GRP; i < cx.n; i += 4) { emit(none, i); emit(none, i + 1); }
+        for (int i = GRP; i < cx.n; i += GM_GROUPS) emit(none, i);
     } else if (cx.use_tma) {
         // raw spans arrive in shared memory by TMA; this thread's row is one box row. The box starts at the 16-byte
         // boundary below the span (TMA needs it); only Q6_K spans (210 B) can be off it.
@@ -447,19 +437,17 @@ __device__ __noinline__ void deq_loop(const DeqCtx cx) {
                 }
             }
             RawKB r;
-            span_block<2 * GRP>(TYPE, W, r); emit(r, sp * 4 + 2 * GRP);
-            span_block<2 * GRP + 1>(TYPE, W, r); emit(r, sp * 4 + 2 * GRP + 1);
+            span_block<GRP>(TYPE, W, r); emit(r, sp * 4 + GRP);
+            span_block<GRP + GM_GROUPS>(TYPE, W, r); emit(r, sp * 4 + GRP + GM_GROUPS);
         }
     } else {
         // rows that are not 16-byte multiples (Q6_K with K % 2048 != 0): direct loads, next block prefetched in registers
         RawKB cur, nxt;
-        load_raw(TYPE, cx.wrow, (cx.kb0 + 2 * GRP) * GM_BK, cur);
-        for (int i = 2 * GRP; i < cx.n;) {
-            const int next = i + (i & 1 ? 3 : 1);
-            if (next < cx.n) load_raw(TYPE, cx.wrow, (cx.kb0 + next) * GM_BK, nxt);
+        load_raw(TYPE, cx.wrow, (cx.kb0 + GRP) * GM_BK, cur);
+        for (int i = GRP; i < cx.n; i += GM_GROUPS) {
+            if (i + GM_GROUPS < cx.n) load_raw(TYPE, cx.wrow, (cx.kb0 + i + GM_GROUPS) * GM_BK, nxt);
             emit(cur, i);
             cur = nxt;
-            i = next;
         }
     }
 }
@@ -714,8 +702,9 @@ int gemm_plan(GemmParams& p, int n_sms, int max_splits) {
     p.n_tiles = tiles;
     const size_t b_st = (size_t)p.t_tile * GM_BK * 2, cap = 227 * 1024 - 1024;
     // activation ring: deep when the tiles are small (their TMA latency must not gate the MMAs)
-    int SB = p.t_tile <= 64 ? 8 : p.ss ? 3 : 6, S = p.ss ? 2 : 4;
-    if (const char* v = getenv("B2_GEMM_STAGES")) if (atoi(v) > 1) S = std::min(atoi(v), p.ss ? 3 : 4);
+    int SB = p.t_tile <= 64 ? 8 : p.ss ? 3 : 6;
+    const char* stages = getenv("B2_GEMM_STAGES");
+    const int S = gm_stages(p.ss, stages ? atoi(stages) : 0);
     if (const char* v = getenv("B2_GEMM_BSTAGES")) if (atoi(v) > 1) SB = std::min(atoi(v), GM_MAX_BSTAGES);
     p.n_raw = GM_RAW_STAGES;
     if (const char* v = getenv("B2_GEMM_RAW")) if (atoi(v) == 1) p.n_raw = 1;
@@ -723,7 +712,6 @@ int gemm_plan(GemmParams& p, int n_sms, int max_splits) {
     while (total() > cap && SB > 3) SB--;
     if (total() > cap) p.n_raw = 1;
     while (total() > cap && SB > 2) SB--;
-    while (total() > cap && S > 2) S--;
     if (total() > cap) { for (int s = 0; s < p.nseg; s++) p.seg[s].use_tma = 0; }
     if (total() > cap) return -4;
     p.n_stages = S; p.n_bstages = SB;
@@ -747,7 +735,7 @@ int gemm_plan(GemmParams& p, int n_sms, int max_splits) {
 }
 
 cudaError_t gemm_launch(const GemmParams& p, cudaStream_t stream) {
-    if (p.n_stages < 2 || p.n_stages > GM_MAX_STAGES || p.n_bstages < 2 || p.n_bstages > GM_MAX_BSTAGES || p.n_splits < 1 ||
+    if (p.n_stages < GM_GROUPS || p.n_stages % GM_GROUPS || p.n_stages > GM_MAX_STAGES || p.n_bstages < 2 || p.n_bstages > GM_MAX_BSTAGES || p.n_splits < 1 ||
         p.n_tiles < 1) return cudaErrorInvalidValue;
     if (p.T_pad < 16 || p.T_pad > 512 || p.T_pad % 16 || p.T > p.T_pad || p.n_splits > p.K / 256) return cudaErrorInvalidValue;
     return launch_chain(p.ss ? gemm_q_kernel<true> : gemm_q_kernel<false>, dim3(p.n_tiles * p.n_tt * p.n_splits), dim3(GM_THREADS), gemm_smem_bytes(p), stream, p);

@@ -3,6 +3,7 @@
 // unpacking and the two-plane int8 activation scheme against the oracle without a GPU.
 #define B2_HOST_EMU 1
 #include <math.h>
+#include "gemm_ring.h"
 #include "quant_blocks.cuh"
 
 template <int T>
@@ -23,6 +24,11 @@ static float host_row(const uint8_t* rowp, int K, const b2::ActView& v, bool act
 }
 
 extern "C" {
+
+// the ring of expanded blocks of the quantised product (gemm_ring.h)
+int b2_host_gemm_stages(int in_smem, int wanted) { return b2::gm_stages(in_smem != 0, wanted); }
+int b2_host_gemm_group(int block) { return b2::gm_group(block); }
+int b2_host_gemm_stage(int block, int stages) { return b2::gm_stage(block, stages); }
 
 // dequantise n_elems elements (whole blocks) with the exact element routine
 int b2_host_dequant(int type, const uint8_t* raw, long n_elems, float* out) {

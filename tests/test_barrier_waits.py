@@ -1,7 +1,9 @@
 """Waits on barriers in the kernels that hand work from warp to warp, checked on the CPU: a barrier tells two phases apart by their parity
 only, so whoever waits must not be able to fall two phases behind."""
+import ctypes
 import os
 import re
+import subprocess
 
 import pytest
 
@@ -32,3 +34,25 @@ def test_issuing_warps_leave_their_waits_together(name):
             rest = b[m.end():]
             sync, issue = rest.find("__syncwarp()"), re.search(r"elect_one\(\)|\(one\)|\(!one\)", rest)
             assert sync >= 0 and (issue is None or sync < issue.start()), (name, rest[:120])
+
+
+@pytest.mark.parametrize("in_smem", [0, 1])
+@pytest.mark.parametrize("wanted", range(8))
+def test_a_stage_of_expanded_weights_belongs_to_one_group(tmp_path_factory, in_smem, wanted):
+    """A group that waits for a use of a stage has to take part in the next one: then no use can pass it by."""
+    lib = host_lib(tmp_path_factory)
+    stages = lib.b2_host_gemm_stages(in_smem, wanted)
+    assert 2 <= stages <= (2 if in_smem else 4)
+    owners = {}
+    for block in range(64):
+        owners.setdefault(lib.b2_host_gemm_stage(block, stages), set()).add(lib.b2_host_gemm_group(block))
+    assert len(owners) == stages and all(len(o) == 1 for o in owners.values())
+    assert set.union(*owners.values()) == {0, 1}
+
+
+def host_lib(tmp_path_factory, made=[]):
+    if not made:
+        out = str(tmp_path_factory.mktemp("ring") / "ring.so")
+        subprocess.run(["g++", "-O2", "-fPIC", "-shared", os.path.join(CSRC, "host_selftest.cpp"), "-o", out], check=True)
+        made.append(ctypes.CDLL(out))
+    return made[0]
