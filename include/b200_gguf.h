@@ -274,7 +274,8 @@ int b2_engine_create_layered(const b2_layered_config* cfg, const b2_layer_desc* 
  * entries' tokens one after another. `want_rows` (indices into host_tokens) are the rows whose logits are copied to
  * host_logits [n_want][n_vocab]. sample[i] != 0: sample from the logits of entry i's last token with the slot's sampler
  * and return the token in host_sampled[i] (-1 elsewhere); those logits also stay in the slot's logit buffer. Any of
- * want_rows / sample / host_sampled may be NULL. */
+ * want_rows / sample / host_sampled may be NULL. A row may be wanted more than once; every token once always fits, and more
+ * than the engine's step description holds is refused before anything runs (B2_ERR_ARG). */
 #define B2_STEP_MAX_ENTRIES 64
 int b2_step(b2_engine* e, int n_entries, const int32_t* slots, const int32_t* n_tokens, const int32_t* host_tokens,
             const int32_t* want_rows, int n_want, float* host_logits, const int32_t* sample, int32_t* host_sampled);

@@ -122,6 +122,7 @@ struct LayeredModel {
     int attn_split_floats = 0;
     int* meta = nullptr;               // device ints: ragged description + wanted rows
     int* meta_host = nullptr;          // pinned
+    size_t meta_ints = 0;              // of either copy of a step's description
     float* logits_host = nullptr;      // pinned [LOGIT_ROWS][n_vocab]
     float* trace = nullptr;            // [n_layer][max_step_tokens][n_embd] when tracing
     int last_T = 0;
@@ -732,7 +733,8 @@ int layered_finalize(b2_engine* e) {
     }
     if ((rc = dev_alloc(m, (void**)&m->rows, (size_t)LOGIT_ROWS * W * 4))) return rc;
     if ((rc = dev_alloc(m, (void**)&m->logits, (size_t)LOGIT_ROWS * V * 4))) return rc;
-    const size_t n_meta = (size_t)5 * Tm + 2 * (Tm / 64 + B2_STEP_MAX_ENTRIES) + 5 * B2_STEP_MAX_ENTRIES + 64;
+    // a wanted row for every token, a sampled one for every entry
+    const size_t n_meta = m->meta_ints = (size_t)5 * Tm + 2 * (Tm / 64 + B2_STEP_MAX_ENTRIES) + 5 * B2_STEP_MAX_ENTRIES + 64;
     if ((rc = dev_alloc(m, (void**)&m->meta, n_meta * 4))) return rc;
     CK(cudaMallocHost(&m->meta_host, n_meta * 4));
     CK(cudaMallocHost(&m->logits_host, (size_t)LOGIT_ROWS * V * 4));
@@ -1724,6 +1726,10 @@ extern "C" int b2_step(b2_engine* e, int n_entries, const int32_t* slots, const 
     }
     for (int i = 0; i < T; i++) if (tokens[i] < 0 || tokens[i] >= c.n_vocab) return b2_fail(B2_ERR_ARG, "token id out of range");
     for (int i = 0; i < n_want; i++) if (want_rows[i] < 0 || want_rows[i] >= T) return b2_fail(B2_ERR_ARG, "wanted row out of range");
+    int n_tiles = 0;
+    for (int i = 0; i < n_entries; i++) n_tiles += (n_tokens[i] + 63) / 64;
+    // (rows may be asked for more than once: as often as the description of the step has room for)
+    if ((size_t)4 * T + 5 * n_entries + 2 * n_tiles + n_want > m->meta_ints) return b2_fail(B2_ERR_ARG, "more wanted rows than a step of this engine holds");
     CK(cudaSetDevice(c.device));
     cudaStream_t st = e->stream;
     StepChainPdl chain(e->chain_pdl);
@@ -1731,8 +1737,6 @@ extern "C" int b2_step(b2_engine* e, int n_entries, const int32_t* slots, const 
     int* h = m->meta_host;
     const int n = n_entries;
     int *h_id = h, *h_seg = h + T, *h_pos = h + 2 * T, *h_prev = h + 3 * T, *h_slot = h + 4 * T, *h_start = h_slot + n, *h_len = h_start + n, *h_p0 = h_len + n;
-    int n_tiles = 0;
-    for (int i = 0; i < n; i++) n_tiles += (n_tokens[i] + 63) / 64;
     int *h_tseg = h_p0 + n, *h_trow = h_tseg + n_tiles;
     int* h_rows = h_trow + n_tiles;
     int row = 0, tile = 0;

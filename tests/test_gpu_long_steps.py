@@ -146,6 +146,24 @@ def test_many_wanted_rows_and_long_rows(native_lib, tmp_path):
     check(zu, zogurax_ref, cfg, tmp_path, [20], "bfloat16")
 
 
+def test_rows_wanted_again_and_again(native_lib, tmp_path):
+    """Repeated rows come as often as asked for; more of them than a step's description holds are refused, and nothing has moved."""
+    from llama_cpp._cabi import B2Error
+    from llama_cpp.kv_pages import SequenceSlots
+    cfg = zu.config([zu.biased()], vocab=203)
+    eng = engine(zu.write_model(str(tmp_path / "m"), cfg, zu.random_weights(cfg, seed=5)), "bfloat16", 16)
+    seqs = SequenceSlots(eng)
+    seqs.open(0)
+    slot, prompt = seqs.extend(0, 4), toks(203, 4, 1)
+    for rows in ([3] * 600, list(range(4)) * 5000):
+        with pytest.raises(B2Error):
+            eng.step([(slot, prompt)], want=[rows])
+    lg, _ = eng.step([(slot, prompt)], want=[[0, 1, 2, 3] * 100 + [2]])
+    eng.close()
+    assert lg.shape == (401, 203) and all(np.array_equal(lg[i], lg[i % 4]) for i in range(400)) and np.array_equal(lg[400], lg[2])
+    assert rows_off(lg[:4], zogurax_ref.forward(cfg, zu.random_weights(cfg, seed=5), prompt)).max() < BF16
+
+
 @pytest.mark.parametrize("tname", ["Q4_K", "Q6_K", "Q8_0", "Q4_0", "Q5_K", "Q4_1"])
 @pytest.mark.parametrize("K,N,T", [(256, 128, 257), (768, 130, 272), (2048, 256, 288), (1024, 257, 385), (512, 384, 512), (4096, 640, 511)])
 def test_two_token_tiles_of_quantised_products(native_lib, tname, K, N, T):
