@@ -50,8 +50,6 @@ __device__ __forceinline__ float lc_rotated(const LatentAttnArgs& a, int t, int 
 // grid (heads x column chunks, 64-query tiles of the step, latest first; odd tiles of a sequence belong to the CTA before them)
 __global__ void __launch_bounds__(192, 1) latent_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_q,
                                                                 const LatentAttnArgs a, const RaggedDev r, int n_chunks, __nv_bfloat16* out, unsigned int* err) {
-    griddep_launch();
-    griddep_wait();
     extern __shared__ uint8_t lc_smem[];
     __shared__ uint64_t rest_full, val_full, rest_empty, val_empty, q_full, s_full[2], p_full[2], pv_done;
     __shared__ uint32_t tmem_at;
@@ -79,6 +77,10 @@ __global__ void __launch_bounds__(192, 1) latent_attn_tc_kernel(const __grid_con
     tc_before_sync();
     __syncthreads();
     tc_after_sync();
+    // The next kernel is let in once tensor memory is this CTA's: had it come first on this SM, it would hold its own and wait for this kernel
+    // to end, and this CTA for that memory. (What is read above is the step's description, older than the kernel before this one.)
+    griddep_launch();
+    griddep_wait();
     const uint32_t tmem = tmem_at, o_at = tmem, s_at = tmem + LC_V, p_at = tmem + LC_V + 2 * LC_K;
 
     if (warp == 4) {

@@ -38,8 +38,6 @@ __device__ __forceinline__ void sx_split(float a, float b, uint32_t& hi, uint32_
 template <bool CAP>
 __global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                                                                    const SoftmaxTcArgs a, const RaggedDev r, unsigned int* err) {
-    griddep_launch();
-    griddep_wait();
     extern __shared__ uint8_t sx_smem[];
     __shared__ uint64_t k_full[2], k_empty[2], v_full[2], v_empty[2], q_full, s_full[2], p_full, pv_done;
     __shared__ uint32_t tmem_at;
@@ -75,6 +73,10 @@ __global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_
     tc_before_sync();
     __syncthreads();
     tc_after_sync();
+    // The next kernel is let in once tensor memory is this CTA's: had it come first on this SM, it would hold its own and wait for this kernel
+    // to end, and this CTA for that memory. (What is read above is the step's description, older than the kernel before this one.)
+    griddep_launch();
+    griddep_wait();
     const uint32_t o_at = tmem_at, s_at = tmem_at + 128, p_at = tmem_at + 384;       // probabilities: 64 columns leading, 64 remainder
 
     if (warp == 8) {

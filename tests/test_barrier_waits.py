@@ -36,6 +36,18 @@ def test_issuing_warps_leave_their_waits_together(name):
             assert sync >= 0 and (issue is None or sync < issue.start()), (name, rest[:120])
 
 
+@pytest.mark.parametrize("name", FILES)
+def test_tensor_memory_is_taken_before_the_next_kernel_is_let_in(name):
+    """A kernel that is launched early and takes its tensor memory waits for the one before it to end; one that has yet to take its own would
+    wait for the other's. So it is taken ahead of griddep_launch(), behind a barrier of the CTA."""
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, name)).read())
+    kernels = [k for k in re.split(r"__global__", text)[1:] if re.search(r"\b(tc_alloc|tmem_alloc)\(", k)]
+    assert kernels
+    for k in kernels:
+        alloc, let_in = re.search(r"\b(tc_alloc|tmem_alloc)\(", k).start(), k.index("griddep_launch()")
+        assert alloc < k.index("__syncthreads()", alloc) < let_in, name
+
+
 @pytest.mark.parametrize("in_smem", [0, 1])
 @pytest.mark.parametrize("wanted", range(8))
 def test_a_stage_of_expanded_weights_belongs_to_one_group(tmp_path_factory, in_smem, wanted):
