@@ -376,10 +376,10 @@ bool bf16_slices_map(CUtensorMap* m, const void* base, long cols, long rows, lon
     const cuuint32_t box[4] = {TC_K, (cuuint32_t)box_rows, (cuuint32_t)slices, 1};
     return cols % TC_K == 0 && encode_map(m, base, dims, strides, box);
 }
-bool bf16_heads_map(CUtensorMap* m, const void* base, long cols, long heads, long rows, int box_rows) {
+bool bf16_heads_map(CUtensorMap* m, const void* base, long cols, long heads, long rows, int box_heads, int box_rows) {
     const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)heads, (cuuint64_t)rows};
     const cuuint64_t strides[2] = {(cuuint64_t)cols * 2, (cuuint64_t)(cols * heads) * 2};
-    const cuuint32_t box[3] = {TC_K, 1, (cuuint32_t)box_rows};
+    const cuuint32_t box[3] = {TC_K, (cuuint32_t)box_heads, (cuuint32_t)box_rows};
     return encode_map(m, base, dims, strides, box);
 }
 

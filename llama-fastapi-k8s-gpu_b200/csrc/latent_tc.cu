@@ -1,6 +1,6 @@
-// Latent attention of long steps on the 5th-generation tensor cores (bf16 pages). Same arithmetic as latent_attn_mma_kernel
-// (latent_attn.cu): queries scaled, then rounded to bf16; cached rows as they are; probabilities rounded to bf16 for the weighted
-// sum, 32-bit everywhere else.
+// Latent attention of steps of more than 8 tokens on the 5th-generation tensor cores (bf16 pages). Rounded where latent_attn_mma_kernel
+// (latent_attn.cu) rounds: queries scaled, then rounded to bf16; cached rows as they are; probabilities rounded to bf16 for the weighted
+// sum, 32-bit everywhere else. (Here the running maximum that a probability is taken against may lag by 2^8, so other bits are rounded.)
 //
 // A CTA takes 128 consecutive queries of one head and up to 256 latent columns of the output (tensor memory holds 128 lanes x 512
 // columns: 256 for the output, two score tiles of 64, two probability tiles of 32, so a 512-wide latent is two CTAs that both
@@ -19,6 +19,7 @@
 #include "tensor_map.h"
 
 #include <algorithm>
+#include <stdlib.h>
 
 namespace b2 {
 
@@ -47,18 +48,22 @@ __device__ __forceinline__ float lc_rotated(const LatentAttnArgs& a, int t, int 
 }
 }  // namespace
 
-// grid (heads x column chunks, 64-query tiles of the step, latest first; odd tiles of a sequence belong to the CTA before them)
+// CTAs: (64-query tile, head, column chunk), latest tiles first (odd tiles of a sequence belong to the CTA before them), then (one-token
+// sequence, chunk) for the first n_packed tiles: there the rows are the heads, which all read the same keys
 __global__ void __launch_bounds__(192, 1) latent_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_q,
-                                                                const LatentAttnArgs a, const RaggedDev r, int n_chunks, __nv_bfloat16* out, unsigned int* err) {
+                                                                const __grid_constant__ CUtensorMap map_h, const LatentAttnArgs a, const RaggedDev r,
+                                                                int n_packed, int n_chunks, __nv_bfloat16* out, unsigned int* err) {
     extern __shared__ uint8_t lc_smem[];
     __shared__ uint64_t rest_full, val_full, rest_empty, val_empty, q_full, s_full[2], p_full[2], pv_done;
     __shared__ uint32_t tmem_at;
-    const int tile = r.n_tiles - 1 - (int)blockIdx.y, h = blockIdx.x / n_chunks, chunk = blockIdx.x % n_chunks;
+    const int whole = (r.n_tiles - n_packed) * a.H, at = blockIdx.x / n_chunks, chunk = blockIdx.x % n_chunks;
+    const bool packed = at >= whole;
+    const int tile = packed ? at - whole : r.n_tiles - 1 - at / a.H, h = packed ? 0 : at % a.H;
     const int seg = r.tile_seg[tile], row0 = r.tile_row0[tile];
     if (((row0 - r.seg_start[seg]) / 64) & 1) return;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (warp: known to be uniform)
-    const int nq = min(LC_Q, r.seg_start[seg] + r.seg_len[seg] - row0);
-    const int p0 = r.seg_pos0[seg] + row0 - r.seg_start[seg], p_last = p0 + nq - 1;
+    const int nq = packed ? a.H : min(LC_Q, r.seg_start[seg] + r.seg_len[seg] - row0);      // rows in use
+    const int p0 = r.seg_pos0[seg] + row0 - r.seg_start[seg], p_last = packed ? p0 : p0 + nq - 1;
     const int* table = a.block_tables[r.seg_slot[seg]];
     const int n_parts = (a.rank + a.dr + LC_PART - 1) / LC_PART, v0 = chunk * (LC_V / LC_PART), n_val = min(LC_V, a.rank - chunk * LC_V) / LC_PART;
     uint8_t* qs = reinterpret_cast<uint8_t*>(((uintptr_t)lc_smem + 1023) & ~(uintptr_t)1023);
@@ -88,7 +93,7 @@ __global__ void __launch_bounds__(192, 1) latent_attn_tc_kernel(const __grid_con
         const bool one = elect_one();
         const int q_parts = a.rank / LC_PART, n_rest = n_parts - n_val;
         if (one) mbar_arrive_expect_tx(&q_full, (uint32_t)(q_parts * LC_QPART));
-        if (one) for (int c = 0; c < q_parts; c++) tma_load_3d(qs + (size_t)c * LC_QPART, &map_q, c * LC_PART, h, row0, &q_full);
+        if (one) for (int c = 0; c < q_parts; c++) tma_load_3d(qs + (size_t)c * LC_QPART, packed ? &map_h : &map_q, c * LC_PART, h, row0, &q_full);
         for (int i = 0; i < n_blocks; i++) {
             const int j0 = (b0 + i) * LC_K, row = table[j0 / a.block_tokens] * a.block_tokens + j0 % a.block_tokens;
             for (int half = 0; half < 2; half++) {
@@ -147,20 +152,21 @@ __global__ void __launch_bounds__(192, 1) latent_attn_tc_kernel(const __grid_con
         }
     } else if (warp < 4) {
         // ================= softmax: thread = query row
-        const int row = threadIdx.x, pos = p0 + row;
+        const int row = threadIdx.x, pos = packed ? p0 : p0 + row;
+        const int t = packed ? row0 : row0 + row, hd = packed ? min(row, a.H - 1) : h;      // the row's token and head
         const uint32_t lanes = (uint32_t)(warp * 32) << 16;
         // the rotated part of the queries (and zeros up to the part's 64 columns), rows past the tile as zeros
         for (int c = a.rank; c < n_parts * LC_PART; c += 8) {
             float v[8];
 #pragma unroll
-            for (int e = 0; e < 8; e++) v[e] = row < nq && c + e < a.rank + a.dr ? lc_rotated(a, row0 + row, h, c + e - a.rank, pos) * a.scale : 0.f;
+            for (int e = 0; e < 8; e++) v[e] = row < nq && c + e < a.rank + a.dr ? lc_rotated(a, t, hd, c + e - a.rank, pos) * a.scale : 0.f;
             uint8_t* dst = qs + (size_t)(c / LC_PART) * LC_QPART + row * 128 + ((((c % LC_PART) / 8) ^ (row & 7)) << 4);
             *reinterpret_cast<uint4*>(dst) = make_uint4(lc_pack(v[0], v[1]), lc_pack(v[2], v[3]), lc_pack(v[4], v[5]), lc_pack(v[6], v[7]));
         }
         fence_proxy_async();
         mbar_arrive(&q_full);
         constexpr float LOG2E = 1.4426950408889634f;
-        float m_ref = a.sink ? a.sink[h] * LOG2E : -INFINITY, l = a.sink ? 1.f : 0.f;           // log2 domain: weights are 2^(score - m_ref)
+        float m_ref = a.sink ? a.sink[hd] * LOG2E : -INFINITY, l = a.sink ? 1.f : 0.f;           // log2 domain: weights are 2^(score - m_ref)
         for (int i = 0; i < n_blocks; i++) {
             const int j0 = (b0 + i) * LC_K;
             mbar_wait(&s_full[i & 1], (i >> 1) & 1, err, 0x60008u, (unsigned)i);
@@ -225,7 +231,7 @@ __global__ void __launch_bounds__(192, 1) latent_attn_tc_kernel(const __grid_con
         mbar_wait(&pv_done, (n_blocks - 1) & 1, err, 0x6000au);
         tc_after_sync();
         const float inv = 1.f / l;
-        __nv_bfloat16* dst = out + ((size_t)(row0 + row) * a.H + h) * a.rank + chunk * LC_V;
+        __nv_bfloat16* dst = out + ((size_t)t * a.H + hd) * a.rank + chunk * LC_V;
         for (int c = 0; c < n_val * LC_PART; c += 32) {
             uint32_t o[32];
             __syncwarp();
@@ -248,24 +254,29 @@ __global__ void __launch_bounds__(192, 1) latent_attn_tc_kernel(const __grid_con
 }
 
 // ---------------------------------------------------------------- host side
-// Rows of 64-column parts that fit shared memory beside the queries (9 of them), whole chunks of output columns, pages of whole blocks.
-bool latent_attn_takes_tc(const LatentAttnArgs& a, int T, int n_seg) {
+// Rows of 64-column parts that fit shared memory beside the queries (9 of them), whole chunks of output columns, pages of whole blocks; of
+// the step only what the few-token kernels do not take (see softmax_tc.cu). 16 heads, rows of 512 + 64, us a layer with the preparation,
+// mma.sync / here: a prompt of 9 tokens 52 / 36, of 64 93 / 44, of 255 120 / 63; 32 prompts of 60 568 / 212; one token of each of 32 sequences
+// behind 60 208 / 38, behind 1900 2087 / 114; 512 tokens beside 31 sequences that decode behind 500, 869 / 97.
+bool latent_attn_takes_tc(const LatentAttnArgs& a, int T) {
+    static const bool no_mma = getenv("B2_NO_ATTN_MMA") != nullptr;        // tuning aid: scalar attention for prompts too
     const int parts = (a.rank + a.dr + LC_PART - 1) / LC_PART;
-    return !a.cache_f32 && T >= LATENT_TC_MIN * n_seg && a.rank % LC_PART == 0 && (a.rank <= LC_V || a.rank % LC_V == 0) && parts <= 9 && a.ld_row % 8 == 0 &&
+    return !no_mma && !a.cache_f32 && T > 8 && a.rank % LC_PART == 0 && (a.rank <= LC_V || a.rank % LC_V == 0) && parts <= 9 && a.ld_row % 8 == 0 &&
            a.block_tokens % LC_K == 0;
 }
 
 cudaError_t latent_attn_tc_launch(const LatentAttnArgs& a, const RaggedDev& r, const __nv_bfloat16* q, long pool_rows, __nv_bfloat16* out, cudaStream_t s) {
     static const bool ready = cudaFuncSetAttribute(latent_attn_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 9 * (LC_QPART + LC_KPART) + 1024) == cudaSuccess;
-    if (!ready || !latent_attn_takes_tc(a, r.T, r.n_seg)) return cudaErrorInvalidValue;
+    if (!ready || !latent_attn_takes_tc(a, r.T)) return cudaErrorInvalidValue;
     const int parts = (a.rank + a.dr + LC_PART - 1) / LC_PART, chunks = (a.rank + LC_V - 1) / LC_V;
-    CUtensorMap mk, mq;
+    CUtensorMap mk, mq, mh;
     // rows of the pages [pages * block_tokens][ld_row]; columns past rank + dr arrive as zeros
     if (!bf16_rows_map(&mk, a.pool, a.rank + a.dr, pool_rows, a.ld_row, 1, 0, LC_K)) return cudaErrorInvalidValue;
-    // queries [T][H][rank]: 128 tokens of one head
-    if (!bf16_heads_map(&mq, q, a.rank, a.H, r.T, LC_Q)) return cudaErrorInvalidValue;
-    return launch_chain(latent_attn_tc_kernel, dim3(a.H * chunks, r.n_tiles), dim3(192), (size_t)parts * (LC_QPART + LC_KPART) + 1024, s, mk, mq, a, r, chunks,
-                        out, kernel_error_word());
+    // queries [T][H][rank]: 128 tokens of one head, or the heads of one token
+    if (!bf16_heads_map(&mq, q, a.rank, a.H, r.T, 1, LC_Q) || !bf16_heads_map(&mh, q, a.rank, a.H, r.T, LC_Q, 1)) return cudaErrorInvalidValue;
+    const int n_packed = a.H <= LC_Q ? r.n_upto[0] : 0;
+    return launch_chain(latent_attn_tc_kernel, dim3(((r.n_tiles - n_packed) * a.H + n_packed) * chunks), dim3(192), (size_t)parts * (LC_QPART + LC_KPART) + 1024, s,
+                        mk, mq, mh, a, r, n_packed, chunks, out, kernel_error_word());
 }
 
 }  // namespace b2

@@ -1118,9 +1118,9 @@ static int mix_latent_attn(b2_engine* e, LayeredModel* m, LyLayer& L, const Ragg
     if (gate) { v.aux = m->proj + L.g_off; v.ldaux = Np; v.aux_bs = head_gate ? 1 : d.la_vdim; v.aux_one = head_gate; }
     const int v_epi = gate ? EPI_MUL_SIGMOID : EPI_NONE;
     DenseArgs op = {};
-    if (latent_attn_takes_tc(a, T, r.n_seg) && dense_takes_rounded(dense_args(m, L.uk_t, q, ldq, m->buf[0], H * Dk, T, nullptr, EPI_NONE, &b)) &&
+    if (latent_attn_takes_tc(a, T) && dense_takes_rounded(dense_args(m, L.uk_t, q, ldq, m->buf[0], H * Dk, T, nullptr, EPI_NONE, &b)) &&
         dense_takes_rounded(dense_args(m, L.uv, m->buf[1], H * d.la_rank, m->buf[2], H * d.la_vdim, T, nullptr, v_epi, &v)) && takes_rounded(m, L.attn_o, T)) {
-        // long steps: what these products and the attention hand on is left rounded
+        // what these products and the attention hand on is left rounded
         __nv_bfloat16* qb = reinterpret_cast<__nv_bfloat16*>(m->buf[1]);
         b.scale = a.scale; b.y_bs = d.la_rank; b.y_rounded = qb;
         if ((rc = dense(e, m, L.uk_t, q, ldq, nullptr, H * d.la_rank, T, nullptr, EPI_NONE, 1, &b))) return rc;
@@ -1739,11 +1739,18 @@ extern "C" int b2_step(b2_engine* e, int n_entries, const int32_t* slots, const 
     int *h_id = h, *h_seg = h + T, *h_pos = h + 2 * T, *h_prev = h + 3 * T, *h_slot = h + 4 * T, *h_start = h_slot + n, *h_len = h_start + n, *h_p0 = h_len + n;
     int *h_tseg = h_p0 + n, *h_trow = h_tseg + n_tiles;
     int* h_rows = h_trow + n_tiles;
-    int row = 0, tile = 0;
+    // tiles of short entries first, by the power of two that holds them (attention takes them apart)
+    auto size_class = [](int n_tok) { int k = 0; while (k < 7 && n_tok > 1 << k) k++; return k; };
+    int tile_of[8] = {}, tile = 0, row = 0;
+    for (int k = 0; k < 8; k++) {
+        tile_of[k] = tile;
+        for (int i = 0; i < n; i++) if (size_class(n_tokens[i]) == k) tile += (n_tokens[i] + 63) / 64;
+    }
     for (int i = 0; i < n; i++) {
         const int p0 = e->slots[slots[i]].n_past;
         h_slot[i] = slots[i]; h_start[i] = row; h_len[i] = n_tokens[i]; h_p0[i] = p0;
-        for (int k = 0; k < n_tokens[i]; k += 64) { h_tseg[tile] = i; h_trow[tile++] = row + k; }
+        int& at = tile_of[size_class(n_tokens[i])];
+        for (int k = 0; k < n_tokens[i]; k += 64) { h_tseg[at] = i; h_trow[at++] = row + k; }
         for (int k = 0; k < n_tokens[i]; k++, row++) {
             h_id[row] = tokens[row]; h_seg[row] = i; h_pos[row] = p0 + k;
             h_prev[row] = k > 0 ? tokens[row - 1] : e->slots[slots[i]].last_token;
@@ -1760,6 +1767,7 @@ extern "C" int b2_step(b2_engine* e, int n_entries, const int32_t* slots, const 
     r.tok_id = m->meta; r.tok_seg = m->meta + T; r.tok_pos = m->meta + 2 * T; r.tok_prev = m->meta + 3 * T; r.seg_slot = m->meta + 4 * T;
     r.seg_start = r.seg_slot + n; r.seg_len = r.seg_start + n; r.seg_pos0 = r.seg_len + n; r.T = T; r.n_seg = n;
     r.tile_seg = r.seg_pos0 + n; r.tile_row0 = r.tile_seg + n_tiles; r.n_tiles = n_tiles;
+    for (int k = 0; k < 7; k++) r.n_upto[k] = tile_of[k];       // (past the tiles of class k by now)
     const int* d_rows = r.tile_row0 + n_tiles;
     if (m->profile) {
         for (auto& pe : m->prof_ev) { cudaEventDestroy(pe.second.first); cudaEventDestroy(pe.second.second); }

@@ -24,7 +24,8 @@ struct RaggedDev {             // device pointers, valid for one step
     const int* seg_len;        // [n_seg]
     const int* seg_pos0;       // [n_seg] position of the segment's first token
     const int* tile_seg;       // [n_tiles] tiles of up to 64 consecutive rows of one segment: its segment ...
-    const int* tile_row0;      // ... and its first row
+    const int* tile_row0;      // ... and its first row. Segments of up to 64 tokens (one tile each) come first, the shortest ahead:
+    int n_upto[7];             // [i] segments, and tiles, of up to 2^i tokens
     int T, n_seg, n_tiles;
 };
 
@@ -257,13 +258,9 @@ struct LatentAttnArgs {
 cudaError_t latent_store_launch(const LatentAttnArgs& a, const RaggedDev& r, cudaStream_t s);
 cudaError_t latent_attn_launch(const LatentAttnArgs& a, const RaggedDev& r, cudaStream_t s);
 
-// Long steps over bf16 pages (latent_tc.cu): queries q [T][H][rank] are the folded ones, scaled and rounded (their rotated parts come
-// from a.q_raw or a.qv); the weighted latents go to `out` [T][H][rank], rounded. pool_rows: rows of the pages in all.
-// Tokens per sequence of the step, on average. 16 heads, rows of 512 (us a launch, mma.sync / tcgen05): 128 tokens 74 / 17, 256 90 / 19, 384
-// 169 / 22. The times cross lower; the line is here because the kernels round probabilities against different running maxima, and
-// answers to short prompts stay what they were.
-constexpr int LATENT_TC_MIN = 256;
-bool latent_attn_takes_tc(const LatentAttnArgs& a, int T, int n_seg);
+// Steps of more than 8 tokens over bf16 pages (latent_tc.cu): queries q [T][H][rank] are the folded ones, scaled and rounded (their rotated
+// parts come from a.q_raw or a.qv); the weighted latents go to `out` [T][H][rank], rounded. pool_rows: rows of the pages in all.
+bool latent_attn_takes_tc(const LatentAttnArgs& a, int T);
 cudaError_t latent_attn_tc_launch(const LatentAttnArgs& a, const RaggedDev& r, const __nv_bfloat16* q, long pool_rows, __nv_bfloat16* out, cudaStream_t s);
 
 // ---------------------------------------------------------------- mixture of experts (moe.cu)

@@ -696,7 +696,7 @@ cudaError_t window_attn_launch(const WindowAttnArgs& a, const RaggedDev& r, cuda
         SoftmaxTcArgs x = {};
         x.q = a.q_rot; x.k_pool = a.k_pool; x.v_pool = a.v_pool; x.pool_rows = a.pool_rows; x.block_tables = a.block_tables; x.block_tokens = a.block_tokens;
         x.H = a.H; x.G = a.G; x.d = x.dv = a.d; x.window = a.window; x.keep_first = a.keep_first; x.scale = a.scale; x.out = a.out; x.ld_out = a.H * a.d;
-        if (softmax_takes_tc(x, r.T, r.n_seg)) return softmax_tc_launch(x, r, s);
+        if (softmax_takes_tc(x)) return softmax_tc_launch(x, r, s);
         const size_t smem = (size_t)4 * 64 * (a.d + 8) * 2;
         if (a.d <= 64) return launch_chain(window_attn_mma_kernel<64>, dim3(r.n_tiles, a.H), dim3(128), smem, s, a, r);
         return launch_chain(window_attn_mma_kernel<128>, dim3(r.n_tiles, a.H), dim3(128), smem, s, a, r);

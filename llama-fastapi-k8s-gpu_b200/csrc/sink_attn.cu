@@ -847,8 +847,7 @@ __global__ void __launch_bounds__(128) sink_attn_mma_kernel(SinkAttnArgs a, Ragg
         }
 }
 
-// Steps in which every sequence brings one token: a CTA takes one sequence and one key/value head, its 16 rows are the query heads that
-// share it. The arithmetic of a row is that of the prompt kernel, operation for operation (the same 64-key blocks, accumulation and sums),
+// Sequences that bring one token: a CTA takes one sequence and one key/value head, its 16 rows are the query heads that share it. The arithmetic of a row is that of the prompt kernel, operation for operation (the same 64-key blocks, accumulation and sums),
 // spread over the warps by columns: a warp forms the scores of its 16 keys, all exchange them, each repeats the softmax of the rows and
 // adds up a quarter of the output columns. (32 sequences of 60 keys, 16 heads over 4: a 64-row tile per query head took 61 us a launch, one
 // warp per key/value head 33, most of it instruction fetch, the four warps of this form 17.)
@@ -864,7 +863,7 @@ __global__ void __launch_bounds__(128) sink_attn_pack_kernel(SinkAttnArgs a, Rag
     __nv_bfloat16* Ks = Ql + 16 * LD;                                   // [64][LD]
     __nv_bfloat16* Vs = Ks + SKM_K * LD;                                // [64][LDV]
     float* Ss = reinterpret_cast<float*>(Vs + SKM_K * LDV);             // [16][LDS] scores of a block
-    const int seg = blockIdx.x, g = blockIdx.y, h0 = g * HG, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int seg = r.tile_seg[blockIdx.x], g = blockIdx.y, h0 = g * HG, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t = r.seg_start[seg], pos = r.tok_pos[t];
     const int* table = a.block_tables[r.seg_slot[seg]];
     const __nv_bfloat16* kp = reinterpret_cast<const __nv_bfloat16*>(a.k_pool);
@@ -1303,8 +1302,12 @@ static bool sink_attn_mixed_launch(const SinkAttnArgs& a, const RaggedDev& r, cu
     return true;
 }
 
+// one-token sequences go through sink_attn_pack_kernel
+static bool sink_attn_packs(const SinkAttnArgs& a) { return !a.talk && a.H / a.G <= 16; }
+
+// only_one: the one-token sequences of the step alone
 template <int DMAX, int DVMAX, bool CAP>
-static cudaError_t sink_attn_mma_pick(const SinkAttnArgs& a, const RaggedDev& r, cudaStream_t s) {
+static cudaError_t sink_attn_mma_pick(const SinkAttnArgs& a, const RaggedDev& r, bool only_one, cudaStream_t s) {
     const size_t smem = (size_t)(3 * 64 * (a.d + 8) + 64 * (a.dv + 8)) * 2;
     static bool attr_done = false;
     if (!attr_done) {
@@ -1313,17 +1316,23 @@ static cudaError_t sink_attn_mma_pick(const SinkAttnArgs& a, const RaggedDev& r,
         cudaFuncSetAttribute(sink_attn_pack_kernel<DMAX, DVMAX, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
         attr_done = true;
     }
-    if (!a.talk && r.T == r.n_seg && a.H / a.G <= 16) {
+    RaggedDev rest = r;
+    if (r.n_upto[0] > 0 && sink_attn_packs(a)) {
         const size_t pack = (size_t)((32 + SKM_K) * (a.d + 8) + SKM_K * (a.dv + 8)) * 2 + 16 * (SKM_K + 8) * 4;
-        return launch_chain(sink_attn_pack_kernel<DMAX, DVMAX, CAP>, dim3(r.n_seg, a.G), dim3(128), pack, s, a, r);
+        const cudaError_t e = launch_chain(sink_attn_pack_kernel<DMAX, DVMAX, CAP>, dim3(r.n_upto[0], a.G), dim3(128), pack, s, a, r);
+        if (e != cudaSuccess || only_one || r.n_upto[0] == r.n_tiles) return e;
+        rest.tile_seg += r.n_upto[0]; rest.tile_row0 += r.n_upto[0]; rest.n_tiles -= r.n_upto[0];
     }
-    return launch_chain(sink_attn_mma_kernel<DMAX, DVMAX, CAP>, dim3(r.n_tiles, a.H * (a.talk ? a.G : 1)), dim3(128), smem, s, a, r);
+    return launch_chain(sink_attn_mma_kernel<DMAX, DVMAX, CAP>, dim3(rest.n_tiles, a.H * (a.talk ? a.G : 1)), dim3(128), smem, s, a, rest);
 }
 
 template <bool CAP>
-static cudaError_t sink_attn_mma_sizes(const SinkAttnArgs& a, const RaggedDev& r, cudaStream_t s) {
-    if (a.d <= 64) return a.dv <= 64 ? sink_attn_mma_pick<64, 64, CAP>(a, r, s) : sink_attn_mma_pick<64, 128, CAP>(a, r, s);
-    return a.dv <= 64 ? sink_attn_mma_pick<128, 64, CAP>(a, r, s) : sink_attn_mma_pick<128, 128, CAP>(a, r, s);
+static cudaError_t sink_attn_mma_sizes(const SinkAttnArgs& a, const RaggedDev& r, bool only_one, cudaStream_t s) {
+    if (a.d <= 64) return a.dv <= 64 ? sink_attn_mma_pick<64, 64, CAP>(a, r, only_one, s) : sink_attn_mma_pick<64, 128, CAP>(a, r, only_one, s);
+    return a.dv <= 64 ? sink_attn_mma_pick<128, 64, CAP>(a, r, only_one, s) : sink_attn_mma_pick<128, 128, CAP>(a, r, only_one, s);
+}
+static cudaError_t sink_attn_mma_launch(const SinkAttnArgs& a, const RaggedDev& r, bool only_one, cudaStream_t s) {
+    return a.softcap > 0.f ? sink_attn_mma_sizes<true>(a, r, only_one, s) : sink_attn_mma_sizes<false>(a, r, only_one, s);
 }
 
 bool sink_attn_on_tensor_cores(const SinkAttnArgs& a, int T) {
@@ -1345,8 +1354,17 @@ cudaError_t sink_attn_launch(const SinkAttnArgs& a, const RaggedDev& r, cudaStre
         x.q = a.q_rot; x.k_pool = a.k_pool; x.v_pool = a.v_pool; x.pool_rows = a.pool_rows; x.block_tables = a.block_tables; x.block_tokens = a.block_tokens;
         x.H = a.H; x.G = a.G; x.d = a.d; x.dv = a.dv; x.window = a.window; x.scale = a.scale; x.softcap = a.softcap; x.sink = a.sink;
         x.gate = a.gate; x.ld_gate = a.ld_gate; x.gate_per_head = a.gate_per_head; x.out = a.out; x.out_bf16 = a.out_bf16; x.ld_out = a.ld_out;
-        if (!a.talk && softmax_takes_tc(x, r.T, r.n_seg)) return softmax_tc_launch(x, r, s);
-        e = a.softcap > 0.f ? sink_attn_mma_sizes<true>(a, r, s) : sink_attn_mma_sizes<false>(a, r, s);
+        if (!a.talk && softmax_takes_tc(x)) {
+            // Which kernel a row goes to depends on its own sequence's share of the step alone: its bits do not change with the company.
+            // One token of each of 32 sequences, 16 heads over 4 (us with the preparation, behind 60 / 500 / 1900 keys): packed mma.sync tiles
+            // 18 / 42 / 119, tensor memory 28 / 34 / 62.
+            if (r.n_upto[0] > 0 && sink_attn_packs(a)) {
+                x.skip = r.n_upto[0];
+                if ((e = sink_attn_mma_launch(a, r, true, s)) != cudaSuccess) return e;
+            }
+            return softmax_tc_launch(x, r, s);
+        }
+        e = sink_attn_mma_launch(a, r, false, s);
     } else if (!a.talk && a.d % 8 == 0 && a.dv % 8 == 0) {
         return a.cache_f32 ? sink_attn_vec_launch<true>(a, r, s) : sink_attn_vec_launch<false>(a, r, s);
     } else {

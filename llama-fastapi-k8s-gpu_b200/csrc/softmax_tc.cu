@@ -1,8 +1,10 @@
-// Softmax attention of long steps on the 5th-generation tensor cores, for the layer-list models (bf16 pages, key and value sizes up to
-// 128). Same precision as the mma.sync kernels that shorter steps take: queries and probabilities enter the products as TWO bf16 each
-// (leading part + remainder), so the only 16-bit rounding is that of the cached keys and values; everything else is 32-bit.
+// Softmax attention of steps of more than 8 tokens on the 5th-generation tensor cores, for the layer-list models (bf16 pages, key and value
+// sizes up to 128). Queries and probabilities enter the products as TWO bf16 each (leading part + remainder), so the only 16-bit rounding is
+// that of the cached keys and values; everything else is 32-bit, with ex2.approx for the exponentials. (The mma.sync kernels, which other
+// sizes take, split at the same places. They round a probability against the exact running maximum, here it may lag by 2^8, and window
+// attention there uses expf on unscaled queries: the two agree to about 1e-5 ahead of the rounding of the output.)
 //
-// A CTA takes 128 consecutive queries of one head; blocks of 128 keys and values come by tensor copies (two pages rows of 64 each, parts
+// A CTA takes 128 consecutive queries of one head (or, of a short sequence, the queries of several heads that share their keys); blocks of 128 keys and values come by tensor copies (two pages rows of 64 each, parts
 // of 64 columns in 128-byte-swizzled rows, two stages). Tensor memory holds the output (128 columns), two score tiles (2 x 128) and the two
 // halves of the probabilities (64 + 64), which are the A operand of the second product. The next block's scores are computed while
 // this one's softmax runs. Eight softmax warps, two threads a query row with 64 key columns each (capped scores take three special-function
@@ -34,20 +36,34 @@ __device__ __forceinline__ void sx_split(float a, float b, uint32_t& hi, uint32_
 }
 }  // namespace
 
-// grid (heads, 64-query tiles of the step, latest first; odd tiles of a sequence belong to the CTA before them)
-template <bool CAP>
+// A sequence of up to 2^k <= 64 tokens shares a CTA between heads[k] query heads of a key/value head, rows token by token; its tiles start at
+// tile0[k], its CTAs at cta0[k]
+struct SxShort { int tile0[7], cta0[7], heads[7]; };
+
+// CTAs: (64-query tile, head) of longer sequences, latest tiles first (odd tiles of a sequence belong to the CTA before them), then (sequence,
+// group of heads) of the others, the longest first. SHORT: there are such (2048 tokens of one sequence take 85 us a layer without that part
+// and 89 with it, preparation included)
+template <bool CAP, bool SHORT>
 __global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-                                                                   const SoftmaxTcArgs a, const RaggedDev r, unsigned int* err) {
+                                                                   const SoftmaxTcArgs a, const RaggedDev r, const __grid_constant__ SxShort sh, unsigned int* err) {
     extern __shared__ uint8_t sx_smem[];
     __shared__ uint64_t k_full[2], k_empty[2], v_full[2], v_empty[2], q_full, s_full[2], p_full, pv_done;
     __shared__ uint32_t tmem_at;
     __shared__ float row_max[2][2][SX_Q], row_sum[2][SX_Q];
-    const int tile = r.n_tiles - 1 - (int)blockIdx.y, h = blockIdx.x;
+    int tile = r.n_tiles - 1 - (int)blockIdx.x / a.H, h = (int)blockIdx.x % a.H, per_tok = 1;      // per_tok: rows of a token, heads h ..
+    if (const int in_short = (int)blockIdx.x - (r.n_tiles - r.n_upto[6]) * a.H; SHORT && in_short >= 0) {
+        int k = 6;
+        while (k > 0 && in_short >= sh.cta0[k - 1]) k--;
+        per_tok = sh.heads[k];
+        tile = sh.tile0[k] + (in_short - sh.cta0[k]) / (a.H / per_tok);
+        h = (in_short - sh.cta0[k]) % (a.H / per_tok) * per_tok;
+    }
     const int seg = r.tile_seg[tile], row0 = r.tile_row0[tile];
     if (((row0 - r.seg_start[seg]) / 64) & 1) return;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (warp: known to be uniform)
-    const int nq = min(SX_Q, r.seg_start[seg] + r.seg_len[seg] - row0);
-    const int p0 = r.seg_pos0[seg] + row0 - r.seg_start[seg], p_last = p0 + nq - 1;
+    const int n_tok = min(SX_Q, r.seg_start[seg] + r.seg_len[seg] - row0);
+    const int nq = n_tok * per_tok, n_thr = SHORT ? (nq + 31) / 32 * 64 : 2 * SX_Q;      // rows in use; softmax threads: two a row, whole warps
+    const int p0 = r.seg_pos0[seg] + row0 - r.seg_start[seg], p_last = p0 + n_tok - 1;
     const int* table = a.block_tables[r.seg_slot[seg]];
     const int g = h / (a.H / a.G), bt = a.block_tokens;
     const int k_parts = (a.d + 63) / 64, v_parts = (a.dv + 63) / 64;
@@ -64,7 +80,7 @@ __global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_
             for (int i = 0; i < 2; i++) {
                 mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); mbar_init(&s_full[i], 1);
             }
-            mbar_init(&q_full, 256); mbar_init(&p_full, 256); mbar_init(&pv_done, 1);
+            mbar_init(&q_full, n_thr); mbar_init(&p_full, n_thr); mbar_init(&pv_done, 1);
             fence_mbar_init();
         }
         __syncwarp();
@@ -131,9 +147,11 @@ __global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_
             tc_commit(&pv_done);
             tc_commit(&v_empty[i & 1]);
         }
-    } else if (warp < 8) {
+    } else if (warp < 8 && (warp & 3) * 64 < n_thr) {
         // ================= softmax: threads t and t + 128 share query row t, key columns 0-63 and 64-127 of a block
-        const int row = threadIdx.x & 127, side = threadIdx.x >> 7, pos = p0 + row;
+        const int row = threadIdx.x & 127, side = threadIdx.x >> 7, tok = SHORT ? row / per_tok : row, pos = p0 + tok;
+        const int t = row0 + tok, hd = SHORT ? h + row % per_tok : h;      // the row's token and query head
+        const int thr = side * (n_thr / 2) + row;
         const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
         constexpr float LOG2E = 1.4426950408889634f;
         // scores live in the log2 domain. Capped: cap tanh(s / cap) = cap - 2 cap / (exp(2 s / cap) + 1), the exponential's factor folded
@@ -142,11 +160,11 @@ __global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_
         [[maybe_unused]] const float cap2 = CAP ? a.softcap * LOG2E : 0.f;
         {   // queries, 8 columns at a time: neighbouring threads take neighbouring pieces of a row
             const int per = k_parts * 8, d8 = a.d / 8;
-            for (int e = threadIdx.x; e < SX_Q * per; e += 256) {
+            for (int e = thr; e < n_thr / 2 * per; e += n_thr) {
                 const int rr = e / per, c8 = e % per;
                 float v[8] = {};
                 if (rr < nq && c8 < d8) {
-                    const float4* src = reinterpret_cast<const float4*>(a.q + ((size_t)(row0 + rr) * a.H + h) * a.d + c8 * 8);
+                    const float4* src = reinterpret_cast<const float4*>(a.q + (SHORT ? (size_t)(row0 + rr / per_tok) * a.H + h + rr % per_tok : (size_t)(row0 + rr) * a.H + h) * a.d + c8 * 8);
                     const float4 x = src[0], y = src[1];
                     v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
                 }
@@ -160,7 +178,7 @@ __global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_
             fence_proxy_async();
             mbar_arrive(&q_full);
         }
-        const float sink = a.sink ? a.sink[h] * LOG2E : -INFINITY;
+        const float sink = a.sink ? a.sink[hd] * LOG2E : -INFINITY;
         float m_ref = sink, l = 0.f;                              // weights are 2^(score - m_ref); the sink's term joins at the end
         const int lo_key = a.window > 0 ? max(0, pos - a.window + 1) : 0;
         for (int i = 0; i < n_blocks; i++) {
@@ -188,7 +206,7 @@ __global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_
 #pragma unroll
             for (int j = 0; j < 64; j++) mx = fmaxf(mx, s[j]);
             row_max[i & 1][side][row] = mx;
-            named_bar_sync(1, 256);
+            named_bar_sync(1, n_thr);
             mx = fmaxf(mx, row_max[i & 1][side ^ 1][row]);
             const bool grow = mx > m_ref + 8.f || (m_ref == -INFINITY && mx > -INFINITY);
             // the previous block's products must be in before the output is rescaled and the probabilities are rewritten
@@ -224,7 +242,7 @@ __global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_
                 // rows past the sequence: whatever shared memory or the page holds must not meet the zero weights as values
                 mbar_wait(&v_full[i & 1], (i >> 1) & 1, err, 0x70008u, (unsigned)i);
                 const int r0 = p_last - j0 + 1, n_bad = SX_K - r0;
-                for (int e = threadIdx.x; e < v_parts * n_bad * 8; e += 256) {
+                for (int e = thr; e < v_parts * n_bad * 8; e += n_thr) {
                     const int c = e / (n_bad * 8), rr = r0 + e / 8 % n_bad;
                     *reinterpret_cast<uint4*>(vs + (size_t)((i & 1) * v_parts + c) * SX_PART + rr * 128 + (e & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
                 }
@@ -234,15 +252,15 @@ __global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_
             mbar_arrive(&p_full);
         }
         row_sum[side][row] = l;
-        named_bar_sync(1, 256);
+        named_bar_sync(1, n_thr);
         l += row_sum[side ^ 1][row];
         if (a.sink) l += sx_exp2(sink - m_ref);
         const float inv = l > 0.f ? 1.f / l : 0.f;
         mbar_wait(&pv_done, (n_blocks - 1) & 1, err, 0x70009u);
         tc_after_sync();
-        const int t = row0 + row, dv = a.dv;
-        const size_t at = (size_t)t * a.ld_out + (size_t)h * dv;
-        const float* gate = a.gate && row < nq ? a.gate + (size_t)t * a.ld_gate + (a.gate_per_head ? h : h * dv) : nullptr;
+        const int dv = a.dv;
+        const size_t at = (size_t)t * a.ld_out + (size_t)hd * dv;
+        const float* gate = a.gate && row < nq ? a.gate + (size_t)t * a.ld_gate + (a.gate_per_head ? hd : hd * dv) : nullptr;
         const float head_gate = gate && a.gate_per_head ? 1.f / (1.f + expf(-gate[0])) : 1.f;
         for (int c = side * 64; c < min(side * 64 + 64, dv); c += 32) {
             uint32_t o[32];
@@ -281,11 +299,12 @@ __global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_
 }
 
 // ---------------------------------------------------------------- host side
-// Steps whose sequences bring at least 256 tokens each on average. 16 heads of 128 (us a launch, mma.sync / here): 128 tokens 54 / 18, 256 61 /
-// 17, 384 63 / 22; over a window 28 / 23, 39 / 18, 49 / 20. The line is not where the times cross, which is lower: the two kernels round
-// differently (where a probability is split depends on the running maximum), and answers to short prompts stay what they were. Sizes that the tiles and 16-byte stores take, pages of whole 64-key halves.
-bool softmax_takes_tc(const SoftmaxTcArgs& a, int T, int n_seg) {
-    return T >= 256 * n_seg && a.d % 16 == 0 && a.dv % 16 == 0 && a.d <= 128 && a.dv <= 128 && a.block_tokens % 64 == 0 && a.ld_out % 8 == 0 &&
+// Sizes that the tiles and 16-byte stores take, pages of whole 64-key halves; nothing of the step, so that a row goes to the same kernel
+// whatever shares its step and wherever its prompt was cut. 16 heads of 128 over 4, us a layer with the preparation, mma.sync / here, capped |
+// over a window of 1024: a prompt of 9 tokens 30 / 24 | 24 / 23, of 64 44 / 24 | 33 / 24, of 255 53 / 26 | 54 / 28; 32 prompts of 16 72 / 33 |
+// 47 / 27, of 60 110 / 56 | 66 / 49; 512 tokens beside 31 sequences that decode behind 500, 168 / 75 | 148 / 46.
+bool softmax_takes_tc(const SoftmaxTcArgs& a) {
+    return a.d % 16 == 0 && a.dv % 16 == 0 && a.d <= 128 && a.dv <= 128 && a.block_tokens % 64 == 0 && a.ld_out % 8 == 0 &&
            ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.out) | reinterpret_cast<uintptr_t>(a.out_bf16)) & 15) == 0;
 }
 
@@ -293,16 +312,31 @@ cudaError_t softmax_tc_launch(const SoftmaxTcArgs& a, const RaggedDev& r, cudaSt
     const int k_parts = (a.d + 63) / 64, v_parts = (a.dv + 63) / 64;
     static const bool ready = [] {
         const int most = 12 * SX_PART + 1024;
-        return cudaFuncSetAttribute(softmax_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess &&
-               cudaFuncSetAttribute(softmax_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess;
+        bool ok = true;
+        for (auto kernel : {softmax_tc_kernel<false, false>, softmax_tc_kernel<false, true>, softmax_tc_kernel<true, false>, softmax_tc_kernel<true, true>})
+            ok = ok && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess;
+        return ok;
     }();
-    if (!ready || !softmax_takes_tc(a, r.T, r.n_seg)) return cudaErrorInvalidValue;
+    if (!ready || !softmax_takes_tc(a)) return cudaErrorInvalidValue;
     CUtensorMap mk, mv;
     if (!bf16_rows_map(&mk, a.k_pool, a.d, a.pool_rows, a.d, 1, 0, 64) || !bf16_rows_map(&mv, a.v_pool, a.dv, a.pool_rows, a.dv, 1, 0, 64)) return cudaErrorInvalidValue;
     const size_t smem = (size_t)(4 * k_parts + 2 * v_parts) * SX_PART + 1024;
-    const dim3 grid(a.H, r.n_tiles), block(SX_THREADS);
-    return a.softcap > 0.f ? launch_chain(softmax_tc_kernel<true>, grid, block, smem, s, mk, mv, a, r, kernel_error_word())
-                           : launch_chain(softmax_tc_kernel<false>, grid, block, smem, s, mk, mv, a, r, kernel_error_word());
+    // heads a CTA: 32 sequences of 2 tokens, 16 heads over 4, 53 us with one and 24 with four; of 40 tokens, 60 with one and 45 with two
+    SxShort sh = {};
+    int ctas = 0;
+    for (int k = 6; k >= 0; k--) {
+        int heads = std::min(a.H / a.G, SX_Q >> k);
+        while (a.H / a.G % heads) heads--;
+        sh.heads[k] = heads;
+        sh.tile0[k] = std::max(k ? r.n_upto[k - 1] : 0, a.skip);
+        sh.cta0[k] = ctas;
+        ctas += (r.n_upto[k] - sh.tile0[k]) * (a.H / heads);
+    }
+    const dim3 grid((r.n_tiles - r.n_upto[6]) * a.H + ctas), block(SX_THREADS);
+    if (grid.x == 0) return cudaSuccess;
+    const auto kernel = a.softcap > 0.f ? (ctas ? softmax_tc_kernel<true, true> : softmax_tc_kernel<true, false>)
+                                        : (ctas ? softmax_tc_kernel<false, true> : softmax_tc_kernel<false, false>);
+    return launch_chain(kernel, grid, block, smem, s, mk, mv, a, r, sh, kernel_error_word());
 }
 
 }  // namespace b2

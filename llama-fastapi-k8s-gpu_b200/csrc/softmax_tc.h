@@ -1,4 +1,4 @@
-// Softmax attention of long steps on the tensor cores (softmax_tc.cu), shared by the mixers of the layer-list models.
+// Softmax attention of steps of more than 8 tokens on the tensor cores (softmax_tc.cu), shared by the mixers of the layer-list models.
 #pragma once
 #include "layered.h"
 
@@ -15,8 +15,9 @@ struct SoftmaxTcArgs {
     const float* sink;                                 // [H] or null
     const float* gate; int ld_gate; int gate_per_head; // sigmoid output gate or null (as in SinkAttnArgs)
     float* out; __nv_bfloat16* out_bf16; int ld_out;   // out[t][h * dv + i], or rounded
+    int skip;                                          // leading tiles of the step that are not this launch's (at most the one-token ones)
 };
-bool softmax_takes_tc(const SoftmaxTcArgs& a, int T, int n_seg);
+bool softmax_takes_tc(const SoftmaxTcArgs& a);
 cudaError_t softmax_tc_launch(const SoftmaxTcArgs& a, const RaggedDev& r, cudaStream_t s);
 
 }  // namespace b2

@@ -9,7 +9,7 @@ bool bf16_rows_map(CUtensorMap* m, const void* base, long cols, long rows, long 
 // the same as [nb][cols / 64][rows][64] (cols a multiple of 64): boxes of `slices` 64-entry slices of box_rows rows; coordinates
 // (0, row, slice, entry)
 bool bf16_slices_map(CUtensorMap* m, const void* base, long cols, long rows, long ld, long nb, long bs, int box_rows, int slices);
-// [rows][heads][cols]: boxes of 64 columns of one head, box_rows rows; coordinates (column, head, row)
-bool bf16_heads_map(CUtensorMap* m, const void* base, long cols, long heads, long rows, int box_rows);
+// [rows][heads][cols]: boxes of 64 columns of box_heads heads, box_rows rows; coordinates (column, head, row)
+bool bf16_heads_map(CUtensorMap* m, const void* base, long cols, long heads, long rows, int box_heads, int box_rows);
 
 }  // namespace b2

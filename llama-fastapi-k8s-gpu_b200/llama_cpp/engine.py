@@ -322,7 +322,9 @@ class LayeredEngine(EngineBase):
         """One ragged step. entries: [(slot, [token, ...]), ...]; want: per entry, indices into its tokens whose logits are
         asked for; sample: per entry, whether to sample after its last token. Returns (logits [n_wanted, n_vocab] in entry
         order, [sampled token or None per entry]). A batch larger than `max_step_tokens` is run as several native steps,
-        cutting entries where needed (the result does not depend on the cut)."""
+        cutting entries where needed. What an entry's rows give does not depend on the entries beside it, nor on the cut, as long as every
+        native step has more than 8 tokens and no cut leaves one token alone (such steps and tokens take kernels of their own, which
+        round elsewhere)."""
         n = len(entries)
         want = want if want is not None else [[] for _ in entries]
         sample = sample if sample is not None else [False] * n

@@ -1,7 +1,8 @@
-"""Kernels that only long steps, one-token steps or certain sizes reach, through one-layer models against the float64 oracles: the
-tensor-memory attention kernels (256 tokens a sequence and more) at the edges of their 128-row tiles and 64-key blocks, the scan at each of
+"""Kernels that only longer steps, one-token steps or certain sizes reach, through one-layer models against the float64 oracles: the
+tensor-memory attention kernels (steps of more than 8 tokens) at the edges of their 128-row tiles and 64-key blocks, the scan at each of
 its state sizes and at lengths around its blocks of 16 and runs of 8 tokens, the matrix memory at partial rows and columns, steps of one
-token per sequence at each count of heads that share a key, sampling more rows than a block, and a replayed step against the first one."""
+token per sequence at each count of heads that share a key, more wanted rows than a head chunk, a replayed step against the first one, and
+a token's bits alone, in company and under other cuts."""
 import numpy as np
 import pytest
 
@@ -17,10 +18,10 @@ pytestmark = pytest.mark.gpu
 F32, BF16 = 3e-4, 6e-2
 
 
-def engine(path, dtype, tokens, seqs=1):
+def engine(path, dtype, tokens, seqs=1, **kw):
     from llama_cpp import models
     return models.open_engine(models.open_model(path), n_ctx=max(tokens + 16, 64), max_seqs=seqs, dtype=dtype, kv_tokens=(tokens + 128) * seqs,
-                              max_step_tokens=max(tokens * seqs, 16))
+                              max_step_tokens=max(tokens * seqs, 16), **kw)
 
 
 def whole(eng, prompts):
@@ -61,25 +62,38 @@ def check(util, ref, cfg, tmp_path, lengths, dtype):
 
 
 @pytest.mark.parametrize("dims,lengths", [((16, 16), [256]), ((32, 48), [257]), ((64, 64), [383]), ((80, 128), [385]), ((128, 80), [300, 260]),
-                                          ((128, 128), [640]), ((64, 32), [500, 12])])
-def test_softmax_attention_of_long_steps(native_lib, tmp_path, dims, lengths):
+                                          ((128, 128), [640]), ((64, 32), [500, 12]), ((32, 32), [9]), ((48, 16), [1, 2, 3, 4, 5, 16, 17, 32, 33, 63, 64, 65])])
+@pytest.mark.parametrize("heads,kv", [(4, 2), (6, 1)])
+def test_softmax_attention_of_long_steps(native_lib, tmp_path, dims, lengths, heads, kv):
     d, dv = dims
-    cfg = zu.config([zu.biased(heads=4, kv_heads=2, dim=d, vdim=dv)])
+    cfg = zu.config([zu.biased(heads=heads, kv_heads=kv, dim=d, vdim=dv)])
     check(zu, zogurax_ref, cfg, tmp_path, lengths, "bfloat16")
 
 
-@pytest.mark.parametrize("d,window,keep,lengths", [(16, 1, 0, [256]), (64, 64, 3, [257]), (80, 100, 70, [400]), (128, 129, 1, [511]), (32, 1000, 4, [300, 280])])
+@pytest.mark.parametrize("d,window,keep,lengths", [(16, 1, 0, [256]), (64, 64, 3, [257]), (80, 100, 70, [400]), (128, 129, 1, [511]), (32, 1000, 4, [300, 280]),
+                                                  (32, 20, 2, [1, 2, 31, 33, 64, 65])])
 def test_window_attention_of_long_steps(native_lib, tmp_path, d, window, keep, lengths):
     cfg = gu.config([gu.parallel(left=gu.attn(heads=4, kv_heads=2, dim=d, rot=8, window=window, keep=keep))])
     check(gu, goponex_ref, cfg, tmp_path, lengths, "bfloat16")
 
 
-@pytest.mark.parametrize("rank,heads,lengths", [(64, 3, [256]), (128, 4, [257]), (192, 2, [385]), (256, 2, [511]), (512, 2, [300, 290])])
+# (head sizes that are multiples of 8: the products around the attention take rounded rows, without which the general kernel runs)
+LATENT = {"plain": lambda heads, rank, **kw: fu.plain(heads=heads, rank=rank, dim=24, vdim=16, **kw),
+          "rotated": lambda heads, rank, **kw: fu.rotated(heads=heads, rank=rank, dim=24, vdim=16, rot_dim=16, **kw)}
+
+
+@pytest.mark.parametrize("rank,heads,lengths", [(64, 3, [256]), (128, 4, [257]), (192, 2, [385]), (256, 2, [511]), (512, 2, [300, 290]), (64, 2, [9]), (512, 3, [65, 1, 2]),
+                                                (128, 5, [129, 64, 1])])
 @pytest.mark.parametrize("kind", ["plain", "rotated"])
 def test_latent_attention_of_long_steps(native_lib, tmp_path, kind, rank, heads, lengths):
-    layer = fu.plain(heads=heads, rank=rank) if kind == "plain" else fu.rotated(heads=heads, rank=rank, rot_dim=16)
-    layers = [layer] + ([fu.plain(heads=heads, rank=rank, kv_from=0)] if kind == "plain" else [])
+    layers = [LATENT[kind](heads, rank)] + ([LATENT[kind](heads, rank, kv_from=0)] if kind == "plain" else [])
     check(fu, fazovik_ref, fu.config(layers), tmp_path, lengths, "bfloat16")
+
+
+@pytest.mark.parametrize("rank,heads", [(64, 3), (128, 1), (512, 16)])
+@pytest.mark.parametrize("kind", ["plain", "rotated"])
+def test_latent_attention_of_one_token_of_every_sequence(native_lib, tmp_path, kind, rank, heads):
+    decode_all(fu, fazovik_ref, fu.config([LATENT[kind](heads, rank)]), tmp_path)
 
 
 @pytest.mark.parametrize("state,inner,conv,lengths", [(1, 24, 2, [67]), (4, 64, 3, [16, 63]), (5, 65, 4, [64]), (8, 40, 4, [9, 70, 3]), (13, 130, 2, [129]),
@@ -96,15 +110,13 @@ def test_matrix_memory_sizes(native_lib, tmp_path, heads, d, dv, lengths):
     check(gu, goponex_ref, cfg, tmp_path, lengths, "float32")
 
 
-@pytest.mark.parametrize("heads,kv,d,dv", [(4, 4, 16, 16), (6, 2, 32, 48), (16, 4, 128, 128), (16, 1, 64, 80), (17, 1, 64, 64), (9, 1, 112, 32)])
-def test_one_token_of_every_sequence(native_lib, tmp_path, heads, kv, d, dv):
-    """Steps that decode all sequences: each key/value head's query rows in one tile, keys across one to three blocks of 64."""
+def decode_all(util, ref, cfg, tmp_path, **kw):
+    """Steps that decode all sequences, keys across one to three blocks of 64."""
     from llama_cpp.kv_pages import SequenceSlots
-    cfg = zu.config([zu.biased(heads=heads, kv_heads=kv, dim=d, vdim=dv)])
-    w = zu.random_weights(cfg, seed=6)
+    w = util.random_weights(cfg, seed=6)
     lengths = [1, 2, 63, 64, 65, 127, 128, 130, 20, 40]
     prompts = [toks(cfg["vocab"], n + 2, 30 + i) for i, n in enumerate(lengths)]
-    eng = engine(zu.write_model(str(tmp_path / "m"), cfg, w), "bfloat16", 136, len(lengths))
+    eng = engine(util.write_model(str(tmp_path / "m"), cfg, w), "bfloat16", 136, len(lengths), **kw)
     seqs = SequenceSlots(eng)
     for i in range(len(lengths)):
         seqs.open(i)
@@ -112,7 +124,84 @@ def test_one_token_of_every_sequence(native_lib, tmp_path, heads, kv, d, dv):
     got = [np.array(eng.step([(seqs.extend(i, 1), [p[n + k]]) for i, (n, p) in enumerate(zip(lengths, prompts))], want=[[0]] * len(lengths))[0]) for k in range(2)]
     eng.close()
     for i, (n, p) in enumerate(zip(lengths, prompts)):
-        assert rows_off(np.stack([got[0][i], got[1][i]]), zogurax_ref.forward(cfg, w, p)[n:]).max() < BF16, i
+        assert rows_off(np.stack([got[0][i], got[1][i]]), ref.forward(cfg, w, p)[n:]).max() < BF16, i
+
+
+# (17 heads over a key are more than a packed tile holds: a tensor-memory tile, or with pages of 48 a tile for each head)
+@pytest.mark.parametrize("heads,kv,d,dv", [(4, 4, 16, 16), (6, 2, 32, 48), (16, 4, 128, 128), (16, 1, 64, 80), (17, 1, 64, 64), (9, 1, 112, 32)])
+@pytest.mark.parametrize("block", [64, 48])
+def test_one_token_of_every_sequence(native_lib, tmp_path, heads, kv, d, dv, block):
+    """Each key/value head's query rows in one tile."""
+    decode_all(zu, zogurax_ref, zu.config([zu.biased(heads=heads, kv_heads=kv, dim=d, vdim=dv)]), tmp_path, kv_block_tokens=block)
+
+
+def test_windows_of_one_token_of_every_sequence(native_lib, tmp_path):
+    layers = [gu.parallel(left=gu.attn(heads=8, kv_heads=2, dim=32, rot=8, window=w, keep=k)) for w, k in ((1, 0), (50, 3), (100, 70))]
+    decode_all(gu, goponex_ref, gu.config(layers), tmp_path)
+
+
+WHOLE = {
+    "softmax": (zu, lambda: zu.config([zu.biased(heads=8, kv_heads=2, dim=32, vdim=48, mlp=zu.moe()), zu.conved(heads=4, kv_heads=4, dim=64, vdim=32, mlp=zu.moe())])),
+    "latent": (fu, lambda: fu.config([LATENT["rotated"](4, 128), LATENT["plain"](3, 64)])),
+    "window": (gu, lambda: gu.config([gu.parallel(left=gu.attn(heads=8, kv_heads=2, dim=32, rot=8, window=70, keep=5)),
+                                      gu.mlstm(), gu.parallel(left=gu.attn(heads=4, kv_heads=4, dim=64, rot=8, window=200, keep=0))])),
+}
+
+
+@pytest.mark.parametrize("block", [64, 48])
+@pytest.mark.parametrize("kind", sorted(WHOLE))
+def test_company_and_cuts_do_not_change_a_token(native_lib, tmp_path, kind, block):
+    """In steps of more than 8 tokens a prompt's logits have the same bits whole, in portions of two tokens and more, beside other prompts
+    and beside sequences that decode; and so have those of the sequences beside it."""
+    from llama_cpp.kv_pages import SequenceSlots
+    util, make = WHOLE[kind]
+    cfg = make()
+    V, N, others = cfg["vocab"], 300, 12
+    eng = engine(util.write_model(str(tmp_path / "m"), cfg, util.random_weights(cfg, seed=9)), "bfloat16", N + 130, others + 2, kv_block_tokens=block)
+    prompt, side, rest = toks(V, N, 1), toks(V, 90, 2), [toks(V, 80, 10 + i) for i in range(others)]
+
+    def run(cuts, company):
+        """Rows of the prompt and, in company, of the sequences that decode beside each portion (the head's form depends on the number of
+        wanted rows: more than 8 in every step)."""
+        seqs, rows, beside = SequenceSlots(eng), [], []
+        for i in range(others + 2):
+            seqs.open(i)
+        eng.step([(seqs.extend(i + 2, 20 + 5 * i), rest[i][:20 + 5 * i]) for i in range(others)])
+        at = 0
+        for k, n in enumerate(cuts):
+            entries, want = [], []
+            if company:
+                entries += [(seqs.extend(i + 2, 1), [rest[i][20 + 5 * i + k]]) for i in range(others)]
+                want += [[0]] * others
+            entries.append((seqs.extend(0, n), prompt[at:at + n]))
+            want.append(list(range(n)))
+            if company and k == 0:
+                entries.append((seqs.extend(1, len(side)), side))
+                want.append([])
+            lg, _ = eng.step(entries, want=want)
+            at += n
+            beside.append(np.array(lg[:len(lg) - n]))
+            rows.append(np.array(lg[len(lg) - n:]))
+        for i in range(others + 2):
+            seqs.close(i)
+        return np.concatenate(rows), beside
+
+    whole_rows, _ = run([N], False)
+    alone = []                                            # the sequences beside it, decoding by themselves
+    seqs = SequenceSlots(eng)
+    for i in range(others):
+        seqs.open(i)
+    eng.step([(seqs.extend(i, 20 + 5 * i), rest[i][:20 + 5 * i]) for i in range(others)])
+    for k in range(4):
+        alone.append(np.array(eng.step([(seqs.extend(i, 1), [rest[i][20 + 5 * i + k]]) for i in range(others)], want=[[0]] * others)[0]))
+    for i in range(others):
+        seqs.close(i)
+    for cuts, company in [([N], True), ([129, 171], False), ([17, 283], True), ([256, 44], False), ([100, 9, 191], True), ([298, 2], True), ([2, 128, 165, 5], True), ([33, 60, 40, 167], True)]:
+        rows, beside = run(cuts, company)
+        assert np.array_equal(rows, whole_rows), (cuts, company, np.abs(rows - whole_rows).max(-1).argmax())
+        for got, want in zip(beside, alone):
+            assert not company or np.array_equal(got, want), (cuts, np.abs(got - want).max())
+    eng.close()
 
 
 def test_replayed_steps_are_the_first_ones_bits(native_lib, tmp_path):
@@ -139,7 +228,7 @@ def test_replayed_steps_are_the_first_ones_bits(native_lib, tmp_path):
 
 
 def test_many_wanted_rows_and_long_rows(native_lib, tmp_path):
-    """More wanted rows than a head chunk of 256 holds, a vocabulary that is not a multiple of four, sampling from the last row."""
+    """More wanted rows than a head chunk of 256 holds, rows of a width and vocabulary that are not multiples of the usual sizes."""
     cfg = zu.config([zu.biased()], vocab=1001)
     check(zu, zogurax_ref, cfg, tmp_path, [300, 7, 41], "bfloat16")
     cfg = zu.config([zu.biased()], width=4104, vocab=203)
