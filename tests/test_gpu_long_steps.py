@@ -227,6 +227,53 @@ def test_replayed_steps_are_the_first_ones_bits(native_lib, tmp_path):
         assert np.array_equal(runs[0], other)
 
 
+@pytest.mark.parametrize("vocab", [203, 512])
+def test_sampling_in_ragged_steps(native_lib, tmp_path, vocab):
+    """Each slot with settings, uniforms and history of its own: sampled rows on both sides of a head chunk's end, some entries sampled and
+    others not, steps that run directly, that are captured and that are replayed. The oracle draws from the logits the step returns."""
+    from dataclasses import asdict
+    from llama_cpp.engine import SamplingSettings
+    from oracle import sampler_ref
+    cfg = zu.config([zu.biased()], vocab=vocab)
+    n = 10
+    kinds = [SamplingSettings(temperature=0.0, repeat_penalty=1.0), SamplingSettings(temperature=0.9, top_k=20, top_p=0.8, min_p=0.02, repeat_penalty=1.3),
+             SamplingSettings(temperature=1.2, top_p=0.9, frequency_penalty=0.7, presence_penalty=0.8),
+             SamplingSettings(temperature=1.5, top_k=vocab, top_p=1.0, min_p=0.0, repeat_penalty=1.8, penalty_last_n=4), SamplingSettings(temperature=0.0, frequency_penalty=2.0)]
+    settings, uniforms = [kinds[i % 5] for i in range(n)], [sampler_ref.MT19937Uniforms(40 + i).take(64) for i in range(n)]
+    eng = engine(zu.write_model(str(tmp_path / "m"), cfg, zu.random_weights(cfg, seed=5)), "bfloat16", 60, n)
+    hist, drawn, seen, off = [toks(vocab, 25, 60 + i) for i in range(n)], [0] * n, 0, 0
+    for i in range(n):
+        eng.ensure_pages(i, 60)
+        eng.seq_begin(i, 0, hist[i], settings[i], uniforms=uniforms[i])
+
+    def draw(entries, sample, rows):
+        """Tokens of one step; the wanted rows end with every entry's last one."""
+        nonlocal seen, off
+        lg, got = eng.step(entries, want=rows, sample=sample)
+        ends = np.cumsum([len(r) for r in rows]) - 1
+        for i, t in enumerate(got):
+            assert (t is not None) == sample[i]
+            if sample[i]:
+                kw = asdict(settings[i])
+                want = sampler_ref.sample(lg[ends[i]], hist[i], float(uniforms[i][drawn[i]]), **kw)
+                drawn[i] += 1
+                seen, off = seen + 1, off + (want != t)
+                assert want == t or settings[i].temperature > 0.0
+                hist[i].append(t)
+        return got
+
+    last = draw([(i, list(hist[i])) for i in range(n)], [True] * n, [list(range(25))] * n)       # sampled rows 250 .. 259
+    for _ in range(4):
+        last = draw([(i, [last[i]]) for i in range(n)], [True] * n, [[0]] * n)
+    odd = [i % 2 == 1 for i in range(n)]
+    for _ in range(3):
+        got = draw([(i, [last[i] if last[i] is not None else 7]) for i in range(n)], odd, [[0]] * n)
+        last = [t if t is not None else 7 for t in got]
+    last = draw([(i, [last[i]] * (1 + 5 * (i == 3))) for i in range(n)], [True] * n, [[0, 5] if i == 3 else [0] for i in range(n)])
+    eng.close()
+    assert seen == 75 and off <= 1, (seen, off)          # at most one draw at the edge of a 32-bit sum
+
+
 def test_many_wanted_rows_and_long_rows(native_lib, tmp_path):
     """More wanted rows than a head chunk of 256 holds, rows of a width and vocabulary that are not multiples of the usual sizes."""
     cfg = zu.config([zu.biased()], vocab=1001)
