@@ -55,10 +55,6 @@ struct Slot {
     int n_sampled = 0;             // host mirror of ints[3]
 };
 
-// A batched decode step of one list of slots, captured the second time the list is seen: positions, pages and tokens are read from
-// device memory, so nothing in its launches changes from step to step.
-struct BatchGraph { cudaGraphExec_t exec = nullptr; int n_launch = 0; bool failed = false; };
-
 struct b2_engine {
     b2_config cfg;
     cudaStream_t stream = nullptr;
@@ -99,7 +95,6 @@ struct b2_engine {
     float *bd_q = nullptr, *bd_att = nullptr, *bd_scratch = nullptr;
     unsigned* bd_counters = nullptr;
     int* bd_out = nullptr;
-    std::unordered_map<std::string, BatchGraph> batch_graphs;     // replayable batched steps, by their list of slots
     int attn_mma = -1;             // tensor-core flash-decode: -1 = batched steps only; 0 never; 1 always
     int batch_min = 3;             // fewer sequences than this step one after another through the mat-vec path (measured: 3 slots 4.1 vs 6.3 ms)
     bool gemm_ok = false;          // every layer matrix is a block format the GEMM reads
