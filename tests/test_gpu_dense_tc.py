@@ -50,3 +50,32 @@ def test_expert_tiles_match_the_oracle(native_lib, T, experts, top, ff):
     logits, _ = e.step([(0, toks)], want=[list(range(T))])
     e.close()
     _rows_close(logits, zogurax_ref.forward(cfg, _weights(tensors), toks), TOL)
+
+
+@pytest.mark.parametrize("family", ["goponex", "zogurax"])
+def test_a_row_has_the_same_bits_in_steps_of_any_length(native_lib, family):
+    """A prompt whole (token tiles of up to 256, 128-row expert tiles) and in portions that take the other forms (tokens as the 128-row operand,
+    one and two tiles of them, several K slices a copy, 64-row expert tiles, the line at 256 tokens from both sides): no sum changes its order."""
+    from llama_cpp import goponex, zogurax
+    from llama_cpp.engine import SamplingSettings
+    N, V = 1100, 301
+    if family == "goponex":
+        cfg, tensors = goponex.synthetic(264, 2, 1, 520, V, pattern="p", seed=3)
+    else:
+        cfg, tensors = zogurax.synthetic(256, 4, 136, V, pattern="b", experts=8, top=2, seed=3)
+    toks = [int(t) for t in np.random.default_rng(3).integers(0, V, size=N)]
+    e = (goponex if family == "goponex" else zogurax).open_synthetic(cfg, tensors, n_ctx=N + 8, max_seqs=1, dtype="bfloat16", max_step_tokens=N)
+    e.ensure_pages(0, N)
+    got = []
+    for cuts in ([N], [9, 256, 257, 578], [128, 129, 300, 16, 17, 510]):
+        e.seq_begin(0, 0, [], SamplingSettings(temperature=0.0))
+        rows, at = np.full((N, V), np.nan, np.float32), 0
+        for n in cuts:
+            want = [i for i in range(n) if n - n % 256 > i or n % 256 > 8]      # (the head takes rows by 256, and up to 8 of them its own way)
+            rows[[at + i for i in want]] = e.step([(0, toks[at:at + n])], want=[want])[0]
+            at += n
+        got.append(rows)
+    e.close()
+    for other in got[1:]:
+        seen = ~np.isnan(got[0][:, 0]) & ~np.isnan(other[:, 0])
+        assert seen.sum() > 1000 and np.array_equal(other[seen], got[0][seen]), int(np.abs(other - got[0])[seen].max(-1).argmax())

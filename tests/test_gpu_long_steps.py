@@ -14,8 +14,9 @@ from oracle import fazovik_ref, goponex_ref, zogurax_ref
 pytestmark = pytest.mark.gpu
 
 # float32: sums of up to a few hundred terms in another order than the oracle's, amplified by one norm (as in the families' own tests).
-# bfloat16: activations rounded (2^-9) ahead of each of about six products; a lost or doubled block, row or key moves a row by its own size.
-F32, BF16 = 3e-4, 6e-2
+# bfloat16: about a dozen independent roundings of 2^-9 / sqrt(3) on the way of a row, 4e-3 together, several times that in a row whose softmax
+# is sharp or whose norm is small (most seen: 1.4e-2); a lost or doubled block, row or key moves a row by its own size.
+F32, BF16 = 3e-4, 2.5e-2
 
 
 def engine(path, dtype, tokens, seqs=1, **kw):
