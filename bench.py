@@ -1,6 +1,6 @@
 #!/usr/bin/env python
 """Headline benchmark: decode tok/s of the Llama-3-8B-arch Q4_K_M synthetic GGUF at batch 1
-(BASELINE.json configs[1]) on N B200s (N independent replicas, weak scaling).
+on N B200s (N independent replicas, weak scaling).
 
     python bench.py --gpus 1 --steps 256 --warmup 16
     torchrun ... bench.py --gpus N ...            (one rank per GPU)
@@ -10,7 +10,7 @@
 One "step" = one decoded token for one sequence (every weight byte and every live KV byte read
 once). `value` times K steps with CUDA events on the engine's stream with the sequence state
 resident in HBM; `e2e` times the same K tokens through the public `Llama.create_completion`
-call (host token ids in, host text out). See DESIGN.md "Measurement".
+call (host token ids in, host text out).
 """
 from __future__ import annotations
 
@@ -29,14 +29,14 @@ for p in (ROOT, PKG):
         sys.path.insert(0, p)
 
 WORKLOADS = {
-    # name: (arch, ftype, prompt tokens, sequences per step)   -- BASELINE.json configs
+    # name: (arch, ftype, prompt tokens, sequences per step)
     "llama3-8b-q4_k_m-bs1": ("llama-3-8b", "Q4_K_M", 512, 1),
     "tinyllama-1.1b-q4_0-bs1": ("tinyllama-1.1b", "Q4_0", 128, 1),
     "llama3-8b-q8_0-bs1": ("llama-3-8b", "Q8_0", 512, 1),
     "llama3-8b-q8_0-bs32": ("llama-3-8b", "Q8_0", 512, 32),
     "llama3-8b-q4_k_m-bs32": ("llama-3-8b", "Q4_K_M", 512, 32),
     "mistral-7b-q4_k_m-8k": ("mistral-7b", "Q4_K_M", 8192 - 512, 1),
-    "llama3-70b-q4_k_m-tp": ("llama-3-70b", "Q4_K_M", 128, 1),       # configs[4]: tensor parallel over all ranks (N = 1: one GPU)
+    "llama3-70b-q4_k_m-tp": ("llama-3-70b", "Q4_K_M", 128, 1),       # tensor parallel over all ranks (N = 1: one GPU)
     "tiny-q4_k_m-tp": ("tiny", "Q4_K_M", 32, 1),
     "tiny-q4_k_m": ("tiny", "Q4_K_M", 32, 1),
     "tiny-q4_k_m-bs8": ("tiny", "Q4_K_M", 32, 8),
@@ -156,7 +156,7 @@ def ensure_model(arch, ftype, seed=1):
 
 
 def algorithmic_bytes(gguf, ctx_mean):
-    """SURVEY.md 8(d): W_read (all tensors but token_embd, plus one embedding row) + ctx * KV bytes."""
+    """W_read (all tensors but token_embd, plus one embedding row) + ctx * KV bytes."""
     md = gguf.metadata
     total = sum(t.nbytes for t in gguf.tensors.values())
     emb = gguf.tensors["token_embd.weight"]
@@ -268,7 +268,7 @@ def parity_check(eng, path, n_vocab, n_prompt=6, n_new=6, seed=5):
     the C restatement of the reference's llama graph (oracle/cpu_ref.c) over the same tokens: all layers at the benchmark
     geometry, checked inside the benchmark process. The restatement runs in its checker mode (float activations against
     dequantised weights, double accumulation): its timed mode quantises activations to int8 as ggml does, and on a
-    32-layer random-init model that noise alone is ~10% of the logit spread (measured, round 2). Raises if it is off."""
+    32-layer random-init model that noise alone is ~10% of the logit spread (measured). Raises if it is off."""
     import numpy as np
     from llama_cpp.engine import SamplingSettings
     from oracle.cpu_ref import CpuRef
@@ -318,7 +318,7 @@ def parity_check(eng, path, n_vocab, n_prompt=6, n_new=6, seed=5):
 
 
 def tp_workload(args, cfg, path, n_prompt, rank, world, local_rank, barrier, torch, dist):
-    """BASELINE.json configs[4]: ONE model sharded over all ranks (column / row splits of the quantised weights, NCCL
+    """ONE model sharded over all ranks (column / row splits of the quantised weights, NCCL
     all-reduce after attn_output and ffn_down, all-gather of the logits); batch-1 greedy decode. Strong scaling: the work
     is one sequence whatever N is. N = 1 runs the whole model on one GPU (the 70B Q4_K_M file is 42.5 GB)."""
     import numpy as np
@@ -437,7 +437,7 @@ def batch_workload(args, cfg, path, n_prompt, batch, rank, world, local_rank, ba
         # end to end: `batch` concurrent callers of the public API (as /response handlers would be), host ids in, text out
         os.environ["B200_MAX_SEQS"] = str(batch)
         n_new = min(K, 64)
-        # through the HTTP API, as BASELINE.json words it ("continuous batching bs32 via /response"): this rank's replica
+        # through the HTTP API, as a server is used ("continuous batching bs32 via /response"): this rank's replica
         # behind llama_cpp.server (the reference's app with permits / consumers / queue raised from 1 / 1 / 5 to the
         # batch size), `batch` concurrent POST /response over a real socket
         e2e = http_burst(path, batch, rank, barrier)
@@ -1076,7 +1076,7 @@ def main():
                        f"{n_prompt} prompt ids, the prompt pass, K decode steps with per-chunk D2H of the sampled ids, stop "
                        "checks, detokenise; generated tokens / wall time (decode_phase_tok_s = first token to last only)"}
 
-    # ---- the other headline numbers of BASELINE.json on the same model: prompt p50 and 32 sequences per step
+    # ---- the other headline numbers on the same model: prompt p50 and 32 sequences per step
     extra = None
     if not args.ncu_mode and args.batch_extra > 0:
         try:

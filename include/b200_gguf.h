@@ -1,9 +1,9 @@
 /* b200_gguf.h -- C ABI of the B200-native GGUF inference engine (libb200gguf.so).
  *
  * This is the boundary the Python host (`llama_cpp.Llama`, the drop-in for the object that
- * /root/reference/api.py:7,24-28,55-63 drives) sits on, through ctypes. The reference reaches
+ * api.py:7,24-28,55-63 drives) sits on, through ctypes. The reference reaches
  * its engine through llama-cpp-python 0.2.77's ctypes binding of libllama (un-vendored
- * upstream, pinned at /root/reference/docker/Dockerfile.base:30); each entry point below names
+ * upstream, pinned at docker/Dockerfile.base:30); each entry point below names
  * the libllama call(s) of that binding it stands in for. Plain pointers and sizes only; no
  * torch or C++ types cross this line.
  *
@@ -86,7 +86,7 @@ int b2_upload_tensor(b2_engine* e, const char* name, int ggml_type, int64_t ne0,
  * and uploading its shard of every matrix (llama_cpp/tp_shard.py: whole rows of attn_q/k/v, ffn_gate/up and output, K
  * ranges of attn_output and ffn_down cut at 256-element block boundaries). The engine then all-reduces (sum, NCCL) the
  * hidden vector after attn_output and ffn_down and all-gathers the logits. No counterpart in the reference, which only
- * runs independent replicas (/root/reference/helm/values.yaml:17). b2_tp_unique_id: rank 0 makes the 128-byte NCCL id,
+ * runs independent replicas (helm/values.yaml:17). b2_tp_unique_id: rank 0 makes the 128-byte NCCL id,
  * the host distributes it; b2_engine_tp_init: collective over all ranks, after b2_engine_create and before
  * b2_engine_finalize. In this mode prompts and multi-slot steps run through the mat-vec path. */
 int b2_tp_unique_id(void* host_out_128_bytes);
@@ -305,7 +305,7 @@ int b2_engine_tp_mode(b2_engine* e, int* rank, int* world, int* peer_memory);
 int b2_profile_decode_step(b2_engine* e, int slot, float* ms_out, int32_t* launches_out,
                            int64_t* bytes_out);
 
-/* Streaming rate of the decode mat-vec kernel alone (scripts/mv_micro.py): synthetic weight bytes made on the
+/* Streaming rate of the decode mat-vec kernel alone: synthetic weight bytes made on the
  * device, `iters` launches back to back on one stream cycling through n_copies weight sets (size them past the
  * L2), chained by programmatic dependent launch when pdl != 0. mode: 0 store, 1 residual add, 3 fused gate|up
  * (two matrices of n_rows). us_per_launch_out = mean device time per launch (CUDA events). */
@@ -328,7 +328,7 @@ int b2_op_gate_up(int device, int type_gate, const void* host_wg, int type_up, c
 /* Prefill / batched GEMM on the tensor cores (tcgen05, in-shared-memory dequantisation):
  * y[t][n] = (y_in ? y_in[t][n] : 0) + sum_k f16(x[t][k]) * W[n][k]; x [T][K] f32 (rounded to f16 on the device),
  * W [n_rows][K] raw GGUF blocks, T <= 512, K % 256 == 0. Replaces ggml-cuda's dequantise-to-f16 + cublasGemmEx
- * prompt path that create_chat_completion reaches (/root/reference/api.py:55-63).
+ * prompt path that create_chat_completion reaches (api.py:55-63).
  * n_splits: K ranges computed by separate CTAs and added in order (0 = the engine's own choice, else 1..16). */
 int b2_op_gemm(int device, int type, const void* host_w, int n_rows, int K, const float* host_x, int T,
                const float* host_y_in, float* host_y, int n_splits);

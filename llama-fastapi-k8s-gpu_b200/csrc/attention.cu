@@ -1,6 +1,6 @@
 // Split-K flash-decode attention over the paged f16 KV cache (one new token per sequence).
 // Replaces ggml-cuda's mul_mat_vec_p021/nc (K.q), soft_max_f32 and the P.V mat-mul that the
-// reference launches separately per layer (SURVEY.md 2.3 K8-K10), on a paged cache instead of
+// reference launches separately per layer, on a paged cache instead of
 // llama.cpp's contiguous one (H7).
 //
 // Grid = (n_splits, n_kv_heads), 256 threads. A CTA owns one KV head and one slice of the context

@@ -1,7 +1,7 @@
 // Flash-decode attention on the tensor cores, for the cases where the scalar kernel (attention.cu) is bound by
 // instruction issue rather than latency: several sequences per step, and long contexts.
-// Same job as attn_decode_kernel (SURVEY.md 2.3 K8-K10: K.q, soft_max, P.V of llama.cpp's decode step behind
-// /root/reference/api.py:55-63) on the same paged f16 KV cache and the same split-K scratch protocol.
+// Same job as attn_decode_kernel (K.q, soft_max, P.V of llama.cpp's decode step behind
+// api.py:55-63) on the same paged f16 KV cache and the same split-K scratch protocol.
 //
 // Grid (n_splits, n_kv_heads, sequences), 4 warps. The MMA's 16 rows are the G <= 8 query heads of one KV head
 // (rows G..15 are zero padding): one m16n8k16 covers 16 heads x 8 positions x 16 dims, ~12x fewer instructions per

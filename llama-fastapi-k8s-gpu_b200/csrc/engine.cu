@@ -2,7 +2,7 @@
 // Owns the device copies of the GGUF tensors (raw quant blocks, unchanged), the paged f16 KV pool,
 // per-slot activation buffers and the captured CUDA graphs of one decode / prefill step.
 // Stands in for libllama's llama_model + llama_context behind llama-cpp-python's Llama object
-// (/root/reference/api.py:24-28,55-63).
+// (api.py:24-28,55-63).
 #include "engine_state.h"
 #include "layered.h"
 #include "ptx.cuh"
@@ -797,14 +797,14 @@ extern "C" int b2_prefill(b2_engine* e, int slot, const int32_t* tokens, int n) 
 __global__ void set_ints_kernel(int* ints, int tok, int pos) { if (tok >= 0) ints[0] = tok; ints[1] = pos; }
 
 // enqueue: sample from the slot's logit buffer (the token at position n_past - 1 was the last one evaluated); the token
-// lands in e->pinned[pinned_index] once the stream has been synchronised
-static int sample_enqueue(b2_engine* e, Slot& s, int pinned_index) {
+// lands in e->pinned[0] once the stream has been synchronised
+static int sample_enqueue(b2_engine* e, Slot& s) {
     // sampler bumps pos: make it point at the last evaluated token first
     set_ints_kernel<<<1, 1, 0, e->stream>>>(s.ints, -1, s.n_past - 1);
     CK(sample_launch(s.logits, e->cfg.n_vocab, s.sp, s.sst, s.uniforms, s.ints + 3, s.ints + 2, s.ints + 0,
                      s.ints + 1, s.ring, e->cfg.n_ctx + 1, e->stream, false));
     e->launches += 2;
-    CK(cudaMemcpyAsync(e->pinned + pinned_index, s.ints + 2, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
+    CK(cudaMemcpyAsync(e->pinned, s.ints + 2, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
     s.n_sampled += 1;
     return B2_OK;
 }
@@ -814,7 +814,7 @@ extern "C" int b2_sample(b2_engine* e, int slot, int32_t* out) {
     std::lock_guard<std::mutex> lk(e->mu);
     Slot& s = e->slots[slot];
     CK(cudaSetDevice(e->cfg.device));
-    if ((rc = sample_enqueue(e, s, 0))) return rc;
+    if ((rc = sample_enqueue(e, s))) return rc;
     CK(cudaStreamSynchronize(e->stream));
     if (out) *out = e->pinned[0];
     return B2_OK;

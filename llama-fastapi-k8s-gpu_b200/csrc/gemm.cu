@@ -1,8 +1,8 @@
 // Prefill / batched-decode GEMM on the 5th-generation tensor cores:
 //     P[s][t][n] = sum_{k in split s} X[t][k] * W[n][k]      X: f16 activations, W: GGUF-quantised [N][K]
 // Replaces ggml-cuda's "dequantise the whole matrix to an f16 scratch copy, then cublasGemmEx" prompt
-// path (convert.cu + cuBLAS; SURVEY.md 2.3 K5) that llama-cpp-python runs under create_chat_completion
-// (/root/reference/api.py:55-63), and its batched mul_mat_q path for several sequences per step. No f16 copy
+// path (convert.cu + cuBLAS) that llama-cpp-python runs under create_chat_completion
+// (api.py:55-63), and its batched mul_mat_q path for several sequences per step. No f16 copy
 // of W ever exists in HBM: quant blocks go from HBM over shared memory and registers to the operand of the MMA.
 //
 // Work decomposition. A CTA owns 256 weight rows (two halves of 128, the MMA's M and the lanes of tensor memory) of one of up to three
@@ -23,9 +23,9 @@
 //   epilogue: the 16 warps read their TMEM lanes (tcgen05.ld 32x32b.x16) and store float32, token-major.
 // Shared-memory operand layout (activations): K-major, no swizzle: 8x8 f16 core matrices (8 rows x 16 B), LBO = byte stride between core
 // matrices along K, SBO = stride between 8-row groups (128 B).
-// Why the weights go to tensor memory: with both operands in shared memory a block of 256 rows costs that memory 32 KB of stores and 48 KB
-// of operand reads for 32 tokens (tokens as the 128-row operand), 96 KB of reads for 256 tokens: 800 and 1400 cycles of its 128 bytes a
-// cycle, against 512 and 1024 of products. The expansion itself needs about 500 with 16 warps (950 with 8, two a scheduler).
+// Why the weights go to tensor memory: with both operands in shared memory a block of 256 rows costs that memory 9 KB of raw Q4_K written and
+// read again, 32 KB of expanded weights stored, and for 32 tokens 4 KB of activations and 48 KB of operand reads (tokens as the 128-row
+// operand), for 256 tokens 32 KB and 96 KB: 102 and 178 KB, 800 and 1400 cycles of its 128 bytes a cycle, against 512 and 1024 of products. The expansion itself needs about 500 with 16 warps (950 with 8, two a scheduler).
 // 32 sequences, 4 layers of 4096 (Q8_0), mean product: 23.1 us with both operands in shared memory and 8 warps; 25.7 with 16; 27 with the
 // weights in tensor memory (the MMA thread, one lane of a busy scheduler, took 1200 cycles a block); 17.5 with that loop run by the whole
 // warp and one lane issuing. A 37-token prompt: 9.7 -> 7 us a product.
@@ -316,7 +316,7 @@ struct GemmBars {
 };
 static_assert(sizeof(GemmBars) <= GM_HDR, "barrier header");
 
-// (tma_load_2d is in ptx.cuh: box (inner = one 256-weight span of a row, outer = 128 rows) -> dense [128][box bytes] in smem)
+// (tma_load_2d is in ptx.cuh: box (inner = one 256-weight span of a row, outer = 256 rows) -> dense [256][box bytes] in smem)
 
 // words of one 64-weight block inside the 256-weight span W (registers; c is a compile-time constant after unrolling)
 template <int C>
@@ -687,7 +687,7 @@ int gemm_plan(GemmParams& p, int n_sms, int max_splits) {
         if ((box / 16) % 2 == 0 || g.type == T_Q6_K) box = g.type == T_Q6_K ? 240 : box + 16;   // Q6_K: room for the 14-byte misalignment
         g.box_bytes = box;
         g.use_tma = 0;
-        const bool fast_type = g.type == T_Q4_0 || g.type == T_Q8_0 || g.type == T_Q4_K || g.type == T_Q5_K || g.type == T_Q6_K;   // the others: dequant_store_generic
+        const bool fast_type = g.type == T_Q4_0 || g.type == T_Q8_0 || g.type == T_Q4_K || g.type == T_Q5_K || g.type == T_Q6_K;   // the others: dequant_block_generic
         if (fast_type && !no_tma && g_encode && g.row_bytes % 16 == 0 && ((uintptr_t)g.w & 15) == 0 && (g.type != T_Q6_K || !getenv("B2_GEMM_Q6K_DIRECT"))) {
             const cuuint64_t dims[2] = {(cuuint64_t)g.row_bytes / 2, (cuuint64_t)g.n_rows};
             const cuuint64_t strides[1] = {(cuuint64_t)g.row_bytes};

@@ -164,7 +164,7 @@ struct GemmParams {
     int ldy;
     long split_stride;
     unsigned int* err;
-    long long* dbg;         // optional: CTA 0 records clock64() per K block (8 slots each), scripts/gemm_micro.py
+    long long* dbg;         // optional: CTA 0 records clock64() per K block (8 slots each; b2_op_gemm with B2_GEMM_DBG)
     int n_tiles, n_splits, n_stages, n_bstages, n_raw;   // filled by gemm_plan
     int n_tt, t_tile, ss;   // token tiles of a step and the tokens of one (a multiple of 16); expanded weights in shared memory
 };

@@ -111,7 +111,7 @@ cudaError_t postsum_norm_launch(float* x, const float* a, const float* wa, const
 // y may be x itself.
 cudaError_t resid_rms_norm_launch(float* x, const float* add, float mult, const float* w, float w_offset, float out_scale,
                                   float eps, int W, int T, float* y, cudaStream_t s);
-// plain layer norm: y[t] = LN(x[t]) * w (+ b)
+// plain layer norm of gathered rows: y[i] = LN(x[rows[i]]) * w (+ b)
 cudaError_t layer_norm_rows_launch(const float* x, const int* rows, const float* w, const float* b, float eps, int W, int n, float* y, cudaStream_t s);
 
 struct RotaryTable {           // cos and sin of position * frequency (frequencies already blended, magnitude factor folded

@@ -1,7 +1,7 @@
 // Decode mat-vec with in-kernel dequantisation: y = W x for GGUF-quantised W (Q4_0, Q8_0, Q4_K,
 // Q5_K, Q6_K), weights streamed unchanged from HBM. Replaces ggml-cuda's quantize_q8_1 +
 // mul_mat_vec_q + the separate rms_norm / rope / cpy / silu / add launches that the reference
-// runs under llm.create_chat_completion (/root/reference/api.py:55-63; SURVEY.md 2.3 K2-K7,K11).
+// runs under llm.create_chat_completion (api.py:55-63).
 //
 // Structure: one CTA per SM, 19 consumer warps + 1 TMA producer warp (20 warps x 96 registers fill the register file),
 // the SM's shared memory as a ring of tiles.
@@ -21,7 +21,7 @@
 //     loads its 64 quantised activations (two int8 planes + packed scales) from shared memory and reuses them
 //     for the 4 rows; weights stay packed and go through dp4a. A warp only ever waits on its own tile's
 //     mbarrier: no block-wide barrier in the main loop.
-//     (A round-2 rewrite with warp teams owning K-slices, register-resident activations and last-reader refill
+//     (A rewrite with warp teams owning K-slices, register-resident activations and last-reader refill
 //     was faster in a back-to-back micro-benchmark and slower inside the decode step -- 2.30 against 2.10 ms per
 //     token on the same box -- because refills depended on the slowest reader and teams finished unevenly.)
 //   * Row sums. A tile's 4 row sums are reduced over the lanes (transposed butterfly). Groups that span several

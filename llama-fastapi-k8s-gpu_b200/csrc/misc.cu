@@ -1,6 +1,6 @@
 // Small kernels: block dequantisation (bit-exact vs gguf-py), embedding-row gather, RMSNorm.
 // Replace ggml-cuda's dequantize_block_* (convert.cu), the host-side get_rows of token_embd and
-// rms_norm_f32 + mul that the reference path uses (SURVEY.md 2.3 K1, K2, K5).
+// rms_norm_f32 + mul that the reference path uses.
 #include "kernels.h"
 #include "ptx.cuh"
 #include "quant_blocks.cuh"

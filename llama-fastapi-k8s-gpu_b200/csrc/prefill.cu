@@ -1,7 +1,7 @@
 // Prompt-processing (prefill) kernels around the tensor-core GEMM (gemm.cu): T tokens of one sequence at once.
 // Replaces the batch > 1 side of ggml-cuda that llama.cpp runs for the prompt under create_chat_completion
-// (/root/reference/api.py:55-63): get_rows (K1), rms_norm_f32 (K2), rope_f32 + the KV-cache copy (K6/K7),
-// the attention mat-muls + soft_max (K8-K10 at batch T), silu/mul (K11) (SURVEY.md 2.3).
+// (api.py:55-63): get_rows (K1), rms_norm_f32 (K2), rope_f32 + the KV-cache copy (K6/K7),
+// the attention mat-muls + soft_max (K8-K10 at batch T), silu/mul (K11).
 //
 // f16 activation matrices that feed the GEMM are written in its operand order [K/8][T_pad][8]; the GEMM's
 // outputs arrive as n_parts K-split partial sums that the consumer adds in a fixed order.

@@ -12,7 +12,7 @@
 //
 // Block layouts: see oracle/ggml_blocks.py (restated from gguf-py quants.py) -- replaces
 // ggml-cuda's dequantize_block_* / vec_dot_*_q8_1 that the reference reaches through
-// llama-cpp-python (SURVEY.md 2.3 K1,K4,K5).
+// llama-cpp-python.
 //
 // Everything here compiles for the host too (B2_HOST_EMU) so tests/host_selftest.cpp can check
 // the bit-twiddling against the oracle without a GPU.

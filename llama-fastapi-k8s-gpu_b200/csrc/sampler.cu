@@ -1,8 +1,8 @@
 // On-device sampler: repetition/frequency/presence penalties over the last 64 tokens, then either
 // greedy arg-max or top-k -> top-p -> min-p -> temperature -> multinomial draw. Restates the order
 // llama-cpp-python 0.2.77 applies under create_chat_completion(temperature=1.2, top_p=0.9,
-// frequency_penalty=0.7, presence_penalty=0.8) (/root/reference/api.py:55-63; SURVEY.md 2.2 H8,
-// 2.3 K12): upstream copies all n_vocab logits to the host every token and sorts on the CPU; here
+// frequency_penalty=0.7, presence_penalty=0.8) (api.py:55-63):
+// upstream copies all n_vocab logits to the host every token and sorts on the CPU; here
 // one CTA selects the k largest logits with a 3-pass radix select, sorts only those, and 4 bytes
 // (the token id) go back to the host. The uniform random numbers come from the host (MT19937
 // stream restated in llama_cpp/sampling.py), one double per token.

@@ -1,8 +1,8 @@
-// Tensor-parallel collectives for 70B-class models (BASELINE.json configs[4]; SURVEY.md 8(e)): one process per GPU, the
+// Tensor-parallel collectives for 70B-class models: one process per GPU, the
 // quantised weights split by columns (attn_q/k/v, ffn_gate/up, output: whole rows per rank) or by rows' K ranges
 // (attn_output, ffn_down: cut at 256-element block boundaries, no re-quantisation), and an all-reduce (sum) of the hidden
 // vector after attn_output and after ffn_down, over NCCL on NVLink. The reference has no counterpart: its only multi-GPU
-// strategy is independent replicas (/root/reference/helm/values.yaml:17); llama.cpp itself has no NCCL path.
+// strategy is independent replicas (helm/values.yaml:17); llama.cpp itself has no NCCL path.
 //
 // The hidden-vector all-reduce itself does not go through NCCL when the ranks can map each other's memory (CUDA IPC):
 // tp_allreduce_kernel below exchanges 32 KB per rank with plain loads from the peers' buffers over NVLink behind a

@@ -1,7 +1,7 @@
 """ctypes binding of libb200gguf.so (the C ABI in include/b200_gguf.h).
 
 The counterpart of llama-cpp-python's `llama_cpp/llama_cpp.py` ctypes layer that the
-reference imports through `from llama_cpp import Llama` (/root/reference/api.py:7).
+reference imports through `from llama_cpp import Llama` (api.py:7).
 There is no CPU fallback: if the library is missing or fails to load this raises.
 """
 from __future__ import annotations

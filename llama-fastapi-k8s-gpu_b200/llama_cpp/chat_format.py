@@ -1,8 +1,8 @@
 """Chat templating: messages -> prompt string (+ stop strings).
 
 Restates the formatters llama-cpp-python 0.2.77 uses under `create_chat_completion`
-(/root/reference/api.py:55-63; upstream `llama_cpp/llama_chat_format.py`, un-vendored, SURVEY.md
-2.2 H4): exact-match guess of the GGUF `tokenizer.chat_template` -> built-in "llama-3" /
+(api.py:55-63; upstream `llama_cpp/llama_chat_format.py`, un-vendored):
+exact-match guess of the GGUF `tokenizer.chat_template` -> built-in "llama-3" /
 "chatml" / "mistral-instruct" formatter, else the template itself through Jinja2, else "llama-2".
 The built-in formatters silently drop messages whose role they do not know -- that matters for the
 reference, which forwards the client's `turn` field as the role (api.py:122-125).

@@ -1,7 +1,7 @@
 """Python handle on one native engine (one GPU): GGUF -> HBM upload and the step calls.
 
 Host-side half of what `Llama.__init__` does in the reference stack
-(/root/reference/api.py:24-28 -> llama-cpp-python `Llama.__init__` -> llama.cpp model loader):
+(api.py:24-28 -> llama-cpp-python `Llama.__init__` -> llama.cpp model loader):
 parse the file, read the `llama.*` hyper-parameters, copy every tensor's raw quant blocks
 unchanged into device memory through the C ABI, size the paged KV pool.
 """

@@ -1,7 +1,7 @@
 """mmap GGUF (v2/v3) reader and a minimal writer.
 
 Replaces the loader the reference reaches through ``Llama(model_path=...)``
-(/root/reference/api.py:24-28 -> llama-cpp-python 0.2.77 -> llama.cpp
+(api.py:24-28 -> llama-cpp-python 0.2.77 -> llama.cpp
 ``llama_model_loader`` / ggml ``gguf_init_from_file``; un-vendored upstream).
 
 File layout (little endian) as published by ggml and implemented in gguf-py

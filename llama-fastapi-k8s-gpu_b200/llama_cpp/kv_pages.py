@@ -1,7 +1,7 @@
 """Paged KV-cache allocator (host side).
 
 llama.cpp keeps one contiguous f16 K and V buffer per layer sized n_ctx and a slot finder
-(`llama_kv_cache`, un-vendored upstream behind /root/reference/api.py:24-28).
+(`llama_kv_cache`, un-vendored upstream behind api.py:24-28).
 This engine pages it: the device holds one pool of fixed-size pages shared by all sequences,
 and each sequence owns a page table. This class hands out page ids; the engine only ever sees
 `b2_seq_set_blocks(slot, pages)`.

@@ -1,11 +1,11 @@
 """`llama_cpp.Llama` -- drop-in for the llama-cpp-python object the reference drives.
 
-The reference uses exactly two things (/root/reference/api.py):
+The reference uses exactly two things (api.py):
     llm = Llama(model_path=file_path, n_gpu_layers=-1, n_ctx=1024)                 # :24-28
     llm.create_chat_completion(messages=..., stream=False, temperature=1.2, top_p=0.9,
                                frequency_penalty=0.7, presence_penalty=0.8) -> dict  # :55-63
 and reads `answer["choices"][i]["message"]["content"]` (:65-74). Same keywords, defaults, return
-shape and error behaviour as llama-cpp-python 0.2.77 (un-vendored upstream; SURVEY.md 8(b)),
+shape and error behaviour as llama-cpp-python 0.2.77 (un-vendored upstream),
 on top of the B200 engine: no CPU path (`n_gpu_layers=0` raises), concurrent callers are batched.
 """
 from __future__ import annotations
@@ -44,7 +44,7 @@ class Llama:
             raise ValueError(f"Model path does not exist: {model_path}")
         if n_gpu_layers == 0:
             raise ValueError("n_gpu_layers=0 requests the CPU path; the B200 engine has no CPU fallback "
-                             "(pass n_gpu_layers=-1 as /root/reference/api.py:26 does)")
+                             "(pass n_gpu_layers=-1 as the reference's api.py:26 does)")
         self.model_path = model_path
         self.verbose = verbose
         self._source = models.open_model(model_path)      # a GGUF file, or a folder with config.json + model.safetensors

@@ -5,7 +5,7 @@ the mat-vec / tcgen05 GEMM path of engine.cu) and a folder with `config.json` + 
 (`architecture` names the graph; layer-list designs go through layered.cu). A family knows how to read its
 hyper-parameters, how to describe itself to the C ABI and which engine class runs it.
 
-The reference loads exactly one kind of file through llama-cpp-python (/root/reference/api.py:24-28); the registry
+The reference loads exactly one kind of file through llama-cpp-python (api.py:24-28); the registry
 is what lets `Llama(model_path=...)`, the scheduler and the trace runner take either without knowing which.
 """
 from __future__ import annotations

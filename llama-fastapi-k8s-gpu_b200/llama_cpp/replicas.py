@@ -1,7 +1,7 @@
 """Multi-GPU plumbing for models that fit one GPU: independent replicas, no data-path collective.
 
 The reference scales out with 4 single-GPU pods behind a k8s Service
-(/root/reference/helm/values.yaml:17, docker/Dockerfile.app:12); here a replica is one engine per
+(helm/values.yaml:17, docker/Dockerfile.app:12); here a replica is one engine per
 GPU (one process per GPU under torchrun). The only cross-rank traffic is bookkeeping: a barrier
 around the timed region and a max-reduction of the per-rank times (bench.py), over NCCL on the GPU
 box and over gloo in the CPU tests.

@@ -1,8 +1,8 @@
 """Host side of sampling: the uniform random stream for the device sampler.
 
 llama.cpp draws the token with `std::discrete_distribution` over a `std::mt19937` seeded from
-the context seed (reached from /root/reference/api.py:55-63 via llama-cpp-python `Llama.sample`;
-SURVEY.md 2.2 H8). The device sampler consumes one double per token; this produces those doubles
+the context seed (reached from api.py:55-63 via llama-cpp-python `Llama.sample`).
+The device sampler consumes one double per token; this produces those doubles
 the way libstdc++ does: `generate_canonical<double, 53>` = two 32-bit MT19937 outputs,
 (r0 + r1 * 2^32) / 2^64.
 """

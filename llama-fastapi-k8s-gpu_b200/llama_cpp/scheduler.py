@@ -1,7 +1,7 @@
 """Continuous-batching scheduler: many concurrent `create_chat_completion` callers, one engine.
 
 The reference admits one generation at a time (asyncio.Queue(5) -> single consumer ->
-Semaphore(1), /root/reference/api.py:80-116) and upstream's `Llama` is not re-entrant. This
+Semaphore(1), api.py:80-116) and upstream's `Llama` is not re-entrant. This
 engine is: callers on any thread (api.py:55 uses asyncio.to_thread) enqueue a Request and block;
 one scheduler thread owns the engine, admits requests into free sequence slots (prefill, with
 longest-common-prefix reuse of the slot's previous KV -- upstream's H5 behaviour), then advances
@@ -9,7 +9,7 @@ all live sequences one token per iteration. With a single live sequence and nobo
 decodes in run-ahead chunks (the sampled token never leaves the GPU between steps) and rewinds
 if a stop condition fell inside the chunk.
 
-Stop handling restates llama-cpp-python 0.2.77 `_create_completion` (SURVEY.md 2.2 H9): an
+Stop handling restates llama-cpp-python 0.2.77 `_create_completion`: an
 end-of-generation token ends with finish_reason "stop" and is not emitted; a stop string cuts the
 text at its first occurrence; reaching max_tokens ends with "length".
 """
@@ -139,7 +139,7 @@ class Scheduler:
     def cancel(self, req: Request):
         """Abandon a request: still queued -> it never starts; running -> its slot is freed at the next step (the caller's
         `wait()` returns with finish_reason "cancelled" and the text so far). The reference cannot do this: after a 408 its
-        worker thread generates to the end while holding the semaphore (/root/reference/api.py:162-170)."""
+        worker thread generates to the end while holding the semaphore (api.py:162-170)."""
         if req.cancel_event is None:
             req.cancel_event = threading.Event()
         req.cancel_event.set()

@@ -1,6 +1,6 @@
 """Serving launcher, per-GPU replica router and /health for the B200 engine.
 
-Re-hosts the reference's HTTP layer (/root/reference/api.py, kept byte-for-byte where it is used as is) with the three
+Re-hosts the reference's HTTP layer (api.py, kept byte-for-byte where it is used as is) with the three
 things it hard-codes made parameters, so that the continuous-batching engine can actually be fed:
 
     reference (api.py)                           here
@@ -42,7 +42,7 @@ MAX_QUEUE_SIZE = 5              # api.py:19
 SAMPLING = dict(stream=False, temperature=1.2, top_p=0.9, frequency_penalty=0.7, presence_penalty=0.8)   # api.py:58-62
 
 
-# request schema: /root/reference/data/requests.py:4-19
+# request schema: data/requests.py:4-19
 class ChatMessage(BaseModel):
     turn: str
     message: str

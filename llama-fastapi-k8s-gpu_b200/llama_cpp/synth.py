@@ -1,14 +1,14 @@
-"""Seeded synthetic GGUF models of the architectures BASELINE.json names.
+"""Seeded synthetic GGUF models of the benchmarked architectures.
 
-There is no network and no checkpoint on the GPU box, so throughput and parity
+There is no network and no checkpoint where these run, so throughput and parity
 runs use random-init GGUF files with the tensor-type mix of the real llama.cpp
-ftypes (SURVEY.md section 8(d)): quant nibbles/bytes are uniform random, the
+ftypes: quant nibbles/bytes are uniform random, the
 fp16 scale fields are overwritten so every tensor dequantises to roughly
 zero-mean values of a chosen std (0.02 by default, like a fresh transformer).
 
 The file is a normal GGUF: the same loader path (`gguf_file.GGUFFile` ->
 C-ABI upload) serves it that would serve `Lexi-Llama-3-8B-Uncensored_Q4_K_M.gguf`
-(/root/reference/api.py:13-15).
+(api.py:13-15).
 """
 from __future__ import annotations
 
@@ -139,7 +139,7 @@ def random_blocks(type_name: str, n_blocks: int, std: float, seed: int) -> np.nd
 
 def _use_more_bits(i: int, n: int) -> bool:
     """llama.cpp's Q4_K_M rule for which layers keep attn_v / ffn_down at Q6_K
-    (restated from SURVEY.md section 8(d): i < n/8 or i >= 7n/8 or (i - n/8) % 3 == 2)."""
+    (restated: i < n/8 or i >= 7n/8 or (i - n/8) % 3 == 2)."""
     return i < n // 8 or i >= 7 * n // 8 or (i - n // 8) % 3 == 2
 
 
@@ -181,7 +181,7 @@ def tensor_types(arch: Arch, ftype: str) -> Dict[str, str]:
         more = ftype == "Q4_K_M" and _use_more_bits(i, L)
         v_t = "Q6_K" if more else base
         if ftype == "Q4_K_M" and not more and arch.n_head // arch.n_head_kv >= 8 and arch.n_layer >= 80:
-            v_t = "Q5_K"  # 70B-class rule
+            v_t = "Q5_K"  # 70B-class rule cfg5)
         put(p + "attn_v.weight", "Q4_K" if ftype == "Q2_K_mix" else v_t)
         put(p + "ffn_down.weight", "Q3_K" if ftype == "Q2_K_mix" else "Q6_K" if more else base)
     return out

@@ -3,7 +3,7 @@
 Host-side replacement for llama.cpp's `llm_tokenizer_spm` / `llm_tokenizer_bpe`, special-token
 partitioning and `llama_token_to_piece`, which the reference reaches through
 `llm.create_chat_completion` -> `Llama.tokenize` / `Llama.detokenize`
-(/root/reference/api.py:55-63; un-vendored upstream). Tokenisation is not on
+(api.py:55-63; un-vendored upstream). Tokenisation is not on
 the per-token GPU path, so it stays in Python.
 
 SPM: text -> (optional leading space) -> ' ' replaced by U+2581 -> UTF-8 characters -> greedily

@@ -1,4 +1,4 @@
-"""Tensor-parallel sharding of GGUF tensors (70B-class models, BASELINE.json configs[4]; SURVEY.md 8(e)).
+"""Tensor-parallel sharding of GGUF tensors (70B-class models).
 
 The quantised blocks are never re-quantised, only selected:
 
@@ -11,7 +11,7 @@ The quantised blocks are never re-quantised, only selected:
     the full mat-vec (all-reduce in the engine).
   * everything else (norm vectors, token_embd) is replicated.
 
-The reference has no tensor parallelism (replicas only, /root/reference/helm/values.yaml:17).
+The reference has no tensor parallelism (replicas only, helm/values.yaml:17).
 """
 from __future__ import annotations
 

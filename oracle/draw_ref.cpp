@@ -1,6 +1,6 @@
 // ORACLE (test infrastructure, not product code) -- pin for the multinomial draw.
 //
-// llama.cpp's llama_sample_token (reached from create_chat_completion at /root/reference/api.py:55-63
+// llama.cpp's llama_sample_token (reached from create_chat_completion at api.py:55-63
 // through llama-cpp-python 0.2.77; un-vendored upstream) ends with
 //     std::discrete_distribution<> dist(probs.begin(), probs.end());  int idx = dist(rng);
 // on the context's std::mt19937. This program IS that call, made with the same libstdc++ <random> the

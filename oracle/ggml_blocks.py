@@ -4,10 +4,10 @@ Only tests/, __graft_entry__.smoke() and bench.py's cpu_baseline / --impl refere
 legs may import this package. The product path (llama_cpp/ + csrc/) never does.
 
 PARITY UNPINNED BY THE REFERENCE: the arithmetic lives in llama-cpp-python==0.2.77
-(pinned at /root/reference/docker/Dockerfile.base:30, /root/reference/README.md:20),
+(pinned at docker/Dockerfile.base:30, README.md:20),
 which vendors llama.cpp/ggml; that source is not under /root/reference, is not
 installed here and cannot be fetched. The reference repo has no tests or golden
-vectors (SURVEY.md section 4). What this file IS pinned against: gguf-py 0.19
+vectors. What this file IS pinned against: gguf-py 0.19
 (`gguf.quants.dequantize`, ggml's own numpy reference, present in this image) --
 tests/test_oracle_blocks.py checks bit-equality on random and hand-built blocks,
 and tests/golden/blocks_*.npz holds committed vectors generated from it.

@@ -1,9 +1,9 @@
 """ORACLE (test infrastructure, not product code) -- llama-architecture forward pass.
 
 CPU float32 restatement of the graph the reference runs inside
-`llm.create_chat_completion(...)` (/root/reference/api.py:55-63 -> llama-cpp-python
-0.2.77 `Llama.eval` -> llama.cpp `llm_build_llama`; un-vendored upstream, SURVEY.md
-section 2.2 H6). PARITY UNPINNED BY THE REFERENCE (no llama_cpp in this image, no
+`llm.create_chat_completion(...)` (api.py:55-63 -> llama-cpp-python
+0.2.77 `Llama.eval` -> llama.cpp `llm_build_llama`; un-vendored upstream).
+PARITY UNPINNED BY THE REFERENCE (no llama_cpp in this image, no
 tests or golden vectors in the reference repo). Pinned instead against an independent
 implementation that is importable here: transformers' GGUF loader -> float32
 `LlamaForCausalLM` (tests/golden/make_golden.py writes the committed fixture,

@@ -2,10 +2,10 @@
 
 CPU restatement of the sampling chain llama-cpp-python 0.2.77 runs per token under
 `create_chat_completion(temperature=1.2, top_p=0.9, frequency_penalty=0.7,
-presence_penalty=0.8)` (/root/reference/api.py:55-63): `Llama.sample` ->
+presence_penalty=0.8)` (api.py:55-63): `Llama.sample` ->
 `_LlamaSamplingContext.sample` -> llama.cpp `llama_sample_repetition_penalties`,
 `llama_sample_top_k`, `llama_sample_top_p`, `llama_sample_min_p`, `llama_sample_temp`,
-`llama_sample_token` (un-vendored upstream; SURVEY.md 2.2 H8). PARITY UNPINNED BY THE
+`llama_sample_token` (un-vendored upstream). PARITY UNPINNED BY THE
 REFERENCE: no llama_cpp here and no golden vectors in the reference repo; this restates the
 published algorithm (tfs_z = typical_p = 1.0 are no-ops and are not modelled).
 

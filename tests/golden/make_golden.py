@@ -9,7 +9,7 @@ transformers are importable; neither needs the GPU):
                   seeded synthetic `tiny` and `tiny128` models -> pins oracle/llama_ref.py
                   (graph, GQA, RoPE pairing convention); the file's sha256 guards the generator.
 
-The reference repo itself has no golden vectors (SURVEY.md section 4).
+The reference repo itself has no golden vectors.
 
     python tests/golden/make_golden.py
 """
@@ -47,7 +47,7 @@ def main():
         raw = finite_random_blocks(tname, 64, rng)
         out[f"{tname}_raw"] = raw
         out[f"{tname}_f32"] = dequantize(raw, getattr(T, tname)).reshape(-1).astype(np.float32)
-    rng2 = np.random.default_rng(2025)          # types added in round 2: their own stream, the entries above stay as they were
+    rng2 = np.random.default_rng(2025)          # types added later: their own stream, the entries above stay as they were
     for tname in ("Q4_1", "Q5_0", "Q5_1", "Q2_K", "Q3_K"):
         raw = finite_random_blocks(tname, 64, rng2)
         out[f"{tname}_raw"] = raw

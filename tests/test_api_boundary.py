@@ -1,5 +1,5 @@
 """The reference's api.py, imported UNCHANGED from /root/reference, served by this repo's
-`llama_cpp` package (fake engine on CPU): status codes and payloads of SURVEY.md 8(b).
+`llama_cpp` package (fake engine on CPU): status codes and payloads.
 Skipped where the reference checkout does not exist (the GPU box)."""
 import importlib.util
 import os

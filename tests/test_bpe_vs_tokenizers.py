@@ -1,7 +1,7 @@
 """The byte-level BPE path (llama-bpe pre-tokeniser, merges, ignore_merges) pinned against an independent implementation:
 Hugging Face `tokenizers` configured the way Llama-3's tokenizer.json is (Split on the Llama-3 regex + ByteLevel, BPE with
 ignore_merges). A small vocabulary is trained in the test itself (deterministic), exported the way a GGUF file carries it
-(tokens, merges, token types) and both sides encode the same texts. Reference call sites: /root/reference/api.py:55-63
+(tokens, merges, token types) and both sides encode the same texts. Reference call sites: api.py:55-63
 (create_chat_completion tokenises the rendered chat template)."""
 import json
 import os

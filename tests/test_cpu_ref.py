@@ -1,5 +1,5 @@
 """The C restatement of ggml's CPU path (oracle/cpu_ref.c, the timed CPU baseline) against the
-float32 oracle: equal up to the int8-activation noise ggml accepts (SURVEY.md 7 hard part #3)."""
+float32 oracle: equal up to the int8-activation noise ggml accepts."""
 import os
 
 import numpy as np

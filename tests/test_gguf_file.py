@@ -64,7 +64,7 @@ def test_q4_k_m_type_mix_matches_survey():
     shapes = synth.tensor_shapes(a)
     from llama_cpp.gguf_file import GGML_TYPE_ID, tensor_nbytes
     total = sum(tensor_nbytes(GGML_TYPE_ID[types[n]], int(np.prod(s))) for n, s in shapes.items())
-    assert abs(total / 1e9 - 4.913) < 0.01            # SURVEY.md 8(d): 4.913 GB
+    assert abs(total / 1e9 - 4.913) < 0.01            # 4.913 GB
     more = [i for i in range(32) if types[f"blk.{i}.ffn_down.weight"] == "Q6_K"]
     assert more == [0, 1, 2, 3, 6, 9, 12, 15, 18, 21, 24, 27, 28, 29, 30, 31]
     w_read = total - tensor_nbytes(GGML_TYPE_ID[types["token_embd.weight"]], a.n_embd * a.n_vocab)

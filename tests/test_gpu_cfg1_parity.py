@@ -1,11 +1,11 @@
-"""The designated CPU-vs-GPU parity run: TinyLlama-1.1B-arch Q4_0
+"""The designated CPU-vs-GPU parity run of TinyLlama-1.1B-arch Q4_0
 synthetic GGUF, 128-token prompt, 128 greedy tokens.
 
-Protocol (hard part #2): the engine decodes greedily; the float32 oracle is then run teacher-forced
+Protocol: the engine decodes greedily; the float32 oracle is then run teacher-forced
 over the engine's own tokens in ONE batched pass, so a near-tie cannot hide the steps after it -- at every one of the
 128 steps the oracle's arg-max is compared with the engine's token and the full logit vectors are compared. Random-init
 logits are nearly flat, so the fixture (model seed, prompt seed, output_std) was screened on the GPU
-(scripts/screen_margin_gpu.py, 400 prompts) for the largest minimum top-2 margin; the test re-measures that margin
+(400 prompts) for the largest minimum top-2 margin; the test re-measures that margin
 with the oracle and records it.
 """
 import os
@@ -17,7 +17,7 @@ pytestmark = pytest.mark.gpu
 
 ARCH, FTYPE, MODEL_SEED, OUTPUT_STD, PROMPT_SEED = "tinyllama-1.1b", "Q4_0", 1, 0.1, 1005
 N_PROMPT = N_NEW = 128
-SCREENED_MIN_MARGIN = 0.071      # engine-side figure from the screening run (gpurun_out/scr_01.log, round 2)
+SCREENED_MIN_MARGIN = 0.071      # engine-side figure from the screening run
 
 
 def test_cfg1_128_prompt_128_greedy_tokens_match_oracle(native_lib, tmp_models):
@@ -56,10 +56,10 @@ def test_cfg1_128_prompt_128_greedy_tokens_match_oracle(native_lib, tmp_models):
     # every step whose oracle margin is clear must agree; with this fixture that is every step
     for i in mism:
         assert margin[i] < 4 * err.max(), f"step {i}: engine {got[i]} != oracle {int(oracle_tok[i])} with margin {margin[i]:.4f}"
-    assert margin.min() > 0.5 * SCREENED_MIN_MARGIN, "fixture drifted: re-run scripts/screen_margin_gpu.py"
+    assert margin.min() > 0.5 * SCREENED_MIN_MARGIN, "fixture drifted: screen the prompt seeds again"
     assert not mism, f"greedy tokens differ at steps {mism} (margins {[float(margin[i]) for i in mism]})"
     # Logits. The 128 prompt tokens go through the f16-operand tensor-core GEMM (operands rounded to 11 bits, the
     # precision class of the reference's own cuBLAS f16 prompt path), so every later step attends to K/V rows that carry
-    # that rounding; the decode steps themselves run the int8x2 mat-vec. Measured on B200 (round 2): max |diff| 0.065 =
+    # that rounding; the decode steps themselves run the int8x2 mat-vec. Measured on B200: max |diff| 0.065 =
     # 1.3e-2 of the logit std 4.93, all 128 tokens identical, smallest oracle margin 0.077. Bar: 2e-2 of the logit std.
     assert err.max() <= 2e-2 * sigma, (err.max(), sigma)

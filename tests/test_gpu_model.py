@@ -1,6 +1,6 @@
 """End-to-end parity of the native engine against the CPU oracle on seeded synthetic models
-(GPU only). Bars from BASELINE.json: per-token logits max-abs <= 1e-2; greedy tokens identical
-(checked where the oracle's top-2 margin exceeds 10x the logit tolerance, SURVEY.md 7 #2)."""
+(GPU only). Bars: per-token logits max-abs <= 1e-2; greedy tokens identical
+(checked where the oracle's top-2 margin exceeds 10x the logit tolerance)."""
 import os
 
 import numpy as np

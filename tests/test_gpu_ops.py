@@ -1,6 +1,6 @@
 """Parity of each CUDA kernel against the CPU oracle, called through the C ABI (GPU only).
 
-Bars (BASELINE.md section 5): block dequantisation bit-exact; mat-vec / attention within the
+Bars: block dequantisation bit-exact; mat-vec / attention within the
 floating-point tolerances written next to each check; sampler: identical token.
 """
 import ctypes

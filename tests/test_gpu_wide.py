@@ -4,7 +4,7 @@ The toy models of test_gpu_model.py never give a mat-vec CTA more than a handful
 the real Llama-3-8B / 70B matrix shapes -- d = 4096 (8192), n_ff = 14336 (28672), a 128256-row output head, the Q6_K
 attn_v / ffn_down / output of the Q4_K_M mix -- so every kernel runs with the row counts per CTA, K-slice counts, ring
 wrap-arounds and tile splits of the timed configuration, and is compared with the float32 oracle (logits max-abs
-<= 1e-2, BASELINE.json north_star). The oracle dequantises ~1 G weights: tens of seconds per model.
+<= 1e-2). The oracle dequantises ~1 G weights: tens of seconds per model.
 """
 import os
 
@@ -82,7 +82,7 @@ def test_wide_model_logits_on_every_path(native_lib, tmp_models, arch, ftype, se
     eng.close()
     sigma = float(want.std())
     print(f"{arch} {ftype}: logit std {sigma:.2f}, max |logit - oracle| per path {({k: round(float(v), 4) for k, v in worst.items()})}")
-    # Relative bars (the error scales with the logits). Measured on B200 (round 2), as a fraction of the logit std:
+    # Relative bars (the error scales with the logits). Measured on B200, as a fraction of the logit std:
     # mat-vec path 1.1e-3 .. 3.6e-3 -- the mat-vec arithmetic itself is good to 3e-5 (tests/test_host_selftest.py); what
     # is left are f16 KV-cache entries that round one ulp apart from the oracle's -- and the f16-operand tensor-core
     # paths 6e-3 .. 2.1e-2 (operands rounded to 11 bits, like the reference's own cuBLAS f16 prompt path). At the logit

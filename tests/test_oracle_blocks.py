@@ -1,5 +1,5 @@
 """The block oracle is pinned against ggml's own numpy reference (gguf-py) and the committed
-golden vectors; the reference repo has no vectors of its own (SURVEY.md section 4)."""
+golden vectors; the reference repo has no vectors of its own."""
 import os
 
 import numpy as np

@@ -6,7 +6,7 @@
    When g++ is on the machine the program is rebuilt and re-run, so a stale fixture cannot hide.
 2. The penalty -> top-k -> top-p -> min-p -> temperature chain against small known-answer vectors worked out by
    hand with the published formulas (every expected number below comes with its derivation). The fixed settings the
-   reference passes at /root/reference/api.py:59-62 are case F.
+   reference passes at api.py:59-62 are case F.
 """
 import json
 import os
