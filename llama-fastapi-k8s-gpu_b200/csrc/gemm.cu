@@ -34,6 +34,7 @@
 #include "kernels.h"
 #include "ptx.cuh"
 #include "quant_blocks.cuh"
+#include "tc05.cuh"
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <stdlib.h>
@@ -53,63 +54,6 @@ constexpr int GM_MAX_BSTAGES = 8;    // activation-tile ring
 constexpr int GM_RAW_STAGES = 2;    // raw weight spans in flight (TMA), at most
 constexpr int GM_SPAN_WORDS = 68;   // largest 256-weight span: Q8_0, 272 bytes
 
-__device__ __forceinline__ void tmem_alloc(uint32_t* smem_dst, uint32_t ncols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_dst)), "r"(ncols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// D (+)= A . B, A [128 lanes][16 f16 in 8 columns] from tensor memory
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
-}
-// the same with A from shared memory
-__device__ __forceinline__ void umma_f16_ss(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-                 "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-                   "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
-                   "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
-                   "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]) : "memory");
-    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
-    uint32_t r[16];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr) : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
-}
-
-// shared-memory matrix descriptor, K-major, no swizzle: start, LBO (K direction), SBO (M/N direction)
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-    uint64_t d = 0;
-    d |= (uint64_t)((addr >> 4) & 0x3FFF);
-    d |= (uint64_t)((lbo >> 4) & 0x3FFF) << 16;
-    d |= (uint64_t)((sbo >> 4) & 0x3FFF) << 32;
-    d |= (uint64_t)1 << 46;                  // descriptor version (sm_100)
-    return d;                                // layout_type = 0: no swizzle
-}
 __device__ __forceinline__ uint64_t desc_join(uint32_t lo, uint32_t hi) {
     uint64_t d;
     asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
@@ -381,9 +325,10 @@ __device__ __noinline__ void deq_loop(const DeqCtx cx) {
             fence_proxy_async();        // generic-proxy writes -> visible to the tensor core (async proxy)
         } else {
             __syncwarp();
-            tc_fence_after();
-            tmem_st32(cx.tmem_a + st * GM_BK, out);      // (a stage: GM_BK / 2 columns for each half of the rows)
-            tc_fence_before();
+            tc_after_sync();
+            tc_st32(cx.tmem_a + st * GM_BK, out);        // (a stage: GM_BK / 2 columns for each half of the rows)
+            tc_wait_st();
+            tc_before_sync();
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&sh.a_full[st]);      // once per warp: the arrivals of 32 lanes go one after the other
@@ -490,11 +435,11 @@ __global__ void __launch_bounds__(GM_THREADS) gemm_q_kernel(const __grid_constan
             fence_mbar_init();
         }
         __syncwarp();
-        tmem_alloc(&sh.tmem_base, ncols);
+        tc_alloc(&sh.tmem_base, ncols);
     }
-    tc_fence_before();
+    tc_before_sync();
     __syncthreads();
-    tc_fence_after();
+    tc_after_sync();
     // Programmatic dependent launch: the next kernel of the chain may start now. In THIS kernel only the threads that
     // touch the previous kernel's data wait for it (the activation producer; the epilogue, which overwrites the planes
     // the previous consumer read): weights stream and dequantise while the predecessor is still running.
@@ -533,14 +478,14 @@ __global__ void __launch_bounds__(GM_THREADS) gemm_q_kernel(const __grid_constan
         // ================= epilogue
         mbar_wait(&sh.done, 0, p.err, 0x40002u, (unsigned)n);
         __syncwarp();
-        tc_fence_after();
+        tc_after_sync();
         griddep_wait();
         const int row = m0 + row_in;                // TMEM lane = weight row, columns = tokens; the two threads of a row take every other 16
         const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(row_in / GM_BM) * T;
         float* ybase = p.y + (size_t)split * p.split_stride + (size_t)t_base * p.ldy + sg.out_off + row;
         for (int c0 = 16 * (tid / ROWS); c0 < T; c0 += 32) {
             float v[16];
-            tmem_ld16(lane_addr + c0, v);
+            tc_ld16(lane_addr + c0, v);
             if (row < sg.n_rows) {
 #pragma unroll
                 for (int j = 0; j < 16; j++)
@@ -562,7 +507,7 @@ __global__ void __launch_bounds__(GM_THREADS) gemm_q_kernel(const __grid_constan
             mbar_wait(&sh.a_full[s], use & 1, p.err, 0x40004u, (unsigned)i);
             if (dbg && i < 64) p.dbg[i * 8 + 4] = clock64();
             __syncwarp();
-            tc_fence_after();
+            tc_after_sync();
             // descriptors differ only in the 14-bit start-address field (units of 16 B): add, do not rebuild
             const uint32_t a_at = tmem_a0 + (uint32_t)s * GM_BK, b_lo = b_lo0 + (uint32_t)sb * (b_bytes >> 4);
             if (elect_one()) {
@@ -572,16 +517,16 @@ __global__ void __launch_bounds__(GM_THREADS) gemm_q_kernel(const __grid_constan
                     const uint32_t acc = (i > 0 || ks > 0) ? 1u : 0u;
                     if constexpr (SS) {
                         const uint32_t at = a_lo0 + (uint32_t)s * (GM_ABYTES >> 4) + ks * (2 * GM_ROWS);
-                        umma_f16_ss(tmem, desc_join(at, desc_hi), db, idesc, acc);
-                        umma_f16_ss(tmem + T, desc_join(at + GM_BM, desc_hi), db, idesc, acc);      // rows 128 ..
+                        tc_mma(tmem, desc_join(at, desc_hi), db, idesc, acc);
+                        tc_mma(tmem + T, desc_join(at + GM_BM, desc_hi), db, idesc, acc);      // rows 128 ..
                     } else {
-                        umma_f16(tmem, a_at + ks * 8, db, idesc, acc);
-                        umma_f16(tmem + T, a_at + GM_BK / 2 + ks * 8, db, idesc, acc);
+                        tc_mma_ts(tmem, a_at + ks * 8, db, idesc, acc);
+                        tc_mma_ts(tmem + T, a_at + GM_BK / 2 + ks * 8, db, idesc, acc);
                     }
                 }
-                umma_commit(&sh.empty[s]);      // both arrive when the MMAs above have finished reading their tiles
-                umma_commit(&sh.b_empty[sb]);
-                if (i + 1 == n) umma_commit(&sh.done);
+                tc_commit(&sh.empty[s]);      // both arrive when the MMAs above have finished reading their tiles
+                tc_commit(&sh.b_empty[sb]);
+                if (i + 1 == n) tc_commit(&sh.done);
             }
             __syncwarp();
             if (dbg && i < 64) p.dbg[i * 8 + 5] = clock64();
@@ -626,9 +571,9 @@ __global__ void __launch_bounds__(GM_THREADS) gemm_q_kernel(const __grid_constan
             __syncwarp();
         }
     }
-    tc_fence_before();
+    tc_before_sync();
     __syncthreads();
-    if (warp == DW) tmem_dealloc(tmem, ncols);
+    if (warp == DW) tc_dealloc(tmem, ncols);
 }
 
 // ---------------------------------------------------------------- host side

@@ -13,6 +13,7 @@
 // Bound by the chain of a block's scores, softmax and sums: six warps an SM, tensor pipe busy for 18 % of the time, issue slots for 13 % (ncu).
 // 2048 tokens, 16 heads, rows of 512 + 64 (B200): 1640 us a layer with mma.sync, 248 here, 210 with the issue loops run by whole warps.
 #include "kernels.h"
+#include "latent_dev.cuh"
 #include "layered.h"
 #include "ptx.cuh"
 #include "tc05.cuh"
@@ -31,20 +32,6 @@ namespace {
 __device__ __forceinline__ uint32_t lc_pack(float lo, float hi) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const uint32_t*>(&v);
-}
-// entry i of the rotated part of a head's query (see latent_attn.cu)
-__device__ __forceinline__ float lc_rotated(const LatentAttnArgs& a, int t, int h, int i, int pos) {
-    if (!a.q_raw) return a.qv[((size_t)t * a.H + h) * (a.rank + a.dr) + a.rank + i];
-    const float* v = a.q_raw + ((size_t)t * a.H + h) * (a.d + a.dr) + a.d;
-    const int half = a.rot.rot_dims / 2;
-    if (i >= a.rot.rot_dims) return v[i];
-    if (a.rot.pairs) {
-        const float cs = a.rot.cos[(size_t)pos * half + i / 2], sn = a.rot.sin[(size_t)pos * half + i / 2];
-        return i & 1 ? v[i] * cs + v[i - 1] * sn : v[i] * cs - v[i + 1] * sn;
-    }
-    const int p = i < half ? i : i - half;
-    const float cs = a.rot.cos[(size_t)pos * half + p], sn = a.rot.sin[(size_t)pos * half + p];
-    return i < half ? v[i] * cs - v[i + half] * sn : v[i] * cs + v[i - half] * sn;
 }
 }  // namespace
 
@@ -159,7 +146,7 @@ __global__ void __launch_bounds__(192, 1) latent_attn_tc_kernel(const __grid_con
         for (int c = a.rank; c < n_parts * LC_PART; c += 8) {
             float v[8];
 #pragma unroll
-            for (int e = 0; e < 8; e++) v[e] = row < nq && c + e < a.rank + a.dr ? lc_rotated(a, t, hd, c + e - a.rank, pos) * a.scale : 0.f;
+            for (int e = 0; e < 8; e++) v[e] = row < nq && c + e < a.rank + a.dr ? query_at(a, t, hd, c + e, pos) * a.scale : 0.f;
             uint8_t* dst = qs + (size_t)(c / LC_PART) * LC_QPART + row * 128 + ((((c % LC_PART) / 8) ^ (row & 7)) << 4);
             *reinterpret_cast<uint4*>(dst) = make_uint4(lc_pack(v[0], v[1]), lc_pack(v[2], v[3]), lc_pack(v[4], v[5]), lc_pack(v[6], v[7]));
         }

@@ -1,4 +1,4 @@
-// Wrappers of the tcgen05 instructions that the layer-list kernels use (one-CTA groups, f16-kind products of bf16 operands).
+// Wrappers of the tcgen05 instructions of both graphs' kernels (one-CTA groups, products of kind f16: bf16 operands, f16 in gemm.cu).
 #pragma once
 #include "ptx.cuh"
 
