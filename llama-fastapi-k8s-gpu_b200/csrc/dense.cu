@@ -1,9 +1,10 @@
 // Dense products for the layer-list models: Y[T][N] = epi(X[T][K] . W[N][K]^T + bias), weights bf16 or f32 as stored
-// in the file, activations f32 in memory. Four kernels:
+// in the file, activations f32 in memory. Five kernels:
 //   dense_rows_kernel   T <= 8 (decode steps): one warp per weight row, the row is streamed once for all tokens
 //   dense_tc_kernel     T > 8, bf16 weights: tensor cores (dense_tc.cu), X rounded to bf16
 //   dense_mma_kernel    the same for rows that tensor copies cannot take (K % 8 != 0): mma.sync m16n8k16 bf16, f32 accumulate
-//   dense_fma_kernel    T > 8, exact mode (or f32 weights): 32-bit multiply-adds, nothing rounded
+//   dense_split_kernel  T > 8, exact mode, bf16 weights: tensor cores, X as three bf16 parts that add up to it (dense_split.cu)
+//   dense_fma_kernel    T > 8, exact mode, weights or rows that the former does not take: 32-bit multiply-adds, nothing rounded
 // Every output element is one sum over k in a fixed order that depends only on the matrix and the kernel, never on the
 // other rows, so a token's result is the same whatever else shares the step. Arbitrary T, N, K (edges are guarded).
 // The llama graph's counterpart (quantised blocks, tcgen05) is gemm.cu / matvec.cu.
@@ -393,6 +394,7 @@ cudaError_t dense_launch(const DenseArgs& a, cudaStream_t s) {
         if (c.aux) c.aux += (size_t)chunks * ROWS_MAX_T * a.ldaux;
         return wb ? launch_rows<__nv_bfloat16>(c, 1, s) : launch_rows<float>(c, 1, s);
     }
+    if (dense_takes_split(a)) return dense_split_launch(a, d, s);
     const unsigned gz = d.grouped ? 1 : a.batch;
     if (dense_takes_rounded(a)) return dense_tc_launch(a, d, s);
     if (a.x_rounded || a.y_rounded || (d.grouped == 2 && a.groups->tile_max != 64)) return cudaErrorInvalidValue;

@@ -83,5 +83,8 @@ __device__ __forceinline__ void epi_store2(const DenseDev& a, float* y, const fl
 
 // tensor cores, more than 8 tokens (dense_tc.cu): operand rows of K % 8 == 0 entries on 16-byte boundaries
 cudaError_t dense_tc_launch(const DenseArgs& a, const DenseDev& d, cudaStream_t s);
+// the same in 32 bits, inputs in three bf16 parts (dense_split.cu)
+bool dense_takes_split(const DenseArgs& a);
+cudaError_t dense_split_launch(const DenseArgs& a, const DenseDev& d, cudaStream_t s);
 
 }  // namespace b2

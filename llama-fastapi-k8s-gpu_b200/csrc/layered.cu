@@ -103,6 +103,7 @@ struct LayeredModel {
     // step workspace (max_step_tokens rows)
     float *xs = nullptr, *hc = nullptr, *cross = nullptr;     // copies of the stream [S][max_step_tokens][W]; convolved sublayer input; per-(query head, value head) attention sums
     float *x = nullptr, *proj = nullptr, *buf[4] = {}, *oL = nullptr, *oR = nullptr, *hn = nullptr, *hn2 = nullptr, *ff = nullptr, *rows = nullptr, *logits = nullptr;
+    __nv_bfloat16* x_parts = nullptr;  // 32-bit engines: a product's input in three bf16 parts
     __nv_bfloat16* xb = nullptr;       // a product's input rounded to bf16 [max_step_tokens][widest input]
     // blocks behind one norm: what a producer leaves already rounded for the large products: the normed row, the mixer's output row;
     // experts' activations (every family)
@@ -705,7 +706,8 @@ int layered_finalize(b2_engine* e) {
     if (parallel && (rc = dev_alloc(m, (void**)&m->hn2, (size_t)Tm * W * 4))) return rc;
     max_ff = std::max(max_ff, max_glu);
     if ((rc = dev_alloc(m, (void**)&m->ff, (size_t)Tm * max_ff * 4))) return rc;
-    if (!m->exact && (rc = dev_alloc(m, (void**)&m->xb, (size_t)(Tm + B2_STEP_MAX_ENTRIES) * std::max<size_t>({max_buf, max_ff, (size_t)(c.loop_times > 0 ? 2 * W : W), moe_xb}) * 2 + 64))) return rc;
+    const size_t widest = (size_t)(Tm + B2_STEP_MAX_ENTRIES) * std::max<size_t>({max_buf, max_ff, (size_t)(c.loop_times > 0 ? 2 * W : W), moe_xb});
+    if (m->exact ? (rc = dev_alloc(m, (void**)&m->x_parts, 3 * widest * 2 + 64)) : (rc = dev_alloc(m, (void**)&m->xb, widest * 2 + 64))) return rc;
     if (one_norm && !m->exact) {
         if ((rc = dev_alloc(m, (void**)&m->hn_b, (size_t)Tm * W * 2 + 64))) return rc;
         if (max_mix > 0 && (rc = dev_alloc(m, (void**)&m->mix_b, (size_t)Tm * max_mix * 2 + 64))) return rc;
@@ -988,7 +990,7 @@ static DenseArgs dense_args(const LayeredModel* m, const DenseW& w, const float*
                             const DenseArgs* more) {
     DenseArgs a = more ? *more : DenseArgs{};
     a.x = x; a.ldx = ldx; a.w = w.w; a.w_type = w.type; a.bias = bias; a.y = y; a.ldy = ldy; a.T = T; a.N = w.N; a.K = w.K;
-    a.epi = epi; a.exact = m->exact || (more && more->exact); a.xb = m->xb;
+    a.epi = epi; a.exact = m->exact || (more && more->exact); a.xb = m->xb; a.x_parts = m->x_parts;
     return a;
 }
 static int dense_run(b2_engine* e, LayeredModel* m, const DenseArgs& a, int kind) {

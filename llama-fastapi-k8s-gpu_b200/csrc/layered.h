@@ -66,6 +66,7 @@ struct DenseArgs {
     int epi;
     bool exact;                     // true: 32-bit multiply-adds (no tensor cores, inputs not rounded)
     __nv_bfloat16* xb;              // scratch for X rounded to bf16, [T][K] ([T][x_span] batched; pair rows when gathered); null: not available
+    __nv_bfloat16* x_parts = nullptr;      // scratch for X as three bf16 parts (exact products with bf16 weights); null: not available
     float scale = 1.f;              // the product (after the epilogue) times this
     int n_act = 0, n_act_end = 0;   // EPI_BIAS_PART_RELU2
     float p0 = 0.f, p1 = 0.f;       // constants of EPI_GLU_CLAMP / EPI_PIECEWISE

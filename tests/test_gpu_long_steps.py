@@ -51,7 +51,7 @@ def rows_off(got, want):
     return np.sqrt((d ** 2).mean(-1)) / np.sqrt((w ** 2).mean())
 
 
-def check(util, ref, cfg, tmp_path, lengths, dtype):
+def check(util, ref, cfg, tmp_path, lengths, dtype, bar=None):
     w = util.random_weights(cfg, seed=5)
     prompts = [toks(cfg["vocab"], n, 7 + i) for i, n in enumerate(lengths)]
     eng = engine(util.write_model(str(tmp_path / "m"), cfg, w), dtype, max(lengths), len(lengths))
@@ -59,7 +59,7 @@ def check(util, ref, cfg, tmp_path, lengths, dtype):
     eng.close()
     for g, p in zip(got, prompts):
         off = rows_off(g, ref.forward(cfg, w, p))
-        assert off.max() < (F32 if dtype == "float32" else BF16), (int(off.argmax()), float(off.max()))
+        assert off.max() < (bar or (F32 if dtype == "float32" else BF16)), (int(off.argmax()), float(off.max()))
 
 
 @pytest.mark.parametrize("dims,lengths", [((16, 16), [256]), ((32, 48), [257]), ((64, 64), [383]), ((80, 128), [385]), ((128, 80), [300, 260]),
@@ -109,6 +109,21 @@ def test_scan_sizes(native_lib, tmp_path, state, inner, conv, lengths):
 def test_matrix_memory_sizes(native_lib, tmp_path, heads, d, dv, lengths):
     cfg = gu.config([gu.mlstm(heads=heads, dim=d, vdim=dv)])
     check(gu, goponex_ref, cfg, tmp_path, lengths, "float32")
+
+
+# 32-bit products whose inputs are cut into three bf16 parts: K around 64-entry slices, tokens around 32-column tiles, rows around 128. Without
+# the last part a row is off by 2^-17 (8e-6) per product; a few dozen 32-bit roundings in a row stay below half of that. (No matrix memory here:
+# its division by a sum that can cancel makes 1.5e-5 of a change of 2e-7 in the embedding, in the oracle itself.)
+SPLIT = {"biases": lambda W, ff: (gu, goponex_ref, gu.config([gu.parallel(mlp=ff, right=gu.scan(inner=W, dt_rank=8)), gu.parallel(mlp=2 * ff, left=gu.attn(dim=16))], width=W)),
+         "latent": lambda W, ff: (fu, fazovik_ref, fu.config([LATENT["rotated"](3, 64, mlp=fu.dense(ff)), LATENT["plain"](2, 128, mlp=fu.dense(ff), kv_from=None)], width=W)),
+         "experts": lambda W, ff: (zu, zogurax_ref, zu.config([zu.biased(heads=4, kv_heads=2, dim=16, vdim=24, mlp=zu.moe(experts=5, ff=ff, shared=40))], width=W))}
+
+
+@pytest.mark.parametrize("W,ff,lengths", [(72, 200, [9]), (136, 72, [31, 33]), (64, 128, [128]), (200, 328, [129, 1, 65]), (256, 1000, [350])])
+@pytest.mark.parametrize("kind", list(SPLIT))
+def test_products_in_32_bits(native_lib, tmp_path, kind, W, ff, lengths):
+    util, ref, cfg = SPLIT[kind](W, ff)
+    check(util, ref, cfg, tmp_path, lengths, "float32", bar=4e-6)
 
 
 def decode_all(util, ref, cfg, tmp_path, **kw):
