@@ -7,6 +7,7 @@ unchanged into device memory through the C ABI, size the paged KV pool.
 """
 from __future__ import annotations
 
+import array
 import ctypes
 import os
 import threading
@@ -19,6 +20,18 @@ from . import _cabi
 from ._cabi import B2Config, B2Sampling, check
 from .gguf_file import GGUFFile
 from .kv_pages import PageAllocator
+
+
+def int32s(values):
+    """A C int array of a list of token ids (or rows, slots). Filled through array.array: one call per list, where a ctypes array sets its
+    entries one by one (2048 tokens: 60 instead of 330 us, a third of a short prompt's time)."""
+    n = len(values)
+    if type(values) in (list, tuple) and n:
+        try:
+            return (ctypes.c_int32 * n).from_buffer(array.array("i", values))
+        except OverflowError:          # ctypes keeps the low 32 bits; the native side then checks the range
+            pass
+    return (ctypes.c_int32 * n)(*values)
 
 
 @dataclass
@@ -94,7 +107,7 @@ class EngineBase:
     def seq_begin(self, slot: int, n_past: int, history: Sequence[int], sampling: SamplingSettings,
                   uniforms: Optional[np.ndarray] = None):
         hist = list(history)[-64:]
-        ha = (ctypes.c_int32 * max(1, len(hist)))(*hist)
+        ha = int32s(hist or [0])
         sp = sampling.to_c()
         if uniforms is None:
             uniforms = np.zeros(1, dtype=np.float64)
@@ -106,7 +119,7 @@ class EngineBase:
         """Make sure the slot's page table covers n_tokens positions (uploads it if it grew)."""
         if self.pages.ensure(slot, n_tokens):
             tbl = self.pages.table(slot)
-            arr = (ctypes.c_int32 * len(tbl))(*tbl)
+            arr = int32s(tbl)
             check(self.lib.b2_seq_set_blocks(self._h, slot, arr, len(tbl)), "b2_seq_set_blocks")
 
     def release(self, slot: int):
@@ -210,7 +223,7 @@ class Engine(EngineBase):
 
     # ---------------------------------------------------------------- forward
     def prefill(self, slot: int, tokens: Sequence[int]):
-        arr = (ctypes.c_int32 * len(tokens))(*tokens)
+        arr = int32s(tokens)
         check(self.lib.b2_prefill(self._h, slot, arr, len(tokens)), "b2_prefill")
 
     def decode(self, slots: Sequence[int]) -> List[int]:
@@ -228,7 +241,7 @@ class Engine(EngineBase):
 
     def rewind(self, slot: int, n_keep: int, pending_token: int, history: Sequence[int]):
         hist = list(history)[-64:]
-        ha = (ctypes.c_int32 * max(1, len(hist)))(*hist)
+        ha = int32s(hist or [0])
         check(self.lib.b2_seq_rewind(self._h, slot, n_keep, pending_token, ha, len(hist)), "b2_seq_rewind")
 
     def set_token(self, slot: int, token: int):
@@ -340,11 +353,9 @@ class LayeredEngine(EngineBase):
                 flat.extend(toks)
                 rows.extend([at + wi for wi in w])
                 at += k
-            ints = ctypes.c_int32
-            out_tok = (ints * n)()
-            check(self.lib.b2_step(self._h, n, (ints * n)(*[slot for slot, _ in entries]), (ints * n)(*lens), (ints * at)(*flat),
-                                   (ints * n_want)(*rows) if n_want else None, n_want,
-                                   logits.ctypes.data_as(ctypes.c_void_p) if n_want else None, (ints * n)(*[1 if f else 0 for f in sample]), out_tok), "b2_step")
+            out_tok = (ctypes.c_int32 * n)()
+            check(self.lib.b2_step(self._h, n, int32s([slot for slot, _ in entries]), int32s(lens), int32s(flat), int32s(rows) if n_want else None, n_want,
+                                   logits.ctypes.data_as(ctypes.c_void_p) if n_want else None, int32s([1 if f else 0 for f in sample]), out_tok), "b2_step")
             return logits, [t if f else None for t, f in zip(out_tok, sample)]
         base, acc = [], 0
         for w in want:
@@ -362,8 +373,8 @@ class LayeredEngine(EngineBase):
                 room -= take
             if not batch:
                 break
-            slots = (ctypes.c_int32 * len(batch))(*[entries[i][0] for i, _, _ in batch])
-            counts = (ctypes.c_int32 * len(batch))(*[k for _, _, k in batch])
+            slots = int32s([entries[i][0] for i, _, _ in batch])
+            counts = int32s([k for _, _, k in batch])
             flat, rows, dest, flags = [], [], [], []
             for i, lo, k in batch:
                 toks = entries[i][1]
@@ -373,9 +384,9 @@ class LayeredEngine(EngineBase):
                         dest.append(base[i] + j)
                 flat.extend(toks[lo:lo + k])
                 flags.append(1 if (sample[i] and lo + k == len(toks)) else 0)
-            tok_arr = (ctypes.c_int32 * len(flat))(*flat)
-            row_arr = (ctypes.c_int32 * max(1, len(rows)))(*rows)
-            flag_arr = (ctypes.c_int32 * len(batch))(*flags)
+            tok_arr = int32s(flat)
+            row_arr = int32s(rows or [0])
+            flag_arr = int32s(flags)
             out_tok = (ctypes.c_int32 * len(batch))()
             part = np.empty((max(1, len(rows)), self.dims.n_vocab), dtype=np.float32)
             check(self.lib.b2_step(self._h, len(batch), slots, counts, tok_arr, row_arr, len(rows),
