@@ -1055,12 +1055,14 @@ static int mix_window_scan(b2_engine* e, LayeredModel* m, LyLayer& L, const Ragg
     }
     if ((rc = dense(e, m, L.scan_x, m->buf[0], d.d_inner, m->buf[2], s.ldx, T))) return rc;
     if ((rc = dense(e, m, L.scan_dt, m->buf[2], s.ldx, m->buf[3], d.d_inner, T))) return rc;
+    DenseArgs so = {};
+    if (takes_rounded(m, L.scan_o, T) && scan_leaves_rounded(s)) so.x_rounded = s.y_rounded = m->xb;
     {
         StepProfiler sp(m, st, 3);
         CK(scan_recurrence_launch(s, r, st));
         e->launches++;
     }
-    return dense(e, m, L.scan_o, m->buf[1], d.d_inner, m->oR, W, T);
+    return dense(e, m, L.scan_o, m->buf[1], d.d_inner, m->oR, W, T, nullptr, EPI_NONE, 1, &so);
 }
 
 static int mix_matrix_memory(b2_engine* e, LayeredModel* m, LyLayer& L, const RaggedDev& r, const float* in) {

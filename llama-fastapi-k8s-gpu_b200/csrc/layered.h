@@ -153,7 +153,9 @@ struct ScanArgs {              // selective scan (Mamba)
     float* ssm_state;          // [slot][inner][N]
     float* y;                  // [T][inner] gated output
     int inner;
+    __nv_bfloat16* y_rounded = nullptr;      // the gated output goes here instead, rounded (scan_leaves_rounded)
 };
+bool scan_leaves_rounded(const ScanArgs& a);
 cudaError_t scan_conv_launch(const ScanArgs& a, const RaggedDev& r, cudaStream_t s);
 cudaError_t scan_recurrence_launch(const ScanArgs& a, const RaggedDev& r, cudaStream_t s);
 

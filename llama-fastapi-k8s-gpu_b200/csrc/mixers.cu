@@ -896,22 +896,46 @@ __global__ void __launch_bounds__(SCAN_CH) scan_recurrence_chan_kernel(ScanArgs 
     }
 }
 
-// States up to a warp wide (N <= 32): four lanes per channel, N / 4 states each (lane q: states q, q + 4, ...), so that what a token
-// costs beside its states -- inputs, loop, read-out -- is paid once per four lanes, not once per state. A CTA owns SC_CH channels;
-// blocks of SC_TB tokens (step size, convolved input and gate of its channels, the B and C rows, ordered so that a lane's states are
-// one 16-byte read) arrive in shared memory as asynchronous copies two blocks ahead, where softplus(dt + bias) and silu(z) are
-// applied once per entry. Every global access is a run of SC_CH channels. The sums over the states keep the order of a butterfly over N
-// lanes, whatever the number of states a lane has. 2048 tokens of 8192 channels with 16 states (B200): 995 us with a lane per state, 413 here.
-// Bound by the exponentials and the latency of two warps a scheduler.
+// States up to a warp wide (N <= 32): four or eight lanes per channel, two or four states each (lane q: states q, q + LANES, ...), so that
+// what a token costs beside its states -- inputs, loop, read-out -- is paid once per lane, not once per state. A CTA owns blockDim / LANES <=
+// SC_CH channels, as few (8 at least) as give every SM one. Blocks of SC_TB tokens (step size, convolved input and gate of its channels, the B
+// and C rows, ordered so that a lane's states are one read) arrive in shared memory as asynchronous copies two blocks ahead; softplus(dt +
+// bias) and silu(z) are applied once per entry, a block ahead. Every global access is a run of the CTA's channels. A decay is one power of
+// two: A is kept times log2(e). What a token does to a channel is the same wherever the token stands in a step.
+// Bound by the exponentials (16 a cycle and SM: 60 us for 2048 tokens of 8192 channels with 16 states) and by the latency of what
+// surrounds them, up to four warps a scheduler. The same on a B200: 995 us with a lane per state, 413 with four lanes, expf, and
+// softplus and gate in a phase of their own, 250 here.
 constexpr int SC_CH = 64, SC_TB = 16;
-template <int SPL>
-__global__ void __launch_bounds__(SC_CH * 4) scan_recurrence_lanes_kernel(ScanArgs a, RaggedDev r) {
+// log(1 + exp(z)) and z / (1 + exp(-z)) without branches, so that they can run between other work; a unit or two in the last place.
+__device__ __forceinline__ float rcp_approx(float y) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
+    return r;
+}
+__device__ __forceinline__ float softplus_inline(float z) {
+    // log(1 + t), t = exp(-|z|) in [0, 1]: twice the inverse hyperbolic tangent of t / (2 + t) <= 1/3, as its power series
+    const float t = expf(-fabsf(z)), s = t * rcp_approx(2.f + t), x = s * s;
+    float p = 1.f / 15.f;
+    p = fmaf(p, x, 1.f / 13.f); p = fmaf(p, x, 1.f / 11.f); p = fmaf(p, x, 1.f / 9.f); p = fmaf(p, x, 1.f / 7.f); p = fmaf(p, x, 1.f / 5.f);
+    p = fmaf(p, x, 1.f / 3.f);
+    return fmaxf(z, 0.f) + 2.f * fmaf(p * x, s, s);
+}
+__device__ __forceinline__ float silu_inline(float z) {
+    const float y = 1.f + fminf(expf(-z), 1e37f), r = rcp_approx(y), v = z * r;
+    return fmaf(fmaf(-y, v, z), r, v);
+}
+template <int LANES, int SPL>
+__global__ void __launch_bounds__(SC_CH * LANES) scan_recurrence_lanes_kernel(ScanArgs a, RaggedDev r) {
     griddep_launch();
     griddep_wait();
-    constexpr int NP = 4 * SPL, STEP = SC_CH * 4;
-    __shared__ __align__(16) float in[3][3][SC_TB][SC_CH];          // [buffer][dt, x, gate][token][channel]
-    __shared__ __align__(16) float bc[3][2][SC_TB][NP];             // [buffer][B, C][token][lane][state of the lane]
-    const int seg = blockIdx.x, q = threadIdx.x & 3, lc = threadIdx.x >> 2, c0 = blockIdx.y * SC_CH, c = c0 + lc;
+    constexpr int ROW = LANES * 2 * SPL;                 // a token's B and C: per lane its states' B, then their C
+    extern __shared__ __align__(16) float sc_smem[];
+    float2* dd = reinterpret_cast<float2*>(sc_smem);     // [3][SC_TB][SC_CH]: dt, x as they come; then step size, step size times x
+    const int step = blockDim.x, n_ch = step / LANES;
+    constexpr int blk = SC_TB * SC_CH;
+    float2* gh = dd + 3 * blk;                           // the same of z, -; then gate, gate times D x
+    float* bc = reinterpret_cast<float*>(gh + 3 * blk);  // [3][SC_TB][ROW]
+    const int seg = blockIdx.x, q = threadIdx.x % LANES, lc = threadIdx.x / LANES, c0 = blockIdx.y * n_ch, c = c0 + lc;
     const int N = a.N;
     const bool c_ok = c < a.inner;
     const int cc = c_ok ? c : a.inner - 1;
@@ -928,118 +952,144 @@ __global__ void __launch_bounds__(SC_CH * 4) scan_recurrence_lanes_kernel(ScanAr
     float A[SPL], S[SPL];
 #pragma unroll
     for (int j = 0; j < SPL; j++) {
-        const int n = q + 4 * j;
-        A[j] = n < N ? -expf(a.A_log[(size_t)cc * N + n]) : 0.f;
+        const int n = q + LANES * j;
+        A[j] = n < N ? -expf(a.A_log[(size_t)cc * N + n]) * 1.4426950408889634f : 0.f;
         S[j] = n < N && c_ok ? sst[n] : 0.f;
     }
-    const float Dc = a.D[cc];
-    const int fch = threadIdx.x % SC_CH, fcc = min(c0 + fch, a.inner - 1);      // the channel this thread fetches for
-    const float dtb = a.dt_bias[fcc];
-    for (int j = threadIdx.x; j < 3 * 2 * SC_TB * NP; j += STEP) (&bc[0][0][0][0])[j] = 0.f;      // states past N stay zero
-    __syncthreads();
-    auto stage = [&](int i0, int buf) {
+    const int fch = threadIdx.x % n_ch, fu = threadIdx.x / n_ch, fcc = min(c0 + fch, a.inner - 1);      // the channel this thread fetches for, every LANES-th token
+    // (channels past the end: nothing. Many lanes that copy one address took the last CTA 346 us where the others took 244.)
+    const bool f_ok = c0 + fch < a.inner;
+    const float dtb = a.dt_bias[fcc], Dc = a.D[fcc];
+    if (N < LANES * SPL) {                               // states past the end stay zero (what idle channels hold goes nowhere)
+        for (int j = threadIdx.x; j < 3 * SC_TB * ROW; j += step) bc[j] = 0.f;
+        __syncthreads();
+    }
+    // the next block's first entries of this thread: its channel's inputs, and one column of the B and C rows (threads past the last whole token fetch none)
+    const int bc_e = threadIdx.x % (2 * N), bc_u = threadIdx.x / (2 * N), bc_du = step / (2 * N), bc_n = bc_e < N ? bc_e : bc_e - N;
+    const int bc_at = bc_n % LANES * 2 * SPL + (bc_e < N ? 0 : SPL) + bc_n / LANES;
+    const float *g_dt = a.dt_raw + (size_t)(start + fu) * a.inner + fcc, *g_x = a.xc + (size_t)(start + fu) * a.inner + fcc;
+    const float *g_z = a.proj + (size_t)(start + fu) * a.ldp + a.z_off + fcc, *g_bc = a.xproj + (size_t)(start + bc_u) * a.ldx + a.R + bc_e;
+    const size_t by_inner = (size_t)LANES * a.inner, by_ldp = (size_t)LANES * a.ldp, by_bc = (size_t)bc_du * a.ldx;
+    auto stage = [&](int i0, int buf) {                  // blocks in order
         const int nb = min(SC_TB, len - i0);
-        for (int u = threadIdx.x / SC_CH; u < nb; u += STEP / SC_CH) {
-            const size_t t = start + i0 + u;
-            cp_async_4(&in[buf][0][u][fch], a.dt_raw + t * a.inner + fcc);
-            cp_async_4(&in[buf][1][u][fch], a.xc + t * a.inner + fcc);
-            cp_async_4(&in[buf][2][u][fch], a.proj + t * a.ldp + a.z_off + fcc);
+        float2 *d = dd + buf * blk + fu * SC_CH + fch, *g = gh + buf * blk + fu * SC_CH + fch;
+#pragma unroll
+        for (int u = 0; u < SC_TB; u += LANES) {
+            if (f_ok && u + fu < nb) {
+                cp_async_4(&d[u * SC_CH].x, g_dt);
+                cp_async_4(&d[u * SC_CH].y, g_x);
+                cp_async_4(&g[u * SC_CH].x, g_z);
+            }
+            g_dt += by_inner; g_x += by_inner; g_z += by_ldp;
         }
-        for (int j = threadIdx.x; j < nb * 2 * N; j += STEP) {
-            const int u = j / (2 * N), e = j % (2 * N), n = e < N ? e : e - N;
-            cp_async_4(&bc[buf][e < N ? 0 : 1][u][(n & 3) * SPL + (n >> 2)], a.xproj + (size_t)(start + i0 + u) * a.ldx + a.R + e);
+        float* w = bc + buf * SC_TB * ROW + bc_at;
+        const float* p = g_bc;
+        if (bc_u < bc_du)
+            for (int u = bc_u; u < nb; u += bc_du, p += by_bc) cp_async_4(w + u * ROW, p);
+        g_bc += SC_TB * (size_t)a.ldx;
+    };
+    // what this thread fetched of a token, made ready in place
+    auto ready = [&](int at) {
+        const float2 v = dd[at];
+        const float dt = softplus_inline(v.x + dtb), gate = silu_inline(gh[at].x);
+        dd[at] = make_float2(dt, dt * v.y);
+        gh[at] = make_float2(gate, Dc * v.y * gate);
+    };
+    // a token's update of this lane's states; their sum times C
+    auto token = [&](const float2* d, const float* b) {
+        float2 v = *d;
+        float B[SPL], C[SPL];
+        if constexpr (SPL == 1) { const float2 w = *reinterpret_cast<const float2*>(b); B[0] = w.x; C[0] = w.y; }
+        else {
+#pragma unroll
+            for (int j = 0; j < 2 * SPL; j += 4) {
+                const float4 w = *reinterpret_cast<const float4*>(b + j);
+                const float k[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                for (int i = 0; i < 4; i++) { if (j + i < SPL) B[(j + i) % SPL] = k[i]; else C[(j + i) % SPL] = k[i]; }
+            }
         }
+        float sum = 0.f;
+#pragma unroll
+        for (int j = 0; j < SPL; j++) {
+            S[j] = fmaf(ex2_approx(v.x * A[j]), S[j], v.y * B[j]);
+            sum = j == 0 ? S[j] * C[j] : fmaf(S[j], C[j], sum);
+        }
+        return sum;
+    };
+    auto store = [&](int t, float y) {
+        if (!c_ok) return;
+        if (a.y_rounded) a.y_rounded[(size_t)t * a.inner + c] = __float2bfloat16(y);
+        else a.y[(size_t)t * a.inner + c] = y;
     };
     stage(0, 0);
     cp_async_commit();
     if (SC_TB < len) stage(SC_TB, 1);
     cp_async_commit();
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    for (int u = fu; u < min(SC_TB, len); u += LANES) ready(u * SC_CH + fch);
     int buf = 0;
     for (int i0 = 0; i0 < len; i0 += SC_TB) {
-        const int nb = min(SC_TB, len - i0);
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
-        // what this thread fetched of the block, made ready in place; then everybody's is visible
-        for (int u = threadIdx.x / SC_CH; u < nb; u += STEP / SC_CH) {
-            in[buf][0][u][fch] = softplus_f(in[buf][0][u][fch] + dtb);
-            in[buf][2][u][fch] = silu_f(in[buf][2][u][fch]);
-        }
+        const int nb = min(SC_TB, len - i0), next = buf == 2 ? 0 : buf + 1;
+        cp_async_wait_all();           // this thread's part of the next block has come; of this block it is ready, everybody's after the barrier
         __syncthreads();
-        const int nxt = buf == 0 ? 2 : buf - 1;
-        if (i0 + 2 * SC_TB < len) stage(i0 + 2 * SC_TB, nxt);        // everybody has left that buffer
+        if (i0 + 2 * SC_TB < len) stage(i0 + 2 * SC_TB, buf == 0 ? 2 : buf - 1);        // everybody has left that buffer
         cp_async_commit();
-        // four tokens at a time: their exponentials do not wait for one another, and the sums over the lanes cost three shuffles for the
-        // four, each lane ending up with the token it stores
+        // LANES tokens at a time: their exponentials do not wait for one another, and the sums over the lanes are exchanged in halves, each
+        // lane ending up with the token it stores. In between, what this thread fetched for one token of the next block is made ready (behind the
+        // last block: what stands in that buffer, for nothing; without a branch the two run side by side).
+        const float2 *d = dd + buf * blk + lc, *g = gh + buf * blk + lc;
+        const float* b = bc + buf * SC_TB * ROW + q * 2 * SPL;
         int u = 0;
-        for (; u + 4 <= nb; u += 4) {
-            float part[4], xu[4];
+        for (; u + LANES <= nb; u += LANES) {
+            float part[LANES];
 #pragma unroll
-            for (int t = 0; t < 4; t++) {
-                const float dt = in[buf][0][u + t][lc], xv = in[buf][1][u + t][lc];
-                xu[t] = xv;
-                const float* Bp = &bc[buf][0][u + t][q * SPL];
-                const float* Cp = &bc[buf][1][u + t][q * SPL];
-                float p[SPL];
+            for (int t = 0; t < LANES; t++) part[t] = token(d + (u + t) * SC_CH, b + (u + t) * ROW);
+            ready(next * blk + (u + fu) * SC_CH + fch);
 #pragma unroll
-                for (int j = 0; j < SPL; j++) {
-                    S[j] = expf(dt * A[j]) * S[j] + dt * xv * Bp[j];
-                    p[j] = __fmul_rn(S[j], Cp[j]);
-                }
+            for (int w = LANES / 2; w > 0; w >>= 1) {
+                const bool up = q & w;
 #pragma unroll
-                for (int w = SPL / 2; w > 0; w >>= 1)
-#pragma unroll
-                    for (int j = 0; j < w; j++) p[j] += p[j + w];
-                part[t] = p[0];
+                for (int t = 0; t < w; t++) part[t] = (up ? part[t + w] : part[t]) + __shfl_xor_sync(0xffffffffu, up ? part[t] : part[t + w], w);
             }
-            // lane q keeps token q: first halves two lanes apart (lanes 0, 1 keep tokens 0, 1), then neighbours
-            const bool up = q & 2, odd = q & 1;
-            const float s0 = (up ? part[2] : part[0]) + __shfl_xor_sync(0xffffffffu, up ? part[0] : part[2], 2);
-            const float s1 = (up ? part[3] : part[1]) + __shfl_xor_sync(0xffffffffu, up ? part[1] : part[3], 2);
-            const float sum = (odd ? s1 : s0) + __shfl_xor_sync(0xffffffffu, odd ? s0 : s1, 1);
-            const float xq = up ? (odd ? xu[3] : xu[2]) : (odd ? xu[1] : xu[0]);
-            if (c_ok) a.y[(size_t)(start + i0 + u + q) * a.inner + c] = (sum + Dc * xq) * in[buf][2][u + q][lc];
+            const float2 gate = g[(u + q) * SC_CH];
+            store(start + i0 + u + q, fmaf(part[0], gate.x, gate.y));
         }
         for (; u < nb; u++) {
-            const float dt = in[buf][0][u][lc], xv = in[buf][1][u][lc], gate = in[buf][2][u][lc];
-            const float* Bp = &bc[buf][0][u][q * SPL];
-            const float* Cp = &bc[buf][1][u][q * SPL];
-            float p[SPL];
+            float sum = token(d + u * SC_CH, b + u * ROW);
 #pragma unroll
-            for (int j = 0; j < SPL; j++) {
-                S[j] = expf(dt * A[j]) * S[j] + dt * xv * Bp[j];
-                p[j] = __fmul_rn(S[j], Cp[j]);
-            }
-#pragma unroll
-            for (int w = SPL / 2; w > 0; w >>= 1)
-#pragma unroll
-                for (int j = 0; j < w; j++) p[j] += p[j + w];
-            float sum = p[0];
-            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-            if (q == 0 && c_ok) a.y[(size_t)(start + i0 + u) * a.inner + c] = (sum + Dc * xv) * gate;
+            for (int w = LANES / 2; w > 0; w >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, w);
+            const float2 gate = g[u * SC_CH];
+            if (q == 0) store(start + i0 + u, fmaf(sum, gate.x, gate.y));
         }
-        buf = buf == 2 ? 0 : buf + 1;
+        buf = next;
     }
     if (c_ok) {
 #pragma unroll
-        for (int j = 0; j < SPL; j++) { const int n = q + 4 * j; if (n < N) sst[n] = S[j]; }
+        for (int j = 0; j < SPL; j++) { const int n = q + LANES * j; if (n < N) sst[n] = S[j]; }
     }
 }
+template <int LANES, int SPL>
+static cudaError_t launch_scan_lanes(const ScanArgs& a, const RaggedDev& r, cudaStream_t s) {
+    const int per_sm = (int)(((long)a.inner * r.n_seg + 147) / 148), n_ch = std::min(SC_CH, std::max(8, (per_sm + 7) / 8 * 8));
+    constexpr int smem = 3 * SC_TB * (SC_CH * 16 + LANES * 2 * SPL * 4);
+    static const bool ready = cudaFuncSetAttribute(scan_recurrence_lanes_kernel<LANES, SPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   smem) == cudaSuccess;
+    if (!ready) return cudaErrorInvalidValue;
+    return launch_chain(scan_recurrence_lanes_kernel<LANES, SPL>, dim3(r.n_seg, (a.inner + n_ch - 1) / n_ch), dim3(n_ch * LANES), smem, s, a, r);
+}
 
+bool scan_leaves_rounded(const ScanArgs& a) { return a.N <= 32; }
 cudaError_t scan_recurrence_launch(const ScanArgs& a, const RaggedDev& r, cudaStream_t s) {
-    if (a.N > SCAN_MAXS * 32) return cudaErrorInvalidValue;
+    if (a.N > SCAN_MAXS * 32 || (a.y_rounded && !scan_leaves_rounded(a))) return cudaErrorInvalidValue;
     PlainLaunch pl;        // latency-bound over the prompt: CTAs spread over all SMs (see kernels.h)
-    if (a.N <= 32) {
-        const dim3 grid(r.n_seg, (a.inner + SC_CH - 1) / SC_CH), block(SC_CH * 4);
-        if (a.N <= 4) return launch_chain(scan_recurrence_lanes_kernel<1>, grid, block, 0, s, a, r);
-        if (a.N <= 8) return launch_chain(scan_recurrence_lanes_kernel<2>, grid, block, 0, s, a, r);
-        if (a.N <= 16) return launch_chain(scan_recurrence_lanes_kernel<4>, grid, block, 0, s, a, r);
-        return launch_chain(scan_recurrence_lanes_kernel<8>, grid, block, 0, s, a, r);
-    }
+    if (a.N <= 4) return launch_scan_lanes<4, 1>(a, r, s);
+    if (a.N <= 8) return launch_scan_lanes<4, 2>(a, r, s);
+    if (a.N <= 16) return launch_scan_lanes<8, 2>(a, r, s);
+    if (a.N <= 32) return launch_scan_lanes<8, 4>(a, r, s);
     if (a.N <= 64) {
         const dim3 grid(r.n_seg, (a.inner + SCAN_CH - 1) / SCAN_CH), block(SCAN_CH);
         const size_t smem = (size_t)SCAN_TB * 2 * a.N * 4;
-        if (a.N <= 16) return launch_chain(scan_recurrence_chan_kernel<16>, grid, block, smem, s, a, r);
-        if (a.N <= 32) return launch_chain(scan_recurrence_chan_kernel<32>, grid, block, smem, s, a, r);
         return launch_chain(scan_recurrence_chan_kernel<64>, grid, block, smem, s, a, r);
     }
     return launch_chain(scan_recurrence_kernel, dim3(r.n_seg, (a.inner + 7) / 8), dim3(256), 0, s, a, r);
