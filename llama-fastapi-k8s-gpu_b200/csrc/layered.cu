@@ -1077,12 +1077,14 @@ static int mix_matrix_memory(b2_engine* e, LayeredModel* m, LyLayer& L, const Ra
     a.i_bias = L.i_b; a.f_bias = L.f_b; a.norm_w = L.mm_norm; a.H = d.mm_heads; a.d = d.mm_dim; a.dv = d.mm_vdim;
     a.cap = (float)d.gate_cap; a.eps = c.norm_eps; a.S = L.S; a.n = L.nvec; a.m = L.mmax; a.o_raw = m->buf[0]; a.out = m->buf[1];
     a.nq = m->buf[2]; a.m_scale = m->buf[2] + (size_t)T * d.mm_heads;
+    DenseArgs op = {};
+    if (takes_rounded(m, L.mm_o, T)) op.x_rounded = a.out_rounded = m->xb;
     {
         StepProfiler sp(m, e->stream, 4);
         CK(matrix_mem_launch(a, r, e->stream));
         e->launches += 3;
     }
-    return dense(e, m, L.mm_o, m->buf[1], vd, m->oL, W, T);
+    return dense(e, m, L.mm_o, m->buf[1], vd, m->oL, W, T, nullptr, EPI_NONE, 1, &op);
 }
 
 static int mix_latent_attn(b2_engine* e, LayeredModel* m, LyLayer& L, const RaggedDev& r, const float* in) {

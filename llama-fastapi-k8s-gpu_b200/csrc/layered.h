@@ -168,6 +168,7 @@ struct MatrixMemArgs {         // mLSTM
     float* o_raw;              // [T][H*dv] scratch: memory read-out before the normaliser and the head norm
     float *nq, *m_scale;       // [T][H] scratch: n . q and exp(-m) of every token
     float* out;                // [T][H*dv]
+    __nv_bfloat16* out_rounded = nullptr;      // the output goes here instead, rounded
 };
 cudaError_t matrix_mem_launch(const MatrixMemArgs& a, const RaggedDev& r, cudaStream_t s);
 

@@ -1101,83 +1101,92 @@ cudaError_t scan_recurrence_launch(const ScanArgs& a, const RaggedDev& r, cudaSt
 // factors exp(f + m_(t-1) - m_t) and exp(i - m_t) that a token's update takes. The maximum is one thread's serial chain over a block
 // of tokens in shared memory (two dependent operations a token); the rest is one token per thread. Left in place: decay over the
 // projection's f column, write weight over its i column; exp(-m_t) in m_scale [T][H].
-constexpr int MG_TB = 256;
+// Bound by that chain (2048 tokens: 10 us) and, per block of tokens, by a read, two gates and a write in a row: long steps take blocks of 1024
+// tokens (57 us in blocks of 256, 28 here).
+constexpr int MG_TB = 1024;
 __global__ void __launch_bounds__(MG_TB) matrix_mem_gates_kernel(MatrixMemArgs a, RaggedDev r) {
     griddep_launch();
     griddep_wait();
-    __shared__ float ig[MG_TB], fg[MG_TB], ms[MG_TB + 1];
-    const int seg = blockIdx.x, h = blockIdx.y;
+    __shared__ float2 g[MG_TB];                // log gates f, i
+    __shared__ float ms[MG_TB + 1];
+    const int seg = blockIdx.x, h = blockIdx.y, block = blockDim.x, u = threadIdx.x;
     const int slot = r.seg_slot[seg], start = r.seg_start[seg], len = r.seg_len[seg];
     const float ib = a.i_bias[h], fb = a.f_bias[h];
-    if (threadIdx.x == 0) ms[0] = a.m[(size_t)slot * a.H + h];
-    for (int i0 = 0; i0 < len; i0 += MG_TB) {
-        const int nb = min(MG_TB, len - i0), u = threadIdx.x;
+    if (u == 0) ms[0] = a.m[(size_t)slot * a.H + h];
+    for (int i0 = 0; i0 < len; i0 += block) {
+        const int nb = min(block, len - i0);
         float* p = const_cast<float*>(a.proj) + (size_t)(start + i0 + min(u, nb - 1)) * a.ldp;
+        float2 mine = make_float2(0.f, 0.f);
         if (u < nb) {
-            ig[u] = a.cap * tanhf((p[a.i_off + h] + ib) / a.cap);
-            fg[u] = log_sigmoid_f(a.cap * tanhf((p[a.f_off + h] + fb) / a.cap));
+            const float ri = p[a.i_off + h], rf = p[a.f_off + h];
+            mine.y = a.cap * tanhf((ri + ib) / a.cap);
+            mine.x = log_sigmoid_f(a.cap * tanhf((rf + fb) / a.cap));
+            g[u] = mine;
         }
         __syncthreads();
         if (u == 0) {
             float m = ms[0];
-#pragma unroll 8
-            for (int k = 0; k < nb; k++) { m = fmaxf(fg[k] + m, ig[k]); ms[k + 1] = m; }
+            int k = 0;
+            for (; k + 8 <= nb; k += 8) {      // read ahead of the chain
+                float2 v[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++) v[j] = g[k + j];
+#pragma unroll
+                for (int j = 0; j < 8; j++) { m = fmaxf(v[j].x + m, v[j].y); ms[k + j + 1] = m; }
+            }
+            for (; k < nb; k++) { m = fmaxf(g[k].x + m, g[k].y); ms[k + 1] = m; }
         }
         __syncthreads();
         if (u < nb) {
             const float m_new = ms[u + 1];
-            p[a.f_off + h] = expf(fg[u] + ms[u] - m_new);
-            p[a.i_off + h] = expf(ig[u] - m_new);
+            p[a.f_off + h] = expf(mine.x + ms[u] - m_new);
+            p[a.i_off + h] = expf(mine.y - m_new);
             a.m_scale[(size_t)(start + i0 + u) * a.H + h] = expf(-m_new);
         }
         const float last = ms[nb];
         __syncthreads();
         if (u == 0) ms[0] = last;
     }
-    if (threadIdx.x == 0) a.m[(size_t)slot * a.H + h] = ms[0];
+    if (u == 0) a.m[(size_t)slot * a.H + h] = ms[0];
 }
 
-// grid (n_seg, H, ceil(dv / 32) + 1): a CTA owns 32 columns of one head's d x dv memory. Thread (pair, grp) keeps rows grp * MM_ROWS ..
-// of two neighbouring columns in registers: a 16-byte read of k or q out of shared memory occupies its pipe for four cycles even when all
-// lanes want the same bytes, so with one column a thread the reads (8 a token and warp, 8 warps) bounded the kernel. Tokens go in blocks of MM_TB: a thread's state update for token t + 1 needs only its own registers
-// after token t, so the block barrier is paid once per block -- for the inputs (q, k, v and the two factors of the next block arrive
-// in shared memory as asynchronous copies while this block is computed) and for the partial read-outs per row group, which all
-// threads then sum in a fixed order, one (token, column) each. The CTA past the last columns carries the normaliser n (a lane per
-// row) and leaves n . q; the division by it waits for matrix_mem_out_kernel.
-// Bound by the latency of the updates and read-outs, one or two warps a scheduler: 64 multiply-adds, 32 products and 8 shared loads per
-// token and warp. A 2048-token prompt of 16 heads of 128 x 256 (B200): 966 us with one column a thread, 580 with two, 428 with the next
-// token's operands fetched ahead and the read-outs apart from the updates.
-constexpr int MM_ROWS = 16, MM_COLS = 32, MM_TB = 16;      // key size <= 16 * 16 = 256 (256 threads)
-__global__ void __launch_bounds__(256, 1) matrix_mem_kernel(MatrixMemArgs a, RaggedDev r, int RG) {
+// grid (n_seg, H, ceil(dv / 32) + 1): a CTA owns 32 columns of one head's d x dv memory, two neighbouring ones and MM_ROWS rows a thread, in
+// registers as pairs of rows. A warp is 16 such column pairs by 2 row groups; a token's k and q are read from shared memory as they lie, in pairs of
+// rows: a read brings 4 bytes a cycle to every lane, whether lanes want the same or not, so the columns a thread has decide how many reads
+// a multiply-add costs. Tokens go in blocks of MM_TB: a state update needs only the thread's own registers, so the block barrier is paid
+// once per block -- for the inputs (q, k, v and the two factors of the next block arrive in shared memory as asynchronous copies while this
+// block is computed) and for the partial read-outs of the row groups, which all threads then sum in a fixed order.
+// The CTA past the last columns carries the normaliser n as one column whose v is 1, and leaves n . q; the division by it waits for
+// matrix_mem_out_kernel.
+// Bound by multiply-adds (24 pairs a token and warp, two cycles each) and shared reads (18 cycles a token and warp, eight warps a pipe) about alike,
+// and by their latency with two warps a scheduler. A 2048-token prompt of 16 heads of 128 x 256 (B200): 966 us with one column a thread, 428 with two columns of 16 rows
+// and one warp a scheduler, 315 here (four columns a thread and one warp: 400; two tokens side by side, single multiply-adds: the same).
+constexpr int MM_ROWS = 8, MM_COLS = 32, MM_TB = 16, MM_MAX_D = 256;      // (16 warps at most)
+__global__ void __launch_bounds__(512, 1) matrix_mem_kernel(MatrixMemArgs a, RaggedDev r) {
     griddep_launch();
     griddep_wait();
-    extern __shared__ float sm[];
-    const int d = a.d, dv = a.dv;
-    float* qs = sm;                                // [2][MM_TB][d]
-    float* ks = qs + 2 * MM_TB * d;                // [2][MM_TB][d]
-    float* vs = ks + 2 * MM_TB * d;                // [2][MM_TB][MM_COLS]
+    extern __shared__ __align__(16) float sm[];
+    const int d = a.d, dv = a.dv, n_warps = blockDim.x / 32;
+    const int dp = n_warps * 2 * MM_ROWS, red_tok = 2 * n_warps * MM_COLS;      // rows, with those past the end; partial read-outs of a token
+    float* qs = sm;                                // [2][MM_TB][dp]
+    float* ks = qs + 2 * MM_TB * dp;               // [2][MM_TB][dp]
+    float* vs = ks + 2 * MM_TB * dp;               // [2][MM_TB][MM_COLS]
     float* gs = vs + 2 * MM_TB * MM_COLS;          // [2][MM_TB][2]: write weight, decay
-    float* red = gs + 2 * MM_TB * 2;               // [2][MM_TB][RG][MM_COLS]: partial read-outs
-    const int red_tok = RG * MM_COLS;
+    float* red = gs + 2 * MM_TB * 2;               // [2][MM_TB][2 n_warps][MM_COLS]: partial read-outs of the row groups
     const bool norm_cta = blockIdx.z == gridDim.z - 1;
-    const int seg = blockIdx.x, h = blockIdx.y, c0 = norm_cta ? 0 : blockIdx.z * MM_COLS, n_cols = norm_cta ? 0 : min(MM_COLS, dv - c0);
+    const int seg = blockIdx.x, h = blockIdx.y, c0 = norm_cta ? 0 : blockIdx.z * MM_COLS, n_cols = norm_cta ? 1 : min(MM_COLS, dv - c0);
     const int slot = r.seg_slot[seg], start = r.seg_start[seg], len = r.seg_len[seg];
-    const int lp = threadIdx.x % 16, grp = threadIdx.x / 16;      // column pair, row group
-    const bool act = grp < RG;                     // threads past the last row group only help with copies and sums
-    const bool mem0 = act && 2 * lp < n_cols, mem1 = act && 2 * lp + 1 < n_cols;
-    float* Sg = a.S + (((size_t)slot * a.H + h) * d) * dv + c0 + 2 * lp;
-    float* ng = a.n + ((size_t)slot * a.H + h) * d;
-    float S0[MM_ROWS], S1[MM_ROWS];
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, col = (lane & 15) * 2, row = (warp * 2 + (lane >> 4)) * MM_ROWS;
+    // this thread's part of the memory (or, one column, of the normaliser)
+    float* Sg = norm_cta ? a.n + ((size_t)slot * a.H + h) * d : a.S + (((size_t)slot * a.H + h) * d) * dv + c0;
+    const int lds = norm_cta ? 1 : dv;
+    uint64_t S[MM_ROWS / 2][2];
+    auto at = [&](int i, int j) { return Sg + (size_t)(row + i) * lds + col + j; };
+    auto own = [&](int i, int j) { return row + i < d && col + j < n_cols; };
 #pragma unroll
-    for (int i = 0; i < MM_ROWS; i++) {
-        const int row = grp * MM_ROWS + i;
-        S0[i] = (mem0 && row < d) ? Sg[(size_t)row * dv] : 0.f;
-        S1[i] = (mem1 && row < d) ? Sg[(size_t)row * dv + 1] : 0.f;
-    }
-    const int nrow = grp * MM_ROWS + lp;                      // a lane per row of n
-    const bool n_ok = norm_cta && act && nrow < d;
-    float nr = n_ok ? ng[nrow] : 0.f;
-    const bool vec4 = (d % 4) == 0;
+    for (int i = 0; i < MM_ROWS / 2; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) S[i][j] = f2_pack(own(2 * i, j) ? *at(2 * i, j) : 0.f, own(2 * i + 1, j) ? *at(2 * i + 1, j) : 0.f);
     const float qscale = 1.f / sqrtf((float)d);
     // q and k rows as 16-byte copies where they start on 16 bytes
     const bool wide = d % 4 == 0 && a.ldp % 4 == 0 && a.q_off % 4 == 0 && a.k_off % 4 == 0 && (reinterpret_cast<uintptr_t>(a.proj) & 15) == 0;
@@ -1188,7 +1197,7 @@ __global__ void __launch_bounds__(256, 1) matrix_mem_kernel(MatrixMemArgs a, Rag
         const int nb = min(MM_TB, len - i0);
         auto copy = [&](int u, int e) {
             const float* p = a.proj + (size_t)(start + i0 + u) * a.ldp + h * d + e;
-            float *qd = &qs[(buf * MM_TB + u) * d + e], *kd = &ks[(buf * MM_TB + u) * d + e];
+            float *qd = &qs[(buf * MM_TB + u) * dp + e], *kd = &ks[(buf * MM_TB + u) * dp + e];
             if (wide) { cp_async_16z(qd, p + a.q_off, 16); cp_async_16z(kd, p + a.k_off, 16); }
             else { cp_async_4(qd, p + a.q_off); cp_async_4(kd, p + a.k_off); }
         };
@@ -1197,24 +1206,29 @@ __global__ void __launch_bounds__(256, 1) matrix_mem_kernel(MatrixMemArgs a, Rag
         for (int j = threadIdx.x; j < nb * MM_COLS; j += blockDim.x) {
             const int u = j / MM_COLS, e = j % MM_COLS;
             const float* p = a.proj + (size_t)(start + i0 + u) * a.ldp;
-            if (e < n_cols) cp_async_4(&vs[(buf * MM_TB + u) * MM_COLS + e], p + a.v_off + h * dv + c0 + e);
+            if (e < n_cols && !norm_cta) cp_async_4(&vs[(buf * MM_TB + u) * MM_COLS + e], p + a.v_off + h * dv + c0 + e);
             if (e < 2) cp_async_4(&gs[(buf * MM_TB + u) * 2 + e], p + (e == 0 ? a.i_off : a.f_off) + h);
         }
     };
-    auto finish = [&](int i0, int buf) {                 // sum of the row groups in a fixed order
-        const int nb = min(MM_TB, len - i0), cols = norm_cta ? 1 : MM_COLS;
-        for (int j = threadIdx.x; j < nb * cols; j += blockDim.x) {
-            const int u = norm_cta ? j : j / MM_COLS, e = norm_cta ? 0 : j % MM_COLS;
-            if (!norm_cta && e >= n_cols) continue;
-            const float* rd = red + (size_t)(buf * MM_TB + u) * red_tok;
+    auto finish = [&](int i0, int buf) {                 // sum over the row groups in a fixed order
+        const int nb = min(MM_TB, len - i0), u0 = threadIdx.x / MM_COLS, e = threadIdx.x % MM_COLS;
+        if (e >= n_cols) return;
+        for (int u = u0; u < nb; u += n_warps) {
+            const float* rd = red + (size_t)(buf * MM_TB + u) * red_tok + e;
             float sum = 0.f;
-            for (int g2 = 0; g2 < RG; g2++) sum += rd[g2 * MM_COLS + e];
-            if (norm_cta) a.nq[(size_t)(start + i0 + u) * a.H + h] = sum;
-            else a.o_raw[(size_t)(start + i0 + u) * a.H * dv + (size_t)h * dv + c0 + e] = sum;
+#pragma unroll 8
+            for (int w = 0; w < 2 * n_warps; w++) sum += rd[w * MM_COLS];
+            const size_t t = start + i0 + u;
+            if (norm_cta) a.nq[t * a.H + h] = sum * qscale;
+            else a.o_raw[t * a.H * dv + (size_t)h * dv + c0 + e] = sum * qscale;
         }
     };
-    for (int j = threadIdx.x; j < 2 * MM_TB * MM_COLS; j += blockDim.x) vs[j] = 0.f;
-    __syncthreads();
+    // what no copy brings: rows past the end stay zero, the normaliser's one column is 1 (what idle columns hold goes nowhere)
+    if (d < dp || norm_cta) {
+        if (d < dp) for (int j = threadIdx.x; j < 4 * MM_TB * dp; j += blockDim.x) qs[j] = 0.f;
+        if (norm_cta) for (int j = threadIdx.x; j < 2 * MM_TB; j += blockDim.x) vs[j * MM_COLS] = 1.f;
+        __syncthreads();
+    }
     if (len > 0) stage(0, 0);
     cp_async_commit();
     for (int i0 = 0; i0 < len; i0 += MM_TB) {
@@ -1224,107 +1238,123 @@ __global__ void __launch_bounds__(256, 1) matrix_mem_kernel(MatrixMemArgs a, Rag
         if (i0 + MM_TB < len) stage(i0 + MM_TB, buf ^ 1);
         cp_async_commit();
         if (i0 > 0) finish(i0 - MM_TB, buf ^ 1);
-        if (norm_cta) {
+        // the next token's row pieces and factors are read while this one is computed: latency hides only behind a warp's own work
+        const float *kr = ks + buf * MM_TB * dp + row, *qr = qs + buf * MM_TB * dp + row, *vr = vs + buf * MM_TB * MM_COLS + col, *gr = gs + buf * MM_TB * 2;
+        float* out = red + (size_t)buf * MM_TB * red_tok + (warp * 2 + (lane >> 4)) * MM_COLS + col;
+        ulonglong2 kn[2], qn[2];
+        float2 vn, gn;
+        auto fetch = [&]() {
+            const ulonglong2 *k = reinterpret_cast<const ulonglong2*>(kr), *q = reinterpret_cast<const ulonglong2*>(qr);
+            kn[0] = k[0]; kn[1] = k[1]; qn[0] = q[0]; qn[1] = q[1];
+            vn = *reinterpret_cast<const float2*>(vr); gn = *reinterpret_cast<const float2*>(gr);
+        };
+        fetch();
+        uint64_t decay = f2_pack(gn.y, gn.y), vv[2] = {f2_pack(gn.x * vn.x, gn.x * vn.x), f2_pack(gn.x * vn.y, gn.x * vn.y)};
 #pragma unroll 4
-            for (int u = 0; u < nb; u++) {
-                const int bu = buf * MM_TB + u;
-                const float ib = gs[bu * 2], da = gs[bu * 2 + 1];
-                float npart = 0.f;
-                if (n_ok) { nr = fmaf(da, nr, ib * ks[bu * d + nrow]); npart = nr * qs[bu * d + nrow]; }
+        for (int u = 0; u < nb; u++) {
+            const uint64_t kk[4] = {kn[0].x, kn[0].y, kn[1].x, kn[1].y}, qq[4] = {qn[0].x, qn[0].y, qn[1].x, qn[1].y};
+            if (u + 1 < nb) { kr += dp; qr += dp; vr += MM_COLS; gr += 2; }
+            fetch();
+            float p[2];
 #pragma unroll
-                for (int o = MM_ROWS / 2; o > 0; o >>= 1) npart += __shfl_xor_sync(0xffffffffu, npart, o);
-                if (act && lp == 0) red[(size_t)bu * red_tok + grp * MM_COLS] = npart * qscale;
+            for (int j = 0; j < 2; j++) {
+#pragma unroll
+                for (int i = 0; i < 4; i++) S[i][j] = f2_fma(decay, S[i][j], f2_mul(kk[i], vv[j]));
+                const uint64_t s0 = f2_fma(S[2][j], qq[2], f2_mul(S[0][j], qq[0])), s1 = f2_fma(S[3][j], qq[3], f2_mul(S[1][j], qq[1]));
+                const float2 x = f2_unpack(s0), y = f2_unpack(s1);
+                p[j] = (x.x + x.y) + (y.x + y.y);
             }
-        } else if (act) {
-            const bool full = vec4 && grp * MM_ROWS + MM_ROWS <= d;
-            if (full) {
-                // the next token's row pieces and factors are read while this one is computed, the updates of all rows stand apart from the
-                // two read-out chains: a scheduler has one warp of this kernel, so latency hides only behind the warp's own work
-                float4 kn[4], qn[4];
-                float2 gn, vn;
-                auto fetch = [&](int u) {
-                    const int bu = buf * MM_TB + u;
-                    const float *kr = ks + bu * d + grp * MM_ROWS, *qr = qs + bu * d + grp * MM_ROWS;
-#pragma unroll
-                    for (int i = 0; i < 4; i++) { kn[i] = *reinterpret_cast<const float4*>(kr + 4 * i); qn[i] = *reinterpret_cast<const float4*>(qr + 4 * i); }
-                    gn = *reinterpret_cast<const float2*>(gs + bu * 2); vn = *reinterpret_cast<const float2*>(vs + bu * MM_COLS + 2 * lp);
-                };
-                fetch(0);
-#pragma unroll 2
-                for (int u = 0; u < nb; u++) {
-                    const float kk[16] = {kn[0].x, kn[0].y, kn[0].z, kn[0].w, kn[1].x, kn[1].y, kn[1].z, kn[1].w,
-                                          kn[2].x, kn[2].y, kn[2].z, kn[2].w, kn[3].x, kn[3].y, kn[3].z, kn[3].w};
-                    const float qq[16] = {qn[0].x, qn[0].y, qn[0].z, qn[0].w, qn[1].x, qn[1].y, qn[1].z, qn[1].w,
-                                          qn[2].x, qn[2].y, qn[2].z, qn[2].w, qn[3].x, qn[3].y, qn[3].z, qn[3].w};
-                    const float da = gn.y, v0 = gn.x * vn.x, v1 = gn.x * vn.y;
-                    fetch(min(u + 1, nb - 1));
-                    float p0 = 0.f, p1 = 0.f;
-#pragma unroll
-                    for (int i = 0; i < 16; i++) { S0[i] = fmaf(da, S0[i], kk[i] * v0); S1[i] = fmaf(da, S1[i], kk[i] * v1); }
-#pragma unroll
-                    for (int i = 0; i < 16; i++) { p0 = fmaf(S0[i], qq[i], p0); p1 = fmaf(S1[i], qq[i], p1); }
-                    *reinterpret_cast<float2*>(red + (size_t)(buf * MM_TB + u) * red_tok + grp * MM_COLS + 2 * lp) = make_float2(p0 * qscale, p1 * qscale);
-                }
-            } else
-            for (int u = 0; u < nb; u++) {
-                const int bu = buf * MM_TB + u;
-                const float2 g2 = *reinterpret_cast<const float2*>(gs + bu * 2), v2 = *reinterpret_cast<const float2*>(vs + bu * MM_COLS + 2 * lp);
-                const float da = g2.y, v0 = g2.x * v2.x, v1 = g2.x * v2.y;
-                float p0 = 0.f, p1 = 0.f;
-                const float* kr = ks + bu * d + grp * MM_ROWS;
-                const float* qr = qs + bu * d + grp * MM_ROWS;
-#pragma unroll
-                    for (int k = 0; k < MM_ROWS; k++)
-                        if (grp * MM_ROWS + k < d) {
-                            S0[k] = fmaf(da, S0[k], kr[k] * v0); p0 = fmaf(S0[k], qr[k], p0);
-                            S1[k] = fmaf(da, S1[k], kr[k] * v1); p1 = fmaf(S1[k], qr[k], p1);
-                        }
-                *reinterpret_cast<float2*>(red + (size_t)bu * red_tok + grp * MM_COLS + 2 * lp) = make_float2(p0 * qscale, p1 * qscale);
-            }
+            *reinterpret_cast<float2*>(out) = make_float2(p[0], p[1]);
+            out += red_tok;
+            decay = f2_pack(gn.y, gn.y);
+            vv[0] = f2_pack(gn.x * vn.x, gn.x * vn.x); vv[1] = f2_pack(gn.x * vn.y, gn.x * vn.y);
         }
     }
     __syncthreads();
     if (len > 0) { const int last0 = (len - 1) / MM_TB * MM_TB; finish(last0, (last0 / MM_TB) & 1); }
 #pragma unroll
-    for (int i = 0; i < MM_ROWS; i++) {
-        const int row = grp * MM_ROWS + i;
-        if (mem0 && row < d) Sg[(size_t)row * dv] = S0[i];
-        if (mem1 && row < d) Sg[(size_t)row * dv + 1] = S1[i];
-    }
-    if (n_ok) ng[nrow] = nr;
+    for (int i = 0; i < MM_ROWS / 2; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const float2 v = f2_unpack(S[i][j]);
+            if (own(2 * i, j)) *at(2 * i, j) = v.x;
+            if (own(2 * i + 1, j)) *at(2 * i + 1, j) = v.y;
+        }
 }
 
-// per (token, head): o = read-out / normaliser; out = o / rms(o) * norm_w * sigmoid(gate)
-__global__ void __launch_bounds__(128) matrix_mem_out_kernel(MatrixMemArgs a) {
+// per (token, head): o = read-out / normaliser; out = o / rms(o) * norm_w * sigmoid(gate). A warp each; a lane keeps its entries (MO_U reads of
+// four ahead of the first use) where the head has at most 128 MO_U of them and rows start on 16 bytes, else reads them again. Bound by memory: 100 MB
+// for 2048 tokens of 16 x 256 (53 us with a CTA per token and head and one entry a read, 37 here).
+constexpr int MO_U = 4;
+__global__ void __launch_bounds__(256) matrix_mem_out_kernel(MatrixMemArgs a, int T, int wide) {
     griddep_launch();
     griddep_wait();
-    __shared__ float red[33];
-    const int t = blockIdx.x, h = blockIdx.y;
+    const int lane = threadIdx.x & 31;
+    const long i = blockIdx.x * 8l + (threadIdx.x >> 5);
+    if (i >= (long)T * a.H) return;
+    const int t = (int)(i / a.H), h = (int)(i % a.H);
     const size_t base = (size_t)t * a.H * a.dv + (size_t)h * a.dv;
-    const float den = fmaxf(fabsf(a.nq[(size_t)t * a.H + h]), a.m_scale[(size_t)t * a.H + h]) + 1e-6f;
+    const float nq = a.nq[i], m_scale = a.m_scale[i];
+    auto inverse = [&] { return 1.f / (fmaxf(fabsf(nq), m_scale) + 1e-6f); };
+    const float* gate = a.proj + (size_t)t * a.ldp + a.g_off + h * a.dv;
+    const float *o = a.o_raw + base, *w = a.norm_w + h * a.dv;
     float ss = 0.f;
-    for (int i = threadIdx.x; i < a.dv; i += blockDim.x) { const float v = a.o_raw[base + i] / den; ss += v * v; }
-    const float rinv = 1.f / sqrtf(block_sum(ss, red) / (float)a.dv + a.eps);
-    for (int i = threadIdx.x; i < a.dv; i += blockDim.x) {
-        const float gate = sigmoid_f(a.proj[(size_t)t * a.ldp + a.g_off + h * a.dv + i]);
-        a.out[base + i] = a.o_raw[base + i] / den * rinv * a.norm_w[h * a.dv + i] * gate;
+    if (wide) {
+        float4 v[MO_U], z[MO_U], n[MO_U];
+#pragma unroll
+        for (int k = 0; k < MO_U; k++) {
+            const int e = (k * 32 + lane) * 4;
+            if (e < a.dv) { v[k] = *reinterpret_cast<const float4*>(o + e); z[k] = *reinterpret_cast<const float4*>(gate + e); n[k] = *reinterpret_cast<const float4*>(w + e); }
+            else v[k] = z[k] = n[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        const float inv = inverse();
+#pragma unroll
+        for (int k = 0; k < MO_U; k++) {
+            if (k * 128 >= a.dv) break;
+            v[k].x *= inv; v[k].y *= inv; v[k].z *= inv; v[k].w *= inv;
+            ss += v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
+        }
+        const float rinv = 1.f / sqrtf(warp_sum(ss) / (float)a.dv + a.eps);
+#pragma unroll
+        for (int k = 0; k < MO_U; k++) {
+            const int e = (k * 32 + lane) * 4;
+            if (e >= a.dv) break;
+            const float4 y = make_float4(v[k].x * rinv * n[k].x * sigmoid_f(z[k].x), v[k].y * rinv * n[k].y * sigmoid_f(z[k].y),
+                                         v[k].z * rinv * n[k].z * sigmoid_f(z[k].z), v[k].w * rinv * n[k].w * sigmoid_f(z[k].w));
+            if (a.out_rounded) {
+                const __nv_bfloat162 lo = __floats2bfloat162_rn(y.x, y.y), hi = __floats2bfloat162_rn(y.z, y.w);
+                *reinterpret_cast<uint2*>(a.out_rounded + base + e) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+            } else *reinterpret_cast<float4*>(a.out + base + e) = y;
+        }
+    } else {
+        const float inv = inverse();
+        for (int e = lane; e < a.dv; e += 32) { const float v = o[e] * inv; ss += v * v; }
+        const float rinv = 1.f / sqrtf(warp_sum(ss) / (float)a.dv + a.eps);
+        for (int e = lane; e < a.dv; e += 32) {
+            const float y = o[e] * inv * rinv * w[e] * sigmoid_f(gate[e]);
+            if (a.out_rounded) a.out_rounded[base + e] = __float2bfloat16(y);
+            else a.out[base + e] = y;
+        }
     }
 }
 
 cudaError_t matrix_mem_launch(const MatrixMemArgs& a, const RaggedDev& r, cudaStream_t s) {
-    if (a.dv <= 0 || a.d <= 0 || a.d > MM_ROWS * 16) return cudaErrorInvalidValue;
-    const int RG = (a.d + MM_ROWS - 1) / MM_ROWS;
-    const size_t smem = (size_t)(2 * MM_TB * (2 * a.d + MM_COLS + 2 + RG * MM_COLS)) * 4;
-    static bool attr_done = false;
-    if (!attr_done) { cudaFuncSetAttribute(matrix_mem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 140 * 1024); attr_done = true; }
-    cudaError_t ce = launch_chain(matrix_mem_gates_kernel, dim3(r.n_seg, a.H), dim3(MG_TB), 0, s, a, r);
+    if (a.dv <= 0 || a.d <= 0 || a.d > MM_MAX_D) return cudaErrorInvalidValue;
+    cudaError_t ce = launch_chain(matrix_mem_gates_kernel, dim3(r.n_seg, a.H), dim3(r.T >= 512 ? MG_TB : 256), 0, s, a, r);
     if (ce != cudaSuccess) return ce;
     {
         PlainLaunch pl;    // latency-bound over the prompt: CTAs spread over all SMs (see kernels.h)
-        ce = launch_chain(matrix_mem_kernel, dim3(r.n_seg, a.H, (a.dv + MM_COLS - 1) / MM_COLS + 1), dim3(std::max((RG * 16 + 31) / 32 * 32, 64)), smem, s, a, r, RG);
+        const int n_warps = (a.d + 2 * MM_ROWS - 1) / (2 * MM_ROWS);
+        const size_t smem = (size_t)2 * MM_TB * (2 * n_warps * 2 * MM_ROWS + MM_COLS + 2 + 2 * n_warps * MM_COLS) * 4;
+        static const bool ready = cudaFuncSetAttribute(matrix_mem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) == cudaSuccess;
+        if (!ready) return cudaErrorInvalidValue;
+        ce = launch_chain(matrix_mem_kernel, dim3(r.n_seg, a.H, (a.dv + MM_COLS - 1) / MM_COLS + 1), dim3(n_warps * 32), smem, s, a, r);
     }
     if (ce != cudaSuccess) return ce;
-    return launch_chain(matrix_mem_out_kernel, dim3(r.T, a.H), dim3(128), 0, s, a);
+    const uintptr_t rows = reinterpret_cast<uintptr_t>(a.o_raw) | reinterpret_cast<uintptr_t>(a.out) | reinterpret_cast<uintptr_t>(a.out_rounded) |
+                           reinterpret_cast<uintptr_t>(a.proj) | reinterpret_cast<uintptr_t>(a.norm_w);
+    const int wide = a.dv % 4 == 0 && a.dv <= 128 * MO_U && a.ldp % 4 == 0 && a.g_off % 4 == 0 && (rows & 15) == 0;
+    return launch_chain(matrix_mem_out_kernel, dim3((unsigned)(((long)r.T * a.H + 7) / 8)), dim3(256), 0, s, a, r.T, wide);
 }
 
 }  // namespace b2
