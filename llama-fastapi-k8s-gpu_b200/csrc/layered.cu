@@ -110,7 +110,9 @@ struct LayeredModel {
     __nv_bfloat16 *hn_b = nullptr, *mix_b = nullptr, *moe_hb = nullptr;
     // few-token steps: an expert product that the mixer's next product takes along in its launch (cleared when it has)
     const DenseArgs* rider = nullptr;
-    const __nv_bfloat16* hn_rounded = nullptr;      // hn_b when the step's boundary kernels fill it
+    __nv_bfloat16 *hn2_b = nullptr, *x_b = nullptr;      // the same of the second norm, of the stream itself (post-sum blocks)
+    // hn_b, hn2_b, x_b when the step's boundary kernels fill them: what a product over hn, hn2, x reads
+    const __nv_bfloat16 *hn_rounded = nullptr, *hn2_rounded = nullptr, *x_rounded = nullptr;
     std::unordered_map<std::string, StepGraph> graphs;     // replayable small steps, by shape (b2_step)
     bool graphs_on = true;
     // mixture of experts: router outputs, choices, the sorted pair table, expert activations and outputs
@@ -708,7 +710,9 @@ int layered_finalize(b2_engine* e) {
     if ((rc = dev_alloc(m, (void**)&m->ff, (size_t)Tm * max_ff * 4))) return rc;
     const size_t widest = (size_t)(Tm + B2_STEP_MAX_ENTRIES) * std::max<size_t>({max_buf, max_ff, (size_t)(c.loop_times > 0 ? 2 * W : W), moe_xb});
     if (m->exact ? (rc = dev_alloc(m, (void**)&m->x_parts, 3 * widest * 2 + 64)) : (rc = dev_alloc(m, (void**)&m->xb, widest * 2 + 64))) return rc;
-    if (one_norm && !m->exact) {
+    if (!m->exact && parallel && (rc = dev_alloc(m, (void**)&m->hn2_b, (size_t)Tm * W * 2 + 64))) return rc;
+    if (!m->exact && c.block_style == B2_BLOCK_POSTSUM_LN && (rc = dev_alloc(m, (void**)&m->x_b, (size_t)Tm * W * 2 + 64))) return rc;
+    if ((one_norm || parallel) && !m->exact) {
         if ((rc = dev_alloc(m, (void**)&m->hn_b, (size_t)Tm * W * 2 + 64))) return rc;
         if (max_mix > 0 && (rc = dev_alloc(m, (void**)&m->mix_b, (size_t)Tm * max_mix * 2 + 64))) return rc;
     }
@@ -991,6 +995,8 @@ static DenseArgs dense_args(const LayeredModel* m, const DenseW& w, const float*
     DenseArgs a = more ? *more : DenseArgs{};
     a.x = x; a.ldx = ldx; a.w = w.w; a.w_type = w.type; a.bias = bias; a.y = y; a.ldy = ldy; a.T = T; a.N = w.N; a.K = w.K;
     a.epi = epi; a.exact = m->exact || (more && more->exact); a.xb = m->xb; a.x_parts = m->x_parts;
+    const __nv_bfloat16* left = x == m->hn ? m->hn_rounded : x == m->hn2 ? m->hn2_rounded : x == m->x ? m->x_rounded : nullptr;
+    if (left && !a.x_rounded && a.batch == 1 && a.K == m->c.n_embd && dense_takes_rounded(a)) a.x_rounded = left;
     return a;
 }
 static int dense_run(b2_engine* e, LayeredModel* m, const DenseArgs& a, int kind) {
@@ -1036,24 +1042,27 @@ static int mix_window_scan(b2_engine* e, LayeredModel* m, LyLayer& L, const Ragg
     a.H = d.n_head; a.G = d.n_head_kv; a.d = d.head_dim; a.window = d.window;
     a.keep_first = d.keep_first; a.scale = (float)d.attn_scale; a.eps = c.norm_eps; a.q_rot = m->buf[0]; a.out = m->buf[1];
     a.split_scratch = m->attn_split; a.split_capacity = m->attn_split_floats;
+    DenseArgs ao = {}, sx = {};
+    if (takes_rounded(m, L.attn_o, T) && window_attn_leaves_rounded(a, T)) ao.x_rounded = a.out_rounded = m->xb;
     {
         StepProfiler sp(m, st, 2);
         CK(window_attn_store_launch(a, r, st));
         CK(window_attn_launch(a, r, st));
         e->launches += 2;
     }
-    if ((rc = dense(e, m, L.attn_o, m->buf[1], qd, m->oL, W, T))) return rc;
+    if ((rc = dense(e, m, L.attn_o, m->buf[1], qd, m->oL, W, T, nullptr, EPI_NONE, 1, &ao))) return rc;
     ScanArgs s = {};
     s.proj = m->proj; s.ldp = Np; s.x_off = L.x_off; s.z_off = L.z_off; s.conv_w = L.conv_w; s.conv_b = L.conv_b;
     s.taps = d.conv_taps; s.conv_state = L.conv_state; s.xc = m->buf[0]; s.xproj = m->buf[2];
     s.ldx = d.dt_rank + 2 * d.d_state; s.R = d.dt_rank; s.N = d.d_state; s.dt_raw = m->buf[3]; s.dt_bias = L.dt_b;
     s.A_log = L.A_log; s.D = L.Dskip; s.ssm_state = L.ssm_state; s.y = m->buf[1]; s.inner = d.d_inner;
+    if (takes_rounded(m, L.scan_x, T)) sx.x_rounded = s.xc_rounded = m->xb;
     {
         StepProfiler sp(m, st, 3);
         CK(scan_conv_launch(s, r, st));
         e->launches++;
     }
-    if ((rc = dense(e, m, L.scan_x, m->buf[0], d.d_inner, m->buf[2], s.ldx, T))) return rc;
+    if ((rc = dense(e, m, L.scan_x, m->buf[0], d.d_inner, m->buf[2], s.ldx, T, nullptr, EPI_NONE, 1, &sx))) return rc;
     if ((rc = dense(e, m, L.scan_dt, m->buf[2], s.ldx, m->buf[3], d.d_inner, T))) return rc;
     DenseArgs so = {};
     if (takes_rounded(m, L.scan_o, T) && scan_leaves_rounded(s)) so.x_rounded = s.y_rounded = m->xb;
@@ -1276,7 +1285,6 @@ static int mix_sink(b2_engine* e, LayeredModel* m, LyLayer& L, const RaggedDev& 
     int rc;
     DenseArgs pj = {};
     pj.n_act = L.su_off; pj.n_act_end = L.su_off + Ko - od;       // the rows of a shared expert that rides along get their activation here
-    if (in == m->hn) pj.x_rounded = m->hn_rounded;
     m->rider = riders ? riders[0] : nullptr;
     if ((rc = dense(e, m, L.sk_proj, in, W, m->proj, Np, T, L.sk_bias, L.su_off >= 0 ? EPI_BIAS_PART_RELU2 : L.sk_bias ? EPI_BIAS : EPI_NONE, 1, &pj))) return rc;
     if (m->rider) { if ((rc = dense_run(e, m, *std::exchange(m->rider, nullptr), 1))) return rc; }
@@ -1431,7 +1439,6 @@ static int moe_prepare(b2_engine* e, LayeredModel* m, LyLayer& L, const RaggedDe
     up.groups = &j.g;
     up.p0 = (float)d.moe_limit; up.p1 = (float)d.moe_alpha;
     if (rounded) {                                 // the activations only feed the down maps: left rounded
-        if (in == m->hn) up.x_rounded = m->hn_rounded;
         up.y_rounded = m->moe_hb;
     }
     const int act = d.moe_expert == B2_EXPERT_CLAMPED ? EPI_GLU_CLAMP : d.moe_expert == B2_EXPERT_RELU2 ? EPI_BIAS_RELU2 : EPI_GLU_SILU;
@@ -1519,7 +1526,17 @@ static int run_layers(b2_engine* e, LayeredModel* m, const RaggedDev& r) {
         pending_moe = MoeJoinArgs{};
         return B2_OK;
     };
-    m->hn_rounded = nullptr;
+    m->hn_rounded = m->hn2_rounded = m->x_rounded = nullptr;
+    // post-sum blocks: the stream is left rounded beside itself for the products of the next sublayer
+    auto postsum = [&](const float* a, const float* wa, const float* b, const float* wb, const float* w) -> int {
+        StepProfiler sp(m, st, 5);
+        PostsumArgs p = {m->x, a, wa, b, wb, w, c.residual_scale, c.norm_eps, nullptr};
+        if (T > 8 && m->x_b && postsum_leaves_rounded(p, W)) p.x_rounded = m->x_b;
+        CK(postsum_norm_launch(p, W, T, st));
+        e->launches++;
+        m->x_rounded = p.x_rounded;
+        return B2_OK;
+    };
     m->rider = nullptr;
     if (c.block_style == B2_BLOCK_HYPER_RMS) {
         // The embedding sits in copy 0. A sublayer's output waits (in m->oL / m->oR / the mixture's rows) until the next boundary:
@@ -1586,7 +1603,9 @@ static int run_layers(b2_engine* e, LayeredModel* m, const RaggedDev& r) {
         auto norms = [&](ParallelJoinArgs& p, const LyLayer& N) {
             p.w1 = N.norm1; p.b1 = N.norm1_b; p.y1 = m->hn;
             if (!one_norm && N.d.n_ff > 0) { p.w2 = N.norm2; p.b2 = N.norm2_b; p.y2 = m->hn2; }
-            m->hn_rounded = nullptr;
+            m->hn_rounded = m->hn2_rounded = nullptr;
+            if (!one_norm && m->hn_b && N.d.mixer == B2_MIX_LATENT_ATTN && takes_rounded(m, N.la_proj, T)) { m->hn_rounded = p.y1_bf16 = m->hn_b; p.y1 = nullptr; }
+            if (p.y2 && m->hn2_b && N.d.ff_kind == B2_FF_GLU && takes_rounded(m, N.glu_gate_up, T)) { m->hn2_rounded = p.y2_bf16 = m->hn2_b; p.y2 = nullptr; }
             if (one_norm && m->hn_b && N.d.mixer == B2_MIX_SINK_ATTN && takes_rounded(m, N.sk_proj, T)) {
                 m->hn_rounded = p.y1_bf16 = m->hn_b;
                 const bool moe = N.d.n_ff > 0 && N.d.ff_kind == B2_FF_MOE;
@@ -1688,16 +1707,10 @@ static int run_layers(b2_engine* e, LayeredModel* m, const RaggedDev& r) {
             if ((rc = run_mixer(e, m, L, r, m->x))) return rc;
             {
                 const bool two = d.mixer == B2_MIX_WINDOW_SCAN;
-                StepProfiler sp(m, st, 5);
-                CK(postsum_norm_launch(m->x, m->oL, two ? L.left_w : nullptr, two ? m->oR : nullptr, two ? L.right_w : nullptr, L.norm1,
-                                       c.residual_scale, c.norm_eps, W, T, st));
-                e->launches++;
+                if ((rc = postsum(m->oL, two ? L.left_w : nullptr, two ? m->oR : nullptr, two ? L.right_w : nullptr, L.norm1))) return rc;
             }
             if (d.n_ff > 0) {
-                if ((rc = run_ff(e, m, L, r, m->x, m->oL))) return rc;
-                StepProfiler sp(m, st, 5);
-                CK(postsum_norm_launch(m->x, m->oL, nullptr, nullptr, nullptr, L.norm2, c.residual_scale, c.norm_eps, W, T, st));
-                e->launches++;
+                if ((rc = run_ff(e, m, L, r, m->x, m->oL)) || (rc = postsum(m->oL, nullptr, nullptr, nullptr, L.norm2))) return rc;
             }
         }
         if (m->trace)

@@ -106,8 +106,13 @@ cudaError_t gather_rows_launch(const float* x, int W, const int* rows, int n, fl
 // Post-sum layer norm: x[t] = LN(alpha * x[t] + y[t]) * w with
 //   y = a                      (b == nullptr)
 //   y = (rms(a) * wa + rms(b) * wb) / 2   (two branches, each RMS-normed over the width first)
-cudaError_t postsum_norm_launch(float* x, const float* a, const float* wa, const float* b, const float* wb, const float* w,
-                                float alpha, float eps, int W, int T, cudaStream_t s);
+struct PostsumArgs {
+    float* x; const float *a, *wa, *b, *wb, *w;
+    float alpha, eps;
+    __nv_bfloat16* x_rounded;      // the result once more, rounded (postsum_leaves_rounded), or null
+};
+bool postsum_leaves_rounded(const PostsumArgs& p, int W);
+cudaError_t postsum_norm_launch(const PostsumArgs& p, int W, int T, cudaStream_t s);
 // Pre-norm blocks: if (add) x[t] += mult * add[t]; if (y) y[t] = x[t] / sqrt(mean(x[t]^2) + eps) * (w_offset + w) * out_scale.
 // y may be x itself.
 cudaError_t resid_rms_norm_launch(float* x, const float* add, float mult, const float* w, float w_offset, float out_scale,
@@ -136,7 +141,9 @@ struct WindowAttnArgs {
     float* out;                // [T][H*d]
     float* split_scratch;      // few-token steps: partial (max, sum, output) per key range, [T][H][splits][d + 2]
     int split_capacity;        // floats in split_scratch
+    __nv_bfloat16* out_rounded = nullptr;      // the output goes here instead, rounded (window_attn_leaves_rounded)
 };
+bool window_attn_leaves_rounded(const WindowAttnArgs& a, int T);
 // norm + rotate q and k, store k (rotated) and v (= k as projected) into the pages
 cudaError_t window_attn_store_launch(const WindowAttnArgs& a, const RaggedDev& r, cudaStream_t s);
 // softmax attention of every step token over the visible cached keys of its sequence
@@ -154,6 +161,7 @@ struct ScanArgs {              // selective scan (Mamba)
     float* y;                  // [T][inner] gated output
     int inner;
     __nv_bfloat16* y_rounded = nullptr;      // the gated output goes here instead, rounded (scan_leaves_rounded)
+    __nv_bfloat16* xc_rounded = nullptr;     // xc once more, rounded, or null
 };
 bool scan_leaves_rounded(const ScanArgs& a);
 cudaError_t scan_conv_launch(const ScanArgs& a, const RaggedDev& r, cudaStream_t s);
@@ -322,7 +330,7 @@ struct ParallelJoinArgs {
     const float *w2, *b2; float* y2;
     float eps;
     float* x_copy; int ld_copy;
-    __nv_bfloat16* y1_bf16;        // the first norm's output rounded, for products that take it that way; y1 may then be null
+    __nv_bfloat16 *y1_bf16, *y2_bf16;      // the norms' outputs rounded, for products that take them that way; y1, y2 may then be null
 };
 cudaError_t parallel_join_launch(const ParallelJoinArgs& a, int W, int T, cudaStream_t s);
 

@@ -42,6 +42,17 @@ __device__ __forceinline__ float silu_f(float z) { return z / (1.f + expf(-z)); 
 __device__ __forceinline__ float softplus_f(float z) { return z > 0.f ? z + log1pf(expf(-z)) : log1pf(expf(z)); }
 __device__ __forceinline__ float log_sigmoid_f(float z) { return -softplus_f(-z); }
 
+// log(1 + exp(z)) and z / (1 + exp(-z)) without branches, so that they can run between other work; a unit or two in the last place.
+__device__ __forceinline__ float softplus_inline(float z) {
+    // log(1 + t), t = exp(-|z|) in [0, 1]: twice the inverse hyperbolic tangent of t / (2 + t) <= 1/3, as its power series
+    const float t = expf(-fabsf(z)), s = t * rcp_approx(2.f + t), x = s * s;
+    float p = 1.f / 15.f;
+    p = fmaf(p, x, 1.f / 13.f); p = fmaf(p, x, 1.f / 11.f); p = fmaf(p, x, 1.f / 9.f); p = fmaf(p, x, 1.f / 7.f); p = fmaf(p, x, 1.f / 5.f);
+    p = fmaf(p, x, 1.f / 3.f);
+    return fmaxf(z, 0.f) + 2.f * fmaf(p * x, s, s);
+}
+__device__ __forceinline__ float silu_inline(float z) { return over_one_plus_exp(z, -z); }
+
 // ---------------------------------------------------------------- embedding, gather
 constexpr int EMBED_COLS = 512;      // columns per CTA
 template <typename TW>
@@ -95,6 +106,11 @@ cudaError_t gather_rows_launch(const float* x, int W, const int* rows, int n, fl
     return launch_chain(gather_rows_kernel, dim3(n), dim3(128), 0, s, x, W, rows, y);
 }
 
+__device__ __forceinline__ void store_bf16x4(__nv_bfloat16* to, const float4& v) {
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(to) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+}
+
 // ---------------------------------------------------------------- norms
 // one CTA per token; the row lives in shared memory between the passes (mean, then squared deviations)
 __global__ void __launch_bounds__(256) postsum_norm_kernel(float* __restrict__ x, const float* __restrict__ a, const float* __restrict__ wa,
@@ -125,9 +141,78 @@ __global__ void __launch_bounds__(256) postsum_norm_kernel(float* __restrict__ x
     const float rstd = 1.f / sqrtf(block_sum(sq, red) / (float)W + eps);
     for (int i = threadIdx.x; i < W; i += blockDim.x) x[base + i] = (row[i] - mean) * rstd * w[i];
 }
-cudaError_t postsum_norm_launch(float* x, const float* a, const float* wa, const float* b, const float* wb, const float* w,
-                                float alpha, float eps, int W, int T, cudaStream_t s) {
-    return launch_chain(postsum_norm_kernel, dim3(T), dim3(256), (size_t)W * 4, s, x, a, wa, b, wb, w, alpha, eps, W);
+// The same for rows of at most 4096 entries on 16-byte boundaries: a thread keeps its entries (NV times four) in registers, all of them read at
+// once. Bound by memory: 134 MB for 2048 rows of 4096 with two branches, 52 us with
+// the row in shared memory and single reads, 39 here; with one branch 34 and 25.
+template <int NV>
+__global__ void __launch_bounds__(256) postsum_norm_vec_kernel(PostsumArgs p, int W) {
+    griddep_launch();
+    griddep_wait();
+    __shared__ float red[33];
+    const size_t base = (size_t)blockIdx.x * W;
+    auto get = [&](const float* from, int k) {
+        const int i = (k * 256 + threadIdx.x) * 4;
+        return i < W ? *reinterpret_cast<const float4*>(from + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    float4 v[NV], a[NV], b[NV];
+#pragma unroll
+    for (int k = 0; k < NV; k++) {
+        v[k] = get(p.x + base, k);
+        a[k] = p.a ? get(p.a + base, k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (p.b) b[k] = get(p.b + base, k);
+    }
+    auto square = [](const float4& u) { return u.x * u.x + u.y * u.y + u.z * u.z + u.w * u.w; };
+    if (p.b) {
+        float sa = 0.f, sb = 0.f;
+#pragma unroll
+        for (int k = 0; k < NV; k++) { sa += square(a[k]); sb += square(b[k]); }
+        sa = block_sum(sa, red); sb = block_sum(sb, red);
+        const float ra = 0.5f / sqrtf(sa / (float)W + p.eps), rb = 0.5f / sqrtf(sb / (float)W + p.eps);
+#pragma unroll
+        for (int k = 0; k < NV; k++) {
+            const float4 wa = get(p.wa, k), wb = get(p.wb, k);
+            a[k].x = a[k].x * ra * wa.x + b[k].x * rb * wb.x; a[k].y = a[k].y * ra * wa.y + b[k].y * rb * wb.y;
+            a[k].z = a[k].z * ra * wa.z + b[k].z * rb * wb.z; a[k].w = a[k].w * ra * wa.w + b[k].w * rb * wb.w;
+        }
+    }
+    float sum = 0.f;
+#pragma unroll
+    for (int k = 0; k < NV; k++) {
+        v[k].x = fmaf(p.alpha, v[k].x, a[k].x); v[k].y = fmaf(p.alpha, v[k].y, a[k].y);
+        v[k].z = fmaf(p.alpha, v[k].z, a[k].z); v[k].w = fmaf(p.alpha, v[k].w, a[k].w);
+        sum += (v[k].x + v[k].y) + (v[k].z + v[k].w);
+    }
+    const float mean = block_sum(sum, red) / (float)W;
+    float sq = 0.f;
+#pragma unroll
+    for (int k = 0; k < NV; k++) {
+        v[k].x -= mean; v[k].y -= mean; v[k].z -= mean; v[k].w -= mean;
+        if ((k * 256 + threadIdx.x) * 4 < W) sq += square(v[k]);
+    }
+    const float rstd = 1.f / sqrtf(block_sum(sq, red) / (float)W + p.eps);
+#pragma unroll
+    for (int k = 0; k < NV; k++) {
+        const int i = (k * 256 + threadIdx.x) * 4;
+        if (i >= W) break;
+        const float4 w = get(p.w, k), y = make_float4(v[k].x * rstd * w.x, v[k].y * rstd * w.y, v[k].z * rstd * w.z, v[k].w * rstd * w.w);
+        *reinterpret_cast<float4*>(p.x + base + i) = y;
+        if (p.x_rounded) store_bf16x4(p.x_rounded + base + i, y);
+    }
+}
+bool postsum_leaves_rounded(const PostsumArgs& p, int W) {
+    const float* const all[] = {p.x, p.a, p.wa, p.b, p.wb, p.w};
+    uintptr_t at = 0;
+    for (const float* q : all) at |= reinterpret_cast<uintptr_t>(q);
+    return W % 4 == 0 && W <= 4096 && (at & 15) == 0;
+}
+cudaError_t postsum_norm_launch(const PostsumArgs& p, int W, int T, cudaStream_t s) {
+    if (postsum_leaves_rounded(p, W)) {
+        if (W <= 1024) return launch_chain(postsum_norm_vec_kernel<1>, dim3(T), dim3(256), 0, s, p, W);
+        if (W <= 2048) return launch_chain(postsum_norm_vec_kernel<2>, dim3(T), dim3(256), 0, s, p, W);
+        return launch_chain(postsum_norm_vec_kernel<4>, dim3(T), dim3(256), 0, s, p, W);
+    }
+    if (p.x_rounded) return cudaErrorInvalidValue;
+    return launch_chain(postsum_norm_kernel, dim3(T), dim3(256), (size_t)W * 4, s, p.x, p.a, p.wa, p.b, p.wb, p.w, p.alpha, p.eps, W);
 }
 
 // pre-norm blocks: the pending branch output joins the 32-bit residual stream, and the next sublayer's input is made in the same pass
@@ -261,7 +346,7 @@ __global__ void __launch_bounds__(NT) parallel_join_kernel(ParallelJoinDev p, in
             const int i = i0 + u * NT;
             const bool in = i < W;
             w1[u] = in && a.w1 ? a.w1[i] : 0.f; b1[u] = in && a.w1 && a.b1 ? a.b1[i] : 0.f;
-            w2[u] = in && a.y2 ? a.w2[i] : 0.f; b2[u] = in && a.y2 && a.b2 ? a.b2[i] : 0.f;
+            w2[u] = in && a.w2 ? a.w2[i] : 0.f; b2[u] = in && a.w2 && a.b2 ? a.b2[i] : 0.f;
         }
 #pragma unroll
         for (int k = 0; k < JOIN_U; k++) {
@@ -273,7 +358,11 @@ __global__ void __launch_bounds__(NT) parallel_join_kernel(ParallelJoinDev p, in
                 if (a.y1) a.y1[base + i] = v;
                 if (a.y1_bf16) a.y1_bf16[base + i] = __float2bfloat16(v);
             }
-            if (a.y2) a.y2[base + i] = fmaf(u, w2[k], b2[k]);
+            if (a.w2) {
+                const float v = fmaf(u, w2[k], b2[k]);
+                if (a.y2) a.y2[base + i] = v;
+                if (a.y2_bf16) a.y2_bf16[base + i] = __float2bfloat16(v);
+            }
         }
     }
 }
@@ -339,8 +428,46 @@ __global__ void __launch_bounds__(256) window_attn_store_kernel(WindowAttnArgs a
         }
     }
 }
+// The same for head sizes up to 128 whose rows are whole 16-byte pieces: a lane has four neighbouring entries, read once (30 -> 22 us).
+__device__ __forceinline__ void cache_store4(void* pool, int f32, size_t i, const float4& v) {
+    if (f32) *reinterpret_cast<float4*>(reinterpret_cast<float*>(pool) + i) = v;
+    else store_bf16x4(reinterpret_cast<__nv_bfloat16*>(pool) + i, v);
+}
+__global__ void __launch_bounds__(256) window_attn_store_vec_kernel(WindowAttnArgs a, RaggedDev r) {
+    griddep_launch();
+    griddep_wait();
+    const int t = blockIdx.x, hs = blockIdx.y * 8 + (threadIdx.x >> 5), i = (threadIdx.x & 31) * 4;
+    if (hs >= a.H + a.G) return;
+    const bool is_q = hs < a.H, in = i < a.d;
+    const int head = is_q ? hs : hs - a.H, pos = r.tok_pos[t];
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 raw = in ? *reinterpret_cast<const float4*>(a.proj + (size_t)t * a.ldp + (is_q ? a.q_off : a.k_off) + head * a.d + i) : zero;
+    const float4 w = in ? *reinterpret_cast<const float4*>((is_q ? a.q_norm_w : a.k_norm_w) + i) : zero;
+    float cs[2] = {1.f, 1.f}, sn[2] = {0.f, 0.f};
+#pragma unroll
+    for (int p = 0; p < 2; p++)
+        if (in && i + 2 * p + 1 < a.rot.rot_dims) {          // pairs (2i, 2i + 1) inside the first rot_dims entries are rotated
+            const size_t at = (size_t)pos * (a.rot.rot_dims / 2) + i / 2 + p;
+            cs[p] = a.rot.cos[at]; sn[p] = a.rot.sin[at];
+        }
+    const float rinv = 1.f / sqrtf(warp_sum(raw.x * raw.x + raw.y * raw.y + raw.z * raw.z + raw.w * raw.w) / (float)a.d + a.eps);
+    if (!in) return;
+    const float4 u = make_float4(raw.x * rinv * w.x, raw.y * rinv * w.y, raw.z * rinv * w.z, raw.w * rinv * w.w);
+    const float4 y = make_float4(u.x * cs[0] - u.y * sn[0], u.y * cs[0] + u.x * sn[0], u.z * cs[1] - u.w * sn[1], u.w * cs[1] + u.z * sn[1]);
+    if (is_q) {
+        *reinterpret_cast<float4*>(a.q_rot + (size_t)t * a.H * a.d + (size_t)head * a.d + i) = y;
+        return;
+    }
+    const int page = a.block_tables[r.seg_slot[r.tok_seg[t]]][pos / a.block_tokens];
+    const size_t dst = (((size_t)page * a.G + head) * a.block_tokens + pos % a.block_tokens) * a.d + i;
+    cache_store4(a.k_pool, a.cache_f32, dst, y);
+    cache_store4(a.v_pool, a.cache_f32, dst, raw);
+}
 cudaError_t window_attn_store_launch(const WindowAttnArgs& a, const RaggedDev& r, cudaStream_t s) {
-    return launch_chain(window_attn_store_kernel, dim3(r.T, (a.H + a.G + 7) / 8), dim3(256), 0, s, a, r);
+    const uintptr_t at = reinterpret_cast<uintptr_t>(a.proj) | reinterpret_cast<uintptr_t>(a.q_norm_w) | reinterpret_cast<uintptr_t>(a.k_norm_w) |
+                         reinterpret_cast<uintptr_t>(a.q_rot) | reinterpret_cast<uintptr_t>(a.k_pool) | reinterpret_cast<uintptr_t>(a.v_pool);
+    const bool vec = a.d % 4 == 0 && a.d <= 128 && a.ldp % 4 == 0 && a.q_off % 4 == 0 && a.k_off % 4 == 0 && (at & 15) == 0;
+    return launch_chain(vec ? window_attn_store_vec_kernel : window_attn_store_kernel, dim3(r.T, (a.H + a.G + 7) / 8), dim3(256), 0, s, a, r);
 }
 
 // grid (T, H), 4 warps: warp w takes visible keys w, w + 4, ...; a lane holds entries lane, lane + 32, ... of the head
@@ -683,19 +810,28 @@ __global__ void __launch_bounds__(128) window_attn_mma_kernel(WindowAttnArgs a, 
         }
 }
 
-cudaError_t window_attn_launch(const WindowAttnArgs& a, const RaggedDev& r, cudaStream_t s) {
-    if (a.d > ATT_MAXE * 32) return cudaErrorInvalidValue;
+static bool window_attn_mma(const WindowAttnArgs& a, int T) {
     static const bool no_mma = getenv("B2_NO_ATTN_MMA") != nullptr;        // tuning aid: scalar attention for prompts too
-    if (!no_mma && !a.cache_f32 && r.T > 8 && a.d % 16 == 0 && a.d <= 128) {
+    return !no_mma && !a.cache_f32 && T > 8 && a.d % 16 == 0 && a.d <= 128;
+}
+static SoftmaxTcArgs window_softmax_args(const WindowAttnArgs& a) {
+    SoftmaxTcArgs x = {};
+    x.q = a.q_rot; x.k_pool = a.k_pool; x.v_pool = a.v_pool; x.pool_rows = a.pool_rows; x.block_tables = a.block_tables; x.block_tokens = a.block_tokens;
+    x.H = a.H; x.G = a.G; x.d = x.dv = a.d; x.window = a.window; x.keep_first = a.keep_first; x.scale = a.scale; x.ld_out = a.H * a.d;
+    x.out = a.out; x.out_bf16 = a.out_rounded;
+    return x;
+}
+bool window_attn_leaves_rounded(const WindowAttnArgs& a, int T) { return window_attn_mma(a, T) && softmax_takes_tc(window_softmax_args(a)); }
+cudaError_t window_attn_launch(const WindowAttnArgs& a, const RaggedDev& r, cudaStream_t s) {
+    if (a.d > ATT_MAXE * 32 || (a.out_rounded && !window_attn_leaves_rounded(a, r.T))) return cudaErrorInvalidValue;
+    if (window_attn_mma(a, r.T)) {
         static bool attr_done = false;
         if (!attr_done) {
             cudaFuncSetAttribute(window_attn_mma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 64 * (64 + 8) * 2);
             cudaFuncSetAttribute(window_attn_mma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 64 * (128 + 8) * 2);
             attr_done = true;
         }
-        SoftmaxTcArgs x = {};
-        x.q = a.q_rot; x.k_pool = a.k_pool; x.v_pool = a.v_pool; x.pool_rows = a.pool_rows; x.block_tables = a.block_tables; x.block_tokens = a.block_tokens;
-        x.H = a.H; x.G = a.G; x.d = x.dv = a.d; x.window = a.window; x.keep_first = a.keep_first; x.scale = a.scale; x.out = a.out; x.ld_out = a.H * a.d;
+        const SoftmaxTcArgs x = window_softmax_args(a);
         if (softmax_takes_tc(x)) return softmax_tc_launch(x, r, s);
         const size_t smem = (size_t)4 * 64 * (a.d + 8) * 2;
         if (a.d <= 64) return launch_chain(window_attn_mma_kernel<64>, dim3(r.n_tiles, a.H), dim3(128), smem, s, a, r);
@@ -733,12 +869,15 @@ __global__ void __launch_bounds__(256) scan_conv_kernel(ScanArgs a, RaggedDev r)
                                       : a.conv_state[((size_t)slot * a.inner + c) * hist + (hist + srci)];
             acc = fmaf(a.conv_w[(size_t)c * a.taps + j], v, acc);
         }
-        a.xc[(size_t)t * a.inner + c] = silu_f(acc);
+        const float y = silu_inline(acc);
+        a.xc[(size_t)t * a.inner + c] = y;
+        if (a.xc_rounded) a.xc_rounded[(size_t)t * a.inner + c] = __float2bfloat16(y);
     }
 }
 // The usual tap counts: a thread makes SCV_T consecutive tokens of one channel, whose inputs it reads once and all ahead of the first
-// use. (A thread per token and channel read every input TAPS times, each read behind the last store: 2048 tokens of
-// 8192 channels, 120 -> 65 us.)
+// use. Runs inside one sequence and past its first taps - 1 tokens, nearly all of them, look at no state and no segment. (2048 tokens of 8192
+// channels: 120 us with a thread per token and channel, 65 with runs that all looked for their state (117 instructions an output), 40 here,
+// with the copy that is left rounded for the next product.)
 constexpr int SCV_T = 8;
 template <int TAPS>
 __global__ void __launch_bounds__(256) scan_conv_taps_kernel(ScanArgs a, RaggedDev r) {
@@ -750,12 +889,32 @@ __global__ void __launch_bounds__(256) scan_conv_taps_kernel(ScanArgs a, RaggedD
     float w[TAPS], v[SCV_T + hist];
 #pragma unroll
     for (int j = 0; j < TAPS; j++) w[j] = a.conv_w[(size_t)c * TAPS + j];
+    const float* from = a.proj + (long)(t0 - hist) * a.ldp + a.x_off + c;
 #pragma unroll
-    for (int k = 0; k < SCV_T + hist; k++) {
+    for (int k = 0; k < SCV_T + hist; k++, from += a.ldp) {
         const int t = t0 + k - hist;
-        v[k] = t >= 0 && t < r.T ? a.proj[(size_t)t * a.ldp + a.x_off + c] : 0.f;
+        v[k] = t >= 0 && t < r.T ? *from : 0.f;
     }
     const float bias = a.conv_b[c];
+    float* xc = a.xc + (size_t)t0 * a.inner + c;
+    __nv_bfloat16* xb = a.xc_rounded ? a.xc_rounded + (size_t)t0 * a.inner + c : nullptr;
+    auto put = [&](float acc) {
+        const float y = silu_inline(acc);
+        *xc = y;
+        xc += a.inner;
+        if (xb) { *xb = __float2bfloat16(y); xb += a.inner; }
+    };
+    const int seg0 = r.tok_seg[t0];
+    if (t0 + SCV_T <= r.T && r.tok_seg[t0 + SCV_T - 1] == seg0 && t0 - r.seg_start[seg0] >= hist) {
+#pragma unroll
+        for (int k = 0; k < SCV_T; k++) {
+            float acc = bias;
+#pragma unroll
+            for (int j = 0; j < TAPS; j++) acc = fmaf(w[j], v[k + j], acc);
+            put(acc);
+        }
+        return;
+    }
 #pragma unroll
     for (int k = 0; k < SCV_T; k++) {
         const int t = t0 + k;
@@ -768,7 +927,7 @@ __global__ void __launch_bounds__(256) scan_conv_taps_kernel(ScanArgs a, RaggedD
             const float in = src >= 0 ? v[k + j] : a.conv_state[((size_t)r.seg_slot[seg] * a.inner + c) * hist + hist + src];
             acc = fmaf(w[j], in, acc);
         }
-        a.xc[(size_t)t * a.inner + c] = silu_f(acc);
+        put(acc);
     }
 }
 cudaError_t scan_conv_launch(const ScanArgs& a, const RaggedDev& r, cudaStream_t s) {
@@ -906,24 +1065,6 @@ __global__ void __launch_bounds__(SCAN_CH) scan_recurrence_chan_kernel(ScanArgs 
 // surrounds them, up to four warps a scheduler. The same on a B200: 995 us with a lane per state, 413 with four lanes, expf, and
 // softplus and gate in a phase of their own, 250 here.
 constexpr int SC_CH = 64, SC_TB = 16;
-// log(1 + exp(z)) and z / (1 + exp(-z)) without branches, so that they can run between other work; a unit or two in the last place.
-__device__ __forceinline__ float rcp_approx(float y) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
-    return r;
-}
-__device__ __forceinline__ float softplus_inline(float z) {
-    // log(1 + t), t = exp(-|z|) in [0, 1]: twice the inverse hyperbolic tangent of t / (2 + t) <= 1/3, as its power series
-    const float t = expf(-fabsf(z)), s = t * rcp_approx(2.f + t), x = s * s;
-    float p = 1.f / 15.f;
-    p = fmaf(p, x, 1.f / 13.f); p = fmaf(p, x, 1.f / 11.f); p = fmaf(p, x, 1.f / 9.f); p = fmaf(p, x, 1.f / 7.f); p = fmaf(p, x, 1.f / 5.f);
-    p = fmaf(p, x, 1.f / 3.f);
-    return fmaxf(z, 0.f) + 2.f * fmaf(p * x, s, s);
-}
-__device__ __forceinline__ float silu_inline(float z) {
-    const float y = 1.f + fminf(expf(-z), 1e37f), r = rcp_approx(y), v = z * r;
-    return fmaf(fmaf(-y, v, z), r, v);
-}
 template <int LANES, int SPL>
 __global__ void __launch_bounds__(SC_CH * LANES) scan_recurrence_lanes_kernel(ScanArgs a, RaggedDev r) {
     griddep_launch();
@@ -1321,10 +1462,8 @@ __global__ void __launch_bounds__(256) matrix_mem_out_kernel(MatrixMemArgs a, in
             if (e >= a.dv) break;
             const float4 y = make_float4(v[k].x * rinv * n[k].x * sigmoid_f(z[k].x), v[k].y * rinv * n[k].y * sigmoid_f(z[k].y),
                                          v[k].z * rinv * n[k].z * sigmoid_f(z[k].z), v[k].w * rinv * n[k].w * sigmoid_f(z[k].w));
-            if (a.out_rounded) {
-                const __nv_bfloat162 lo = __floats2bfloat162_rn(y.x, y.y), hi = __floats2bfloat162_rn(y.z, y.w);
-                *reinterpret_cast<uint2*>(a.out_rounded + base + e) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
-            } else *reinterpret_cast<float4*>(a.out + base + e) = y;
+            if (a.out_rounded) store_bf16x4(a.out_rounded + base + e, y);
+            else *reinterpret_cast<float4*>(a.out + base + e) = y;
         }
     } else {
         const float inv = inverse();

@@ -132,6 +132,19 @@ __device__ __forceinline__ float ex2_approx(float x) {
     return r;
 }
 
+__device__ __forceinline__ float rcp_approx(float y) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
+    return r;
+}
+// z / (1 + exp(w)) without a branch (a division has one): the approximate quotient, corrected once by its remainder; within two units of the last place
+__device__ __forceinline__ float over_one_plus_exp(float z, float w) {
+    float y = 1.f + expf(w);
+    y = y > 1e37f ? 1e37f : y;                     // (its reciprocal is still a normal number; NaN passes)
+    const float r = rcp_approx(y), v = z * r;
+    return y == 1.f ? z : fmaf(fmaf(-y, v, z), r, v);         // (an infinite z too)
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
