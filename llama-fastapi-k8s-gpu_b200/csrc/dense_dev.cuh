@@ -2,6 +2,7 @@
 #pragma once
 #include "kernels.h"
 #include "layered.h"
+#include "ptx.cuh"
 
 namespace b2 {
 
@@ -48,13 +49,16 @@ __device__ __forceinline__ bool dense_tile(const DenseDev& a, int rows_per_cta, 
 }
 __device__ __forceinline__ int x_row(const DenseDev& a, int t) { return (a.grouped && a.g.x_rows) ? a.g.x_rows[t] : t; }
 
-__device__ __forceinline__ float silu_act(float z) { return z / (1.f + expf(-z)); }
-__device__ __forceinline__ float gelu_tanh_act(float z) { return 0.5f * z * (1.f + tanhf(0.7978845608028654f * fmaf(0.044715f * z * z, z, z))); }
+// gates of the epilogues, without branches (see tc_store)
+__device__ __forceinline__ float silu_act(float z) { return over_one_plus_exp(z, -z); }
+__device__ __forceinline__ float sigmoid_act(float z) { return over_one_plus_exp(1.f, -z); }
+// z (1 + tanh u) / 2 = z / (1 + exp(-2u)), which does not cancel where tanh is near -1
+__device__ __forceinline__ float gelu_tanh_act(float z) { return over_one_plus_exp(z, -1.5957691216057308f * fmaf(0.044715f * z * z, z, z)); }
 __device__ __forceinline__ float epi_value(const DenseDev& a, const float* aux, int t, int n, float v) {
     const int epi = a.epi;
     if (epi == EPI_BIAS || epi == EPI_BIAS_RELU2 || epi == EPI_BIAS_PART_RELU2) { if (a.bias) v += a.bias[n]; }
     if (epi == EPI_BIAS_RELU2 || (epi == EPI_BIAS_PART_RELU2 && n >= a.n_act && n < a.n_act_end)) { v = fmaxf(v, 0.f); v = v * v; }
-    if (epi == EPI_MUL_SIGMOID) v *= 1.f / (1.f + expf(-aux[(size_t)t * a.ldaux + n * a.aux_ns]));
+    if (epi == EPI_MUL_SIGMOID) v *= sigmoid_act(aux[(size_t)t * a.ldaux + n * a.aux_ns]);
     if (epi == EPI_PIECEWISE) v = v > 0.f ? fmaf(a.p0 * v, v, 0.5f * v) : fmaf(a.p1, expm1f(v) - v, 0.5f * v);
     return v * a.scale;
 }

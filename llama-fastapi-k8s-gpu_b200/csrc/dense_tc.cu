@@ -53,7 +53,7 @@ __device__ __forceinline__ void tc_store_rows(const DenseDev& a, float* y, __nv_
             v[j] = acc[j];
             if ((EPI == EPI_BIAS || EPI == EPI_BIAS_RELU2 || EPI == EPI_BIAS_PART_RELU2) && a.bias) v[j] += a.bias[c];
             if (EPI == EPI_BIAS_RELU2 || (EPI == EPI_BIAS_PART_RELU2 && c >= a.n_act && c < a.n_act_end)) { v[j] = fmaxf(v[j], 0.f); v[j] = v[j] * v[j]; }
-            if (EPI == EPI_MUL_SIGMOID) v[j] *= 1.f / (1.f + expf(-aux[(size_t)t * a.ldaux + c * a.aux_ns]));
+            if (EPI == EPI_MUL_SIGMOID) v[j] *= sigmoid_act(aux[(size_t)t * a.ldaux + c * a.aux_ns]);
             if (EPI == EPI_PIECEWISE) v[j] = v[j] > 0.f ? fmaf(a.p0 * v[j], v[j], 0.5f * v[j]) : fmaf(a.p1, expm1f(v[j]) - v[j], 0.5f * v[j]);
             v[j] *= a.scale;
         }
