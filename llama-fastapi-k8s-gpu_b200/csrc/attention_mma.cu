@@ -6,11 +6,13 @@
 // Grid (n_splits, n_kv_heads, sequences), 4 warps. The MMA's 16 rows are the G <= 8 query heads of one KV head
 // (rows G..15 are zero padding): one m16n8k16 covers 16 heads x 8 positions x 16 dims, ~12x fewer instructions per
 // K/V byte than the scalar kernel. K/V tiles of 64 positions go global -> shared with cp.async (16 B per request,
-// double buffered) into rows padded by 16 B, so the fragment loads (LDS.32 for K, ldmatrix.trans for V) are
-// conflict-free; pages are looked up per position, so any kv_block_tokens works. Inside a tile warp w owns
+// AM_STAGES buffers: two CTAs of three fit an SM, and two tiles of each are in flight while one is used) into rows padded by 16 B, so the
+// fragment loads (ldmatrix, four 8 x 8 matrices each) are conflict-free; pages are looked up per position, so any kv_block_tokens works. Inside a tile warp w owns
 // positions 16w..16w+15 end to end (scores, online softmax, P.V) -- no block barrier between the phases -- and the
 // four per-warp (max, sum, output) triples are merged once at the end; splits are merged by the last CTA of the
 // KV head (atomic ticket), in the log2 domain.
+// Bound by the latency of a CTA's tiles, one after another (32 sequences of 500 positions, 8 KV heads of 128, a CTA each: 23.5 us with two buffers and
+// single fragment reads, 17.3 here; the bytes would take 10).
 // q is rounded to f16 for the MMA (as llama.cpp's own flash-attention kernels do); accumulation is f32.
 #include "kernels.h"
 #include "ptx.cuh"
@@ -21,14 +23,18 @@ namespace b2 {
 
 constexpr int AM_THREADS = 128;
 constexpr int AM_TT = 64;           // positions per tile (16 per warp)
+constexpr int AM_STAGES = 3;
 
 __device__ __forceinline__ void am_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void am_ldmatrix_x2_trans(uint32_t& r0, uint32_t& r1, const void* p) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(smem_u32(p)));
+__device__ __forceinline__ void am_ldmatrix_x4(uint32_t (&r)[4], const void* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)));
+}
+__device__ __forceinline__ void am_ldmatrix_x4_trans(uint32_t (&r)[4], const void* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)));
 }
 __device__ __forceinline__ uint32_t am_pack(float a, float b) {
     __half2 h = __floats2half2_rn(a, b);
@@ -51,8 +57,8 @@ __global__ void __launch_bounds__(AM_THREADS) attn_decode_mma_kernel(const AttnP
                                                                      float scale_log2) {
     constexpr int LD = HD + 8;                                  // padded row (halves)
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    __half* ks = reinterpret_cast<__half*>(smem_raw);           // [2][AM_TT][LD]
-    __half* vs = ks + 2 * AM_TT * LD;                           // [2][AM_TT][LD]
+    __half* ks = reinterpret_cast<__half*>(smem_raw);           // [AM_STAGES][AM_TT][LD]
+    __half* vs = ks + AM_STAGES * AM_TT * LD;                   // [AM_STAGES][AM_TT][LD]
     __shared__ unsigned int s_ticket;
     griddep_launch();
     griddep_wait();                                             // q, this step's K/V and the slot registers come from earlier kernels
@@ -93,29 +99,38 @@ __global__ void __launch_bounds__(AM_THREADS) attn_decode_mma_kernel(const AttnP
     for (int i = 0; i < HD / 8; i++) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
     float m_run = -INFINITY, l_run = 0.f;                        // row g of this warp's positions (l: this thread's share)
 
-    auto issue = [&](int ti) {                                   // all threads: tile ti -> buffer ti & 1
-        const int st = ti & 1, t0 = q0 + ti * AM_TT;
-        __half* kd = ks + st * AM_TT * LD;
-        __half* vd = vs + st * AM_TT * LD;
-        constexpr int CPR = HD / 8;                              // 16-byte chunks per row
-        for (int i = tid; i < AM_TT * CPR; i += AM_THREADS) {
-            const int j = i / CPR, c = i % CPR, pos = t0 + j;
-            if (pos < q1) {
-                const size_t off = (((size_t)p.block_table[pos / bt] * p.n_kv + h) * bt + pos % bt) * HD + c * 8;
-                am_cp16(kd + j * LD + c * 8, p.k_cache + off);
-                am_cp16(vd + j * LD + c * 8, p.v_cache + off);
-            } else {                                             // 0 * garbage must stay 0 in P.V
-                *reinterpret_cast<uint4*>(kd + j * LD + c * 8) = make_uint4(0, 0, 0, 0);
-                *reinterpret_cast<uint4*>(vd + j * LD + c * 8) = make_uint4(0, 0, 0, 0);
+    // all threads: tile ti -> buffer ti % AM_STAGES (a group of copies per call, empty past the last tile). A thread copies one 16-byte piece of every eighth
+    // (sixteenth) row; a page is looked up once a row.
+    constexpr int CPR = HD / 8, RPP = AM_THREADS / CPR;          // pieces of a row, rows of a pass
+    const int c8 = tid % CPR * 8;
+    auto issue = [&](int ti) {
+        const int st = ti % AM_STAGES, t0 = q0 + ti * AM_TT;
+        __half *kd = ks + st * AM_TT * LD + c8, *vd = vs + st * AM_TT * LD + c8;
+        if (ti < ntile) {
+            int page[AM_TT / RPP];
+#pragma unroll
+            for (int m = 0; m < AM_TT / RPP; m++) page[m] = p.block_table[min(t0 + tid / CPR + m * RPP, q1 - 1) / bt];
+#pragma unroll
+            for (int m = 0; m < AM_TT / RPP; m++) {
+                const int j = tid / CPR + m * RPP, pos = t0 + j;
+                if (pos < q1) {
+                    const size_t off = (((size_t)page[m] * p.n_kv + h) * bt + pos % bt) * HD + c8;
+                    am_cp16(kd + j * LD, p.k_cache + off);
+                    am_cp16(vd + j * LD, p.v_cache + off);
+                } else {                                         // 0 * garbage must stay 0 in P.V
+                    *reinterpret_cast<uint4*>(kd + j * LD) = make_uint4(0, 0, 0, 0);
+                    *reinterpret_cast<uint4*>(vd + j * LD) = make_uint4(0, 0, 0, 0);
+                }
             }
         }
         am_commit();
     };
-    if (ntile > 0) issue(0);
+    for (int i = 0; i < AM_STAGES - 1; i++) issue(i);
     for (int ti = 0; ti < ntile; ti++) {
-        if (ti + 1 < ntile) { issue(ti + 1); am_wait<1>(); } else { am_wait<0>(); }
-        __syncthreads();                                         // tile ti is in shared memory for every warp
-        const int st = ti & 1, w0 = q0 + ti * AM_TT + 16 * warp; // first position of this warp's slice
+        am_wait<AM_STAGES - 2>();
+        __syncthreads();                                         // tile ti is in shared memory for every warp, and every warp is done with the one before
+        issue(ti + AM_STAGES - 1);                               // into that one's buffer
+        const int st = ti % AM_STAGES, w0 = q0 + ti * AM_TT + 16 * warp; // first position of this warp's slice
         if (w0 < q1) {
             const __half* kb = ks + (st * AM_TT + 16 * warp) * LD;
             const __half* vb = vs + (st * AM_TT + 16 * warp) * LD;
@@ -123,11 +138,14 @@ __global__ void __launch_bounds__(AM_THREADS) attn_decode_mma_kernel(const AttnP
 #pragma unroll
             for (int nt = 0; nt < 2; nt++) {
                 sc[nt][0] = sc[nt][1] = sc[nt][2] = sc[nt][3] = 0.f;
-                const __half* kr = kb + (nt * 8 + g) * LD + 2 * tq;
+                const __half* kr = kb + (nt * 8 + (lane & 7)) * LD + (lane >> 3) * 8;
 #pragma unroll
-                for (int kk = 0; kk < HD / 16; kk++)
-                    am_mma(sc[nt], qa[kk], *reinterpret_cast<const uint32_t*>(kr + kk * 16),
-                           *reinterpret_cast<const uint32_t*>(kr + kk * 16 + 8));
+                for (int kk = 0; kk < HD / 16; kk += 2) {
+                    uint32_t b4[4];                              // dims kk * 16 .. + 31 of eight positions
+                    am_ldmatrix_x4(b4, kr + kk * 16);
+                    am_mma(sc[nt], qa[kk], b4[0], b4[1]);
+                    am_mma(sc[nt], qa[kk + 1], b4[2], b4[3]);
+                }
             }
             // ---- mask + online softmax of row g (log2 domain); columns 2tq, 2tq+1 of each 8-position group
             float mx = m_run;
@@ -147,15 +165,17 @@ __global__ void __launch_bounds__(AM_THREADS) attn_decode_mma_kernel(const AttnP
             l_run = l_run * f + (e0 + e1) + (e2 + e3);
             pa[0] = am_pack(e0, e1); pa[2] = am_pack(e2, e3); pa[1] = 0u; pa[3] = 0u;
 #pragma unroll
-            for (int nt = 0; nt < HD / 8; nt++) {
-                o[nt][0] *= f; o[nt][1] *= f;
-                uint32_t b0, b1;
-                am_ldmatrix_x2_trans(b0, b1, vb + (lane & 15) * LD + nt * 8);
-                am_mma(o[nt], pa, b0, b1);
+            for (int nt = 0; nt < HD / 8; nt += 2) {
+                o[nt][0] *= f; o[nt][1] *= f; o[nt + 1][0] *= f; o[nt + 1][1] *= f;
+                uint32_t b4[4];                                  // 16 positions x 16 dims, transposed on load
+                am_ldmatrix_x4_trans(b4, vb + (lane & 15) * LD + nt * 8 + (lane >> 4) * 8);
+                am_mma(o[nt], pa, b4[0], b4[1]);
+                am_mma(o[nt + 1], pa, b4[2], b4[3]);
             }
         }
-        __syncthreads();                                         // everyone is done with buffer st before it is refilled
     }
+    am_wait<0>();
+    __syncthreads();                                             // everyone is done with the buffers
     // ---- merge the four warps (their position slices are disjoint): (m, l, o) per head row, in the tile buffers
     l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
     l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
@@ -235,7 +255,7 @@ __global__ void __launch_bounds__(AM_THREADS) attn_decode_mma_kernel(const AttnP
     if (tid == 0) p.counters[h] = 0;                             // ready for the next launch
 }
 
-static size_t am_smem_bytes(int hd) { return (size_t)2 * 2 * AM_TT * (hd + 8) * 2; }
+static size_t am_smem_bytes(int hd) { return (size_t)AM_STAGES * 2 * AM_TT * (hd + 8) * 2; }
 
 cudaError_t attn_mma_init() {
     cudaError_t e = cudaFuncSetAttribute(attn_decode_mma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)am_smem_bytes(64));
