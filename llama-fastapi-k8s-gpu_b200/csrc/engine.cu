@@ -114,6 +114,7 @@ static int engine_create_impl(b2_engine* e, const b2_config* c) {
     CK(cudaEventCreate(&e->ev0));
     CK(cudaEventCreate(&e->ev1));
     CK(cudaMallocHost(&e->pinned, sizeof(int32_t) * (size_t)(c->max_seqs + c->n_ctx + 16)));
+    CK(cudaMallocHost(&e->slot_token, sizeof(int32_t) * (size_t)c->max_seqs));
     // KV pool: [layer][block][kv_head][token][dim] f16
     e->layer_kv_elems = (size_t)c->kv_num_blocks * c->n_head_kv * c->kv_block_tokens * c->head_dim;
     size_t kvb = e->layer_kv_elems * c->n_layer * sizeof(__half);
@@ -206,8 +207,9 @@ extern "C" int b2_engine_destroy(b2_engine* e) {
     cudaFree(e->k_pool); cudaFree(e->v_pool); cudaFree(e->rope_freq);
     cudaFree(e->attn_scratch); cudaFree(e->attn_counters);
     cudaFree(e->pf_x); cudaFree(e->pf_part); cudaFree(e->pf_xn); cudaFree(e->pf_qh); cudaFree(e->pf_att); cudaFree(e->pf_h);
-    cudaFree(e->slot_tab); cudaFree(e->bd_q); cudaFree(e->bd_att); cudaFree(e->bd_scratch); cudaFree(e->bd_counters); cudaFree(e->bd_out);
+    cudaFree(e->slot_tab); cudaFree(e->bd_q); cudaFree(e->bd_att); cudaFree(e->bd_scratch); cudaFree(e->bd_counters);
     if (e->pinned) cudaFreeHost(e->pinned);
+    if (e->slot_token) cudaFreeHost(e->slot_token);
     if (e->ev0) cudaEventDestroy(e->ev0);
     if (e->ev1) cudaEventDestroy(e->ev1);
     if (e->stream) cudaStreamDestroy(e->stream);
@@ -552,7 +554,7 @@ static int forward_launches(b2_engine* e, Slot& s, bool with_head, bool with_sam
     if (!kt) e->tl_n = tl_k;
     if (with_sample) {
         tick(7, &ye);
-        CK(sample_launch(s.logits, c.n_vocab, s.sp, s.sst, s.uniforms, s.ints + 3, s.ints + 2, tok, pos, s.ring, c.n_ctx + 1, st, pdl));
+        CK(sample_launch(s.logits, c.n_vocab, s.sp, s.sst, s.uniforms, s.ints + 3, s.ints + 2, tok, pos, s.ring, c.n_ctx + 1, st, pdl, e->slot_token + (&s - e->slots.data())));
         tock(ye);
         e->launches++;
     }
@@ -797,14 +799,13 @@ extern "C" int b2_prefill(b2_engine* e, int slot, const int32_t* tokens, int n) 
 __global__ void set_ints_kernel(int* ints, int tok, int pos) { if (tok >= 0) ints[0] = tok; ints[1] = pos; }
 
 // enqueue: sample from the slot's logit buffer (the token at position n_past - 1 was the last one evaluated); the token
-// lands in e->pinned[0] once the stream has been synchronised
+// is in e->slot_token once the stream has been synchronised
 static int sample_enqueue(b2_engine* e, Slot& s) {
     // sampler bumps pos: make it point at the last evaluated token first
     set_ints_kernel<<<1, 1, 0, e->stream>>>(s.ints, -1, s.n_past - 1);
     CK(sample_launch(s.logits, e->cfg.n_vocab, s.sp, s.sst, s.uniforms, s.ints + 3, s.ints + 2, s.ints + 0,
-                     s.ints + 1, s.ring, e->cfg.n_ctx + 1, e->stream, false));
+                     s.ints + 1, s.ring, e->cfg.n_ctx + 1, e->stream, false, e->slot_token + (&s - e->slots.data())));
     e->launches += 2;
-    CK(cudaMemcpyAsync(e->pinned, s.ints + 2, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
     s.n_sampled += 1;
     return B2_OK;
 }
@@ -816,7 +817,7 @@ extern "C" int b2_sample(b2_engine* e, int slot, int32_t* out) {
     CK(cudaSetDevice(e->cfg.device));
     if ((rc = sample_enqueue(e, s))) return rc;
     CK(cudaStreamSynchronize(e->stream));
-    if (out) *out = e->pinned[0];
+    if (out) *out = e->slot_token[slot];
     return B2_OK;
 }
 
@@ -830,7 +831,6 @@ static int ensure_batch_workspace(b2_engine* e) {
     CK(cudaMalloc(&e->bd_scratch, BATCH_MAX * attn_scratch_floats(c.n_head, c.n_head_kv, c.head_dim, e->n_splits) * 4));
     CK(cudaMalloc(&e->bd_counters, sizeof(unsigned) * BATCH_MAX * c.n_head_kv));
     CK(cudaMemsetAsync(e->bd_counters, 0, sizeof(unsigned) * BATCH_MAX * c.n_head_kv, e->stream));
-    CK(cudaMalloc(&e->bd_out, sizeof(int) * BATCH_MAX));
     return B2_OK;
 }
 
@@ -838,7 +838,7 @@ static int ensure_batch_workspace(b2_engine* e) {
 // tensor-core GEMM; attention and sampling run one CTA group per sequence from the per-slot device tables.
 // Enqueued kernel by kernel. Captured per list of slots, 8 steps of 32 sequences (4 layers of 4096) took 6580 us instead of 6750; but the list
 // changes whenever a chat starts or ends, and lists that live for three steps cost 5150 us instead of 4740 (16 layers: 16600 and 15600).
-static int batch_step(b2_engine* e, const BatchIdx& b) {
+static int batch_step(b2_engine* e, const BatchIdx& b, int32_t* tokens_out) {
     ChainPdl chain(e->chain_pdl && e->use_pdl);
     const b2_config& c = e->cfg;
     cudaStream_t st = e->stream;
@@ -895,7 +895,7 @@ static int batch_step(b2_engine* e, const BatchIdx& b) {
         }
         CK(gemm_launch(it->second, st));
     }
-    CK(sample_batch_launch(e->pf_part, c.n_vocab, c.n_vocab, e->slot_tab, b, c.n_ctx + 1, e->bd_out, st));
+    CK(sample_batch_launch(e->pf_part, c.n_vocab, c.n_vocab, e->slot_tab, b, c.n_ctx + 1, tokens_out, st));
     e->launches += 3;
     return B2_OK;
 }
@@ -921,10 +921,9 @@ extern "C" int b2_decode(b2_engine* e, const int32_t* slots, int n, int32_t* out
             b.n = n - i0 < BATCH_MAX ? n - i0 : BATCH_MAX;
             for (int i = 0; i < b.n; i++) b.slot[i] = slots[i0 + i];
             if ((size_t)b.n * e->cfg.n_vocab > e->pf_part_floats) return fail(B2_ERR_UNSUPPORTED, "vocabulary too large for the batch workspace");
-            if ((rc = batch_step(e, b))) return rc;
+            if ((rc = batch_step(e, b, e->pinned + i0))) return rc;
             // logits of this step stay in the batch output until the next GEMM call reuses the buffer
             for (int i = 0; i < b.n; i++) e->slots[b.slot[i]].logits_view = e->pf_part + (size_t)i * e->cfg.n_vocab;
-            CK(cudaMemcpyAsync(e->pinned + i0, e->bd_out, sizeof(int) * b.n, cudaMemcpyDeviceToHost, e->stream));
         }
         for (int i = 0; i < n; i++) { Slot& s = e->slots[slots[i]]; s.n_past += 1; s.n_sampled += 1; }
     } else {
@@ -932,14 +931,13 @@ extern "C" int b2_decode(b2_engine* e, const int32_t* slots, int n, int32_t* out
             Slot& s = e->slots[slots[i]];
             int rc = run_step(e, s, GK_DECODE);
             if (rc) return rc;
-            CK(cudaMemcpyAsync(e->pinned + i, s.ints + 2, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
             s.n_past += 1;
             s.n_sampled += 1;
         }
     }
     CK(cudaStreamSynchronize(e->stream));
     { int rc2 = b2_check_kernel_error(); if (rc2) return rc2; }
-    if (out) for (int i = 0; i < n; i++) out[i] = e->pinned[i];
+    if (out) for (int i = 0; i < n; i++) out[i] = batched ? e->pinned[i] : e->slot_token[slots[i]];
     return B2_OK;
 }
 

@@ -69,7 +69,8 @@ struct b2_engine {
     unsigned* attn_counters = nullptr;
     int n_splits = 1, max_blocks = 0, n_ctas = 148;
     std::vector<Slot> slots;
-    int32_t* pinned = nullptr;
+    int32_t* pinned = nullptr;     // host memory that kernels write too: sampled tokens arrive here without a copy of their own
+    int32_t* slot_token = nullptr; // the same, one entry per slot: written by the slot's (captured) sampler launches
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int64_t launches = 0, weight_bytes = 0, kv_bytes = 0;
     bool use_graph = true, use_pdl = true, act2 = true, finalized = false, chain_pdl = true;
@@ -94,7 +95,6 @@ struct b2_engine {
     SlotDev* slot_tab = nullptr;   // device table, one entry per slot
     float *bd_q = nullptr, *bd_att = nullptr, *bd_scratch = nullptr;
     unsigned* bd_counters = nullptr;
-    int* bd_out = nullptr;
     int attn_mma = -1;             // tensor-core flash-decode: -1 = batched steps only; 0 never; 1 always
     int batch_min = 3;             // fewer sequences than this step one after another through the mat-vec path (measured: 3 slots 4.1 vs 6.3 ms)
     bool gemm_ok = false;          // every layer matrix is a block format the GEMM reads

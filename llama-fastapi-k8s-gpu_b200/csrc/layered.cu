@@ -99,7 +99,6 @@ struct LayeredModel {
     int** block_tables = nullptr;      // device [max_seqs] -> page table
     SlotDev* slot_tab = nullptr;       // device [max_seqs]: what the sampler needs of a slot
     float** slot_logits = nullptr;     // device [max_seqs] -> the slot's logit buffer
-    int* sampled = nullptr;            // device [B2_STEP_MAX_ENTRIES]: tokens sampled in a step, by entry
     // step workspace (max_step_tokens rows)
     float *xs = nullptr, *hc = nullptr, *cross = nullptr;     // copies of the stream [S][max_step_tokens][W]; convolved sublayer input; per-(query head, value head) attention sums
     float *x = nullptr, *proj = nullptr, *buf[4] = {}, *oL = nullptr, *oR = nullptr, *hn = nullptr, *hn2 = nullptr, *ff = nullptr, *rows = nullptr, *logits = nullptr;
@@ -756,8 +755,7 @@ int layered_finalize(b2_engine* e) {
             dev[i] = SlotDev{sl.ints, sl.block_table, sl.ring, sl.sst, sl.sp, sl.uniforms};
             lg[i] = sl.logits;
         }
-        if ((rc = dev_alloc(m, (void**)&m->slot_tab, sizeof(SlotDev) * S)) || (rc = dev_alloc(m, (void**)&m->slot_logits, sizeof(float*) * S)) ||
-            (rc = dev_alloc(m, (void**)&m->sampled, sizeof(int) * B2_STEP_MAX_ENTRIES))) return rc;
+        if ((rc = dev_alloc(m, (void**)&m->slot_tab, sizeof(SlotDev) * S)) || (rc = dev_alloc(m, (void**)&m->slot_logits, sizeof(float*) * S))) return rc;
         CK(cudaMemcpy(m->slot_tab, dev.data(), sizeof(SlotDev) * S, cudaMemcpyHostToDevice));
         CK(cudaMemcpy(m->slot_logits, lg.data(), sizeof(float*) * S, cudaMemcpyHostToDevice));
     }
@@ -951,6 +949,7 @@ extern "C" int b2_engine_create_layered(const b2_layered_config* c, const b2_lay
         CK(cudaEventCreate(&e->ev0));
         CK(cudaEventCreate(&e->ev1));
         CK(cudaMallocHost(&e->pinned, sizeof(int32_t) * (size_t)(c->max_seqs + B2_STEP_MAX_ENTRIES + 16)));
+        CK(cudaMallocHost(&e->slot_token, sizeof(int32_t) * (size_t)c->max_seqs));
         e->max_blocks = (c->n_ctx + c->kv_block_tokens - 1) / c->kv_block_tokens;
         e->slots.resize(c->max_seqs);
         for (auto& s : e->slots) {
@@ -1816,15 +1815,13 @@ extern "C" int b2_step(b2_engine* e, int n_entries, const int32_t* slots, const 
         for (int i = 0; i < n; i++)
             if (samp_row[i] >= r0 && samp_row[i] < r0 + nr) { sr.entry[sr.n] = i; sr.row[sr.n++] = samp_row[i] - r0; }
         if (sr.n > 0) {
-            CK(sample_rows_launch(m->logits, V, m->slot_tab, m->slot_logits, sr, r.seg_slot, r.seg_pos0, r.seg_len, c.n_ctx + 1, m->sampled, st));
-            CK(cudaMemcpyAsync(e->pinned, m->sampled, sizeof(int) * n, cudaMemcpyDeviceToHost, st));
+            CK(sample_rows_launch(m->logits, V, m->slot_tab, m->slot_logits, sr, r.seg_slot, r.seg_pos0, r.seg_len, c.n_ctx + 1, e->pinned, st));
             e->launches++;
         }
         return B2_OK;
     };
     // everything the step enqueues up to the logits, for steps whose rows fit one head chunk
     auto forward_once = [&]() -> int {
-        CK(cudaMemcpyAsync(m->meta, h, n_meta * 4, cudaMemcpyHostToDevice, st));
         int rc2 = run_layers(e, m, r);
         if (rc2) return rc2;
         return n_rows > 0 ? head_chunk(0, n_rows) : B2_OK;
@@ -1832,6 +1829,8 @@ extern "C" int b2_step(b2_engine* e, int n_entries, const int32_t* slots, const 
     // Small steps that repeat (the same slots decoding token after token) are replayed as a CUDA graph: the batch description
     // is read from device memory, so nothing in the launches changes from one such step to the next. A shape is captured the
     // second time it is seen.
+    // (The description goes ahead of the graph: as its first node, the copy kept the kernels behind it waiting for a while.)
+    CK(cudaMemcpyAsync(m->meta, h, n_meta * 4, cudaMemcpyHostToDevice, st));
     bool done = false;
     if (m->graphs_on && !m->trace && !m->profile && T <= 64 && n_rows <= LOGIT_ROWS) {
         std::string key;
@@ -1870,10 +1869,7 @@ extern "C" int b2_step(b2_engine* e, int n_entries, const int32_t* slots, const 
     if (!done) {
         if (n_rows <= LOGIT_ROWS) {
             if ((rc = forward_once())) return rc;
-        } else {
-            CK(cudaMemcpyAsync(m->meta, h, n_meta * 4, cudaMemcpyHostToDevice, st));
-            if ((rc = run_layers(e, m, r))) return rc;
-        }
+        } else if ((rc = run_layers(e, m, r))) return rc;
     }
     m->last_T = T;
     for (int i = 0; i < n; i++) if (samp_row[i] >= 0) e->slots[slots[i]].logits_view = e->slots[slots[i]].logits;
