@@ -628,6 +628,42 @@ extern "C" int b2_seq_set_blocks(b2_engine* e, int slot, const int32_t* blocks, 
     return B2_OK;
 }
 
+// What a sequence's start or rewind changes of its slot, by value in one launch (as copies from pageable memory, and a clearing of every layer's state of its
+// own, each cost 3 us of the caller: 20 us ahead of a prompt, 500 us for 32 sequences that start).
+struct SeqUpdate {
+    SamplerState history;
+    SampleParams params;
+    double uniform;
+    int ints[8], n_ints;
+    bool start, has_uniform;   // start: parameters and recurrent state too
+};
+constexpr int SEQ_RESET_CTAS = 32;      // per region
+__global__ void __launch_bounds__(256) seq_update_kernel(const SeqUpdate v, SamplerState* sst, SampleParams* sp, int* ints, double* uniforms,
+                                                         const ResetRegion* regions, int slot) {
+    const int t = threadIdx.x;
+    if (blockIdx.x > 0) {
+        const ResetRegion g = regions[(blockIdx.x - 1) / SEQ_RESET_CTAS];
+        float* base = g.base + (size_t)slot * g.floats;
+        for (size_t i = (blockIdx.x - 1) % SEQ_RESET_CTAS * 256 + t; i < g.floats; i += SEQ_RESET_CTAS * 256) base[i] = 0.f;
+        return;
+    }
+    if (t < HISTORY_LEN) sst->history[t] = v.history.history[t];
+    if (t < v.n_ints) ints[t] = v.ints[t];
+    if (t == 0) {
+        sst->n_hist = v.history.n_hist;
+        if (v.start) *sp = v.params;
+        if (v.has_uniform) uniforms[0] = v.uniform;
+    }
+}
+static int seq_update(b2_engine* e, int slot, const SeqUpdate& u) {
+    Slot& s = e->slots[slot];
+    const int ctas = 1 + (u.start ? e->n_resets * SEQ_RESET_CTAS : 0);
+    seq_update_kernel<<<ctas, 256, 0, e->stream>>>(u, s.sst, s.sp, s.ints, s.uniforms, e->resets, slot);
+    CK(cudaGetLastError());
+    e->launches++;
+    return B2_OK;
+}
+
 extern "C" int b2_seq_begin(b2_engine* e, int slot, int n_past, const int32_t* hist, int n_hist,
                             const b2_sampling* sp, const double* uni, int n_uni) {
     int rc = check_slot(e, slot); if (rc) return rc;
@@ -642,22 +678,23 @@ extern "C" int b2_seq_begin(b2_engine* e, int slot, int n_past, const int32_t* h
     Slot& s = e->slots[slot];
     if (e->layered) {      // recurrent state cannot be cut back to a prefix: a sequence always starts from nothing
         if (n_past != 0) return fail(B2_ERR_UNSUPPORTED, "layer-list models start every sequence at position 0 (no prefix reuse)");
-        if ((rc = layered_seq_reset(e, slot))) return rc;
     }
-    SamplerState h = {};
-    for (int i = 0; i < n_hist; i++) h.history[i] = hist[i];
-    h.n_hist = n_hist;
-    SampleParams p = {};
+    SeqUpdate u = {};
+    for (int i = 0; i < n_hist; i++) u.history.history[i] = hist[i];
+    u.history.n_hist = n_hist;
+    SampleParams& p = u.params;
     p.temperature = sp->temperature; p.top_p = sp->top_p; p.min_p = sp->min_p;
     p.repeat_penalty = sp->repeat_penalty; p.freq_penalty = sp->frequency_penalty;
     p.presence_penalty = sp->presence_penalty; p.top_k = sp->top_k;
     p.penalty_last_n = sp->penalty_last_n;
-    int ints[8] = {0, n_past, 0, 0, 0, n_past, 0, 0};
-    CK(cudaMemcpyAsync(s.sst, &h, sizeof(h), cudaMemcpyHostToDevice, e->stream));
-    CK(cudaMemcpyAsync(s.sp, &p, sizeof(p), cudaMemcpyHostToDevice, e->stream));
-    CK(cudaMemcpyAsync(s.ints, ints, sizeof(ints), cudaMemcpyHostToDevice, e->stream));
-    if (n_uni) CK(cudaMemcpyAsync(s.uniforms, uni, sizeof(double) * n_uni, cudaMemcpyHostToDevice, e->stream));
-    CK(cudaStreamSynchronize(e->stream));
+    u.ints[1] = u.ints[5] = n_past; u.n_ints = 8; u.start = true;
+    u.has_uniform = n_uni > 0;
+    if (n_uni) u.uniform = uni[0];
+    if ((rc = seq_update(e, slot, u))) return rc;
+    if (n_uni > 1) {
+        CK(cudaMemcpyAsync(s.uniforms, uni, sizeof(double) * n_uni, cudaMemcpyHostToDevice, e->stream));
+        CK(cudaStreamSynchronize(e->stream));
+    }
     s.n_past = n_past;
     s.last_token = -1;
     s.n_sampled = 0;
@@ -765,26 +802,24 @@ extern "C" int b2_prefill(b2_engine* e, int slot, const int32_t* tokens, int n) 
     for (int i = 0; i < n; i++)
         if (tokens[i] < 0 || tokens[i] >= e->cfg.n_vocab) return fail(B2_ERR_ARG, "token id out of range");
     CK(cudaSetDevice(e->cfg.device));
-    int hdr[2] = {0, s.n_past};   // cursor, pos_base
     CK(cudaMemcpyAsync(s.prompt, tokens, sizeof(int) * n, cudaMemcpyHostToDevice, e->stream));
-    CK(cudaMemcpyAsync(s.ints + 4, hdr, sizeof(hdr), cudaMemcpyHostToDevice, e->stream));
     if (e->gemm_ok && n >= e->prefill_min) {
         // tensor-core path: all layers for up to PF_T tokens at a time, then the output head for the last token only
         if ((rc = ensure_prefill_workspace(e))) return rc;
         for (int c0 = 0; c0 < n; c0 += PF_T) {
             int T = n - c0 < PF_T ? n - c0 : PF_T;
             if ((rc = prefill_chunk(e, s, s.prompt + c0, T, s.n_past + c0))) return rc;
-            if (c0 + T == n)
-                CK(cudaMemcpyAsync(s.x, e->pf_x + (size_t)(T - 1) * e->cfg.n_embd, sizeof(float) * e->cfg.n_embd,
-                                   cudaMemcpyDeviceToDevice, e->stream));
         }
-        CK(prefill_finish_launch(s.prompt, n, s.n_past + n - 1, s.ints, s.sst, e->stream));
+        // the head reads the last token's row where it is, its weights stream in while the chain before it ends
         MvParams h = e->p_head;
-        h.x = s.x; h.y = s.logits;
-        CK(mv_launch(h, e->n_ctas, e->stream, e->act2, false));
+        h.x = e->pf_x + (size_t)((n - 1) % PF_T) * e->cfg.n_embd; h.y = s.logits;
+        CK(mv_launch(h, e->n_ctas, e->stream, e->act2, e->chain_pdl && e->use_pdl));
+        CK(prefill_finish_launch(s.prompt, n, s.n_past + n - 1, s.ints, s.sst, e->stream));
         s.logits_view = s.logits;
         e->launches += 2;
     } else {
+        const int hdr[2] = {0, s.n_past};   // cursor, pos_base
+        CK(cudaMemcpyAsync(s.ints + 4, hdr, sizeof(hdr), cudaMemcpyHostToDevice, e->stream));
         for (int i = 0; i < n; i++) {
             rc = run_step(e, s, i == n - 1 ? GK_PRE_LAST : GK_PRE_STEP);
             if (rc) return rc;
@@ -801,11 +836,10 @@ __global__ void set_ints_kernel(int* ints, int tok, int pos) { if (tok >= 0) int
 // enqueue: sample from the slot's logit buffer (the token at position n_past - 1 was the last one evaluated); the token
 // is in e->slot_token once the stream has been synchronised
 static int sample_enqueue(b2_engine* e, Slot& s) {
-    // sampler bumps pos: make it point at the last evaluated token first
-    set_ints_kernel<<<1, 1, 0, e->stream>>>(s.ints, -1, s.n_past - 1);
+    // (the sampler moves the position on from the last evaluated token)
     CK(sample_launch(s.logits, e->cfg.n_vocab, s.sp, s.sst, s.uniforms, s.ints + 3, s.ints + 2, s.ints + 0,
-                     s.ints + 1, s.ring, e->cfg.n_ctx + 1, e->stream, false, e->slot_token + (&s - e->slots.data())));
-    e->launches += 2;
+                     s.ints + 1, s.ring, e->cfg.n_ctx + 1, e->stream, false, e->slot_token + (&s - e->slots.data()), s.n_past - 1));
+    e->launches++;
     s.n_sampled += 1;
     return B2_OK;
 }
@@ -1002,14 +1036,12 @@ extern "C" int b2_seq_rewind(b2_engine* e, int slot, int n_keep, int32_t pending
     if (n_hist < 0 || n_hist > HISTORY_LEN) return fail(B2_ERR_ARG, "history longer than 64");
     CK(cudaSetDevice(e->cfg.device));
     int dropped = s.n_past - n_keep;
-    SamplerState h = {};
-    for (int i = 0; i < n_hist; i++) h.history[i] = hist[i];
-    h.n_hist = n_hist;
+    SeqUpdate u = {};
+    for (int i = 0; i < n_hist; i++) u.history.history[i] = hist[i];
+    u.history.n_hist = n_hist;
     s.n_sampled = s.n_sampled > dropped ? s.n_sampled - dropped : 0;
-    int ints[4] = {pending, n_keep, pending, s.n_sampled};
-    CK(cudaMemcpyAsync(s.sst, &h, sizeof(h), cudaMemcpyHostToDevice, e->stream));
-    CK(cudaMemcpyAsync(s.ints, ints, sizeof(ints), cudaMemcpyHostToDevice, e->stream));
-    CK(cudaStreamSynchronize(e->stream));
+    u.ints[0] = u.ints[2] = pending; u.ints[1] = n_keep; u.ints[3] = s.n_sampled; u.n_ints = 4;
+    if ((rc = seq_update(e, slot, u))) return rc;
     s.n_past = n_keep;
     return B2_OK;
 }

@@ -55,6 +55,9 @@ struct Slot {
     int n_sampled = 0;             // host mirror of ints[3]
 };
 
+// recurrent state that starts from zero with every sequence: `floats` of them per slot
+struct ResetRegion { float* base; size_t floats; };
+
 struct b2_engine {
     b2_config cfg;
     cudaStream_t stream = nullptr;
@@ -69,6 +72,8 @@ struct b2_engine {
     unsigned* attn_counters = nullptr;
     int n_splits = 1, max_blocks = 0, n_ctas = 148;
     std::vector<Slot> slots;
+    ResetRegion* resets = nullptr; // device
+    int n_resets = 0;
     int32_t* pinned = nullptr;     // host memory that kernels write too: sampled tokens arrive here without a copy of their own
     int32_t* slot_token = nullptr; // the same, one entry per slot: written by the slot's (captured) sampler launches
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;

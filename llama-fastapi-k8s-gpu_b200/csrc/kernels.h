@@ -243,10 +243,10 @@ struct SamplerState {            // per sequence slot, device resident
 // logits[V] (modified in place by the penalties) -> *out_token; also pushes the token into the
 // history ring, stores it in *next_token_ptr, bumps *pos_ptr and records the token at
 // out_ring[new pos] (device-resident decode loop: the host can read many steps back at once). out_token2: the token goes here too (host memory,
-// say), or null.
+// say), or null. pos: the position to move on from, instead of *pos_ptr, or -2.
 cudaError_t sample_launch(float* logits, int n_vocab, const SampleParams* params_dev, SamplerState* st,
                           const double* uniforms, int* step_ptr, int* out_token, int* next_token_ptr,
-                          int* pos_ptr, int* out_ring, int ring_len, cudaStream_t s, bool pdl, int* out_token2 = nullptr);
+                          int* pos_ptr, int* out_ring, int ring_len, cudaStream_t s, bool pdl, int* out_token2 = nullptr, int pos = -2);
 
 // logits row z (row_stride floats apart) belongs to slot b.slot[z]; also writes the token to out_tokens[z]
 cudaError_t sample_batch_launch(float* logits, long row_stride, int n_vocab, const SlotDev* tab, const BatchIdx& b,

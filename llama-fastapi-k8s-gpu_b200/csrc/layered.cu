@@ -320,6 +320,33 @@ static int build_rotary(b2_engine* e, LayeredModel* m, LyLayer& L) {
     return B2_OK;
 }
 
+// what a slot that starts a new sequence sets back to zero (cache pages are simply overwritten)
+static std::vector<ResetRegion> slot_states(const LayeredModel* m) {
+    std::vector<ResetRegion> out;
+    auto add = [&](float* base, size_t floats) { if (base) out.push_back({base, floats}); };
+    for (auto& L : m->layers) {
+        const b2_layer_desc& d = L.d;
+        for (int q = 0; q < 2; q++) add(L.canon_state[q], (size_t)std::max(1, m->c.canon_taps - 1) * m->c.n_embd);
+        const size_t conv = (size_t)std::max(1, d.conv_taps - 1) * L.conv_C;
+        if (d.mixer == B2_MIX_SINK_ATTN) {
+            add(L.st_conv_state, conv);
+        } else if (d.mixer == B2_MIX_SINK_DELTA || d.mixer == B2_MIX_DELTA_RULE || d.mixer == B2_MIX_SSD) {
+            add(L.st_conv_state, conv);
+            add(L.st_state, col_state_floats(d.mm_heads, d.mixer == B2_MIX_SSD ? d.d_state : d.mm_dim, d.mm_vdim));
+        } else if (d.mixer == B2_MIX_WINDOW_SCAN) {
+            add(L.conv_state, (size_t)d.d_inner * std::max(1, d.conv_taps - 1));
+            add(L.ssm_state, (size_t)d.d_inner * d.d_state);
+        } else if (d.mixer == B2_MIX_CHUNK_LINEAR) {
+            add(L.la_state, col_state_floats(d.mm_heads, d.mm_dim, d.mm_vdim));
+        } else if (d.mixer != B2_MIX_LATENT_ATTN) {
+            add(L.S, (size_t)d.mm_heads * d.mm_dim * d.mm_vdim);
+            add(L.nvec, (size_t)d.mm_heads * d.mm_dim);
+            add(L.mmax, (size_t)d.mm_heads);
+        }
+    }
+    return out;
+}
+
 int layered_finalize(b2_engine* e) {
     LayeredModel* m = e->layered;
     const b2_layered_config& c = m->c;
@@ -759,6 +786,12 @@ int layered_finalize(b2_engine* e) {
         CK(cudaMemcpy(m->slot_tab, dev.data(), sizeof(SlotDev) * S, cudaMemcpyHostToDevice));
         CK(cudaMemcpy(m->slot_logits, lg.data(), sizeof(float*) * S, cudaMemcpyHostToDevice));
     }
+    const std::vector<ResetRegion> states = slot_states(m);
+    if (!states.empty()) {
+        if ((rc = dev_alloc(m, (void**)&e->resets, sizeof(ResetRegion) * states.size()))) return rc;
+        CK(cudaMemcpy(e->resets, states.data(), sizeof(ResetRegion) * states.size(), cudaMemcpyHostToDevice));
+        e->n_resets = (int)states.size();
+    }
     CK(cudaStreamSynchronize(e->stream));
     e->finalized = true;
     return B2_OK;
@@ -776,46 +809,6 @@ void layered_destroy(b2_engine* e) {
     e->layered = nullptr;
 }
 
-// a slot starts a new sequence: its recurrent state goes back to zero (cache pages are simply overwritten)
-int layered_seq_reset(b2_engine* e, int slot) {
-    LayeredModel* m = e->layered;
-    for (auto& L : m->layers) {
-        const b2_layer_desc& d = L.d;
-        for (int q = 0; q < 2; q++)
-            if (L.canon_state[q]) {
-                const size_t cs = (size_t)std::max(1, m->c.canon_taps - 1) * m->c.n_embd;
-                CK(cudaMemsetAsync(L.canon_state[q] + slot * cs, 0, cs * 4, e->stream));
-            }
-        if (d.mixer == B2_MIX_SINK_ATTN) {          // cache pages are overwritten
-            const size_t cs = (size_t)std::max(1, d.conv_taps - 1) * L.conv_C;
-            if (L.st_conv_state) CK(cudaMemsetAsync(L.st_conv_state + slot * cs, 0, cs * 4, e->stream));
-        } else if (d.mixer == B2_MIX_SINK_DELTA) {
-            const size_t cs = (size_t)std::max(1, d.conv_taps - 1) * L.conv_C, ss = col_state_floats(d.mm_heads, d.mm_dim, d.mm_vdim);
-            CK(cudaMemsetAsync(L.st_conv_state + slot * cs, 0, cs * 4, e->stream));
-            CK(cudaMemsetAsync(L.st_state + slot * ss, 0, ss * 4, e->stream));
-        } else if (d.mixer == B2_MIX_WINDOW_SCAN) {
-            const size_t cs = (size_t)d.d_inner * std::max(1, d.conv_taps - 1), ss = (size_t)d.d_inner * d.d_state;
-            CK(cudaMemsetAsync(L.conv_state + slot * cs, 0, cs * 4, e->stream));
-            CK(cudaMemsetAsync(L.ssm_state + slot * ss, 0, ss * 4, e->stream));
-        } else if (d.mixer == B2_MIX_LATENT_ATTN) {
-            // nothing but cache pages, which are overwritten
-        } else if (d.mixer == B2_MIX_CHUNK_LINEAR) {
-            const size_t ss = col_state_floats(d.mm_heads, d.mm_dim, d.mm_vdim);
-            CK(cudaMemsetAsync(L.la_state + slot * ss, 0, ss * 4, e->stream));
-        } else if (d.mixer == B2_MIX_DELTA_RULE || d.mixer == B2_MIX_SSD) {
-            const size_t cs = (size_t)std::max(1, d.conv_taps - 1) * L.conv_C;
-            const size_t ss = col_state_floats(d.mm_heads, d.mixer == B2_MIX_SSD ? d.d_state : d.mm_dim, d.mm_vdim);
-            CK(cudaMemsetAsync(L.st_conv_state + slot * cs, 0, cs * 4, e->stream));
-            CK(cudaMemsetAsync(L.st_state + slot * ss, 0, ss * 4, e->stream));
-        } else {
-            const size_t s1 = (size_t)d.mm_heads * d.mm_dim * d.mm_vdim, s2 = (size_t)d.mm_heads * d.mm_dim;
-            CK(cudaMemsetAsync(L.S + slot * s1, 0, s1 * 4, e->stream));
-            CK(cudaMemsetAsync(L.nvec + slot * s2, 0, s2 * 4, e->stream));
-            CK(cudaMemsetAsync(L.mmax + slot * d.mm_heads, 0, (size_t)d.mm_heads * 4, e->stream));
-        }
-    }
-    return B2_OK;
-}
 
 }  // namespace b2
 

@@ -434,6 +434,5 @@ cudaError_t hyper_join_conv_launch(const HyperJoinArgs& a, const ConvArgs& cv, c
 struct LayeredModel;
 int layered_finalize(b2_engine* e);
 void layered_destroy(b2_engine* e);
-int layered_seq_reset(b2_engine* e, int slot);
 
 }  // namespace b2

@@ -270,9 +270,10 @@ __global__ void __launch_bounds__(SM_THREADS) sample_kernel(float* logits, int V
                                                             SamplerState* st, const double* uniforms,
                                                             int n_uniform, int* step_ptr, int* out_token,
                                                             int* next_token_ptr, int* pos_ptr, int* out_ring,
-                                                            int ring_len, int* out_token2) {
+                                                            int ring_len, int* out_token2, int pos) {
     griddep_launch();
     griddep_wait();
+    if (pos >= -1 && threadIdx.x == 0) *pos_ptr = pos;      // (thread 0 also moves it on)
     sample_body(logits, V, prm, st, uniforms, n_uniform, step_ptr, out_token, next_token_ptr, pos_ptr, out_ring, ring_len, out_token2);
 }
 
@@ -316,7 +317,7 @@ cudaError_t sample_batch_launch(float* logits, long row_stride, int n_vocab, con
 
 cudaError_t sample_launch(float* logits, int n_vocab, const SampleParams* params_dev, SamplerState* st,
                           const double* uniforms, int* step_ptr, int* out_token, int* next_token_ptr,
-                          int* pos_ptr, int* out_ring, int ring_len, cudaStream_t s, bool pdl, int* out_token2) {
+                          int* pos_ptr, int* out_ring, int ring_len, cudaStream_t s, bool pdl, int* out_token2, int pos) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(1); cfg.blockDim = dim3(SM_THREADS); cfg.stream = s;
     cudaLaunchAttribute at[1];
@@ -325,7 +326,7 @@ cudaError_t sample_launch(float* logits, int n_vocab, const SampleParams* params
     cfg.attrs = at; cfg.numAttrs = pdl ? 1 : 0;
     int n_uniform = 8192;
     return cudaLaunchKernelEx(&cfg, sample_kernel, logits, n_vocab, params_dev, st, uniforms, n_uniform,
-                              step_ptr, out_token, next_token_ptr, pos_ptr, out_ring, ring_len, out_token2);
+                              step_ptr, out_token, next_token_ptr, pos_ptr, out_ring, ring_len, out_token2, pos);
 }
 
 }  // namespace b2
