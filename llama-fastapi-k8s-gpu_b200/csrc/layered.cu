@@ -1757,11 +1757,18 @@ extern "C" int b2_step(b2_engine* e, int n_entries, const int32_t* slots, const 
         tile_of[k] = tile;
         for (int i = 0; i < n; i++) if (size_class(n_tokens[i]) == k) tile += (n_tokens[i] + 63) / 64;
     }
+    // (of longer entries the odd tiles ahead: 128-query tiles begin at the even ones)
+    int n_odd = 0;
+    for (int i = 0; i < n; i++) if (n_tokens[i] > 64) n_odd += (n_tokens[i] + 63) / 64 / 2;
+    int at_even = tile_of[7] + n_odd;
     for (int i = 0; i < n; i++) {
         const int p0 = e->slots[slots[i]].n_past;
         h_slot[i] = slots[i]; h_start[i] = row; h_len[i] = n_tokens[i]; h_p0[i] = p0;
-        int& at = tile_of[size_class(n_tokens[i])];
-        for (int k = 0; k < n_tokens[i]; k += 64) { h_tseg[at] = i; h_trow[at++] = row + k; }
+        int& at_any = tile_of[size_class(n_tokens[i])];
+        for (int k = 0; k < n_tokens[i]; k += 64) {
+            int& at = n_tokens[i] > 64 && k % 128 == 0 ? at_even : at_any;
+            h_tseg[at] = i; h_trow[at++] = row + k;
+        }
         for (int k = 0; k < n_tokens[i]; k++, row++) {
             h_id[row] = tokens[row]; h_seg[row] = i; h_pos[row] = p0 + k;
             h_prev[row] = k > 0 ? tokens[row - 1] : e->slots[slots[i]].last_token;
@@ -1777,7 +1784,7 @@ extern "C" int b2_step(b2_engine* e, int n_entries, const int32_t* slots, const 
     RaggedDev r = {};
     r.tok_id = m->meta; r.tok_seg = m->meta + T; r.tok_pos = m->meta + 2 * T; r.tok_prev = m->meta + 3 * T; r.seg_slot = m->meta + 4 * T;
     r.seg_start = r.seg_slot + n; r.seg_len = r.seg_start + n; r.seg_pos0 = r.seg_len + n; r.T = T; r.n_seg = n;
-    r.tile_seg = r.seg_pos0 + n; r.tile_row0 = r.tile_seg + n_tiles; r.n_tiles = n_tiles;
+    r.tile_seg = r.seg_pos0 + n; r.tile_row0 = r.tile_seg + n_tiles; r.n_tiles = n_tiles; r.n_odd = n_odd;
     for (int k = 0; k < 7; k++) r.n_upto[k] = tile_of[k];       // (past the tiles of class k by now)
     const int* d_rows = r.tile_row0 + n_tiles;
     if (m->profile) {

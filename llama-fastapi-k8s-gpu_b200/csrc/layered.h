@@ -27,6 +27,7 @@ struct RaggedDev {             // device pointers, valid for one step
     const int* tile_row0;      // ... and its first row. Segments of up to 64 tokens (one tile each) come first, the shortest ahead:
     int n_upto[7];             // [i] segments, and tiles, of up to 2^i tokens
     int T, n_seg, n_tiles;
+    int n_odd;                 // behind the short ones: this many odd tiles of longer segments (second, fourth, ...), then the even ones
 };
 
 // ---------------------------------------------------------------- dense products (dense.cu)

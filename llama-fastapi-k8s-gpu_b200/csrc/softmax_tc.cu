@@ -11,7 +11,10 @@
 // operations a score; that unit is busy for 35 % of 2048 tokens' time, the tensor pipe for 23 %: what bounds the kernel is the chain of a block, and
 // 256 CTAs of unequal length on 148 SMs); they exchange their maxima through shared memory. The output is rescaled only
 // when a row's maximum has grown by more than 2^8.
-// 2048 tokens (B200): 16 capped heads of 128, 300 us a layer with mma.sync, 67 here; 32 heads of 128 over a window of 1024 keys, 326 and 99.
+// 2048 tokens (B200): 16 capped heads of 128, 300 us a layer with mma.sync, 65 here; 32 heads of 128 over a window of 1024 keys, 326 and 92.
+// (70 and 100 with the wait for the previous block's products ahead of the exponentials and all eight warps at one barrier for the maxima.
+// Blocks of 64 keys with one thread a row, of which two CTAs fit on an SM: 80 and 80; there the first product reads its queries from shared
+// memory twice as often, and 256 CTAs of unequal length leave an SM two long ones.)
 #include "kernels.h"
 #include "layered.h"
 #include "ptx.cuh"
@@ -41,7 +44,7 @@ __device__ __forceinline__ void sx_split(float a, float b, uint32_t& hi, uint32_
 // tile0[k], its CTAs at cta0[k]
 struct SxShort { int tile0[7], cta0[7], heads[7]; };
 
-// CTAs: (64-query tile, head) of longer sequences, latest tiles first (odd tiles of a sequence belong to the CTA before them), then (sequence,
+// CTAs: (even tile, head) of longer sequences, the last tiles first, then (sequence,
 // group of heads) of the others, the longest first. SHORT: there are such (2048 tokens of one sequence take 85 us a layer without that part
 // and 89 with it, preparation included)
 template <bool CAP, bool SHORT>
@@ -52,7 +55,7 @@ __global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_
     __shared__ uint32_t tmem_at;
     __shared__ float row_max[2][2][SX_Q], row_sum[2][SX_Q];
     int tile = r.n_tiles - 1 - (int)blockIdx.x / a.H, h = (int)blockIdx.x % a.H, per_tok = 1;      // per_tok: rows of a token, heads h ..
-    if (const int in_short = (int)blockIdx.x - (r.n_tiles - r.n_upto[6]) * a.H; SHORT && in_short >= 0) {
+    if (const int in_short = (int)blockIdx.x - (r.n_tiles - r.n_upto[6] - r.n_odd) * a.H; SHORT && in_short >= 0) {
         int k = 6;
         while (k > 0 && in_short >= sh.cta0[k - 1]) k--;
         per_tok = sh.heads[k];
@@ -60,7 +63,6 @@ __global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_
         h = (in_short - sh.cta0[k]) % (a.H / per_tok) * per_tok;
     }
     const int seg = r.tile_seg[tile], row0 = r.tile_row0[tile];
-    if (((row0 - r.seg_start[seg]) / 64) & 1) return;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (warp: known to be uniform)
     const int n_tok = min(SX_Q, r.seg_start[seg] + r.seg_len[seg] - row0);
     const int nq = n_tok * per_tok, n_thr = SHORT ? (nq + 31) / 32 * 64 : 2 * SX_Q;      // rows in use; softmax threads: two a row, whole warps
@@ -207,26 +209,11 @@ __global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_
 #pragma unroll
             for (int j = 0; j < 64; j++) mx = fmaxf(mx, s[j]);
             row_max[i & 1][side][row] = mx;
-            named_bar_sync(1, n_thr);
+            named_bar_sync(1 + (warp & 3), 64);                   // (the two warps of these rows)
             mx = fmaxf(mx, row_max[i & 1][side ^ 1][row]);
             const bool grow = mx > m_ref + 8.f || (m_ref == -INFINITY && mx > -INFINITY);
-            // the previous block's products must be in before the output is rescaled and the probabilities are rewritten
-            if (i > 0) { mbar_wait(&pv_done, (i - 1) & 1, err, 0x70007u, (unsigned)i); tc_after_sync(); }
-            if (__any_sync(0xffffffffu, grow)) {
-                const float m_new = grow ? mx : m_ref, f = grow ? sx_exp2(m_ref - m_new) : 1.f;
-                m_ref = m_new;
-                l *= f;
-                if (i > 0) {                                      // this side's 64 columns of the output
-                    for (int c = side * 64; c < min(side * 64 + 64, v_parts * 64); c += 32) {
-                        uint32_t o[32];
-                        tc_ld32(o_at + c + lanes, o);
-                        tc_wait_ld();
-#pragma unroll
-                        for (int e = 0; e < 32; e++) o[e] = __float_as_uint(__uint_as_float(o[e]) * f);
-                        tc_st32(o_at + c + lanes, o);
-                    }
-                }
-            }
+            float f = 1.f;
+            if (grow) { f = sx_exp2(m_ref - mx); m_ref = mx; l *= f; }
             const float ref = m_ref > -INFINITY ? m_ref : 0.f;    // nothing visible yet and no sink: every weight is 0
             uint32_t hi[32], lo[32];
 #pragma unroll
@@ -234,6 +221,19 @@ __global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_
                 const float e0 = sx_exp2(s[j] - ref), e1 = sx_exp2(s[j + 1] - ref);
                 l += e0 + e1;
                 sx_split(e0, e1, hi[j >> 1], lo[j >> 1]);
+            }
+            // the previous block's products run until here; they must be in before the output is rescaled and the probabilities are rewritten
+            if (i > 0) {
+                mbar_wait(&pv_done, (i - 1) & 1, err, 0x70007u, (unsigned)i);
+                tc_after_sync();
+                if (__any_sync(0xffffffffu, grow))                // this side's 64 columns of the output
+                    for (int c = side * 64; c < min(side * 64 + 64, a.dv); c += 16) {
+                        float o[16];
+                        tc_ld16(o_at + c + lanes, o);
+#pragma unroll
+                        for (int e = 0; e < 16; e++) o[e] *= f;
+                        tc_st16(o_at + c + lanes, o);
+                    }
             }
             __syncwarp();
             tc_st32(p_at + side * 32 + lanes, hi);
@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(SX_THREADS, 1) softmax_tc_kernel(const __grid_
             mbar_arrive(&p_full);
         }
         row_sum[side][row] = l;
-        named_bar_sync(1, n_thr);
+        named_bar_sync(1 + (warp & 3), 64);
         l += row_sum[side ^ 1][row];
         if (a.sink) l += sx_exp2(sink - m_ref);
         const float inv = l > 0.f ? 1.f / l : 0.f;
@@ -333,7 +333,7 @@ cudaError_t softmax_tc_launch(const SoftmaxTcArgs& a, const RaggedDev& r, cudaSt
         sh.cta0[k] = ctas;
         ctas += (r.n_upto[k] - sh.tile0[k]) * (a.H / heads);
     }
-    const dim3 grid((r.n_tiles - r.n_upto[6]) * a.H + ctas), block(SX_THREADS);
+    const dim3 grid((r.n_tiles - r.n_upto[6] - r.n_odd) * a.H + ctas), block(SX_THREADS);
     if (grid.x == 0) return cudaSuccess;
     const auto kernel = a.softcap > 0.f ? (ctas ? softmax_tc_kernel<true, true> : softmax_tc_kernel<true, false>)
                                         : (ctas ? softmax_tc_kernel<false, true> : softmax_tc_kernel<false, false>);
