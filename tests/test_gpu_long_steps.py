@@ -126,6 +126,36 @@ def test_products_in_32_bits(native_lib, tmp_path, kind, W, ff, lengths):
     check(util, ref, cfg, tmp_path, lengths, "float32", bar=4e-6)
 
 
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("W,dim,inner", [(66, 10, 34), (72, 130, 36), (1020, 20, 24), (1024, 64, 40), (1028, 12, 40), (2052, 16, 40), (4100, 16, 24)])
+def test_rows_between_products(native_lib, tmp_path, W, dim, inner, dtype):
+    """The row kernels on both sides of their rules: widths that are not multiples of 4, of one, two and four reads a thread and beyond 4096 entries;
+    heads of 4-entry groups, of other sizes and beyond 128."""
+    cfg = gu.config([gu.parallel(mlp=48, left=gu.attn(heads=2, kv_heads=1, dim=dim, window=9), right=gu.scan(inner=inner)), gu.mlstm(mlp=40, heads=2, dim=24, vdim=20)], width=W)
+    check(gu, goponex_ref, cfg, tmp_path, [21, 9], dtype)
+
+
+def test_slots_start_from_empty_states(native_lib, tmp_path):
+    """Every recurrent state, tail and stabiliser of a slot is cleared when its next sequence starts, and no other slot's."""
+    from llama_cpp.kv_pages import SequenceSlots
+    cfg = gu.config([gu.parallel(mlp=40), gu.mlstm(heads=2, dim=17, vdim=33), gu.parallel(right=gu.scan(inner=41, conv=4))])
+    w = gu.random_weights(cfg, seed=5)
+    eng = engine(gu.write_model(str(tmp_path / "m"), cfg, w), "float32", 40, 3)
+    prompts = [toks(cfg["vocab"], n, 7 + n) for n in (20, 33, 12)]
+    seqs = SequenceSlots(eng)
+    for i in range(3):
+        seqs.open(i)
+    eng.step([(seqs.extend(i, len(p)), p) for i, p in enumerate(prompts)])
+    seqs.close(1)
+    seqs.open("again")
+    p = toks(cfg["vocab"], 15, 3)
+    lg, _ = eng.step([(seqs.extend("again", 15), p), (seqs.extend(0, 1), [5]), (seqs.extend(2, 1), [6])], want=[list(range(15)), [0], [0]])
+    eng.close()
+    want = [goponex_ref.forward(cfg, w, t) for t in (p, prompts[0] + [5], prompts[2] + [6])]
+    assert rows_off(lg[:15], want[0]).max() < F32
+    assert rows_off(lg[15:], np.stack([want[1][-1], want[2][-1]])).max() < F32
+
+
 def decode_all(util, ref, cfg, tmp_path, **kw):
     """Steps that decode all sequences, keys across one to three blocks of 64."""
     from llama_cpp.kv_pages import SequenceSlots

@@ -225,6 +225,28 @@ def test_tensor_core_prefill_agrees_with_token_by_token(native_lib, tmp_models, 
     assert outs[0][0] == outs[1][0]
 
 
+@pytest.mark.parametrize("n,first", [(255, 0), (256, 0), (257, 0), (259, 0), (512 + 258, 0), (300, 41), (37, 300)])
+def test_prompts_at_the_edges_of_row_groups(native_lib, tmp_models, monkeypatch, n, first):
+    """From 256 tokens four rows share a CTA between the products, below each has its own; prompts behind `first` cached positions too. Against
+    the mat-vec path, as above."""
+    path = _model(tmp_models, "tiny128", "Q4_K_M", 9)
+    prompt = [int(t) for t in np.random.default_rng(n).integers(3, 700, size=first + n)]
+    outs = []
+    for by_token in (False, True):
+        if by_token:
+            monkeypatch.setenv("B2_PREFILL_MIN", "100000")
+        else:
+            monkeypatch.delenv("B2_PREFILL_MIN", raising=False)
+        eng = _engine(path, n_ctx=1024, bt=64)
+        eng.ensure_pages(0, 900)
+        eng.seq_begin(0, 0, [], _greedy())
+        for part in ([prompt[:first], prompt[first:]] if first else [prompt]):
+            eng.prefill(0, part)
+        outs.append(eng.logits(0).copy())
+        eng.close()
+    assert np.abs(outs[0] - outs[1]).max() <= LOGIT_TOL
+
+
 @pytest.mark.parametrize("attn_splits", [0, 1])      # 1: one split per sequence (what 32-sequence steps use)
 @pytest.mark.parametrize("arch,ftype,seed", [("tiny", "Q4_K_M", 1), ("tiny128", "Q8_0", 6)])
 def test_batched_decode_matches_oracle_and_serial_path(native_lib, tmp_models, arch, ftype, seed, attn_splits, monkeypatch):

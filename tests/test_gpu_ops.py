@@ -250,6 +250,16 @@ def test_sampler_greedy_ties_take_lowest_id(native_lib):
     assert _sample(native_lib, logits, [], 0.5, temperature=0.0, repeat_penalty=1.0) == 77
 
 
+@pytest.mark.parametrize("V", [4, 5, 4096, 32767, 32768, 32772, 65541])
+def test_sampler_greedy_at_the_edges_of_reads(native_lib, V):
+    # 16-byte reads, eight of them a thread of 1024 (32768 entries a round), or single ones: the first of equal maxima, wherever it stands
+    for at in {0, 3, V - 1, V // 2, min(V - 1, 32767), min(V - 1, 32768)}:
+        logits = np.full(V, -np.inf, np.float32)
+        logits[at:] = np.linspace(-2.0, -1.0, V - at, dtype=np.float32)
+        logits[[at, V - 1]] = 3.5
+        assert _sample(native_lib, logits, [], 0.5, temperature=0.0, repeat_penalty=1.0) == at
+
+
 def test_sampler_topk_ties_at_threshold(native_lib):
     # 100 equal logits compete for the last top-k places: the lowest ids must be kept
     from oracle import sampler_ref as sr
