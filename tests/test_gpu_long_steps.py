@@ -135,6 +135,13 @@ def test_rows_between_products(native_lib, tmp_path, W, dim, inner, dtype):
     check(gu, goponex_ref, cfg, tmp_path, [21, 9], dtype)
 
 
+@pytest.mark.parametrize("W,n", [(70, 17), (1020, 17), (1024, 16), (1028, 40), (1030, 17), (2052, 33), (4096, 17)])
+def test_joins_at_the_edges_of_rows(native_lib, tmp_path, W, n):
+    """Joins with and without experts, rows of one, two and four reads a thread, rows that are no whole reads, few tokens and more."""
+    cfg = zu.config([zu.biased(mlp=zu.moe(experts=5, ff=24, shared=40)), zu.conved()], width=W)
+    check(zu, zogurax_ref, cfg, tmp_path, [n], "float32")
+
+
 def test_slots_start_from_empty_states(native_lib, tmp_path):
     """Every recurrent state, tail and stabiliser of a slot is cleared when its next sequence starts, and no other slot's."""
     from llama_cpp.kv_pages import SequenceSlots
