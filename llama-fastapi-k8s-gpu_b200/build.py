@@ -67,7 +67,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
             raise RuntimeError("link failed")
     host = os.path.join(LIB, "libb200_hosttest.so")
     hsrc = os.path.join(CSRC, "host_selftest.cpp")
-    if force or _newer(host, [hsrc, os.path.join(CSRC, "quant_blocks.cuh"), os.path.join(CSRC, "gemm_ring.h")]):
+    if force or _newer(host, [hsrc, os.path.join(CSRC, "quant_blocks.cuh"), os.path.join(CSRC, "gemm_ring.h"), os.path.join(CSRC, "per_device.h")]):
         subprocess.run(["g++", "-O2", "-ffp-contract=off", "-fPIC", "-shared", hsrc, "-o", host], check=True)
     return out
 

@@ -209,8 +209,7 @@ __global__ void rows_to_parts_kernel(const float* __restrict__ x, int ldx, const
 typedef void (*SplitKernel)(const CUtensorMap, const CUtensorMap, const TcParams);
 template <int EPI>
 static SplitKernel split_kernel_of() {
-    static const bool ready = cudaFuncSetAttribute(dense_split_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_RING + 1024) == cudaSuccess;
-    return ready ? dense_split_kernel<EPI> : nullptr;
+    return allow_smem<dense_split_kernel<EPI>>(TC_RING + 1024) ? dense_split_kernel<EPI> : nullptr;
 }
 static SplitKernel split_kernel(int epi) {
     switch (epi) {

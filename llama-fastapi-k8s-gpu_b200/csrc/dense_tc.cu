@@ -319,11 +319,8 @@ bool bf16_heads_map(CUtensorMap* m, const void* base, long cols, long heads, lon
 typedef void (*TcKernel)(const CUtensorMap, const CUtensorMap, const TcParams);
 template <int EPI, bool ROUNDED = false>
 static TcKernel tc_kernel_of(bool short_step) {
-    static const bool ready = [] {
-        return cudaFuncSetAttribute(dense_tc_kernel<EPI, ROUNDED, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) == cudaSuccess &&
-               cudaFuncSetAttribute(dense_tc_kernel<EPI, ROUNDED, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) == cudaSuccess;
-    }();
-    return !ready ? nullptr : short_step ? dense_tc_kernel<EPI, ROUNDED, true> : dense_tc_kernel<EPI, ROUNDED, false>;
+    if (short_step) return allow_smem<dense_tc_kernel<EPI, ROUNDED, true>>(TC_SMEM) ? dense_tc_kernel<EPI, ROUNDED, true> : nullptr;
+    return allow_smem<dense_tc_kernel<EPI, ROUNDED, false>>(TC_SMEM) ? dense_tc_kernel<EPI, ROUNDED, false> : nullptr;
 }
 static TcKernel tc_kernel(int epi, bool rounded, bool short_step) {
     if (rounded) {

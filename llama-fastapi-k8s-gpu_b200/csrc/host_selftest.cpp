@@ -4,6 +4,7 @@
 #define B2_HOST_EMU 1
 #include <math.h>
 #include "gemm_ring.h"
+#include "per_device.h"
 #include "quant_blocks.cuh"
 
 template <int T>
@@ -29,6 +30,15 @@ extern "C" {
 int b2_host_gemm_stages(int in_smem, int wanted) { return b2::gm_stages(in_smem != 0, wanted); }
 int b2_host_gemm_group(int block) { return b2::gm_group(block); }
 int b2_host_gemm_stage(int block, int stages) { return b2::gm_stage(block, stages); }
+
+// what is done once per device (per_device.h): `calls` devices in turn, refused (-1 - device) or not; how often each of the n was set up
+void b2_host_per_device(const int* calls, int n_calls, int* times, int* ready) {
+    b2::PerDevice once;
+    for (int i = 0; i < n_calls; i++) {
+        const int device = calls[i] < 0 ? -1 - calls[i] : calls[i];
+        ready[i] = once.ready(device, [&] { times[device]++; return calls[i] >= 0; });
+    }
+}
 
 // dequantise n_elems elements (whole blocks) with the exact element routine
 int b2_host_dequant(int type, const uint8_t* raw, long n_elems, float* out) {

@@ -163,21 +163,13 @@ __global__ void __launch_bounds__(1024) hyper_join_conv_kernel(HyperDev p, ConvA
 
 template <int SM>
 static cudaError_t hyper_join_pick(const HyperDev& p, bool few, int T, size_t smem, cudaStream_t s) {
-    if (smem > 48 * 1024) {
-        static bool attr_done = false;
-        if (!attr_done) {
-            cudaFuncSetAttribute(hyper_join_kernel<256, SM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            cudaFuncSetAttribute(hyper_join_kernel<1024, SM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            attr_done = true;
-        }
-    }
+    if (smem > 48 * 1024 && !(allow_smem<hyper_join_kernel<256, SM>>(200 * 1024) && allow_smem<hyper_join_kernel<1024, SM>>(200 * 1024))) return cudaErrorInvalidValue;
     if (few && SM <= 8) return launch_chain(hyper_join_kernel<1024, SM>, dim3(T), dim3(1024), smem, s, p);
     return launch_chain(hyper_join_kernel<256, SM>, dim3(T), dim3(256), smem, s, p);
 }
 template <int SM>
 static cudaError_t hyper_join_conv_pick(const HyperDev& p, const ConvArgs& cv, const RaggedDev& r, int W, size_t smem, cudaStream_t s) {
-    static bool attr_done = false;
-    if (!attr_done) { cudaFuncSetAttribute(hyper_join_conv_kernel<SM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024); attr_done = true; }
+    if (!allow_smem<hyper_join_conv_kernel<SM>>(160 * 1024)) return cudaErrorInvalidValue;
     return launch_chain(hyper_join_conv_kernel<SM>, dim3(r.n_seg), dim3(W >= 1024 ? 1024 : 256), smem, s, p, cv, r);
 }
 

@@ -8,7 +8,19 @@
 #include <string>
 #include <utility>
 
+#include "per_device.h"
+
 namespace b2 {
+
+// Lets Kernel take up to `bytes` (always the same for one kernel) of dynamic shared memory on the current device; false: the device refuses.
+// The limit belongs to the kernel on ONE device, so a flag that is set once per process would leave a second GPU's engine without it.
+template <auto Kernel>
+bool allow_smem(int bytes) {
+    static PerDevice limits;
+    int device;
+    if (cudaGetDevice(&device) != cudaSuccess) return false;
+    return limits.ready(device, [bytes] { return cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess; });
+}
 
 // Kernels of the prompt / batched-decode chains are launched with programmatic dependent launch while this is set
 // (engine.cu sets it around a chain): a kernel may start while its predecessor still runs and must execute

@@ -407,12 +407,7 @@ cudaError_t latent_attn_launch(const LatentAttnArgs& a, const RaggedDev& r, cuda
     if (Dk > 640) return cudaErrorInvalidValue;
     static const bool no_mma = getenv("B2_NO_ATTN_MMA") != nullptr;        // tuning aid: scalar attention for prompts too
     if (!no_mma && !a.cache_f32 && r.T > 8 && a.rank % 16 == 0 && Dk % 16 == 0 && a.ld_row % 8 == 0) {
-        static bool attr_done = false;
-        if (!attr_done) {
-            cudaFuncSetAttribute(latent_attn_mma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 64 * (640 + 8) * 2);
-            cudaFuncSetAttribute(latent_attn_mma_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 64 * (640 + 8) * 2);
-            attr_done = true;
-        }
+        if (!allow_smem<latent_attn_mma_kernel<128>>(2 * 64 * (640 + 8) * 2) || !allow_smem<latent_attn_mma_kernel<256>>(2 * 64 * (640 + 8) * 2)) return cudaErrorInvalidValue;
         const size_t smem = (size_t)2 * 64 * (Dk + 8) * 2;
         if (a.rank <= 128) return launch_chain(latent_attn_mma_kernel<128>, dim3(r.n_tiles, a.H, 1), dim3(128), smem, s, a, r);
         return launch_chain(latent_attn_mma_kernel<256>, dim3(r.n_tiles, a.H, (a.rank + 255) / 256), dim3(128), smem, s, a, r);

@@ -286,8 +286,7 @@ bool latent_attn_takes_tc(const LatentAttnArgs& a, int T) {
 }
 
 cudaError_t latent_attn_tc_launch(const LatentAttnArgs& a, const RaggedDev& r, const __nv_bfloat16* q, long pool_rows, __nv_bfloat16* out, cudaStream_t s) {
-    static const bool ready = cudaFuncSetAttribute(latent_attn_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 9 * (LC_QPART + LC_KPART) + 1024) == cudaSuccess;
-    if (!ready || !latent_attn_takes_tc(a, r.T)) return cudaErrorInvalidValue;
+    if (!allow_smem<latent_attn_tc_kernel>(9 * (LC_QPART + LC_KPART) + 1024) || !latent_attn_takes_tc(a, r.T)) return cudaErrorInvalidValue;
     const int parts = (a.rank + a.dr + LC_PART - 1) / LC_PART, chunks = (a.rank + LC_V - 1) / LC_V;
     CUtensorMap mk, mq, mh;
     // rows of the pages [pages * block_tokens][ld_row]; columns past rank + dr arrive as zeros

@@ -911,14 +911,9 @@ bool window_attn_leaves_rounded(const WindowAttnArgs& a, int T) { return window_
 cudaError_t window_attn_launch(const WindowAttnArgs& a, const RaggedDev& r, cudaStream_t s) {
     if (a.d > ATT_MAXE * 32 || (a.out_rounded && !window_attn_leaves_rounded(a, r.T))) return cudaErrorInvalidValue;
     if (window_attn_mma(a, r.T)) {
-        static bool attr_done = false;
-        if (!attr_done) {
-            cudaFuncSetAttribute(window_attn_mma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 64 * (64 + 8) * 2);
-            cudaFuncSetAttribute(window_attn_mma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 64 * (128 + 8) * 2);
-            attr_done = true;
-        }
         const SoftmaxTcArgs x = window_softmax_args(a);
         if (softmax_takes_tc(x)) return softmax_tc_launch(x, r, s);
+        if (!allow_smem<window_attn_mma_kernel<128>>(4 * 64 * (128 + 8) * 2)) return cudaErrorInvalidValue;
         const size_t smem = (size_t)4 * 64 * (a.d + 8) * 2;
         if (a.d <= 64) return launch_chain(window_attn_mma_kernel<64>, dim3(r.n_tiles, a.H), dim3(128), smem, s, a, r);
         return launch_chain(window_attn_mma_kernel<128>, dim3(r.n_tiles, a.H), dim3(128), smem, s, a, r);
@@ -1300,9 +1295,7 @@ template <int LANES, int SPL>
 static cudaError_t launch_scan_lanes(const ScanArgs& a, const RaggedDev& r, cudaStream_t s) {
     const int per_sm = (int)(((long)a.inner * r.n_seg + 147) / 148), n_ch = std::min(SC_CH, std::max(8, (per_sm + 7) / 8 * 8));
     constexpr int smem = 3 * SC_TB * (SC_CH * 16 + LANES * 2 * SPL * 4);
-    static const bool ready = cudaFuncSetAttribute(scan_recurrence_lanes_kernel<LANES, SPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   smem) == cudaSuccess;
-    if (!ready) return cudaErrorInvalidValue;
+    if (!allow_smem<scan_recurrence_lanes_kernel<LANES, SPL>>(smem)) return cudaErrorInvalidValue;
     return launch_chain(scan_recurrence_lanes_kernel<LANES, SPL>, dim3(r.n_seg, (a.inner + n_ch - 1) / n_ch), dim3(n_ch * LANES), smem, s, a, r);
 }
 
@@ -1571,8 +1564,7 @@ cudaError_t matrix_mem_launch(const MatrixMemArgs& a, const RaggedDev& r, cudaSt
         PlainLaunch pl;    // latency-bound over the prompt: CTAs spread over all SMs (see kernels.h)
         const int n_warps = (a.d + 2 * MM_ROWS - 1) / (2 * MM_ROWS);
         const size_t smem = (size_t)2 * MM_TB * (2 * n_warps * 2 * MM_ROWS + MM_COLS + 2 + 2 * n_warps * MM_COLS) * 4;
-        static const bool ready = cudaFuncSetAttribute(matrix_mem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) == cudaSuccess;
-        if (!ready) return cudaErrorInvalidValue;
+        if (!allow_smem<matrix_mem_kernel>(200 * 1024)) return cudaErrorInvalidValue;
         ce = launch_chain(matrix_mem_kernel, dim3(r.n_seg, a.H, (a.dv + MM_COLS - 1) / MM_COLS + 1), dim3(n_warps * 32), smem, s, a, r);
     }
     if (ce != cudaSuccess) return ce;

@@ -470,8 +470,7 @@ cudaError_t attn_prefill_launch(const __half* qh, const __half* k_cache, const _
     dim3 grid((T + q_tile - 1) / q_tile, n_kv), block(32 * G * QW);
     const float scale_log2 = 1.4426950408889634f / sqrtf((float)hd);
     const size_t smem = (size_t)2 * 2 * PA_KT * (hd + 8) * 2;
-    static const bool ready = cudaFuncSetAttribute(attn_prefill_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * PA_KT * (128 + 8) * 2) == cudaSuccess;
-    if (!ready) return cudaErrorInvalidValue;
+    if (!allow_smem<attn_prefill_kernel<128>>(4 * PA_KT * (128 + 8) * 2)) return cudaErrorInvalidValue;
     if (hd == 64) return launch_chain(attn_prefill_kernel<64>, grid, block, smem, s, qh, k_cache, v_cache, block_table, T, T_pad, pos0, n_head, n_kv, bt, QW, scale_log2, out);
     if (hd == 128) return launch_chain(attn_prefill_kernel<128>, grid, block, smem, s, qh, k_cache, v_cache, block_table, T, T_pad, pos0, n_head, n_kv, bt, QW, scale_log2, out);
     return cudaErrorInvalidValue;

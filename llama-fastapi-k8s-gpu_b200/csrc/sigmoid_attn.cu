@@ -285,11 +285,7 @@ __global__ void __launch_bounds__(128) sigmoid_attn_mma_kernel(SigmoidAttnArgs a
 template <int DMAX, int DVMAX>
 static cudaError_t sigmoid_attn_mma_pick(const SigmoidAttnArgs& a, const RaggedDev& r, cudaStream_t s) {
     const size_t smem = (size_t)(3 * 64 * (a.d + 8) + 64 * (a.dv + 8)) * 2;
-    static bool attr_done = false;
-    if (!attr_done) {
-        cudaFuncSetAttribute(sigmoid_attn_mma_kernel<DMAX, DVMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (3 * 64 * (DMAX + 8) + 64 * (DVMAX + 8)) * 2);
-        attr_done = true;
-    }
+    if (!allow_smem<sigmoid_attn_mma_kernel<DMAX, DVMAX>>((3 * 64 * (DMAX + 8) + 64 * (DVMAX + 8)) * 2)) return cudaErrorInvalidValue;
     return launch_chain(sigmoid_attn_mma_kernel<DMAX, DVMAX>, dim3(r.n_tiles, a.H), dim3(128), smem, s, a, r);
 }
 

@@ -276,8 +276,7 @@ __global__ void __launch_bounds__(NT, NT <= 256 ? 3 : 1) sink_attn_prepare_kerne
 
 template <int NT, int TB, int TAPS, int VEC>
 static cudaError_t sink_attn_prepare_go(const SinkAttnArgs& a, const RaggedDev& r, dim3 grid, size_t smem, int by_segment, cudaStream_t s) {
-    static bool attr_done = false;
-    if (!attr_done) { cudaFuncSetAttribute(sink_attn_prepare_kernel<NT, TB, TAPS, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); attr_done = true; }
+    if (!allow_smem<sink_attn_prepare_kernel<NT, TB, TAPS, VEC>>(200 * 1024)) return cudaErrorInvalidValue;
     return launch_chain(sink_attn_prepare_kernel<NT, TB, TAPS, VEC>, grid, dim3(NT), smem, s, a, r, by_segment);
 }
 template <int NT, int TB>
@@ -1274,8 +1273,7 @@ __global__ void __launch_bounds__(128) sink_attn_pv_kernel(SinkAttnArgs a, Ragge
 
 template <int DMAX>
 static cudaError_t sink_attn_probs_pick(const SinkAttnArgs& a, const RaggedDev& r, const SinkMix& mx, int nt, cudaStream_t s) {
-    static bool attr_done = false;
-    if (!attr_done) { cudaFuncSetAttribute(sink_attn_probs_kernel<DMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * 64 * (DMAX + 8) * 2); attr_done = true; }
+    if (!allow_smem<sink_attn_probs_kernel<DMAX>>(3 * 64 * (DMAX + 8) * 2)) return cudaErrorInvalidValue;
     return launch_chain(sink_attn_probs_kernel<DMAX>, dim3(nt, a.H), dim3(128), (size_t)3 * 64 * (a.d + 8) * 2, s, a, r, mx);
 }
 template <int DVMAX>
@@ -1288,10 +1286,8 @@ static bool sink_attn_mixed_launch(const SinkAttnArgs& a, const RaggedDev& r, cu
     const size_t per_tile = (size_t)a.H * SKM_Q * span;
     const size_t mix_smem = (size_t)(a.H * a.H + a.H * 256) * 4;
     if (!a.pbuf || per_tile > a.pbuf_floats || mix_smem > 96 * 1024) return false;
-    static bool attr_done = false;
-    if (!attr_done) { cudaFuncSetAttribute(sink_attn_mix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024); attr_done = true; }
     const int group = (int)std::min<size_t>(a.pbuf_floats / per_tile, (size_t)r.n_tiles);
-    e = cudaSuccess;
+    e = allow_smem<sink_attn_mix_kernel>(96 * 1024) ? cudaSuccess : cudaErrorInvalidValue;
     for (int t0 = 0; t0 < r.n_tiles && e == cudaSuccess; t0 += group) {
         const int nt = std::min(group, r.n_tiles - t0);
         SinkMix mx = {t0, span};
@@ -1309,13 +1305,8 @@ static bool sink_attn_packs(const SinkAttnArgs& a) { return !a.talk && a.H / a.G
 template <int DMAX, int DVMAX, bool CAP>
 static cudaError_t sink_attn_mma_pick(const SinkAttnArgs& a, const RaggedDev& r, bool only_one, cudaStream_t s) {
     const size_t smem = (size_t)(3 * 64 * (a.d + 8) + 64 * (a.dv + 8)) * 2;
-    static bool attr_done = false;
-    if (!attr_done) {
-        const int most = (3 * 64 * (DMAX + 8) + 64 * (DVMAX + 8)) * 2;
-        cudaFuncSetAttribute(sink_attn_mma_kernel<DMAX, DVMAX, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-        cudaFuncSetAttribute(sink_attn_pack_kernel<DMAX, DVMAX, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-        attr_done = true;
-    }
+    constexpr int most = (3 * 64 * (DMAX + 8) + 64 * (DVMAX + 8)) * 2;
+    if (!allow_smem<sink_attn_mma_kernel<DMAX, DVMAX, CAP>>(most) || !allow_smem<sink_attn_pack_kernel<DMAX, DVMAX, CAP>>(most)) return cudaErrorInvalidValue;
     RaggedDev rest = r;
     if (r.n_upto[0] > 0 && sink_attn_packs(a)) {
         const size_t pack = (size_t)((32 + SKM_K) * (a.d + 8) + SKM_K * (a.dv + 8)) * 2 + 16 * (SKM_K + 8) * 4;

@@ -311,14 +311,9 @@ bool softmax_takes_tc(const SoftmaxTcArgs& a) {
 
 cudaError_t softmax_tc_launch(const SoftmaxTcArgs& a, const RaggedDev& r, cudaStream_t s) {
     const int k_parts = (a.d + 63) / 64, v_parts = (a.dv + 63) / 64;
-    static const bool ready = [] {
-        const int most = 12 * SX_PART + 1024;
-        bool ok = true;
-        for (auto kernel : {softmax_tc_kernel<false, false>, softmax_tc_kernel<false, true>, softmax_tc_kernel<true, false>, softmax_tc_kernel<true, true>})
-            ok = ok && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess;
-        return ok;
-    }();
-    if (!ready || !softmax_takes_tc(a)) return cudaErrorInvalidValue;
+    constexpr int most = 12 * SX_PART + 1024;
+    if (!allow_smem<softmax_tc_kernel<false, false>>(most) || !allow_smem<softmax_tc_kernel<false, true>>(most) || !allow_smem<softmax_tc_kernel<true, false>>(most) ||
+        !allow_smem<softmax_tc_kernel<true, true>>(most) || !softmax_takes_tc(a)) return cudaErrorInvalidValue;
     CUtensorMap mk, mv;
     if (!bf16_rows_map(&mk, a.k_pool, a.d, a.pool_rows, a.d, 1, 0, 64) || !bf16_rows_map(&mv, a.v_pool, a.dv, a.pool_rows, a.dv, 1, 0, 64)) return cudaErrorInvalidValue;
     const size_t smem = (size_t)(4 * k_parts + 2 * v_parts) * SX_PART + 1024;

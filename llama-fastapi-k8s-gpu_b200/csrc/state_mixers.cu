@@ -255,10 +255,7 @@ static cudaError_t col_state_pick(const ColStateArgs& a, const RaggedDev& r, cud
     const int Rp = (a.R + 3) / 4 * 4;
     const size_t smem = (size_t)((a.row_decay ? 6 : 4) * CS_TB * Rp + 2 * CS_TB * (COLS + 2)) * 4;
     const dim3 grid(r.n_seg, a.H, (a.P + COLS - 1) / COLS), block(CS_WARPS * 32);
-    if (smem > 48 * 1024) {
-        cudaFuncSetAttribute(col_state_kernel<NCH, CPL, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-        cudaFuncSetAttribute(col_state_kernel<NCH, CPL, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-    }
+    if (smem > 48 * 1024 && !(allow_smem<col_state_kernel<NCH, CPL, true, true>>(64 * 1024) && allow_smem<col_state_kernel<NCH, CPL, false, true>>(64 * 1024))) return cudaErrorInvalidValue;
     if (a.delta && a.row_decay) return launch_chain(col_state_kernel<NCH, CPL, true, true>, grid, block, smem, s, a, r);
     if (a.delta) return launch_chain(col_state_kernel<NCH, CPL, true, false>, grid, block, smem, s, a, r);
     if (a.row_decay) return launch_chain(col_state_kernel<NCH, CPL, false, true>, grid, block, smem, s, a, r);
