@@ -334,6 +334,12 @@ int b2_op_gemm(int device, int type, const void* host_w, int n_rows, int K, cons
                const float* host_y_in, float* host_y, int n_splits);
 /* ggml rms_norm_f32 * weight */
 int b2_op_rmsnorm(int device, const float* host_x, const float* host_w, float eps, int K, int rows, float* host_y);
+/* Selective scan of one sequence, all in 32 bits: x (convolved input), z (gate), dt [T][inner], bc [T][B | C of n_state entries each],
+ * A_log [inner][n_state], dt_bias and D [inner], state [inner][n_state] (read and written). With step = softplus(dt + dt_bias):
+ * state = exp(-step exp(A_log)) state + step x B; y [T][inner] = (state . C + D x) silu(z). n_state <= 256. */
+int b2_op_scan(int device, int T, int inner, int n_state, const float* host_x, const float* host_z, const float* host_dt,
+               const float* host_dt_bias, const float* host_bc, const float* host_A_log, const float* host_D,
+               float* host_state, float* host_y);
 /* Decode attention for one sequence: q [n_head*head_dim] f32 (already rotated), K/V as f16
  * [n_ctx_tokens][n_kv][head_dim] (token-major; the op scatters them into pages in the order
  * host_blocks gives), attends to all n_ctx_tokens. out [n_head*head_dim] f32. * n_splits < 0 selects the tensor-core kernel (attention_mma.cu, q rounded to f16) with -n_splits splits. */

@@ -1378,6 +1378,33 @@ extern "C" int b2_op_rmsnorm(int device, const float* x, const float* w, float e
     return B2_OK;
 }
 
+extern "C" int b2_op_scan(int device, int T, int inner, int n_state, const float* x, const float* z, const float* dt, const float* dt_bias, const float* bc,
+                          const float* A_log, const float* D, float* state, float* y) {
+    if (!x || !z || !dt || !dt_bias || !bc || !A_log || !D || !state || !y || T <= 0 || inner <= 0 || n_state <= 0) return fail(B2_ERR_ARG, "bad arguments");
+    CK(cudaSetDevice(device));
+    DevBuf b[9], meta;
+    const size_t ti = (size_t)T * inner * 4, in = (size_t)inner * n_state * 4;
+    const float* from[9] = {x, z, dt, dt_bias, bc, A_log, D, state, nullptr};
+    const size_t bytes[9] = {ti, ti, ti, (size_t)inner * 4, (size_t)T * 2 * n_state * 4, in, (size_t)inner * 4, in, ti};
+    for (int i = 0; i < 9; i++) {
+        CK(b[i].alloc(bytes[i]));
+        if (from[i]) CK(cudaMemcpy(b[i].p, from[i], bytes[i], cudaMemcpyHostToDevice));
+    }
+    const int one[3] = {0, 0, T};               // slot, first row and length of the step's one sequence
+    CK(meta.alloc(sizeof(one)));
+    CK(cudaMemcpy(meta.p, one, sizeof(one), cudaMemcpyHostToDevice));
+    RaggedDev r = {};
+    r.seg_slot = meta.as<int>(); r.seg_start = r.seg_slot + 1; r.seg_len = r.seg_slot + 2; r.T = T; r.n_seg = 1;
+    ScanArgs a = {};
+    a.xc = b[0].as<float>(); a.proj = b[1].as<float>(); a.ldp = inner; a.taps = 1; a.conv_state = b[7].as<float>();      // (one tap: no state of it is touched)
+    a.dt_raw = b[2].as<float>(); a.dt_bias = b[3].as<float>(); a.xproj = b[4].as<float>(); a.ldx = 2 * n_state; a.N = n_state; a.A_log = b[5].as<float>();
+    a.D = b[6].as<float>(); a.ssm_state = b[7].as<float>(); a.y = b[8].as<float>(); a.inner = inner;
+    CK(scan_recurrence_launch(a, r, 0));
+    CK(cudaMemcpy(state, b[7].p, in, cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(y, b[8].p, ti, cudaMemcpyDeviceToHost));
+    return B2_OK;
+}
+
 extern "C" int b2_op_attention_decode(int device, const float* q, const uint16_t* k, const uint16_t* v, int T,
                                       int n_head, int n_kv, int hd, int bt, const int32_t* blocks, int nblk_total,
                                       int n_splits, float* out) {

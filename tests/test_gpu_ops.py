@@ -329,3 +329,33 @@ def test_gemm_rejects_bad_shapes(native_lib):
     assert native_lib.b2_op_gemm(0, TYPE_IDS["Q4_K"], ptr(w), 128, 128, ptr(x), 4, None, ptr(y), 0) != 0     # K % 256
     assert native_lib.b2_op_gemm(0, TYPE_IDS["Q4_K"], ptr(w), 128, 256, ptr(x), 513, None, ptr(y), 0) != 0   # too many tokens
     assert native_lib.b2_op_gemm(0, TYPE_IDS["F32"], ptr(w), 128, 256, ptr(x), 4, None, ptr(y), 0) != 0      # not a block format
+
+
+def _scan_ref(x, z, dt, dt_bias, bc, A_log, D, state):
+    """The recurrence in 64 bits."""
+    x, z, bc, S = x.astype(np.float64), z.astype(np.float64), bc.astype(np.float64), state.astype(np.float64)
+    step, A, N = np.logaddexp(0.0, dt.astype(np.float64) + dt_bias), np.exp(A_log.astype(np.float64)), A_log.shape[1]
+    y = np.empty_like(x)
+    for t in range(len(x)):
+        S = np.exp(-step[t][:, None] * A) * S + (step[t] * x[t])[:, None] * bc[t, :N]
+        y[t] = (S @ bc[t, N:] + D * x[t]) * z[t] / (1.0 + np.exp(-z[t]))
+    return y, S
+
+
+# Long memories sum up what a decay's rounding errs to one side. Step sizes of 0.01 to 0.02 remember about 100 tokens: the state is off by 4e-7 to 5.2e-7
+# (library functions), the output by half of 1e-7 (1 + sqrt(N)); with the decay as one approximate power of two by 1.6e-6 to 2e-6 and three times
+# as much. Shorter memories (second set): state 0.9e-7, output 1.3e-7 at most. Bars: about twice these.
+@pytest.mark.parametrize("steps,A,y_bar,y_per_root,state_bar", [((0.01, 0.02), (0.5, 1.0), 1e-7, 1e-7, 9e-7), ((0.05, 0.5), (0.5, 8.0), 2.6e-7, 0.0, 1.9e-7)])
+@pytest.mark.parametrize("N,inner,T", [(1, 24, 2000), (4, 64, 2000), (5, 65, 1999), (8, 40, 2001), (13, 130, 1700), (16, 64, 2000), (17, 40, 1601), (32, 72, 1000), (33, 40, 700),
+                                       (65, 16, 500)])
+def test_scan_in_32_bits(native_lib, N, inner, T, steps, A, y_bar, y_per_root, state_bar):
+    rng = np.random.default_rng(N)
+    f = lambda v: np.ascontiguousarray(v, dtype=np.float32)
+    x, z, dt, bc = (f(rng.standard_normal(s) * k) for s, k in (((T, inner), 1), ((T, inner), 1.5), ((T, inner), 0.3), ((T, 2 * N), 1)))
+    dt_bias, A_log, D = f(np.log(np.expm1(rng.uniform(*steps, inner)))), f(np.log(rng.uniform(*A, (inner, N)))), f(rng.uniform(0.5, 1.5, inner))
+    state = f(rng.standard_normal((inner, N)))
+    want_y, want_s = _scan_ref(x, z, dt, dt_bias, bc, A_log, D, state)
+    y = np.empty_like(x)
+    lib_check(native_lib, native_lib.b2_op_scan(0, T, inner, N, *map(ptr, (x, z, dt, dt_bias, bc, A_log, D, state, y))))
+    off = [float(np.linalg.norm(a - b) / np.linalg.norm(b)) for a, b in ((y, want_y), (state, want_s))]
+    assert off[0] < y_bar + y_per_root * N ** 0.5 and off[1] < state_bar, off
