@@ -334,6 +334,10 @@ int b2_op_gemm(int device, int type, const void* host_w, int n_rows, int K, cons
                const float* host_y_in, float* host_y, int n_splits);
 /* ggml rms_norm_f32 * weight */
 int b2_op_rmsnorm(int device, const float* host_x, const float* host_w, float eps, int K, int rows, float* host_y);
+/* Product of a layer-list model: x [T][K] f32, w [N][K] bf16, in 32 bits (exact) or with x rounded to bf16. epilogue 0: y [T][N] = x w^T;
+ * 1: the same times sigmoid(aux [T][N]); 2, 3: y [T][N / 2] = act(row 2i) * (row 2i + 1) of it, act = SiLU, GELU (tanh form). */
+int b2_op_product(int device, int exact, int T, int N, int K, const float* host_x, const uint16_t* host_w_bf16, int epilogue,
+                  const float* host_aux, float* host_y);
 /* Selective scan of one sequence, all in 32 bits: x (convolved input), z (gate), dt [T][inner], bc [T][B | C of n_state entries each],
  * A_log [inner][n_state], dt_bias and D [inner], state [inner][n_state] (read and written). With step = softplus(dt + dt_bias):
  * state = exp(-step exp(A_log)) state + step x B; y [T][inner] = (state . C + D x) silu(z). n_state <= 256. */

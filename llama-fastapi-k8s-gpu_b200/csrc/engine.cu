@@ -1378,6 +1378,27 @@ extern "C" int b2_op_rmsnorm(int device, const float* x, const float* w, float e
     return B2_OK;
 }
 
+extern "C" int b2_op_product(int device, int exact, int T, int N, int K, const float* x, const uint16_t* w, int epilogue, const float* aux, float* y) {
+    const int epis[4] = {EPI_NONE, EPI_MUL_SIGMOID, EPI_GLU_SILU, EPI_GLU_GELU};
+    if (!x || !w || !y || T <= 0 || N <= 0 || K <= 0 || epilogue < 0 || epilogue > 3 || (epilogue == 1 && !aux)) return fail(B2_ERR_ARG, "bad arguments");
+    CK(cudaSetDevice(device));
+    DenseArgs a = {};
+    a.T = T; a.N = N; a.K = a.ldx = K; a.w_type = T_BF16; a.epi = epis[epilogue]; a.exact = exact != 0; a.ldy = epilogue >= 2 ? N / 2 : N; a.ldaux = N;
+    const size_t xn = (size_t)T * K, wn = (size_t)N * K, yn = (size_t)T * a.ldy;
+    DevBuf dx, dw, da, dy, scratch;
+    CK(dx.alloc(xn * 4)); CK(dw.alloc(wn * 2)); CK(dy.alloc(yn * 4)); CK(scratch.alloc(3 * xn * 2 + 64));
+    CK(cudaMemcpy(dx.p, x, xn * 4, cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(dw.p, w, wn * 2, cudaMemcpyHostToDevice));
+    if (epilogue == 1) { CK(da.alloc((size_t)T * N * 4)); CK(cudaMemcpy(da.p, aux, (size_t)T * N * 4, cudaMemcpyHostToDevice)); }
+    a.x = dx.as<float>(); a.w = dw.p; a.y = dy.as<float>(); a.aux = da.as<float>();
+    (a.exact ? a.x_parts : a.xb) = scratch.as<__nv_bfloat16>();
+    CK(dense_launch(a, 0));
+    CK(cudaDeviceSynchronize());
+    { int rc = b2_check_kernel_error(); if (rc) return rc; }
+    CK(cudaMemcpy(y, dy.p, yn * 4, cudaMemcpyDeviceToHost));
+    return B2_OK;
+}
+
 extern "C" int b2_op_scan(int device, int T, int inner, int n_state, const float* x, const float* z, const float* dt, const float* dt_bias, const float* bc,
                           const float* A_log, const float* D, float* state, float* y) {
     if (!x || !z || !dt || !dt_bias || !bc || !A_log || !D || !state || !y || T <= 0 || inner <= 0 || n_state <= 0) return fail(B2_ERR_ARG, "bad arguments");

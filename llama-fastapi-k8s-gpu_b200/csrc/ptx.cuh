@@ -132,12 +132,12 @@ __device__ __forceinline__ float rcp_approx(float y) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
     return r;
 }
-// z / (1 + exp(w)) without a branch (a division has one): the approximate quotient, corrected once by its remainder; within two units of the last place
+// z / (1 + exp(w)) without a branch (a division has one): the approximate quotient and one correction by its remainder (a step of Newton's
+// method); within two units of the last place of expf's denominator. The reciprocal is taken of a quarter: past 2^126 it would be flushed to 0. Past
+// the largest number (w > 88.7) the quotient is 0. NaN and an infinite z come out as from a division.
 __device__ __forceinline__ float over_one_plus_exp(float z, float w) {
-    float y = 1.f + expf(w);
-    y = y > 1e37f ? 1e37f : y;                     // (its reciprocal is still a normal number; NaN passes)
-    const float r = rcp_approx(y), v = z * r;
-    return y == 1.f ? z : fmaf(fmaf(-y, v, z), r, v);         // (an infinite z too)
+    const float y = 1.f + expf(w), r = 0.25f * rcp_approx(0.25f * y), v = z * r, q = fmaf(fmaf(-y, v, z), r, v);
+    return y == 1.f ? z : y == INFINITY ? 0.f * z : q;
 }
 
 __device__ __forceinline__ float warp_sum(float v) {

@@ -359,3 +359,44 @@ def test_scan_in_32_bits(native_lib, N, inner, T, steps, A, y_bar, y_per_root, s
     lib_check(native_lib, native_lib.b2_op_scan(0, T, inner, N, *map(ptr, (x, z, dt, dt_bias, bc, A_log, D, state, y))))
     off = [float(np.linalg.norm(a - b) / np.linalg.norm(b)) for a, b in ((y, want_y), (state, want_s))]
     assert off[0] < y_bar + y_per_root * N ** 0.5 and off[1] < state_bar, off
+
+
+def product(native_lib, x, w, exact=True, epilogue=0, aux=None):
+    """The native product; w: float array of bf16 values."""
+    x, bits = np.ascontiguousarray(x, np.float32), np.ascontiguousarray(np.ascontiguousarray(w, np.float32).view(np.uint32) >> 16, np.uint16)
+    aux = None if aux is None else np.ascontiguousarray(aux, np.float32)
+    (T, K), N = x.shape, len(w)
+    y = np.full((T, N // 2 if epilogue >= 2 else N), -7.0, np.float32)
+    lib_check(native_lib, native_lib.b2_op_product(0, int(exact), T, N, K, ptr(x), ptr(bits), epilogue, None if aux is None else ptr(aux), ptr(y)))
+    return y
+
+
+@pytest.mark.parametrize("T", [3, 8, 9, 40])
+@pytest.mark.parametrize("kind", ["sigmoid", "silu", "gelu"])
+def test_gates_of_products(native_lib, kind, T):
+    """Gates of the epilogues in 32 bits, against 64: every value of a gate is one input picked by a weight of 1. Far to the left too, where the
+    denominator passes what its reciprocal and then what 32 bits hold."""
+    rng = np.random.default_rng(T)
+    K = 128
+    z = rng.uniform(-30.0, 30.0, (T, K)).astype(np.float32)
+    z[:, :16] = [-84, -85.5, -86.5, -87.5, -88, -88.6, -88.8, -90, -104, -1e4, -1e20, -1e37, -3e38, 100, 3e38, 0]
+    z64 = z.astype(np.float64)
+    pick = np.eye(K, dtype=np.float32)
+    if kind == "sigmoid":
+        z[:, 16:19] = z64[:, 16:19] = [np.inf, -np.inf, np.nan]
+        ones = np.zeros((K, K), np.float32)
+        ones[:, 0] = 1.0
+        got, w = product(native_lib, np.ones((T, K)), ones, epilogue=1, aux=z), -z64
+        want, scale = 1.0 / (1.0 + np.exp(np.minimum(w, 700.0))), np.ones_like(z64)
+        assert np.isnan(got[:, 18]).all() and (got[:, 16] == 1.0).all() and (got[:, 17] == 0.0).all()
+    else:
+        x = np.concatenate([z, np.ones((T, 8), np.float32)], 1)
+        rows = np.zeros((2 * K, K + 8), np.float32)
+        rows[0::2, :K], rows[1::2, K] = pick, 1.0
+        got = product(native_lib, x, rows, epilogue=2 if kind == "silu" else 3)
+        w = -z64 if kind == "silu" else -2.0 * np.sqrt(2.0 / np.pi) * (z64 + 0.044715 * z64 ** 3)
+        want, scale = z64 / (1.0 + np.exp(np.minimum(w, 700.0))), np.abs(z64)
+    # expf, the sum, the quotient: two to three units; GELU's exponent is itself off by a few units. Past 88.7 the exponential is infinite: 0.
+    units = 2.0 ** -24 * (4.0 + (4.0 * np.minimum(np.abs(w), 100.0) if kind == "gelu" else 0.0))
+    fine = np.isfinite(z64)
+    assert (np.abs(got - want) <= units * np.abs(want) + 3e-39 * scale)[fine].all(), np.argwhere((np.abs(got - want) > units * np.abs(want) + 3e-39 * scale) & fine)[:5]
