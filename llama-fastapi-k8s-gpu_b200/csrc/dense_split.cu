@@ -6,7 +6,8 @@
 // product; only the sums round. Tensor memory sums without rounding to nearest, and over a whole K that would show; so a sum stays there for
 // 64 entries of K only (three parts, the smallest first) and is then added to a 32-bit register in the order of k, as the multiply-add kernel
 // adds single terms. Errors against 64 bits are below that kernel's (below).
-// (An infinite WEIGHT meets the zeros behind an input's leading part as NaN, where multiply-adds keep the infinity; an infinite input stays one.)
+// (An infinite input stays one. An infinite WEIGHT would meet the zeros behind an input's leading part as NaN, where multiply-adds keep the
+// infinity: models with one never come here, see bf16_any_infinite.)
 //
 // Tiles of 128 weight rows (the lanes of tensor memory) and NT tokens, one after another per CTA. Ten warps: 0-7 add up and store (four
 // lanes' quarters, two halves of the token columns), 8 copies, 9 matrix instructions. Four accumulators of NT columns: the products of up to
@@ -205,7 +206,18 @@ __global__ void rows_to_parts_kernel(const float* __restrict__ x, int ldx, const
     }
 }
 
+__global__ void any_infinite_kernel(const uint16_t* __restrict__ w, size_t n, int* found) {
+    bool any = false;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) any |= (w[i] & 0x7fff) == 0x7f80;
+    if (any) *found = 1;
+}
+
 // ---------------------------------------------------------------- host side
+cudaError_t bf16_any_infinite(const void* w, size_t n, int* found, cudaStream_t s) {
+    any_infinite_kernel<<<148 * 8, 256, 0, s>>>(static_cast<const uint16_t*>(w), n, found);
+    return cudaGetLastError();
+}
+
 typedef void (*SplitKernel)(const CUtensorMap, const CUtensorMap, const TcParams);
 template <int EPI>
 static SplitKernel split_kernel_of() {

@@ -1385,13 +1385,18 @@ extern "C" int b2_op_product(int device, int exact, int T, int N, int K, const f
     DenseArgs a = {};
     a.T = T; a.N = N; a.K = a.ldx = K; a.w_type = T_BF16; a.epi = epis[epilogue]; a.exact = exact != 0; a.ldy = epilogue >= 2 ? N / 2 : N; a.ldaux = N;
     const size_t xn = (size_t)T * K, wn = (size_t)N * K, yn = (size_t)T * a.ldy;
-    DevBuf dx, dw, da, dy, scratch;
+    DevBuf dx, dw, da, dy, scratch, found;
     CK(dx.alloc(xn * 4)); CK(dw.alloc(wn * 2)); CK(dy.alloc(yn * 4)); CK(scratch.alloc(3 * xn * 2 + 64));
     CK(cudaMemcpy(dx.p, x, xn * 4, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(dw.p, w, wn * 2, cudaMemcpyHostToDevice));
     if (epilogue == 1) { CK(da.alloc((size_t)T * N * 4)); CK(cudaMemcpy(da.p, aux, (size_t)T * N * 4, cudaMemcpyHostToDevice)); }
     a.x = dx.as<float>(); a.w = dw.p; a.y = dy.as<float>(); a.aux = da.as<float>();
-    (a.exact ? a.x_parts : a.xb) = scratch.as<__nv_bfloat16>();
+    int infinite = 0;
+    CK(found.alloc(4)); CK(cudaMemset(found.p, 0, 4));
+    CK(bf16_any_infinite(dw.p, wn, found.as<int>(), 0));
+    CK(cudaMemcpy(&infinite, found.p, 4, cudaMemcpyDeviceToHost));
+    if (!a.exact) a.xb = scratch.as<__nv_bfloat16>();
+    else if (!infinite) a.x_parts = scratch.as<__nv_bfloat16>();
     CK(dense_launch(a, 0));
     CK(cudaDeviceSynchronize());
     { int rc = b2_check_kernel_error(); if (rc) return rc; }

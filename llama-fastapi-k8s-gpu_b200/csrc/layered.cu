@@ -102,7 +102,7 @@ struct LayeredModel {
     // step workspace (max_step_tokens rows)
     float *xs = nullptr, *hc = nullptr, *cross = nullptr;     // copies of the stream [S][max_step_tokens][W]; convolved sublayer input; per-(query head, value head) attention sums
     float *x = nullptr, *proj = nullptr, *buf[4] = {}, *oL = nullptr, *oR = nullptr, *hn = nullptr, *hn2 = nullptr, *ff = nullptr, *rows = nullptr, *logits = nullptr;
-    __nv_bfloat16* x_parts = nullptr;  // 32-bit engines: a product's input in three bf16 parts
+    __nv_bfloat16* x_parts = nullptr;  // 32-bit engines without infinite weights: a product's input in three bf16 parts
     __nv_bfloat16* xb = nullptr;       // a product's input rounded to bf16 [max_step_tokens][widest input]
     // blocks behind one norm: what a producer leaves already rounded for the large products: the normed row, the mixer's output row;
     // experts' activations (every family)
@@ -735,7 +735,17 @@ int layered_finalize(b2_engine* e) {
     max_ff = std::max(max_ff, max_glu);
     if ((rc = dev_alloc(m, (void**)&m->ff, (size_t)Tm * max_ff * 4))) return rc;
     const size_t widest = (size_t)(Tm + B2_STEP_MAX_ENTRIES) * std::max<size_t>({max_buf, max_ff, (size_t)(c.loop_times > 0 ? 2 * W : W), moe_xb});
-    if (m->exact ? (rc = dev_alloc(m, (void**)&m->x_parts, 3 * widest * 2 + 64)) : (rc = dev_alloc(m, (void**)&m->xb, widest * 2 + 64))) return rc;
+    if (m->exact) {
+        int* found = nullptr;
+        if ((rc = dev_alloc(m, (void**)&found, 4))) return rc;
+        CK(cudaMemsetAsync(found, 0, 4, e->stream));
+        for (auto& t : e->tensors)
+            if (t.second.type == T_BF16) CK(bf16_any_infinite(t.second.ptr, (size_t)t.second.nbytes / 2, found, e->stream));
+        int infinite = 0;
+        CK(cudaMemcpyAsync(&infinite, found, 4, cudaMemcpyDeviceToHost, e->stream));
+        CK(cudaStreamSynchronize(e->stream));
+        if (!infinite && (rc = dev_alloc(m, (void**)&m->x_parts, 3 * widest * 2 + 64))) return rc;
+    } else if ((rc = dev_alloc(m, (void**)&m->xb, widest * 2 + 64))) return rc;
     if (!m->exact && parallel && (rc = dev_alloc(m, (void**)&m->hn2_b, (size_t)Tm * W * 2 + 64))) return rc;
     if (!m->exact && c.block_style == B2_BLOCK_POSTSUM_LN && (rc = dev_alloc(m, (void**)&m->x_b, (size_t)Tm * W * 2 + 64))) return rc;
     if ((one_norm || parallel) && !m->exact) {

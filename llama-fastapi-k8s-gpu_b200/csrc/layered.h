@@ -67,7 +67,7 @@ struct DenseArgs {
     int epi;
     bool exact;                     // true: 32-bit multiply-adds (no tensor cores, inputs not rounded)
     __nv_bfloat16* xb;              // scratch for X rounded to bf16, [T][K] ([T][x_span] batched; pair rows when gathered); null: not available
-    __nv_bfloat16* x_parts = nullptr;      // scratch for X as three bf16 parts (exact products with bf16 weights); null: not available
+    __nv_bfloat16* x_parts = nullptr;      // scratch for X as three bf16 parts (exact products with finite bf16 weights); null: not available
     float scale = 1.f;              // the product (after the epilogue) times this
     int n_act = 0, n_act_end = 0;   // EPI_BIAS_PART_RELU2
     float p0 = 0.f, p1 = 0.f;       // constants of EPI_GLU_CLAMP / EPI_PIECEWISE
@@ -86,6 +86,8 @@ cudaError_t dense_launch(const DenseArgs& a, cudaStream_t s);
 bool dense_pairs(const DenseArgs& a, const DenseArgs& b);
 cudaError_t dense_pair_launch(const DenseArgs& a, const DenseArgs& b, cudaStream_t s);
 bool dense_takes_rounded(const DenseArgs& a);          // dense_launch takes the kernel that reads rounded inputs
+// *found (device) = 1 if one of n bf16 weights is infinite: then a.x_parts must be null
+cudaError_t bf16_any_infinite(const void* w, size_t n, int* found, cudaStream_t s);
 
 // ---------------------------------------------------------------- mixers and norms (mixers.cu)
 // x[t] = table[tok_id[t]] * scale (+ bigram row of (tok_prev[t], tok_id[t])) (+ a sinusoid of the position)

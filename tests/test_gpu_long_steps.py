@@ -126,6 +126,21 @@ def test_products_in_32_bits(native_lib, tmp_path, kind, W, ff, lengths):
     check(util, ref, cfg, tmp_path, lengths, "float32", bar=4e-6)
 
 
+def test_infinite_weight_of_a_32_bit_model(native_lib, tmp_path):
+    """A write gate's map with an infinity: the gate is its cap or minus it (the embedding's entries, which the map reads, are not 0), and every
+    token's logits are finite, in steps of more than 8 tokens as in short ones."""
+    cfg = gu.config([gu.mlstm(heads=2, dim=24, vdim=20, mlp=40)])
+    w = gu.random_weights(cfg, seed=5)
+    w["l0.mix.i"][1, 7] = np.inf
+    prompt = toks(cfg["vocab"], 20, 7)
+    assert (w["embed"][prompt, 7] != 0).all()
+    eng = engine(gu.write_model(str(tmp_path / "m"), cfg, w), "float32", 20, 1)
+    long, short = whole(eng, [prompt])[0], whole(eng, [prompt[:8]])[0]
+    eng.close()
+    want = goponex_ref.forward(cfg, w, prompt)
+    assert rows_off(long, want).max() < F32 and rows_off(short, want[:8]).max() < F32
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("W,dim,inner", [(66, 10, 34), (72, 130, 36), (1020, 20, 24), (1024, 64, 40), (1028, 12, 40), (2052, 16, 40), (4100, 16, 24)])
 def test_rows_between_products(native_lib, tmp_path, W, dim, inner, dtype):

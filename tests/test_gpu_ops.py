@@ -400,3 +400,27 @@ def test_gates_of_products(native_lib, kind, T):
     units = 2.0 ** -24 * (4.0 + (4.0 * np.minimum(np.abs(w), 100.0) if kind == "gelu" else 0.0))
     fine = np.isfinite(z64)
     assert (np.abs(got - want) <= units * np.abs(want) + 3e-39 * scale)[fine].all(), np.argwhere((np.abs(got - want) > units * np.abs(want) + 3e-39 * scale) & fine)[:5]
+
+
+@pytest.mark.parametrize("T", [8, 9, 40])
+def test_infinite_weights_and_inputs_of_products_in_32_bits(native_lib, T):
+    """What a multiply-add makes of them, and only in their own rows and columns. Inputs that are bf16 values themselves too: nothing is left of those
+    behind the leading part, and 0 times an infinite weight would be NaN."""
+    rng = np.random.default_rng(T)
+    N, K = 130, 136
+    x, w = rng.standard_normal((T, K)).astype(np.float32), rng.standard_normal((N, K)).astype(np.float32)
+    w, short = ((a.view(np.uint32) & np.uint32(0xffff0000)).view(np.float32) for a in (w, x))
+    for rows in (x, short):
+        for inf in (False, True):
+            a, b = rows.copy(), w.copy()
+            if inf:
+                b[3, 5], b[129, 135] = np.inf, -np.inf
+            if rows is x:
+                a[2, 7] = np.inf
+                a.view(np.uint32)[5, 64], a.view(np.uint32)[6, 1] = 0x7f800001, 0xff80ffff      # NaN whose leading 16 bits are those of an infinity
+            with np.errstate(invalid="ignore"):
+                want = (a.astype(np.float64)[:, None, :] * b.astype(np.float64)[None]).sum(-1)
+            got = product(native_lib, a, b)
+            assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isposinf(got), np.isposinf(want)) and np.array_equal(np.isneginf(got), np.isneginf(want))
+            fine = np.isfinite(want)
+            assert fine.sum() > (T - 3) * (N - 2) - 1 and np.abs(got[fine] - want[fine]).max() < 4e-6 * np.sqrt(K)
