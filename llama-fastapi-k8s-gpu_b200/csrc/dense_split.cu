@@ -1,8 +1,10 @@
 // 32-bit products of more than 8 tokens with bf16 weights on the 5th-generation tensor cores:
 //     Y[t][n] = epi(sum_k X[t][k] * W[n][k])      X, Y f32, W bf16 as stored.
 //
-// An f32 value is the sum of three bf16 values, exactly: its 24 significant bits cut into runs of 8 (truncated, not rounded, so that nothing
-// overflows). A product of two bf16 values is exact in f32, so X . W is three bf16 products whose terms are the terms of the 32-bit
+// An f32 value of 2^-110 and more is the sum of three bf16 values, exactly: its 24 significant bits cut into runs of 8 (truncated, not rounded, so
+// that nothing overflows; the split of Henry, Tang and Heinecke, "Leveraging the bfloat16 artificial intelligence datatype for higher-precision
+// computations", 2019). Of smaller values what lies below bf16's last subnormal bit is cut off, less than 2^-133: a row whose largest entry is
+// 2^-120 is off by 7e-5, beside larger entries it does not show. A product of two bf16 values is exact in f32, so X . W is three bf16 products whose terms are the terms of the 32-bit
 // product; only the sums round. Tensor memory sums without rounding to nearest, and over a whole K that would show; so a sum stays there for
 // 64 entries of K only (three parts, the smallest first) and is then added to a 32-bit register in the order of k, as the multiply-add kernel
 // adds single terms. Errors against 64 bits are below that kernel's (below).
@@ -13,8 +15,8 @@
 // lanes' quarters, two halves of the token columns), 8 copies, 9 matrix instructions. Four accumulators of NT columns: the products of up to
 // three K slices run ahead of the additions.
 // Bound by the copies from L2 where tiles are wide (16 + 48 KB a slice of 128 x 128) and by the length of K where a matrix has few
-// tiles. 459 tokens of two layers of 1024 (B200): ten products 1320 us as multiply-adds, 20 to 37 each here, the whole step 1830 -> 710; against 64 bits the
-// logits are off by 4.6e-7 of their norm, 1.6e-6 before.
+// tiles. 459 tokens of two layers of 1024 (B200): ten products 1320 us as multiply-adds, 20 to 37 each here, the whole step 1820 -> 550; against 64 bits the
+// logits are off by 4.8e-7 of their norm, 1.5e-6 before.
 #include "dense_tc.cuh"
 #include "quant_blocks.cuh"
 #include "tc05.cuh"
@@ -167,7 +169,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) dense_split_kernel(const __grid
 }
 
 // ---------------------------------------------------------------- inputs in three parts
-// parts[j][r][0..K), j = 0 .. 2: leading, middle and last 8 significant bits of x[rows ? rows[r] : r][0..K), 8 entries a thread. K % 8 == 0.
+// parts[j][r][0..K), j = 0 .. 2: leading, middle and last 8 significant bits (as far as bf16 reaches) of x[rows ? rows[r] : r][0..K), 8 entries a thread. K % 8 == 0.
 // Infinities and NaN stay what they are in the leading part, with zeros behind them.
 __global__ void rows_to_parts_kernel(const float* __restrict__ x, int ldx, const int* __restrict__ rows, int n_src, int T, int K, __nv_bfloat16* __restrict__ parts) {
     griddep_launch();

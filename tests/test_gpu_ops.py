@@ -424,3 +424,16 @@ def test_infinite_weights_and_inputs_of_products_in_32_bits(native_lib, T):
             assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isposinf(got), np.isposinf(want)) and np.array_equal(np.isneginf(got), np.isneginf(want))
             fine = np.isfinite(want)
             assert fine.sum() > (T - 3) * (N - 2) - 1 and np.abs(got[fine] - want[fine]).max() < 4e-6 * np.sqrt(K)
+
+
+@pytest.mark.parametrize("power", [-140, -124, -120, -116, -110, -60, 0, 60, 100])
+@pytest.mark.parametrize("T,N,K", [(9, 130, 72), (40, 128, 1024)])
+def test_scales_of_products_in_32_bits(native_lib, T, N, K, power):
+    """Sums of 64 entries, added up in 32 bits: off by 9e-8 of the result's norm. Inputs below 2^-110 lose what bf16 cannot hold, less than 2^-133 each."""
+    rng = np.random.default_rng(K + power + 200)
+    x = np.ldexp(rng.standard_normal((T, K)), power).astype(np.float32)
+    w = (np.ldexp(rng.standard_normal((N, K)), -5).astype(np.float32).view(np.uint32) & np.uint32(0xffff0000)).view(np.float32)
+    x64, w64 = x.astype(np.float64), w.astype(np.float64)
+    want, got = x64 @ w64.T, product(native_lib, x, w)
+    cut = np.ldexp(1.0, -133) * (np.abs(x64) < np.ldexp(1.0, -110)) @ np.abs(w64).T + np.ldexp(1.0, -149)
+    assert (np.linalg.norm(got - want) <= 3e-7 * np.linalg.norm(want) + np.linalg.norm(cut)), np.linalg.norm(got - want) / np.linalg.norm(want)
