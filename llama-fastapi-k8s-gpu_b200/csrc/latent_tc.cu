@@ -10,8 +10,9 @@
 // Warps 0-3: softmax, one query a thread; 4: copies; 5: matrix instructions. The parts that are not values of this CTA are reloaded
 // while the softmax runs, and their share of the next block's scores is computed under it. The output is rescaled only when a
 // row's maximum has grown by more than 2^8 since the last time.
-// Bound by the chain of a block's scores, softmax and sums: six warps an SM, tensor pipe busy for 18 % of the time, issue slots for 13 % (ncu).
-// 2048 tokens, 16 heads, rows of 512 + 64 (B200): 1640 us a layer with mma.sync, 248 here, 210 with the issue loops run by whole warps.
+// Bound by the chain of a block's scores, softmax and sums: six warps an SM, tensor pipe busy for 26 to 30 % of the time, issue slots for 18 % (ncu).
+// 2048 tokens, 16 heads, rows of 512 + 64 (B200): 1640 us a layer with mma.sync, 207 here (the rotated parts of the queries: below); rows of 512,
+// nothing rotated: 170.
 #include "kernels.h"
 #include "latent_dev.cuh"
 #include "layered.h"

@@ -1134,9 +1134,9 @@ __global__ void __launch_bounds__(SCAN_CH) scan_recurrence_chan_kernel(ScanArgs 
 // and C rows, ordered so that a lane's states are one read) arrive in shared memory as asynchronous copies two blocks ahead; softplus(dt +
 // bias) and silu(z) are applied once per entry, a block ahead. Every global access is a run of the CTA's channels. What a token does to a
 // channel is the same wherever the token stands in a step.
-// Bound by the exponentials (the special-function unit's 16 a cycle and SM: 60 us for 2048 tokens of 8192 channels with 16 states) and by
-// the latency of what surrounds them, up to four warps a scheduler. The same on a B200: 995 us with a lane per state, 416 with four lanes and
-// softplus and gate in a phase of their own, 273 here. (The decays stay expf: one approximate power of two each takes 248 us, but errs to one
+// Bound by its instructions and shared reads: 2048 tokens of 8192 channels with 16 states keep 70 % of the issue slots and 57 % of the shared-memory
+// pipe busy (ncu), three to four warps a scheduler; the exponentials alone would take 70 us. The same on a B200: 995 us with a lane per state, 416 with
+// four lanes and softplus and gate in a phase of their own, 273 here. (The decays stay expf: one approximate power of two each takes 248 us, but errs to one
 // side, and the states sum that up. Step sizes 0.01 to 0.02, A 0.5 to 1, 4000 tokens: output off by 6.8e-7 of its norm, 1.7e-7 here; step sizes
 // 0.001 to 0.1, A 1 to 16, 2048 tokens: 1.19e-7 and 0.84e-7.)
 constexpr int SC_CH = 64, SC_TB = 16;
@@ -1372,8 +1372,8 @@ __global__ void __launch_bounds__(MG_TB) matrix_mem_gates_kernel(MatrixMemArgs a
 // block is computed) and for the partial read-outs of the row groups, which all threads then sum in a fixed order.
 // The CTA past the last columns carries the normaliser n as one column whose v is 1, and leaves n . q; the division by it waits for
 // matrix_mem_out_kernel.
-// Bound by multiply-adds (24 pairs a token and warp, two cycles each) and shared reads (18 cycles a token and warp, eight warps a pipe) about alike,
-// and by their latency with two warps a scheduler. A 2048-token prompt of 16 heads of 128 x 256 (B200): 966 us with one column a thread, 428 with two columns of 16 rows
+// Bound by multiply-adds (24 pairs a token and warp, two cycles each; 31 % of the pipe's instruction rate) and shared reads (18 cycles a token and
+// warp, eight warps a pipe; 44 % of its rate), and by their latency with two warps a scheduler (issue slots 52 %). A 2048-token prompt of 16 heads of 128 x 256 (B200): 966 us with one column a thread, 428 with two columns of 16 rows
 // and one warp a scheduler, 315 here (four columns a thread and one warp: 400; two tokens side by side, single multiply-adds: the same).
 constexpr int MM_ROWS = 8, MM_COLS = 32, MM_TB = 16, MM_MAX_D = 256;      // (16 warps at most)
 __global__ void __launch_bounds__(512, 1) matrix_mem_kernel(MatrixMemArgs a, RaggedDev r) {

@@ -8,7 +8,7 @@
 // of 64 columns in 128-byte-swizzled rows, two stages). Tensor memory holds the output (128 columns), two score tiles (2 x 128) and the two
 // halves of the probabilities (64 + 64), which are the A operand of the second product. The next block's scores are computed while
 // this one's softmax runs. Eight softmax warps, two threads a query row with 64 key columns each (capped scores take three special-function
-// operations a score; that unit is busy for 35 % of 2048 tokens' time, the tensor pipe for 23 %: what bounds the kernel is the chain of a block, and
+// operations a score; that unit is busy for 35 % of 2048 tokens' time, the tensor pipe for 25 %: what bounds the kernel is the chain of a block, and
 // 256 CTAs of unequal length on 148 SMs); they exchange their maxima through shared memory. The output is rescaled only
 // when a row's maximum has grown by more than 2^8.
 // 2048 tokens (B200): 16 capped heads of 128, 300 us a layer with mma.sync, 65 here; 32 heads of 128 over a window of 1024 keys, 326 and 92.
