@@ -254,6 +254,7 @@ __device__ __forceinline__ void sample_body(float* logits, int V, const SamplePa
         }
     }
     if (t == 0) {
+        if (result < 0 || result >= V) result = 0;      // nothing above -infinity, or NaN among the candidates: the next step reads this token's embedding
         *out_token = result;
         if (out_token2) *out_token2 = result;
         *next_token_ptr = result;

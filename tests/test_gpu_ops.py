@@ -437,3 +437,21 @@ def test_scales_of_products_in_32_bits(native_lib, T, N, K, power):
     want, got = x64 @ w64.T, product(native_lib, x, w)
     cut = np.ldexp(1.0, -133) * (np.abs(x64) < np.ldexp(1.0, -110)) @ np.abs(w64).T + np.ldexp(1.0, -149)
     assert (np.linalg.norm(got - want) <= 3e-7 * np.linalg.norm(want) + np.linalg.norm(cut)), np.linalg.norm(got - want) / np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("V", [203, 4096])
+@pytest.mark.parametrize("kind", ["-inf", "nan", "nan_in_front", "one_number"])
+def test_sampled_tokens_are_ids_whatever_the_logits(native_lib, kind, V):
+    """The token's embedding is read by the next step without the host in between: rows with nothing above -infinity, or NaN among the candidates, give an id
+    of the vocabulary too (a greedy row of -infinity the first, as an argmax)."""
+    logits = np.full(V, -np.inf if kind == "-inf" else np.nan, np.float32)
+    if kind == "nan_in_front":
+        logits[V // 2:] = np.linspace(-3, 3, V - V // 2)
+    if kind == "one_number":
+        logits[V - 1] = -7.0
+    for kw in (dict(temperature=0.0, repeat_penalty=1.0), dict(temperature=0.0), dict(top_k=5), dict(top_k=1000, top_p=1.0, min_p=0.0), dict(top_k=7, temperature=2.0)):
+        for u in (0.0, 0.5, 0.999999):
+            got = _sample(native_lib, logits, [3, 5], u, **kw)
+            assert 0 <= got < V
+            if kw.get("temperature") == 0.0:
+                assert got == {"-inf": 0, "nan": 0}.get(kind, V - 1)
