@@ -37,6 +37,20 @@ inline cudaError_t launch_chain(void (*k)(KArgs...), dim3 grid, dim3 block, size
     return cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...);
 }
 
+// the same in clusters of `cluster` neighbouring CTAs
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_chain_cluster(void (*k)(KArgs...), int cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cluster; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = g_chain_pdl ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...);
+}
+
 // Launches inside this scope carry no dependent-launch attribute: the kernel starts when its predecessor has ended, so its
 // CTAs are spread over all SMs. For long-running latency-bound kernels with few CTAs (recurrences over a prompt).
 struct PlainLaunch {

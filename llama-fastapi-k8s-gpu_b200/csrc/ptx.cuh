@@ -39,17 +39,17 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // in the host-visible error word and carries on with garbage instead of hanging the GPU; every
 // engine call checks that word after it synchronises and fails loudly.
 // try_wait already suspends the thread for a hardware time slice.
+__device__ __forceinline__ void mbar_give_up(uint32_t parity, unsigned int* err, unsigned int code, unsigned int info) {
+    if (err) {          // plain stores: the words live in host memory. [0] code [1] block [2] thread [3] info [4] parity
+        volatile unsigned int* e = reinterpret_cast<volatile unsigned int*>(err);
+        if (e[0] == 0) { e[1] = blockIdx.x; e[2] = threadIdx.x; e[3] = info; e[4] = parity; e[0] = code; }
+    }
+}
 __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, unsigned int* err, unsigned int code,
                                           unsigned int info = 0) {
     uint32_t spins = 0;
     while (!mbar_try_wait(bar, parity)) {
-        if (++spins > (1u << 22)) {
-            if (err) {          // plain stores: the words live in host memory. [0] code [1] block [2] thread [3] info [4] parity
-                volatile unsigned int* e = reinterpret_cast<volatile unsigned int*>(err);
-                if (e[0] == 0) { e[1] = blockIdx.x; e[2] = threadIdx.x; e[3] = info; e[4] = parity; e[0] = code; }
-            }
-            return;
-        }
+        if (++spins > (1u << 22)) { mbar_give_up(parity, err, code, info); return; }
     }
 }
 // The wait of a loop that a whole warp runs while one lane issues copies or products. The lanes leave it together: what is issued next
@@ -95,6 +95,24 @@ __device__ __forceinline__ bool elect_one() {
 }
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
+
+// ---- thread-block clusters: all threads of all CTAs meet (ordering nothing but what a fence before it orders); an address in CTA `rank`'s shared memory; an arrival at a barrier there (ordered like one at
+// home: with a release to the whole cluster it held its warp for 1500 cycles. What precedes it must have completed: reads, by what depends on them)
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ uint32_t cluster_address(uint32_t own, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(own), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// 16 bytes into another CTA's shared memory, counted by a barrier there
+__device__ __forceinline__ void st_async_16(uint32_t to, const uint32_t* v, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+                 ::"r"(to), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(bar) : "memory");
 }
 
 // timeline records (debugging aid, B2_TIMELINE=1): slot 0 keeps the earliest time, the others the latest

@@ -91,6 +91,12 @@ def test_latent_attention_of_long_steps(native_lib, tmp_path, kind, rank, heads,
     check(fu, fazovik_ref, fu.config(layers), tmp_path, lengths, "bfloat16")
 
 
+# pairs of CTAs with rotated parts of their own (half of 64 columns each, and fewer), and sizes that leave two stages of values, one of the rotated parts
+@pytest.mark.parametrize("rank,rot,lengths", [(512, 64, [300, 129, 2]), (512, 48, [64, 257]), (512, 16, [1, 65]), (256, 256, [257]), (192, 384, [385]), (64, 512, [129, 200])])
+def test_rotated_parts_of_latent_attention(native_lib, tmp_path, rank, rot, lengths):
+    check(fu, fazovik_ref, fu.config([fu.rotated(heads=3, rank=rank, dim=24, vdim=16, rot_dim=rot)]), tmp_path, lengths, "bfloat16")
+
+
 @pytest.mark.parametrize("rank,heads", [(64, 3), (128, 1), (512, 16)])
 @pytest.mark.parametrize("kind", ["plain", "rotated"])
 def test_latent_attention_of_one_token_of_every_sequence(native_lib, tmp_path, kind, rank, heads):
