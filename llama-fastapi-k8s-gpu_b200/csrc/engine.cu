@@ -572,6 +572,18 @@ static int record_step(b2_engine* e, Slot& s, GraphKind k, bool pdl) {
     return forward_launches(e, s, head, samp, pdl, nullptr);
 }
 
+// A token set on the host (b2_seq_set_token) enters the slot's registers with the next step that reads them: a batched step takes its slots' tokens
+// along with its first kernel (32 launches of their own took 140 of a step's 760 us), everything else asks for them here.
+__global__ void set_ints_kernel(int* ints, int tok, int pos) { if (tok >= 0) ints[0] = tok; ints[1] = pos; }
+static int enter_set_token(b2_engine* e, Slot& s) {
+    if (s.set_token < 0) return B2_OK;
+    set_ints_kernel<<<1, 1, 0, e->stream>>>(s.ints, s.set_token, s.n_past);
+    CK(cudaGetLastError());
+    e->launches++;
+    s.set_token = -1;
+    return B2_OK;
+}
+
 // run one step of kind k for slot s, through a captured graph when enabled
 static int run_step(b2_engine* e, Slot& s, GraphKind k) {
     s.logits_view = s.logits;
@@ -691,6 +703,7 @@ extern "C" int b2_seq_begin(b2_engine* e, int slot, int n_past, const int32_t* h
     u.has_uniform = n_uni > 0;
     if (n_uni) u.uniform = uni[0];
     if ((rc = seq_update(e, slot, u))) return rc;
+    s.set_token = -1;
     if (n_uni > 1) {
         CK(cudaMemcpyAsync(s.uniforms, uni, sizeof(double) * n_uni, cudaMemcpyHostToDevice, e->stream));
         CK(cudaStreamSynchronize(e->stream));
@@ -802,6 +815,7 @@ extern "C" int b2_prefill(b2_engine* e, int slot, const int32_t* tokens, int n) 
     for (int i = 0; i < n; i++)
         if (tokens[i] < 0 || tokens[i] >= e->cfg.n_vocab) return fail(B2_ERR_ARG, "token id out of range");
     CK(cudaSetDevice(e->cfg.device));
+    if ((rc = enter_set_token(e, s))) return rc;
     CK(cudaMemcpyAsync(s.prompt, tokens, sizeof(int) * n, cudaMemcpyHostToDevice, e->stream));
     if (e->gemm_ok && n >= e->prefill_min) {
         // tensor-core path: all layers for up to PF_T tokens at a time, then the output head for the last token only
@@ -831,7 +845,6 @@ extern "C" int b2_prefill(b2_engine* e, int slot, const int32_t* tokens, int n) 
     return B2_OK;
 }
 
-__global__ void set_ints_kernel(int* ints, int tok, int pos) { if (tok >= 0) ints[0] = tok; ints[1] = pos; }
 
 // enqueue: sample from the slot's logit buffer (the token at position n_past - 1 was the last one evaluated); the token
 // is in e->slot_token once the stream has been synchronised
@@ -849,6 +862,7 @@ extern "C" int b2_sample(b2_engine* e, int slot, int32_t* out) {
     std::lock_guard<std::mutex> lk(e->mu);
     Slot& s = e->slots[slot];
     CK(cudaSetDevice(e->cfg.device));
+    if ((rc = enter_set_token(e, s))) return rc;
     if ((rc = sample_enqueue(e, s))) return rc;
     CK(cudaStreamSynchronize(e->stream));
     if (out) *out = e->slot_token[slot];
@@ -872,14 +886,15 @@ static int ensure_batch_workspace(b2_engine* e) {
 // tensor-core GEMM; attention and sampling run one CTA group per sequence from the per-slot device tables.
 // Enqueued kernel by kernel. Captured per list of slots, 8 steps of 32 sequences (4 layers of 4096) took 6580 us instead of 6750; but the list
 // changes whenever a chat starts or ends, and lists that live for three steps cost 5150 us instead of 4740 (16 layers: 16600 and 15600).
-static int batch_step(b2_engine* e, const BatchIdx& b, int32_t* tokens_out) {
+static int batch_step(b2_engine* e, const BatchIdx& b, const BatchTokens& set, int32_t* tokens_out) {
     ChainPdl chain(e->chain_pdl && e->use_pdl);
     const b2_config& c = e->cfg;
     cudaStream_t st = e->stream;
     const int T = b.n, T_pad = (T + 15) / 16 * 16, E = c.n_embd, F = c.n_ff, hd = c.head_dim, qd = c.n_head * hd;
     int rc, np = 0;
     long ps = 0;
-    CK(embed_batch_launch(e->tok_embd.type, e->tok_embd.ptr, E, e->slot_tab, b, e->pf_x, st));
+    CK(embed_batch_launch(e->tok_embd.type, e->tok_embd.ptr, E, e->slot_tab, b, set, e->pf_x, st));
+    for (int i = 0; i < T; i++) e->slots[b.slot[i]].set_token = -1;
     e->launches++;
     for (int l = 0; l < c.n_layer; l++) {
         Layer& L = e->layers[l];
@@ -952,10 +967,14 @@ extern "C" int b2_decode(b2_engine* e, const int32_t* slots, int n, int32_t* out
         int rc = ensure_batch_workspace(e); if (rc) return rc;
         for (int i0 = 0; i0 < n; i0 += BATCH_MAX) {
             BatchIdx b = {};
+            BatchTokens set;
             b.n = n - i0 < BATCH_MAX ? n - i0 : BATCH_MAX;
-            for (int i = 0; i < b.n; i++) b.slot[i] = slots[i0 + i];
+            for (int i = 0; i < b.n; i++) {
+                const Slot& s = e->slots[slots[i0 + i]];
+                b.slot[i] = slots[i0 + i]; set.token[i] = s.set_token; set.pos[i] = s.n_past;
+            }
             if ((size_t)b.n * e->cfg.n_vocab > e->pf_part_floats) return fail(B2_ERR_UNSUPPORTED, "vocabulary too large for the batch workspace");
-            if ((rc = batch_step(e, b, e->pinned + i0))) return rc;
+            if ((rc = batch_step(e, b, set, e->pinned + i0))) return rc;
             // logits of this step stay in the batch output until the next GEMM call reuses the buffer
             for (int i = 0; i < b.n; i++) e->slots[b.slot[i]].logits_view = e->pf_part + (size_t)i * e->cfg.n_vocab;
         }
@@ -963,7 +982,8 @@ extern "C" int b2_decode(b2_engine* e, const int32_t* slots, int n, int32_t* out
     } else {
         for (int i = 0; i < n; i++) {
             Slot& s = e->slots[slots[i]];
-            int rc = run_step(e, s, GK_DECODE);
+            int rc = enter_set_token(e, s);
+            if (!rc) rc = run_step(e, s, GK_DECODE);
             if (rc) return rc;
             s.n_past += 1;
             s.n_sampled += 1;
@@ -983,6 +1003,7 @@ extern "C" int b2_decode_n(b2_engine* e, int slot, int n, int32_t* out) {
     if (n <= 0) return fail(B2_ERR_ARG, "n must be positive");
     if (s.n_past + n > e->cfg.n_ctx) return fail(B2_ERR_ARG, "context window full");
     CK(cudaSetDevice(e->cfg.device));
+    if ((rc = enter_set_token(e, s))) return rc;
     for (int i = 0; i < n; i++) {
         if (e->tl && i == n - 1) {      // debugging aid: record the last step of the call
             std::vector<unsigned long long> init(4 * 1024, 0ull);
@@ -1042,6 +1063,7 @@ extern "C" int b2_seq_rewind(b2_engine* e, int slot, int n_keep, int32_t pending
     s.n_sampled = s.n_sampled > dropped ? s.n_sampled - dropped : 0;
     u.ints[0] = u.ints[2] = pending; u.ints[1] = n_keep; u.ints[3] = s.n_sampled; u.n_ints = 4;
     if ((rc = seq_update(e, slot, u))) return rc;
+    s.set_token = -1;
     s.n_past = n_keep;
     return B2_OK;
 }
@@ -1050,12 +1072,12 @@ extern "C" int b2_seq_set_token(b2_engine* e, int slot, int32_t token) {
     int rc = check_slot(e, slot); if (rc) return rc;
     std::lock_guard<std::mutex> lk(e->mu);
     if (token < 0 || token >= e->cfg.n_vocab) return fail(B2_ERR_ARG, "token id out of range");
-    CK(cudaSetDevice(e->cfg.device));
     Slot& s = e->slots[slot];
-    set_ints_kernel<<<1, 1, 0, e->stream>>>(s.ints, token, s.n_past);
-    e->launches++;
-    CK(cudaGetLastError());
-    return B2_OK;
+    s.set_token = token;
+    // engines without batched steps: at once, under the caller's way to the step (ahead of the step itself, a single chat's token took 1.4 us longer)
+    if (!e->layered && e->gemm_ok && (int)e->slots.size() >= e->batch_min) return B2_OK;
+    CK(cudaSetDevice(e->cfg.device));
+    return enter_set_token(e, s);
 }
 
 extern "C" int b2_forward_pending(b2_engine* e, int slot) {
@@ -1065,8 +1087,10 @@ extern "C" int b2_forward_pending(b2_engine* e, int slot) {
     Slot& s = e->slots[slot];
     if (s.n_past + 1 > e->cfg.n_ctx) return fail(B2_ERR_ARG, "context window full");
     CK(cudaSetDevice(e->cfg.device));
-    set_ints_kernel<<<1, 1, 0, e->stream>>>(s.ints, -1, s.n_past);
+    set_ints_kernel<<<1, 1, 0, e->stream>>>(s.ints, s.set_token, s.n_past);
+    CK(cudaGetLastError());
     e->launches++;
+    s.set_token = -1;
     rc = run_step(e, s, GK_FWD);
     if (rc) return rc;
     CK(cudaStreamSynchronize(e->stream));
@@ -1132,6 +1156,7 @@ extern "C" int b2_profile_decode_step(b2_engine* e, int slot, float* ms, int32_t
     Slot& s = e->slots[slot];
     if (s.n_past + 1 > e->cfg.n_ctx) return fail(B2_ERR_ARG, "context window full");
     CK(cudaSetDevice(e->cfg.device));
+    if ((rc = enter_set_token(e, s))) return rc;
     KindTimer kt;
     rc = forward_launches(e, s, true, true, false, &kt);
     if (rc) return rc;

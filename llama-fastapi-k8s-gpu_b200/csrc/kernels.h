@@ -137,6 +137,7 @@ struct SlotDev {              // one entry per sequence slot, device-resident ta
 };
 constexpr int BATCH_MAX = 64;
 struct BatchIdx { int n; int slot[BATCH_MAX]; };   // passed by value: which slots take part in this step
+struct BatchTokens { int token[BATCH_MAX], pos[BATCH_MAX]; };      // the same: tokens the caller has set (-1: the slot's own) and their positions
 
 // ---------------------------------------------------------------- flash-decode (attention.cu)
 struct AttnParams {
@@ -219,7 +220,7 @@ cudaError_t attn_prefill_launch(const __half* qh, const __half* k_cache, const _
 // gate|up parts [T][2F] -> h = f16(silu(gate) * up) in operand order
 cudaError_t silu_mul_half_launch(const float* parts, int n_parts, long part_stride, int F, int T, int T_pad, __half* h, cudaStream_t s);
 // batched decode step (one token per slot of b)
-cudaError_t embed_batch_launch(int type, const uint8_t* table, int K, const SlotDev* tab, const BatchIdx& b, float* x, cudaStream_t s);
+cudaError_t embed_batch_launch(int type, const uint8_t* table, int K, const SlotDev* tab, const BatchIdx& b, const BatchTokens& set, float* x, cudaStream_t s);
 cudaError_t rope_store_batch_launch(const float* parts, int n_parts, long part_stride, const SlotDev* tab, const BatchIdx& b,
                                     int n_head, int n_kv, int hd, int bt, const float* rope_freq, float* q_out,
                                     __half* k_cache, __half* v_cache, cudaStream_t s);

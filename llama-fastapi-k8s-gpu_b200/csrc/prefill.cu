@@ -257,18 +257,21 @@ cudaError_t silu_mul_half_launch(const float* parts, int n_parts, long part_stri
 }
 
 // ---------------------------------------------------------------- batched decode step: one token per slot
-__global__ void embed_batch_kernel(int type, const uint8_t* table, int K, const SlotDev* tab, const BatchIdx b, float* x) {
+// (a token that the caller has set, and its position, go into the slot's registers here)
+__global__ void embed_batch_kernel(int type, const uint8_t* table, int K, const SlotDev* tab, const BatchIdx b, const BatchTokens set, float* x) {
     griddep_launch();
     griddep_wait();
-    const int t = blockIdx.x;
-    const int tok = tab[b.slot[t]].ints[0];
+    const int t = blockIdx.x, given = set.token[t];
+    int* ints = tab[b.slot[t]].ints;
+    const int tok = given >= 0 ? given : ints[0];
+    if (given >= 0 && threadIdx.x == 0) { ints[0] = given; ints[1] = set.pos[t]; }
     const int be = block_elems(type), bb = block_bytes(type);
     const uint8_t* row = table + (size_t)tok * (K / be) * bb;
     for (int i = threadIdx.x; i < K; i += blockDim.x)
         x[(size_t)t * K + i] = dequant_elem(type, row + (size_t)(i / be) * bb, i % be);
 }
-cudaError_t embed_batch_launch(int type, const uint8_t* table, int K, const SlotDev* tab, const BatchIdx& b, float* x, cudaStream_t s) {
-    return launch_chain(embed_batch_kernel, dim3(b.n), dim3(1024), 0, s, type, table, K, tab, b, x);
+cudaError_t embed_batch_launch(int type, const uint8_t* table, int K, const SlotDev* tab, const BatchIdx& b, const BatchTokens& set, float* x, cudaStream_t s) {
+    return launch_chain(embed_batch_kernel, dim3(b.n), dim3(1024), 0, s, type, table, K, tab, b, set, x);
 }
 
 // like rope_store, but row t belongs to slot b.slot[t] at that slot's own position; q stays float32 for flash-decode

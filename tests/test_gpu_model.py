@@ -332,3 +332,40 @@ def test_long_context_uses_more_attention_splits_and_matches_oracle(native_lib, 
             assert t2 == int(np.argmax(nxt))
         tok = t2
     eng.close()
+
+
+@pytest.mark.parametrize("how", ["batch", "batch_of_others", "two", "decode_n", "forward", "twice", "rewind"])
+def test_a_set_token_enters_the_next_step_whichever_it_is(native_lib, tmp_models, how):
+    """A token set on the host reaches batched steps (with and without set tokens beside it), single ones, runs of steps and plain forward
+    passes; the last one set counts, and a rewind's token replaces it."""
+    from oracle.llama_ref import RefModel
+    path = _model(tmp_models, "tiny128", "Q4_0", 2)
+    ref = RefModel(path).forward(TOKENS[:13])
+    eng = _engine(path, max_seqs=5)
+    for s in range(5):
+        eng.ensure_pages(s, 32)
+        eng.seq_begin(s, 0, [], _greedy())
+        eng.prefill(s, TOKENS[:12])
+    other = (TOKENS[12] + 1) % 700
+    eng.set_token(0, other)
+    if how != "rewind":
+        eng.set_token(0, TOKENS[12])
+    if how.startswith("batch"):
+        for s in range(1, 5):
+            eng.set_token(s, TOKENS[12]) if how == "batch" else eng.sample(s)
+        eng.decode([3, 0, 1, 2])
+    elif how == "two":
+        eng.set_token(1, TOKENS[12])
+        eng.decode([0, 1])
+    elif how == "decode_n":
+        eng.decode_n(0, 1)
+    elif how == "rewind":
+        eng.rewind(0, 12, TOKENS[12], TOKENS[:12])
+        eng.decode([0])
+    else:
+        eng.forward_pending(0)
+    assert np.abs(eng.logits(0) - ref[12]).max() <= LOGIT_TOL
+    if how == "batch":
+        eng.decode_n(4, 1)                                     # its token was set and stayed set while the others stepped
+        assert np.abs(eng.logits(4) - ref[12]).max() <= LOGIT_TOL
+    eng.close()
