@@ -2,6 +2,7 @@
 
   lib/libb200gguf.so       CUDA kernels + C ABI (include/b200_gguf.h), nvcc, sm_100a only
   lib/libb200_hosttest.so  host build of the block arithmetic (CPU self-test, g++)
+  lib/libb200_pylists.so   Python lists to C arrays (g++, Python's headers; without them the package converts in Python)
 
 nvcc cross-compiles without a GPU; the .so files are git-ignored but travel to the GPU box.
 """
@@ -10,6 +11,7 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -69,6 +71,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
     hsrc = os.path.join(CSRC, "host_selftest.cpp")
     if force or _newer(host, [hsrc, os.path.join(CSRC, "quant_blocks.cuh"), os.path.join(CSRC, "gemm_ring.h"), os.path.join(CSRC, "per_device.h")]):
         subprocess.run(["g++", "-O2", "-ffp-contract=off", "-fPIC", "-shared", hsrc, "-o", host], check=True)
+    lists, lsrc, include = os.path.join(LIB, "libb200_pylists.so"), os.path.join(CSRC, "py_lists.cpp"), sysconfig.get_paths()["include"]
+    if os.path.exists(os.path.join(include, "Python.h")) and (force or _newer(lists, [lsrc])):
+        subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-I", include, lsrc, "-o", lists], check=True)
     return out
 
 

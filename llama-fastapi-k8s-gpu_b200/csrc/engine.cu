@@ -115,6 +115,7 @@ static int engine_create_impl(b2_engine* e, const b2_config* c) {
     CK(cudaEventCreate(&e->ev1));
     CK(cudaMallocHost(&e->pinned, sizeof(int32_t) * (size_t)(c->max_seqs + c->n_ctx + 16)));
     CK(cudaMallocHost(&e->slot_token, sizeof(int32_t) * (size_t)c->max_seqs));
+    CK(cudaMallocHost(&e->logits_stage, sizeof(float) * (size_t)c->n_vocab));
     // KV pool: [layer][block][kv_head][token][dim] f16
     e->layer_kv_elems = (size_t)c->kv_num_blocks * c->n_head_kv * c->kv_block_tokens * c->head_dim;
     size_t kvb = e->layer_kv_elems * c->n_layer * sizeof(__half);
@@ -210,6 +211,7 @@ extern "C" int b2_engine_destroy(b2_engine* e) {
     cudaFree(e->slot_tab); cudaFree(e->bd_q); cudaFree(e->bd_att); cudaFree(e->bd_scratch); cudaFree(e->bd_counters);
     if (e->pinned) cudaFreeHost(e->pinned);
     if (e->slot_token) cudaFreeHost(e->slot_token);
+    if (e->logits_stage) cudaFreeHost(e->logits_stage);
     if (e->ev0) cudaEventDestroy(e->ev0);
     if (e->ev1) cudaEventDestroy(e->ev1);
     if (e->stream) cudaStreamDestroy(e->stream);
@@ -1104,8 +1106,12 @@ extern "C" int b2_get_logits(b2_engine* e, int slot, float* out) {
     std::lock_guard<std::mutex> lk(e->mu);
     CK(cudaSetDevice(e->cfg.device));
     const Slot& s = e->slots[slot];
-    CK(cudaMemcpyAsync(out, s.logits_view ? s.logits_view : s.logits, sizeof(float) * e->cfg.n_vocab, cudaMemcpyDeviceToHost, e->stream));
+    const size_t bytes = sizeof(float) * e->cfg.n_vocab;
+    // through pinned memory of the engine's own (straight into pageable memory, 32000 logits took 24 us)
+    if (!e->logits_stage) CK(cudaMallocHost(&e->logits_stage, bytes));      // (layer-list engines: b2_step hands logits out itself)
+    CK(cudaMemcpyAsync(e->logits_stage, s.logits_view ? s.logits_view : s.logits, bytes, cudaMemcpyDeviceToHost, e->stream));
     CK(cudaStreamSynchronize(e->stream));
+    memcpy(out, e->logits_stage, bytes);
     return B2_OK;
 }
 

@@ -77,6 +77,7 @@ struct b2_engine {
     int n_resets = 0;
     int32_t* pinned = nullptr;     // host memory that kernels write too: sampled tokens arrive here without a copy of their own
     int32_t* slot_token = nullptr; // the same, one entry per slot: written by the slot's (captured) sampler launches
+    float* logits_stage = nullptr; // pinned [n_vocab]
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int64_t launches = 0, weight_bytes = 0, kv_bytes = 0;
     bool use_graph = true, use_pdl = true, act2 = true, finalized = false, chain_pdl = true;

@@ -126,6 +126,7 @@ struct LayeredModel {
     int* meta_host = nullptr;          // pinned
     size_t meta_ints = 0;              // of either copy of a step's description
     float* logits_host = nullptr;      // pinned [LOGIT_ROWS][n_vocab]
+    cudaEvent_t logits_here = nullptr; // the copy of wanted rows into it has ended
     float* trace = nullptr;            // [n_layer][max_step_tokens][n_embd] when tracing
     int last_T = 0;
     bool profile = false;
@@ -780,6 +781,7 @@ int layered_finalize(b2_engine* e) {
     if ((rc = dev_alloc(m, (void**)&m->meta, n_meta * 4))) return rc;
     CK(cudaMallocHost(&m->meta_host, n_meta * 4));
     CK(cudaMallocHost(&m->logits_host, (size_t)LOGIT_ROWS * V * 4));
+    CK(cudaEventCreateWithFlags(&m->logits_here, cudaEventDisableTiming));
     {
         std::vector<int*> tabs(S);
         for (int i = 0; i < S; i++) tabs[i] = e->slots[i].block_table;
@@ -813,6 +815,7 @@ void layered_destroy(b2_engine* e) {
     for (void* p : m->owned) cudaFree(p);
     if (m->meta_host) cudaFreeHost(m->meta_host);
     if (m->logits_host) cudaFreeHost(m->logits_host);
+    if (m->logits_here) cudaEventDestroy(m->logits_here);
     for (auto& pe : m->prof_ev) { cudaEventDestroy(pe.second.first); cudaEventDestroy(pe.second.second); }
     for (auto& kv : m->graphs) if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
     delete m;
@@ -1804,6 +1807,7 @@ extern "C" int b2_step(b2_engine* e, int n_entries, const int32_t* slots, const 
     const int W = c.n_embd, V = c.n_vocab;
     int rc;
     // logits of rows [r0, r0 + nr): final norm, head, wanted rows to the pinned buffer, sampled rows to their slots and sampled there
+    bool in_graph = false;
     auto head_chunk = [&](int r0, int nr) -> int {
         {
             StepProfiler sp(m, st, 5);
@@ -1820,7 +1824,10 @@ extern "C" int b2_step(b2_engine* e, int n_entries, const int32_t* slots, const 
         int rc2 = dense(e, m, m->head, m->rows, W, m->logits, V, nr, nullptr, EPI_NONE, 6, &hs);
         if (rc2) return rc2;
         const int n_w = std::max(0, std::min(n_want - r0, nr));
-        if (n_w > 0) CK(cudaMemcpyAsync(m->logits_host, m->logits, (size_t)n_w * V * 4, cudaMemcpyDeviceToHost, st));
+        if (n_w > 0) {
+            CK(cudaMemcpyAsync(m->logits_host, m->logits, (size_t)n_w * V * 4, cudaMemcpyDeviceToHost, st));
+            if (!in_graph) CK(cudaEventRecord(m->logits_here, st));
+        }
         SampleRows sr = {};
         for (int i = 0; i < n; i++)
             if (samp_row[i] >= r0 && samp_row[i] < r0 + nr) { sr.entry[sr.n] = i; sr.row[sr.n++] = samp_row[i] - r0; }
@@ -1861,7 +1868,9 @@ extern "C" int b2_step(b2_engine* e, int n_entries, const int32_t* slots, const 
                 const int64_t before = e->launches;
                 cudaGraph_t g = nullptr;
                 CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+                in_graph = true;
                 const int crc = forward_once();
+                in_graph = false;
                 const cudaError_t ce = cudaStreamEndCapture(st, &g);
                 sg.n_launch = (int)(e->launches - before);
                 e->launches = before;
@@ -1885,7 +1894,8 @@ extern "C" int b2_step(b2_engine* e, int n_entries, const int32_t* slots, const 
     for (int i = 0; i < n; i++) if (samp_row[i] >= 0) e->slots[slots[i]].logits_view = e->slots[slots[i]].logits;
     if (n_rows <= LOGIT_ROWS) {
         if (n_want > 0) {
-            CK(cudaStreamSynchronize(st));
+            // (to the caller while the sampler runs, unless a graph has hidden where the copy ends)
+            CK(done ? cudaStreamSynchronize(st) : cudaEventSynchronize(m->logits_here));
             memcpy(host_logits, m->logits_host, (size_t)n_want * V * 4);
         }
     } else {
@@ -1894,7 +1904,7 @@ extern "C" int b2_step(b2_engine* e, int n_entries, const int32_t* slots, const 
             if ((rc = head_chunk(r0, nr))) return rc;
             const int n_w = std::max(0, std::min(n_want - r0, nr));
             if (n_w > 0) {
-                CK(cudaStreamSynchronize(st));
+                CK(cudaEventSynchronize(m->logits_here));
                 memcpy(host_logits + (size_t)r0 * V, m->logits_host, (size_t)n_w * V * 4);
             }
         }

@@ -136,6 +136,23 @@ def load_library(path: str | None = None) -> ctypes.CDLL:
     return lib
 
 
+_lists = False
+
+
+def load_lists() -> ctypes.PyDLL | None:
+    """libb200_pylists.so: Python lists to C arrays, and a step's lists together with the call; None where it has not been built (no Python headers)."""
+    global _lists
+    if _lists is False:
+        path = os.path.join(os.path.dirname(LIB_PATH), "libb200_pylists.so")
+        lib = ctypes.PyDLL(path) if os.path.exists(path) else None
+        if lib:
+            lib.b2_py_int32s.restype, lib.b2_py_int32s.argtypes = c_int, [ctypes.py_object, c_void_p, ctypes.c_ssize_t]
+            lib.b2_py_step.restype = ctypes.py_object
+            lib.b2_py_step.argtypes = [c_void_p, c_void_p, ctypes.py_object, ctypes.py_object, ctypes.py_object, c_int, c_int, c_void_p, c_int]
+        _lists = lib
+    return _lists
+
+
 class B2Error(RuntimeError):
     pass
 

@@ -23,10 +23,15 @@ from .kv_pages import PageAllocator
 
 
 def int32s(values):
-    """A C int array of a list of token ids (or rows, slots). Filled through array.array: one call per list, where a ctypes array sets its
-    entries one by one (2048 tokens: 60 instead of 330 us, a third of a short prompt's time; a dozen cost the same either way)."""
+    """A C int array of a list of token ids (or rows, slots). Filled by native code, or through array.array: one call per list, where a ctypes array
+    sets its entries one by one (2048 tokens: 2 and 60 instead of 330 us; a dozen cost the same either way)."""
     n = len(values)
     if n > 12 and type(values) in (list, tuple):
+        lists = _cabi.load_lists()
+        if lists is not None:
+            out = (ctypes.c_int32 * n)()
+            if lists.b2_py_int32s(values, ctypes.addressof(out), n):
+                return out
         try:
             return (ctypes.c_int32 * n).from_buffer(array.array("i", values))
         except OverflowError:          # ctypes keeps the low 32 bits; the native side then checks the range
@@ -314,6 +319,7 @@ class LayeredEngine(EngineBase):
         check(self.lib.b2_engine_create_layered(ctypes.byref(cfg), descs, ctypes.byref(h)), "b2_engine_create_layered")
         self._h = h
         self.lock = threading.RLock()
+        self._lists, self._step = _cabi.load_lists(), ctypes.cast(self.lib.b2_step, ctypes.c_void_p).value
         type_ids = {"BF16": _cabi.B2_TYPE_BF16, "F32": _cabi.B2_TYPE_F32, "I32": _cabi.B2_TYPE_I32}
         try:
             for name, t in tensors.items():
@@ -339,15 +345,23 @@ class LayeredEngine(EngineBase):
         native step has more than 8 tokens and no cut leaves one token alone (such steps and tokens take kernels of their own, which
         round elsewhere)."""
         n = len(entries)
+        n_want = sum(map(len, want)) if want is not None else 0
+        logits = np.empty((n_want, self.dims.n_vocab), dtype=np.float32)
+        if self._lists is not None:
+            # the usual case, plain lists of one native step, in one call
+            sampled = self._lists.b2_py_step(self._step, self._h, entries, want, sample, _cabi.B2_STEP_MAX_ENTRIES, self.max_step_tokens,
+                                             logits.ctypes.data if n_want else None, n_want)
+            if type(sampled) is list:
+                return logits, sampled
+            if sampled is not None:
+                check(sampled, "b2_step")
         want = want if want is not None else [[] for _ in entries]
         sample = sample if sample is not None else [False] * n
-        n_want = sum(len(w) for w in want)
-        logits = np.empty((n_want, self.dims.n_vocab), dtype=np.float32)
         sampled = [None] * n
         lens = [len(toks) for _, toks in entries]
         if (0 < n <= _cabi.B2_STEP_MAX_ENTRIES and n == len(want) == len(sample) and min(lens) > 0 and sum(lens) <= self.max_step_tokens and
                 all(0 <= wi < k for w, k in zip(want, lens) for wi in w)):
-            # the usual case: one native step, whose wanted rows are the result
+            # one native step, whose wanted rows are the result
             flat, rows, at = [], [], 0
             for (_, toks), w, k in zip(entries, want, lens):
                 flat.extend(toks)
