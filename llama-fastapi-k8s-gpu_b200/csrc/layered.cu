@@ -1496,27 +1496,31 @@ static int run_layers(b2_engine* e, LayeredModel* m, const RaggedDev& r) {
     const int T = r.T, W = c.n_embd;
     const bool prenorm = c.block_style == B2_BLOCK_PRENORM_RMS;
     int rc;
-    {
+    if (m->n_table > 0) {
+        StepProfiler sp(m, st, 7);
+        CK(moe_table_launch(m->table_layers, m->n_table, m->table_experts, r.tok_id, T, st));
+        e->launches++;
+    }
+    EmbedDev embed = {};
+    embed.table = m->embed.w; embed.w_type = m->embed.type; embed.scale = c.embed_scale != 0.f ? c.embed_scale : 1.f;
+    embed.tok = r.tok_id; embed.tok_prev = r.tok_prev; embed.tok_pos = r.tok_pos; embed.turns = m->turns;
+    embed.bg.table = m->bigram.w; embed.bg.w_type = m->bigram.type;
+    embed.bg.buckets = c.bigram_buckets; embed.bg.mul_prev = c.bigram_mul_prev; embed.bg.mul_cur = c.bigram_mul_cur;
+    // parallel blocks without passes: the first boundary makes the stream itself
+    const bool embed_joins = (c.block_style == B2_BLOCK_PARALLEL_LN || c.block_style == B2_BLOCK_PARALLEL_ONE_LN) && !m->loop_x && m->layers[0].d.loop_pass == 0;
+    if (!embed_joins) {
         StepProfiler sp(m, st, 0);
-        BigramTable bg;
-        bg.table = m->bigram.w; bg.w_type = m->bigram.type; bg.buckets = c.bigram_buckets; bg.mul_prev = c.bigram_mul_prev; bg.mul_cur = c.bigram_mul_cur;
-        EmbedExtra ex;
-        ex.turns = m->turns; ex.tok_pos = r.tok_pos;
+        EmbedCopies ec;
         if (m->loop_x) {                   // the embedding output stays beside the stream for the passes' input maps
-            ex.ld_copy = 2 * W; ex.copy[0] = m->loop_x + W;
-            if (m->layers[0].d.loop_pass > 0) ex.copy[1] = m->loop_x;
+            ec.ld_copy = 2 * W; ec.copy[0] = m->loop_x + W;
+            if (m->layers[0].d.loop_pass > 0) ec.copy[1] = m->loop_x;
         }
-        CK(embed_ragged_launch(m->embed.w, m->embed.type, W, r.tok_id, T, m->x, c.embed_scale != 0.f ? c.embed_scale : 1.f, st, r.tok_prev, &bg, &ex));
+        CK(embed_ragged_launch(embed, W, T, m->x, ec, st));
         e->launches++;
         if (prenorm) {
             CK(resid_rms_norm_launch(m->x, nullptr, 0.f, m->embed_norm, 1.f, 1.f, c.norm_eps, W, T, m->x, st));
             e->launches++;
         }
-    }
-    if (m->n_table > 0) {
-        StepProfiler sp(m, st, 7);
-        CK(moe_table_launch(m->table_layers, m->n_table, m->table_experts, r.tok_id, T, st));
-        e->launches++;
     }
     // pre-norm blocks: a branch output waits in m->oL until the next norm (or the end of the layer) adds it to the stream
     // (a mixture's weighted sum is not even formed before: the same kernel adds it up)
@@ -1618,6 +1622,7 @@ static int run_layers(b2_engine* e, LayeredModel* m, const RaggedDev& r) {
             }
         };
         ParallelJoinArgs pj = {};
+        if (embed_joins) pj.embed = &embed;
         MoeJoinArgs pj_moe = {};
         auto boundary = [&]() -> int {
             StepProfiler sp(m, st, 5);

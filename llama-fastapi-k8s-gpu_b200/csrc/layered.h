@@ -95,14 +95,14 @@ struct BigramTable {           // row (prev * mul_prev + cur * mul_cur) mod buck
     const void* table = nullptr; int w_type = 0;
     int buckets = 0, mul_prev = 0, mul_cur = 0;
 };
-struct EmbedExtra {
-    const double* turns = nullptr;     // sinusoid: turns per position of pair i, [(W + 1) / 2] (entry 2i: sin, 2i + 1: cos); null: none
-    const int* tok_pos = nullptr;
-    float* copy[2] = {};               // the result also goes here (row stride ld_copy); null: not
-    int ld_copy = 0;
+struct EmbedDev {              // rows of the embedding for a step's tokens
+    const void* table; int w_type; float scale;
+    const int *tok, *tok_prev, *tok_pos;       // [T] ids, the ids before them (pairs), positions (turns)
+    BigramTable bg;
+    const double* turns;       // sinusoid: turns per position of pair i, [(W + 1) / 2] (entry 2i: sin, 2i + 1: cos); null: none
 };
-cudaError_t embed_ragged_launch(const void* table, int w_type, int W, const int* tok_id, int T, float* x, float scale, cudaStream_t s,
-                                const int* tok_prev = nullptr, const BigramTable* bigram = nullptr, const EmbedExtra* extra = nullptr);
+struct EmbedCopies { float* copy[2] = {}; int ld_copy = 0; };      // the result also goes here (row stride ld_copy); null: not
+cudaError_t embed_ragged_launch(const EmbedDev& d, int W, int T, float* x, const EmbedCopies& c, cudaStream_t s);
 // gather rows: y[i] = x[rows[i]]
 cudaError_t gather_rows_launch(const float* x, int W, const int* rows, int n, float* y, cudaStream_t s);
 
@@ -326,13 +326,14 @@ cudaError_t moe_join_launch(const MoeJoinArgs& j, float* x, float mult, const fl
 
 // Parallel blocks: x[t] += a[t] + (b[t], or a mixture's sum of expert rows); then every norm given, all of the new x[t]:
 // y = (x - mean) / sqrt(var + eps) * w + bias (bias may be null). Any part may be absent (a == b == moe == null: x stays as it is).
-// x_copy: the new stream also goes there (row stride ld_copy).
+// x_copy: the new stream also goes there (row stride ld_copy). embed: x is not read but starts here as the embedding's rows (the step's first boundary).
 struct ParallelJoinArgs {
     float* x; const float* a; const float* b; const MoeJoinArgs* moe;
     const float *w1, *b1; float* y1;
     const float *w2, *b2; float* y2;
     float eps;
     float* x_copy; int ld_copy;
+    const EmbedDev* embed;
     __nv_bfloat16 *y1_bf16, *y2_bf16;      // the norms' outputs rounded, for products that take them that way; y1, y2 may then be null
 };
 cudaError_t parallel_join_launch(const ParallelJoinArgs& a, int W, int T, cudaStream_t s);

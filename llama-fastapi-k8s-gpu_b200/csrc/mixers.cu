@@ -46,46 +46,69 @@ __device__ __forceinline__ float log_sigmoid_f(float z) { return -softplus_f(-z)
 __device__ __forceinline__ float silu_inline(float z) { return over_one_plus_exp(z, -z); }
 
 // ---------------------------------------------------------------- embedding, gather
-constexpr int EMBED_COLS = 512;      // columns per CTA
-template <typename TW>
-__global__ void embed_ragged_kernel(const TW* __restrict__ table, int W, const int* __restrict__ tok, float* __restrict__ x, float scale,
-                                    const int* __restrict__ tok_prev, BigramTable bg, EmbedExtra ex) {
-    griddep_launch();
-    griddep_wait();
-    const int t = blockIdx.x, cur = tok[t];
-    const TW* row = table + (size_t)cur * W;
-    size_t pair_row = 0;
-    if (bg.table) {
-        const int prev = tok_prev[t];
-        pair_row = prev < 0 ? bg.buckets : (size_t)(((long long)prev * bg.mul_prev + (long long)cur * bg.mul_cur) % bg.buckets);
+// Entries i .. i + N - 1 of token t's row (N: 1, or 4 from a multiple of 4 in rows on 16-byte boundaries): the table's, times the scale, plus its pair's, plus
+// its position's turns
+template <int N>
+__device__ __forceinline__ void embed_at(const EmbedDev& d, int W, int t, int i, float (&v)[N]) {
+    auto read = [&](const void* table, int type, size_t row, float (&to)[N]) {
+        if constexpr (N == 4) {
+            if (type == T_BF16) {
+                const uint2 u = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(table) + row * W + i);
+                const __nv_bfloat162 lo = *reinterpret_cast<const __nv_bfloat162*>(&u.x), hi = *reinterpret_cast<const __nv_bfloat162*>(&u.y);
+                to[0] = __low2float(lo); to[1] = __high2float(lo); to[2] = __low2float(hi); to[3] = __high2float(hi);
+            } else {
+                const float4 f = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(table) + row * W + i);
+                to[0] = f.x; to[1] = f.y; to[2] = f.z; to[3] = f.w;
+            }
+        } else to[0] = type == T_BF16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(table)[row * W + i]) : reinterpret_cast<const float*>(table)[row * W + i];
+    };
+    const int cur = d.tok[t];
+    read(d.table, d.w_type, (size_t)cur, v);
+#pragma unroll
+    for (int k = 0; k < N; k++) v[k] *= d.scale;
+    if (d.bg.table) {
+        const int prev = d.tok_prev[t];
+        float w[N];
+        read(d.bg.table, d.bg.w_type, prev < 0 ? d.bg.buckets : (size_t)(((long long)prev * d.bg.mul_prev + (long long)cur * d.bg.mul_cur) % d.bg.buckets), w);
+#pragma unroll
+        for (int k = 0; k < N; k++) v[k] += w[k];
     }
-    const int i1 = min(W, (int)(blockIdx.y + 1) * EMBED_COLS);
-    for (int i = blockIdx.y * EMBED_COLS + threadIdx.x; i < i1; i += blockDim.x) {
-        float v;
-        if constexpr (sizeof(TW) == 2) v = __bfloat162float(row[i]) * scale;
-        else v = row[i] * scale;
-        if (bg.table) {
-            const size_t j = pair_row * W + i;
-            v += bg.w_type == T_BF16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(bg.table)[j]) : reinterpret_cast<const float*>(bg.table)[j];
-        }
-        if (ex.turns) {                       // whole turns are dropped in double precision, so far positions lose nothing
-            const double a = (double)ex.tok_pos[t] * ex.turns[i >> 1];
+    if (d.turns) {                               // whole turns are dropped in double precision, so far positions lose nothing
+        const double pos = (double)d.tok_pos[t];
+#pragma unroll
+        for (int k = 0; k < N; k += 2) {
+            const double a = pos * d.turns[(i + k) >> 1];
             const float half_turns = (float)(2.0 * (a - rint(a)));
-            v += i & 1 ? cospif(half_turns) : sinpif(half_turns);
+            if constexpr (N == 1) v[0] += i & 1 ? cospif(half_turns) : sinpif(half_turns);
+            else { v[k] += sinpif(half_turns); v[k + 1] += cospif(half_turns); }
         }
-        x[(size_t)t * W + i] = v;
-        for (int k = 0; k < 2; k++) if (ex.copy[k]) ex.copy[k][(size_t)t * ex.ld_copy + i] = v;
     }
 }
-cudaError_t embed_ragged_launch(const void* table, int w_type, int W, const int* tok_id, int T, float* x, float scale, cudaStream_t s,
-                                const int* tok_prev, const BigramTable* bigram, const EmbedExtra* extra) {
-    const EmbedExtra ex = extra ? *extra : EmbedExtra{};
-    const BigramTable bg = bigram ? *bigram : BigramTable{};
-    if (bg.table && !tok_prev) return cudaErrorInvalidValue;
-    const dim3 grid(T, (W + EMBED_COLS - 1) / EMBED_COLS);
-    if (w_type == T_BF16) return launch_chain(embed_ragged_kernel<__nv_bfloat16>, grid, dim3(128), 0, s, (const __nv_bfloat16*)table, W, tok_id, x, scale, tok_prev, bg, ex);
-    if (w_type == T_F32) return launch_chain(embed_ragged_kernel<float>, grid, dim3(128), 0, s, (const float*)table, W, tok_id, x, scale, tok_prev, bg, ex);
-    return cudaErrorInvalidValue;
+static bool embed_wide(const EmbedDev& d, int W) {
+    return W % 4 == 0 && ((reinterpret_cast<uintptr_t>(d.table) | reinterpret_cast<uintptr_t>(d.bg.table)) & 15) == 0;
+}
+// N entries a thread, 256 threads a CTA. (2048 rows of 4096: one entry of two bytes a thread 20 us, 11 here. 2048 rows of 2048 with turns: both functions of a turn
+// in every warp 19 us; as part of the first norms below, embedding, experts' tables and norms take 25 us instead of 43, a chat's 7 instead of 10.)
+template <int N>
+__global__ void __launch_bounds__(256) embed_ragged_kernel(const EmbedDev d, int W, float* __restrict__ x, EmbedCopies c) {
+    griddep_launch();
+    griddep_wait();
+    const int t = blockIdx.x, i = (blockIdx.y * 256 + threadIdx.x) * N;
+    if (i >= W) return;
+    float v[N];
+    embed_at(d, W, t, i, v);
+    auto put = [&](float* to) {
+        if constexpr (N == 4) *reinterpret_cast<float4*>(to) = make_float4(v[0], v[1], v[2], v[3]);
+        else *to = v[0];
+    };
+    put(x + (size_t)t * W + i);
+    for (int k = 0; k < 2; k++) if (c.copy[k]) put(c.copy[k] + (size_t)t * c.ld_copy + i);
+}
+cudaError_t embed_ragged_launch(const EmbedDev& d, int W, int T, float* x, const EmbedCopies& c, cudaStream_t s) {
+    if (d.bg.table && !d.tok_prev) return cudaErrorInvalidValue;
+    const uintptr_t out = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(c.copy[0]) | reinterpret_cast<uintptr_t>(c.copy[1]);
+    if (embed_wide(d, W) && c.ld_copy % 4 == 0 && (out & 15) == 0) return launch_chain(embed_ragged_kernel<4>, dim3(T, (W + 1023) / 1024), dim3(256), 0, s, d, W, x, c);
+    return launch_chain(embed_ragged_kernel<1>, dim3(T, (W + 255) / 256), dim3(256), 0, s, d, W, x, c);
 }
 
 __global__ void gather_rows_kernel(const float* __restrict__ x, int W, const int* __restrict__ rows, float* __restrict__ y) {
@@ -276,11 +299,13 @@ cudaError_t layer_norm_rows_launch(const float* x, const int* rows, const float*
 // entries of a thread are read JOIN_U at a time (the stores between them would otherwise keep every read behind the last one), with an
 // expert row's number looked up once per batch. 32 rows of 2048 with two experts each: 12.1 -> 7.0 us.
 constexpr int JOIN_U = 4;
-struct ParallelJoinDev { ParallelJoinArgs a; MoeJoinArgs j; int moe; };
-template <int NT>
-__global__ void __launch_bounds__(NT) parallel_join_kernel(ParallelJoinDev p, int W) {
+struct ParallelJoinDev { ParallelJoinArgs a; MoeJoinArgs j; EmbedDev e; int moe; };
+// EMBED: the stream starts here, from the embedding. That reads nothing of a kernel before it (the step's description is a copy ahead of all kernels), so the
+// tables of the step's experts may still be made; it ends after them, since what comes next waits for this kernel alone.
+template <int NT, bool EMBED>
+__global__ void __launch_bounds__(NT) parallel_join_kernel(const __grid_constant__ ParallelJoinDev p, int W) {
     griddep_launch();
-    griddep_wait();
+    if constexpr (!EMBED) griddep_wait();
     extern __shared__ float row[];
     __shared__ float red[33];
     const ParallelJoinArgs& a = p.a;
@@ -295,7 +320,8 @@ __global__ void __launch_bounds__(NT) parallel_join_kernel(ParallelJoinDev p, in
         for (int u = 0; u < JOIN_U; u++) {
             const int i = i0 + u * NT;
             const bool in = i < W;
-            v[u] = in ? a.x[base + i] : 0.f;
+            if constexpr (EMBED) { float e[1] = {0.f}; if (in) embed_at(p.e, W, t, i, e); v[u] = e[0]; }
+            else v[u] = in ? a.x[base + i] : 0.f;
             y[u] = in && a.a ? a.a[base + i] : 0.f;
             z[u] = in && a.b ? a.b[base + i] : 0.f;
         }
@@ -320,13 +346,17 @@ __global__ void __launch_bounds__(NT) parallel_join_kernel(ParallelJoinDev p, in
         for (int u = 0; u < JOIN_U; u++) {
             const int i = i0 + u * NT;
             if (i >= W) continue;
-            if (adds) { v[u] += y[u]; a.x[base + i] = v[u]; }
+            if (adds) v[u] += y[u];
+            if (adds || EMBED) a.x[base + i] = v[u];
             if (a.x_copy) a.x_copy[(size_t)t * a.ld_copy + i] = v[u];
             row[i] = v[u];
             sum += v[u];
         }
     }
-    if (!a.w1 && !a.w2) return;
+    if (!a.w1 && !a.w2) {
+        if constexpr (EMBED) griddep_wait();
+        return;
+    }
     const float mean = block_sum(sum, red) / (float)W;
     float sq = 0.f;
     for (int i = threadIdx.x; i < W; i += NT) { const float dlt = row[i] - mean; sq = fmaf(dlt, dlt, sq); }
@@ -357,14 +387,15 @@ __global__ void __launch_bounds__(NT) parallel_join_kernel(ParallelJoinDev p, in
             }
         }
     }
+    if constexpr (EMBED) griddep_wait();
 }
 // The same for rows of at most 4096 entries on 16-byte boundaries: a thread keeps its entries (NV times four) in registers. Bound by memory:
 // 2048 rows of 2048 with two experts' rows each, both norms' outputs among 100 MB: 46 us with single reads and the row in shared memory, 34 here
 // (from the launch, which is ahead of the product before it: prompts 748 -> 732 and 1593 -> 1558). Wider rows than 4096 would not fit the registers.
-template <int NV>
-__global__ void __launch_bounds__(256) parallel_join_vec_kernel(ParallelJoinDev p, int W) {
+template <int NV, bool EMBED>
+__global__ void __launch_bounds__(256) parallel_join_vec_kernel(const __grid_constant__ ParallelJoinDev p, int W) {
     griddep_launch();
-    griddep_wait();
+    if constexpr (!EMBED) griddep_wait();
     __shared__ float red[33];
     const ParallelJoinArgs& a = p.a;
     const MoeJoinArgs& j = p.j;
@@ -376,7 +407,15 @@ __global__ void __launch_bounds__(256) parallel_join_vec_kernel(ParallelJoinDev 
     auto put = [&](float* to, int k, const float4& v) { *reinterpret_cast<float4*>(to + at(k)) = v; };
     float4 v[NV], y[NV], z[NV];
 #pragma unroll
-    for (int k = 0; k < NV; k++) { v[k] = get(a.x + base, k); y[k] = get(a.a ? a.a + base : nullptr, k); z[k] = get(a.b ? a.b + base : nullptr, k); }
+    for (int k = 0; k < NV; k++) {
+        if constexpr (EMBED) {
+            float e[4] = {0.f, 0.f, 0.f, 0.f};
+            if (at(k) < W) embed_at(p.e, W, t, at(k), e);
+            v[k] = make_float4(e[0], e[1], e[2], e[3]);
+        } else v[k] = get(a.x + base, k);
+    }
+#pragma unroll
+    for (int k = 0; k < NV; k++) { y[k] = get(a.a ? a.a + base : nullptr, k); z[k] = get(a.b ? a.b + base : nullptr, k); }
 #pragma unroll
     for (int k = 0; k < NV; k++) { y[k].x += z[k].x; y[k].y += z[k].y; y[k].z += z[k].z; y[k].w += z[k].w; }
     if (p.moe) {
@@ -404,11 +443,15 @@ __global__ void __launch_bounds__(256) parallel_join_vec_kernel(ParallelJoinDev 
 #pragma unroll
     for (int k = 0; k < NV; k++) {
         if (at(k) >= W) break;
-        if (adds) { v[k].x += y[k].x; v[k].y += y[k].y; v[k].z += y[k].z; v[k].w += y[k].w; put(a.x + base, k, v[k]); }
+        if (adds) { v[k].x += y[k].x; v[k].y += y[k].y; v[k].z += y[k].z; v[k].w += y[k].w; }
+        if (adds || EMBED) put(a.x + base, k, v[k]);
         if (a.x_copy) put(a.x_copy + (size_t)t * a.ld_copy, k, v[k]);
         sum += (v[k].x + v[k].y) + (v[k].z + v[k].w);
     }
-    if (!a.w1 && !a.w2) return;
+    if (!a.w1 && !a.w2) {
+        if constexpr (EMBED) griddep_wait();
+        return;
+    }
     const float mean = block_sum(sum, red) / (float)W;
     float sq = 0.f;
 #pragma unroll
@@ -435,22 +478,31 @@ __global__ void __launch_bounds__(256) parallel_join_vec_kernel(ParallelJoinDev 
             if (to_b) store_bf16x4(to_b + base + at(k), o);
         }
     }
+    if constexpr (EMBED) griddep_wait();
 }
-cudaError_t parallel_join_launch(const ParallelJoinArgs& a, int W, int T, cudaStream_t s) {
+template <bool EMBED>
+static cudaError_t launch_join(const ParallelJoinArgs& a, int W, int T, cudaStream_t s) {
     ParallelJoinDev p = {};
     p.a = a;
     if (a.moe) { p.j = *a.moe; p.moe = 1; }
+    if (EMBED) {
+        p.e = *a.embed;
+        if (p.e.bg.table && !p.e.tok_prev) return cudaErrorInvalidValue;
+    }
     // few tokens: more threads per row, one CTA's latency is all there is
-    if (T <= 16 && W >= 1024) return launch_chain(parallel_join_kernel<1024>, dim3(T), dim3(1024), (size_t)W * 4, s, p, W);
+    if (T <= 16 && W >= 1024) return launch_chain(parallel_join_kernel<1024, EMBED>, dim3(T), dim3(1024), (size_t)W * 4, s, p, W);
     const void* const all[] = {a.x, a.a, a.b, a.w1, a.b1, a.y1, a.w2, a.b2, a.y2, a.x_copy, a.y1_bf16, a.y2_bf16, p.j.rows, p.j.h};
     uintptr_t at = 0;
     for (const void* q : all) at |= reinterpret_cast<uintptr_t>(q);
-    if (W % 4 == 0 && W <= 4096 && a.ld_copy % 4 == 0 && (at & 15) == 0) {
-        if (W <= 1024) return launch_chain(parallel_join_vec_kernel<1>, dim3(T), dim3(256), 0, s, p, W);
-        if (W <= 2048) return launch_chain(parallel_join_vec_kernel<2>, dim3(T), dim3(256), 0, s, p, W);
-        return launch_chain(parallel_join_vec_kernel<4>, dim3(T), dim3(256), 0, s, p, W);
+    if (W % 4 == 0 && W <= 4096 && a.ld_copy % 4 == 0 && (at & 15) == 0 && (!EMBED || embed_wide(p.e, W))) {
+        if (W <= 1024) return launch_chain(parallel_join_vec_kernel<1, EMBED>, dim3(T), dim3(256), 0, s, p, W);
+        if (W <= 2048) return launch_chain(parallel_join_vec_kernel<2, EMBED>, dim3(T), dim3(256), 0, s, p, W);
+        return launch_chain(parallel_join_vec_kernel<4, EMBED>, dim3(T), dim3(256), 0, s, p, W);
     }
-    return launch_chain(parallel_join_kernel<256>, dim3(T), dim3(256), (size_t)W * 4, s, p, W);
+    return launch_chain(parallel_join_kernel<256, EMBED>, dim3(T), dim3(256), (size_t)W * 4, s, p, W);
+}
+cudaError_t parallel_join_launch(const ParallelJoinArgs& a, int W, int T, cudaStream_t s) {
+    return a.embed ? launch_join<true>(a, W, T, s) : launch_join<false>(a, W, T, s);
 }
 
 // ---------------------------------------------------------------- window attention

@@ -128,16 +128,19 @@ cudaError_t moe_route_launch(const MoeRouteArgs& a, int T, cudaStream_t s) {
 
 // One CTA: histogram of the pairs by expert, tile table, placement. Which row of an expert's range a pair
 // gets depends on the order of the atomics, but every output row is computed from its own input row alone, so the
-// order changes no number. ms: [3 n_experts + 1] ints of shared memory.
+// order changes no number. A warp's pairs of one expert are counted with one atomic operation: few experts share the same few words (4096 pairs of 8 experts,
+// 14 us a pair at a time, 12 so: reads behind one another are the rest). ms: [3 n_experts + 1] ints of shared memory.
 __device__ void moe_sort_cta(const MoeSortArgs& a, int* ms) {
     int* count = ms;                       // [n_experts]
     int* offset = count + a.n_experts;     // [n_experts + 1]
     int* cursor = offset + a.n_experts + 1;
     for (int e = threadIdx.x; e < a.n_experts; e += blockDim.x) { count[e] = 0; cursor[e] = 0; }
     __syncthreads();
-    for (int p = threadIdx.x; p < a.n_pairs; p += blockDim.x) {
-        const int e = a.sel[p];
-        if (e >= 0 && e < a.n_experts) atomicAdd(&count[e], 1);
+    const int lane = threadIdx.x & 31;
+    for (int p0 = 0; p0 < a.n_pairs; p0 += blockDim.x) {       // (whole warps: blockDim is a multiple of 32)
+        const int p = p0 + threadIdx.x, e = p < a.n_pairs ? a.sel[p] : -1;
+        const unsigned same = __match_any_sync(0xffffffffu, e);
+        if (e >= 0 && e < a.n_experts && lane == __ffs(same) - 1) atomicAdd(&count[e], __popc(same));
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -153,11 +156,16 @@ __device__ void moe_sort_cta(const MoeSortArgs& a, int* ms) {
         *a.n_tiles = tiles;
     }
     __syncthreads();
-    for (int p = threadIdx.x; p < a.n_pairs; p += blockDim.x) {
-        const int e = a.sel[p];
-        int row = -1;
-        if (e >= 0 && e < a.n_experts) {
-            row = offset[e] + atomicAdd(&cursor[e], 1);
+    for (int p0 = 0; p0 < a.n_pairs; p0 += blockDim.x) {
+        const int p = p0 + threadIdx.x, e = p < a.n_pairs ? a.sel[p] : -1;
+        const bool placed = e >= 0 && e < a.n_experts;
+        const unsigned same = __match_any_sync(0xffffffffu, e);
+        const int first = __ffs(same) - 1;
+        int at = placed && lane == first ? atomicAdd(&cursor[e], __popc(same)) : 0;
+        at = __shfl_sync(0xffffffffu, at, first) + __popc(same & ((1u << lane) - 1));
+        if (p >= a.n_pairs) continue;
+        const int row = placed ? offset[e] + at : -1;
+        if (placed) {
             a.x_rows[row] = p / a.top;
             if (a.weight) a.row_weight[row] = a.weight[p];
         }
