@@ -399,7 +399,9 @@ __device__ __noinline__ void deq_loop(const DeqCtx cx) {
 
 // SS: expanded weights in shared memory (K-major core matrices like the activations), T up to 256. Above 256 tokens tensor memory cannot hold
 // two halves of 256 sums and weights as well, and three narrower token tiles lose more than they save: 112 row tiles x 3 are 2.3 waves
-// (512 tokens, the four products of a layer of 4096: 304 us, this form 251; 128 rows and all tokens a CTA before: 290).
+// (512 tokens, the four products of a layer of 4096: 304 us, this form 251; 128 rows and all tokens a CTA before: 290). Only the last wave, where two tiles a row
+// tile would leave SMs idle, takes three: a launch of its own (28672 rows: 112 row tiles are 148 + 76 CTAs of two, or 148 + 114 of two and three; the second wave
+// then takes 47 us to the first one's 66, both together 115 instead of 125).
 template <bool SS>
 __global__ void __launch_bounds__(GM_THREADS) gemm_q_kernel(const __grid_constant__ GemmParams p) {
     constexpr int DW = GM_DW, ROWS = GM_ROWS;      // dequantising warps; then: MMA warp, weight producer, activation producer
@@ -416,7 +418,7 @@ __global__ void __launch_bounds__(GM_THREADS) gemm_q_kernel(const __grid_constan
     while ((int)ncols < 2 * T + (SS ? 0 : S * GM_BK)) ncols <<= 1;
 
     // ---- which tile / K range (in 256-weight spans = 4 blocks)
-    const int split = blockIdx.x % p.n_splits, tile_g = blockIdx.x / p.n_splits / p.n_tt;
+    const int split = blockIdx.x % p.n_splits, tile_g = p.tile_base + blockIdx.x / p.n_splits / p.n_tt;
     int seg = 0;
     while (seg + 1 < p.nseg && tile_g >= p.seg[seg + 1].tile0) seg++;
     const GemmSeg& sg = p.seg[seg];
@@ -676,6 +678,18 @@ int gemm_plan(GemmParams& p, int n_sms, int max_splits) {
         if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = s; }
     }
     p.n_splits = best;
+    // row tiles past the last whole wave of two token tiles: three tiles of their tokens, if those are one wave too
+    p.tile_base = p.n_rest = 0;
+    const int whole = tiles / (n_sms / 2) * (n_sms / 2), rest = tiles - whole;
+    if (p.ss && p.n_tt == 2 && p.n_splits == 1 && whole > 0 && rest > 0 && 3 * rest <= n_sms) {
+        GemmParams q = p;
+        q.ss = 0; q.n_tt = 3; q.t_tile = ((p.T_pad + 2) / 3 + 15) / 16 * 16;
+        q.n_stages = GM_GROUPS; q.n_raw = GM_RAW_STAGES;               // beside two halves of up to 176 sums
+        for (q.n_bstages = 6; gemm_smem_bytes(q) > cap && q.n_bstages > 2;) q.n_bstages--;
+        if (2 * q.t_tile + q.n_stages * GM_BK <= 512 && gemm_smem_bytes(q) <= cap) {
+            p.n_rest = rest; p.rest_stages = q.n_stages; p.rest_bstages = q.n_bstages; p.rest_raw = q.n_raw; p.rest_t_tile = q.t_tile;
+        }
+    }
     return 0;
 }
 
@@ -683,7 +697,12 @@ cudaError_t gemm_launch(const GemmParams& p, cudaStream_t stream) {
     if (p.n_stages < GM_GROUPS || p.n_stages % GM_GROUPS || p.n_stages > GM_MAX_STAGES || p.n_bstages < 2 || p.n_bstages > GM_MAX_BSTAGES || p.n_splits < 1 ||
         p.n_tiles < 1) return cudaErrorInvalidValue;
     if (p.T_pad < 16 || p.T_pad > 512 || p.T_pad % 16 || p.T > p.T_pad || p.n_splits > p.K / 256) return cudaErrorInvalidValue;
-    return launch_chain(p.ss ? gemm_q_kernel<true> : gemm_q_kernel<false>, dim3(p.n_tiles * p.n_tt * p.n_splits), dim3(GM_THREADS), gemm_smem_bytes(p), stream, p);
+    const int n_tiles = p.n_tiles - p.n_rest;
+    const cudaError_t e = launch_chain(p.ss ? gemm_q_kernel<true> : gemm_q_kernel<false>, dim3(n_tiles * p.n_tt * p.n_splits), dim3(GM_THREADS), gemm_smem_bytes(p), stream, p);
+    if (e != cudaSuccess || p.n_rest == 0) return e;
+    GemmParams q = p;
+    q.ss = 0; q.n_tt = 3; q.t_tile = p.rest_t_tile; q.n_stages = p.rest_stages; q.n_bstages = p.rest_bstages; q.n_raw = p.rest_raw; q.tile_base = n_tiles;
+    return launch_chain(gemm_q_kernel<false>, dim3(p.n_rest * q.n_tt * p.n_splits), dim3(GM_THREADS), gemm_smem_bytes(q), stream, q);
 }
 
 // x [T][K] float32 -> f16 in the MMA operand order [K/8][T_pad][8] (rows >= T zero)

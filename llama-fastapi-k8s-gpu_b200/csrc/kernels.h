@@ -194,6 +194,9 @@ struct GemmParams {
     long long* dbg;         // optional: CTA 0 records clock64() per K block (8 slots each; b2_op_gemm with B2_GEMM_DBG)
     int n_tiles, n_splits, n_stages, n_bstages, n_raw;   // filled by gemm_plan
     int n_tt, t_tile, ss;   // token tiles of a step and the tokens of one (a multiple of 16); expanded weights in shared memory
+    int tile_base;          // first row tile of a launch
+    int n_rest;             // row tiles at the end that a second launch takes in three token tiles, weights in tensor memory (0: none); its plan:
+    int rest_stages, rest_bstages, rest_raw, rest_t_tile;
 };
 cudaError_t gemm_init();
 int gemm_plan(GemmParams& p, int n_sms, int max_splits);

@@ -385,3 +385,28 @@ def test_two_token_tiles_of_quantised_products(native_lib, tname, K, N, T):
     from test_gpu_ops import _gemm_case
     assert _gemm_case(native_lib, tname, K, N, T) < 2e-3
     assert _gemm_case(native_lib, tname, K, N, T, n_splits=min(3, K // 256)) < 2e-3
+
+
+@pytest.mark.parametrize("tname", ["Q4_K", "Q6_K", "Q8_0", "Q4_1"])
+@pytest.mark.parametrize("K,N,T", [(256, 74 * 256 + 1, 512), (512, 75 * 256 + 130, 257), (256, 123 * 256, 400)])
+def test_last_wave_of_quantised_products(native_lib, tname, K, N, T):
+    """Row tiles past whole waves of two token tiles: one and two, and as many as fit three token tiles each on the SMs of one wave. Their sums have the
+    same bits as in a product of few rows (two token tiles, test above), and so have those of the rows before them."""
+    from test_gpu_ops import TYPE_IDS, lib_check, ptr
+    from llama_cpp.synth import random_blocks
+    from oracle import ggml_blocks as gb
+    t = TYPE_IDS[tname]
+    w = random_blocks(tname, N * K // gb.BLOCK[t][0], 0.02, seed=N + T).reshape(N, -1)
+    x = np.random.default_rng(T).standard_normal((T, K)).astype(np.float32)
+
+    def product(rows, n_splits):
+        y = np.zeros((T, len(rows)), np.float32)
+        lib_check(native_lib, native_lib.b2_op_gemm(0, t, ptr(rows), len(rows), K, ptr(x), T, None, ptr(y), n_splits))
+        return y
+
+    for n_splits in (1, K // 256):
+        y = product(w, n_splits)
+        for n0 in (0, 73 * 256, 74 * 256):
+            part = np.ascontiguousarray(w[n0:n0 + 600])
+            assert np.array_equal(y[:, n0:n0 + 600], product(part, n_splits)), (n0, n_splits)
+        assert np.array_equal(y[:, -300:], product(np.ascontiguousarray(w[-300:]), n_splits))
