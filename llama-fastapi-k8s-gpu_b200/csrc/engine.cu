@@ -791,7 +791,10 @@ static int prefill_chunk(b2_engine* e, Slot& s, const int* tokens, int T, int po
         if ((rc = gemm_call(e, qkv, 3, e->pf_xn, T, &np, &ps))) return rc;
         CK(rope_store_launch(e->pf_part, np, ps, T, pos0, c.n_head, c.n_head_kv, hd, c.kv_block_tokens, s.block_table, e->rope_freq,
                              e->pf_qh, kc, vc, st));
-        CK(attn_prefill_launch(e->pf_qh, kc, vc, s.block_table, T, T_pad, pos0, c.n_head, c.n_head_kv, hd, c.kv_block_tokens, e->pf_att, st));
+        if (attn_prefill_takes_tc(T, pos0, hd, c.kv_block_tokens))
+            CK(attn_prefill_tc_launch(e->pf_qh, kc, vc, (long)c.kv_num_blocks * c.n_head_kv * c.kv_block_tokens, s.block_table, T, T_pad, pos0, c.n_head, c.n_head_kv, hd,
+                                      c.kv_block_tokens, e->pf_att, st));
+        else CK(attn_prefill_launch(e->pf_qh, kc, vc, s.block_table, T, T_pad, pos0, c.n_head, c.n_head_kv, hd, c.kv_block_tokens, e->pf_att, st));
         const DevTensor* wo[1] = {&L.wo};
         if ((rc = gemm_call(e, wo, 1, e->pf_att, T, &np, &ps))) return rc;
         CK(resid_norm_half_launch(e->pf_x, e->pf_part, np, ps, (const float*)L.ffn_norm.ptr, c.rms_eps, E, T, T_pad, e->pf_xn, st));

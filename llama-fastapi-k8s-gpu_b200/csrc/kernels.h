@@ -218,6 +218,10 @@ cudaError_t rope_store_launch(const float* parts, int n_parts, long part_stride,
                               int bt, const int* block_table, const float* rope_freq, __half* qh, __half* k_cache,
                               __half* v_cache, cudaStream_t s);
 // causal attention of T queries at pos0.. over the paged cache; out in operand order (T_pad)
+// the same on tensor memory (prefill_tc.cu), for the sizes attn_prefill_takes_tc says; pool_rows: rows of a layer's pool, pages * n_kv * bt
+bool attn_prefill_takes_tc(int T, int pos0, int hd, int bt);
+cudaError_t attn_prefill_tc_launch(const __half* qh, const __half* k_cache, const __half* v_cache, long pool_rows, const int* block_table, int T, int T_pad, int pos0,
+                                   int n_head, int n_kv, int hd, int bt, __half* out, cudaStream_t s);
 cudaError_t attn_prefill_launch(const __half* qh, const __half* k_cache, const __half* v_cache, const int* block_table,
                                 int T, int T_pad, int pos0, int n_head, int n_kv, int hd, int bt, __half* out, cudaStream_t s);
 // gate|up parts [T][2F] -> h = f16(silu(gate) * up) in operand order

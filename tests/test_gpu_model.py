@@ -369,3 +369,25 @@ def test_a_set_token_enters_the_next_step_whichever_it_is(native_lib, tmp_models
         eng.decode_n(4, 1)                                     # its token was set and stayed set while the others stepped
         assert np.abs(eng.logits(4) - ref[12]).max() <= LOGIT_TOL
     eng.close()
+
+
+@pytest.mark.parametrize("arch", ["tiny", "tiny128"])
+@pytest.mark.parametrize("portions", [(129,), (128, 2), (64, 65, 9), (300,), (200, 57), (8, 511, 20), (700,)])
+def test_prompts_over_pages_of_64(native_lib, tmp_models, arch, portions):
+    """Attention on tensor memory (more than 128 keys, pages of 64 tokens): partial tiles of 128 queries, partial blocks of 128 keys, one half of a
+    block, keys of earlier portions, two chunks of 512; every portion's last logits against the oracle."""
+    from oracle.llama_ref import RefModel
+    path = _model(tmp_models, arch, "Q8_0", 3)
+    n = sum(portions)
+    prompt = [int(t) for t in np.random.default_rng(n).integers(3, 700, size=n)]
+    ref = RefModel(path).forward(prompt)
+    eng = _engine(path, n_ctx=n + 8, bt=64)
+    eng.ensure_pages(0, n)
+    eng.seq_begin(0, 0, [], _greedy())
+    at = 0
+    for k in portions:
+        eng.prefill(0, prompt[at:at + k])
+        at += k
+        assert np.abs(eng.logits(0) - ref[at - 1]).max() <= LOGIT_TOL, at
+    eng.close()
+
