@@ -658,13 +658,14 @@ __device__ __forceinline__ float2 cache_load2(const void* pool, size_t i) {
     const uint32_t u = *reinterpret_cast<const uint32_t*>(reinterpret_cast<const __nv_bfloat16*>(pool) + i);
     return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
 }
+// of_tiles: CTA x takes the token of tile x (the one-token tiles come first) instead of token x
 template <bool F32>
-__global__ void __launch_bounds__(ATT2_WARPS * 32) window_attn_pairs_kernel(WindowAttnArgs a, RaggedDev r) {
+__global__ void __launch_bounds__(ATT2_WARPS * 32) window_attn_pairs_kernel(WindowAttnArgs a, RaggedDev r, int of_tiles) {
     griddep_launch();
     griddep_wait();
     __shared__ float sm_m[ATT2_WARPS], sm_l[ATT2_WARPS];
     __shared__ float sm_o[ATT2_WARPS][ATT2_PASS * 64];
-    const int t = blockIdx.x, h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int t = of_tiles ? r.tile_row0[blockIdx.x] : (int)blockIdx.x, h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int pos = r.tok_pos[t];
     const int slot = r.seg_slot[r.tok_seg[t]];
     const int* table = a.block_tables[slot];
@@ -952,6 +953,166 @@ static SoftmaxTcArgs window_softmax_args(const WindowAttnArgs& a) {
     return x;
 }
 bool window_attn_leaves_rounded(const WindowAttnArgs& a, int T) { return window_attn_mma(a, T) && softmax_takes_tc(window_softmax_args(a)); }
+// 32-bit pages, sequences that bring two tokens or more to a step of more than 8: 32 queries of one head a CTA, blocks of 64 keys and values (a
+// block starts at a multiple of 64 whatever the query, so a row's sums do not depend on the tile it is in) by asynchronous copies one block ahead. A warp has
+// four queries and one half of every block; the halves' sums meet at the end. Scores: a lane multiplies four queries with four keys over every fourth piece of four entries, 8 multiply-adds a read; the four lanes of a key
+// group add their parts up, each ending up with one query's. Sums: a lane has four entries of the output of all four queries. Nothing is less than 32 bits.
+// Bound by shared-memory reads. (459 tokens of 8 heads of 128 in two sequences: 105 us with a CTA per token and head, every key read from L2 by each; 60 with one warp a query group and blocks of 32 keys, 34 here. 900 tokens, a whole prompt of two layers: 1044 -> 622 us.)
+constexpr int WT_Q = 32, WT_K = 64, WT_OWN = 32, WT_WARPS = 16, WT_D = 128;
+__global__ void __launch_bounds__(WT_WARPS * 32, 1) window_attn_tile_kernel(WindowAttnArgs a, RaggedDev r, int first_tile) {
+    griddep_launch();
+    griddep_wait();
+    extern __shared__ __align__(16) float wt_sm[];
+    const int d = a.d, ldk = d + 4, tile = first_tile + blockIdx.x / 2, h = blockIdx.y, g = h / (a.H / a.G);
+    const int seg = r.tile_seg[tile], row0 = r.tile_row0[tile] + (blockIdx.x & 1) * WT_Q;
+    const int nq = min(WT_Q, r.seg_start[seg] + r.seg_len[seg] - row0);
+    if (nq <= 0) return;
+    float* qs = wt_sm;                                     // [32][d + 4]
+    float* ks = qs + WT_Q * ldk;                           // [2][64][d + 4]
+    float* vs = ks + 2 * WT_K * ldk;                       // [2][64][d]
+    float* ps = vs + 2 * WT_K * d;                         // [half, warp][32 keys][4 queries]
+    const int warp = threadIdx.x >> 5 & 7, half = threadIdx.x >> 8, own = half * WT_OWN, lane = threadIdx.x & 31, kg = lane >> 2, part = lane & 3;
+    const int p0 = r.seg_pos0[seg] + row0 - r.seg_start[seg], p_last = p0 + nq - 1;
+    const int* table = a.block_tables[r.seg_slot[seg]];
+    const float *k_pool = reinterpret_cast<const float*>(a.k_pool), *v_pool = reinterpret_cast<const float*>(a.v_pool);
+    // key blocks: those of the kept prefix, then those of the window
+    const int lo_first = max(0, p0 - a.window + 1), n_kept = lo_first > 0 ? (min(a.keep_first, lo_first) + WT_K - 1) / WT_K : 0;
+    const int w0 = max(lo_first / WT_K, n_kept), n_blocks = n_kept + p_last / WT_K + 1 - w0;
+    auto block_at = [&](int i) { return (i < n_kept ? i : w0 + i - n_kept) * WT_K; };
+    const int per = d / 4;
+    // eight threads a row of a block, whose page is looked up a block ahead of its copies
+    const int my_row = threadIdx.x / 8, my_c = threadIdx.x % 8 * 4;
+    auto page_of = [&](int i) { return i < n_blocks ? table[min(block_at(i) + my_row, p_last) / a.block_tokens] : 0; };
+    int page = page_of(0);
+    auto stage = [&](int i, int buf) {                     // blocks in order; keys past the last query's are zeros (their weights are)
+        const int pos = block_at(i) + my_row;
+        const bool have = pos <= p_last;
+        const size_t from = have ? (((size_t)page * a.G + g) * a.block_tokens + pos % a.block_tokens) * d : 0;
+        page = page_of(i + 1);
+        float *kd = ks + (buf * WT_K + my_row) * ldk, *vd = vs + (buf * WT_K + my_row) * d;
+        for (int c = my_c; c < d; c += 32) {
+            cp_async_16z(kd + c, k_pool + from + c, have ? 16 : 0);
+            cp_async_16z(vd + c, v_pool + from + c, have ? 16 : 0);
+        }
+    };
+    for (int e = threadIdx.x; e < WT_Q * per; e += WT_WARPS * 32) {      // (rows past the tile: the last one's, dropped at the end)
+        const int q = e / per, c = e % per * 4;
+        const float4 v = *reinterpret_cast<const float4*>(a.q_rot + ((size_t)(row0 + min(q, nq - 1)) * a.H + h) * d + c);
+        *reinterpret_cast<float4*>(qs + q * ldk + c) = make_float4(v.x * a.scale, v.y * a.scale, v.z * a.scale, v.w * a.scale);
+    }
+    stage(0, 0);
+    cp_async_commit();
+    const int pos = p0 + warp * 4 + part, lo = max(0, pos - a.window + 1);      // of the query whose scores this lane ends up with
+    float m = -INFINITY, l = 0.f;                          // of that query (l: this lane's keys)
+    float4 o[4];                                           // entries 4 lane .. of the warp's four queries
+#pragma unroll
+    for (int u = 0; u < 4; u++) o[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    float* pw = ps + (half * 8 + warp) * WT_OWN * 4;
+    for (int i = 0; i < n_blocks; i++) {
+        const int buf = i & 1, j0 = block_at(i) + own;
+        cp_async_wait_all();
+        __syncthreads();                                   // this block has come, everybody has left the other buffer
+        if (i + 1 < n_blocks) stage(i + 1, buf ^ 1);
+        cp_async_commit();
+        float sc[4][4];                                    // [query][key of the group]
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+#pragma unroll
+            for (int v = 0; v < 4; v++) sc[u][v] = 0.f;
+        const float *qr = qs + warp * 4 * ldk + part * 4, *kr = ks + (buf * WT_K + own + kg * 4) * ldk + part * 4;
+#pragma unroll 4
+        for (int c = 0; c < d; c += 16) {
+            float4 q[4], k[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) { q[u] = *reinterpret_cast<const float4*>(qr + u * ldk + c); k[u] = *reinterpret_cast<const float4*>(kr + u * ldk + c); }
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+#pragma unroll
+                for (int v = 0; v < 4; v++) sc[u][v] += fmaf(q[u].x, k[v].x, fmaf(q[u].y, k[v].y, fmaf(q[u].z, k[v].z, q[u].w * k[v].w)));
+        }
+        // the four parts of every score: lane `part` ends up with query `part`
+        float s[4];
+#pragma unroll
+        for (int v = 0; v < 4; v++) {
+            const bool up = part & 2, odd = part & 1;
+            const float x0 = (up ? sc[2][v] : sc[0][v]) + __shfl_xor_sync(0xffffffffu, up ? sc[0][v] : sc[2][v], 2);
+            const float x1 = (up ? sc[3][v] : sc[1][v]) + __shfl_xor_sync(0xffffffffu, up ? sc[1][v] : sc[3][v], 2);
+            s[v] = (odd ? x1 : x0) + __shfl_xor_sync(0xffffffffu, odd ? x0 : x1, 1);
+        }
+        float mx = m;
+#pragma unroll
+        for (int v = 0; v < 4; v++) {
+            const int j = j0 + kg * 4 + v;
+            if (j > pos || (j < lo && j >= a.keep_first)) s[v] = -INFINITY;
+            mx = fmaxf(mx, s[v]);
+        }
+#pragma unroll
+        for (int w = 4; w < 32; w <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, w));
+        const float ref = mx > -INFINITY ? mx : 0.f, corr = m > -INFINITY ? expf(m - ref) : 0.f;      // (nothing visible yet: all weights are 0)
+        m = mx;
+        l *= corr;
+#pragma unroll
+        for (int v = 0; v < 4; v++) {
+            const float e = expf(s[v] - ref);
+            l += e;
+            pw[(kg * 4 + v) * 4 + part] = e;
+        }
+        __syncwarp();
+        float4 b[4];                                       // the block's own sums: short chains of additions
+#pragma unroll
+        for (int u = 0; u < 4; u++) b[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (4 * lane < d) {
+            const float* vr = vs + (buf * WT_K + own) * d + 4 * lane;
+            auto add = [&](int j, bool all) {
+                const float4 v = *reinterpret_cast<const float4*>(vr + j * d), p = *reinterpret_cast<const float4*>(pw + j * 4);
+                const float w[4] = {p.x, p.y, p.z, p.w};
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (all || w[u] != 0.f) { b[u].x = fmaf(w[u], v.x, b[u].x); b[u].y = fmaf(w[u], v.y, b[u].y); b[u].z = fmaf(w[u], v.z, b[u].z); b[u].w = fmaf(w[u], v.w, b[u].w); }
+            };
+            // (a key that some of the warp's queries do not see must not reach them, not even as 0 times infinity)
+            if (j0 + WT_OWN - 1 <= p0 + warp * 4 && j0 >= p0 + warp * 4 + 3 - a.window + 1) {
+#pragma unroll 8
+                for (int j = 0; j < WT_OWN; j++) add(j, true);
+            } else for (int j = 0; j < WT_OWN; j++) add(j, false);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const float f = __shfl_sync(0xffffffffu, corr, u);
+            o[u].x = fmaf(o[u].x, f, b[u].x); o[u].y = fmaf(o[u].y, f, b[u].y); o[u].z = fmaf(o[u].z, f, b[u].z); o[u].w = fmaf(o[u].w, f, b[u].w);
+        }
+        __syncwarp();
+    }
+#pragma unroll
+    for (int w = 4; w < 32; w <<= 1) l += __shfl_xor_sync(0xffffffffu, l, w);
+    // the second half's maxima, sums and outputs, where the keys were
+    float4* other = reinterpret_cast<float4*>(ks) + warp * 4 * 32 + lane;      // [warp][query][lane]
+    float2* other_ml = reinterpret_cast<float2*>(ps) + warp * 4;
+    __syncthreads();
+    if (half == 1) {
+#pragma unroll
+        for (int u = 0; u < 4; u++) other[u * 32] = o[u];
+        if (kg == 0) other_ml[part] = make_float2(m, l);
+    }
+    __syncthreads();
+    if (half == 1) return;
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const float m0 = __shfl_sync(0xffffffffu, m, u), l0 = __shfl_sync(0xffffffffu, l, u);
+        const float2 ml = other_ml[u];
+        const float4 y = other[u * 32];
+        const float M = fmaxf(m0, ml.x), f0 = m0 > -INFINITY ? expf(m0 - M) : 0.f, f1 = ml.x > -INFINITY ? expf(ml.x - M) : 0.f, sum = fmaf(l0, f0, ml.y * f1);
+        const int q = warp * 4 + u;
+        if (q < nq && 4 * lane < d)
+            *reinterpret_cast<float4*>(a.out + ((size_t)(row0 + q) * a.H + h) * d + 4 * lane) =
+                make_float4(fmaf(o[u].x, f0, y.x * f1) / sum, fmaf(o[u].y, f0, y.y * f1) / sum, fmaf(o[u].z, f0, y.z * f1) / sum, fmaf(o[u].w, f0, y.w * f1) / sum);
+    }
+}
+// Heads of whole 16-entry pieces up to 128, rows on 16-byte boundaries.
+static bool window_attn_tiles(const WindowAttnArgs& a, int T) {
+    return a.cache_f32 && T > 8 && a.d % 16 == 0 && a.d <= WT_D && ((reinterpret_cast<uintptr_t>(a.q_rot) | reinterpret_cast<uintptr_t>(a.out)) & 15) == 0;
+}
+
 cudaError_t window_attn_launch(const WindowAttnArgs& a, const RaggedDev& r, cudaStream_t s) {
     if (a.d > ATT_MAXE * 32 || (a.out_rounded && !window_attn_leaves_rounded(a, r.T))) return cudaErrorInvalidValue;
     if (window_attn_mma(a, r.T)) {
@@ -962,6 +1123,18 @@ cudaError_t window_attn_launch(const WindowAttnArgs& a, const RaggedDev& r, cuda
         if (a.d <= 64) return launch_chain(window_attn_mma_kernel<64>, dim3(r.n_tiles, a.H), dim3(128), smem, s, a, r);
         return launch_chain(window_attn_mma_kernel<128>, dim3(r.n_tiles, a.H), dim3(128), smem, s, a, r);
     }
+    if (window_attn_tiles(a, r.T)) {
+        // (tokens that come alone: a CTA per token and head, below)
+        const int alone = r.n_upto[0];
+        constexpr int most = ((WT_Q + 2 * WT_K) * (WT_D + 4) + 2 * WT_K * WT_D + WT_WARPS * WT_OWN * 4) * 4;
+        if (!allow_smem<window_attn_tile_kernel>(most)) return cudaErrorInvalidValue;
+        const size_t smem = (size_t)((WT_Q + 2 * WT_K) * (a.d + 4) + 2 * WT_K * a.d + WT_WARPS * WT_OWN * 4) * 4;
+        if (r.n_tiles > alone) {
+            const cudaError_t e = launch_chain(window_attn_tile_kernel, dim3((r.n_tiles - alone) * 2, a.H), dim3(WT_WARPS * 32), smem, s, a, r, alone);
+            if (e != cudaSuccess) return e;
+        }
+        return alone ? launch_chain(window_attn_pairs_kernel<true>, dim3(alone, a.H), dim3(ATT2_WARPS * 32), 0, s, a, r, 1) : cudaSuccess;
+    }
     if (a.d % 2 == 0) {
         // a step of a few tokens does not fill the GPU with one CTA per (token, head): split the keys (up to 16 ranges)
         int splits = 1;
@@ -970,8 +1143,8 @@ cudaError_t window_attn_launch(const WindowAttnArgs& a, const RaggedDev& r, cuda
             while (splits > 1 && (size_t)r.T * a.H * splits * (a.d + 2) > (size_t)a.split_capacity) splits--;
         }
         const dim3 grid(r.T, a.H, splits);
-        cudaError_t ce = a.cache_f32 ? launch_chain(window_attn_pairs_kernel<true>, grid, dim3(ATT2_WARPS * 32), 0, s, a, r)
-                                     : launch_chain(window_attn_pairs_kernel<false>, grid, dim3(ATT2_WARPS * 32), 0, s, a, r);
+        cudaError_t ce = a.cache_f32 ? launch_chain(window_attn_pairs_kernel<true>, grid, dim3(ATT2_WARPS * 32), 0, s, a, r, 0)
+                                     : launch_chain(window_attn_pairs_kernel<false>, grid, dim3(ATT2_WARPS * 32), 0, s, a, r, 0);
         if (ce != cudaSuccess || splits == 1) return ce;
         return launch_chain(window_attn_merge_kernel, dim3(r.T, a.H), dim3(128), 0, s, a, splits);
     }

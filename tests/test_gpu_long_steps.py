@@ -78,6 +78,35 @@ def test_window_attention_of_long_steps(native_lib, tmp_path, d, window, keep, l
     check(gu, goponex_ref, cfg, tmp_path, lengths, "bfloat16")
 
 
+# the same over 32-bit pages: tiles of 32 queries, blocks of 32 keys; tokens that come alone
+@pytest.mark.parametrize("d,window,keep,lengths", [(16, 1, 0, [33]), (64, 64, 3, [257]), (80, 100, 70, [200]), (128, 129, 1, [300, 1, 31]), (32, 1000, 4, [100, 64, 2]),
+                                                  (112, 20, 40, [1, 2, 31, 33, 64, 65])])
+def test_window_attention_of_long_steps_in_32_bits(native_lib, tmp_path, d, window, keep, lengths):
+    cfg = gu.config([gu.parallel(left=gu.attn(heads=4, kv_heads=2, dim=d, rot=8, window=window, keep=keep))])
+    check(gu, goponex_ref, cfg, tmp_path, lengths, "float32")
+
+
+def test_cuts_do_not_change_a_token_in_32_bits(native_lib, tmp_path):
+    """Window attention over 32-bit pages: in portions of two tokens and more, each in a step of more than 8, a prompt's logits have the bits of the whole."""
+    from llama_cpp.kv_pages import SequenceSlots
+    cfg = gu.config([gu.parallel(left=gu.attn(heads=4, kv_heads=2, dim=64, rot=8, window=70, keep=5))])
+    eng = engine(gu.write_model(str(tmp_path / "m"), cfg, gu.random_weights(cfg, seed=9)), "float32", 300, 2)
+    prompt, side = toks(cfg["vocab"], 200, 1), toks(cfg["vocab"], 90, 2)
+    rows = []
+    for cuts in ([200], [33, 167], [2, 60, 7, 131], [64, 64, 72]):
+        seqs, got, at = SequenceSlots(eng), [], 0
+        seqs.open(0), seqs.open(1)
+        for k, n in enumerate(cuts):
+            entries = [(seqs.extend(0, n), prompt[at:at + n]), (seqs.extend(1, 20), side[20 * k:20 * k + 20])]
+            got.append(np.array(eng.step(entries, want=[list(range(n)), list(range(20))])[0])[:n])      # (more than 8 rows for the head: one form of it)
+            at += n
+        seqs.close(0), seqs.close(1)
+        rows.append(np.concatenate(got))
+    eng.close()
+    for other in rows[1:]:
+        assert np.array_equal(rows[0], other)
+
+
 # (head sizes that are multiples of 8: the products around the attention take rounded rows, without which the general kernel runs)
 LATENT = {"plain": lambda heads, rank, **kw: fu.plain(heads=heads, rank=rank, dim=24, vdim=16, **kw),
           "rotated": lambda heads, rank, **kw: fu.rotated(heads=heads, rank=rank, dim=24, vdim=16, rot_dim=16, **kw)}
