@@ -750,10 +750,10 @@ __global__ void __launch_bounds__(ATT2_WARPS * 32) window_attn_pairs_kernel(Wind
 }
 
 // sum of the key ranges of one (token, head) in range order
-__global__ void __launch_bounds__(128) window_attn_merge_kernel(WindowAttnArgs a, int n_splits) {
+__global__ void __launch_bounds__(128) window_attn_merge_kernel(WindowAttnArgs a, RaggedDev r, int n_splits, int of_tiles) {
     griddep_launch();
     griddep_wait();
-    const int t = blockIdx.x, h = blockIdx.y, d = a.d;
+    const int t = of_tiles ? r.tile_row0[blockIdx.x] : (int)blockIdx.x, h = blockIdx.y, d = a.d;
     const float* part = a.split_scratch + ((size_t)t * a.H + h) * n_splits * (d + 2);
     float M = -INFINITY;
     for (int s2 = 0; s2 < n_splits; s2++) M = fmaxf(M, part[(size_t)s2 * (d + 2)]);
@@ -953,42 +953,68 @@ static SoftmaxTcArgs window_softmax_args(const WindowAttnArgs& a) {
     return x;
 }
 bool window_attn_leaves_rounded(const WindowAttnArgs& a, int T) { return window_attn_mma(a, T) && softmax_takes_tc(window_softmax_args(a)); }
-// 32-bit pages, sequences that bring two tokens or more to a step of more than 8: 32 queries of one head a CTA, blocks of 64 keys and values (a
-// block starts at a multiple of 64 whatever the query, so a row's sums do not depend on the tile it is in) by asynchronous copies one block ahead. A warp has
-// four queries and one half of every block; the halves' sums meet at the end. Scores: a lane multiplies four queries with four keys over every fourth piece of four entries, 8 multiply-adds a read; the four lanes of a key
-// group add their parts up, each ending up with one query's. Sums: a lane has four entries of the output of all four queries. Nothing is less than 32 bits.
-// Bound by shared-memory reads. (459 tokens of 8 heads of 128 in two sequences: 105 us with a CTA per token and head, every key read from L2 by each; 60 with one warp a query group and blocks of 32 keys, 34 here. 900 tokens, a whole prompt of two layers: 1044 -> 622 us.)
-constexpr int WT_Q = 32, WT_K = 64, WT_OWN = 32, WT_WARPS = 16, WT_D = 128;
-__global__ void __launch_bounds__(WT_WARPS * 32, 1) window_attn_tile_kernel(WindowAttnArgs a, RaggedDev r, int first_tile) {
+// 32-bit pages, sequences that bring two tokens or more to a step of more than 8: 32 queries of one head a CTA, blocks of 64 keys and values by asynchronous
+// copies one block ahead. A warp has four queries and one half of every block. Scores: a lane multiplies four queries with four keys over every fourth piece of
+// four entries, 8 multiply-adds a read; the four lanes of a key group add their parts up, each ending up with one query's. Sums: a lane has four entries of the
+// output of all four queries. Nothing is less than 32 bits. Blocks start at multiples of 64 keys and are summed up in ranges of 128, whose sums meet in
+// the order of the keys: a row's bits depend neither on the tile that it is in nor on `company`, the CTAs of a cluster that share a tile's ranges (and then its
+// queries' sums over ranges) where a step has too few tiles to fill the GPU.
+// Bound by shared-memory reads. (459 tokens of 8 heads of 128 in two sequences: 105 us with a CTA per token and head, every key read from L2 by each; 60 with one
+// warp a query group and blocks of 32 keys, 35 here. 900 tokens, a whole prompt of two layers: 1044 -> 622 us. A step of few tokens behind many keys, two layers
+// with a window of 1024: 20 tokens 323 -> 249, 64 tokens 432 -> 306. Ranges of 256 give a window of 300 too few to share:
+// 32 tokens 245 us against 227, of 237 before.)
+constexpr int WT_Q = 32, WT_K = 64, WT_OWN = 32, WT_WARPS = 16, WT_D = 128, WT_RANGE = 2;
+__global__ void __launch_bounds__(WT_WARPS * 32, 1) window_attn_tile_kernel(WindowAttnArgs a, RaggedDev r, int first_tile, int cluster) {
     griddep_launch();
     griddep_wait();
     extern __shared__ __align__(16) float wt_sm[];
-    const int d = a.d, ldk = d + 4, tile = first_tile + blockIdx.x / 2, h = blockIdx.y, g = h / (a.H / a.G);
-    const int seg = r.tile_seg[tile], row0 = r.tile_row0[tile] + (blockIdx.x & 1) * WT_Q;
+    const int d = a.d, ldk = d + 4, rank = blockIdx.x % cluster, x = blockIdx.x / cluster, tile = first_tile + x / 2, h = blockIdx.y, g = h / (a.H / a.G);
+    const int seg = r.tile_seg[tile], row0 = r.tile_row0[tile] + (x & 1) * WT_Q;
     const int nq = min(WT_Q, r.seg_start[seg] + r.seg_len[seg] - row0);
-    if (nq <= 0) return;
+    if (nq <= 0) return;                                   // (all of a cluster)
     float* qs = wt_sm;                                     // [32][d + 4]
     float* ks = qs + WT_Q * ldk;                           // [2][64][d + 4]
     float* vs = ks + 2 * WT_K * ldk;                       // [2][64][d]
     float* ps = vs + 2 * WT_K * d;                         // [half, warp][32 keys][4 queries]
+    float* xs = ps + WT_WARPS * WT_OWN * 4;                // [half][32 queries][d]: a range's sums ...
+    float2* xml = reinterpret_cast<float2*>(xs + 2 * WT_Q * d);      // [half][32]: ... and its maxima and sums of weights
     const int warp = threadIdx.x >> 5 & 7, half = threadIdx.x >> 8, own = half * WT_OWN, lane = threadIdx.x & 31, kg = lane >> 2, part = lane & 3;
     const int p0 = r.seg_pos0[seg] + row0 - r.seg_start[seg], p_last = p0 + nq - 1;
     const int* table = a.block_tables[r.seg_slot[seg]];
     const float *k_pool = reinterpret_cast<const float*>(a.k_pool), *v_pool = reinterpret_cast<const float*>(a.v_pool);
     // key blocks: those of the kept prefix, then those of the window
     const int lo_first = max(0, p0 - a.window + 1), n_kept = lo_first > 0 ? (min(a.keep_first, lo_first) + WT_K - 1) / WT_K : 0;
-    const int w0 = max(lo_first / WT_K, n_kept), n_blocks = n_kept + p_last / WT_K + 1 - w0;
+    const int w0 = max(lo_first / WT_K, n_kept), w1 = p_last / WT_K + 1;
+    // ranges that have any, in order; block `i` of all (the first of a range: the number of blocks before it)
+    const int kept_ranges = (n_kept + WT_RANGE - 1) / WT_RANGE, w_range = max(w0 / WT_RANGE, kept_ranges), n_ranges = kept_ranges + max(0, (w1 - 1) / WT_RANGE + 1 - w_range);
+    const int company = n_ranges > 1 ? cluster : 1;        // (one range: one CTA)
+    if (rank >= company) return;
+    auto first_of = [&](int n) {
+        const int at = (n < kept_ranges ? n : w_range + n - kept_ranges) * WT_RANGE;
+        return min(at, n_kept) + max(0, min(at, w1) - w0);
+    };
+    auto end_of = [&](int n) {
+        const int at = ((n < kept_ranges ? n : w_range + n - kept_ranges) + 1) * WT_RANGE;
+        return min(at, n_kept) + max(0, min(at, w1) - w0);
+    };
     auto block_at = [&](int i) { return (i < n_kept ? i : w0 + i - n_kept) * WT_K; };
     const int per = d / 4;
     // eight threads a row of a block, whose page is looked up a block ahead of its copies
     const int my_row = threadIdx.x / 8, my_c = threadIdx.x % 8 * 4;
-    auto page_of = [&](int i) { return i < n_blocks ? table[min(block_at(i) + my_row, p_last) / a.block_tokens] : 0; };
-    int page = page_of(0);
-    auto stage = [&](int i, int buf) {                     // blocks in order; keys past the last query's are zeros (their weights are)
-        const int pos = block_at(i) + my_row;
+    int next_range = rank, next = rank < n_ranges ? first_of(rank) : -1, next_end = rank < n_ranges ? end_of(rank) : 0;      // of this CTA's blocks: the one to copy next
+    auto page_of_next = [&]() { return next >= 0 ? table[min(block_at(next) + my_row, p_last) / a.block_tokens] : 0; };
+    int page = page_of_next();
+    auto stage = [&](int buf) {                            // keys past the last query's are zeros (their weights are)
+        if (next < 0) return;
+        const int pos = block_at(next) + my_row;
         const bool have = pos <= p_last;
         const size_t from = have ? (((size_t)page * a.G + g) * a.block_tokens + pos % a.block_tokens) * d : 0;
-        page = page_of(i + 1);
+        if (++next == next_end) {
+            next_range += company;
+            next = next_range < n_ranges ? first_of(next_range) : -1;
+            next_end = next_range < n_ranges ? end_of(next_range) : 0;
+        }
+        page = page_of_next();
         float *kd = ks + (buf * WT_K + my_row) * ldk, *vd = vs + (buf * WT_K + my_row) * d;
         for (int c = my_c; c < d; c += 32) {
             cp_async_16z(kd + c, k_pool + from + c, have ? 16 : 0);
@@ -1000,112 +1026,131 @@ __global__ void __launch_bounds__(WT_WARPS * 32, 1) window_attn_tile_kernel(Wind
         const float4 v = *reinterpret_cast<const float4*>(a.q_rot + ((size_t)(row0 + min(q, nq - 1)) * a.H + h) * d + c);
         *reinterpret_cast<float4*>(qs + q * ldk + c) = make_float4(v.x * a.scale, v.y * a.scale, v.z * a.scale, v.w * a.scale);
     }
-    stage(0, 0);
+    stage(0);
     cp_async_commit();
     const int pos = p0 + warp * 4 + part, lo = max(0, pos - a.window + 1);      // of the query whose scores this lane ends up with
-    float m = -INFINITY, l = 0.f;                          // of that query (l: this lane's keys)
-    float4 o[4];                                           // entries 4 lane .. of the warp's four queries
-#pragma unroll
-    for (int u = 0; u < 4; u++) o[u] = make_float4(0.f, 0.f, 0.f, 0.f);
     float* pw = ps + (half * 8 + warp) * WT_OWN * 4;
-    for (int i = 0; i < n_blocks; i++) {
-        const int buf = i & 1, j0 = block_at(i) + own;
-        cp_async_wait_all();
-        __syncthreads();                                   // this block has come, everybody has left the other buffer
-        if (i + 1 < n_blocks) stage(i + 1, buf ^ 1);
-        cp_async_commit();
-        float sc[4][4];                                    // [query][key of the group]
+    // state over ranges: this warp has queries rank + company * (its number of 16, and 16 more)
+    const int w16 = threadIdx.x >> 5;
+    float M[2] = {-INFINITY, -INFINITY}, L[2] = {0.f, 0.f};
+    float4 O[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+    int count = 0;
+    for (int n0 = 0; n0 < n_ranges; n0 += company) {
+        const int n = n0 + rank, i0 = n < n_ranges ? first_of(n) : 0, i1 = n < n_ranges ? end_of(n) : 0;
+        float m = -INFINITY, l = 0.f;                          // of this lane's query in the range (l: this lane's keys)
+        float4 o[4];                                           // entries 4 lane .. of the warp's four queries
 #pragma unroll
-        for (int u = 0; u < 4; u++)
-#pragma unroll
-            for (int v = 0; v < 4; v++) sc[u][v] = 0.f;
-        const float *qr = qs + warp * 4 * ldk + part * 4, *kr = ks + (buf * WT_K + own + kg * 4) * ldk + part * 4;
-#pragma unroll 4
-        for (int c = 0; c < d; c += 16) {
-            float4 q[4], k[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++) { q[u] = *reinterpret_cast<const float4*>(qr + u * ldk + c); k[u] = *reinterpret_cast<const float4*>(kr + u * ldk + c); }
+        for (int u = 0; u < 4; u++) o[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int i = i0; i < i1; i++) {
+            const int buf = count++ & 1, j0 = block_at(i) + own;
+            cp_async_wait_all();
+            __syncthreads();                                   // this block has come, everybody has left the other buffer
+            stage(buf ^ 1);
+            cp_async_commit();
+            if (warp * 4 >= nq) continue;                  // (none of the tile's: ten sequences of two tokens behind 1500 keys 387 -> 336 us)
+            float sc[4][4];                                    // [query][key of the group]
 #pragma unroll
             for (int u = 0; u < 4; u++)
 #pragma unroll
-                for (int v = 0; v < 4; v++) sc[u][v] += fmaf(q[u].x, k[v].x, fmaf(q[u].y, k[v].y, fmaf(q[u].z, k[v].z, q[u].w * k[v].w)));
-        }
-        // the four parts of every score: lane `part` ends up with query `part`
-        float s[4];
+                for (int v = 0; v < 4; v++) sc[u][v] = 0.f;
+            const float *qr = qs + warp * 4 * ldk + part * 4, *kr = ks + (buf * WT_K + own + kg * 4) * ldk + part * 4;
+#pragma unroll 4
+            for (int c = 0; c < d; c += 16) {
+                float4 q[4], k[4];
 #pragma unroll
-        for (int v = 0; v < 4; v++) {
-            const bool up = part & 2, odd = part & 1;
-            const float x0 = (up ? sc[2][v] : sc[0][v]) + __shfl_xor_sync(0xffffffffu, up ? sc[0][v] : sc[2][v], 2);
-            const float x1 = (up ? sc[3][v] : sc[1][v]) + __shfl_xor_sync(0xffffffffu, up ? sc[1][v] : sc[3][v], 2);
-            s[v] = (odd ? x1 : x0) + __shfl_xor_sync(0xffffffffu, odd ? x0 : x1, 1);
-        }
-        float mx = m;
-#pragma unroll
-        for (int v = 0; v < 4; v++) {
-            const int j = j0 + kg * 4 + v;
-            if (j > pos || (j < lo && j >= a.keep_first)) s[v] = -INFINITY;
-            mx = fmaxf(mx, s[v]);
-        }
-#pragma unroll
-        for (int w = 4; w < 32; w <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, w));
-        const float ref = mx > -INFINITY ? mx : 0.f, corr = m > -INFINITY ? expf(m - ref) : 0.f;      // (nothing visible yet: all weights are 0)
-        m = mx;
-        l *= corr;
-#pragma unroll
-        for (int v = 0; v < 4; v++) {
-            const float e = expf(s[v] - ref);
-            l += e;
-            pw[(kg * 4 + v) * 4 + part] = e;
-        }
-        __syncwarp();
-        float4 b[4];                                       // the block's own sums: short chains of additions
-#pragma unroll
-        for (int u = 0; u < 4; u++) b[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (4 * lane < d) {
-            const float* vr = vs + (buf * WT_K + own) * d + 4 * lane;
-            auto add = [&](int j, bool all) {
-                const float4 v = *reinterpret_cast<const float4*>(vr + j * d), p = *reinterpret_cast<const float4*>(pw + j * 4);
-                const float w[4] = {p.x, p.y, p.z, p.w};
+                for (int u = 0; u < 4; u++) { q[u] = *reinterpret_cast<const float4*>(qr + u * ldk + c); k[u] = *reinterpret_cast<const float4*>(kr + u * ldk + c); }
 #pragma unroll
                 for (int u = 0; u < 4; u++)
-                    if (all || w[u] != 0.f) { b[u].x = fmaf(w[u], v.x, b[u].x); b[u].y = fmaf(w[u], v.y, b[u].y); b[u].z = fmaf(w[u], v.z, b[u].z); b[u].w = fmaf(w[u], v.w, b[u].w); }
-            };
-            // (a key that some of the warp's queries do not see must not reach them, not even as 0 times infinity)
-            if (j0 + WT_OWN - 1 <= p0 + warp * 4 && j0 >= p0 + warp * 4 + 3 - a.window + 1) {
+#pragma unroll
+                    for (int v = 0; v < 4; v++) sc[u][v] += fmaf(q[u].x, k[v].x, fmaf(q[u].y, k[v].y, fmaf(q[u].z, k[v].z, q[u].w * k[v].w)));
+            }
+            // the four parts of every score: lane `part` ends up with query `part`
+            float s[4];
+#pragma unroll
+            for (int v = 0; v < 4; v++) {
+                const bool up = part & 2, odd = part & 1;
+                const float x0 = (up ? sc[2][v] : sc[0][v]) + __shfl_xor_sync(0xffffffffu, up ? sc[0][v] : sc[2][v], 2);
+                const float x1 = (up ? sc[3][v] : sc[1][v]) + __shfl_xor_sync(0xffffffffu, up ? sc[1][v] : sc[3][v], 2);
+                s[v] = (odd ? x1 : x0) + __shfl_xor_sync(0xffffffffu, odd ? x0 : x1, 1);
+            }
+            float mx = m;
+#pragma unroll
+            for (int v = 0; v < 4; v++) {
+                const int j = j0 + kg * 4 + v;
+                if (j > pos || (j < lo && j >= a.keep_first)) s[v] = -INFINITY;
+                mx = fmaxf(mx, s[v]);
+            }
+#pragma unroll
+            for (int w = 4; w < 32; w <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, w));
+            const float ref = mx > -INFINITY ? mx : 0.f, corr = m > -INFINITY ? expf(m - ref) : 0.f;      // (nothing visible yet: all weights are 0)
+            m = mx;
+            l *= corr;
+#pragma unroll
+            for (int v = 0; v < 4; v++) {
+                const float e = expf(s[v] - ref);
+                l += e;
+                pw[(kg * 4 + v) * 4 + part] = e;
+            }
+            __syncwarp();
+            float4 b[4];                                       // the block's own sums: short chains of additions
+#pragma unroll
+            for (int u = 0; u < 4; u++) b[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (4 * lane < d) {
+                const float* vr = vs + (buf * WT_K + own) * d + 4 * lane;
+                auto add = [&](int j, bool all) {
+                    const float4 v = *reinterpret_cast<const float4*>(vr + j * d), p = *reinterpret_cast<const float4*>(pw + j * 4);
+                    const float w[4] = {p.x, p.y, p.z, p.w};
+#pragma unroll
+                    for (int u = 0; u < 4; u++)
+                        if (all || w[u] != 0.f) { b[u].x = fmaf(w[u], v.x, b[u].x); b[u].y = fmaf(w[u], v.y, b[u].y); b[u].z = fmaf(w[u], v.z, b[u].z); b[u].w = fmaf(w[u], v.w, b[u].w); }
+                };
+                // (a key that some of the warp's queries do not see must not reach them, not even as 0 times infinity)
+                if (j0 + WT_OWN - 1 <= p0 + warp * 4 && j0 >= p0 + warp * 4 + 3 - a.window + 1) {
 #pragma unroll 8
-                for (int j = 0; j < WT_OWN; j++) add(j, true);
-            } else for (int j = 0; j < WT_OWN; j++) add(j, false);
-        }
+                    for (int j = 0; j < WT_OWN; j++) add(j, true);
+                } else for (int j = 0; j < WT_OWN; j++) add(j, false);
+            }
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const float f = __shfl_sync(0xffffffffu, corr, u);
-            o[u].x = fmaf(o[u].x, f, b[u].x); o[u].y = fmaf(o[u].y, f, b[u].y); o[u].z = fmaf(o[u].z, f, b[u].z); o[u].w = fmaf(o[u].w, f, b[u].w);
+            for (int u = 0; u < 4; u++) {
+                const float f = __shfl_sync(0xffffffffu, corr, u);
+                o[u].x = fmaf(o[u].x, f, b[u].x); o[u].y = fmaf(o[u].y, f, b[u].y); o[u].z = fmaf(o[u].z, f, b[u].z); o[u].w = fmaf(o[u].w, f, b[u].w);
+            }
+            __syncwarp();
         }
-        __syncwarp();
+        if (n < n_ranges) {
+#pragma unroll
+            for (int w = 4; w < 32; w <<= 1) l += __shfl_xor_sync(0xffffffffu, l, w);
+            if (4 * lane < d)
+#pragma unroll
+                for (int u = 0; u < 4; u++) *reinterpret_cast<float4*>(xs + (half * WT_Q + warp * 4 + u) * d + 4 * lane) = o[u];
+            if (kg == 0) xml[half * WT_Q + warp * 4 + part] = make_float2(m, l);
+        }
+        if (company > 1) cluster_sync();
+        else __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const int q = rank + company * (w16 + WT_WARPS * k);
+            if (q >= WT_Q) break;
+            for (int c = 0; c < company && n0 + c < n_ranges; c++) {
+                const uint32_t at = cluster_address(smem_u32(xs + q * d + (4 * lane < d ? 4 * lane : 0)), c), at_ml = cluster_address(smem_u32(xml + q), c);
+                const float2 x0 = cluster_load2(at_ml), x1 = cluster_load2(at_ml + WT_Q * 8);
+                const float4 y0 = cluster_load4(at), y1 = cluster_load4(at + WT_Q * d * 4);
+                const float top = fmaxf(M[k], fmaxf(x0.x, x1.x)), ref = top > -INFINITY ? top : 0.f;      // (nothing visible yet: all factors are 0)
+                const float f = expf(M[k] - ref), f0 = expf(x0.x - ref), f1 = expf(x1.x - ref);
+                M[k] = top;
+                L[k] = fmaf(L[k], f, fmaf(x0.y, f0, x1.y * f1));
+                O[k].x = fmaf(O[k].x, f, fmaf(y0.x, f0, y1.x * f1)); O[k].y = fmaf(O[k].y, f, fmaf(y0.y, f0, y1.y * f1));
+                O[k].z = fmaf(O[k].z, f, fmaf(y0.z, f0, y1.z * f1)); O[k].w = fmaf(O[k].w, f, fmaf(y0.w, f0, y1.w * f1));
+            }
+        }
+        if (company > 1) cluster_sync();                       // (nobody overwrites, or leaves, what another still reads)
+        else __syncthreads();
     }
 #pragma unroll
-    for (int w = 4; w < 32; w <<= 1) l += __shfl_xor_sync(0xffffffffu, l, w);
-    // the second half's maxima, sums and outputs, where the keys were
-    float4* other = reinterpret_cast<float4*>(ks) + warp * 4 * 32 + lane;      // [warp][query][lane]
-    float2* other_ml = reinterpret_cast<float2*>(ps) + warp * 4;
-    __syncthreads();
-    if (half == 1) {
-#pragma unroll
-        for (int u = 0; u < 4; u++) other[u * 32] = o[u];
-        if (kg == 0) other_ml[part] = make_float2(m, l);
-    }
-    __syncthreads();
-    if (half == 1) return;
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-        const float m0 = __shfl_sync(0xffffffffu, m, u), l0 = __shfl_sync(0xffffffffu, l, u);
-        const float2 ml = other_ml[u];
-        const float4 y = other[u * 32];
-        const float M = fmaxf(m0, ml.x), f0 = m0 > -INFINITY ? expf(m0 - M) : 0.f, f1 = ml.x > -INFINITY ? expf(ml.x - M) : 0.f, sum = fmaf(l0, f0, ml.y * f1);
-        const int q = warp * 4 + u;
+    for (int k = 0; k < 2; k++) {
+        const int q = rank + company * (w16 + WT_WARPS * k);
         if (q < nq && 4 * lane < d)
-            *reinterpret_cast<float4*>(a.out + ((size_t)(row0 + q) * a.H + h) * d + 4 * lane) =
-                make_float4(fmaf(o[u].x, f0, y.x * f1) / sum, fmaf(o[u].y, f0, y.y * f1) / sum, fmaf(o[u].z, f0, y.z * f1) / sum, fmaf(o[u].w, f0, y.w * f1) / sum);
+            *reinterpret_cast<float4*>(a.out + ((size_t)(row0 + q) * a.H + h) * d + 4 * lane) = make_float4(O[k].x / L[k], O[k].y / L[k], O[k].z / L[k], O[k].w / L[k]);
     }
 }
 // Heads of whole 16-entry pieces up to 128, rows on 16-byte boundaries.
@@ -1123,17 +1168,20 @@ cudaError_t window_attn_launch(const WindowAttnArgs& a, const RaggedDev& r, cuda
         if (a.d <= 64) return launch_chain(window_attn_mma_kernel<64>, dim3(r.n_tiles, a.H), dim3(128), smem, s, a, r);
         return launch_chain(window_attn_mma_kernel<128>, dim3(r.n_tiles, a.H), dim3(128), smem, s, a, r);
     }
-    if (window_attn_tiles(a, r.T)) {
-        // (tokens that come alone: a CTA per token and head, below)
-        const int alone = r.n_upto[0];
-        constexpr int most = ((WT_Q + 2 * WT_K) * (WT_D + 4) + 2 * WT_K * WT_D + WT_WARPS * WT_OWN * 4) * 4;
+    const int alone = r.n_upto[0];                         // (tokens that come alone: a CTA per token and head, below)
+    const bool tiles = window_attn_tiles(a, r.T) && r.n_tiles > alone;
+    if (tiles) {
+        constexpr int most = ((WT_Q + 2 * WT_K) * (WT_D + 4) + 2 * WT_K * WT_D + WT_WARPS * WT_OWN * 4 + 2 * WT_Q * (WT_D + 2)) * 4;
         if (!allow_smem<window_attn_tile_kernel>(most)) return cudaErrorInvalidValue;
-        const size_t smem = (size_t)((WT_Q + 2 * WT_K) * (a.d + 4) + 2 * WT_K * a.d + WT_WARPS * WT_OWN * 4) * 4;
-        if (r.n_tiles > alone) {
-            const cudaError_t e = launch_chain(window_attn_tile_kernel, dim3((r.n_tiles - alone) * 2, a.H), dim3(WT_WARPS * 32), smem, s, a, r, alone);
-            if (e != cudaSuccess) return e;
-        }
-        return alone ? launch_chain(window_attn_pairs_kernel<true>, dim3(alone, a.H), dim3(ATT2_WARPS * 32), 0, s, a, r, 1) : cudaSuccess;
+        const size_t smem = (size_t)((WT_Q + 2 * WT_K) * (a.d + 4) + 2 * WT_K * a.d + WT_WARPS * WT_OWN * 4 + 2 * WT_Q * (a.d + 2)) * 4;
+        // as many CTAs a tile as fit side by side in clusters (of 8: 128), and no more than a window has ranges
+        const int n = (r.n_tiles - alone) * 2 - (r.n_upto[5] - alone), ranges = (int)std::min<long long>(8, ((long long)a.window + a.keep_first + WT_Q) / (WT_RANGE * WT_K) + 2);
+        int company = 1;
+        while (company < 8 && company < ranges && n * a.H * company * 2 <= 128) company *= 2;
+        const dim3 grid((r.n_tiles - alone) * 2 * company, a.H), block(WT_WARPS * 32);
+        const cudaError_t e = company > 1 ? launch_chain_cluster(window_attn_tile_kernel, company, grid, block, smem, s, a, r, alone, company)
+                                          : launch_chain(window_attn_tile_kernel, grid, block, smem, s, a, r, alone, company);
+        if (e != cudaSuccess || alone == 0) return e;
     }
     if (a.d % 2 == 0) {
         // a step of a few tokens does not fill the GPU with one CTA per (token, head): split the keys (up to 16 ranges)
@@ -1142,11 +1190,11 @@ cudaError_t window_attn_launch(const WindowAttnArgs& a, const RaggedDev& r, cuda
             splits = std::min(16, (2 * 148) / (r.T * a.H));
             while (splits > 1 && (size_t)r.T * a.H * splits * (a.d + 2) > (size_t)a.split_capacity) splits--;
         }
-        const dim3 grid(r.T, a.H, splits);
-        cudaError_t ce = a.cache_f32 ? launch_chain(window_attn_pairs_kernel<true>, grid, dim3(ATT2_WARPS * 32), 0, s, a, r, 0)
+        const dim3 grid(tiles ? alone : r.T, a.H, splits);
+        cudaError_t ce = a.cache_f32 ? launch_chain(window_attn_pairs_kernel<true>, grid, dim3(ATT2_WARPS * 32), 0, s, a, r, tiles ? 1 : 0)
                                      : launch_chain(window_attn_pairs_kernel<false>, grid, dim3(ATT2_WARPS * 32), 0, s, a, r, 0);
         if (ce != cudaSuccess || splits == 1) return ce;
-        return launch_chain(window_attn_merge_kernel, dim3(r.T, a.H), dim3(128), 0, s, a, splits);
+        return launch_chain(window_attn_merge_kernel, dim3(grid.x, a.H), dim3(128), 0, s, a, r, splits, tiles ? 1 : 0);
     }
     return launch_chain(window_attn_kernel, dim3(r.T, a.H), dim3(ATT_WARPS * 32), 0, s, a, r);
 }

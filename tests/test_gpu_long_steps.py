@@ -78,28 +78,30 @@ def test_window_attention_of_long_steps(native_lib, tmp_path, d, window, keep, l
     check(gu, goponex_ref, cfg, tmp_path, lengths, "bfloat16")
 
 
-# the same over 32-bit pages: tiles of 32 queries, blocks of 32 keys; tokens that come alone
-@pytest.mark.parametrize("d,window,keep,lengths", [(16, 1, 0, [33]), (64, 64, 3, [257]), (80, 100, 70, [200]), (128, 129, 1, [300, 1, 31]), (32, 1000, 4, [100, 64, 2]),
+# the same over 32-bit pages: tiles of 32 queries, ranges of 128 keys; tokens that come alone
+@pytest.mark.parametrize("d,window,keep,lengths", [(16, 1, 0, [33]), (64, 64, 3, [257]), (80, 100, 70, [200]), (128, 129, 1, [300, 1, 31]), (32, 1000, 4, [100, 64, 2]), (128, 700, 300, [900]), (64, 3000, 1, [1100]),
                                                   (112, 20, 40, [1, 2, 31, 33, 64, 65])])
 def test_window_attention_of_long_steps_in_32_bits(native_lib, tmp_path, d, window, keep, lengths):
     cfg = gu.config([gu.parallel(left=gu.attn(heads=4, kv_heads=2, dim=d, rot=8, window=window, keep=keep))])
     check(gu, goponex_ref, cfg, tmp_path, lengths, "float32")
 
 
-def test_cuts_do_not_change_a_token_in_32_bits(native_lib, tmp_path):
-    """Window attention over 32-bit pages: in portions of two tokens and more, each in a step of more than 8, a prompt's logits have the bits of the whole."""
+@pytest.mark.parametrize("n,window,keep", [(200, 70, 5), (900, 600, 300)])
+def test_cuts_do_not_change_a_token_in_32_bits(native_lib, tmp_path, n, window, keep):
+    """Window attention over 32-bit pages: in portions of two tokens and more, each in a step of more than 8, a prompt's logits have the bits of the whole
+    (the longer one: with one to eight CTAs a tile, over one to eight ranges of keys)."""
     from llama_cpp.kv_pages import SequenceSlots
-    cfg = gu.config([gu.parallel(left=gu.attn(heads=4, kv_heads=2, dim=64, rot=8, window=70, keep=5))])
-    eng = engine(gu.write_model(str(tmp_path / "m"), cfg, gu.random_weights(cfg, seed=9)), "float32", 300, 2)
-    prompt, side = toks(cfg["vocab"], 200, 1), toks(cfg["vocab"], 90, 2)
+    cfg = gu.config([gu.parallel(left=gu.attn(heads=4, kv_heads=2, dim=64, rot=8, window=window, keep=keep))])
+    eng = engine(gu.write_model(str(tmp_path / "m"), cfg, gu.random_weights(cfg, seed=9)), "float32", n + 100, 2)
+    prompt, side = toks(cfg["vocab"], n, 1), toks(cfg["vocab"], 90, 2)
     rows = []
-    for cuts in ([200], [33, 167], [2, 60, 7, 131], [64, 64, 72]):
+    for cuts in ([n], [33, n - 33], [2, 60, 7, n - 69], [n - 72, 64, 8]):
         seqs, got, at = SequenceSlots(eng), [], 0
         seqs.open(0), seqs.open(1)
-        for k, n in enumerate(cuts):
-            entries = [(seqs.extend(0, n), prompt[at:at + n]), (seqs.extend(1, 20), side[20 * k:20 * k + 20])]
-            got.append(np.array(eng.step(entries, want=[list(range(n)), list(range(20))])[0])[:n])      # (more than 8 rows for the head: one form of it)
-            at += n
+        for k, c in enumerate(cuts):
+            entries = [(seqs.extend(0, c), prompt[at:at + c]), (seqs.extend(1, 20), side[20 * k:20 * k + 20])]
+            got.append(np.array(eng.step(entries, want=[list(range(c)), list(range(20))])[0])[:c])      # (more than 8 rows for the head: one form of it)
+            at += c
         seqs.close(0), seqs.close(1)
         rows.append(np.concatenate(got))
     eng.close()
