@@ -304,6 +304,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) latent_attn_tc_kernel(const __g
             for (int j = 0; j < HALF; j++) s[j] = __uint_as_float(raw[j]);
             if constexpr (PAIR) {                              // a sum of two: the same in both CTAs
                 mbar_wait(&x_full[st], phase, err, 0x6000bu, (unsigned)i);
+                __syncwarp();
 #pragma unroll
                 for (int j = 0; j < HALF / 4; j++) {
                     const float4 x = xs[(st * (LC_K / 4) + side * (HALF / 4) + j) * LC_Q + row];
