@@ -120,8 +120,12 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const __
             tc_after_sync();
             if (!one) continue;
             const uint64_t dv = tc_desc(va + (i & 1) * PARTS * PT_PART, PT_PART);
+            // 16 keys a product: queries ahead of all of them take no part (a value that is no number would reach them through a weight of 0)
 #pragma unroll
-            for (int k = 0; k < PT_K / 16; k++) tc_mma_ts(o_at, p_at + (i & 1) * (PT_K / 2) + k * 8, dv + k * (2048 >> 4), id_o, (i | k) ? 1u : 0u);
+            for (int k = 0; k < PT_K / 16; k++) {
+                const int j = i * PT_K + 16 * k;
+                if (j <= p_last) tc_mma_ts_from_row(o_at, p_at + (i & 1) * (PT_K / 2) + k * 8, dv + k * (2048 >> 4), id_o, (i | k) ? 1u : 0u, j - p0);
+            }
             tc_commit(&pv_done[i & 1]);
             tc_commit(&v_empty[i & 1]);
             if (i == n_blocks - 1) tc_commit(&o_full);
@@ -185,10 +189,10 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const __
             __syncwarp();
             tc_st32(p_at + st * (PT_K / 2) + side * 32 + lanes, p);
             tc_wait_st();
-            if (i == n_blocks - 1 && p_last - j0 + 1 < PT_K) {
-                // rows past the sequence: whatever shared memory or the page holds must not meet the zero weights as values
+            if (i == n_blocks - 1 && (p_last + 1) % 16) {
+                // rows past the sequence in the last 16 that are multiplied: whatever the page holds must not meet the zero weights as values
                 mbar_wait(&v_full[st], phase, err, 0x80009u, (unsigned)i);
-                const int r0 = p_last - j0 + 1, n_bad = PT_K - r0;
+                const int r0 = p_last - j0 + 1, n_bad = 16 - r0 % 16;
                 for (int e = threadIdx.x; e < PARTS * n_bad * 8; e += 256) {
                     const int c = e / (n_bad * 8), rr = r0 + e / 8 % n_bad;
                     *reinterpret_cast<uint4*>(vs + (st * PARTS + c) * PT_PART + rr * 128 + (e & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);

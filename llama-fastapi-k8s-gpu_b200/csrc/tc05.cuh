@@ -23,6 +23,14 @@ __device__ __forceinline__ void tc_mma_ts(uint32_t d, uint32_t a, uint64_t b, ui
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
                  ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
 }
+// the same with the first `skip` rows of D (lanes of tensor memory) left as they are
+__device__ __forceinline__ void tc_mma_ts_from_row(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate, int skip) {
+    uint32_t off[4];
+#pragma unroll
+    for (int w = 0; w < 4; w++) { const int n = skip - 32 * w; off[w] = n <= 0 ? 0u : n >= 32 ? 0xffffffffu : (1u << n) - 1u; }
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}"
+                 ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(off[0]), "r"(off[1]), "r"(off[2]), "r"(off[3]) : "memory");
+}
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }

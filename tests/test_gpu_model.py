@@ -391,3 +391,45 @@ def test_prompts_over_pages_of_64(native_lib, tmp_models, arch, portions):
         assert np.abs(eng.logits(0) - ref[at - 1]).max() <= LOGIT_TOL, at
     eng.close()
 
+
+@pytest.mark.parametrize("arch", ["tiny", "tiny128"])
+@pytest.mark.parametrize("portions,at,keep", [((200,), 100, 64), ((200,), 191, 176), ((130, 70), 150, 144), ((140, 64, 30), 203, 192), ((64, 120), 130, 128)])
+def test_a_token_without_numbers_reaches_no_token_ahead_of_it(native_lib, tmp_models, arch, portions, at, keep):
+    """A token whose keys and values are no numbers (they overflowed 16 bits, say), in the block of 128 keys that earlier ones read: what is cached of those
+    has the bits that it has with any other token there. So does what is continued over pages that hold its rows."""
+    from llama_cpp.gguf_file import GGUFFile
+    path, bad = _model(tmp_models, arch, "Q8_0", 3), 699
+    nan = path + ".nan"
+    with open(path, "rb") as f:
+        raw = bytearray(f.read())
+    table = GGUFFile(path).tensors["token_embd.weight"]
+    row = table.shape[0] // 32 * 34                            # bytes of a token's blocks: a scale, 32 weights
+    for b in range(table.offset + bad * row, table.offset + (bad + 1) * row, 34):
+        raw[b:b + 2] = np.float16(np.nan).tobytes()
+    with open(nan, "wb") as f:
+        f.write(raw)
+    n = sum(portions)
+    prompt = [int(t) for t in np.random.default_rng(n).integers(3, 699, size=n)]
+    more = [int(t) for t in np.random.default_rng(1).integers(3, 699, size=140)]
+    got = []
+    for there in (prompt[at], bad):
+        eng = _engine(nan, n_ctx=n + 200, bt=64)
+        eng.ensure_pages(0, n + 150)
+        eng.seq_begin(0, 0, [], _greedy())
+        i = 0
+        for k in portions:
+            eng.prefill(0, [there if j == at else prompt[j] for j in range(i, i + k)])
+            i += k
+        got.append([eng.logits(0).copy()])
+        for first in (1, 9, 131):                              # a step, a short portion, a long one over what the pages hold
+            eng.rewind(0, keep, more[0], prompt[:keep])
+            if first == 1:
+                eng.forward_pending(0)
+            else:
+                eng.prefill(0, more[:first])
+            got[-1].append(eng.logits(0).copy())
+        eng.close()
+    os.remove(nan)
+    assert np.isfinite(got[0]).all() and np.isnan(got[1][0]).all()
+    for a, b in zip(got[0][1:], got[1][1:]):
+        assert np.array_equal(a, b)
