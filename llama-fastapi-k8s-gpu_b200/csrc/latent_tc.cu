@@ -13,8 +13,8 @@
 // while the softmax of two blocks runs. The output is rescaled only when a row's maximum has grown by more than 2^8.
 // Bound by shared memory, which holds every operand but the probabilities and a quarter of the queries and passes the score parts on (about 190 KB a block and CTA,
 // 1500 of its 2900 cycles), and by what a CTA costs beside its blocks: 9000 cycles, four times in 2048 tokens.
-// 2048 tokens, 16 heads (B200), us a layer: rows of 512 + 64 1640 with mma.sync, 207 with both CTAs computing all scores, 158 here; rows of 512, nothing
-// rotated, 170 and 120. (Six warps and one thread a query: 180, 165. An arrival at the other CTA with a release to the cluster: 500 more cycles a block. Four
+// 2048 tokens, 16 heads (B200), us a layer: rows of 512 + 64 1640 with mma.sync, 207 with both CTAs computing all scores, 149 here; rows of 512, nothing
+// rotated, 170 and 130. (Six warps and one thread a query: 180, 165. One barrier a block for all rows of the score parts: 163, 139. Four
 // tiles of 32 scores with all of the queries in tensor memory: 182, 140: a product takes 50 to 70 cycles whether 32 or 64 keys wide.)
 #include "kernels.h"
 #include "latent_dev.cuh"
@@ -54,7 +54,8 @@ __global__ void __launch_bounds__(LC_THREADS, 1) latent_attn_tc_kernel(const __g
                                                                        const __grid_constant__ CUtensorMap map_h, const LatentAttnArgs a, const RaggedDev r,
                                                                        const LcPlan plan, __nv_bfloat16* out, unsigned int* err) {
     extern __shared__ uint8_t lc_smem[];
-    __shared__ uint64_t rest_full[2], val_full[LC_NV], rest_empty[2], val_empty[LC_NV], q_come, q_full, s_full[2], s_read[2], p_full[2], pv_done[2], x_full[2], x_empty[2], o_full;
+    __shared__ uint64_t rest_full[2], val_full[LC_NV], rest_empty[2], val_empty[LC_NV], q_come, q_full, s_full[2], s_read[2], p_full[2], pv_done[2], o_full;
+    __shared__ uint64_t x_full[2][4], x_taken[2][4], x_empty[2][4];      // PAIR: [stage][32 rows]
     __shared__ uint32_t tmem_at;
     __shared__ float both[2][LC_Q];                        // what the two threads of a row tell each other (one buffer: shared memory is full)
     constexpr int CHUNKS = PAIR ? 2 : 1;
@@ -81,8 +82,9 @@ __global__ void __launch_bounds__(LC_THREADS, 1) latent_attn_tc_kernel(const __g
         else if (lane < LC_NV + 2) {
             const int i = lane - LC_NV;
             mbar_init(&rest_full[i], 1); mbar_init(&rest_empty[i], 1); mbar_init(&s_full[i], 1); mbar_init(&s_read[i], PAIR ? 384 : 256); mbar_init(&p_full[i], 256);
-            mbar_init(&pv_done[i], 1); mbar_init(&x_full[i], 1); mbar_init(&x_empty[i], 8);
+            mbar_init(&pv_done[i], 1);
         } else if (lane == LC_NV + 2) { mbar_init(&q_come, 1); mbar_init(&q_full, 256); mbar_init(&o_full, 1); }
+        if (PAIR && lane < 8) { mbar_init(&x_full[0][0] + lane, 1); mbar_init(&x_taken[0][0] + lane, 2); mbar_init(&x_empty[0][0] + lane, 1); }
         fence_mbar_init();
         __syncwarp();
         tc_alloc(&tmem_at, 512);
@@ -254,9 +256,11 @@ __global__ void __launch_bounds__(LC_THREADS, 1) latent_attn_tc_kernel(const __g
     } else if (warp >= 8) {
         // ================= this CTA's parts of the scores, to the other's shared memory
         if constexpr (PAIR) {
-            const int row = threadIdx.x & 127;
-            const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
-            const uint32_t to = cluster_address(smem_u32(xs) + row * 16, chunk ^ 1), bar = cluster_address(smem_u32(x_full), chunk ^ 1);
+            // (a warp sends 32 rows, which two softmax warps read there; the barriers of other rows are not its own)
+            const int row = threadIdx.x & 127, rows = warp & 3;
+            const uint32_t lanes = (uint32_t)(rows * 32) << 16;
+            const uint32_t to = cluster_address(smem_u32(xs) + row * 16, chunk ^ 1), bar = cluster_address(smem_u32(x_full) + rows * 8, chunk ^ 1);
+            const uint32_t x_free = cluster_address(smem_u32(x_empty) + rows * 8, chunk ^ 1);
             cluster_wait();
             for (int i = 0; i < n_blocks; i++) {
                 const int st = i & 1;
@@ -269,9 +273,16 @@ __global__ void __launch_bounds__(LC_THREADS, 1) latent_attn_tc_kernel(const __g
                 tc_wait_ld();
                 tc_before_sync();
                 mbar_arrive(&s_read[st]);
-                if (i > 1) mbar_wait(&x_empty[st], ((i >> 1) - 1) & 1, err, 0x60009u, (unsigned)i);
+                if (i > 1) {
+                    // each may send this block's parts once the softmax warps over there have read those of the block before last. (The arrival orders for
+                    // the cluster and waits for what its warp has under way: by a softmax warp it took 1500 cycles; ahead of the scores 160 and 129 us)
+                    const uint32_t phase = ((i >> 1) - 1) & 1;
+                    mbar_wait_warp(&x_taken[st][rows], phase, err, 0x60010u, (unsigned)i);
+                    if (lane == 0) mbar_arrive_cluster(x_free + st * 32);
+                    mbar_wait_cluster(&x_empty[st][rows], phase, err, 0x60009u, (unsigned)i);
+                }
 #pragma unroll
-                for (int j = 0; j < 16; j++) st_async_16(to + st * LC_XPART + j * (LC_Q * 16), &raw[j >> 3][(j & 7) * 4], bar + st * 8);
+                for (int j = 0; j < 16; j++) st_async_16(to + st * LC_XPART + j * (LC_Q * 16), &raw[j >> 3][(j & 7) * 4], bar + st * 32);
             }
         }
     } else {
@@ -281,9 +292,8 @@ __global__ void __launch_bounds__(LC_THREADS, 1) latent_attn_tc_kernel(const __g
         const int t = packed ? row0 : row0 + row, hd = packed ? min(row, a.H - 1) : h;      // the row's token and head
         const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
         const int my_cols = n_val * LC_PART / 2, col0 = side * my_cols;                    // of the output
-        [[maybe_unused]] const uint32_t x_free = PAIR ? cluster_address(smem_u32(x_empty), chunk ^ 1) : 0u;
         if constexpr (PAIR) {
-            if (threadIdx.x == 0) for (int i = 0; i < 2; i++) mbar_arrive_expect_tx(&x_full[i], LC_XPART);
+            if (warp < 4 && lane == 0) for (int i = 0; i < 2; i++) mbar_arrive_expect_tx(&x_full[i][warp], LC_XPART / 4);
             cluster_wait();
         }
         constexpr float LOG2E = 1.4426950408889634f;
@@ -303,12 +313,17 @@ __global__ void __launch_bounds__(LC_THREADS, 1) latent_attn_tc_kernel(const __g
 #pragma unroll
             for (int j = 0; j < HALF; j++) s[j] = __uint_as_float(raw[j]);
             if constexpr (PAIR) {                              // a sum of two: the same in both CTAs
-                mbar_wait(&x_full[st], phase, err, 0x6000bu, (unsigned)i);
+                mbar_wait_cluster(&x_full[st][warp & 3], phase, err, 0x6000bu, (unsigned)i);
                 __syncwarp();
 #pragma unroll
                 for (int j = 0; j < HALF / 4; j++) {
                     const float4 x = xs[(st * (LC_K / 4) + side * (HALF / 4) + j) * LC_Q + row];
                     s[4 * j] += x.x; s[4 * j + 1] += x.y; s[4 * j + 2] += x.z; s[4 * j + 3] += x.w;
+                }
+                __syncwarp();
+                if (i + 2 < n_blocks && lane == 0) {           // this warp has read its share
+                    if (warp < 4) mbar_arrive_expect_tx(&x_full[st][warp], LC_XPART / 4);
+                    mbar_arrive(&x_taken[st][warp & 3]);
                 }
             }
 #pragma unroll
@@ -324,10 +339,6 @@ __global__ void __launch_bounds__(LC_THREADS, 1) latent_attn_tc_kernel(const __g
             named_bar_sync(1 + (warp & 3), 64);                   // (the two warps of these rows) the last block's maxima have been read
             both[side][row] = mx;
             named_bar_sync(1 + (warp & 3), 64);
-            if (PAIR && i + 2 < n_blocks && lane == 0) {             // other parts may come in their place: the maxima above took everything these ones held
-                if (warp == 0) mbar_arrive_expect_tx(&x_full[st], LC_XPART);
-                mbar_arrive_cluster(x_free + st * 8);
-            }
             mx = fmaxf(mx, both[side ^ 1][row]);
             const bool grow = mx > m_ref + 8.f || (m_ref == -INFINITY && mx > -INFINITY);
             const float m_old = m_ref;

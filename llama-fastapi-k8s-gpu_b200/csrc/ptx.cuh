@@ -97,8 +97,7 @@ __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
-// ---- thread-block clusters: all threads of all CTAs meet (ordering nothing but what a fence before it orders); an address in CTA `rank`'s shared memory; an arrival at a barrier there (ordered like one at
-// home: with a release to the whole cluster it held its warp for 1500 cycles. What precedes it must have completed: reads, by what depends on them)
+// ---- thread-block clusters: all threads of all CTAs meet (ordering nothing but what a fence before it orders); an address in CTA `rank`'s shared memory
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 // the same with what was written to shared memory before it visible to the cluster behind it
@@ -118,8 +117,17 @@ __device__ __forceinline__ float2 cluster_load2(uint32_t address) {
     asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(address) : "memory");
     return v;
 }
+// an arrival at another CTA's barrier: what its thread has done and seen before is before what whoever waits with mbar_wait_cluster does next
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// the wait for a barrier that another CTA arrives at, or counts bytes of (st_async_16)
+__device__ __forceinline__ void mbar_wait_cluster(uint64_t* bar, uint32_t parity, unsigned int* err, unsigned int code, unsigned int info = 0) {
+    for (uint32_t spins = 0, ok = 0; !ok;) {
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+        if (!ok && ++spins > (1u << 22)) { mbar_give_up(parity, err, code, info); return; }
+    }
 }
 // 16 bytes into another CTA's shared memory, counted by a barrier there
 __device__ __forceinline__ void st_async_16(uint32_t to, const uint32_t* v, uint32_t bar) {

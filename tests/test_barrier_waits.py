@@ -68,3 +68,33 @@ def host_lib(tmp_path_factory, made=[]):
         subprocess.run(["g++", "-O2", "-fPIC", "-shared", os.path.join(CSRC, "host_selftest.cpp"), "-o", out], check=True)
         made.append(ctypes.CDLL(out))
     return made[0]
+
+
+CLUSTER_FILES = sorted(f for f in os.listdir(CSRC) if f.endswith(".cu") and "cluster_address(" in open(os.path.join(CSRC, f)).read())
+
+
+def test_arrivals_at_another_ctas_barrier_order_for_the_cluster():
+    """An arrival without a scope orders for its own CTA only: reads of what the other CTA then overwrites could still be under way."""
+    text = open(os.path.join(CSRC, "ptx.cuh")).read()
+    arrivals = re.findall(r"mbarrier\.arrive[\w.:]*shared::cluster[\w.:]*", text)
+    assert arrivals and all(".release.cluster." in a for a in arrivals)
+    assert "mbarrier.try_wait.parity.acquire.cluster." in text[text.index("void mbar_wait_cluster"):]
+
+
+@pytest.mark.parametrize("name", CLUSTER_FILES)
+def test_barriers_that_another_cta_reaches_are_waited_for_in_the_cluster(name):
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, name)).read())
+    barriers = set(re.findall(r"cluster_address\(smem_u32\(&?(\w+)", text)) & set(re.findall(r"mbar_init\(&(\w+)", text))
+    assert barriers or "st_async_16(" not in text
+    for b in barriers:
+        waits = re.findall(r"\b(mbar_wait\w*)\(&%s\b" % b, text)
+        assert waits and set(waits) == {"mbar_wait_cluster"}, (b, waits)
+
+
+def test_score_parts_are_given_back_after_they_have_been_read():
+    """latent_tc.cu: each warp's own arrival at x_taken comes after its reads of the other CTA's parts, and the arrival there after all of these."""
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, "latent_tc.cu")).read())
+    read, taken = text.rindex("xs["), text.index("mbar_arrive(&x_taken")
+    assert read < text.index("__syncwarp()", read) < taken
+    wait, give = text.index("mbar_wait_warp(&x_taken"), text.index("mbar_arrive_cluster(")
+    assert wait < give and text.count("mbar_arrive_cluster(") == 1 and "(&x_empty" in text[give:]
