@@ -2,7 +2,8 @@
 
   lib/libb200gguf.so       CUDA kernels + C ABI (include/b200_gguf.h), nvcc, sm_100a only
   lib/libb200_hosttest.so  host build of the block arithmetic (CPU self-test, g++)
-  lib/libb200_pylists.so   Python lists to C arrays (g++, Python's headers; without them the package converts in Python)
+  lib/libb200_pylists.<interpreter>.so   Python lists to C arrays (g++, Python's headers; without them the package converts in Python). Its code knows how
+                           this interpreter lays its objects out, so the name ends as its own extension modules' do and another one builds another
 
 nvcc cross-compiles without a GPU; the .so files are git-ignored but travel to the GPU box.
 """
@@ -71,7 +72,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     hsrc = os.path.join(CSRC, "host_selftest.cpp")
     if force or _newer(host, [hsrc, os.path.join(CSRC, "quant_blocks.cuh"), os.path.join(CSRC, "gemm_ring.h"), os.path.join(CSRC, "per_device.h")]):
         subprocess.run(["g++", "-O2", "-ffp-contract=off", "-fPIC", "-shared", hsrc, "-o", host], check=True)
-    lists, lsrc, include = os.path.join(LIB, "libb200_pylists.so"), os.path.join(CSRC, "py_lists.cpp"), sysconfig.get_paths()["include"]
+    lists, lsrc, include = os.path.join(LIB, "libb200_pylists" + sysconfig.get_config_var("EXT_SUFFIX")), os.path.join(CSRC, "py_lists.cpp"), sysconfig.get_paths()["include"]
     if os.path.exists(os.path.join(include, "Python.h")) and (force or _newer(lists, [lsrc])):
         subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-I", include, lsrc, "-o", lists], check=True)
     return out

@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import sysconfig
 from ctypes import POINTER, c_char_p, c_double, c_float, c_int, c_int32, c_int64, c_void_p
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
@@ -140,11 +141,14 @@ _lists = False
 
 
 def load_lists() -> ctypes.PyDLL | None:
-    """libb200_pylists.so: Python lists to C arrays, and a step's lists together with the call; None where it has not been built (no Python headers)."""
+    """libb200_pylists: Python lists to C arrays, and a step's lists together with the call; None where it has not been built for this interpreter (no
+    Python headers, a library of another one) or does not load."""
     global _lists
     if _lists is False:
-        path = os.path.join(os.path.dirname(LIB_PATH), "libb200_pylists.so")
-        lib = ctypes.PyDLL(path) if os.path.exists(path) else None
+        try:
+            lib = ctypes.PyDLL(os.path.join(os.path.dirname(LIB_PATH), "libb200_pylists" + sysconfig.get_config_var("EXT_SUFFIX")))
+        except OSError:
+            lib = None
         if lib:
             lib.b2_py_int32s.restype, lib.b2_py_int32s.argtypes = c_int, [ctypes.py_object, c_void_p, ctypes.c_ssize_t]
             lib.b2_py_step.restype = ctypes.py_object

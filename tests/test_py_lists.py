@@ -1,6 +1,9 @@
 """Lists that native code converts: the same calls and results as the conversion in Python, on the CPU (the native step is a recording stand-in)."""
 import ctypes
+import os
 import random
+import shutil
+import sysconfig
 
 import numpy as np
 import pytest
@@ -75,3 +78,27 @@ def test_int_arrays():
     for values in ([], [3] * 12, list(range(-20, 20)), tuple(range(40)), [2 ** 31 - 1, -2 ** 31] * 8, [np.int64(3)] * 20, [True] * 13, range(30), np.arange(20)):
         assert list(int32s(values)) == [int(v) for v in values]
     assert list(int32s([2 ** 32 + 5] * 20)) == [5] * 20        # (ctypes keeps the low bits; the engine then checks the range)
+
+
+def load_from(folder, monkeypatch):
+    monkeypatch.setattr(_cabi, "LIB_PATH", str(folder / "libb200gguf.so"))
+    monkeypatch.setattr(_cabi, "_lists", False)
+    return _cabi.load_lists()
+
+
+def test_a_library_of_another_interpreter_is_not_loaded(tmp_path, monkeypatch):
+    """What it compiled in of CPython's objects holds for the interpreter whose headers it was built with."""
+    built = [f for f in os.listdir(os.path.dirname(_cabi.LIB_PATH)) if f.startswith("libb200_pylists") and sysconfig.get_config_var("SOABI") in f]
+    assert len(built) == 1
+    whole = os.path.join(os.path.dirname(_cabi.LIB_PATH), built[0])
+    for name in ("libb200_pylists.so", "libb200_pylists.cpython-39-x86_64-linux-gnu.so"):
+        shutil.copy(whole, tmp_path / name)
+    assert load_from(tmp_path, monkeypatch) is None
+    shutil.copy(whole, tmp_path / built[0])
+    assert load_from(tmp_path, monkeypatch) is not None
+
+
+def test_a_library_that_does_not_load_is_none(tmp_path, monkeypatch):
+    (tmp_path / ("libb200_pylists" + sysconfig.get_config_var("EXT_SUFFIX"))).write_bytes(b"not a library")
+    assert load_from(tmp_path, monkeypatch) is None
+    assert list(int32s(list(range(30)))) == list(range(30))
