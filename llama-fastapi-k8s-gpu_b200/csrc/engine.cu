@@ -759,7 +759,7 @@ static int gemm_call(b2_engine* e, const DevTensor* const* ws, int nw, const __h
     GemmParams& p = it->second;
     if (p.x != x || p.y != e->pf_part) return fail(B2_ERR_STATE, "GEMM plan cache: workspace moved");
     CK(gemm_launch(p, e->stream));
-    e->launches++;
+    e->launches += p.n_rest > 0 ? 2 : 1;
     *n_parts = p.n_splits; *part_stride = p.split_stride;
     return B2_OK;
 }

@@ -433,3 +433,17 @@ def test_a_token_without_numbers_reaches_no_token_ahead_of_it(native_lib, tmp_mo
     assert np.isfinite(got[0]).all() and np.isnan(got[1][0]).all()
     for a, b in zip(got[0][1:], got[1][1:]):
         assert np.array_equal(a, b)
+
+
+def test_launches_of_a_prompt_are_counted(native_lib, tmp_models, monkeypatch):
+    """A prompt of one layer is 13 kernels; above 256 tokens gate and up, two row tiles more than a whole wave of 74, are two launches."""
+    from llama_cpp import synth
+    monkeypatch.setitem(synth.ARCHS, "tiny-ff", synth.Arch("tiny-ff", 1, 256, 4, 2, 38 * 256, 1024))
+    eng = _engine(_model(tmp_models, "tiny-ff", "Q8_0", 1), n_ctx=600, bt=64)
+    for n, kernels in ((256, 13), (257, 14), (512, 14)):
+        eng.ensure_pages(0, n)
+        eng.seq_begin(0, 0, [], _greedy())
+        before = eng.launch_count()
+        eng.prefill(0, [5 + i % 600 for i in range(n)])
+        assert eng.launch_count() - before == kernels, n
+    eng.close()
