@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) latent_attn_tc_kernel(const __g
         for (int i = 0; i < n_blocks; i++) {
             const int j0 = (b0 + i) * LC_K, row = table[j0 / a.block_tokens] * a.block_tokens + j0 % a.block_tokens;
             if (n_rest > 0) {
-                if (ur > 0) mbar_wait_warp(&rest_empty[sr], (ur - 1) & 1, err, 0x60001u, (unsigned)i);
+                if (ur > 0) mbar_wait_warp(&rest_empty[sr], (ur - 1) & 1, err, 0x60011u, (unsigned)i);
                 if (one) {
                     mbar_arrive_expect_tx(&rest_full[sr], (uint32_t)(n_rest * LC_KPART));
                     for (int c = 0; c < n_rest; c++) tma_load_3d(rs + (size_t)(sr * n_rest + c) * LC_KPART, &map_k, (rest0 + c) * LC_PART, row, 0, &rest_full[sr]);
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) latent_attn_tc_kernel(const __g
             if (++sv == NV) sv = 0;
             if (sv == 1) uv++;
         };
-        mbar_wait_warp(&q_come, 0, err, 0x6000eu);
+        mbar_wait_warp(&q_come, 0, err, 0x60012u);
         mbar_wait_warp(&q_full, 0, err, 0x60006u);
         tc_after_sync();
         scores(0);

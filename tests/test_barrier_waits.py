@@ -98,3 +98,9 @@ def test_score_parts_are_given_back_after_they_have_been_read():
     assert read < text.index("__syncwarp()", read) < taken
     wait, give = text.index("mbar_wait_warp(&x_taken"), text.index("mbar_arrive_cluster(")
     assert wait < give and text.count("mbar_arrive_cluster(") == 1 and "(&x_empty" in text[give:]
+
+
+@pytest.mark.parametrize("name", FILES)
+def test_a_wait_that_gave_up_names_itself(name):
+    codes = re.findall(r"mbar_wait\w*\([^;]*?\b(0x[0-9a-f]+)u", re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, name)).read()))
+    assert codes and len(codes) == len(set(codes))
