@@ -964,21 +964,123 @@ bool window_attn_leaves_rounded(const WindowAttnArgs& a, int T) { return window_
 // with a window of 1024: 20 tokens 323 -> 249, 64 tokens 432 -> 306. Ranges of 256 give a window of 300 too few to share:
 // 32 tokens 245 us against 227, of 237 before.)
 constexpr int WT_Q = 32, WT_K = 64, WT_OWN = 32, WT_WARPS = 16, WT_D = 128, WT_RANGE = 2;
-__global__ void __launch_bounds__(WT_WARPS * 32, 1) window_attn_tile_kernel(WindowAttnArgs a, RaggedDev r, int first_tile, int cluster) {
+constexpr int WT_FEW = 4, WT_SLOTS = 16;                   // queries of a tile whose warps take ranges of their own; ranges of such a CTA between two merges
+
+// What a warp has of a range: maxima and sums of weights of the query whose scores a lane ends up with (the sums: of the lane's keys), four entries of the
+// weighted sums of all four
+struct WtSums { float m, l; float4 o[4]; };
+// One block's half, 32 keys, added to them. `qr`: this lane's piece of the first query; `key(u, c)`: this lane's piece c of key u of its four;
+// `value(j)`: this lane's four entries of key j; `pos`, `lo`: of the lane's query; `first`: position of the warp's first query. (Explicit operations
+// where a compiler could fuse: both callers' sums have the same bits.)
+template <int AHEAD, typename Key, typename Value>
+__device__ __forceinline__ void wt_add_half(WtSums& w, const WindowAttnArgs& a, const float* qr, int ldk, float* pw, int j0, int pos, int lo, int first, int lane, Key key, Value value) {
+    const int kg = lane >> 2, part = lane & 3, d = a.d;
+    float sc[4][4];                                        // [query][key of the group]
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+#pragma unroll
+        for (int v = 0; v < 4; v++) sc[u][v] = 0.f;
+    // (AHEAD steps of 16 entries are read before the first is used: shared memory answers in time, a page does not)
+#pragma unroll 1
+    for (int c = 0; c < d; c += 16 * AHEAD) {
+        float4 k[AHEAD][4];
+#pragma unroll
+        for (int i = 0; i < AHEAD; i++)
+#pragma unroll
+            for (int u = 0; u < 4; u++) k[i][u] = key(u, min(c + 16 * i, d - 16));
+#pragma unroll
+        for (int i = 0; i < AHEAD; i++) {
+            if (c + 16 * i >= d) break;
+            float4 q[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) q[u] = *reinterpret_cast<const float4*>(qr + u * ldk + c + 16 * i);
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+#pragma unroll
+                for (int v = 0; v < 4; v++) sc[u][v] += fmaf(q[u].x, k[i][v].x, fmaf(q[u].y, k[i][v].y, fmaf(q[u].z, k[i][v].z, q[u].w * k[i][v].w)));
+        }
+    }
+    // the four parts of every score: lane `part` ends up with query `part`
+    float s[4];
+#pragma unroll
+    for (int v = 0; v < 4; v++) {
+        const bool up = part & 2, odd = part & 1;
+        const float x0 = (up ? sc[2][v] : sc[0][v]) + __shfl_xor_sync(0xffffffffu, up ? sc[0][v] : sc[2][v], 2);
+        const float x1 = (up ? sc[3][v] : sc[1][v]) + __shfl_xor_sync(0xffffffffu, up ? sc[1][v] : sc[3][v], 2);
+        s[v] = (odd ? x1 : x0) + __shfl_xor_sync(0xffffffffu, odd ? x0 : x1, 1);
+    }
+    float mx = w.m;
+#pragma unroll
+    for (int v = 0; v < 4; v++) {
+        const int j = j0 + kg * 4 + v;
+        if (j > pos || (j < lo && j >= a.keep_first)) s[v] = -INFINITY;
+        mx = fmaxf(mx, s[v]);
+    }
+#pragma unroll
+    for (int x = 4; x < 32; x <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, x));
+    const float ref = mx > -INFINITY ? mx : 0.f, corr = w.m > -INFINITY ? expf(w.m - ref) : 0.f;      // (nothing visible yet: all weights are 0)
+    w.m = mx;
+    w.l = __fmul_rn(w.l, corr);
+#pragma unroll
+    for (int v = 0; v < 4; v++) {
+        const float e = expf(s[v] - ref);
+        w.l = __fadd_rn(w.l, e);
+        pw[(kg * 4 + v) * 4 + part] = e;
+    }
+    __syncwarp();
+    float4 b[4];                                           // the block's own sums: short chains of additions
+#pragma unroll
+    for (int u = 0; u < 4; u++) b[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto add = [&](auto all) {
+#pragma unroll 1
+        for (int j = 0; j < WT_OWN; j += 8) {
+            float4 v[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[i] = value(j + i);
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const float4 p = *reinterpret_cast<const float4*>(pw + (j + i) * 4);
+                const float e[4] = {p.x, p.y, p.z, p.w};
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (all || e[u] != 0.f) { b[u].x = fmaf(e[u], v[i].x, b[u].x); b[u].y = fmaf(e[u], v[i].y, b[u].y); b[u].z = fmaf(e[u], v[i].z, b[u].z); b[u].w = fmaf(e[u], v[i].w, b[u].w); }
+            }
+        }
+    };
+    // (a key that some of the warp's queries do not see must not reach them, not even as 0 times infinity)
+    if (j0 + WT_OWN - 1 <= first && j0 >= first + 3 - a.window + 1) add(std::true_type{});
+    else add(std::false_type{});
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const float f = __shfl_sync(0xffffffffu, corr, u);
+        w.o[u].x = fmaf(w.o[u].x, f, b[u].x); w.o[u].y = fmaf(w.o[u].y, f, b[u].y); w.o[u].z = fmaf(w.o[u].z, f, b[u].z); w.o[u].w = fmaf(w.o[u].w, f, b[u].w);
+    }
+    __syncwarp();
+}
+
+// Tiles of few queries (4 and less: portions of two to four tokens; and tokens that come alone, where they are let in) leave seven of eight warps of the above
+// without any. Where a CTA has more than one range of such a tile, a warp takes half a range by itself, keys and values straight from the pages, and the
+// ranges' sums wait in the place of the copies until they are merged, in the same order and to the same bits. Bound by the latency of a page's rows (twelve reads of a lane under way, eight for
+// values). (Steps of two layers, 8 heads of 128, window 1024, behind 1500 keys, us: a CTA per token and head / tiles / here: ten sequences of two tokens
+// 357 / 375 / 289, five 291 / 319 / 273, ten of four 429 / 374 / 288; eight lone tokens beside two 293 / 326 / 271, seven beside 20 382 / 427 / 351,
+// fifteen beside 40 of 4 heads of 64 and a window of 300 289 / 299 / 259. Values read one by one in blocks at a window's edge: 353 where 271 stand.)
+// CTAs x: the tiles from `first_tile` on, `cluster` for each 32 rows, then one for each of the `n_alone` tiles ahead of them.
+__global__ void __launch_bounds__(WT_WARPS * 32, 1) window_attn_tile_kernel(WindowAttnArgs a, RaggedDev r, int first_tile, int cluster, int n_alone) {
     griddep_launch();
     griddep_wait();
     extern __shared__ __align__(16) float wt_sm[];
-    const int d = a.d, ldk = d + 4, rank = blockIdx.x % cluster, x = blockIdx.x / cluster, tile = first_tile + x / 2, h = blockIdx.y, g = h / (a.H / a.G);
-    const int seg = r.tile_seg[tile], row0 = r.tile_row0[tile] + (x & 1) * WT_Q;
+    const int tiled = (r.n_tiles - first_tile) * 2 * cluster, lone = (int)blockIdx.x - tiled;
+    if (lone >= n_alone) return;
+    const int d = a.d, ldk = d + 4, own_rank = blockIdx.x % cluster, rank = lone >= 0 ? 0 : own_rank, x = blockIdx.x / cluster, tile = lone >= 0 ? lone : first_tile + x / 2;
+    const int h = blockIdx.y, g = h / (a.H / a.G);
+    const int seg = r.tile_seg[tile], row0 = r.tile_row0[tile] + (lone >= 0 ? 0 : (x & 1) * WT_Q);
     const int nq = min(WT_Q, r.seg_start[seg] + r.seg_len[seg] - row0);
     if (nq <= 0) return;                                   // (all of a cluster)
     float* qs = wt_sm;                                     // [32][d + 4]
     float* ks = qs + WT_Q * ldk;                           // [2][64][d + 4]
     float* vs = ks + 2 * WT_K * ldk;                       // [2][64][d]
     float* ps = vs + 2 * WT_K * d;                         // [half, warp][32 keys][4 queries]
-    float* xs = ps + WT_WARPS * WT_OWN * 4;                // [half][32 queries][d]: a range's sums ...
-    float2* xml = reinterpret_cast<float2*>(xs + 2 * WT_Q * d);      // [half][32]: ... and its maxima and sums of weights
-    const int warp = threadIdx.x >> 5 & 7, half = threadIdx.x >> 8, own = half * WT_OWN, lane = threadIdx.x & 31, kg = lane >> 2, part = lane & 3;
+    const int warp = threadIdx.x >> 5 & 7, half = threadIdx.x >> 8, own = half * WT_OWN, lane = threadIdx.x & 31, kg = lane >> 2, part = lane & 3, w16 = threadIdx.x >> 5;
     const int p0 = r.seg_pos0[seg] + row0 - r.seg_start[seg], p_last = p0 + nq - 1;
     const int* table = a.block_tables[r.seg_slot[seg]];
     const float *k_pool = reinterpret_cast<const float*>(a.k_pool), *v_pool = reinterpret_cast<const float*>(a.v_pool);
@@ -987,8 +1089,13 @@ __global__ void __launch_bounds__(WT_WARPS * 32, 1) window_attn_tile_kernel(Wind
     const int w0 = max(lo_first / WT_K, n_kept), w1 = p_last / WT_K + 1;
     // ranges that have any, in order; block `i` of all (the first of a range: the number of blocks before it)
     const int kept_ranges = (n_kept + WT_RANGE - 1) / WT_RANGE, w_range = max(w0 / WT_RANGE, kept_ranges), n_ranges = kept_ranges + max(0, (w1 - 1) / WT_RANGE + 1 - w_range);
-    const int company = n_ranges > 1 ? cluster : 1;        // (one range: one CTA)
+    const int company = n_ranges > 1 && lone < 0 ? cluster : 1;      // (one range: one CTA)
     if (rank >= company) return;
+    const bool few = nq <= WT_FEW && n_ranges > company;
+    // sums of a range [half][row][d], and their maxima and sums of weights [half][row]. Rows: 32 queries, or (few) 16 ranges' 4 queries, in the place of the copies
+    const int rows = few ? WT_SLOTS * WT_FEW : WT_Q;
+    float* xs = few ? ks : ps + WT_WARPS * WT_OWN * 4;
+    float2* xml = reinterpret_cast<float2*>(xs + 2 * rows * d);
     auto first_of = [&](int n) {
         const int at = (n < kept_ranges ? n : w_range + n - kept_ranges) * WT_RANGE;
         return min(at, n_kept) + max(0, min(at, w1) - w0);
@@ -1001,7 +1108,7 @@ __global__ void __launch_bounds__(WT_WARPS * 32, 1) window_attn_tile_kernel(Wind
     const int per = d / 4;
     // eight threads a row of a block, whose page is looked up a block ahead of its copies
     const int my_row = threadIdx.x / 8, my_c = threadIdx.x % 8 * 4;
-    int next_range = rank, next = rank < n_ranges ? first_of(rank) : -1, next_end = rank < n_ranges ? end_of(rank) : 0;      // of this CTA's blocks: the one to copy next
+    int next_range = rank, next = !few && rank < n_ranges ? first_of(rank) : -1, next_end = rank < n_ranges ? end_of(rank) : 0;      // of this CTA's blocks: the one to copy next
     auto page_of_next = [&]() { return next >= 0 ? table[min(block_at(next) + my_row, p_last) / a.block_tokens] : 0; };
     int page = page_of_next();
     auto stage = [&](int buf) {                            // keys past the last query's are zeros (their weights are)
@@ -1021,120 +1128,87 @@ __global__ void __launch_bounds__(WT_WARPS * 32, 1) window_attn_tile_kernel(Wind
             cp_async_16z(vd + c, v_pool + from + c, have ? 16 : 0);
         }
     };
-    for (int e = threadIdx.x; e < WT_Q * per; e += WT_WARPS * 32) {      // (rows past the tile: the last one's, dropped at the end)
+    for (int e = threadIdx.x; e < (few ? WT_FEW : WT_Q) * per; e += WT_WARPS * 32) {      // (rows past the tile: the last one's, dropped at the end)
         const int q = e / per, c = e % per * 4;
         const float4 v = *reinterpret_cast<const float4*>(a.q_rot + ((size_t)(row0 + min(q, nq - 1)) * a.H + h) * d + c);
         *reinterpret_cast<float4*>(qs + q * ldk + c) = make_float4(v.x * a.scale, v.y * a.scale, v.z * a.scale, v.w * a.scale);
     }
     stage(0);
     cp_async_commit();
-    const int pos = p0 + warp * 4 + part, lo = max(0, pos - a.window + 1);      // of the query whose scores this lane ends up with
+    if (few) __syncthreads();                              // (the queries are here; the others meet at every block)
+    const int first = p0 + (few ? 0 : warp * 4), pos = first + part, lo = max(0, pos - a.window + 1);      // of the query whose scores this lane ends up with
     float* pw = ps + (half * 8 + warp) * WT_OWN * 4;
+    auto start = [](WtSums& w) {
+        w.m = -INFINITY; w.l = 0.f;
+#pragma unroll
+        for (int u = 0; u < 4; u++) w.o[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    auto leave = [&](WtSums& w, int row) {                 // a range's sums, to rows `row` ... of its half
+#pragma unroll
+        for (int x = 4; x < 32; x <<= 1) w.l += __shfl_xor_sync(0xffffffffu, w.l, x);
+        if (4 * lane < d)
+#pragma unroll
+            for (int u = 0; u < 4; u++) *reinterpret_cast<float4*>(xs + (half * rows + row + u) * d + 4 * lane) = w.o[u];
+        if (kg == 0) xml[half * rows + row + part] = make_float2(w.m, w.l);
+    };
     // state over ranges: this warp has queries rank + company * (its number of 16, and 16 more)
-    const int w16 = threadIdx.x >> 5;
     float M[2] = {-INFINITY, -INFINITY}, L[2] = {0.f, 0.f};
     float4 O[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
     int count = 0;
-    for (int n0 = 0; n0 < n_ranges; n0 += company) {
-        const int n = n0 + rank, i0 = n < n_ranges ? first_of(n) : 0, i1 = n < n_ranges ? end_of(n) : 0;
-        float m = -INFINITY, l = 0.f;                          // of this lane's query in the range (l: this lane's keys)
-        float4 o[4];                                           // entries 4 lane .. of the warp's four queries
-#pragma unroll
-        for (int u = 0; u < 4; u++) o[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int i = i0; i < i1; i++) {
-            const int buf = count++ & 1, j0 = block_at(i) + own;
-            cp_async_wait_all();
-            __syncthreads();                                   // this block has come, everybody has left the other buffer
-            stage(buf ^ 1);
-            cp_async_commit();
-            if (warp * 4 >= nq) continue;                  // (none of the tile's: ten sequences of two tokens behind 1500 keys 387 -> 336 us)
-            float sc[4][4];                                    // [query][key of the group]
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-#pragma unroll
-                for (int v = 0; v < 4; v++) sc[u][v] = 0.f;
-            const float *qr = qs + warp * 4 * ldk + part * 4, *kr = ks + (buf * WT_K + own + kg * 4) * ldk + part * 4;
-#pragma unroll 4
-            for (int c = 0; c < d; c += 16) {
-                float4 q[4], k[4];
-#pragma unroll
-                for (int u = 0; u < 4; u++) { q[u] = *reinterpret_cast<const float4*>(qr + u * ldk + c); k[u] = *reinterpret_cast<const float4*>(kr + u * ldk + c); }
-#pragma unroll
-                for (int u = 0; u < 4; u++)
-#pragma unroll
-                    for (int v = 0; v < 4; v++) sc[u][v] += fmaf(q[u].x, k[v].x, fmaf(q[u].y, k[v].y, fmaf(q[u].z, k[v].z, q[u].w * k[v].w)));
-            }
-            // the four parts of every score: lane `part` ends up with query `part`
-            float s[4];
-#pragma unroll
-            for (int v = 0; v < 4; v++) {
-                const bool up = part & 2, odd = part & 1;
-                const float x0 = (up ? sc[2][v] : sc[0][v]) + __shfl_xor_sync(0xffffffffu, up ? sc[0][v] : sc[2][v], 2);
-                const float x1 = (up ? sc[3][v] : sc[1][v]) + __shfl_xor_sync(0xffffffffu, up ? sc[1][v] : sc[3][v], 2);
-                s[v] = (odd ? x1 : x0) + __shfl_xor_sync(0xffffffffu, odd ? x0 : x1, 1);
-            }
-            float mx = m;
-#pragma unroll
-            for (int v = 0; v < 4; v++) {
-                const int j = j0 + kg * 4 + v;
-                if (j > pos || (j < lo && j >= a.keep_first)) s[v] = -INFINITY;
-                mx = fmaxf(mx, s[v]);
-            }
-#pragma unroll
-            for (int w = 4; w < 32; w <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, w));
-            const float ref = mx > -INFINITY ? mx : 0.f, corr = m > -INFINITY ? expf(m - ref) : 0.f;      // (nothing visible yet: all weights are 0)
-            m = mx;
-            l *= corr;
-#pragma unroll
-            for (int v = 0; v < 4; v++) {
-                const float e = expf(s[v] - ref);
-                l += e;
-                pw[(kg * 4 + v) * 4 + part] = e;
-            }
-            __syncwarp();
-            float4 b[4];                                       // the block's own sums: short chains of additions
-#pragma unroll
-            for (int u = 0; u < 4; u++) b[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (4 * lane < d) {
-                const float* vr = vs + (buf * WT_K + own) * d + 4 * lane;
-                auto add = [&](int j, bool all) {
-                    const float4 v = *reinterpret_cast<const float4*>(vr + j * d), p = *reinterpret_cast<const float4*>(pw + j * 4);
-                    const float w[4] = {p.x, p.y, p.z, p.w};
-#pragma unroll
-                    for (int u = 0; u < 4; u++)
-                        if (all || w[u] != 0.f) { b[u].x = fmaf(w[u], v.x, b[u].x); b[u].y = fmaf(w[u], v.y, b[u].y); b[u].z = fmaf(w[u], v.z, b[u].z); b[u].w = fmaf(w[u], v.w, b[u].w); }
+    const int slots = few ? WT_SLOTS : 1;
+    for (int n0 = 0; n0 < n_ranges; n0 += company * slots) {
+        WtSums w;
+        if (few) {
+            for (int slot = warp; slot < WT_SLOTS; slot += 8) {
+                const int n = n0 + slot * company + rank;
+                if (n >= n_ranges) break;
+                start(w);
+                const int i0 = first_of(n), i1 = end_of(n);
+                auto row_of = [&](int i) {                     // of this lane's key (keys past the last query: that one's, whose weight is dropped)
+                    const int j = min(block_at(i) + own + lane, p_last);
+                    return ((unsigned)table[j / a.block_tokens] * a.G + g) * a.block_tokens + j % a.block_tokens;
                 };
-                // (a key that some of the warp's queries do not see must not reach them, not even as 0 times infinity)
-                if (j0 + WT_OWN - 1 <= p0 + warp * 4 && j0 >= p0 + warp * 4 + 3 - a.window + 1) {
-#pragma unroll 8
-                    for (int j = 0; j < WT_OWN; j++) add(j, true);
-                } else for (int j = 0; j < WT_OWN; j++) add(j, false);
+                unsigned ahead = row_of(i0);
+                for (int i = i0; i < i1; i++) {
+                    const int j0 = block_at(i) + own;
+                    const unsigned at = ahead;
+                    if (i + 1 < i1) ahead = row_of(i + 1);
+                    const float* k_at[4];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) k_at[u] = k_pool + (size_t)__shfl_sync(0xffffffffu, at, kg * 4 + u) * d + part * 4;
+                    const float* v_lane = v_pool + (4 * lane < d ? 4 * lane : 0);
+                    wt_add_half<3>(w, a, qs + part * 4, ldk, pw, j0, pos, lo, first, lane, [&](int u, int c) { return *reinterpret_cast<const float4*>(k_at[u] + c); },
+                                [&](int jj) { return *reinterpret_cast<const float4*>(v_lane + (size_t)__shfl_sync(0xffffffffu, at, jj) * d); });
+                }
+                leave(w, slot * WT_FEW);
             }
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const float f = __shfl_sync(0xffffffffu, corr, u);
-                o[u].x = fmaf(o[u].x, f, b[u].x); o[u].y = fmaf(o[u].y, f, b[u].y); o[u].z = fmaf(o[u].z, f, b[u].z); o[u].w = fmaf(o[u].w, f, b[u].w);
+        } else {
+            const int n = n0 + rank, i0 = n < n_ranges ? first_of(n) : 0, i1 = n < n_ranges ? end_of(n) : 0;
+            start(w);
+            for (int i = i0; i < i1; i++) {
+                const int buf = count++ & 1, j0 = block_at(i) + own;
+                cp_async_wait_all();
+                __syncthreads();                           // this block has come, everybody has left the other buffer
+                stage(buf ^ 1);
+                cp_async_commit();
+                if (warp * 4 >= nq) continue;              // (none of the tile's)
+                const float *kr = ks + (buf * WT_K + own + kg * 4) * ldk + part * 4, *vr = vs + (buf * WT_K + own) * d + (4 * lane < d ? 4 * lane : 0);
+                wt_add_half<1>(w, a, qs + warp * 4 * ldk + part * 4, ldk, pw, j0, pos, lo, first, lane, [&](int u, int c) { return *reinterpret_cast<const float4*>(kr + u * ldk + c); },
+                            [&](int jj) { return *reinterpret_cast<const float4*>(vr + jj * d); });
             }
-            __syncwarp();
-        }
-        if (n < n_ranges) {
-#pragma unroll
-            for (int w = 4; w < 32; w <<= 1) l += __shfl_xor_sync(0xffffffffu, l, w);
-            if (4 * lane < d)
-#pragma unroll
-                for (int u = 0; u < 4; u++) *reinterpret_cast<float4*>(xs + (half * WT_Q + warp * 4 + u) * d + 4 * lane) = o[u];
-            if (kg == 0) xml[half * WT_Q + warp * 4 + part] = make_float2(m, l);
+            if (n < n_ranges) leave(w, warp * 4);
         }
         if (company > 1) cluster_sync();
         else __syncthreads();
 #pragma unroll
         for (int k = 0; k < 2; k++) {
             const int q = rank + company * (w16 + WT_WARPS * k);
-            if (q >= WT_Q) break;
-            for (int c = 0; c < company && n0 + c < n_ranges; c++) {
-                const uint32_t at = cluster_address(smem_u32(xs + q * d + (4 * lane < d ? 4 * lane : 0)), c), at_ml = cluster_address(smem_u32(xml + q), c);
-                const float2 x0 = cluster_load2(at_ml), x1 = cluster_load2(at_ml + WT_Q * 8);
-                const float4 y0 = cluster_load4(at), y1 = cluster_load4(at + WT_Q * d * 4);
+            if (q >= nq) break;
+            for (int i = 0; i < company * slots && n0 + i < n_ranges; i++) {
+                const int c = i & (company - 1), row = few ? (i >> __ffs(company) - 1) * WT_FEW + q : q;
+                const uint32_t at = cluster_address(smem_u32(xs + row * d + (4 * lane < d ? 4 * lane : 0)), lone < 0 ? c : own_rank), at_ml = cluster_address(smem_u32(xml + row), lone < 0 ? c : own_rank);
+                const float2 x0 = cluster_load2(at_ml), x1 = cluster_load2(at_ml + rows * 8);
+                const float4 y0 = cluster_load4(at), y1 = cluster_load4(at + rows * d * 4);
                 const float top = fmaxf(M[k], fmaxf(x0.x, x1.x)), ref = top > -INFINITY ? top : 0.f;      // (nothing visible yet: all factors are 0)
                 const float f = expf(M[k] - ref), f0 = expf(x0.x - ref), f1 = expf(x1.x - ref);
                 M[k] = top;
@@ -1174,14 +1248,31 @@ cudaError_t window_attn_launch(const WindowAttnArgs& a, const RaggedDev& r, cuda
         constexpr int most = ((WT_Q + 2 * WT_K) * (WT_D + 4) + 2 * WT_K * WT_D + WT_WARPS * WT_OWN * 4 + 2 * WT_Q * (WT_D + 2)) * 4;
         if (!allow_smem<window_attn_tile_kernel>(most)) return cudaErrorInvalidValue;
         const size_t smem = (size_t)((WT_Q + 2 * WT_K) * (a.d + 4) + 2 * WT_K * a.d + WT_WARPS * WT_OWN * 4 + 2 * WT_Q * (a.d + 2)) * 4;
-        // as many CTAs a tile as fit side by side in clusters (of 8: 128), and no more than a window has ranges
-        const int n = (r.n_tiles - alone) * 2 - (r.n_upto[5] - alone), ranges = (int)std::min<long long>(8, ((long long)a.window + a.keep_first + WT_Q) / (WT_RANGE * WT_K) + 2);
-        int company = 1;
-        while (company < 8 && company < ranges && n * a.H * company * 2 <= 128) company *= 2;
-        const dim3 grid((r.n_tiles - alone) * 2 * company, a.H), block(WT_WARPS * 32);
-        const cudaError_t e = company > 1 ? launch_chain_cluster(window_attn_tile_kernel, company, grid, block, smem, s, a, r, alone, company)
-                                          : launch_chain(window_attn_tile_kernel, grid, block, smem, s, a, r, alone, company);
-        if (e != cudaSuccess || alone == 0) return e;
+        // as many CTAs a tile as fit side by side in clusters (of 2: 148, of 8: 128), and no more than a window has ranges
+        const int ranges = (int)std::min<long long>(8, ((long long)a.window + a.keep_first + WT_Q) / (WT_RANGE * WT_K) + 2);
+        auto company_of = [&](int n) {
+            int c = 1;
+            while (c < 8 && c < ranges && n * a.H * c * 2 <= (c == 1 ? 148 : 128)) c *= 2;
+            return c;
+        };
+        int n = (r.n_tiles - alone) * 2 - (r.n_upto[5] - alone), first = alone, company = company_of(n), lone = 0;
+        auto fits = [&](int c) { return (n * c + (alone + c - 1) / c * c) * a.H <= 128; };
+        if (alone > 0 && r.n_tiles == r.n_upto[2] && r.n_tiles * a.H <= (ranges < 8 ? 1 : 4) * 148) {
+            // none of more than four tokens: those that come alone are tiles like the others (eight beside two: 271 us, with one CTA each 317). Several waves
+            // of them where a window holds enough ranges to keep their warps busy (16 heads of 128, 31 beside two behind 1500: window 1024 591 us apart
+            // from the others, 490 as tiles; window 300 376, 397)
+            first = 0; n = r.n_tiles; company = company_of(n);
+        } else if (alone > 0 && (fits(company) || (company > 1 && fits(company / 2)))) {
+            // a CTA for each of them beside the tiles, or beside half as many for each tile. (Where they do not fit they take a launch of their own, which holds
+            // many to an SM: fifteen beside 256 1145 us with a CTA per token and head, 622 so)
+            if (!fits(company)) company /= 2;
+            lone = alone;
+        }
+        const dim3 grid((r.n_tiles - first) * 2 * company + (lone + company - 1) / company * company, a.H), block(WT_WARPS * 32);
+        const cudaError_t e = company > 1 ? launch_chain_cluster(window_attn_tile_kernel, company, grid, block, smem, s, a, r, first, company, lone)
+                                          : launch_chain(window_attn_tile_kernel, grid, block, smem, s, a, r, first, company, lone);
+        const bool joined = first == 0 || lone > 0;
+        if (e != cudaSuccess || joined) return e;
     }
     if (a.d % 2 == 0) {
         // a step of a few tokens does not fill the GPU with one CTA per (token, head): split the keys (up to 16 ranges)

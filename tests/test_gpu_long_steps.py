@@ -109,6 +109,30 @@ def test_cuts_do_not_change_a_token_in_32_bits(native_lib, tmp_path, n, window, 
         assert np.array_equal(rows[0], other)
 
 
+@pytest.mark.parametrize("d,window,keep,past,pieces", [
+    (64, 100, 5, 200, [2] * 10), (128, 600, 300, 900, [2, 3, 4, 5, 2, 2]), (16, 1000, 0, 300, [2, 2, 2, 2, 2, 4]), (48, 40, 1, 63, [4, 3, 2]), (32, 3000, 0, 2200, [2] * 17),
+    (80, 70, 3, 150, [1] * 8 + [2]), (128, 3000, 4, 2400, [1, 1, 9]), (64, 300, 4, 310, [1] * 15 + [40]), (64, 300, 0, 290, [1] * 20 + [40]), (112, 20, 40, 64, [1, 1, 1, 65])])
+def test_short_portions_in_32_bits(native_lib, tmp_path, d, window, keep, past, pieces):
+    """Window attention over 32-bit pages: portions of a few tokens behind others, whose tiles' warps take ranges of keys, more than one round of them, and
+    tokens that come alone beside longer ones and join their launch, have the bits that they have in the whole prompts."""
+    from llama_cpp.kv_pages import SequenceSlots
+    cfg = gu.config([gu.parallel(left=gu.attn(heads=4, kv_heads=2, dim=d, rot=8, window=window, keep=keep))])
+    eng = engine(gu.write_model(str(tmp_path / "m"), cfg, gu.random_weights(cfg, seed=9)), "float32", past + 80, len(pieces))
+    prompts = [toks(cfg["vocab"], past + k, 20 + i) for i, k in enumerate(pieces)]
+    seqs, wholes = SequenceSlots(eng), []
+    for p, k in zip(prompts, pieces):
+        seqs.open(0)
+        wholes.append(np.array(eng.step([(seqs.extend(0, len(p)), p)], want=[list(range(len(p)))])[0])[past:])
+        seqs.close(0)
+    for i, p in enumerate(prompts):
+        seqs.open(i)
+        eng.step([(seqs.extend(i, past), p[:past])])
+    got = np.array(eng.step([(seqs.extend(i, k), p[past:]) for i, (p, k) in enumerate(zip(prompts, pieces))], want=[list(range(k)) for k in pieces])[0])
+    eng.close()
+    for i, (g, w) in enumerate(zip(np.split(got, np.cumsum(pieces)[:-1]), wholes)):
+        assert np.isfinite(w).all() and np.array_equal(g, w), i
+
+
 # (head sizes that are multiples of 8: the products around the attention take rounded rows, without which the general kernel runs)
 LATENT = {"plain": lambda heads, rank, **kw: fu.plain(heads=heads, rank=rank, dim=24, vdim=16, **kw),
           "rotated": lambda heads, rank, **kw: fu.rotated(heads=heads, rank=rank, dim=24, vdim=16, rot_dim=16, **kw)}
