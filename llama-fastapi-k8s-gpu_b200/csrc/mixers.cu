@@ -1091,141 +1091,145 @@ __global__ void __launch_bounds__(WT_WARPS * 32, 1) window_attn_tile_kernel(Wind
     const int kept_ranges = (n_kept + WT_RANGE - 1) / WT_RANGE, w_range = max(w0 / WT_RANGE, kept_ranges), n_ranges = kept_ranges + max(0, (w1 - 1) / WT_RANGE + 1 - w_range);
     const int company = n_ranges > 1 && lone < 0 ? cluster : 1;      // (one range: one CTA)
     if (rank >= company) return;
-    const bool few = nq <= WT_FEW && n_ranges > company;
-    // sums of a range [half][row][d], and their maxima and sums of weights [half][row]. Rows: 32 queries, or (few) 16 ranges' 4 queries, in the place of the copies
-    const int rows = few ? WT_SLOTS * WT_FEW : WT_Q;
-    float* xs = few ? ks : ps + WT_WARPS * WT_OWN * 4;
-    float2* xml = reinterpret_cast<float2*>(xs + 2 * rows * d);
-    auto first_of = [&](int n) {
-        const int at = (n < kept_ranges ? n : w_range + n - kept_ranges) * WT_RANGE;
-        return min(at, n_kept) + max(0, min(at, w1) - w0);
-    };
-    auto end_of = [&](int n) {
-        const int at = ((n < kept_ranges ? n : w_range + n - kept_ranges) + 1) * WT_RANGE;
-        return min(at, n_kept) + max(0, min(at, w1) - w0);
-    };
-    auto block_at = [&](int i) { return (i < n_kept ? i : w0 + i - n_kept) * WT_K; };
-    const int per = d / 4;
-    // eight threads a row of a block, whose page is looked up a block ahead of its copies
-    const int my_row = threadIdx.x / 8, my_c = threadIdx.x % 8 * 4;
-    int next_range = rank, next = !few && rank < n_ranges ? first_of(rank) : -1, next_end = rank < n_ranges ? end_of(rank) : 0;      // of this CTA's blocks: the one to copy next
-    auto page_of_next = [&]() { return next >= 0 ? table[min(block_at(next) + my_row, p_last) / a.block_tokens] : 0; };
-    int page = page_of_next();
-    auto stage = [&](int buf) {                            // keys past the last query's are zeros (their weights are)
-        if (next < 0) return;
-        const int pos = block_at(next) + my_row;
-        const bool have = pos <= p_last;
-        const size_t from = have ? (((size_t)page * a.G + g) * a.block_tokens + pos % a.block_tokens) * d : 0;
-        if (++next == next_end) {
-            next_range += company;
-            next = next_range < n_ranges ? first_of(next_range) : -1;
-            next_end = next_range < n_ranges ? end_of(next_range) : 0;
+    auto body = [&](auto is_few) {
+        constexpr bool few = is_few;
+        // sums of a range [half][row][d], and their maxima and sums of weights [half][row]. Rows: 32 queries, or (few) 16 ranges' 4 queries, in the place of the copies
+        const int rows = few ? WT_SLOTS * WT_FEW : WT_Q;
+        float* xs = few ? ks : ps + WT_WARPS * WT_OWN * 4;
+        float2* xml = reinterpret_cast<float2*>(xs + 2 * rows * d);
+        auto first_of = [&](int n) {
+            const int at = (n < kept_ranges ? n : w_range + n - kept_ranges) * WT_RANGE;
+            return min(at, n_kept) + max(0, min(at, w1) - w0);
+        };
+        auto end_of = [&](int n) {
+            const int at = ((n < kept_ranges ? n : w_range + n - kept_ranges) + 1) * WT_RANGE;
+            return min(at, n_kept) + max(0, min(at, w1) - w0);
+        };
+        auto block_at = [&](int i) { return (i < n_kept ? i : w0 + i - n_kept) * WT_K; };
+        const int per = d / 4;
+        // eight threads a row of a block, whose page is looked up a block ahead of its copies
+        const int my_row = threadIdx.x / 8, my_c = threadIdx.x % 8 * 4;
+        int next_range = rank, next = !few && rank < n_ranges ? first_of(rank) : -1, next_end = rank < n_ranges ? end_of(rank) : 0;      // of this CTA's blocks: the one to copy next
+        auto page_of_next = [&]() { return next >= 0 ? table[min(block_at(next) + my_row, p_last) / a.block_tokens] : 0; };
+        int page = page_of_next();
+        auto stage = [&](int buf) {                            // keys past the last query's are zeros (their weights are)
+            if (next < 0) return;
+            const int pos = block_at(next) + my_row;
+            const bool have = pos <= p_last;
+            const size_t from = have ? (((size_t)page * a.G + g) * a.block_tokens + pos % a.block_tokens) * d : 0;
+            if (++next == next_end) {
+                next_range += company;
+                next = next_range < n_ranges ? first_of(next_range) : -1;
+                next_end = next_range < n_ranges ? end_of(next_range) : 0;
+            }
+            page = page_of_next();
+            float *kd = ks + (buf * WT_K + my_row) * ldk, *vd = vs + (buf * WT_K + my_row) * d;
+            for (int c = my_c; c < d; c += 32) {
+                cp_async_16z(kd + c, k_pool + from + c, have ? 16 : 0);
+                cp_async_16z(vd + c, v_pool + from + c, have ? 16 : 0);
+            }
+        };
+        for (int e = threadIdx.x; e < (few ? WT_FEW : WT_Q) * per; e += WT_WARPS * 32) {      // (rows past the tile: the last one's, dropped at the end)
+            const int q = e / per, c = e % per * 4;
+            const float4 v = *reinterpret_cast<const float4*>(a.q_rot + ((size_t)(row0 + min(q, nq - 1)) * a.H + h) * d + c);
+            *reinterpret_cast<float4*>(qs + q * ldk + c) = make_float4(v.x * a.scale, v.y * a.scale, v.z * a.scale, v.w * a.scale);
         }
-        page = page_of_next();
-        float *kd = ks + (buf * WT_K + my_row) * ldk, *vd = vs + (buf * WT_K + my_row) * d;
-        for (int c = my_c; c < d; c += 32) {
-            cp_async_16z(kd + c, k_pool + from + c, have ? 16 : 0);
-            cp_async_16z(vd + c, v_pool + from + c, have ? 16 : 0);
-        }
-    };
-    for (int e = threadIdx.x; e < (few ? WT_FEW : WT_Q) * per; e += WT_WARPS * 32) {      // (rows past the tile: the last one's, dropped at the end)
-        const int q = e / per, c = e % per * 4;
-        const float4 v = *reinterpret_cast<const float4*>(a.q_rot + ((size_t)(row0 + min(q, nq - 1)) * a.H + h) * d + c);
-        *reinterpret_cast<float4*>(qs + q * ldk + c) = make_float4(v.x * a.scale, v.y * a.scale, v.z * a.scale, v.w * a.scale);
-    }
-    stage(0);
-    cp_async_commit();
-    if (few) __syncthreads();                              // (the queries are here; the others meet at every block)
-    const int first = p0 + (few ? 0 : warp * 4), pos = first + part, lo = max(0, pos - a.window + 1);      // of the query whose scores this lane ends up with
-    float* pw = ps + (half * 8 + warp) * WT_OWN * 4;
-    auto start = [](WtSums& w) {
-        w.m = -INFINITY; w.l = 0.f;
+        stage(0);
+        cp_async_commit();
+        if (few) __syncthreads();                              // (the queries are here; the others meet at every block)
+        const int first = p0 + (few ? 0 : warp * 4), pos = first + part, lo = max(0, pos - a.window + 1);      // of the query whose scores this lane ends up with
+        float* pw = ps + (half * 8 + warp) * WT_OWN * 4;
+        auto start = [](WtSums& w) {
+            w.m = -INFINITY; w.l = 0.f;
 #pragma unroll
-        for (int u = 0; u < 4; u++) w.o[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-    };
-    auto leave = [&](WtSums& w, int row) {                 // a range's sums, to rows `row` ... of its half
+            for (int u = 0; u < 4; u++) w.o[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        };
+        auto leave = [&](WtSums& w, int row) {                 // a range's sums, to rows `row` ... of its half
 #pragma unroll
-        for (int x = 4; x < 32; x <<= 1) w.l += __shfl_xor_sync(0xffffffffu, w.l, x);
-        if (4 * lane < d)
+            for (int x = 4; x < 32; x <<= 1) w.l += __shfl_xor_sync(0xffffffffu, w.l, x);
+            if (4 * lane < d)
 #pragma unroll
-            for (int u = 0; u < 4; u++) *reinterpret_cast<float4*>(xs + (half * rows + row + u) * d + 4 * lane) = w.o[u];
-        if (kg == 0) xml[half * rows + row + part] = make_float2(w.m, w.l);
-    };
-    // state over ranges: this warp has queries rank + company * (its number of 16, and 16 more)
-    float M[2] = {-INFINITY, -INFINITY}, L[2] = {0.f, 0.f};
-    float4 O[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
-    int count = 0;
-    const int slots = few ? WT_SLOTS : 1;
-    for (int n0 = 0; n0 < n_ranges; n0 += company * slots) {
-        WtSums w;
-        if (few) {
-            for (int slot = warp; slot < WT_SLOTS; slot += 8) {
-                const int n = n0 + slot * company + rank;
-                if (n >= n_ranges) break;
-                start(w);
-                const int i0 = first_of(n), i1 = end_of(n);
-                auto row_of = [&](int i) {                     // of this lane's key (keys past the last query: that one's, whose weight is dropped)
-                    const int j = min(block_at(i) + own + lane, p_last);
-                    return ((unsigned)table[j / a.block_tokens] * a.G + g) * a.block_tokens + j % a.block_tokens;
-                };
-                unsigned ahead = row_of(i0);
-                for (int i = i0; i < i1; i++) {
-                    const int j0 = block_at(i) + own;
-                    const unsigned at = ahead;
-                    if (i + 1 < i1) ahead = row_of(i + 1);
-                    const float* k_at[4];
+                for (int u = 0; u < 4; u++) *reinterpret_cast<float4*>(xs + (half * rows + row + u) * d + 4 * lane) = w.o[u];
+            if (kg == 0) xml[half * rows + row + part] = make_float2(w.m, w.l);
+        };
+        // state over ranges: this warp has queries rank + company * (its number of 16, and 16 more)
+        float M[2] = {-INFINITY, -INFINITY}, L[2] = {0.f, 0.f};
+        float4 O[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+        int count = 0;
+        const int slots = few ? WT_SLOTS : 1;
+        for (int n0 = 0; n0 < n_ranges; n0 += company * slots) {
+            WtSums w;
+            if constexpr (few) {
+                for (int slot = warp; slot < WT_SLOTS; slot += 8) {
+                    const int n = n0 + slot * company + rank;
+                    if (n >= n_ranges) break;
+                    start(w);
+                    const int i0 = first_of(n), i1 = end_of(n);
+                    auto row_of = [&](int i) {                     // of this lane's key (keys past the last query: that one's, whose weight is dropped)
+                        const int j = min(block_at(i) + own + lane, p_last);
+                        return ((unsigned)table[j / a.block_tokens] * a.G + g) * a.block_tokens + j % a.block_tokens;
+                    };
+                    unsigned ahead = row_of(i0);
+                    for (int i = i0; i < i1; i++) {
+                        const int j0 = block_at(i) + own;
+                        const unsigned at = ahead;
+                        if (i + 1 < i1) ahead = row_of(i + 1);
+                        const float* k_at[4];
 #pragma unroll
-                    for (int u = 0; u < 4; u++) k_at[u] = k_pool + (size_t)__shfl_sync(0xffffffffu, at, kg * 4 + u) * d + part * 4;
-                    const float* v_lane = v_pool + (4 * lane < d ? 4 * lane : 0);
-                    wt_add_half<3>(w, a, qs + part * 4, ldk, pw, j0, pos, lo, first, lane, [&](int u, int c) { return *reinterpret_cast<const float4*>(k_at[u] + c); },
-                                [&](int jj) { return *reinterpret_cast<const float4*>(v_lane + (size_t)__shfl_sync(0xffffffffu, at, jj) * d); });
+                        for (int u = 0; u < 4; u++) k_at[u] = k_pool + (size_t)__shfl_sync(0xffffffffu, at, kg * 4 + u) * d + part * 4;
+                        const float* v_lane = v_pool + (4 * lane < d ? 4 * lane : 0);
+                        wt_add_half<3>(w, a, qs + part * 4, ldk, pw, j0, pos, lo, first, lane, [&](int u, int c) { return *reinterpret_cast<const float4*>(k_at[u] + c); },
+                                    [&](int jj) { return *reinterpret_cast<const float4*>(v_lane + (size_t)__shfl_sync(0xffffffffu, at, jj) * d); });
+                    }
+                    leave(w, slot * WT_FEW);
                 }
-                leave(w, slot * WT_FEW);
+            } else {
+                const int n = n0 + rank, i0 = n < n_ranges ? first_of(n) : 0, i1 = n < n_ranges ? end_of(n) : 0;
+                start(w);
+                for (int i = i0; i < i1; i++) {
+                    const int buf = count++ & 1, j0 = block_at(i) + own;
+                    cp_async_wait_all();
+                    __syncthreads();                           // this block has come, everybody has left the other buffer
+                    stage(buf ^ 1);
+                    cp_async_commit();
+                    if (warp * 4 >= nq) continue;              // (none of the tile's)
+                    const float *kr = ks + (buf * WT_K + own + kg * 4) * ldk + part * 4, *vr = vs + (buf * WT_K + own) * d + (4 * lane < d ? 4 * lane : 0);
+                    wt_add_half<1>(w, a, qs + warp * 4 * ldk + part * 4, ldk, pw, j0, pos, lo, first, lane, [&](int u, int c) { return *reinterpret_cast<const float4*>(kr + u * ldk + c); },
+                                [&](int jj) { return *reinterpret_cast<const float4*>(vr + jj * d); });
+                }
+                if (n < n_ranges) leave(w, warp * 4);
             }
-        } else {
-            const int n = n0 + rank, i0 = n < n_ranges ? first_of(n) : 0, i1 = n < n_ranges ? end_of(n) : 0;
-            start(w);
-            for (int i = i0; i < i1; i++) {
-                const int buf = count++ & 1, j0 = block_at(i) + own;
-                cp_async_wait_all();
-                __syncthreads();                           // this block has come, everybody has left the other buffer
-                stage(buf ^ 1);
-                cp_async_commit();
-                if (warp * 4 >= nq) continue;              // (none of the tile's)
-                const float *kr = ks + (buf * WT_K + own + kg * 4) * ldk + part * 4, *vr = vs + (buf * WT_K + own) * d + (4 * lane < d ? 4 * lane : 0);
-                wt_add_half<1>(w, a, qs + warp * 4 * ldk + part * 4, ldk, pw, j0, pos, lo, first, lane, [&](int u, int c) { return *reinterpret_cast<const float4*>(kr + u * ldk + c); },
-                            [&](int jj) { return *reinterpret_cast<const float4*>(vr + jj * d); });
+            if (company > 1) cluster_sync();
+            else __syncthreads();
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                const int q = rank + company * (w16 + WT_WARPS * k);
+                if (q >= nq) break;
+                for (int i = 0; i < company * slots && n0 + i < n_ranges; i++) {
+                    const int c = i & (company - 1), row = few ? (i >> __ffs(company) - 1) * WT_FEW + q : q;
+                    const uint32_t at = cluster_address(smem_u32(xs + row * d + (4 * lane < d ? 4 * lane : 0)), lone < 0 ? c : own_rank), at_ml = cluster_address(smem_u32(xml + row), lone < 0 ? c : own_rank);
+                    const float2 x0 = cluster_load2(at_ml), x1 = cluster_load2(at_ml + rows * 8);
+                    const float4 y0 = cluster_load4(at), y1 = cluster_load4(at + rows * d * 4);
+                    const float top = fmaxf(M[k], fmaxf(x0.x, x1.x)), ref = top > -INFINITY ? top : 0.f;      // (nothing visible yet: all factors are 0)
+                    const float f = expf(M[k] - ref), f0 = expf(x0.x - ref), f1 = expf(x1.x - ref);
+                    M[k] = top;
+                    L[k] = fmaf(L[k], f, fmaf(x0.y, f0, x1.y * f1));
+                    O[k].x = fmaf(O[k].x, f, fmaf(y0.x, f0, y1.x * f1)); O[k].y = fmaf(O[k].y, f, fmaf(y0.y, f0, y1.y * f1));
+                    O[k].z = fmaf(O[k].z, f, fmaf(y0.z, f0, y1.z * f1)); O[k].w = fmaf(O[k].w, f, fmaf(y0.w, f0, y1.w * f1));
+                }
             }
-            if (n < n_ranges) leave(w, warp * 4);
+            if (company > 1) cluster_sync();                       // (nobody overwrites, or leaves, what another still reads)
+            else __syncthreads();
         }
-        if (company > 1) cluster_sync();
-        else __syncthreads();
 #pragma unroll
         for (int k = 0; k < 2; k++) {
             const int q = rank + company * (w16 + WT_WARPS * k);
-            if (q >= nq) break;
-            for (int i = 0; i < company * slots && n0 + i < n_ranges; i++) {
-                const int c = i & (company - 1), row = few ? (i >> __ffs(company) - 1) * WT_FEW + q : q;
-                const uint32_t at = cluster_address(smem_u32(xs + row * d + (4 * lane < d ? 4 * lane : 0)), lone < 0 ? c : own_rank), at_ml = cluster_address(smem_u32(xml + row), lone < 0 ? c : own_rank);
-                const float2 x0 = cluster_load2(at_ml), x1 = cluster_load2(at_ml + rows * 8);
-                const float4 y0 = cluster_load4(at), y1 = cluster_load4(at + rows * d * 4);
-                const float top = fmaxf(M[k], fmaxf(x0.x, x1.x)), ref = top > -INFINITY ? top : 0.f;      // (nothing visible yet: all factors are 0)
-                const float f = expf(M[k] - ref), f0 = expf(x0.x - ref), f1 = expf(x1.x - ref);
-                M[k] = top;
-                L[k] = fmaf(L[k], f, fmaf(x0.y, f0, x1.y * f1));
-                O[k].x = fmaf(O[k].x, f, fmaf(y0.x, f0, y1.x * f1)); O[k].y = fmaf(O[k].y, f, fmaf(y0.y, f0, y1.y * f1));
-                O[k].z = fmaf(O[k].z, f, fmaf(y0.z, f0, y1.z * f1)); O[k].w = fmaf(O[k].w, f, fmaf(y0.w, f0, y1.w * f1));
-            }
+            if (q < nq && 4 * lane < d)
+                *reinterpret_cast<float4*>(a.out + ((size_t)(row0 + q) * a.H + h) * d + 4 * lane) = make_float4(O[k].x / L[k], O[k].y / L[k], O[k].z / L[k], O[k].w / L[k]);
         }
-        if (company > 1) cluster_sync();                       // (nobody overwrites, or leaves, what another still reads)
-        else __syncthreads();
-    }
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-        const int q = rank + company * (w16 + WT_WARPS * k);
-        if (q < nq && 4 * lane < d)
-            *reinterpret_cast<float4*>(a.out + ((size_t)(row0 + q) * a.H + h) * d + 4 * lane) = make_float4(O[k].x / L[k], O[k].y / L[k], O[k].z / L[k], O[k].w / L[k]);
-    }
+    };
+    if (nq <= WT_FEW && n_ranges > company) body(std::true_type{});
+    else body(std::false_type{});
 }
 // Heads of whole 16-entry pieces up to 128, rows on 16-byte boundaries.
 static bool window_attn_tiles(const WindowAttnArgs& a, int T) {
