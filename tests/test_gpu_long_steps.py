@@ -133,6 +133,39 @@ def test_short_portions_in_32_bits(native_lib, tmp_path, d, window, keep, past, 
         assert np.isfinite(w).all() and np.array_equal(g, w), i
 
 
+@pytest.mark.parametrize("d,window,keep,past,pieces,at", [(64, 100, 5, 0, [300, 1, 20], 130), (128, 600, 40, 0, [200], 101), (16, 1000, 0, 0, [64, 2, 2, 9], 33),
+                                                          (64, 200, 5, 310, [4, 3, 2], 2), (32, 1000, 4, 300, [4, 1, 1, 1, 4], 1), (128, 90, 1, 70, [33, 2], 32)])
+def test_window_attention_in_32_bits_beside_a_token_without_numbers(native_lib, tmp_path, d, window, keep, past, pieces, at):
+    """Window attention over 32-bit pages: a token whose keys and values are no numbers changes no bit of the tokens ahead of it and of other sequences, nor do
+    pages that hold its rows, or others of a longer prompt, when they are used again."""
+    from llama_cpp.kv_pages import SequenceSlots
+    cfg, bad = gu.config([gu.parallel(left=gu.attn(heads=4, kv_heads=2, dim=d, rot=8, window=window, keep=keep))]), 130
+    w = gu.random_weights(cfg, seed=9)
+    w["embed"][bad] = np.nan
+    eng = engine(gu.write_model(str(tmp_path / "m"), cfg, w), "float32", past + max(pieces), len(pieces))
+    prompts, seqs, got = [toks(bad, past + k, 20 + i) for i, k in enumerate(pieces)], SequenceSlots(eng), []
+
+    def run(there, lens):
+        for i, p in enumerate(prompts):
+            seqs.open(i)
+            if past:
+                eng.step([(seqs.extend(i, past), p[:past])])
+        entries = [(seqs.extend(i, k), [there if i == 0 and j == at else t for j, t in enumerate(p[past:past + k])]) for i, (p, k) in enumerate(zip(prompts, lens))]
+        rows = np.split(np.array(eng.step(entries, want=[list(range(k)) for k in lens])[0])[:, :bad], np.cumsum(lens)[:-1])
+        for i in range(len(pieces)):
+            seqs.close(i)
+        return rows
+
+    clean, beside = run(prompts[0][past + at], pieces), run(bad, pieces)
+    again = run(prompts[0][past + at], pieces)
+    assert all(np.isfinite(g).all() for g in clean) and np.isnan(beside[0][at:]).all()
+    assert np.array_equal(beside[0][:at], clean[0][:at])
+    for a, b, c in zip(clean[1:], beside[1:], again[1:]):
+        assert np.array_equal(a, b) and np.array_equal(a, c)
+    assert np.array_equal(clean[0], again[0])
+    eng.close()
+
+
 # (head sizes that are multiples of 8: the products around the attention take rounded rows, without which the general kernel runs)
 LATENT = {"plain": lambda heads, rank, **kw: fu.plain(heads=heads, rank=rank, dim=24, vdim=16, **kw),
           "rotated": lambda heads, rank, **kw: fu.rotated(heads=heads, rank=rank, dim=24, vdim=16, rot_dim=16, **kw)}
@@ -150,6 +183,26 @@ def test_latent_attention_of_long_steps(native_lib, tmp_path, kind, rank, heads,
 @pytest.mark.parametrize("rank,rot,lengths", [(512, 64, [300, 129, 2]), (512, 48, [64, 257]), (512, 16, [1, 65]), (256, 256, [257]), (192, 384, [385]), (64, 512, [129, 200])])
 def test_rotated_parts_of_latent_attention(native_lib, tmp_path, rank, rot, lengths):
     check(fu, fazovik_ref, fu.config([fu.rotated(heads=3, rank=rank, dim=24, vdim=16, rot_dim=rot)]), tmp_path, lengths, "bfloat16")
+
+
+@pytest.mark.parametrize("kind,rank", [("rotated", 512), ("plain", 512), ("rotated", 256), ("plain", 64)])
+def test_latent_attention_whose_later_keys_outweigh_the_first(native_lib, tmp_path, monkeypatch, kind, rank):
+    """Scores spread so far that blocks of 64 keys after the first raise many rows' maxima by more than 2^8, where the sum in tensor memory is rescaled.
+    Bar: bf16 queries and cached rows put a score of spread 9 (natural units) off by 9 * 2^-9 * sqrt(2/3) = 1.4e-2, and its row by as much beside what the
+    others' are off by; twice their sum."""
+    from test_gpu_model import lagging_growth
+    layer = LATENT[kind](3, rank, scale=0.45 if kind == "rotated" else 0.9)
+    cfg, grown, spread, softmax = fu.config([layer]), [], [], fazovik_ref.causal_softmax
+
+    def seen(scores):
+        visible = np.tri(len(scores), dtype=bool)
+        grown.append(lagging_growth(np.where(visible, scores * np.log2(np.e), -np.inf), 64)[:, 1:].sum())
+        spread.append(scores[visible].std())
+        return softmax(scores)
+
+    monkeypatch.setattr(fazovik_ref, "causal_softmax", seen)
+    check(fu, fazovik_ref, cfg, tmp_path, [300], "bfloat16", bar=8e-2)
+    assert len(grown) == 3 and min(grown) >= 20 and 7 < min(spread) and max(spread) < 11
 
 
 @pytest.mark.parametrize("rank,heads", [(64, 3), (128, 1), (512, 16)])

@@ -15,6 +15,7 @@ MODELS = [("tiny", "Q4_K_M", 1), ("tiny128", "Q4_0", 2), ("tiny", "Q8_0", 3), ("
           ("tiny", "Q2_K_mix", 11)]          # one launch mixes formats of both kernel instantiations
 GOLD = np.load(os.path.join(os.path.dirname(__file__), "golden", "tiny_model.npz"))
 TOKENS = [int(t) for t in GOLD["tokens"]]
+SHARP = {64: 6.0, 128: 5.0}          # gains of a norm that spread scores
 
 
 def _model(tmp_models, arch, ftype, seed):
@@ -334,13 +335,13 @@ def test_long_context_uses_more_attention_splits_and_matches_oracle(native_lib, 
     eng.close()
 
 
-@pytest.mark.parametrize("how", ["batch", "batch_of_others", "two", "decode_n", "forward", "twice", "rewind"])
+@pytest.mark.parametrize("how", ["batch", "batch_of_others", "two", "decode_n", "forward", "twice", "rewind", "sample", "prefill"])
 def test_a_set_token_enters_the_next_step_whichever_it_is(native_lib, tmp_models, how):
     """A token set on the host reaches batched steps (with and without set tokens beside it), single ones, runs of steps and plain forward
-    passes; the last one set counts, and a rewind's token replaces it."""
+    passes; the last one set counts, and a rewind's, a sampled or a prompt's token replaces it."""
     from oracle.llama_ref import RefModel
     path = _model(tmp_models, "tiny128", "Q4_0", 2)
-    ref = RefModel(path).forward(TOKENS[:13])
+    ref = RefModel(path).forward(TOKENS[:24])
     eng = _engine(path, max_seqs=5)
     for s in range(5):
         eng.ensure_pages(s, 32)
@@ -362,6 +363,23 @@ def test_a_set_token_enters_the_next_step_whichever_it_is(native_lib, tmp_models
     elif how == "rewind":
         eng.rewind(0, 12, TOKENS[12], TOKENS[:12])
         eng.decode([0])
+    elif how == "twice":                                       # set, stepped, set again
+        eng.decode([3, 0, 1, 2])
+        assert np.abs(eng.logits(0) - ref[12]).max() <= LOGIT_TOL
+        eng.set_token(0, TOKENS[13])
+        eng.decode([2, 3, 1, 0])
+        ref = ref[1:]
+    elif how == "sample":                                      # of the prompt's logits
+        tok = eng.sample(0)
+        assert tok == int(np.argmax(ref[11]))
+        eng.decode([3, 0, 1, 2])
+        ref = RefModel(path).forward(TOKENS[:12] + [tok])
+    elif how == "prefill":
+        eng.prefill(0, TOKENS[12:21])
+        assert np.abs(eng.logits(0) - ref[20]).max() <= LOGIT_TOL
+        tok = eng.sample(0)
+        eng.decode([3, 0, 1, 2])
+        ref = RefModel(path).forward(TOKENS[:21] + [tok])[9:]
     else:
         eng.forward_pending(0)
     assert np.abs(eng.logits(0) - ref[12]).max() <= LOGIT_TOL
@@ -447,3 +465,58 @@ def test_launches_of_a_prompt_are_counted(native_lib, tmp_models, monkeypatch):
         eng.prefill(0, [5 + i % 600 for i in range(n)])
         assert eng.launch_count() - before == kernels, n
     eng.close()
+
+
+def lagging_growth(s, block, bar=8):
+    """[rows, blocks]: where a row's maximum over a block of its visible scores (log2; the others -inf) exceeds by more than `bar` the one that its
+    weights are taken against, which moves only then; the first block, which sets it, aside."""
+    m, out = np.full(len(s), -np.inf), []
+    for b in range(0, s.shape[1], block):
+        mx = s[:, b:b + block].max(1)
+        grow = mx > m + bar
+        out.append(grow & (m > -np.inf))
+        m = np.where(grow, mx, m)
+    return np.array(out).T
+
+
+@pytest.mark.parametrize("head", [64, 128])
+def test_prompts_whose_later_keys_outweigh_the_first(native_lib, tmp_models, monkeypatch, head):
+    """Attention on tensor memory rescales a row's sum where a later block of 128 keys raises its maximum by more than 2^8: in some rows of a warp and not in
+    others, in the second block and later ones. One layer whose queries and keys are large, so that scores are spread over +-30; every length's last row
+    against the oracle.
+    Bar: a score of spread 9 (natural units) of f16 queries and keys is off by 9 * 2^-11 * sqrt(2/3) = 4e-3, and so are weights and rows; five times that."""
+    from llama_cpp import synth
+    from llama_cpp.gguf_file import GGUFFile
+    from oracle import llama_ref
+    monkeypatch.setitem(synth.ARCHS, f"one{head}", synth.Arch(f"one{head}", 1, 512, 512 // head, 2, 1024, 1024))
+    path = _model(tmp_models, f"one{head}", "Q8_0", 3)
+    with open(path, "rb") as f:
+        raw = bytearray(f.read())
+    t = GGUFFile(path).tensors["blk.0.attn_norm.weight"]
+    gain = np.frombuffer(raw, np.float32, 512, t.offset) * np.float32(SHARP[head])
+    raw[t.offset:t.offset + 4 * 512] = gain.tobytes()
+    with open(path + ".sharp", "wb") as f:
+        f.write(raw)
+    n = 700
+    prompt = [int(x) for x in np.random.default_rng(head).integers(3, 700, size=n)]
+    model = llama_ref.RefModel(path + ".sharp")
+    ref, c, w = model.forward(prompt), model.cfg, model.w
+    h = llama_ref.rmsnorm(w["token_embd.weight"][prompt], w["blk.0.attn_norm.weight"], c.rms_eps)
+    q = llama_ref.rope((h @ w["blk.0.attn_q.weight"].T).reshape(n, c.n_head, head), np.arange(n), model.freqs)
+    k = np.repeat(model.k_cache[0].astype(np.float32), c.n_head // 2, axis=1)
+    scores = np.where(np.tri(n, dtype=bool), np.einsum("thd,shd->hts", q, k) / np.sqrt(head) * np.log2(np.e), -np.inf)
+    grows = np.array([lagging_growth(s, 128) for s in scores])                     # [head, row, block]
+    assert 4 < np.std(scores[:, np.tri(n, dtype=bool)]) / np.log2(np.e) < 11
+    lengths = [m for m in range(129, n + 1) if grows[:, m - 1, 1:].any() and m % 3 != 1][::6] + [129, 256, 300, 384, 512]
+    last = {((m - 1) % 512 % 128) // 32 for m in lengths}
+    assert len(lengths) > 20 and last == {0, 1, 2, 3} and all(grows[:, [m - 1 for m in lengths], b].any() for b in (1, 2, 3))
+    assert any(grows[i, r:r + 32, b].any() and not grows[i, r:r + 32, b].all() for i in range(c.n_head) for b in (1, 2, 3) for r in range(128 * b, 640, 32))
+    eng = _engine(path + ".sharp", n_ctx=n + 8, bt=64)
+    eng.ensure_pages(0, n)
+    for m in lengths:
+        eng.seq_begin(0, 0, [], _greedy())
+        eng.prefill(0, prompt[:m])
+        off = eng.logits(0) - ref[m - 1]
+        assert np.sqrt((off ** 2).mean()) < 2e-2 * ref[m - 1].std(), m
+    eng.close()
+    os.remove(path + ".sharp")
