@@ -422,8 +422,8 @@ __global__ void __launch_bounds__(LC_THREADS, 1) latent_attn_tc_kernel(const __g
 // ---------------------------------------------------------------- host side
 // Rows of 64-column parts that fit shared memory beside the queries (9 of them), whole chunks of output columns, pages of whole blocks; of
 // the step only what the few-token kernels do not take (see softmax_tc.cu). 16 heads, rows of 512 + 64, us a layer with the preparation,
-// mma.sync / here: a prompt of 9 tokens 52 / 36, of 64 93 / 44, of 255 120 / 63; 32 prompts of 60 568 / 212; one token of each of 32 sequences
-// behind 60 208 / 38, behind 1900 2087 / 114; 512 tokens beside 31 sequences that decode behind 500, 869 / 97.
+// mma.sync / here: a prompt of 9 tokens 52 / 25, of 64 93 / 25, of 255 120 / 32; 32 prompts of 60 568 / 93; one token of each of 32 sequences
+// behind 60 208 / 26, behind 1900 2087 / 91; 512 tokens beside 31 sequences that decode behind 500, 869 / 56.
 bool latent_attn_takes_tc(const LatentAttnArgs& a, int T) {
     static const bool no_mma = getenv("B2_NO_ATTN_MMA") != nullptr;        // tuning aid: scalar attention for prompts too
     const int parts = (a.rank + a.dr + LC_PART - 1) / LC_PART;
