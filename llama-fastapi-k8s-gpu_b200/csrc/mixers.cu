@@ -959,7 +959,7 @@ bool window_attn_leaves_rounded(const WindowAttnArgs& a, int T) { return window_
 // output of all four queries. Nothing is less than 32 bits. Blocks start at multiples of 64 keys and are summed up in ranges of 128, whose sums meet in
 // the order of the keys: a row's bits depend neither on the tile that it is in nor on `company`, the CTAs of a cluster that share a tile's ranges (and then its
 // queries' sums over ranges) where a step has too few tiles to fill the GPU.
-// Bound by shared-memory reads. (459 tokens of 8 heads of 128 in two sequences: 105 us with a CTA per token and head, every key read from L2 by each; 60 with one
+// Bound by its instructions on the SMs that have a CTA (issue slots 60 %, multiply-adds 37 %, the shared-memory pipe 22 %, by counters) and by the longest tile. (459 tokens of 8 heads of 128 in two sequences: 105 us with a CTA per token and head, every key read from L2 by each; 60 with one
 // warp a query group and blocks of 32 keys, 35 here. 900 tokens, a whole prompt of two layers: 1044 -> 622 us. A step of few tokens behind many keys, two layers
 // with a window of 1024: 20 tokens 323 -> 249, 64 tokens 432 -> 306. Ranges of 256 give a window of 300 too few to share:
 // 32 tokens 245 us against 227, of 237 before.)
