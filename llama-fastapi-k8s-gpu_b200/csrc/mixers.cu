@@ -959,10 +959,10 @@ bool window_attn_leaves_rounded(const WindowAttnArgs& a, int T) { return window_
 // output of all four queries. Nothing is less than 32 bits. Blocks start at multiples of 64 keys and are summed up in ranges of 128, whose sums meet in
 // the order of the keys: a row's bits depend neither on the tile that it is in nor on `company`, the CTAs of a cluster that share a tile's ranges (and then its
 // queries' sums over ranges) where a step has too few tiles to fill the GPU.
-// Bound by its instructions on the SMs that have a CTA (issue slots 60 %, multiply-adds 37 %, the shared-memory pipe 22 %, by counters) and by the longest tile. (459 tokens of 8 heads of 128 in two sequences: 105 us with a CTA per token and head, every key read from L2 by each; 60 with one
-// warp a query group and blocks of 32 keys, 35 here. 900 tokens, a whole prompt of two layers: 1044 -> 622 us. A step of few tokens behind many keys, two layers
-// with a window of 1024: 20 tokens 323 -> 249, 64 tokens 432 -> 306. Ranges of 256 give a window of 300 too few to share:
-// 32 tokens 245 us against 227, of 237 before.)
+// Bound by its instructions on the SMs that have a CTA (issue slots 60 %, multiply-adds 37 %, the shared-memory pipe 22 %, by counters) and by the longest
+// tile. (459 tokens of 8 heads of 128 in two sequences: 105 us with a CTA per token and head, every key read from L2 by each; 60 with one warp a query group
+// and blocks of 32 keys, 37 here. 900 tokens, a whole prompt of two layers: 1044 -> 622 us. A step of few tokens behind many keys, two layers with a window of
+// 1024: 20 tokens 323 -> 249, 64 tokens 432 -> 306. Ranges of 256 give a window of 300 too few to share: 32 tokens 245 us against 227, of 237 before.)
 constexpr int WT_Q = 32, WT_K = 64, WT_OWN = 32, WT_WARPS = 16, WT_D = 128, WT_RANGE = 2;
 constexpr int WT_FEW = 4, WT_SLOTS = 16;                   // queries of a tile whose warps take ranges of their own; ranges of such a CTA between two merges
 
@@ -1060,9 +1060,9 @@ __device__ __forceinline__ void wt_add_half(WtSums& w, const WindowAttnArgs& a, 
 
 // Tiles of few queries (4 and less: portions of two to four tokens; and tokens that come alone, where they are let in) leave seven of eight warps of the above
 // without any. Where a CTA has more than one range of such a tile, a warp takes half a range by itself, keys and values straight from the pages, and the
-// ranges' sums wait in the place of the copies until they are merged, in the same order and to the same bits. Bound by the latency of a page's rows (twelve reads of a lane under way, eight for
-// values). (Steps of two layers, 8 heads of 128, window 1024, behind 1500 keys, us: a CTA per token and head / tiles / here: ten sequences of two tokens
-// 357 / 375 / 289, five 291 / 319 / 273, ten of four 429 / 374 / 288; eight lone tokens beside two 293 / 326 / 271, seven beside 20 382 / 427 / 351,
+// ranges' sums wait in the place of the copies until they are merged, in the same order and to the same bits. Bound by the latency of a page's rows (twelve
+// reads of a lane under way, eight for values). (Steps of two layers, 8 heads of 128, window 1024, behind 1500 keys, us: a CTA per token and head / tiles /
+// here: ten sequences of two tokens 357 / 375 / 289, five 291 / 319 / 273, ten of four 429 / 374 / 288; eight lone tokens beside two 293 / 326 / 271, seven beside 20 382 / 427 / 351,
 // fifteen beside 40 of 4 heads of 64 and a window of 300 289 / 299 / 259. Values read one by one in blocks at a window's edge: 353 where 271 stand.)
 // CTAs x: the tiles from `first_tile` on, `cluster` for each 32 rows, then one for each of the `n_alone` tiles ahead of them.
 __global__ void __launch_bounds__(WT_WARPS * 32, 1) window_attn_tile_kernel(WindowAttnArgs a, RaggedDev r, int first_tile, int cluster, int n_alone) {
@@ -1207,7 +1207,8 @@ __global__ void __launch_bounds__(WT_WARPS * 32, 1) window_attn_tile_kernel(Wind
                 if (q >= nq) break;
                 for (int i = 0; i < company * slots && n0 + i < n_ranges; i++) {
                     const int c = i & (company - 1), row = few ? (i >> __ffs(company) - 1) * WT_FEW + q : q;
-                    const uint32_t at = cluster_address(smem_u32(xs + row * d + (4 * lane < d ? 4 * lane : 0)), lone < 0 ? c : own_rank), at_ml = cluster_address(smem_u32(xml + row), lone < 0 ? c : own_rank);
+                    const int of = lone < 0 ? c : own_rank;
+                    const uint32_t at = cluster_address(smem_u32(xs + row * d + (4 * lane < d ? 4 * lane : 0)), of), at_ml = cluster_address(smem_u32(xml + row), of);
                     const float2 x0 = cluster_load2(at_ml), x1 = cluster_load2(at_ml + rows * 8);
                     const float4 y0 = cluster_load4(at), y1 = cluster_load4(at + rows * d * 4);
                     const float top = fmaxf(M[k], fmaxf(x0.x, x1.x)), ref = top > -INFINITY ? top : 0.f;      // (nothing visible yet: all factors are 0)
